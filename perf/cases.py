@@ -13,6 +13,7 @@ Four kinds, all through the package's public entry points:
 import math
 
 import torch
+import torch.nn.functional as F
 
 from pcf_nat_b200 import NAttention, getNA1dFunction, na1d_fused
 from pcf_nat_b200 import ops
@@ -260,3 +261,106 @@ def tolerance(case):
     if kind == "layer":
         return {"rel": 0.002, "max": 0.012} if case["dtype"] == "fp16" else {"rel": 0.018, "max": 0.1}
     return {"rel": 0.0012, "max": 0.015} if case["dtype"] == "fp16" else {"rel": 0.01, "max": 0.1}
+
+
+def _exact_attention(q, k, v, win, left, dil, scale, bias, valid):
+    """softmax(scale q.k + bias + mask) . v over each token's window; q, k, v (batch, heads, T, C), bias (heads, win) or None,
+    valid (batch,) tokens or None. A neighbour outside the sequence is a zero row under the mask's -100."""
+    T = q.shape[2]
+    lo, hi = left * dil, (win - 1 - left) * dil
+    kp, vp = F.pad(k, (0, 0, lo, hi)), F.pad(v, (0, 0, lo, hi))
+    t = torch.arange(T, device=q.device)
+    n = torch.full((q.shape[0], 1), T, device=q.device) if valid is None else valid.long().view(-1, 1)
+    logits = []
+    for kk in range(win):
+        j = t + (kk - left) * dil
+        off = ((j < 0) | (j >= n) | (t >= n)).to(q.dtype).mul(-100.0)                                # (batch, T)
+        x = (q * kp[:, :, kk * dil:kk * dil + T]).sum(-1) * scale + off[:, None]
+        logits.append(x if bias is None else x + bias[:, kk].view(1, -1, 1))
+    p = torch.softmax(torch.stack(logits, -1), -1)
+    o = torch.zeros_like(q)
+    for kk in range(win):
+        o = o + p[..., kk, None] * vp[:, :, kk * dil:kk * dil + T]
+    return o
+
+
+def _exact_layer(x, w, layout, heads, groups, win, left, dil, scale, valid):
+    """The attention layer on x with its parameters w[...]: projection, heads, attention, merge, projection."""
+    if layout == "channels_first":
+        B, D, T = x.shape
+        y = F.conv1d(x, w["qkv.weight"], w["qkv.bias"], groups=groups)
+        y = y.view(B, D // groups, groups, 3, T).transpose(1, 2).reshape(B, heads, D // heads, 3, T).permute(3, 0, 1, 4, 2)
+    else:
+        B, T, D = x.shape
+        y = F.linear(x, w["qkv.weight"], w["qkv.bias"]).view(B, T, 3, heads, D // heads).permute(2, 0, 3, 1, 4)
+    o = _exact_attention(y[0], y[1], y[2], win, left, dil, scale, w["relative_position_bias"].view(heads, win), valid)
+    if layout == "channels_first":
+        return F.conv1d(o.transpose(2, 3).reshape(B, D, T), w["proj.weight"], w["proj.bias"], groups=groups)
+    return F.linear(o.transpose(1, 2).reshape(B, T, D), w["proj.weight"], w["proj.bias"])
+
+
+def _exact_model(case, m, w, fbank, labels, valid):
+    def norm(x, name):
+        return F.layer_norm(x, x.shape[-1:], w[name + ".weight"], w[name + ".bias"], 1e-5)
+
+    def linear(x, name):
+        return F.linear(x, w[name + ".weight"], w[name + ".bias"])
+
+    win, left = case["win"], case["win"] - 1 - case["win"] // 2
+    x = F.conv1d(fbank, w["front.weight"], w["front.bias"], padding=2).transpose(1, 2)
+    feats, outs, stages = [x], [], len(m.stages)
+    for s in range(stages):
+        for i in range(len(m.stages[s])):
+            name = "stages.%d.%d." % (s, i)
+            attn = {n[len(name) + 5:]: p for n, p in w.items() if n.startswith(name + "attn.")}
+            x = x + _exact_layer(norm(x, name + "norm1"), attn, "channels_last", case["heads"], 1, win, left, 1,
+                                 (x.shape[-1] // case["heads"]) ** -0.5, valid)
+            x = x + linear(F.gelu(linear(norm(x, name + "norm2"), name + "fc1")), name + "fc2")
+        outs.append(x)
+        feats.append(x)
+        if s + 1 < stages:
+            x = linear(torch.cat(feats, -1), "fuse.%d" % s)
+    y = torch.cat(outs, -1)
+    a = torch.softmax(linear(torch.tanh(linear(y, "pool.a")), "pool.b"), 1)
+    mu = (a * y).sum(1)
+    y = torch.cat([mu, ((a * y * y).sum(1) - mu * mu).clamp_min(1e-5).sqrt()], 1)
+    stats = (None, None) if case["train"] else (m.bn.running_mean.double(), m.bn.running_var.double())
+    y = linear(F.batch_norm(y, stats[0], stats[1], w["bn.weight"], w["bn.bias"], case["train"], 0.0, 1e-5), "embed")
+    if labels is None:
+        return y
+    cos = F.linear(F.normalize(y), F.normalize(w["loss.weight"])).clamp(-1 + 1e-7, 1 - 1e-7)
+    target = torch.cos(torch.acos(cos.gather(1, labels[:, None])) + 0.2)
+    return F.cross_entropy(cos.scatter(1, labels[:, None], target) * 30.0, labels)
+
+
+def exact(case, seed):
+    """What ``run`` returns, in 64 bits by plain torch on the same inputs. Not for attention dropout (its mask is the
+    operator's own) and not for the network's larger batches, whose activations do not fit in 64 bits."""
+    kind = case["kind"]
+    if case.get("drop") or (kind == "model" and case["batch"] * case["frames"] > (9600 if case["train"] else 80000)):
+        return None
+    st = prepare(case, seed)
+    train = case.get("train", True)
+    with torch.set_grad_enabled(train):
+        if kind in ("op", "pair"):
+            B, H, T, C, win = (case[n] for n in ("batch", "heads", "T", "C", "win"))
+            left = st["left"] if kind == "pair" else case["left"]
+            q, k, v = (st[n].detach().double().requires_grad_(train) for n in "qkv")
+            r = None if st["rpb"] is None else st["rpb"].detach().double().requires_grad_(train)
+            o = _exact_attention(*(x.view(B, H, T, C) for x in (q, k, v)), win, left, case["dil"], C ** -0.5,
+                                 None if r is None else r.view(H, win), st.get("valid_len")).reshape(B * H, T, C)
+            if not train:
+                return o
+            return (o.detach(),) + torch.autograd.grad(o, [q, k, v] + ([] if r is None else [r]), st["d_o"].double())
+        m = st["layer" if kind == "layer" else "model"]
+        w = {n: p.detach().double().requires_grad_(train) for n, p in m.named_parameters()}
+        valid = (case["T"] if kind == "layer" else case["frames"]) - st["padding"] if "padding" in st else None
+        if kind == "layer":
+            x = st["x"].detach().double().requires_grad_(train)
+            y = _exact_layer(x, w, case["layout"], case["heads"], case["groups"], case["win"], case["win"] - 1 - case["win"] // 2,
+                             case["dil"], (case["dim"] // case["heads"]) ** -0.5, valid)
+            return (y.detach(),) + torch.autograd.grad(y, [x] + list(w.values()), st["d_y"].double()) if train else y
+        out = _exact_model(case, m, w, st["fbank"].double(), st.get("labels"), valid)
+        if not train:
+            return out
+        return out.detach(), torch.cat([g.reshape(-1) for g in torch.autograd.grad(out, list(w.values()))])
