@@ -206,6 +206,40 @@ int na1d_fused_backward_dropout(void* dq, void* dk, void* dv, float* d_rpb, cons
                                 float scale, float drop_p, uint64_t seed, int dtype, void* stream);
 
 /* ------------------------------------------------------------------------------------------
+ * The passes of a transformer block and of attentive statistics pooling that are not contractions (LayerNorm and residual,
+ * GELU, column sums, rounding of parameters, pooling; models/PCF_NATransformer.py:228-303). 16-bit activations of `dtype`,
+ * fp32 parameters and statistics. Rows are dense; D, F, C are multiples of 8, D <= 1024; every pointer 16-byte aligned.
+ * `scratch` holds at least na1d_block_scratch_floats(rows, D, F) floats (column sums leave the CTAs as partial rows and
+ * are added in a fixed order: the same bits from run to run).
+ * ---------------------------------------------------------------------------------------- */
+int64_t na1d_block_scratch_floats(int64_t rows, int64_t D, int64_t F);
+/* y = LN(s) * w + b over rows of D; s = x, or with dx: s = x + dx, rounded and written to `sum`. mean, rstd: (rows) or NULL. */
+int na1d_layer_norm_forward(void* y, void* sum, float* mean, float* rstd, const void* x, const void* dx, const float* w,
+                            const float* b, int64_t rows, int64_t D, float eps, int dtype, void* stream);
+/* dx = gradient of the normalised rows x + res (res may be NULL); sums (3, D): gradients of w and b, column sums of dx. */
+int na1d_layer_norm_backward(void* dx, float* sums, float* scratch, const void* dy, const void* x, const float* mean,
+                             const float* rstd, const float* w, const void* res, int64_t rows, int64_t D, int dtype, void* stream);
+/* y = x Phi(x) (the exact form), n elements (n a multiple of 8). */
+int na1d_gelu_forward(void* y, const void* x, int64_t n, int dtype, void* stream);
+/* dx = dy * d gelu(x), (rows, F); sums (F): column sums of dx. */
+int na1d_gelu_backward(void* dx, float* sums, float* scratch, const void* dy, const void* x, int64_t rows, int64_t F, int dtype,
+                       void* stream);
+/* sums (F) = column sums of x (rows, F). */
+int na1d_column_sums(float* sums, float* scratch, const void* x, int64_t rows, int64_t F, int dtype, void* stream);
+/* Rounds `count` fp32 tensors (DEVICE pointers in the HOST array src, n[i] elements) to 16 bits at out + dst[i] (elements,
+ * multiples of 8; each slot is padded with zeros to a multiple of 8) in one launch; count <= NA1D_CAST_MAX. */
+#define NA1D_CAST_MAX 16
+int na1d_cast_parameters(void* out, const float* const* src, const int64_t* dst, const int64_t* n, int count, int dtype,
+                         void* stream);
+/* out (N, 2C) fp32 = [mu, std] with a = softmax over T of logits (N, T, C), mu = sum a x, std = sqrt(max(sum a x^2 - mu^2,
+ * floor)). stats (3, N, C), for the backward (may be NULL): the logits' maximum, 1 / sum exp, sum a x^2. N <= 65535. */
+int na1d_stats_pool_forward(float* out, float* stats, const void* logits, const void* x, int64_t N, int64_t T,
+                            int64_t C, float floor, int dtype, void* stream);
+int na1d_stats_pool_backward(void* d_logits, void* dx, const float* d_out, const float* out, const float* stats,
+                             const void* logits, const void* x, int64_t N, int64_t T, int64_t C,
+                             float floor, int dtype, void* stream);
+
+/* ------------------------------------------------------------------------------------------
  * Window index arithmetic as the kernels compute it, for bit-exact checking:
  * j_out[t,kk] = t + (kk-left)*dil (int32, (T,win)); in_range[t,kk] = 1 if 0 <= j < T else 0.
  * Restates the implicit pad+unfold indexing of models/PCF_NATransformer.py:158-165.

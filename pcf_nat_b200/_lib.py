@@ -80,6 +80,20 @@ _lib.na1d_fused_forward_strided.restype = _i32
 _lib.na1d_fused_forward_strided.argtypes = [_ptr] * 7 + [_ptr] * 4 + [_i64] * 7 + [_f32, _i32, _ptr]
 _lib.na1d_fused_backward_strided.restype = _i32
 _lib.na1d_fused_backward_strided.argtypes = [_ptr] * 12 + [_i64] + [_ptr] * 7 + [_i64] * 7 + [_f32, _i32, _ptr]
+_lib.na1d_block_scratch_floats.restype = _i64
+_lib.na1d_block_scratch_floats.argtypes = [_i64, _i64, _i64]
+for _name, _args in (
+        ("na1d_layer_norm_forward", [_ptr] * 8 + [_i64, _i64, _f32]),
+        ("na1d_layer_norm_backward", [_ptr] * 9 + [_i64, _i64]),
+        ("na1d_gelu_forward", [_ptr, _ptr, _i64]),
+        ("na1d_gelu_backward", [_ptr] * 5 + [_i64, _i64]),
+        ("na1d_column_sums", [_ptr] * 3 + [_i64, _i64]),
+        ("na1d_cast_parameters", [_ptr] * 4 + [_i32]),
+        ("na1d_stats_pool_forward", [_ptr] * 4 + [_i64] * 3 + [_f32]),
+        ("na1d_stats_pool_backward", [_ptr] * 7 + [_i64] * 3 + [_f32])):
+    _f = getattr(_lib, _name)
+    _f.restype = _i32
+    _f.argtypes = _args + [_i32, _ptr]
 _lib.na1d_tensor_map_cache_stats.restype = _i32
 _lib.na1d_tensor_map_cache_stats.argtypes = [_ptr, _ptr]
 _lib.na1d_set_kernel_family.restype = _i32

@@ -40,6 +40,17 @@ int check_geometry(int64_t N, int64_t heads, int64_t T, int64_t C, int64_t win, 
 // 121 us); the band-out and band-in modes win everywhere (94 against 174 us, 84 against 107 us) and are not affected.
 bool narrow_rows_wide_window(const na1d::Geometry& g) { return g.C == 16 && (g.win - 1) * g.dil + 1 > 17; }
 
+// arguments of the row and column kernels of a transformer block
+int check_block(int64_t rows, int64_t cols, int64_t most_cols, int dtype) {
+    if (dtype != NA1D_BF16 && dtype != NA1D_FP16) return NA1D_ERR_BAD_DTYPE;
+    if (rows <= 0 || cols <= 0 || cols % 8 != 0 || cols > most_cols || rows > INT_MAX / 2 || rows > (1ll << 40) / cols) return NA1D_ERR_BAD_SHAPE;
+    return NA1D_OK;
+}
+template <typename... P> int check_pointers(const P*... p) {
+    if (((p == nullptr) || ...)) return NA1D_ERR_NULL_POINTER;
+    return (aligned16(p) && ...) ? NA1D_OK : NA1D_ERR_MISALIGNED;
+}
+
 #define NA1D_REQUIRE_PTR(p) do { if ((p) == nullptr) return NA1D_ERR_NULL_POINTER; } while (0)
 #define NA1D_REQUIRE_ALIGNED(p) do { if (!aligned16(p)) return NA1D_ERR_MISALIGNED; } while (0)
 
@@ -347,6 +358,74 @@ int na1d_fused_backward_dropout(void* dq, void* dk, void* dv, float* d_rpb, cons
     if (!na1d::tc_bwd_supports(g, rpb != nullptr, d_rpb != nullptr)) return NA1D_ERR_UNSUPPORTED;
     return cuda_status(na1d::tc_fused_bwd_dropout(dq, dk, dv, d_rpb, d_o, q, k, v, lse, rpb, valid_len, scratch, (size_t)scratch_floats,
                                                   g, dtype, cfg, (cudaStream_t)stream));
+}
+
+// ---- row and column kernels of a transformer block (na1d_block.cu)
+int64_t na1d_block_scratch_floats(int64_t rows, int64_t D, int64_t F) {
+    if (rows <= 0 || D < 0 || F < 0 || rows > INT_MAX / 2 || D > (1 << 20) || F > (1 << 20)) return 0;
+    const int64_t cols = 3 * D > 256 ? 3 * D : 256, n = na1d::block_partial_rows(rows) * cols;
+    return n > F ? n : F;
+}
+int na1d_layer_norm_forward(void* y, void* sum, float* mean, float* rstd, const void* x, const void* dx, const float* w,
+                            const float* b, int64_t rows, int64_t D, float eps, int dtype, void* stream) {
+    if (int s = check_pointers(y, x, w, b)) return s;
+    if ((dx == nullptr) != (sum == nullptr) || (mean == nullptr) != (rstd == nullptr)) return NA1D_ERR_NULL_POINTER;
+    if (!aligned16(sum) || !aligned16(dx)) return NA1D_ERR_MISALIGNED;
+    if (int s = check_block(rows, D, 1024, dtype)) return s;
+    return cuda_status(na1d::block_ln_fwd(y, sum, mean, rstd, x, dx, w, b, (int)rows, (int)D, eps, dtype, (cudaStream_t)stream));
+}
+int na1d_layer_norm_backward(void* dx, float* sums, float* scratch, const void* dy, const void* x, const float* mean,
+                             const float* rstd, const float* w, const void* res, int64_t rows, int64_t D, int dtype, void* stream) {
+    if (int s = check_pointers(dx, sums, scratch, dy, x, mean, rstd, w)) return s;
+    if (!aligned16(res)) return NA1D_ERR_MISALIGNED;
+    if (int s = check_block(rows, D, 1024, dtype)) return s;
+    return cuda_status(na1d::block_ln_bwd(dx, sums, scratch, dy, x, mean, rstd, w, res, (int)rows, (int)D, dtype, (cudaStream_t)stream));
+}
+int na1d_gelu_forward(void* y, const void* x, int64_t n, int dtype, void* stream) {
+    if (int s = check_pointers(y, x)) return s;
+    if (dtype != NA1D_BF16 && dtype != NA1D_FP16) return NA1D_ERR_BAD_DTYPE;
+    if (n <= 0 || n % 8 != 0 || n > (1ll << 40)) return NA1D_ERR_BAD_SHAPE;
+    return cuda_status(na1d::block_gelu_fwd(y, x, n, dtype, (cudaStream_t)stream));
+}
+int na1d_gelu_backward(void* dx, float* sums, float* scratch, const void* dy, const void* x, int64_t rows, int64_t F, int dtype,
+                       void* stream) {
+    if (int s = check_pointers(dx, sums, scratch, dy, x)) return s;
+    if (int s = check_block(rows, F, 1 << 20, dtype)) return s;
+    return cuda_status(na1d::block_gelu_bwd(dx, sums, scratch, dy, x, (int)rows, (int)F, dtype, (cudaStream_t)stream));
+}
+int na1d_column_sums(float* sums, float* scratch, const void* x, int64_t rows, int64_t F, int dtype, void* stream) {
+    if (int s = check_pointers(sums, scratch, x)) return s;
+    if (int s = check_block(rows, F, 1 << 20, dtype)) return s;
+    return cuda_status(na1d::block_column_sums(sums, scratch, x, (int)rows, (int)F, dtype, (cudaStream_t)stream));
+}
+int na1d_cast_parameters(void* out, const float* const* src, const int64_t* dst, const int64_t* n, int count, int dtype,
+                         void* stream) {
+    if (int s = check_pointers(out)) return s;
+    NA1D_REQUIRE_PTR(src); NA1D_REQUIRE_PTR(dst); NA1D_REQUIRE_PTR(n);
+    if (dtype != NA1D_BF16 && dtype != NA1D_FP16) return NA1D_ERR_BAD_DTYPE;
+    if (count <= 0 || count > NA1D_CAST_MAX) return NA1D_ERR_TOO_LARGE;
+    for (int i = 0; i < count; ++i) {
+        NA1D_REQUIRE_PTR(src[i]);
+        if (dst[i] < 0 || dst[i] % 8 != 0 || n[i] <= 0 || n[i] > INT_MAX / 16) return NA1D_ERR_BAD_SHAPE;
+    }
+    return cuda_status(na1d::block_cast(out, src, dst, n, count, dtype, (cudaStream_t)stream));
+}
+int na1d_stats_pool_forward(float* out, float* stats, const void* logits, const void* x, int64_t N, int64_t T,
+                            int64_t C, float floor, int dtype, void* stream) {
+    if (int s = check_pointers(out, logits, x)) return s;
+    if (!aligned16(stats)) return NA1D_ERR_MISALIGNED;
+    if (int s = check_block(T, C, 1 << 20, dtype)) return s;
+    if (N <= 0 || N > 65535 || T > (1 << 20)) return NA1D_ERR_BAD_SHAPE;
+    return cuda_status(na1d::block_pool_fwd(out, stats, logits, x, (int)N, (int)T, (int)C, floor, dtype, (cudaStream_t)stream));
+}
+int na1d_stats_pool_backward(void* d_logits, void* dx, const float* d_out, const float* out, const float* stats,
+                             const void* logits, const void* x, int64_t N, int64_t T, int64_t C,
+                             float floor, int dtype, void* stream) {
+    if (int s = check_pointers(d_logits, dx, d_out, out, stats, logits, x)) return s;
+    if (int s = check_block(T, C, 1 << 20, dtype)) return s;
+    if (N <= 0 || N > 65535 || T > (1 << 20)) return NA1D_ERR_BAD_SHAPE;
+    return cuda_status(na1d::block_pool_bwd(d_logits, dx, d_out, out, stats, logits, x, (int)N, (int)T, (int)C, floor, dtype,
+                                            (cudaStream_t)stream));
 }
 
 int na1d_window_index(int32_t* j_out, uint8_t* in_range, int64_t T, int64_t win, int64_t left, int64_t dil,

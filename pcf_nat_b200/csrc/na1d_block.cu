@@ -1,0 +1,538 @@
+// Row and column kernels around the projections of a transformer block and of the statistics pooling: residual add +
+// LayerNorm, GELU, their backward passes with the parameter and bias gradients (column sums) taken in the same pass, the
+// rounding of a block's fp32 parameters to 16 bits in one launch, and attentive statistics pooling.
+//
+// All of them are bound by HBM: every 16-bit activation is read once and every result written once, all arithmetic is fp32.
+// A lane owns 8 adjacent columns (one 16-byte access), a warp 256 columns of one row. Column sums stay in the lane's
+// registers over all rows of its CTA, meet in shared memory once, and leave as one fp32 row per CTA that a second small
+// kernel adds up in a fixed order: no atomics, the same bits from run to run.
+#include "../../include/na1d_b200.h"
+#include "na1d_internal.h"
+#include "na1d_tc_common.cuh"
+
+namespace na1d {
+namespace {
+
+constexpr int kWarps = 8, kRowThreads = kWarps * 32;
+
+__device__ __forceinline__ float warp_sum(float x) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+    return x;
+}
+using tc::fast_exp2;
+using tc::fast_rcp;
+template <typename E> __device__ __forceinline__ void load8(const E* p, float* f) {
+    Cvt<E>::unpack(*reinterpret_cast<const uint4*>(p), f);
+}
+template <typename E> __device__ __forceinline__ void store8(E* p, const float* f) { *reinterpret_cast<uint4*>(p) = Cvt<E>::pack(f); }
+// through 16 bits and back: what a reader of the stored tensor sees
+template <typename E> __device__ __forceinline__ void round8(float* f) {
+    const uint4 u = Cvt<E>::pack(f);
+    Cvt<E>::unpack(u, f);
+}
+__device__ __forceinline__ void load8f(const float* p, float* f) {
+    const float4 a = __ldg(reinterpret_cast<const float4*>(p)), b = __ldg(reinterpret_cast<const float4*>(p) + 1);
+    f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w; f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
+}
+
+// ---------------------------------------------------------------- LayerNorm
+// y = LN(s) w + b with s = x, or s = round(x + dx) written to `sum` (the residual stream): one warp per row, the row stays in
+// registers (mean first, then the centred squares). 153600 rows of 256: 231 us (framework kernel) + 37 us (residual add)
+// before.
+template <typename E, int CH>
+__global__ void __launch_bounds__(kRowThreads) ln_fwd_kernel(E* __restrict__ y, E* __restrict__ sum, float* __restrict__ mean,
+                                                             float* __restrict__ rstd, const E* __restrict__ x,
+                                                             const E* __restrict__ dx, const float* __restrict__ w,
+                                                             const float* __restrict__ b, int rows, int D, float eps) {
+    const int lane = threadIdx.x & 31;
+    const float inv_d = 1.f / (float)D;
+    for (int row = blockIdx.x * kWarps + (threadIdx.x >> 5); row < rows; row += gridDim.x * kWarps) {
+        const size_t base = (size_t)row * D;
+        float v[CH][8], s = 0.f;
+#pragma unroll
+        for (int c = 0; c < CH; ++c) {
+            const int col = c * 256 + lane * 8;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) v[c][i] = 0.f;
+            if (col < D) {
+                load8(x + base + col, v[c]);
+                if (dx) {
+                    float r[8];
+                    load8(dx + base + col, r);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) v[c][i] += r[i];
+                    round8<E>(v[c]);
+                    store8(sum + base + col, v[c]);
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < 8; ++i) s += v[c][i];
+        }
+        const float mu = warp_sum(s) * inv_d;
+        float q = 0.f;
+#pragma unroll
+        for (int c = 0; c < CH; ++c)
+            if (c * 256 + lane * 8 < D) {
+#pragma unroll
+                for (int i = 0; i < 8; ++i) q = fmaf(v[c][i] - mu, v[c][i] - mu, q);
+            }
+        const float rs = rsqrtf(fmaf(warp_sum(q), inv_d, eps));
+#pragma unroll
+        for (int c = 0; c < CH; ++c) {
+            const int col = c * 256 + lane * 8;
+            if (col < D) {
+                float wf[8], bf[8];
+                load8f(w + col, wf);
+                load8f(b + col, bf);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) v[c][i] = fmaf((v[c][i] - mu) * rs, wf[i], bf[i]);
+                store8(y + base + col, v[c]);
+            }
+        }
+        if (mean && lane == 0) { mean[row] = mu; rstd[row] = rs; }
+    }
+}
+
+// Adds up the warps' column sums (K sums of 8 columns per lane and chunk) through shared memory and writes the CTA's row of
+// partial sums: part[((cta * K) + k) * D + column].
+template <int K, int CH>
+__device__ __forceinline__ void cta_column_sums(float (&acc)[K][CH][8], float* part, int cta, int D, int col0) {
+    __shared__ float sm[kWarps][256];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+#pragma unroll
+        for (int c = 0; c < CH; ++c) {
+            __syncthreads();
+#pragma unroll
+            for (int i = 0; i < 8; ++i) sm[warp][i * 32 + lane] = acc[k][c][i];   // conflict-free: column 8 lane + i at i*32 + lane
+            __syncthreads();
+            const int col = col0 + c * 256 + threadIdx.x, at = (threadIdx.x & 7) * 32 + (threadIdx.x >> 3);
+            float s = 0.f;
+#pragma unroll
+            for (int q = 0; q < kWarps; ++q) s += sm[q][at];
+            if (col < D) part[((size_t)cta * K + k) * D + col] = s;
+        }
+}
+
+// out[i] = sum over g of part[g * n + i], in a fixed order: 32 warps share the rows of a group of 32 columns (at most 444 rows:
+// 14 independent loads a thread)
+__global__ void __launch_bounds__(1024) partial_sum_kernel(float* __restrict__ out, const float* __restrict__ part, int n, int groups) {
+    __shared__ float sm[32][33];
+    const int lane = threadIdx.x & 31, sub = threadIdx.x >> 5, i = blockIdx.x * 32 + lane;
+    float s = 0.f;
+    if (i < n) {
+#pragma unroll 8
+        for (int g = sub; g < groups; g += 32) s += __ldg(part + (size_t)g * n + i);
+    }
+    sm[sub][lane] = s;
+    __syncthreads();
+    const float t = warp_sum(sm[lane][sub]);   // warp q adds up column q
+    if (lane == 0 && blockIdx.x * 32 + sub < n) out[blockIdx.x * 32 + sub] = t;
+}
+
+// dx = rstd (g - mean(g) - xhat mean(g xhat)) + res with g = dy w, and the column sums of dy xhat (weight gradient), dy (bias
+// gradient) and dx as stored (the bias gradient of the projection whose output was added to the residual stream).
+// 38400 rows of 256: 35 us (input gradient) + 173 us (parameter gradients) + 47 us (bias gradient) before.
+template <typename E, int CH>
+__global__ void __launch_bounds__(kRowThreads) ln_bwd_kernel(E* __restrict__ dx, float* __restrict__ part, const E* __restrict__ dy,
+                                                             const E* __restrict__ x, const float* __restrict__ mean,
+                                                             const float* __restrict__ rstd, const float* __restrict__ w,
+                                                             const E* __restrict__ res, int rows, int D) {
+    const int lane = threadIdx.x & 31;
+    const float inv_d = 1.f / (float)D;
+    float acc[3][CH][8], wf[CH][8];
+#pragma unroll
+    for (int c = 0; c < CH; ++c) {
+        const int col = c * 256 + lane * 8;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) { acc[0][c][i] = acc[1][c][i] = acc[2][c][i] = 0.f; wf[c][i] = 0.f; }
+        if (col < D) load8f(w + col, wf[c]);
+    }
+    for (int row = blockIdx.x * kWarps + (threadIdx.x >> 5); row < rows; row += gridDim.x * kWarps) {
+        const size_t base = (size_t)row * D;
+        const float mu = __ldg(mean + row), rs = __ldg(rstd + row);
+        float g[CH][8], h[CH][8], r[CH][8], a = 0.f, b = 0.f;
+#pragma unroll
+        for (int c = 0; c < CH; ++c) {
+            const int col = c * 256 + lane * 8;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) { g[c][i] = 0.f; h[c][i] = mu; r[c][i] = 0.f; }
+            if (col < D) {
+                load8(dy + base + col, g[c]);
+                load8(x + base + col, h[c]);
+                if (res) load8(res + base + col, r[c]);
+            }
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                h[c][i] = (h[c][i] - mu) * rs;
+                acc[0][c][i] = fmaf(g[c][i], h[c][i], acc[0][c][i]);
+                acc[1][c][i] += g[c][i];
+                g[c][i] *= wf[c][i];
+                a += g[c][i];
+                b = fmaf(g[c][i], h[c][i], b);
+            }
+        }
+        a = warp_sum(a) * inv_d;
+        b = warp_sum(b) * inv_d;
+#pragma unroll
+        for (int c = 0; c < CH; ++c) {
+            const int col = c * 256 + lane * 8;
+            if (col < D) {
+                float o[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) o[i] = fmaf(rs, g[c][i] - a - h[c][i] * b, r[c][i]);
+                const uint4 u = Cvt<E>::pack(o);
+                *reinterpret_cast<uint4*>(dx + base + col) = u;
+                Cvt<E>::unpack(u, o);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) acc[2][c][i] += o[i];
+            }
+        }
+    }
+    cta_column_sums<3, CH>(acc, part, blockIdx.x, D, 0);
+}
+
+// ---------------------------------------------------------------- GELU (exact form x Phi(x)) and column sums
+// Phi(x) = erfc(-x / sqrt 2) / 2 from Abramowitz & Stegun 7.1.26 (erfc(z) = t (a1 + t (a2 + ...)) e^{-z^2}, t = 1 / (1 + p z),
+// z >= 0, |error| <= 1.5e-7): the negative tail is a product, not 1 - erf, so it keeps its relative accuracy, and e^{-x^2/2} is
+// shared with the density in the derivative. Two special-function operations and ~14 fp32 operations a value instead of the
+// library erff's ~25 with a branch, which is what bound the framework kernel (178 us for 153600 x 1024 values, 98 us of HBM
+// time).
+__device__ __forceinline__ void phi(float x, float& cdf, float& e) {
+    const float z = fabsf(x) * 0.70710678118654752f;
+    const float t = fast_rcp(fmaf(0.3275911f, z, 1.f));
+    e = fast_exp2(x * x * (-0.5f * kLog2e));
+    float p = fmaf(t, 1.061405429f, -1.453152027f);
+    p = fmaf(t, p, 1.421413741f);
+    p = fmaf(t, p, -0.284496736f);
+    p = fmaf(t, p, 0.254829592f);
+    const float tail = 0.5f * p * t * e;
+    cdf = x >= 0.f ? 1.f - tail : tail;
+}
+__device__ __forceinline__ float gelu(float x) {
+    float c, e;
+    phi(x, c, e);
+    return x * c;
+}
+
+template <typename E>
+__global__ void __launch_bounds__(256) gelu_fwd_kernel(E* __restrict__ y, const E* __restrict__ x, long long chunks) {
+    // four independent 16-byte loads in flight per thread
+    const long long stride = (long long)gridDim.x * 256;
+    for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < chunks; i += 4 * stride) {
+        uint4 u[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (i + k * stride < chunks) u[k] = reinterpret_cast<const uint4*>(x)[i + k * stride];
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (i + k * stride < chunks) {
+                float f[8];
+                Cvt<E>::unpack(u[k], f);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) f[j] = gelu(f[j]);
+                reinterpret_cast<uint4*>(y)[i + k * stride] = Cvt<E>::pack(f);
+            }
+    }
+}
+
+// Column sums of a (rows, F) matrix with leading dimension F; GELU: the matrix is dx = dy gelu'(x), which is written too
+// (38400 x 1024: 63 us backward + 47 us bias gradient before).
+// CTA (bx, by): columns 256 bx .. +255, rows by * 8 + warp, stepping by 8 gridDim.y.
+template <typename E, bool GELU>
+__global__ void __launch_bounds__(kRowThreads) column_kernel(E* __restrict__ dx, float* __restrict__ part, const E* __restrict__ dy,
+                                                             const E* __restrict__ x, int rows, int F) {
+    const int lane = threadIdx.x & 31, col = blockIdx.x * 256 + lane * 8;
+    float acc[1][1][8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) acc[0][0][i] = 0.f;
+    constexpr int U = GELU ? 2 : 4;
+    const int step = gridDim.y * kWarps;
+    if (col < F)
+        for (int row = blockIdx.y * kWarps + (threadIdx.x >> 5); row < rows; row += U * step) {
+            uint4 a[U], b[U];
+#pragma unroll
+            for (int k = 0; k < U; ++k)
+                if (row + k * step < rows) {
+                    const size_t at = (size_t)(row + k * step) * F + col;
+                    a[k] = *reinterpret_cast<const uint4*>(dy + at);
+                    if constexpr (GELU) b[k] = *reinterpret_cast<const uint4*>(x + at);
+                }
+#pragma unroll
+            for (int k = 0; k < U; ++k)
+                if (row + k * step < rows) {
+                    float g[8];
+                    Cvt<E>::unpack(a[k], g);
+                    if constexpr (GELU) {
+                        float v[8];
+                        Cvt<E>::unpack(b[k], v);
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) {
+                            float c, e;
+                            phi(v[i], c, e);
+                            g[i] *= fmaf(v[i] * 0.3989422804014327f, e, c);   // Phi(x) + x phi(x)
+                        }
+                        const uint4 u = Cvt<E>::pack(g);
+                        *reinterpret_cast<uint4*>(dx + (size_t)(row + k * step) * F + col) = u;
+                        Cvt<E>::unpack(u, g);
+                    }
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) acc[0][0][i] += g[i];
+                }
+        }
+    cta_column_sums<1, 1>(acc, part, blockIdx.y, F, blockIdx.x * 256);
+}
+
+// ---------------------------------------------------------------- parameters to 16 bits, several tensors in one launch
+struct CastList {
+    const float* src[NA1D_CAST_MAX];
+    long long dst[NA1D_CAST_MAX];   // element offset in the packed output, a multiple of 8
+    int n[NA1D_CAST_MAX];
+    int first[NA1D_CAST_MAX + 1];   // first CTA of each tensor
+    int count;
+};
+constexpr int kCastPerCta = 256 * 8;
+template <typename E> __global__ void __launch_bounds__(256) cast_kernel(E* __restrict__ out, const __grid_constant__ CastList L) {
+    int k = 0;
+    while (k + 1 < L.count && (int)blockIdx.x >= L.first[k + 1]) ++k;
+    const int i0 = ((int)blockIdx.x - L.first[k]) * kCastPerCta + threadIdx.x * 8, n = L.n[k];
+    if (i0 >= n) return;
+    const float* s = L.src[k] + i0;
+    float f[8];
+    if (i0 + 8 <= n && (reinterpret_cast<uintptr_t>(s) & 15u) == 0) {
+        load8f(s, f);
+    } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) f[i] = i0 + i < n ? s[i] : 0.f;
+    }
+    *reinterpret_cast<uint4*>(out + L.dst[k] + i0) = Cvt<E>::pack(f);   // the slot of each tensor is padded to 8 elements
+}
+
+// ---------------------------------------------------------------- attentive statistics pooling
+// a = softmax over time of the logits; mu = sum a x, std = sqrt(max(sum a x^2 - mu^2, floor)), per channel. One pass: a lane
+// keeps the running maximum and the three sums of its 8 channels; the CTA's warps share the time axis and meet in shared
+// memory. Reads logits and x once (512 x 300 x 1536: 0.94 GB; the framework's chain of fp32 copies, strided softmax, products
+// and sums took 6.2 ms there).
+constexpr int kPoolWarps = 8;
+template <typename E>
+__global__ void __launch_bounds__(kPoolWarps * 32) pool_fwd_kernel(float* __restrict__ out, float* __restrict__ stats,
+                                                                  const E* __restrict__ logits, const E* __restrict__ x, int T, int C,
+                                                                  float floor_var) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, col = blockIdx.x * 256 + lane * 8;
+    const size_t base = (size_t)blockIdx.y * T * C;
+    float m[8], s[8], sx[8], sxx[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) { m[i] = -INFINITY; s[i] = sx[i] = sxx[i] = 0.f; }
+    if (col < C)
+#pragma unroll 2
+        for (int t = warp; t < T; t += kPoolWarps) {
+            float l[8], v[8];
+            load8(logits + base + (size_t)t * C + col, l);
+            load8(x + base + (size_t)t * C + col, v);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const float z = l[i];
+                if (z > m[i]) {   // a new maximum: rescale (rare after the first steps)
+                    const float r = fast_exp2((m[i] - z) * kLog2e);
+                    s[i] *= r; sx[i] *= r; sxx[i] *= r;
+                    m[i] = z;
+                }
+                // (an infinite logit gives NaN, as the softmax of it does; a logit of -inf next to finite ones gives 0)
+                const float p = m[i] == -INFINITY && z == -INFINITY ? 0.f : fast_exp2((z - m[i]) * kLog2e);
+                s[i] += p;
+                const float px = p * v[i];
+                sx[i] += px;
+                sxx[i] = fmaf(px, v[i], sxx[i]);
+            }
+        }
+    __shared__ float sm[4][kPoolWarps][256];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        sm[0][warp][i * 32 + lane] = m[i];
+        sm[1][warp][i * 32 + lane] = s[i];
+        sm[2][warp][i * 32 + lane] = sx[i];
+        sm[3][warp][i * 32 + lane] = sxx[i];
+    }
+    __syncthreads();
+    const int c = blockIdx.x * 256 + threadIdx.x, at = (threadIdx.x & 7) * 32 + (threadIdx.x >> 3);
+    if (c >= C) return;
+    float M = -INFINITY;
+#pragma unroll
+    for (int w = 0; w < kPoolWarps; ++w) M = fmaxf(M, sm[0][w][at]);
+    float S = 0.f, X = 0.f, XX = 0.f;
+#pragma unroll
+    for (int w = 0; w < kPoolWarps; ++w) {
+        const float r = sm[0][w][at] == -INFINITY ? 0.f : fast_exp2((sm[0][w][at] - M) * kLog2e);
+        S = fmaf(sm[1][w][at], r, S);
+        X = fmaf(sm[2][w][at], r, X);
+        XX = fmaf(sm[3][w][at], r, XX);
+    }
+    const float inv = 1.f / S, mu = X * inv, e2 = XX * inv;
+    const float var = fmaf(-mu, mu, e2);
+    float* o = out + (size_t)blockIdx.y * 2 * C;
+    o[c] = mu;
+    o[C + c] = sqrtf(var < floor_var ? floor_var : var);
+    if (stats) {   // (3, N, C); the maximum and the sum apart: their logarithm's sum loses the sum next to a large maximum
+        const size_t at3 = (size_t)blockIdx.y * C + c, plane = (size_t)gridDim.y * C;
+        stats[at3] = M;
+        stats[at3 + plane] = inv;
+        stats[at3 + 2 * plane] = e2;
+    }
+}
+
+// d_logits = a (q - sum a q) and dx = a (dm + 2 x dv) with q = x dm + x^2 dv, dv = d_std / (2 std) where the variance is not at
+// its floor, dm = d_mu - 2 mu dv. The inner sum is mu dm + E[x^2] dv: known per channel, so this is one pass.
+template <typename E>
+__global__ void __launch_bounds__(kPoolWarps * 32) pool_bwd_kernel(E* __restrict__ d_logits, E* __restrict__ dx,
+                                                                  const float* __restrict__ d_out, const float* __restrict__ out,
+                                                                  const float* __restrict__ stats, const E* __restrict__ logits,
+                                                                  const E* __restrict__ x, int T, int C, float floor_var) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, col = blockIdx.x * 256 + lane * 8;
+    if (col >= C) return;
+    const size_t base = (size_t)blockIdx.y * T * C, row = (size_t)blockIdx.y * C + col, row2 = (size_t)blockIdx.y * 2 * C + col;
+    float top[8], inv[8], dm[8], dv[8], inner[8];
+    {
+        float mu[8], sd[8], gm[8], gs[8], e2[8];
+        const size_t plane = (size_t)gridDim.y * C;
+        load8f(stats + row, top);
+        load8f(stats + row + plane, inv);
+        load8f(stats + row + 2 * plane, e2);
+        load8f(out + row2, mu);
+        load8f(out + row2 + C, sd);
+        load8f(d_out + row2, gm);
+        load8f(d_out + row2 + C, gs);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const float var = fmaf(-mu[i], mu[i], e2[i]);   // as the forward pass computed it
+            dv[i] = var < floor_var ? 0.f : gs[i] * 0.5f / sd[i];
+            dm[i] = gm[i] - 2.f * mu[i] * dv[i];
+            inner[i] = mu[i] * dm[i] + e2[i] * dv[i];
+        }
+    }
+#pragma unroll 2
+    for (int t = blockIdx.z * kPoolWarps + warp; t < T; t += kPoolWarps * gridDim.z) {
+        const size_t at = base + (size_t)t * C + col;
+        float l[8], v[8];
+        load8(logits + at, l);
+        load8(x + at, v);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const float a = fast_exp2((l[i] - top[i]) * kLog2e) * inv[i];
+            const float xv = v[i];
+            const float q = xv * fmaf(xv, dv[i], dm[i]);
+            l[i] = a * (q - inner[i]);
+            v[i] = a * fmaf(2.f * xv, dv[i], dm[i]);
+        }
+        store8(d_logits + at, l);
+        store8(dx + at, v);
+    }
+}
+
+// rows are shared out over the warps of at most per_sm CTAs per SM
+int row_grid(long long rows, int per_sm) {
+    const long long need = (rows + kWarps - 1) / kWarps, most = (long long)device_sm_count() * per_sm;
+    return (int)(need < most ? need : most);
+}
+
+template <typename E>
+cudaError_t ln_fwd(void* y, void* sum, float* mean, float* rstd, const void* x, const void* dx, const float* w, const float* b,
+                   int rows, int D, float eps, cudaStream_t st) {
+    const int grid = row_grid(rows, 8), ch = (D + 255) / 256;
+#define NA1D_LN(CH) ln_fwd_kernel<E, CH><<<grid, kRowThreads, 0, st>>>((E*)y, (E*)sum, mean, rstd, (const E*)x, (const E*)dx, w, b, rows, D, eps)
+    switch (ch) { case 1: NA1D_LN(1); break; case 2: NA1D_LN(2); break; case 3: NA1D_LN(3); break; default: NA1D_LN(4); }
+#undef NA1D_LN
+    return cudaGetLastError();
+}
+cudaError_t add_partials(float* out, const float* part, int n, int groups, cudaStream_t st) {
+    partial_sum_kernel<<<(n + 31) / 32, 1024, 0, st>>>(out, part, n, groups);
+    return cudaGetLastError();
+}
+template <typename E>
+cudaError_t ln_bwd(void* dx, float* sums, float* part, const void* dy, const void* x, const float* mean, const float* rstd,
+                   const float* w, const void* res, int rows, int D, cudaStream_t st) {
+    const int grid = block_partial_rows(rows), ch = (D + 255) / 256;
+#define NA1D_LN(CH) ln_bwd_kernel<E, CH><<<grid, kRowThreads, 0, st>>>((E*)dx, part, (const E*)dy, (const E*)x, mean, rstd, w, (const E*)res, rows, D)
+    switch (ch) { case 1: NA1D_LN(1); break; case 2: NA1D_LN(2); break; case 3: NA1D_LN(3); break; default: NA1D_LN(4); }
+#undef NA1D_LN
+    if (cudaError_t e = cudaGetLastError()) return e;
+    return add_partials(sums, part, 3 * D, grid, st);
+}
+template <typename E, bool GELU>
+cudaError_t columns(void* dx, float* sums, float* part, const void* dy, const void* x, int rows, int F, cudaStream_t st) {
+    const int bx = (F + 255) / 256;
+    int by = block_partial_rows(rows) / bx;
+    if (by < 1) by = 1;
+    column_kernel<E, GELU><<<dim3(bx, by), kRowThreads, 0, st>>>((E*)dx, part, (const E*)dy, (const E*)x, rows, F);
+    if (cudaError_t e = cudaGetLastError()) return e;
+    return add_partials(sums, part, F, by, st);
+}
+
+}  // namespace
+
+// CTAs of a column-sum pass over `rows` rows, and so the rows of partial sums it needs room for
+int block_partial_rows(long long rows) { return row_grid(rows, 3); }
+
+cudaError_t block_ln_fwd(void* y, void* sum, float* mean, float* rstd, const void* x, const void* dx, const float* w, const float* b,
+                         int rows, int D, float eps, int dtype, cudaStream_t st) {
+    return dtype == 0 ? ln_fwd<__nv_bfloat16>(y, sum, mean, rstd, x, dx, w, b, rows, D, eps, st)
+                      : ln_fwd<__half>(y, sum, mean, rstd, x, dx, w, b, rows, D, eps, st);
+}
+cudaError_t block_ln_bwd(void* dx, float* sums, float* part, const void* dy, const void* x, const float* mean, const float* rstd,
+                         const float* w, const void* res, int rows, int D, int dtype, cudaStream_t st) {
+    return dtype == 0 ? ln_bwd<__nv_bfloat16>(dx, sums, part, dy, x, mean, rstd, w, res, rows, D, st)
+                      : ln_bwd<__half>(dx, sums, part, dy, x, mean, rstd, w, res, rows, D, st);
+}
+cudaError_t block_gelu_fwd(void* y, const void* x, long long n, int dtype, cudaStream_t st) {
+    const long long chunks = n / 8, need = (chunks + 1023) / 1024, most = (long long)device_sm_count() * 8;
+    const int grid = (int)(need < most ? need : most);
+    if (dtype == 0) gelu_fwd_kernel<<<grid, 256, 0, st>>>((__nv_bfloat16*)y, (const __nv_bfloat16*)x, chunks);
+    else gelu_fwd_kernel<<<grid, 256, 0, st>>>((__half*)y, (const __half*)x, chunks);
+    return cudaGetLastError();
+}
+cudaError_t block_gelu_bwd(void* dx, float* sums, float* part, const void* dy, const void* x, int rows, int F, int dtype, cudaStream_t st) {
+    return dtype == 0 ? columns<__nv_bfloat16, true>(dx, sums, part, dy, x, rows, F, st) : columns<__half, true>(dx, sums, part, dy, x, rows, F, st);
+}
+cudaError_t block_column_sums(float* sums, float* part, const void* x, int rows, int F, int dtype, cudaStream_t st) {
+    return dtype == 0 ? columns<__nv_bfloat16, false>(nullptr, sums, part, x, nullptr, rows, F, st)
+                      : columns<__half, false>(nullptr, sums, part, x, nullptr, rows, F, st);
+}
+cudaError_t block_cast(void* out, const float* const* src, const int64_t* dst, const int64_t* n, int count, int dtype, cudaStream_t st) {
+    CastList L;
+    L.count = count;
+    L.first[0] = 0;
+    for (int i = 0; i < count; ++i) {
+        L.src[i] = src[i];
+        L.dst[i] = dst[i];
+        L.n[i] = (int)n[i];
+        L.first[i + 1] = L.first[i] + (int)((n[i] + kCastPerCta - 1) / kCastPerCta);
+    }
+    if (dtype == 0) cast_kernel<<<L.first[count], 256, 0, st>>>((__nv_bfloat16*)out, L);
+    else cast_kernel<<<L.first[count], 256, 0, st>>>((__half*)out, L);
+    return cudaGetLastError();
+}
+cudaError_t block_pool_fwd(float* out, float* stats, const void* logits, const void* x, int N, int T, int C, float floor_var,
+                           int dtype, cudaStream_t st) {
+    const dim3 grid((C + 255) / 256, N);
+    if (dtype == 0) pool_fwd_kernel<<<grid, kPoolWarps * 32, 0, st>>>(out, stats, (const __nv_bfloat16*)logits, (const __nv_bfloat16*)x, T, C, floor_var);
+    else pool_fwd_kernel<<<grid, kPoolWarps * 32, 0, st>>>(out, stats, (const __half*)logits, (const __half*)x, T, C, floor_var);
+    return cudaGetLastError();
+}
+cudaError_t block_pool_bwd(void* d_logits, void* dx, const float* d_out, const float* out, const float* stats,
+                           const void* logits, const void* x, int N, int T, int C, float floor_var, int dtype, cudaStream_t st) {
+    // few utterances: share the time axis among CTAs
+    const int cols = (C + 255) / 256, steps = (T + kPoolWarps - 1) / kPoolWarps;
+    int split = (int)((4ll * device_sm_count() + (long long)cols * N - 1) / ((long long)cols * N));
+    split = split < 1 ? 1 : split > steps ? steps : split;
+    const dim3 grid(cols, N, split);
+    if (dtype == 0)
+        pool_bwd_kernel<<<grid, kPoolWarps * 32, 0, st>>>((__nv_bfloat16*)d_logits, (__nv_bfloat16*)dx, d_out, out, stats, (const __nv_bfloat16*)logits,
+                                                          (const __nv_bfloat16*)x, T, C, floor_var);
+    else
+        pool_bwd_kernel<<<grid, kPoolWarps * 32, 0, st>>>((__half*)d_logits, (__half*)dx, d_out, out, stats, (const __half*)logits, (const __half*)x,
+                                                          T, C, floor_var);
+    return cudaGetLastError();
+}
+
+}  // namespace na1d

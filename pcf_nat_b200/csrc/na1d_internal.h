@@ -65,4 +65,19 @@ cudaError_t tc_fused_bwd(void* dq, void* dk, void* dv, float* d_rpb, const void*
                          const void* v, const float* lse, const float* rpb, const int* valid_len, float* scratch,
                          size_t scratch_floats, const Geometry& gm, int dtype, cudaStream_t st);
 
+// ---- row and column kernels of a transformer block and of the statistics pooling (na1d_block.cu)
+int block_partial_rows(long long rows);
+cudaError_t block_ln_fwd(void* y, void* sum, float* mean, float* rstd, const void* x, const void* dx, const float* w, const float* b,
+                         int rows, int D, float eps, int dtype, cudaStream_t st);
+cudaError_t block_ln_bwd(void* dx, float* sums, float* part, const void* dy, const void* x, const float* mean, const float* rstd,
+                         const float* w, const void* res, int rows, int D, int dtype, cudaStream_t st);
+cudaError_t block_gelu_fwd(void* y, const void* x, long long n, int dtype, cudaStream_t st);
+cudaError_t block_gelu_bwd(void* dx, float* sums, float* part, const void* dy, const void* x, int rows, int F, int dtype, cudaStream_t st);
+cudaError_t block_column_sums(float* sums, float* part, const void* x, int rows, int F, int dtype, cudaStream_t st);
+cudaError_t block_cast(void* out, const float* const* src, const int64_t* dst, const int64_t* n, int count, int dtype, cudaStream_t st);
+cudaError_t block_pool_fwd(float* out, float* stats, const void* logits, const void* x, int N, int T, int C, float floor_var,
+                           int dtype, cudaStream_t st);
+cudaError_t block_pool_bwd(void* d_logits, void* dx, const float* d_out, const float* out, const float* stats,
+                           const void* logits, const void* x, int N, int T, int C, float floor_var, int dtype, cudaStream_t st);
+
 }  // namespace na1d

@@ -17,7 +17,8 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
-from .nattention import NAttention, _merge_heads, _split_heads
+from . import block
+from .nattention import NAttention, _merge_heads, _split_heads, _valid_tokens
 from .nattn import getNA1dFunction
 
 
@@ -74,7 +75,11 @@ class AttentiveStatsPool(nn.Module):
         self.b = nn.Linear(bottleneck, dim)
 
     def forward(self, x):
-        w = torch.softmax(self.b(torch.tanh(self.a(x))).float(), dim=1)
+        logits = self.b(torch.tanh(self.a(x)))
+        out = block.stats_pool(logits, x, 1e-5)
+        if out is not None:
+            return out
+        w = torch.softmax(logits.float(), dim=1)
         xf = x.float()
         mu = (w * xf).sum(1)
         var = (w * xf * xf).sum(1) - mu * mu
@@ -120,9 +125,16 @@ class PCFNATExtractor(nn.Module):
         x = self.front(fbank).transpose(1, 2).contiguous()  # (N, T, C)
         feats = [x]
         outs = []
+        valid = None
+        if not self.training and padding is not None and x.is_cuda:
+            valid = _valid_tokens(x.shape[1], padding, x.shape[0])
         for s, stage in enumerate(self.stages):
-            for blk in stage:
-                x = blk(x, padding)
+            y = block.run_blocks(stage, x, valid, NAttention) if all(m.attn.training == self.training for m in stage) else None
+            if y is None:
+                for blk in stage:
+                    x = blk(x, padding)
+            else:
+                x = y
             outs.append(x)
             feats.append(x)
             if s + 1 < len(self.stages):

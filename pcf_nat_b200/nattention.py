@@ -120,6 +120,11 @@ def _fused_forward_channels_first_packed(self, x, valid_len):
     return self.proj_drop(y.transpose(1, 2).contiguous())
 
 
+def _valid_tokens(T, padding, N):
+    """int32 (N,): tokens of each utterance that are not padding."""
+    return (T - padding.to(torch.int64)).clamp_(0, T).to(torch.int32).expand(N).contiguous()
+
+
 def _fused_forward(self, x, padding=None):
     layout = self._na1d_layout
     if layout == "channels_first":
@@ -138,7 +143,7 @@ def _fused_forward(self, x, padding=None):
     valid_len = None
     if not self.training and padding is not None:
         # eval: the mask follows the utterance's padding (PCF_NATransformer.py:131-134); training uses the constant mask
-        valid_len = (T - padding.to(torch.int64)).clamp_(0, T).to(torch.int32).expand(N).contiguous()
+        valid_len = _valid_tokens(T, padding, N)
     hd = C // self.num_heads
     if layout == "channels_first" and not drop_p and type(x) is torch.Tensor and x.is_cuda and not torch.compiler.is_compiling():
         # the dtype the projections will produce: the input's own 16-bit type, or autocast's

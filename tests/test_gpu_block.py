@@ -1,0 +1,229 @@
+"""The block's row and column kernels and the fused block node against plain PyTorch in 64 bits (or the same module run
+part by part). Sizes sit at the edges: one row, row counts around a CTA's eight, rows of 8 channels, of one chunk of 256 and
+one more, the largest of 1024; time axes shorter than the CTA's warps."""
+import pytest
+import torch
+import torch.nn.functional as F
+
+pytestmark = pytest.mark.gpu
+
+DT = [torch.bfloat16, torch.float16]
+EPS = {torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11}    # rounding step of one 16-bit store
+
+
+def _rand(*shape, dtype, seed, scale=1.0):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    return (torch.randn(*shape, device="cuda", generator=g) * scale).to(dtype)
+
+
+def _close(got, ref, dtype, steps=1.0):
+    """Within ``steps`` 16-bit rounding steps of the value, plus fp32 noise relative to the tensor's largest value."""
+    err = (got.double() - ref).abs()
+    bound = steps * EPS[dtype] * ref.abs() + 4e-6 * ref.abs().max() + 1e-7
+    assert bool((err <= bound).all()), float((err - bound).max())
+
+
+@pytest.mark.parametrize("dtype", DT)
+@pytest.mark.parametrize("rows,D", [(1, 8), (7, 64), (8, 256), (9, 264), (300, 256), (5000, 192), (33, 512), (17, 776), (20, 1024)])
+def test_layer_norm_with_residual(rows, D, dtype):
+    from pcf_nat_b200 import block
+    x, dx, dy, res = (_rand(rows, D, dtype=dtype, seed=s) for s in range(4))
+    w, b = 1 + _rand(D, dtype=torch.float32, seed=5, scale=0.2), _rand(D, dtype=torch.float32, seed=6, scale=0.2)
+    y, s, mean, rstd = block.layer_norm(x, dx, w, b, 1e-5, True)
+    assert torch.equal(s, x + dx)
+    s64, w64, b64 = s.double().requires_grad_(), w.double().requires_grad_(), b.double().requires_grad_()
+    ref = F.layer_norm(s64, (D,), w64, b64, 1e-5)
+    _close(y, ref.detach(), dtype)
+    y0, s0, none, _ = block.layer_norm(s, None, w, b, 1e-5, False)
+    assert torch.equal(y0, y) and s0 is s and none is None
+    for r in (res, None):
+        ds, sums = block.layer_norm_backward(dy, s, mean, rstd, w, r, block._scratch(rows, D, 8, x.device))
+        gs, gw, gb = torch.autograd.grad(ref, (s64, w64, b64), dy.double(), retain_graph=True)
+        gs = gs if r is None else gs + r.double()
+        # the row sums cancel: fp32 noise of the terms, not of the result
+        err = (ds.double() - gs).abs()
+        assert bool((err <= EPS[dtype] * gs.abs() + 2e-5 * float(dy.double().abs().max() * rstd.max())).all())
+        for got, want, terms in ((sums[0], gw, rows ** 0.5), (sums[1], gb, rows ** 0.5), (sums[2], ds.double().sum(0), rows ** 0.5)):
+            assert float((got.double() - want).abs().max()) <= 1e-5 * (terms + 3) * 4
+
+
+@pytest.mark.parametrize("dtype", DT)
+@pytest.mark.parametrize("rows,F_", [(1, 8), (9, 256), (700, 264), (4099, 1024), (65, 2048)])
+def test_gelu_and_column_sums(rows, F_, dtype):
+    from pcf_nat_b200 import block
+    x, dy = _rand(rows, F_, dtype=dtype, seed=1, scale=2.0), _rand(rows, F_, dtype=dtype, seed=2)
+    x64 = x.double().requires_grad_()
+    ref = F.gelu(x64)
+    got = block.gelu(x)
+    # half a rounding step, and the approximation's 0.75e-7 |x| (fp16 subnormals: their own spacing)
+    bound = EPS[dtype] * ref.detach().abs() + 2e-7 * x64.detach().abs() + (6e-8 if dtype == torch.float16 else 0)
+    assert bool(((got.double() - ref.detach()).abs() <= bound).all())
+    torch_err = (F.gelu(x).double() - ref.detach()).norm()
+    assert float((got.double() - ref.detach()).norm()) <= 1.001 * float(torch_err)      # no less exact than the framework's
+    scratch = block._scratch(rows, 8, F_, x.device)
+    dx, sums = block.gelu_backward(dy, x, scratch)
+    want = torch.autograd.grad(ref, x64, dy.double())[0]
+    _close(dx, want, dtype)
+    assert float((sums.double() - dx.double().sum(0)).abs().max()) <= 1e-5 * (rows ** 0.5 + 3)
+    assert float((block.column_sums(dy, scratch).double() - dy.double().sum(0)).abs().max()) <= 1e-5 * (rows ** 0.5 + 3)
+
+
+def test_gelu_of_special_values():
+    from pcf_nat_b200 import block
+    for dtype in DT:
+        x = torch.tensor([0.0, -0.0, float("inf"), float("-inf"), float("nan"), 3e4, -3e4, -8.0], device="cuda", dtype=dtype)
+        got, ref = block.gelu(x).float(), F.gelu(x).float()
+        assert torch.equal(torch.isnan(got), torch.isnan(ref))
+        ok = ~torch.isnan(ref)
+        assert torch.allclose(got[ok], ref[ok], rtol=1e-2, atol=1e-6)
+
+
+def test_cast_parameters_is_the_rounding_of_each_tensor():
+    from pcf_nat_b200 import block
+    for dtype in DT:
+        ps = [_rand(n, dtype=torch.float32, seed=n) for n in (1, 7, 8, 63, 64, 2048, 2049, 70001)]
+        ps.append(_rand(33, dtype=torch.float32, seed=3)[1:])          # not 16-byte aligned
+        buf, offs = block.cast_parameters(ps, dtype)
+        for p, o in zip(ps, offs):
+            assert torch.equal(buf[o:o + p.numel()], p.to(dtype))
+
+
+@pytest.mark.parametrize("dtype", DT)
+@pytest.mark.parametrize("N,T,C", [(1, 1, 8), (2, 7, 256), (3, 9, 264), (5, 300, 1536), (2, 1000, 40)])
+def test_statistics_pooling(N, T, C, dtype):
+    from pcf_nat_b200 import block
+    logits, x = _rand(N, T, C, dtype=dtype, seed=1, scale=3.0).requires_grad_(), _rand(N, T, C, dtype=dtype, seed=2).requires_grad_()
+    d_out = _rand(N, 2 * C, dtype=torch.float32, seed=3)
+    out = block.stats_pool(logits, x, 1e-5)
+    l64, x64 = logits.detach().double().requires_grad_(), x.detach().double().requires_grad_()
+    w = torch.softmax(l64, 1)
+    mu = (w * x64).sum(1)
+    var = (w * x64 * x64).sum(1) - mu * mu
+    ref = torch.cat([mu, var.clamp_min(1e-5).sqrt()], 1)
+    mean_ref, std_ref, var = ref[:, :C].detach(), ref[:, C:].detach(), var.detach()
+    assert float((out[:, :C].detach().double() - mean_ref).abs().max()) <= 2e-5
+    # the variance is a difference of two fp32 sums: 4e-6 of it, through the square root
+    assert bool(((out[:, C:].detach().double() - std_ref).abs() <= 4e-6 * (1 + mean_ref ** 2) / std_ref + 1e-6).all())
+    clear = (var > 1e-3)                      # away from the floor, where the gradient of the square root is steep
+    d_out[:, C:] *= clear
+    g = torch.autograd.grad(out, (logits, x), d_out)
+    r = torch.autograd.grad(ref, (l64, x64), d_out.double())
+    for got, want in zip(g, r):
+        err = float((got.double() - want).norm()), float(want.norm())
+        assert err[0] <= (EPS[dtype] + 2e-4) * err[1] + 1e-6, err
+
+
+def test_pooling_with_infinite_logits_and_a_constant_channel():
+    from pcf_nat_b200 import block
+    logits = torch.zeros(1, 20, 8, device="cuda", dtype=torch.bfloat16)
+    x = _rand(1, 20, 8, dtype=torch.bfloat16, seed=1)
+    logits[0, :10, 0] = float("-inf")          # half of the frames have no weight
+    logits[0, :, 1] = float("-inf")            # none has: 0 / 0
+    logits[0, 3, 2] = float("inf")
+    logits[0, 3, 3] = float("nan")
+    logits[0, :, 4] = -3e38
+    x[0, :, 5] = 1.0                           # variance 0: the floor
+    w = torch.softmax(logits.float(), 1)
+    mu = (w * x.float()).sum(1)
+    ref = torch.cat([mu, ((w * x.float() ** 2).sum(1) - mu * mu).clamp_min(1e-5).sqrt()], 1)
+    assert torch.allclose(block.stats_pool(logits, x, 1e-5), ref, rtol=1e-5, atol=1e-5, equal_nan=True)
+
+
+def _stage(dim, heads, frames, hidden=4, n=2):
+    from pcf_nat_b200.model import NABlock
+    torch.manual_seed(3)
+    return torch.nn.ModuleList(NABlock(frames, dim, heads, 7, hidden, "fused") for _ in range(n)).cuda()
+
+
+@pytest.mark.parametrize("dtype", DT)
+@pytest.mark.parametrize("dim,heads,T", [(64, 2, 50), (256, 4, 131), (512, 8, 40)])
+def test_block_node_against_its_modules(dim, heads, T, dtype):
+    """Outputs and all gradients of the fused node, of the module-by-module network and of the same network in fp32: the node
+    is no further from fp32 than the modules are."""
+    from pcf_nat_b200 import block
+    from pcf_nat_b200.nattention import NAttention
+    st = _stage(dim, heads, T)
+    x0 = _rand(3, T, dim, dtype=dtype, seed=1)
+    dy = _rand(3, T, dim, dtype=dtype, seed=2)
+    got = {}
+    for kind in ("node", "modules"):
+        x = x0.clone().requires_grad_()
+        with torch.autocast("cuda", dtype=dtype):
+            if kind == "node":
+                y = block.run_blocks(st, x, None, NAttention)
+                assert y is not None
+            else:
+                y = x
+                for b in st:
+                    y = b(y)
+        got[kind] = [y.detach()] + list(torch.autograd.grad(y, [x] + list(st.parameters()), dy))
+    ref = _reference(st, x0, dy, heads)
+    for a, b, r in zip(got["node"], got["modules"], ref):
+        assert a.dtype == b.dtype and a.shape == b.shape
+        ea, eb = float((a.double() - r).norm()), float((b.double() - r).norm())
+        # the norm of n independent rounding errors scatters by 1 / sqrt(2 n) of itself: four times that for the two of them
+        n = r.numel()
+        assert ea <= (1.1 + 4 / n ** 0.5) * eb + 1e-6 * float(r.norm()), (ea, eb, float(r.norm()), tuple(r.shape))
+
+
+def _reference(st, x0, dy, heads):
+    from oracle import na1d_oracle as orc
+    w = [p.detach().double().cpu().requires_grad_() for p in st.parameters()]
+    named = dict(zip([n for n, _ in st.named_parameters()], w))
+    x = x0.double().cpu().requires_grad_()
+    y = x
+    B, T, D = x.shape
+    C = D // heads
+    for i in range(len(st)):
+        p = {n[2:]: v for n, v in named.items() if n.startswith("%d." % i)}
+        h = F.layer_norm(y, (D,), p["norm1.weight"], p["norm1.bias"])
+        q, k, v = F.linear(h, p["attn.qkv.weight"], p["attn.qkv.bias"]).view(B, T, 3, heads, C).permute(2, 0, 3, 1, 4).reshape(3, B * heads, T, C)
+        o = orc.na1d_fused(q, k, v, 7, 3, 1, C ** -0.5, p["attn.relative_position_bias"].view(heads, 7), None, heads)
+        o = o.view(B, heads, T, C).transpose(1, 2).reshape(B, T, D)
+        y = y + F.linear(o, p["attn.proj.weight"], p["attn.proj.bias"])
+        h = F.layer_norm(y, (D,), p["norm2.weight"], p["norm2.bias"])
+        y = y + F.linear(F.gelu(F.linear(h, p["fc1.weight"], p["fc1.bias"])), p["fc2.weight"], p["fc2.bias"])
+    g = torch.autograd.grad(y, [x] + w, dy.double().cpu())
+    return [t.detach().cuda() for t in (y,) + g]
+
+
+def test_block_node_evaluation_with_padding_and_frozen_parameters():
+    from pcf_nat_b200 import block
+    from pcf_nat_b200.nattention import NAttention, _valid_tokens
+    st = _stage(128, 4, 60).eval()
+    x = _rand(3, 60, 128, dtype=torch.bfloat16, seed=1)
+    pad = torch.tensor([0, 13, 60], device="cuda")
+    with torch.no_grad(), torch.autocast("cuda", dtype=torch.bfloat16):
+        y = block.run_blocks(st, x, _valid_tokens(60, pad, 3), NAttention)
+        z = x
+        for b in st:
+            z = b(z, pad)
+    assert float((y.double() - z.double()).norm() / z.double().norm()) < 1e-2
+    st.train()
+    for n, p in st.named_parameters():
+        p.requires_grad_("fc1" in n)
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        y = block.run_blocks(st, x, None, NAttention)
+    y.float().sum().backward()
+    assert all((p.grad is not None) == ("fc1" in n) for n, p in st.named_parameters())
+
+
+def test_block_node_leaves_other_blocks_to_their_modules():
+    from pcf_nat_b200 import block
+    from pcf_nat_b200.nattention import NAttention
+    x = _rand(2, 40, 64, dtype=torch.bfloat16, seed=1)
+
+    def refused(change, x=x, enabled=True):
+        st = _stage(64, 2, 40)
+        change(st)
+        with torch.autocast("cuda", dtype=torch.bfloat16, enabled=enabled):
+            return block.run_blocks(st, x, None, NAttention) is None
+
+    assert not refused(lambda st: None)
+    assert refused(lambda st: None, enabled=False)
+    assert refused(lambda st: None, x=x.float())
+    assert refused(lambda st: st[1].fc1.register_forward_hook(lambda *a: None))
+    assert refused(lambda st: st.bfloat16())
+    assert refused(lambda st: setattr(st[0].attn.proj_drop, "p", 0.1))
+    assert refused(lambda st: setattr(st[0], "norm1", torch.nn.LayerNorm(64, bias=False).cuda()))
+    assert refused(lambda st: setattr(st[0], "fc2", torch.nn.Sequential(st[0].fc2)))
