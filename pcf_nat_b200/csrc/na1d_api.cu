@@ -122,7 +122,7 @@ int na1d_v_backward(void* v_gd, const float* attn, const void* result_gd, int64_
     return na1d_k_backward(v_gd, attn, result_gd, N, T, C, win, left, dil, dtype, stream);
 }
 
-// 0 = CUDA-core kernels, 1 = tcgen05 kernels on the flat tiling, 2 = tcgen05 kernels on the segmented tiling.
+// 0 = the general kernels (warp-level matrix instructions up to 128 channels, CUDA-core kernels above), 1 = tcgen05 kernels on the flat tiling, 2 = tcgen05 kernels on the segmented tiling.
 // The flat tiling takes dilation 1 and those power-of-two dilations whose dilated window still fits the widest band bucket;
 // the segmented tiling takes every dilation (each residue class of a sequence is a dilation-1 problem) at the price of
 // partly empty last tiles. With a dilation both can run, the one with the cheaper band bucket per useful row wins.
@@ -130,7 +130,7 @@ static int pick_family(const na1d::Geometry& g, int backward, bool has_bias = fa
     const int forced = g_family_override.load();
     const bool flat_ok = backward ? na1d::tc_bwd_supports(g, has_bias, wants_bias_grad) : na1d::tc_fwd_supports(g);
     const bool seg_ok = backward ? na1d::tc_bwd_seg_supports(g, has_bias, wants_bias_grad) : na1d::tc_seg_supports(g);
-    if (forced == 0) return 0;
+    if (forced == 0 || forced == 3) return 0;
     if (forced == 2) return seg_ok ? 2 : NA1D_ERR_UNSUPPORTED;
     if (forced == 1 && flat_ok) return 1;   // forced: the flat tiling wherever it can run (the choice below is for the automatic mode)
     int pick = 0;
@@ -170,7 +170,7 @@ int na1d_fused_kernel_tiling(int64_t N, int64_t T, int64_t C, int64_t win, int64
 }
 
 int na1d_set_kernel_family(int family) {
-    if (family < -1 || family > 2) family = -1;
+    if (family < -1 || family > 3) family = -1;
     return g_family_override.exchange(family);
 }
 
@@ -211,6 +211,8 @@ int na1d_fused_forward(void* o, float* lse, const void* q, const void* k, const 
         const na1d::Strides d = na1d::dense_strides(g.H, g.T, g.C);
         return cuda_status(na1d::tc_fused_fwd_seg(o, lse, q, k, v, rpb, valid_len, d, d, d, d, g, dtype, (cudaStream_t)stream));
     }
+    if (g_family_override.load() != 0 && na1d::mma_supports(g))
+        return cuda_status(na1d::mma_fused_fwd(o, lse, q, k, v, rpb, valid_len, g, dtype, (cudaStream_t)stream));
     return cuda_status(na1d::simt_fused_fwd(o, lse, q, k, v, rpb, valid_len, g, dtype, (cudaStream_t)stream));
 }
 
@@ -301,6 +303,8 @@ int na1d_fused_backward(void* dq, void* dk, void* dv, float* d_rpb, const void* 
         return cuda_status(na1d::tc_fused_bwd_seg(dq, dk, dv, d_rpb, d_o, q, k, v, lse, rpb, valid_len, delta_ws,
                                                   (size_t)g.N * (size_t)g.T, d, d, d, d, d, d, d, g, dtype, st));
     }
+    if (g_family_override.load() != 0 && na1d::mma_supports(g))
+        return cuda_status(na1d::mma_fused_bwd(dq, dk, dv, d_rpb, d_o, q, k, v, o, lse, rpb, valid_len, g, dtype, st));
     if (int s = cuda_status(na1d::simt_delta(delta_ws, d_o, o, g.N * g.T, g.C, dtype, st))) return s;
     return cuda_status(na1d::simt_fused_bwd(dq, dk, dv, d_rpb, d_o, q, k, v, lse, delta_ws, rpb, valid_len, g, dtype, st));
 }

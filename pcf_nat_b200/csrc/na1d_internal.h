@@ -17,6 +17,14 @@ cudaError_t simt_fused_bwd(void* dq, void* dk, void* dv, float* d_rpb, const voi
                            const Geometry& gm, int dtype, cudaStream_t st);
 cudaError_t window_index(int* j_out, unsigned char* inr, int T, int win, int left, int dil, cudaStream_t st);
 
+// ---- fused pair on warp-level matrix instructions (na1d_mma.cu): what the tcgen05 kernels do not take, up to 128 channels
+bool mma_supports(const Geometry& gm);
+cudaError_t mma_fused_fwd(void* o, float* lse, const void* q, const void* k, const void* v, const float* rpb, const int* valid_len,
+                          const Geometry& gm, int dtype, cudaStream_t st);
+cudaError_t mma_fused_bwd(void* dq, void* dk, void* dv, float* d_rpb, const void* d_o, const void* q, const void* k, const void* v,
+                          const void* o, const float* lse, const float* rpb, const int* valid_len, const Geometry& gm, int dtype,
+                          cudaStream_t st);
+
 // ---- tcgen05 / TMA family (na1d_tc_fwd.cu)
 bool tc_fwd_supports(const Geometry& gm);  // shape limits of the tcgen05 forward
 cudaError_t tc_fused_fwd(void* o, float* lse, const void* q, const void* k, const void* v, const float* rpb,

@@ -339,7 +339,7 @@ def window_index(T, win, left, dil=1, device="cuda"):
     return j, inr.bool()
 
 
-FAMILY_AUTO, FAMILY_CUDA_CORE, FAMILY_TCGEN05, FAMILY_TCGEN05_SEGMENTED = -1, 0, 1, 2
+FAMILY_AUTO, FAMILY_CUDA_CORE, FAMILY_TCGEN05, FAMILY_TCGEN05_SEGMENTED, FAMILY_WARP_MMA = -1, 0, 1, 2, 3
 
 
 def set_kernel_family(family):

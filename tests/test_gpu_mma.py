@@ -1,0 +1,119 @@
+"""The general kernels on warp-level matrix instructions against plain PyTorch in 64 bits and against the CUDA-core kernels:
+every padded channel count, windows around a multiple of the 16-row chunk, asymmetric and one-sided windows, dilations with
+empty and uneven residues, sequences shorter than a tile and around its 64 rows, padding, values that are not finite."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+#      B  H  T    C   win left dil bias  padded
+CASES = [
+    (1, 1, 1, 8, 1, 0, 1, True, False),
+    (2, 3, 64, 8, 80, 40, 1, True, True),
+    (1, 2, 65, 16, 34, 33, 1, False, True),
+    (2, 4, 203, 48, 41, 20, 1, True, True),
+    (1, 2, 130, 24, 7, 0, 3, True, False),
+    (2, 1, 5, 48, 9, 4, 7, True, True),          # more residues than tokens
+    (1, 2, 63, 96, 17, 8, 2, True, True),
+    (1, 2, 150, 128, 33, 16, 1, False, False),
+    (1, 1, 200, 128, 128, 64, 1, True, True),
+    (1, 2, 97, 64, 50, 3, 1, True, True),
+    (1, 1, 300, 32, 49, 48, 4, True, False),
+    (1, 40, 50, 16, 18, 9, 1, True, True),        # more heads than the tcgen05 kernels take
+]
+
+
+def _inputs(case, dtype, seed=0):
+    B, H, T, C, win, left, dil, bias, padded = case
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    q, k, v, d_o = (torch.randn(B * H, T, C, device="cuda", generator=g).to(dtype) for _ in range(4))
+    rpb = torch.randn(H, win, device="cuda", generator=g) if bias else None
+    vl = torch.randint(0, T + 1, (B,), device="cuda", generator=g, dtype=torch.int32) if padded else None
+    return q, k, v, d_o, rpb, vl
+
+
+def _reference(case, q, k, v, d_o, rpb, vl):
+    B, H, T, C, win, left, dil, _, _ = case
+    q, k, v = (x.double().view(B, H, T, C).requires_grad_() for x in (q, k, v))
+    r = None if rpb is None else rpb.double().requires_grad_()
+    j = torch.arange(T, device="cuda")[:, None] + (torch.arange(win, device="cuda") - left) * dil
+    inr = (j >= 0) & (j < T)
+    n = torch.full((B, 1, 1), T, device="cuda") if vl is None else vl.view(B, 1, 1)
+    masked = (j < 0) | (j >= n) | (torch.arange(T, device="cuda").view(1, T, 1) >= n)
+    kg, vg = (x[:, :, j.clamp(0, T - 1)] * inr[..., None] for x in (k, v))
+    x = torch.einsum("bhtc,bhtwc->bhtw", q, kg) * C ** -0.5 - 100.0 * masked[:, None]
+    p = torch.softmax(x if r is None else x + r[None, :, None], -1)
+    o = torch.einsum("bhtw,bhtwc->bhtc", p, vg)
+    grads = torch.autograd.grad(o, [q, k, v] + ([] if r is None else [r]), d_o.double().view(B, H, T, C))
+    return [t.detach().reshape(B * H, T, C) for t in (o,) + grads[:3]] + list(grads[3:])
+
+
+def _run(family, case, q, k, v, d_o, rpb, vl):
+    from pcf_nat_b200 import ops
+    B, H, T, C, win, left, dil, _, _ = case
+    old = ops.set_kernel_family(family)
+    try:
+        o, lse = ops.fused_forward(q, k, v, win, left, dil, C ** -0.5, rpb, vl, H)
+        dq, dk, dv, dr = ops.fused_backward(d_o, q, k, v, o, lse, win, left, dil, C ** -0.5, rpb, vl, H, need_d_rpb=rpb is not None)
+    finally:
+        ops.set_kernel_family(old)
+    return [o, dq, dk, dv] + ([] if dr is None else [dr])
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("case", CASES)
+def test_against_64_bits_and_the_cuda_core_kernels(case, dtype):
+    from pcf_nat_b200 import ops
+    args = _inputs(case, dtype)
+    ref = _reference(case, *args)
+    mma, core = _run(ops.FAMILY_WARP_MMA, case, *args), _run(ops.FAMILY_CUDA_CORE, case, *args)
+    eps = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    for i, (a, b, r) in enumerate(zip(mma, core, ref)):
+        ea, eb, n = float((a.double() - r).norm()), float((b.double() - r).norm()), float(r.norm())
+        # both are one 16-bit rounding of an fp32 result: their errors agree but for the scatter of a few elements that round the
+        # other way (the fp32 bias gradient: its own summation order)
+        assert ea <= eb * (1.02 + 2 / r.numel() ** 0.5) + (1e-6 if i < 4 else 4e-6) * n + 1e-6, (i, ea, eb, n)
+        # delta uses the rounded output, as the CUDA-core kernel does: its rounding enters the gradients
+        assert float((a.double() - r).abs().max()) <= 4 * eps * float(r.abs().max()) + 1e-5, i
+
+
+@pytest.mark.parametrize("scale", [1e-4, 3e3])
+def test_gradients_far_from_one_keep_their_precision(scale):
+    """fp16 output gradients near both ends of their range: dS must not lose bits to an fp16 exponent on the way."""
+    from pcf_nat_b200 import ops
+    case = (1, 2, 100, 48, 41, 20, 1, True, False)
+    q, k, v, d_o, rpb, vl = _inputs(case, torch.float16)
+    args = (q, k, v, (d_o.float() * scale).to(torch.float16), rpb, vl)
+    ref = _reference(case, *args)
+    for a, b, r in zip(_run(ops.FAMILY_WARP_MMA, case, *args), _run(ops.FAMILY_CUDA_CORE, case, *args), ref):
+        ok = torch.isfinite(b.double())
+        assert torch.equal(ok, torch.isfinite(a.double()))
+        ea, eb = float((a.double() - r)[ok].norm()), float((b.double() - r)[ok].norm())
+        assert ea <= 1.05 * eb + 4e-6 * float(r.norm()), (ea, eb)
+
+
+@pytest.mark.parametrize("which", [0, 1, 2, 3])
+@pytest.mark.parametrize("value", [float("nan"), float("inf")])
+def test_values_that_are_not_finite_reach_their_window_only(which, value):
+    from pcf_nat_b200 import ops
+    case = (1, 1, 150, 48, 9, 4, 1, True, False)
+    args = _inputs(case, torch.bfloat16)
+    args[which][0, 70, 5] = value
+    for i, (a, r) in enumerate(zip(_run(ops.FAMILY_WARP_MMA, case, *args), _reference(case, *args))):
+        ok = torch.isfinite(r)
+        assert torch.equal(ok, torch.isfinite(a)), (i, int((~ok).sum()), int((~torch.isfinite(a)).sum()))
+        if bool(ok.any()):
+            assert float((a.double() - r)[ok].abs().max()) <= 2.0 ** -6 * float(r[ok].abs().max()), i
+
+
+def test_routes():
+    """Above 128 channels the CUDA-core kernels stay; the automatic route of a general shape is the warp-level one, bit for bit."""
+    from pcf_nat_b200 import ops
+    case = (1, 2, 70, 48, 20, 9, 1, True, True)
+    args = _inputs(case, torch.bfloat16)
+    for a, b in zip(_run(ops.FAMILY_AUTO, case, *args)[:4], _run(ops.FAMILY_WARP_MMA, case, *args)[:4]):
+        assert torch.equal(a, b)
+    case = (1, 2, 70, 192, 20, 9, 1, True, True)
+    args = _inputs(case, torch.bfloat16)
+    for a, b in zip(_run(ops.FAMILY_WARP_MMA, case, *args)[:4], _run(ops.FAMILY_CUDA_CORE, case, *args)[:4]):
+        assert torch.equal(a, b)
