@@ -212,6 +212,8 @@ int na1d_fused_backward_dropout(void* dq, void* dk, void* dv, float* d_rpb, cons
  * `scratch` holds at least na1d_block_scratch_floats(rows, D, F) floats (column sums leave the CTAs as partial rows and
  * are added in a fixed order: the same bits from run to run).
  * ---------------------------------------------------------------------------------------- */
+/* out (N): clamp(T - padding, 0, T); padding is int32 or (is64) int64, n_padding = N or 1 (one value for all). Any alignment. */
+int na1d_valid_tokens(int32_t* out, const void* padding, int is64, int64_t n_padding, int64_t N, int64_t T, void* stream);
 int64_t na1d_block_scratch_floats(int64_t rows, int64_t D, int64_t F);
 /* y = LN(s) * w + b over rows of D; s = x, or with dx: s = x + dx, rounded and written to `sum`. mean, rstd: (rows) or NULL. */
 int na1d_layer_norm_forward(void* y, void* sum, float* mean, float* rstd, const void* x, const void* dx, const float* w,

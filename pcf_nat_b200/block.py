@@ -11,7 +11,6 @@ Rounding points are those of the autocast network: 16-bit activations and projec
 LayerNorm parameters and the weight gradients are not rounded to 16 bits on the way.
 """
 import ctypes
-import functools
 
 import torch
 import torch.nn as nn
@@ -95,109 +94,7 @@ def cast_parameters(params, dtype):
     return buf, offs
 
 
-@functools.lru_cache(maxsize=256)
-def _packed_strides(T, H, C):
-    """{batch, head, token} element strides of q, k, v in a packed (batch, T, 3, H, C) tensor and of o in (batch, T, H, C)."""
-    return (ctypes.c_int64 * 3)(T * 3 * H * C, C, 3 * H * C), (ctypes.c_int64 * 3)(T * H * C, C, H * C)
-
-
-def _attention(qkv, cfg, rpb, valid, stats):
-    B, T, H, C, win, left, scale = cfg
-    sp, so = _packed_strides(T, H, C)
-    o = torch.empty((B, T, H * C), dtype=qkv.dtype, device=qkv.device)
-    lse = torch.empty((B * H, T), dtype=torch.float32, device=qkv.device) if stats else None
-    p, step = qkv.data_ptr(), H * C * 2
-    check(_L.na1d_fused_forward_strided(o.data_ptr(), lse.data_ptr() if stats else None, p, p + step, p + 2 * step, rpb.data_ptr(),
-                                        None if valid is None else valid.data_ptr(), so, sp, sp, sp, B * H, H, T, C, win, left, 1,
-                                        scale, _CODE[qkv.dtype], _stream(qkv)), "na1d_fused_forward_strided")
-    return o, lse
-
-
-def _attention_backward(d_o, qkv, lse, cfg, rpb, valid, need_rpb):
-    B, T, H, C, win, left, scale = cfg
-    sp, so = _packed_strides(T, H, C)
-    d_qkv = torch.empty_like(qkv)
-    d_rpb = scratch = None
-    n = 0
-    if need_rpb:
-        n = 160 * H * win                  # one partial row per CTA (one CTA per SM)
-        d_rpb = torch.zeros((H, win), dtype=torch.float32, device=qkv.device)
-        scratch = torch.empty(n, dtype=torch.float32, device=qkv.device)
-    p, g, step = qkv.data_ptr(), d_qkv.data_ptr(), H * C * 2
-    check(_L.na1d_fused_backward_strided(g, g + step, g + 2 * step, None if d_rpb is None else d_rpb.data_ptr(), d_o.data_ptr(), p, p + step,
-                                         p + 2 * step, lse.data_ptr(), rpb.data_ptr(), None if valid is None else valid.data_ptr(),
-                                         None if scratch is None else scratch.data_ptr(), n, sp, sp, sp, so, sp, sp, sp, B * H, H, T, C,
-                                         win, left, 1, scale, _CODE[qkv.dtype], _stream(qkv)), "na1d_fused_backward_strided")
-    return d_qkv, d_rpb
-
-
-# ------------------------------------------------------------------ the block
-_PROJ = 8   # qkv.w, qkv.b, proj.w, proj.b, fc1.w, fc1.b, fc2.w, fc2.b
-
-
-def _block_forward(x, dx, valid, cfg, eps, params, stats):
-    """x (+ dx): the residual stream, (batch, T, D) 16-bit. Returns the stream after the attention branch, the output of the
-    MLP branch (their sum is the block's output), and what the backward needs."""
-    w, (n1w, n1b, n2w, n2b), rpb = params[:_PROJ], params[_PROJ:_PROJ + 4], params[_PROJ + 4]
-    B, T, D = x.shape
-    Fh = w[4].shape[0]
-    buf, offs = cast_parameters(w, x.dtype)
-    qw, qb, pw, pb, w1, b1, w2, b2 = (buf[o:o + p.numel()].view(p.shape) for o, p in zip(offs, w))
-    h1, s1, m1, r1 = layer_norm(x, dx, n1w, n1b, eps[0], stats)
-    qkv = torch.addmm(qb, h1.view(-1, D), qw.t()).view(B, T, 3 * D)
-    o, lse = _attention(qkv, cfg, rpb, valid, stats)
-    y = torch.addmm(pb, o.view(-1, D), pw.t()).view(B, T, D)
-    h2, s2, m2, r2 = layer_norm(s1, y, n2w, n2b, eps[1], stats)
-    del y
-    f = torch.addmm(b1, h2.view(-1, D), w1.t())
-    g = gelu(f)
-    z = torch.addmm(b2, g, w2.t()).view(B, T, D)
-    return s2, z, (s1, m1, r1, h1, qkv, lse, o, s2, m2, r2, h2, f, g, buf) if stats else None
-
-
-class _BlockFunction(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, x, dx, valid, cfg, eps, *params):
-        s2, z, saved = _block_forward(x, dx, valid, cfg, eps, params, True)
-        ctx.save_for_backward(*saved, params[_PROJ], params[_PROJ + 2], params[_PROJ + 4], valid)
-        ctx.cfg, ctx.has_dx = cfg, dx is not None
-        ctx.shapes = [p.shape for p in params[:_PROJ]]
-        return s2, z
-
-    @staticmethod
-    def backward(ctx, d_s2, d_z):
-        s1, m1, r1, h1, qkv, lse, o, s2, m2, r2, h2, f, g, buf, n1w, n2w, rpb, valid = ctx.saved_tensors
-        need = ctx.needs_input_grad[5:]
-        B, T, D = s1.shape
-        rows, Fh = B * T, f.shape[-1]
-        w, off = [], 0
-        for sh in ctx.shapes:
-            w.append(buf[off:off + sh.numel()].view(sh))
-            off += (sh.numel() + 63) // 64 * 64
-        scratch = _scratch(rows, D, Fh, s1.device)
-        d_z = d_z.contiguous().view(rows, D)
-        d_s2 = d_s2.contiguous()
-
-        def weight_grad(k, dy, inp):     # dy^T . inp, accumulated and returned in fp32
-            return torch.mm(dy.t(), inp, out_dtype=torch.float32) if need[k] else None
-
-        # MLP branch
-        d_w2, d_b2 = weight_grad(6, d_z, g), column_sums(d_z, scratch) if need[7] else None
-        d_f, d_b1 = gelu_backward(torch.mm(d_z, w[6]), f, scratch)
-        d_w1 = weight_grad(4, d_f, h2.view(rows, D))
-        d_y, sums2 = layer_norm_backward(torch.mm(d_f, w[4]), s2, m2, r2, n2w, d_s2, scratch)   # also the residual stream's gradient
-        del d_f
-        # attention branch
-        dy2 = d_y.view(rows, D)
-        d_pw = weight_grad(2, dy2, o.view(rows, D))
-        d_qkv, d_rpb = _attention_backward(torch.mm(dy2, w[2]), qkv, lse, ctx.cfg, rpb, valid, need[_PROJ + 4])
-        d_qkv = d_qkv.view(rows, 3 * D)
-        d_qw, d_qb = weight_grad(0, d_qkv, h1.view(rows, D)), column_sums(d_qkv, scratch) if need[1] else None
-        d_x, sums1 = layer_norm_backward(torch.mm(d_qkv, w[0]), s1, m1, r1, n1w, d_y, scratch)
-        return (d_x, d_x if ctx.has_dx else None, None, None, None, d_qw, d_qb, d_pw, sums2[2], d_w1, d_b1, d_w2, d_b2, sums1[0], sums1[1],
-                sums2[0], sums2[1], None if d_rpb is None else d_rpb.view(rpb.shape))
-
-
+# ------------------------------------------------------------------ the block (its autograd node is in csrc/torch_nodes.cpp)
 def _hooked(m):
     return bool(m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks)
 
@@ -208,7 +105,7 @@ def _global_hooks():
 
 
 def _block_parameters(blk, attention_class, x):
-    """The parameters of a block in the order of ``_block_forward``, or None where the block is anything but the plain one
+    """The parameters of a block in the order of the node's arguments, or None where the block is anything but the plain one
     on fp32 parameters (a replaced or hooked submodule, another dtype, an odd size): it then runs module by module."""
     a, n1, n2, f1, f2 = blk.attn, blk.norm1, blk.norm2, blk.fc1, blk.fc2
     if type(a) is not attention_class or type(n1) is not nn.LayerNorm or type(n2) is not nn.LayerNorm or a._na1d_layout != "channels_last":
@@ -236,7 +133,8 @@ def _block_parameters(blk, attention_class, x):
 def run_blocks(blocks, x, valid, attention_class):
     """The blocks applied to the residual stream x (batch, T, D), or None where they have to run module by module.
     ``valid``: valid tokens per utterance (int32, contiguous) or None."""
-    if type(x) is not torch.Tensor or not x.is_cuda or x.dim() != 3 or x.numel() == 0 or torch.compiler.is_compiling() or not torch.is_autocast_enabled():
+    if (type(x) is not torch.Tensor or not x.is_cuda or x.dim() != 3 or x.numel() == 0 or torch.compiler.is_compiling() or
+            not torch.is_autocast_enabled() or not ops.native.eager_mode() or torch.autograd.forward_ad._current_level >= 0):
         return None
     dt = torch.get_autocast_dtype("cuda")
     if x.dtype != dt or dt not in _CODE or _global_hooks() or x.shape[0] * x.shape[1] * x.shape[2] >= 2 ** 31:
@@ -251,17 +149,12 @@ def run_blocks(blocks, x, valid, attention_class):
         C = D // a.num_heads
         if not ops.packed_supported(a.num_heads, T, C, a.win_size, a.left, 1, dt):
             return None
-        plan.append((ps, (B, T, a.num_heads, C, a.win_size, a.left, float(a.scale)), (blk.norm1.eps, blk.norm2.eps)))
+        plan.append((ps, (a.num_heads, a.win_size, a.left, float(a.scale)), (blk.norm1.eps, blk.norm2.eps)))
     x, dx = x.contiguous(), None
     if x.data_ptr() % 16:
         return None
-    grad = torch.is_grad_enabled()
-    with ops._on_device(x.device):
-        for ps, cfg, eps in plan:
-            if grad:
-                x, dx = _BlockFunction.apply(x, dx, valid, cfg, eps, *ps)
-            else:
-                x, dx, _ = _block_forward(x, dx, valid, cfg, eps, ps, False)
+    for ps, cfg, eps in plan:
+        x, dx = ops.native.block(x, dx, valid, *cfg, *eps, ps)
     return x if dx is None else x + dx
 
 
@@ -298,7 +191,8 @@ def stats_pool(logits, x, floor):
     """(N, 2C) fp32: mean and standard deviation of x (N, T, C) over T under softmax-over-T weights, or None where the inputs
     are not a pair of dense 16-bit CUDA tensors that the kernel takes."""
     if (type(x) is not torch.Tensor or type(logits) is not torch.Tensor or not x.is_cuda or x.dtype not in _CODE or logits.dtype != x.dtype or
-            logits.shape != x.shape or x.dim() != 3 or torch.compiler.is_compiling()):
+            logits.shape != x.shape or x.dim() != 3 or torch.compiler.is_compiling() or not ops.native.eager_mode() or
+            torch.autograd.forward_ad._current_level >= 0):
         return None
     N, T, C = x.shape
     if not 0 < N <= 65535 or not 0 < T <= 1 << 20 or C == 0 or C % 8 or C > 1 << 20:

@@ -365,6 +365,11 @@ int na1d_fused_backward_dropout(void* dq, void* dk, void* dv, float* d_rpb, cons
 }
 
 // ---- row and column kernels of a transformer block (na1d_block.cu)
+int na1d_valid_tokens(int32_t* out, const void* padding, int is64, int64_t n_padding, int64_t N, int64_t T, void* stream) {
+    NA1D_REQUIRE_PTR(out); NA1D_REQUIRE_PTR(padding);
+    if (N <= 0 || N > INT_MAX / 2 || T <= 0 || T > INT_MAX || (n_padding != 1 && n_padding != N)) return NA1D_ERR_BAD_SHAPE;
+    return cuda_status(na1d::block_valid_tokens(out, padding, is64 != 0, (int)n_padding, (int)N, (int)T, (cudaStream_t)stream));
+}
 int64_t na1d_block_scratch_floats(int64_t rows, int64_t D, int64_t F) {
     if (rows <= 0 || D < 0 || F < 0 || rows > INT_MAX / 2 || D > (1 << 20) || F > (1 << 20)) return 0;
     const int64_t cols = 3 * D > 256 ? 3 * D : 256, n = na1d::block_partial_rows(rows) * cols;

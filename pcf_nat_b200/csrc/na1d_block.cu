@@ -310,6 +310,15 @@ template <typename E> __global__ void __launch_bounds__(256) cast_kernel(E* __re
     *reinterpret_cast<uint4*>(out + L.dst[k] + i0) = Cvt<E>::pack(f);   // the slot of each tensor is padded to 8 elements
 }
 
+// valid tokens of each utterance from its padding: one launch for what four elementwise ones did
+__global__ void __launch_bounds__(256) valid_tokens_kernel(int* __restrict__ out, const void* __restrict__ padding, bool is64, int n_padding, int N, int T) {
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    if (i >= N) return;
+    const int at = n_padding == 1 ? 0 : i;
+    const long long v = T - (is64 ? static_cast<const long long*>(padding)[at] : (long long)static_cast<const int*>(padding)[at]);
+    out[i] = (int)(v < 0 ? 0 : v > T ? T : v);
+}
+
 // ---------------------------------------------------------------- attentive statistics pooling
 // a = softmax over time of the logits; mu = sum a x, std = sqrt(max(sum a x^2 - mu^2, floor)), per channel. One pass: a lane
 // keeps the running maximum and the three sums of its 8 channels; the CTA's warps share the time axis and meet in shared
@@ -474,6 +483,10 @@ cudaError_t columns(void* dx, float* sums, float* part, const void* dy, const vo
 // CTAs of a column-sum pass over `rows` rows, and so the rows of partial sums it needs room for
 int block_partial_rows(long long rows) { return row_grid(rows, 3); }
 
+cudaError_t block_valid_tokens(int* out, const void* padding, bool is64, int n_padding, int N, int T, cudaStream_t st) {
+    valid_tokens_kernel<<<(N + 255) / 256, 256, 0, st>>>(out, padding, is64, n_padding, N, T);
+    return cudaGetLastError();
+}
 cudaError_t block_ln_fwd(void* y, void* sum, float* mean, float* rstd, const void* x, const void* dx, const float* w, const float* b,
                          int rows, int D, float eps, int dtype, cudaStream_t st) {
     return dtype == 0 ? ln_fwd<__nv_bfloat16>(y, sum, mean, rstd, x, dx, w, b, rows, D, eps, st)

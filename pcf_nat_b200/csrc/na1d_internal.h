@@ -75,6 +75,7 @@ cudaError_t tc_fused_bwd(void* dq, void* dk, void* dv, float* d_rpb, const void*
 
 // ---- row and column kernels of a transformer block and of the statistics pooling (na1d_block.cu)
 int block_partial_rows(long long rows);
+cudaError_t block_valid_tokens(int* out, const void* padding, bool is64, int n_padding, int N, int T, cudaStream_t st);
 cudaError_t block_ln_fwd(void* y, void* sum, float* mean, float* rstd, const void* x, const void* dx, const float* w, const float* b,
                          int rows, int D, float eps, int dtype, cudaStream_t st);
 cudaError_t block_ln_bwd(void* dx, float* sums, float* part, const void* dy, const void* x, const float* mean, const float* rstd,

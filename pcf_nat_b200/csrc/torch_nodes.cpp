@@ -1,0 +1,483 @@
+// The package's autograd nodes in C++: the fused operator, the fused operator on a packed projection output, the
+// drop-in pair, and the transformer block. They call the C ABI (include/na1d_b200.h) and nothing else of their own.
+//
+// A forward and backward of the operator through a Python autograd.Function cost 140 to 170 us of host time (argument
+// conversions through ctypes, and a backward that needs the interpreter on the autograd thread) while its kernels take 5 to
+// 60 us at the usual sizes: the host bound them all.
+//
+// Every entry returns None where the call is anything but plain eager tensors of the forms the kernels take -- wrapped
+// tensors, dispatch modes, tracing, functorch transforms, forward-mode derivatives, other types, layouts, sizes -- and the
+// caller goes on to the Python route, which supports or refuses it as it always has.
+#include <torch/extension.h>
+
+#include <ATen/cuda/CUDAContext.h>
+#include <c10/core/impl/LocalDispatchKeySet.h>
+#include <c10/core/impl/TorchDispatchModeTLS.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <torch/csrc/autograd/custom_function.h>
+#include <torch/csrc/jit/frontend/tracer.h>
+
+#include "../../include/na1d_b200.h"
+
+namespace {
+
+namespace py = pybind11;
+using at::Tensor;
+using torch::autograd::AutogradContext;
+using torch::autograd::variable_list;
+using OptTensor = std::optional<Tensor>;
+
+// Raises the package's own exception; also from a thread that does not hold the interpreter lock.
+[[noreturn]] void raise_status(int status, const char* where) {
+    py::gil_scoped_acquire gil;
+    py::object cls = py::module_::import("pcf_nat_b200._lib").attr("Na1dError");
+    py::object exc = cls(status, where);
+    PyErr_SetObject(cls.ptr(), exc.ptr());
+    throw py::error_already_set();
+}
+inline void check(int status, const char* where) {
+    if (status != 0) raise_status(status, where);
+}
+inline void* stream() { return at::cuda::getCurrentCUDAStream().stream(); }
+inline int code(const Tensor& t) { return t.scalar_type() == at::kBFloat16 ? NA1D_BF16 : NA1D_FP16; }
+inline void* ptr(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
+inline float* fptr(const Tensor& t) { return static_cast<float*>(ptr(t)); }
+inline Tensor empty_f32(at::IntArrayRef shape, const Tensor& like) { return at::empty(shape, like.options().dtype(at::kFloat)); }
+
+bool eager_mode() {
+    return c10::impl::TorchDispatchModeTLS::stack_len() == 0 && !torch::jit::tracer::isTracing() &&
+           !c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::FuncTorchDynamicLayerFrontMode);
+}
+bool plain(const Tensor& t) {
+    return t.defined() && t.has_storage() && t.is_cuda() && t.layout() == at::kStrided && !t.key_set().has(c10::DispatchKey::Python) &&
+           !t._is_zerotensor() && !t.is_neg() && !t._fw_grad(0).defined();
+}
+bool plain16(const Tensor& t) { return plain(t) && (t.scalar_type() == at::kBFloat16 || t.scalar_type() == at::kHalf); }
+// bias and valid lengths as the kernels want them; false: not a form this route takes
+bool prepare_rpb(const OptTensor& rpb, int64_t n, const Tensor& like) {
+    return !rpb || !rpb->defined() || (plain(*rpb) && rpb->device() == like.device() && rpb->numel() == n && at::isFloatingType(rpb->scalar_type()));
+}
+Tensor rpb32(const OptTensor& rpb) {
+    if (!rpb || !rpb->defined()) return Tensor();
+    const Tensor r = rpb->detach();
+    return (r.scalar_type() == at::kFloat ? r : r.to(at::kFloat)).contiguous();
+}
+bool prepare_valid(OptTensor& v, int64_t batch, const Tensor& like) {
+    if (!v || !v->defined()) { v.reset(); return true; }
+    if (!v->has_storage() || v->layout() != at::kStrided || v->key_set().has(c10::DispatchKey::Python) || v->numel() != batch || v->is_floating_point() || v->is_complex() ||
+        v->requires_grad())
+        return false;
+    v = v->to(like.device(), at::kInt).reshape({batch}).contiguous();
+    return true;
+}
+
+// ---------------------------------------------------------------- the operator on (N, T, C) tensors
+struct Cfg {
+    int64_t N, T, C, heads, win, left, dil;
+    double scale, drop_p;
+    uint64_t seed;
+};
+
+void op_forward(const Tensor& o, const Tensor& lse, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& r, const Tensor& vl, const Cfg& c) {
+    if (c.drop_p != 0.0)
+        check(na1d_fused_forward_dropout(ptr(o), fptr(lse), ptr(q), ptr(k), ptr(v), fptr(r), static_cast<int32_t*>(ptr(vl)), c.N, c.heads, c.T, c.C,
+                                         c.win, c.left, c.dil, (float)c.scale, (float)c.drop_p, c.seed, code(q), stream()),
+              "na1d_fused_forward_dropout");
+    else
+        check(na1d_fused_forward(ptr(o), fptr(lse), ptr(q), ptr(k), ptr(v), fptr(r), static_cast<int32_t*>(ptr(vl)), c.N, c.heads, c.T, c.C, c.win,
+                                 c.left, c.dil, (float)c.scale, code(q), stream()),
+              "na1d_fused_forward");
+}
+
+struct NA1dFused : public torch::autograd::Function<NA1dFused> {
+    static Tensor forward(AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& v, const OptTensor& rpb, const OptTensor& vl,
+                          int64_t heads, int64_t win, int64_t left, int64_t dil, double scale, double drop_p, int64_t seed) {
+        const Cfg c{q.size(0), q.size(1), q.size(2), heads, win, left, dil, scale, drop_p, (uint64_t)seed};
+        Tensor o = at::empty_like(q), lse = empty_f32({c.N, c.T}, q);
+        const Tensor valid = vl ? *vl : Tensor();
+        op_forward(o, lse, q, k, v, rpb32(rpb), valid, c);
+        ctx->save_for_backward({q, k, v, o, lse, rpb ? *rpb : Tensor(), valid});
+        auto& d = ctx->saved_data;
+        d["heads"] = heads; d["win"] = win; d["left"] = left; d["dil"] = dil; d["scale"] = scale; d["drop_p"] = drop_p; d["seed"] = seed;
+        return o;
+    }
+    static variable_list backward(AutogradContext* ctx, variable_list grads) {
+        const variable_list s = ctx->get_saved_variables();
+        const Tensor &q = s[0], &k = s[1], &v = s[2], &o = s[3], &lse = s[4], &rpb = s[5], &vl = s[6];
+        auto& d = ctx->saved_data;
+        const Cfg c{q.size(0), q.size(1), q.size(2), d["heads"].toInt(), d["win"].toInt(), d["left"].toInt(), d["dil"].toInt(), d["scale"].toDouble(),
+                    d["drop_p"].toDouble(), (uint64_t)d["seed"].toInt()};
+        const c10::cuda::CUDAGuard guard(q.device());
+        const Tensor d_o = grads[0].defined() ? grads[0].contiguous() : at::zeros_like(q);
+        Tensor dq = at::empty_like(q), dk = at::empty_like(k), dv = at::empty_like(v), delta = empty_f32({c.N, c.T}, q), d_rpb;
+        if (rpb.defined() && ctx->needs_input_grad(3)) d_rpb = at::zeros({c.heads, c.win}, q.options().dtype(at::kFloat));
+        const Tensor r = rpb32(rpb);
+        if (c.drop_p != 0.0)
+            check(na1d_fused_backward_dropout(ptr(dq), ptr(dk), ptr(dv), fptr(d_rpb), ptr(d_o), ptr(q), ptr(k), ptr(v), fptr(lse), fptr(r),
+                                              static_cast<int32_t*>(ptr(vl)), fptr(delta), c.N * c.T, c.N, c.heads, c.T, c.C, c.win, c.left, c.dil,
+                                              (float)c.scale, (float)c.drop_p, c.seed, code(q), stream()),
+                  "na1d_fused_backward_dropout");
+        else
+            check(na1d_fused_backward(ptr(dq), ptr(dk), ptr(dv), fptr(d_rpb), ptr(d_o), ptr(q), ptr(k), ptr(v), ptr(o), fptr(lse), fptr(r),
+                                      static_cast<int32_t*>(ptr(vl)), fptr(delta), c.N, c.heads, c.T, c.C, c.win, c.left, c.dil, (float)c.scale, code(q),
+                                      stream()),
+                  "na1d_fused_backward");
+        if (d_rpb.defined()) d_rpb = d_rpb.view(rpb.sizes()).to(rpb.scalar_type());
+        return {dq, dk, dv, d_rpb, Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
+    }
+};
+
+OptTensor fused(const Tensor& q, const Tensor& k, const Tensor& v, int64_t win, int64_t left, int64_t dil, double scale, OptTensor rpb, OptTensor vl,
+                int64_t heads, double drop_p, uint64_t seed) {
+    if (!eager_mode() || !plain16(q) || !plain16(k) || !plain16(v) || q.dim() != 3 || q.sizes() != k.sizes() || q.sizes() != v.sizes() ||
+        q.scalar_type() != k.scalar_type() || q.scalar_type() != v.scalar_type() || q.device() != k.device() || q.device() != v.device() ||
+        !q.is_contiguous() || !k.is_contiguous() || !v.is_contiguous() || heads <= 0 || win <= 0 || q.size(0) % heads != 0 || q.numel() == 0 ||
+        !prepare_rpb(rpb, heads * win, q))
+        return std::nullopt;
+    const c10::cuda::OptionalCUDAGuard guard(q.device());
+    if (!prepare_valid(vl, q.size(0) / heads, q)) return std::nullopt;
+    if (rpb && !rpb->defined()) rpb.reset();
+    if (at::GradMode::is_enabled() && (q.requires_grad() || k.requires_grad() || v.requires_grad() || (rpb && rpb->requires_grad())))
+        return NA1dFused::apply(q, k, v, rpb, vl, heads, win, left, dil, scale, drop_p, (int64_t)seed);
+    const Cfg c{q.size(0), q.size(1), q.size(2), heads, win, left, dil, scale, drop_p, seed};
+    Tensor o = at::empty_like(q);
+    op_forward(o, Tensor(), q, k, v, rpb32(rpb), vl ? *vl : Tensor(), c);
+    return o;
+}
+
+// ---------------------------------------------------------------- the drop-in pair: q.k^T over the window, and its product with v
+// rows (N, T, C) 16-bit, band (N, T, win) fp32; the six entry points differ in which of the three they write
+struct Band {
+    int64_t N, T, C, win, left, dil;
+    Band(const Tensor& rows, int64_t win_, int64_t left_, int64_t dil_)
+        : N(rows.size(0)), T(rows.size(1)), C(rows.size(2)), win(win_), left(left_), dil(dil_) {}
+    Tensor products(int (*f)(float*, const void*, const void*, int64_t, int64_t, int64_t, int64_t, int64_t, int64_t, int, void*), const char* name,
+                    const Tensor& a, const Tensor& b) const {
+        Tensor out = empty_f32({N, T, win}, a);
+        check(f(fptr(out), ptr(a), ptr(b), N, T, C, win, left, dil, code(a), stream()), name);
+        return out;
+    }
+    Tensor rows(int (*f)(void*, const float*, const void*, int64_t, int64_t, int64_t, int64_t, int64_t, int64_t, int, void*), const char* name,
+                const Tensor& band, const Tensor& x) const {
+        Tensor out = at::empty_like(x);
+        check(f(ptr(out), fptr(band), ptr(x), N, T, C, win, left, dil, code(x), stream()), name);
+        return out;
+    }
+};
+void keep_window(AutogradContext* ctx, int64_t win, int64_t left, int64_t dil) {
+    auto& d = ctx->saved_data;
+    d["win"] = win; d["left"] = left; d["dil"] = dil;
+}
+Band kept_window(AutogradContext* ctx, const Tensor& rows) {
+    auto& d = ctx->saved_data;
+    return Band(rows, d["win"].toInt(), d["left"].toInt(), d["dil"].toInt());
+}
+
+struct NA1dQK : public torch::autograd::Function<NA1dQK> {
+    static Tensor forward(AutogradContext* ctx, const Tensor& q, const Tensor& k, int64_t win, int64_t left, int64_t dil) {
+        ctx->save_for_backward({q, k});
+        keep_window(ctx, win, left, dil);
+        return Band(q, win, left, dil).products(na1d_qk_forward, "na1d_qk_forward", q, k);
+    }
+    static variable_list backward(AutogradContext* ctx, variable_list grads) {
+        const variable_list s = ctx->get_saved_variables();
+        const Band b = kept_window(ctx, s[0]);
+        const c10::cuda::CUDAGuard guard(s[0].device());
+        const Tensor g = grads[0].defined() ? grads[0].contiguous() : at::zeros({b.N, b.T, b.win}, s[0].options().dtype(at::kFloat));
+        Tensor dq = b.rows(na1d_q_backward, "na1d_q_backward", g, s[1]);
+        return {dq, b.rows(na1d_k_backward, "na1d_k_backward", g, s[0]), Tensor(), Tensor(), Tensor()};
+    }
+};
+struct NA1dAV : public torch::autograd::Function<NA1dAV> {
+    static Tensor forward(AutogradContext* ctx, const Tensor& attn, const Tensor& v, int64_t win, int64_t left, int64_t dil) {
+        ctx->save_for_backward({attn, v});
+        keep_window(ctx, win, left, dil);
+        return Band(v, win, left, dil).rows(na1d_av_forward, "na1d_av_forward", attn, v);
+    }
+    static variable_list backward(AutogradContext* ctx, variable_list grads) {
+        const variable_list s = ctx->get_saved_variables();
+        const Band b = kept_window(ctx, s[1]);
+        const c10::cuda::CUDAGuard guard(s[1].device());
+        const Tensor g = grads[0].defined() ? grads[0].contiguous() : at::zeros_like(s[1]);
+        Tensor da = b.products(na1d_a_backward, "na1d_a_backward", g, s[1]);
+        return {da, b.rows(na1d_v_backward, "na1d_v_backward", s[0], g), Tensor(), Tensor(), Tensor()};
+    }
+};
+
+bool band_rows(const Tensor& t) { return plain16(t) && t.dim() == 3 && t.numel() != 0 && t.is_contiguous(); }
+OptTensor qk(const Tensor& q, const Tensor& k, int64_t win, int64_t left, int64_t dil, bool bf16) {
+    if (!eager_mode() || !band_rows(q) || !band_rows(k) || q.sizes() != k.sizes() || q.device() != k.device() || win <= 0 ||
+        q.scalar_type() != k.scalar_type() || q.scalar_type() != (bf16 ? at::kBFloat16 : at::kHalf))
+        return std::nullopt;
+    const c10::cuda::OptionalCUDAGuard guard(q.device());
+    if (at::GradMode::is_enabled() && (q.requires_grad() || k.requires_grad())) return NA1dQK::apply(q, k, win, left, dil);
+    return Band(q, win, left, dil).products(na1d_qk_forward, "na1d_qk_forward", q, k);
+}
+OptTensor av(const Tensor& attn, const Tensor& v, int64_t win, int64_t left, int64_t dil, bool bf16) {
+    if (!eager_mode() || !band_rows(v) || !plain(attn) || attn.scalar_type() != at::kFloat || !attn.is_contiguous() || attn.dim() != 3 ||
+        attn.size(0) != v.size(0) || attn.size(1) != v.size(1) || attn.size(2) != win || attn.device() != v.device() ||
+        v.scalar_type() != (bf16 ? at::kBFloat16 : at::kHalf))
+        return std::nullopt;
+    const c10::cuda::OptionalCUDAGuard guard(v.device());
+    if (at::GradMode::is_enabled() && (attn.requires_grad() || v.requires_grad())) return NA1dAV::apply(attn, v, win, left, dil);
+    return Band(v, win, left, dil).rows(na1d_av_forward, "na1d_av_forward", attn, v);
+}
+
+// ---------------------------------------------------------------- the operator on a packed (batch, T, 3, heads, C) tensor
+struct Packed {
+    int64_t B, T, H, C, win, left, dil;
+    double scale;
+    int64_t in[3], out[3];   // {batch, head, token} element strides of q, k, v and of o
+    Packed(int64_t B_, int64_t T_, int64_t D, int64_t heads, int64_t win_, int64_t left_, int64_t dil_, double scale_)
+        : B(B_), T(T_), H(heads), C(D / heads), win(win_), left(left_), dil(dil_), scale(scale_), in{T * 3 * D, C, 3 * D}, out{T * D, C, D} {}
+    Packed(const Tensor& qkv, int64_t heads, int64_t win_, int64_t left_, int64_t dil_, double scale_)
+        : Packed(qkv.size(0), qkv.size(1), qkv.size(2) / 3, heads, win_, left_, dil_, scale_) {}
+};
+void packed_forward(const Tensor& o, const Tensor& lse, const Tensor& qkv, const Tensor& r, const Tensor& vl, const Packed& c) {
+    char* p = static_cast<char*>(ptr(qkv));
+    const int64_t step = c.H * c.C * 2;
+    check(na1d_fused_forward_strided(ptr(o), fptr(lse), p, p + step, p + 2 * step, fptr(r), static_cast<int32_t*>(ptr(vl)), c.out, c.in, c.in, c.in,
+                                     c.B * c.H, c.H, c.T, c.C, c.win, c.left, c.dil, (float)c.scale, code(qkv), stream()),
+          "na1d_fused_forward_strided");
+}
+void packed_backward(const Tensor& d_qkv, const Tensor& d_rpb, const Tensor& d_o, const Tensor& qkv, const Tensor& lse, const Tensor& r, const Tensor& vl,
+                     const Packed& c) {
+    char *p = static_cast<char*>(ptr(qkv)), *g = static_cast<char*>(ptr(d_qkv));
+    const int64_t step = c.H * c.C * 2, n = d_rpb.defined() ? 160 * c.H * c.win : 0;   // one partial row per CTA (one CTA per SM)
+    Tensor scratch;
+    if (n) scratch = empty_f32({n}, qkv);
+    check(na1d_fused_backward_strided(g, g + step, g + 2 * step, fptr(d_rpb), ptr(d_o), p, p + step, p + 2 * step, fptr(lse), fptr(r),
+                                      static_cast<int32_t*>(ptr(vl)), fptr(scratch), n, c.in, c.in, c.in, c.out, c.in, c.in, c.in, c.B * c.H, c.H, c.T,
+                                      c.C, c.win, c.left, c.dil, (float)c.scale, code(qkv), stream()),
+          "na1d_fused_backward_strided");
+}
+
+struct NA1dFusedPacked : public torch::autograd::Function<NA1dFusedPacked> {
+    static Tensor forward(AutogradContext* ctx, const Tensor& qkv, const OptTensor& rpb, const OptTensor& vl, int64_t heads, int64_t win, int64_t left,
+                          int64_t dil, double scale) {
+        const Packed c(qkv, heads, win, left, dil, scale);
+        Tensor o = at::empty({c.B, c.T, c.H * c.C}, qkv.options()), lse = empty_f32({c.B * c.H, c.T}, qkv);
+        const Tensor valid = vl ? *vl : Tensor();
+        packed_forward(o, lse, qkv, rpb32(rpb), valid, c);
+        ctx->save_for_backward({qkv, lse, rpb ? *rpb : Tensor(), valid});
+        auto& d = ctx->saved_data;
+        d["heads"] = heads; d["win"] = win; d["left"] = left; d["dil"] = dil; d["scale"] = scale;
+        return o;
+    }
+    static variable_list backward(AutogradContext* ctx, variable_list grads) {
+        const variable_list s = ctx->get_saved_variables();
+        const Tensor &qkv = s[0], &lse = s[1], &rpb = s[2], &vl = s[3];
+        auto& d = ctx->saved_data;
+        const Packed c(qkv, d["heads"].toInt(), d["win"].toInt(), d["left"].toInt(), d["dil"].toInt(), d["scale"].toDouble());
+        const c10::cuda::CUDAGuard guard(qkv.device());
+        const Tensor d_o = grads[0].defined() ? grads[0].contiguous() : at::zeros({c.B, c.T, c.H * c.C}, qkv.options());
+        Tensor d_qkv = at::empty_like(qkv), d_rpb;
+        if (rpb.defined() && ctx->needs_input_grad(1)) d_rpb = at::zeros({c.H, c.win}, qkv.options().dtype(at::kFloat));
+        packed_backward(d_qkv, d_rpb, d_o, qkv, lse, rpb32(rpb), vl, c);
+        if (d_rpb.defined()) d_rpb = d_rpb.view(rpb.sizes()).to(rpb.scalar_type());
+        return {d_qkv, d_rpb, Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
+    }
+};
+
+OptTensor packed(const Tensor& qkv, int64_t heads, int64_t win, int64_t left, int64_t dil, double scale, OptTensor rpb, OptTensor vl) {
+    if (!eager_mode() || !plain16(qkv) || qkv.dim() != 3 || qkv.numel() == 0 || !qkv.is_contiguous() || heads <= 0 || win <= 0 ||
+        qkv.size(2) % (3 * heads) != 0 || !prepare_rpb(rpb, heads * win, qkv))
+        return std::nullopt;
+    const c10::cuda::OptionalCUDAGuard guard(qkv.device());
+    if (!prepare_valid(vl, qkv.size(0), qkv)) return std::nullopt;
+    if (rpb && !rpb->defined()) rpb.reset();
+    if (at::GradMode::is_enabled() && (qkv.requires_grad() || (rpb && rpb->requires_grad())))
+        return NA1dFusedPacked::apply(qkv, rpb, vl, heads, win, left, dil, scale);
+    const Packed c(qkv, heads, win, left, dil, scale);
+    Tensor o = at::empty({c.B, c.T, c.H * c.C}, qkv.options());
+    packed_forward(o, Tensor(), qkv, rpb32(rpb), vl ? *vl : Tensor(), c);
+    return o;
+}
+
+// ---------------------------------------------------------------- the transformer block
+// Parameters in the order qkv.w, qkv.b, proj.w, proj.b, fc1.w, fc1.b, fc2.w, fc2.b, norm1.w, norm1.b, norm2.w, norm2.b, bias table.
+constexpr int kProj = 8, kParams = 13;
+constexpr int64_t kSlot = 64;   // elements: 128-byte slots of the packed 16-bit parameters
+
+struct Projections {
+    Tensor buf, t[kProj];
+    void views(at::IntArrayRef (&shapes)[kProj]) {
+        int64_t off = 0;
+        for (int i = 0; i < kProj; ++i) {
+            const int64_t n = c10::multiply_integers(shapes[i]);
+            t[i] = buf.narrow(0, off, n).view(shapes[i]);
+            off += (n + kSlot - 1) / kSlot * kSlot;
+        }
+    }
+    void cast(const Tensor* params, const Tensor& like) {
+        const float* src[kProj];
+        int64_t dst[kProj], n[kProj], total = 0;
+        at::IntArrayRef shapes[kProj];
+        for (int i = 0; i < kProj; ++i) {
+            shapes[i] = params[i].sizes();
+            src[i] = fptr(params[i]);
+            n[i] = params[i].numel();
+            dst[i] = total;
+            total += (n[i] + kSlot - 1) / kSlot * kSlot;
+        }
+        buf = at::empty({total}, like.options());
+        check(na1d_cast_parameters(ptr(buf), src, dst, n, kProj, code(like), stream()), "na1d_cast_parameters");
+        views(shapes);
+    }
+};
+
+struct BlockState {   // what the backward needs
+    Tensor s1, st1, h1, qkv, lse, o, s2, st2, h2, f, g, buf;
+};
+// one row of padding keeps both halves of the statistics 16-byte aligned
+inline Tensor row_stats(int64_t rows, const Tensor& like) { return empty_f32({2, (rows + 3) / 4 * 4}, like); }
+
+void layer_norm(Tensor& y, Tensor& sum, Tensor& st, const Tensor& x, const Tensor& dx, const Tensor& w, const Tensor& b, double eps, bool stats) {
+    const int64_t D = x.size(2), rows = x.size(0) * x.size(1);
+    y = at::empty_like(x);
+    sum = dx.defined() ? at::empty_like(x) : x;
+    if (stats) st = row_stats(rows, x);
+    check(na1d_layer_norm_forward(ptr(y), dx.defined() ? ptr(sum) : nullptr, fptr(st), stats ? fptr(st) + st.size(1) : nullptr, ptr(x), ptr(dx), fptr(w),
+                                  fptr(b), rows, D, (float)eps, code(x), stream()),
+          "na1d_layer_norm_forward");
+}
+Tensor layer_norm_backward(Tensor& sums, const Tensor& dy, const Tensor& s, const Tensor& st, const Tensor& w, const Tensor& res, const Tensor& scratch) {
+    const int64_t D = s.size(2);
+    Tensor ds = at::empty_like(s);
+    sums = empty_f32({3, D}, s);
+    check(na1d_layer_norm_backward(ptr(ds), fptr(sums), fptr(scratch), ptr(dy), ptr(s), fptr(st), fptr(st) + st.size(1), fptr(w), ptr(res),
+                                   s.size(0) * s.size(1), D, code(s), stream()),
+          "na1d_layer_norm_backward");
+    return ds;
+}
+
+// x (+ dx): the residual stream. Returns the stream after the attention branch and the MLP branch's output; their sum is the
+// block's output, taken inside the next block's first LayerNorm.
+std::pair<Tensor, Tensor> block_forward(const Tensor& x, const Tensor& dx, const Tensor& vl, const Packed& c, double eps1, double eps2,
+                                        const Tensor* p, BlockState* keep) {
+    const int64_t D = x.size(2), rows = c.B * c.T;
+    const bool stats = keep != nullptr;
+    BlockState st;
+    Projections w;
+    w.cast(p, x);
+    layer_norm(st.h1, st.s1, st.st1, x, dx, p[8], p[9], eps1, stats);
+    st.qkv = at::addmm(w.t[1], st.h1.view({rows, D}), w.t[0].t()).view({c.B, c.T, 3 * D});
+    st.o = at::empty({c.B, c.T, D}, x.options());
+    if (stats) st.lse = empty_f32({c.B * c.H, c.T}, x);
+    packed_forward(st.o, st.lse, st.qkv, p[12], vl, c);
+    const Tensor y = at::addmm(w.t[3], st.o.view({rows, D}), w.t[2].t()).view({c.B, c.T, D});
+    layer_norm(st.h2, st.s2, st.st2, st.s1, y, p[10], p[11], eps2, stats);
+    st.f = at::addmm(w.t[5], st.h2.view({rows, D}), w.t[4].t());
+    st.g = at::empty_like(st.f);
+    check(na1d_gelu_forward(ptr(st.g), ptr(st.f), st.f.numel(), code(x), stream()), "na1d_gelu_forward");
+    Tensor z = at::addmm(w.t[7], st.g, w.t[6].t()).view({c.B, c.T, D});
+    Tensor s2 = st.s2;
+    if (keep) {
+        st.buf = w.buf;
+        *keep = std::move(st);
+    }
+    return {s2, z};
+}
+
+struct NA1dBlock : public torch::autograd::Function<NA1dBlock> {
+    static variable_list forward(AutogradContext* ctx, const Tensor& x, const OptTensor& dx, const OptTensor& vl, int64_t heads, int64_t win, int64_t left,
+                                 double scale, double eps1, double eps2, const Tensor& p0, const Tensor& p1, const Tensor& p2, const Tensor& p3,
+                                 const Tensor& p4, const Tensor& p5, const Tensor& p6, const Tensor& p7, const Tensor& p8, const Tensor& p9,
+                                 const Tensor& p10, const Tensor& p11, const Tensor& p12) {
+        const Tensor p[kParams] = {p0, p1, p2, p3, p4, p5, p6, p7, p8, p9, p10, p11, p12};
+        const Packed c(x.size(0), x.size(1), x.size(2), heads, win, left, 1, scale);
+        BlockState st;
+        auto out = block_forward(x, dx ? *dx : Tensor(), vl ? *vl : Tensor(), c, eps1, eps2, p, &st);
+        ctx->save_for_backward({st.s1, st.st1, st.h1, st.qkv, st.lse, st.o, st.s2, st.st2, st.h2, st.f, st.g, st.buf, p8, p10, p12, vl ? *vl : Tensor()});
+        auto& d = ctx->saved_data;
+        d["heads"] = heads; d["win"] = win; d["left"] = left; d["scale"] = scale; d["dx"] = dx.has_value();
+        return {out.first, out.second};
+    }
+    static variable_list backward(AutogradContext* ctx, variable_list grads) {
+        const variable_list s = ctx->get_saved_variables();
+        const Tensor &s1 = s[0], &st1 = s[1], &h1 = s[2], &qkv = s[3], &lse = s[4], &o = s[5], &s2 = s[6], &st2 = s[7], &h2 = s[8], &f = s[9], &g = s[10],
+                     &buf = s[11], &n1w = s[12], &n2w = s[13], &rpb = s[14], &vl = s[15];
+        auto& data = ctx->saved_data;
+        const Packed c(qkv, data["heads"].toInt(), data["win"].toInt(), data["left"].toInt(), 1, data["scale"].toDouble());
+        const c10::cuda::CUDAGuard guard(s1.device());
+        const bool has_dx = data["dx"].toBool();
+        const int first = 1 + (has_dx ? 1 : 0) + (vl.defined() ? 1 : 0);   // edge of the first parameter
+        auto need = [&](int k) { return ctx->needs_input_grad(first + k); };
+        const int64_t D = s1.size(2), rows = c.B * c.T, F = f.size(1);
+        const std::vector<int64_t> shapes[kProj] = {{3 * D, D}, {3 * D}, {D, D}, {D}, {F, D}, {F}, {D, F}, {D}};
+        at::IntArrayRef refs[kProj];
+        for (int i = 0; i < kProj; ++i) refs[i] = shapes[i];
+        Projections w;
+        w.buf = buf;
+        w.views(refs);
+        const Tensor scratch = empty_f32({na1d_block_scratch_floats(rows, D, std::max(F, 3 * D))}, s1);
+        const Tensor d_z = (grads[1].defined() ? grads[1].contiguous() : at::zeros_like(s2)).view({rows, D});
+        const Tensor d_s2 = grads[0].defined() ? grads[0].contiguous() : Tensor();
+        // dy^T . inp, accumulated and returned in fp32
+        auto weight_grad = [&](int k, const Tensor& dy, const Tensor& inp) { return need(k) ? at::mm(dy.t(), inp, at::kFloat) : Tensor(); };
+        auto bias_grad = [&](int k, const Tensor& dy) {
+            if (!need(k)) return Tensor();
+            Tensor sums = empty_f32({dy.size(1)}, dy);
+            check(na1d_column_sums(fptr(sums), fptr(scratch), ptr(dy), rows, dy.size(1), code(dy), stream()), "na1d_column_sums");
+            return sums;
+        };
+        // MLP branch
+        Tensor d_w2 = weight_grad(6, d_z, g), d_b2 = bias_grad(7, d_z), d_b1 = empty_f32({F}, s1), d_f = at::empty_like(f);
+        {
+            const Tensor d_g = at::mm(d_z, w.t[6]);
+            check(na1d_gelu_backward(ptr(d_f), fptr(d_b1), fptr(scratch), ptr(d_g), ptr(f), rows, F, code(f), stream()), "na1d_gelu_backward");
+        }
+        Tensor d_w1 = weight_grad(4, d_f, h2.view({rows, D})), sums2, sums1;
+        const Tensor d_y = layer_norm_backward(sums2, at::mm(d_f, w.t[4]), s2, st2, n2w, d_s2, scratch);   // also the residual stream's gradient
+        d_f.reset();
+        // attention branch
+        const Tensor dy2 = d_y.view({rows, D});
+        Tensor d_pw = weight_grad(2, dy2, o.view({rows, D})), d_qkv = at::empty_like(qkv), d_rpb;
+        if (need(12)) d_rpb = at::zeros({c.H, c.win}, s1.options().dtype(at::kFloat));
+        packed_backward(d_qkv, d_rpb, at::mm(dy2, w.t[2]), qkv, lse, rpb, vl, c);
+        const Tensor dq2 = d_qkv.view({rows, 3 * D});
+        Tensor d_qw = weight_grad(0, dq2, h1.view({rows, D})), d_qb = bias_grad(1, dq2);
+        const Tensor d_x = layer_norm_backward(sums1, at::mm(dq2, w.t[0]), s1, st1, n1w, d_y, scratch);
+        if (d_rpb.defined()) d_rpb = d_rpb.view(rpb.sizes());
+        const Tensor none;
+        return {d_x, has_dx ? d_x : none, none, none, none, none, none, none, none, d_qw, d_qb, d_pw, sums2.select(0, 2), d_w1, d_b1, d_w2, d_b2,
+                sums1.select(0, 0), sums1.select(0, 1), sums2.select(0, 0), sums2.select(0, 1), d_rpb};
+    }
+};
+
+std::pair<Tensor, Tensor> block(const Tensor& x, const OptTensor& dx, const OptTensor& vl, int64_t heads, int64_t win, int64_t left, double scale,
+                                double eps1, double eps2, const std::vector<Tensor>& p) {
+    TORCH_CHECK(p.size() == kParams, "a block has 13 parameters");
+    const c10::cuda::OptionalCUDAGuard guard(x.device());
+    if (at::GradMode::is_enabled()) {
+        const variable_list r = NA1dBlock::apply(x, dx, vl, heads, win, left, scale, eps1, eps2, p[0], p[1], p[2], p[3], p[4], p[5], p[6], p[7], p[8],
+                                                 p[9], p[10], p[11], p[12]);
+        return {r[0], r[1]};
+    }
+    const Packed c(x.size(0), x.size(1), x.size(2), heads, win, left, 1, scale);
+    return block_forward(x, dx ? *dx : Tensor(), vl ? *vl : Tensor(), c, eps1, eps2, p.data(), nullptr);
+}
+
+// int32 (N): clamp(T - padding, 0, T); padding of one element counts for every utterance
+OptTensor valid_tokens(const Tensor& padding, int64_t T, int64_t N) {
+    if (!eager_mode() || !plain(padding) || (padding.scalar_type() != at::kInt && padding.scalar_type() != at::kLong) || !padding.is_contiguous() ||
+        padding.dim() > 1 || (padding.numel() != 1 && padding.numel() != N) || N <= 0 || T <= 0 || T > INT32_MAX)
+        return std::nullopt;
+    const c10::cuda::OptionalCUDAGuard guard(padding.device());
+    Tensor out = at::empty({N}, padding.options().dtype(at::kInt));
+    check(na1d_valid_tokens(static_cast<int32_t*>(ptr(out)), ptr(padding), padding.scalar_type() == at::kLong, padding.numel(), N, T, stream()),
+          "na1d_valid_tokens");
+    return out;
+}
+
+}  // namespace
+
+PYBIND11_MODULE(_na1d_torch, m) {
+    m.def("fused", &fused);
+    m.def("qk", &qk);
+    m.def("av", &av);
+    m.def("packed", &packed);
+    m.def("block", &block);
+    m.def("valid_tokens", &valid_tokens);
+    m.def("eager_mode", &eager_mode);
+}

@@ -74,7 +74,7 @@ def na1d_fused(q, k, v, win_size, left, dilation=1, scale=1.0, rpb=None, valid_l
     """``softmax(scale q.k^T + rpb + mask) . v`` over each query's window; (N*heads, T, C) in, same shape out.
 
     Under ``torch.compile`` / tracing (fake, functional or otherwise wrapped tensors) the call goes through the registered
-    ``torch.library`` ops; on plain eager tensors through ``NA1dFusedFunction``.
+    ``torch.library`` ops; on plain eager tensors through an autograd node (C++, or ``NA1dFusedFunction``).
 
     ``rpb``: ``(1, heads, 1, win)`` (or any shape with heads*win elements) fp32 parameter or None; ``valid_len``: int tensor
     or sequence of length N/heads (``T - padding``) or None. ``drop_p`` > 0 applies attention dropout (the reference's
@@ -82,8 +82,12 @@ def na1d_fused(q, k, v, win_size, left, dilation=1, scale=1.0, rpb=None, valid_l
     if drop_p and (type(q) is not Tensor or torch.compiler.is_compiling()):
         raise NotImplementedError("attention dropout is available on the eager route only")
     if type(q) is Tensor and not torch.compiler.is_compiling():
-        # plain eager tensors: the autograd.Function route skips the dispatcher's generated backward (host time of a
-        # forward+backward pair measured 5 to 35 % lower, depending on the host); same kernels, same saved tensors
+        # plain eager tensors: the C++ node (a forward and backward pass costs the host about a third of what the Python
+        # autograd.Function does, which in turn is cheaper than the dispatcher's generated backward); the Python node for
+        # what the C++ one leaves to it
+        o = ops.native_fused(q, k, v, win_size, left, dilation, scale, rpb, valid_len, heads, drop_p, seed)
+        if o is not None:
+            return o
         return ops.NA1dFusedFunction.apply(q, k, v, int(win_size), int(left), int(dilation), float(scale), rpb, valid_len,
                                            int(heads), float(drop_p), int(seed))
     if valid_len is not None and not isinstance(valid_len, Tensor):

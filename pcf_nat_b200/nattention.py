@@ -122,6 +122,10 @@ def _fused_forward_channels_first_packed(self, x, valid_len):
 
 def _valid_tokens(T, padding, N):
     """int32 (N,): tokens of each utterance that are not padding."""
+    if type(padding) is torch.Tensor and padding.is_cuda and not torch.compiler.is_compiling():
+        v = ops.native.valid_tokens(padding, T, N)
+        if v is not None:
+            return v
     return (T - padding.to(torch.int64)).clamp_(0, T).to(torch.int32).expand(N).contiguous()
 
 

@@ -16,8 +16,22 @@ import torch
 from . import ops
 
 
+def _plain(a, b):
+    return type(a) is torch.Tensor and type(b) is torch.Tensor and not torch.compiler.is_compiling()
+
+
 def _make_pair(tag, dtype):
+    bf16 = dtype == torch.bfloat16
+
     class QK(torch.autograd.Function):
+        @classmethod
+        def apply(cls, q, k, win_size, left, dilation=1):
+            if _plain(q, k):     # the same through the C++ node; None for what that leaves to this class
+                out = ops.native.qk(q, k, win_size, left, dilation, bf16)
+                if out is not None:
+                    return out
+            return super().apply(q, k, win_size, left, dilation)
+
         @staticmethod
         def forward(ctx, q, k, win_size, left, dilation=1):
             assert q.is_contiguous() and k.is_contiguous()
@@ -36,6 +50,14 @@ def _make_pair(tag, dtype):
             return q_gd, k_gd, None, None, None
 
     class AV(torch.autograd.Function):
+        @classmethod
+        def apply(cls, attn, v, win_size, left, dilation=1):
+            if _plain(attn, v):
+                out = ops.native.av(attn, v, win_size, left, dilation, bf16)
+                if out is not None:
+                    return out
+            return super().apply(attn, v, win_size, left, dilation)
+
         @staticmethod
         def forward(ctx, attn, v, win_size, left, dilation=1):
             assert attn.is_contiguous() and v.is_contiguous()

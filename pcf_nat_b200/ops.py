@@ -8,6 +8,11 @@ from . import _lib
 from ._lib import check
 
 _L = _lib.lib()
+try:
+    from . import _na1d_torch as native     # the C++ autograd nodes; each returns None for calls that take the Python route
+except ImportError as e:
+    raise ImportError("pcf_nat_b200: _na1d_torch.so is missing or was built for another torch (%s). Build it with "
+                      "`python pcf_nat_b200/_build.py`." % e) from e
 
 
 def _dtype_code(t):
@@ -268,6 +273,10 @@ class NA1dFusedPackedFunction(torch.autograd.Function):
 
 def na1d_fused_packed(qkv, heads, win_size, left, dilation=1, scale=1.0, rpb=None, valid_len=None):
     """``(batch, T, 3*heads*C)`` packed projection output -> ``(batch, T, heads*C)`` attention output, no layout copies."""
+    if type(qkv) is torch.Tensor and (valid_len is None or type(valid_len) is torch.Tensor) and not torch.compiler.is_compiling():
+        out = native.packed(qkv, int(heads), int(win_size), int(left), int(dilation), float(scale), rpb, valid_len)
+        if out is not None:
+            return out
     return NA1dFusedPackedFunction.apply(qkv, int(heads), int(win_size), int(left), int(dilation), float(scale), rpb, valid_len)
 
 
@@ -310,7 +319,19 @@ class NA1dFusedFunction(torch.autograd.Function):
         return dq, dk, dv, None, None, None, None, d_rpb, None, None, None, None
 
 
+def native_fused(q, k, v, win_size, left, dilation, scale, rpb, valid_len, heads, drop_p, seed):
+    """The fused operator through its C++ node, or None where the call has to take the Python route."""
+    if valid_len is not None and type(valid_len) is not torch.Tensor:
+        return None
+    return native.fused(q, k, v, int(win_size), int(left), int(dilation), float(scale), rpb, valid_len, int(heads), float(drop_p),
+                        int(seed) & 0xFFFFFFFFFFFFFFFF)
+
+
 def na1d_fused(q, k, v, win_size, left, dilation=1, scale=1.0, rpb=None, valid_len=None, heads=1, drop_p=0.0, seed=0):
+    if type(q) is torch.Tensor and not torch.compiler.is_compiling():
+        o = native_fused(q, k, v, win_size, left, dilation, scale, rpb, valid_len, heads, drop_p, seed)
+        if o is not None:
+            return o
     return NA1dFusedFunction.apply(q, k, v, win_size, left, dilation, scale, rpb, valid_len, heads, drop_p, seed)
 
 
