@@ -233,6 +233,19 @@ int na1d_column_sums(float* sums, float* scratch, const void* x, int64_t rows, i
 #define NA1D_CAST_MAX 16
 int na1d_cast_parameters(void* out, const float* const* src, const int64_t* dst, const int64_t* n, int count, int dtype,
                          void* stream);
+/* (N, C, T) -> (N, T, C) (to_tokens) or (N, T, C) -> (N, C, T), 16-bit; C a multiple of 8, the (N, T, C) side 16-byte aligned.
+ * Replaces the transposing copies around the channels-first layer, models/PCF_NATransformer.py:126-151. */
+int na1d_transpose(void* out, const void* in, int64_t N, int64_t C, int64_t T, int to_tokens, int dtype, void* stream);
+/* A grouped 1x1 convolution (models/PCF_NATransformer.py:66-68) as one dense matrix: w (parts*C, C/groups) and b (parts*C or
+ * NULL), fp32 (src32) or 16-bit, to out_w (parts*C, C) and out_b, 16-bit, zeros outside the group's columns. parts = 3 orders
+ * the rows as (q|k|v, head, channel): row which*C + f is output channel ((f % (C/groups))*groups + f / (C/groups))*3 + which, the
+ * channel shuffle and head split of :127-129. parts = 1 keeps the order. */
+int na1d_pack_grouped(void* out_w, void* out_b, const void* w, const void* b, int src32, int64_t C, int64_t groups, int parts,
+                      int dtype, void* stream);
+/* The transposed step for gradients: dense (parts*C, C) and sums (parts*C or NULL), fp32, to d_w (parts*C, C/groups) and d_b (or
+ * NULL), fp32 (dst32) or 16-bit. */
+int na1d_unpack_grouped(void* d_w, void* d_b, const float* dense, const float* sums, int dst32, int64_t C, int64_t groups, int parts,
+                        int dtype, void* stream);
 /* out (N, 2C) fp32 = [mu, std] with a = softmax over T of logits (N, T, C), mu = sum a x, std = sqrt(max(sum a x^2 - mu^2,
  * floor)). stats (3, N, C), for the backward (may be NULL): the logits' maximum, 1 / sum exp, sum a x^2. N <= 65535. */
 int na1d_stats_pool_forward(float* out, float* stats, const void* logits, const void* x, int64_t N, int64_t T,

@@ -91,6 +91,9 @@ for _name, _args in (
         ("na1d_gelu_backward", [_ptr] * 5 + [_i64, _i64]),
         ("na1d_column_sums", [_ptr] * 3 + [_i64, _i64]),
         ("na1d_cast_parameters", [_ptr] * 4 + [_i32]),
+        ("na1d_transpose", [_ptr, _ptr, _i64, _i64, _i64, _i32]),
+        ("na1d_pack_grouped", [_ptr] * 4 + [_i32, _i64, _i64, _i32]),
+        ("na1d_unpack_grouped", [_ptr] * 4 + [_i32, _i64, _i64, _i32]),
         ("na1d_stats_pool_forward", [_ptr] * 4 + [_i64] * 3 + [_f32]),
         ("na1d_stats_pool_backward", [_ptr] * 7 + [_i64] * 3 + [_f32])):
     _f = getattr(_lib, _name)

@@ -17,6 +17,7 @@ import torch.nn as nn
 
 from . import _lib, ops
 from ._lib import check
+from .nattention import NAttention, global_hooks, hooked
 
 _L = _lib.lib()
 _CODE = {torch.bfloat16: _lib.NA1D_BF16, torch.float16: _lib.NA1D_FP16}
@@ -95,25 +96,16 @@ def cast_parameters(params, dtype):
 
 
 # ------------------------------------------------------------------ the block (its autograd node is in csrc/torch_nodes.cpp)
-def _hooked(m):
-    return bool(m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks)
-
-
-def _global_hooks():
-    g = torch.nn.modules.module
-    return bool(g._global_forward_hooks or g._global_forward_pre_hooks or g._global_backward_hooks or g._global_backward_pre_hooks)
-
-
-def _block_parameters(blk, attention_class, x):
+def _block_parameters(blk, x):
     """The parameters of a block in the order of the node's arguments, or None where the block is anything but the plain one
     on fp32 parameters (a replaced or hooked submodule, another dtype, an odd size): it then runs module by module."""
     a, n1, n2, f1, f2 = blk.attn, blk.norm1, blk.norm2, blk.fc1, blk.fc2
-    if type(a) is not attention_class or type(n1) is not nn.LayerNorm or type(n2) is not nn.LayerNorm or a._na1d_layout != "channels_last":
+    if type(a) is not NAttention or type(n1) is not nn.LayerNorm or type(n2) is not nn.LayerNorm or a._na1d_layout != "channels_last":
         return None
     if "forward" in a.__dict__ or any(type(m) is not nn.Linear for m in (a.qkv, a.proj, f1, f2)):
         return None
     mods = (blk, a, n1, n2, f1, f2, a.qkv, a.proj, a.attn_drop, a.proj_drop)
-    if any(_hooked(m) for m in mods) or any("forward" in m.__dict__ for m in mods):
+    if any(hooked(m) for m in mods) or any("forward" in m.__dict__ for m in mods):
         return None
     if a.training and (a.attn_drop.p or a.proj_drop.p) or a.dilation != 1 or type(a.attn_drop) is not nn.Dropout or type(a.proj_drop) is not nn.Dropout:
         return None
@@ -130,19 +122,19 @@ def _block_parameters(blk, attention_class, x):
     return ps
 
 
-def run_blocks(blocks, x, valid, attention_class):
+def run_blocks(blocks, x, valid):
     """The blocks applied to the residual stream x (batch, T, D), or None where they have to run module by module.
     ``valid``: valid tokens per utterance (int32, contiguous) or None."""
     if (type(x) is not torch.Tensor or not x.is_cuda or x.dim() != 3 or x.numel() == 0 or torch.compiler.is_compiling() or
             not torch.is_autocast_enabled() or not ops.native.eager_mode() or torch.autograd.forward_ad._current_level >= 0):
         return None
     dt = torch.get_autocast_dtype("cuda")
-    if x.dtype != dt or dt not in _CODE or _global_hooks() or x.shape[0] * x.shape[1] * x.shape[2] >= 2 ** 31:
+    if x.dtype != dt or dt not in _CODE or global_hooks() or x.shape[0] * x.shape[1] * x.shape[2] >= 2 ** 31:
         return None
     B, T, D = x.shape
     plan = []
     for blk in blocks:
-        ps = _block_parameters(blk, attention_class, x)
+        ps = _block_parameters(blk, x)
         if ps is None:
             return None
         a = blk.attn

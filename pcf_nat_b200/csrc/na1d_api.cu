@@ -419,6 +419,33 @@ int na1d_cast_parameters(void* out, const float* const* src, const int64_t* dst,
     }
     return cuda_status(na1d::block_cast(out, src, dst, n, count, dtype, (cudaStream_t)stream));
 }
+int na1d_transpose(void* out, const void* in, int64_t N, int64_t C, int64_t T, int to_tokens, int dtype, void* stream) {
+    NA1D_REQUIRE_PTR(out); NA1D_REQUIRE_PTR(in);
+    NA1D_REQUIRE_ALIGNED(to_tokens ? out : in);
+    if (reinterpret_cast<uintptr_t>(to_tokens ? in : out) & 1u) return NA1D_ERR_MISALIGNED;
+    if (int s = check_block(T, C, 1 << 20, dtype)) return s;
+    if (N <= 0 || N > 65535 || T > (1 << 20)) return NA1D_ERR_BAD_SHAPE;
+    return cuda_status(na1d::block_transpose(out, in, (int)N, (int)C, (int)T, to_tokens != 0, dtype, (cudaStream_t)stream));
+}
+static int check_grouped(int64_t C, int64_t groups, int parts, int dtype) {
+    if (dtype != NA1D_BF16 && dtype != NA1D_FP16) return NA1D_ERR_BAD_DTYPE;
+    if (C <= 0 || C % 8 != 0 || C > 8192 || groups <= 0 || C % groups != 0 || (parts != 1 && parts != 3)) return NA1D_ERR_BAD_SHAPE;
+    return NA1D_OK;
+}
+int na1d_pack_grouped(void* out_w, void* out_b, const void* w, const void* b, int src32, int64_t C, int64_t groups, int parts,
+                      int dtype, void* stream) {
+    NA1D_REQUIRE_PTR(out_w); NA1D_REQUIRE_PTR(w);
+    if ((out_b == nullptr) != (b == nullptr)) return NA1D_ERR_NULL_POINTER;
+    if (int s = check_grouped(C, groups, parts, dtype)) return s;
+    return cuda_status(na1d::block_pack_grouped(out_w, out_b, w, b, src32 != 0, (int)C, (int)groups, parts, dtype, (cudaStream_t)stream));
+}
+int na1d_unpack_grouped(void* d_w, void* d_b, const float* dense, const float* sums, int dst32, int64_t C, int64_t groups, int parts,
+                        int dtype, void* stream) {
+    if (d_w == nullptr && d_b == nullptr) return NA1D_ERR_NULL_POINTER;
+    if ((d_w == nullptr) != (dense == nullptr) || (d_b == nullptr) != (sums == nullptr)) return NA1D_ERR_NULL_POINTER;
+    if (int s = check_grouped(C, groups, parts, dtype)) return s;
+    return cuda_status(na1d::block_unpack_grouped(d_w, d_b, dense, sums, dst32 != 0, (int)C, (int)groups, parts, dtype, (cudaStream_t)stream));
+}
 int na1d_stats_pool_forward(float* out, float* stats, const void* logits, const void* x, int64_t N, int64_t T,
                             int64_t C, float floor, int dtype, void* stream) {
     if (int s = check_pointers(out, logits, x)) return s;

@@ -319,6 +319,90 @@ __global__ void __launch_bounds__(256) valid_tokens_kernel(int* __restrict__ out
     out[i] = (int)(v < 0 ? 0 : v > T ? T : v);
 }
 
+// ---------------------------------------------------------------- channels-first layers: transposes and grouped weights
+// A 64-channel x 64-token tile through shared memory. The token side is read or written in pairs (4 bytes) where the rows allow
+// it (an even token count, an even base), the channel side in 16-byte units; the odd pitch of 65 elements keeps both
+// phases free of bank conflicts. 512 x 256 x 150: 72 us per copy before, 12 us of HBM time.
+constexpr int kTile = 64, kTilePitch = 65;
+template <bool TO_TOKENS, bool PAIRS>
+__global__ void __launch_bounds__(256) transpose_kernel(uint16_t* __restrict__ out, const uint16_t* __restrict__ in, int C, int T) {
+    __shared__ uint16_t sm[kTile * kTilePitch];   // [token][channel]
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c0 = blockIdx.x * kTile, t0 = blockIdx.y * kTile;
+    const size_t base = (size_t)blockIdx.z * C * T;
+    const int t = t0 + 2 * lane;                  // channel-major side: lane -> two tokens, warp -> channels warp, warp + 8, ...
+    auto tokens_phase = [&](auto&& f) {
+#pragma unroll
+        for (int i = 0; i < kTile / 8; ++i) {
+            const int c = warp + 8 * i;
+            if (c0 + c < C && t < T) f(c, base + (size_t)(c0 + c) * T + t);
+        }
+    };
+    auto channels_phase = [&](auto&& f) {         // token-major side: 8 lanes cover a token's 64 channels
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const int row = (threadIdx.x >> 3) + 32 * i, c = (threadIdx.x & 7) * 8;
+            if (t0 + row < T && c0 + c < C) f(sm + row * kTilePitch + c, base + (size_t)(t0 + row) * C + c0 + c);
+        }
+    };
+    if constexpr (TO_TOKENS) {
+        uint32_t v[kTile / 8];
+        tokens_phase([&](int c, size_t at) {
+            v[c >> 3] = PAIRS ? *reinterpret_cast<const uint32_t*>(in + at) : (uint32_t)in[at] | (t + 1 < T ? (uint32_t)in[at + 1] << 16 : 0u);
+        });
+        tokens_phase([&](int c, size_t) {
+            sm[2 * lane * kTilePitch + c] = (uint16_t)v[c >> 3];
+            sm[(2 * lane + 1) * kTilePitch + c] = (uint16_t)(v[c >> 3] >> 16);
+        });
+        __syncthreads();
+        channels_phase([&](const uint16_t* s, size_t at) {
+            uint4 u;
+            u.x = s[0] | (uint32_t)s[1] << 16; u.y = s[2] | (uint32_t)s[3] << 16; u.z = s[4] | (uint32_t)s[5] << 16; u.w = s[6] | (uint32_t)s[7] << 16;
+            *reinterpret_cast<uint4*>(out + at) = u;
+        });
+    } else {
+        channels_phase([&](uint16_t* s, size_t at) {
+            const uint4 u = *reinterpret_cast<const uint4*>(in + at);
+            const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) { s[2 * e] = (uint16_t)w[e]; s[2 * e + 1] = (uint16_t)(w[e] >> 16); }
+        });
+        __syncthreads();
+        tokens_phase([&](int c, size_t at) {
+            const uint16_t a = sm[2 * lane * kTilePitch + c], b = sm[(2 * lane + 1) * kTilePitch + c];
+            if constexpr (PAIRS) {
+                *reinterpret_cast<uint32_t*>(out + at) = a | (uint32_t)b << 16;
+            } else {
+                out[at] = a;
+                if (t + 1 < T) out[at + 1] = b;
+            }
+        });
+    }
+}
+
+// convolution output channel of row r of the dense matrix
+__device__ __forceinline__ int grouped_channel(int r, int C, int groups, int parts) {
+    if (parts == 1) return r;
+    const int which = r / C, f = r - which * C, P = C / groups;
+    return ((f % P) * groups + f / P) * 3 + which;
+}
+// one CTA per row of the dense matrix
+template <typename E, typename S>
+__global__ void __launch_bounds__(128) pack_grouped_kernel(E* __restrict__ out_w, E* __restrict__ out_b, const S* __restrict__ w,
+                                                           const S* __restrict__ b, int C, int groups, int parts) {
+    const int r = blockIdx.x, P = C / groups, ch = grouped_channel(r, C, groups, parts), first = ch / (parts * P) * P;
+    for (int c = threadIdx.x; c < C; c += 128)
+        out_w[(size_t)r * C + c] = c >= first && c < first + P ? (E)(float)w[(size_t)ch * P + c - first] : (E)0.f;
+    if (b && threadIdx.x == 0) out_b[r] = (E)(float)b[ch];
+}
+template <typename D>
+__global__ void __launch_bounds__(128) unpack_grouped_kernel(D* __restrict__ d_w, D* __restrict__ d_b, const float* __restrict__ dense,
+                                                             const float* __restrict__ sums, int C, int groups, int parts) {
+    const int r = blockIdx.x, P = C / groups, ch = grouped_channel(r, C, groups, parts), first = ch / (parts * P) * P;
+    if (d_w)
+        for (int c = threadIdx.x; c < P; c += 128) d_w[(size_t)ch * P + c] = (D)dense[(size_t)r * C + first + c];
+    if (d_b && threadIdx.x == 0) d_b[ch] = (D)sums[r];
+}
+
 // ---------------------------------------------------------------- attentive statistics pooling
 // a = softmax over time of the logits; mu = sum a x, std = sqrt(max(sum a x^2 - mu^2, floor)), per channel. One pass: a lane
 // keeps the running maximum and the three sums of its 8 channels; the CTA's warps share the time axis and meet in shared
@@ -523,6 +607,36 @@ cudaError_t block_cast(void* out, const float* const* src, const int64_t* dst, c
     }
     if (dtype == 0) cast_kernel<<<L.first[count], 256, 0, st>>>((__nv_bfloat16*)out, L);
     else cast_kernel<<<L.first[count], 256, 0, st>>>((__half*)out, L);
+    return cudaGetLastError();
+}
+cudaError_t block_transpose(void* out, const void* in, int N, int C, int T, bool to_tokens, int dtype, cudaStream_t st) {
+    const dim3 grid((C + kTile - 1) / kTile, (T + kTile - 1) / kTile, N);
+    const bool pairs = T % 2 == 0 && (reinterpret_cast<uintptr_t>(to_tokens ? in : out) & 3u) == 0;
+    uint16_t* o = (uint16_t*)out;
+    const uint16_t* i = (const uint16_t*)in;
+    if (to_tokens) { if (pairs) transpose_kernel<true, true><<<grid, 256, 0, st>>>(o, i, C, T); else transpose_kernel<true, false><<<grid, 256, 0, st>>>(o, i, C, T); }
+    else { if (pairs) transpose_kernel<false, true><<<grid, 256, 0, st>>>(o, i, C, T); else transpose_kernel<false, false><<<grid, 256, 0, st>>>(o, i, C, T); }
+    return cudaGetLastError();
+}
+cudaError_t block_pack_grouped(void* out_w, void* out_b, const void* w, const void* b, bool src32, int C, int groups, int parts, int dtype,
+                               cudaStream_t st) {
+    const int rows = parts * C;
+    using B = __nv_bfloat16;
+    if (dtype == 0) {
+        if (src32) pack_grouped_kernel<<<rows, 128, 0, st>>>((B*)out_w, (B*)out_b, (const float*)w, (const float*)b, C, groups, parts);
+        else pack_grouped_kernel<<<rows, 128, 0, st>>>((B*)out_w, (B*)out_b, (const B*)w, (const B*)b, C, groups, parts);
+    } else {
+        if (src32) pack_grouped_kernel<<<rows, 128, 0, st>>>((__half*)out_w, (__half*)out_b, (const float*)w, (const float*)b, C, groups, parts);
+        else pack_grouped_kernel<<<rows, 128, 0, st>>>((__half*)out_w, (__half*)out_b, (const __half*)w, (const __half*)b, C, groups, parts);
+    }
+    return cudaGetLastError();
+}
+cudaError_t block_unpack_grouped(void* d_w, void* d_b, const float* dense, const float* sums, bool dst32, int C, int groups, int parts, int dtype,
+                                 cudaStream_t st) {
+    const int rows = parts * C;
+    if (dst32) unpack_grouped_kernel<<<rows, 128, 0, st>>>((float*)d_w, (float*)d_b, dense, sums, C, groups, parts);
+    else if (dtype == 0) unpack_grouped_kernel<<<rows, 128, 0, st>>>((__nv_bfloat16*)d_w, (__nv_bfloat16*)d_b, dense, sums, C, groups, parts);
+    else unpack_grouped_kernel<<<rows, 128, 0, st>>>((__half*)d_w, (__half*)d_b, dense, sums, C, groups, parts);
     return cudaGetLastError();
 }
 cudaError_t block_pool_fwd(float* out, float* stats, const void* logits, const void* x, int N, int T, int C, float floor_var,

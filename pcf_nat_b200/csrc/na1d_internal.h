@@ -84,6 +84,11 @@ cudaError_t block_gelu_fwd(void* y, const void* x, long long n, int dtype, cudaS
 cudaError_t block_gelu_bwd(void* dx, float* sums, float* part, const void* dy, const void* x, int rows, int F, int dtype, cudaStream_t st);
 cudaError_t block_column_sums(float* sums, float* part, const void* x, int rows, int F, int dtype, cudaStream_t st);
 cudaError_t block_cast(void* out, const float* const* src, const int64_t* dst, const int64_t* n, int count, int dtype, cudaStream_t st);
+cudaError_t block_transpose(void* out, const void* in, int N, int C, int T, bool to_tokens, int dtype, cudaStream_t st);
+cudaError_t block_pack_grouped(void* out_w, void* out_b, const void* w, const void* b, bool src32, int C, int groups, int parts, int dtype,
+                               cudaStream_t st);
+cudaError_t block_unpack_grouped(void* d_w, void* d_b, const float* dense, const float* sums, bool dst32, int C, int groups, int parts, int dtype,
+                                 cudaStream_t st);
 cudaError_t block_pool_fwd(float* out, float* stats, const void* logits, const void* x, int N, int T, int C, float floor_var,
                            int dtype, cudaStream_t st);
 cudaError_t block_pool_bwd(void* d_logits, void* dx, const float* d_out, const float* out, const float* stats,

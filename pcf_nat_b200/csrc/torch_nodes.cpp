@@ -1,5 +1,5 @@
 // The package's autograd nodes in C++: the fused operator, the fused operator on a packed projection output, the
-// drop-in pair, and the transformer block. They call the C ABI (include/na1d_b200.h) and nothing else of their own.
+// drop-in pair, the attention layer, and the transformer block. They call the C ABI (include/na1d_b200.h) and nothing else of their own.
 //
 // A forward and backward of the operator through a Python autograd.Function cost 140 to 170 us of host time (argument
 // conversions through ctypes, and a backward that needs the interpreter on the autograd thread) while its kernels take 5 to
@@ -10,6 +10,7 @@
 // caller goes on to the Python route, which supports or refuses it as it always has.
 #include <torch/extension.h>
 
+#include <ATen/autocast_mode.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/core/impl/LocalDispatchKeySet.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
@@ -458,6 +459,161 @@ std::pair<Tensor, Tensor> block(const Tensor& x, const OptTensor& dx, const OptT
     return block_forward(x, dx ? *dx : Tensor(), vl ? *vl : Tensor(), c, eps1, eps2, p.data(), nullptr);
 }
 
+// ---------------------------------------------------------------- the attention layer
+// Channels first ((N, C, T) in and out, grouped 1x1 convolutions): the layout changes once on the C-channel input and once on
+// the output; in between both convolutions are one GEMM each over all N*T tokens (dense block-diagonal weights: at these
+// sizes the tensor cores make the zeros free), their rows ordered so that the result is the packed tensor the attention reads.
+// Channels last ((N, T, C), linear projections): the projections as they are. In both, parameters are rounded to 16 bits by one
+// launch per projection (or layer) and bias gradients are column sums of this library.
+struct LayerShape {
+    int64_t B, T, D, groups;
+    bool first;
+    LayerShape(const Tensor& x, bool first_, int64_t groups_)
+        : B(x.size(0)), T(x.size(first_ ? 2 : 1)), D(x.size(first_ ? 1 : 2)), groups(groups_), first(first_) {}
+    int64_t rows() const { return B * T; }
+};
+struct LayerWeights {
+    Tensor qw, qb, pw, pb;   // 16-bit, dense (3D, D), (3D), (D, D), (D); biases may be undefined
+    LayerWeights(const Tensor& x, const LayerShape& l, const Tensor& qw_, const OptTensor& qb_, const Tensor& pw_, const OptTensor& pb_) {
+        const Tensor src[4] = {qw_, qb_ ? *qb_ : Tensor(), pw_, pb_ ? *pb_ : Tensor()};
+        Tensor* dst[4] = {&qw, &qb, &pw, &pb};
+        const int64_t n[4] = {3 * l.D * l.D, 3 * l.D, l.D * l.D, l.D};
+        const bool src32 = qw_.scalar_type() == at::kFloat;
+        if (l.first || src32) {
+            const Tensor buf = at::empty({n[0] + n[1] + n[2] + n[3] + 4 * kSlot}, x.options());
+            const float* from[4];
+            int64_t offs[4], sizes[4], off = 0;
+            int count = 0;
+            for (int i = 0; i < 4; ++i) {
+                if (!src[i].defined()) continue;
+                *dst[i] = i & 1 ? buf.narrow(0, off, n[i]) : buf.narrow(0, off, n[i]).view({n[i] / l.D, l.D});
+                from[count] = fptr(src[i]); offs[count] = off; sizes[count] = n[i]; ++count;
+                off += (n[i] + kSlot - 1) / kSlot * kSlot;
+            }
+            if (l.first) {
+                check(na1d_pack_grouped(ptr(qw), ptr(qb), ptr(src[0]), ptr(src[1]), src32, l.D, l.groups, 3, code(x), stream()), "na1d_pack_grouped");
+                check(na1d_pack_grouped(ptr(pw), ptr(pb), ptr(src[2]), ptr(src[3]), src32, l.D, l.groups, 1, code(x), stream()), "na1d_pack_grouped");
+            } else {
+                check(na1d_cast_parameters(ptr(buf), from, offs, sizes, count, code(x), stream()), "na1d_cast_parameters");
+            }
+        } else {
+            for (int i = 0; i < 4; ++i) *dst[i] = src[i].defined() ? src[i].detach() : Tensor();
+        }
+    }
+};
+Tensor project(const Tensor& x, const Tensor& w, const Tensor& b) { return b.defined() ? at::addmm(b, x, w.t()) : at::mm(x, w.t()); }
+Tensor transposed(const Tensor& in, const LayerShape& l, bool to_tokens) {
+    Tensor out = to_tokens ? at::empty({l.B, l.T, l.D}, in.options()) : at::empty({l.B, l.D, l.T}, in.options());
+    check(na1d_transpose(ptr(out), ptr(in), l.B, l.D, l.T, to_tokens, code(in), stream()), "na1d_transpose");
+    return out;
+}
+// gradients of one projection's parameters, fp32 sums in the parameters' own type, shape and order
+struct ProjectionGrads {
+    Tensor w, b;
+    ProjectionGrads(bool need_w, bool need_b, const Tensor& dy, const Tensor& x, const Tensor& scratch, at::IntArrayRef w_shape, at::ScalarType type,
+                    const LayerShape& l, int parts) {
+        if (!need_w && !need_b) return;
+        Tensor dense, sums;
+        if (need_w) dense = at::mm(dy.t(), x, at::kFloat);
+        if (need_b) {
+            sums = empty_f32({parts * l.D}, dy);
+            check(na1d_column_sums(fptr(sums), fptr(scratch), ptr(dy), dy.size(0), dy.size(1), code(dy), stream()), "na1d_column_sums");
+        }
+        if (!l.first) {
+            if (need_w) w = dense.to(type);
+            if (need_b) b = sums.to(type);
+            return;
+        }
+        const auto opts = dy.options().dtype(type);
+        if (need_w) w = at::empty(w_shape, opts);
+        if (need_b) b = at::empty({parts * l.D}, opts);
+        check(na1d_unpack_grouped(ptr(w), ptr(b), fptr(dense), fptr(sums), type == at::kFloat, l.D, l.groups, parts, code(dy), stream()),
+              "na1d_unpack_grouped");
+    }
+};
+struct LayerState { Tensor xt, qkv, lse, o, qw, pw; };
+Tensor layer_forward(const Tensor& x, const LayerShape& l, const Tensor& vl, const Tensor& r, const Tensor& qw, const OptTensor& qb, const Tensor& pw,
+                     const OptTensor& pb, const Packed& c, LayerState* keep) {
+    const LayerWeights w(x, l, qw, qb, pw, pb);
+    LayerState s;
+    s.xt = l.first ? transposed(x, l, true) : x;
+    s.qkv = project(s.xt.view({l.rows(), l.D}), w.qw, w.qb).view({l.B, l.T, 3 * l.D});
+    s.o = at::empty({l.B, l.T, l.D}, x.options());
+    if (keep) s.lse = empty_f32({l.B * c.H, l.T}, x);
+    packed_forward(s.o, s.lse, s.qkv, r, vl, c);
+    Tensor y = project(s.o.view({l.rows(), l.D}), w.pw, w.pb);
+    y = l.first ? transposed(y, l, false) : y.view({l.B, l.T, l.D});
+    if (keep) { s.qw = w.qw; s.pw = w.pw; *keep = std::move(s); }
+    return y;
+}
+struct NA1dLayer : public torch::autograd::Function<NA1dLayer> {
+    static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& rpb, const Tensor& qw, const Tensor& pw, const OptTensor& qb,
+                          const OptTensor& pb, const OptTensor& vl, bool first, int64_t heads, int64_t groups, int64_t win, int64_t left, int64_t dil,
+                          double scale) {
+        const LayerShape l(x, first, groups);
+        const Packed c(l.B, l.T, l.D, heads, win, left, dil, scale);
+        LayerState s;
+        Tensor y = layer_forward(x, l, vl ? *vl : Tensor(), rpb32(rpb), qw, qb, pw, pb, c, &s);
+        ctx->save_for_backward({s.xt, s.qkv, s.lse, s.o, s.qw, s.pw, rpb, vl ? *vl : Tensor()});
+        auto& d = ctx->saved_data;
+        d["first"] = first; d["heads"] = heads; d["groups"] = groups; d["win"] = win; d["left"] = left; d["dil"] = dil; d["scale"] = scale;
+        d["qb"] = qb.has_value(); d["pb"] = pb.has_value();
+        d["qw_shape"] = qw.sizes().vec(); d["pw_shape"] = pw.sizes().vec(); d["type"] = (int64_t)qw.scalar_type();
+        return y;
+    }
+    static variable_list backward(AutogradContext* ctx, variable_list grads) {
+        const variable_list s = ctx->get_saved_variables();
+        const Tensor &xt = s[0], &qkv = s[1], &lse = s[2], &o = s[3], &qw = s[4], &pw = s[5], &rpb = s[6], &vl = s[7];
+        auto& d = ctx->saved_data;
+        const Packed c(qkv, d["heads"].toInt(), d["win"].toInt(), d["left"].toInt(), d["dil"].toInt(), d["scale"].toDouble());
+        LayerShape l(xt, false, d["groups"].toInt());
+        l.first = d["first"].toBool();
+        const c10::cuda::CUDAGuard guard(qkv.device());
+        const auto type = (at::ScalarType)d["type"].toInt();
+        const bool has_qb = d["qb"].toBool(), has_pb = d["pb"].toBool();
+        const int qb_edge = 4, pb_edge = 4 + (has_qb ? 1 : 0);
+        const Tensor scratch = empty_f32({na1d_block_scratch_floats(l.rows(), 0, 3 * l.D)}, xt);
+        Tensor dy = grads[0].defined() ? grads[0].contiguous() : at::zeros(l.first ? at::IntArrayRef({l.B, l.D, l.T}) : xt.sizes(), xt.options());
+        dy = (l.first ? transposed(dy, l, true) : dy).view({l.rows(), l.D});
+        ProjectionGrads gp(ctx->needs_input_grad(3), has_pb && ctx->needs_input_grad(pb_edge), dy, o.view({l.rows(), l.D}), scratch,
+                           d["pw_shape"].toIntVector(), type, l, 1);
+        Tensor d_qkv = at::empty_like(qkv), d_rpb, d_x;
+        if (ctx->needs_input_grad(1)) d_rpb = at::zeros({c.H, c.win}, xt.options().dtype(at::kFloat));
+        packed_backward(d_qkv, d_rpb, at::mm(dy, pw), qkv, lse, rpb32(rpb), vl, c);
+        const Tensor dq = d_qkv.view({l.rows(), 3 * l.D});
+        ProjectionGrads gq(ctx->needs_input_grad(2), has_qb && ctx->needs_input_grad(qb_edge), dq, xt.view({l.rows(), l.D}), scratch,
+                           d["qw_shape"].toIntVector(), type, l, 3);
+        if (ctx->needs_input_grad(0)) {
+            d_x = at::mm(dq, qw);
+            d_x = l.first ? transposed(d_x, l, false) : d_x.view({l.B, l.T, l.D});
+        }
+        if (d_rpb.defined()) d_rpb = d_rpb.view(rpb.sizes()).to(rpb.scalar_type());
+        const Tensor none;
+        return {d_x, d_rpb, gq.w, gp.w, gq.b, gp.b, none, none, none, none, none, none, none, none};
+    }
+};
+
+// 16-bit x; weights and biases all of x's type, or (under autocast to x's type) all fp32
+OptTensor layer(const Tensor& x, bool first, const Tensor& rpb, const Tensor& qw, const OptTensor& qb, const Tensor& pw, const OptTensor& pb,
+                int64_t heads, int64_t groups, int64_t win, int64_t left, int64_t dil, double scale, OptTensor vl) {
+    if (!eager_mode() || !plain16(x) || x.dim() != 3 || x.numel() == 0 || !x.is_contiguous() || x.size(0) > 65535 || heads <= 0 || win <= 0 || groups <= 0)
+        return std::nullopt;
+    const LayerShape l(x, first, groups);
+    const bool cast = at::autocast::is_autocast_enabled(at::kCUDA);
+    const auto type = qw.scalar_type();
+    if ((cast && at::autocast::get_autocast_dtype(at::kCUDA) != x.scalar_type()) || (type != x.scalar_type() && !(cast && type == at::kFloat)) || l.D % 8 != 0 ||
+        l.D % groups != 0 || l.D % heads != 0 || (!first && groups != 1) || !prepare_rpb(rpb, heads * win, x))
+        return std::nullopt;
+    auto fits = [&](const Tensor& t, int64_t n) { return plain(t) && t.device() == x.device() && t.scalar_type() == type && t.is_contiguous() && t.numel() == n; };
+    if (!fits(qw, 3 * l.D * (l.D / groups)) || !fits(pw, l.D * (l.D / groups)) || (qb && !fits(*qb, 3 * l.D)) || (pb && !fits(*pb, l.D))) return std::nullopt;
+    const c10::cuda::OptionalCUDAGuard guard(x.device());
+    if (!prepare_valid(vl, l.B, x)) return std::nullopt;
+    if (at::GradMode::is_enabled() && (x.requires_grad() || rpb.requires_grad() || qw.requires_grad() || pw.requires_grad() ||
+                                       (qb && qb->requires_grad()) || (pb && pb->requires_grad())))
+        return NA1dLayer::apply(x, rpb, qw, pw, qb, pb, vl, first, heads, groups, win, left, dil, scale);
+    return layer_forward(x, l, vl ? *vl : Tensor(), rpb32(rpb), qw, qb, pw, pb, Packed(l.B, l.T, l.D, heads, win, left, dil, scale), nullptr);
+}
+
 // int32 (N): clamp(T - padding, 0, T); padding of one element counts for every utterance
 OptTensor valid_tokens(const Tensor& padding, int64_t T, int64_t N) {
     if (!eager_mode() || !plain(padding) || (padding.scalar_type() != at::kInt && padding.scalar_type() != at::kLong) || !padding.is_contiguous() ||
@@ -478,6 +634,7 @@ PYBIND11_MODULE(_na1d_torch, m) {
     m.def("av", &av);
     m.def("packed", &packed);
     m.def("block", &block);
+    m.def("layer", &layer);
     m.def("valid_tokens", &valid_tokens);
     m.def("eager_mode", &eager_mode);
 }

@@ -129,7 +129,7 @@ class PCFNATExtractor(nn.Module):
         if not self.training and padding is not None and x.is_cuda:
             valid = _valid_tokens(x.shape[1], padding, x.shape[0])
         for s, stage in enumerate(self.stages):
-            y = block.run_blocks(stage, x, valid, NAttention) if all(m.attn.training == self.training for m in stage) else None
+            y = block.run_blocks(stage, x, valid) if all(m.attn.training == self.training for m in stage) else None
             if y is None:
                 for blk in stage:
                     x = blk(x, padding)

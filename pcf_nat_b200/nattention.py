@@ -99,6 +99,25 @@ def _packed_row_order(C, num_heads, groups, device):
     return torch.cat([ch, ch + 1, ch + 2])
 
 
+def _native_layer(self, x, channels_first, groups, valid_len):
+    """Projection, attention and projection as one C++ node, or None where a projection is not a plain one."""
+    return ops.native.layer(x, channels_first, self.relative_position_bias, self.qkv.weight, self.qkv.bias, self.proj.weight, self.proj.bias,
+                            self.num_heads, groups, self.win_size, self.left, self.dilation, float(self.scale), valid_len)
+
+
+def _plain_linear(m):
+    return type(m) is nn.Linear and "forward" not in m.__dict__ and not hooked(m)
+
+
+def hooked(m):
+    return bool(m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks)
+
+
+def global_hooks():
+    g = torch.nn.modules.module
+    return bool(g._global_forward_hooks or g._global_forward_pre_hooks or g._global_backward_hooks or g._global_backward_pre_hooks)
+
+
 def _fused_forward_channels_first_packed(self, x, valid_len):
     """The channels-first (PCF) layer on the packed route. The operator's operands need channel-contiguous rows, the network
     around the layer is (batch, C, T): the layout changes once on the C-channel input and once on the output; in between,
@@ -111,6 +130,11 @@ def _fused_forward_channels_first_packed(self, x, valid_len):
     transposes are instead absorbed by batched GEMMs on strided views: 512 small GEMMs and a batch-sized weight gradient)."""
     N, C, T = x.shape
     g = getattr(self, "groups", 1)
+    if type(self.qkv) is nn.Conv1d and type(self.proj) is nn.Conv1d:
+        # the same in one C++ node: own transposes, one launch per weight matrix, bias gradients as column sums
+        y = _native_layer(self, x, True, g, valid_len)
+        if y is not None:
+            return self.proj_drop(y)
     order = _packed_row_order(C, self.num_heads, g, x.device)
     xt = x.transpose(1, 2).contiguous()                            # (N, T, C)
     qkv = F.linear(xt, _dense_1x1(self.qkv, g)[order], None if self.qkv.bias is None else self.qkv.bias[order])
@@ -156,6 +180,12 @@ def _fused_forward(self, x, padding=None):
         if dt in (torch.bfloat16, torch.float16) and ops.packed_supported(self.num_heads, T, hd, self.win_size, self.left,
                                                                          self.dilation, dt):
             return _fused_forward_channels_first_packed(self, x, valid_len)
+    if (layout == "channels_last" and not drop_p and type(x) is torch.Tensor and x.is_cuda and not torch.compiler.is_compiling() and
+            _plain_linear(self.qkv) and _plain_linear(self.proj) and not global_hooks() and
+            ops.packed_supported(self.num_heads, T, hd, self.win_size, self.left, self.dilation, x.dtype)):
+        y = _native_layer(self, x, False, 1, valid_len)
+        if y is not None:
+            return self.proj_drop(y)
     qkv = self.qkv(x)
     if (layout == "channels_last" and not drop_p and type(qkv) is torch.Tensor and qkv.is_cuda and not torch.compiler.is_compiling() and
             ops.packed_supported(self.num_heads, T, hd, self.win_size, self.left, self.dilation, qkv.dtype)):

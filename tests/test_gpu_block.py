@@ -141,7 +141,6 @@ def test_block_node_against_its_modules(dim, heads, T, dtype):
     """Outputs and all gradients of the fused node, of the module-by-module network and of the same network in fp32: the node
     is no further from fp32 than the modules are."""
     from pcf_nat_b200 import block
-    from pcf_nat_b200.nattention import NAttention
     st = _stage(dim, heads, T)
     x0 = _rand(3, T, dim, dtype=dtype, seed=1)
     dy = _rand(3, T, dim, dtype=dtype, seed=2)
@@ -150,7 +149,7 @@ def test_block_node_against_its_modules(dim, heads, T, dtype):
         x = x0.clone().requires_grad_()
         with torch.autocast("cuda", dtype=dtype):
             if kind == "node":
-                y = block.run_blocks(st, x, None, NAttention)
+                y = block.run_blocks(st, x, None)
                 assert y is not None
             else:
                 y = x
@@ -189,12 +188,12 @@ def _reference(st, x0, dy, heads):
 
 def test_block_node_evaluation_with_padding_and_frozen_parameters():
     from pcf_nat_b200 import block
-    from pcf_nat_b200.nattention import NAttention, _valid_tokens
+    from pcf_nat_b200.nattention import _valid_tokens
     st = _stage(128, 4, 60).eval()
     x = _rand(3, 60, 128, dtype=torch.bfloat16, seed=1)
     pad = torch.tensor([0, 13, 60], device="cuda")
     with torch.no_grad(), torch.autocast("cuda", dtype=torch.bfloat16):
-        y = block.run_blocks(st, x, _valid_tokens(60, pad, 3), NAttention)
+        y = block.run_blocks(st, x, _valid_tokens(60, pad, 3))
         z = x
         for b in st:
             z = b(z, pad)
@@ -203,21 +202,20 @@ def test_block_node_evaluation_with_padding_and_frozen_parameters():
     for n, p in st.named_parameters():
         p.requires_grad_("fc1" in n)
     with torch.autocast("cuda", dtype=torch.bfloat16):
-        y = block.run_blocks(st, x, None, NAttention)
+        y = block.run_blocks(st, x, None)
     y.float().sum().backward()
     assert all((p.grad is not None) == ("fc1" in n) for n, p in st.named_parameters())
 
 
 def test_block_node_leaves_other_blocks_to_their_modules():
     from pcf_nat_b200 import block
-    from pcf_nat_b200.nattention import NAttention
     x = _rand(2, 40, 64, dtype=torch.bfloat16, seed=1)
 
     def refused(change, x=x, enabled=True):
         st = _stage(64, 2, 40)
         change(st)
         with torch.autocast("cuda", dtype=torch.bfloat16, enabled=enabled):
-            return block.run_blocks(st, x, None, NAttention) is None
+            return block.run_blocks(st, x, None) is None
 
     assert not refused(lambda st: None)
     assert refused(lambda st: None, enabled=False)
@@ -227,3 +225,77 @@ def test_block_node_leaves_other_blocks_to_their_modules():
     assert refused(lambda st: setattr(st[0].attn.proj_drop, "p", 0.1))
     assert refused(lambda st: setattr(st[0], "norm1", torch.nn.LayerNorm(64, bias=False).cuda()))
     assert refused(lambda st: setattr(st[0], "fc2", torch.nn.Sequential(st[0].fc2)))
+
+
+@pytest.mark.parametrize("dtype", DT)
+@pytest.mark.parametrize("N,C,T", [(1, 8, 1), (2, 64, 64), (3, 72, 65), (2, 256, 150), (2, 136, 97), (1, 64, 2)])
+def test_transpose(N, C, T, dtype):
+    from pcf_nat_b200 import _lib, ops
+    code = _lib.NA1D_BF16 if dtype == torch.bfloat16 else _lib.NA1D_FP16
+    for off in (0, 1):                       # an odd base cannot be read in pairs
+        x = _rand(N * C * T + 1, dtype=dtype, seed=1)[off:off + N * C * T].view(N, C, T)
+        y, z = torch.empty(N, T, C, device="cuda", dtype=dtype), torch.full((N * C * T + 1,), 7.0, device="cuda", dtype=dtype)
+        s = torch.cuda.current_stream().cuda_stream
+        assert ops._L.na1d_transpose(y.data_ptr(), x.data_ptr(), N, C, T, 1, code, s) == 0
+        assert torch.equal(y, x.transpose(1, 2))
+        assert ops._L.na1d_transpose(z[off:].data_ptr(), y.data_ptr(), N, C, T, 0, code, s) == 0
+        assert torch.equal(z[off:off + N * C * T].view(N, C, T), x) and float(z[-1 if off == 0 else 0]) == 7.0
+
+
+@pytest.mark.parametrize("autocast", [True, False])
+@pytest.mark.parametrize("layout,groups,dim,heads,T,bias", [("channels_first", 8, 128, 8, 150, True), ("channels_first", 1, 64, 1, 77, False),
+                                                            ("channels_first", 2, 192, 4, 65, True), ("channels_last", 1, 256, 8, 51, True),
+                                                            ("channels_last", 1, 64, 2, 64, False)])
+def test_layer_node_against_the_layer_in_fp32(layout, groups, dim, heads, T, bias, autocast):
+    """Output and every gradient of the layer in 16 bits against its own parameters and input in 64 bits: four rounding steps of
+    the intermediate tensors, relative to each result."""
+    from oracle import na1d_oracle as orc
+    from pcf_nat_b200 import NAttention, ops
+    torch.manual_seed(5)
+    m = NAttention(T, dim, heads, 9, 1, groups, layout=layout, qkv_bias=bias, proj_bias=bias).cuda()
+    if not autocast:
+        m = m.to(torch.float16)
+    dt = torch.bfloat16 if autocast else torch.float16
+    first = layout == "channels_first"
+    x = _rand(*((2, dim, T) if first else (2, T, dim)), dtype=dt, seed=1).requires_grad_()
+    dy = _rand(*x.shape, dtype=dt, seed=2)
+    with torch.autocast("cuda", dtype=torch.bfloat16, enabled=autocast):
+        y = m(x)
+    # (sizes the packed route does not take run module by module, as before)
+    assert ("NA1dLayer" in y.grad_fn.name()) == ops.packed_supported(heads, T, dim // heads, 9, 4, 1, dt)
+    ps = dict(m.named_parameters())
+    got = [y.detach()] + list(torch.autograd.grad(y, [x] + list(ps.values()), dy))
+    w = {n: p.detach().double().cpu().requires_grad_() for n, p in ps.items()}
+    x64 = x.detach().double().cpu().requires_grad_()
+    C = dim // heads
+    if first:
+        h = F.conv1d(x64, w["qkv.weight"], w.get("qkv.bias"), groups=groups)
+        h = h.view(2, dim // groups, groups, 3, T).transpose(1, 2).reshape(2, heads, C, 3, T).permute(3, 0, 1, 4, 2)
+    else:
+        h = F.linear(x64, w["qkv.weight"], w.get("qkv.bias")).view(2, T, 3, heads, C).permute(2, 0, 3, 1, 4)
+    q, k, v = h.reshape(3, 2 * heads, T, C)
+    o = orc.na1d_fused(q, k, v, 9, 4, 1, C ** -0.5, w["relative_position_bias"].view(heads, 9), None, heads).view(2, heads, T, C)
+    if first:
+        ref = F.conv1d(o.transpose(2, 3).reshape(2, dim, T), w["proj.weight"], w.get("proj.bias"), groups=groups)
+    else:
+        ref = F.linear(o.transpose(1, 2).reshape(2, T, dim), w["proj.weight"], w.get("proj.bias"))
+    want = [ref.detach()] + list(torch.autograd.grad(ref, [x64] + list(w.values()), dy.double().cpu()))
+    for name, a, r in zip(["y", "x"] + list(w), got, want):
+        assert a.shape == r.shape and a.dtype == (dt if name in ("y", "x") or not autocast else torch.float32)
+        assert float((a.double().cpu() - r).norm()) <= 4 * EPS[dt] * float(r.norm()) + 1e-6, name
+
+
+def test_layer_node_leaves_mixed_types_and_hooks_alone():
+    from pcf_nat_b200 import NAttention
+    for layout in ("channels_first", "channels_last"):
+        m = NAttention(64, 64, 2, 7, layout=layout).cuda()
+        x = _rand(2, 64, 64, dtype=torch.bfloat16, seed=1)
+        with pytest.raises(RuntimeError):
+            m(x)                                                        # fp32 weights without autocast
+        with torch.autocast("cuda", dtype=torch.float16):
+            assert m(x).dtype == torch.float16                          # autocast's type wins over the input's
+    seen = []
+    m.qkv.register_forward_hook(lambda *a: seen.append(1))
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        m(x)
+    assert seen == [1]
