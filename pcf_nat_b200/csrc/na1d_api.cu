@@ -35,10 +35,19 @@ int check_geometry(int64_t N, int64_t heads, int64_t T, int64_t C, int64_t win, 
     return NA1D_OK;
 }
 
-// 32-byte rows with a window in the widest band bucket: the band-transposed mode of the tcgen05 backward kernel is bound by
-// the fp32 band's gather there and loses to the CUDA-core kernel (measured at N=8192, T=150, C=16, win=27: 197 us against
-// 121 us); the band-out and band-in modes win everywhere (94 against 174 us, 84 against 107 us) and are not affected.
-bool narrow_rows_wide_window(const na1d::Geometry& g) { return g.C == 16 && (g.win - 1) * g.dil + 1 > 17; }
+// Which kernels run an unfused operator: the tcgen05 ones (tiles of 128 rows, a fixed cost per row), the CUDA-core ones (no fixed
+// cost, C * win operations a row) or the ones on warp-level matrix instructions (band staged in shared memory).
+enum class Unfused { core, tcgen05, warp };
+Unfused pick_unfused(const na1d::Geometry& g, int core_most, bool tc_ok, bool tc_preferred) {
+    const int forced = g_family_override.load();
+    const bool warp_ok = na1d::mma_band_supports(g);
+    if (forced == 0) return Unfused::core;
+    if (forced == 3) return warp_ok ? Unfused::warp : Unfused::core;
+    if (forced == 1 && tc_ok) return Unfused::tcgen05;
+    if (g.C * g.win <= core_most) return Unfused::core;
+    if (tc_ok && tc_preferred) return Unfused::tcgen05;
+    return warp_ok ? Unfused::warp : Unfused::core;
+}
 
 // arguments of the row and column kernels of a transformer block
 int check_block(int64_t rows, int64_t cols, int64_t most_cols, int dtype) {
@@ -85,9 +94,14 @@ int na1d_qk_forward(float* attn, const void* q, const void* k, int64_t N, int64_
     NA1D_REQUIRE_ALIGNED(q); NA1D_REQUIRE_ALIGNED(k);
     na1d::Geometry g;
     if (int s = check_geometry(N, 1, T, C, win, left, dil, dtype, 1.f, g)) return s;
-    if (g_family_override.load() != 0 && na1d::tc_unfused_supports(g) && aligned16(attn))   // the band goes out in 16-byte stores
-        return cuda_status(na1d::tc_qk(attn, q, k, g, dtype, (cudaStream_t)stream));
-    return cuda_status(na1d::simt_qk(attn, q, k, g, dtype, (cudaStream_t)stream));
+    // measured at 4096 x 150 and 512 x 997 rows, us (CUDA core / tcgen05 / warp-level): 16 channels, window 3: 12 / 20 / 32,
+    // window 7: 21 / 20 / 34, window 27: 81 / 31 / 43; 64 channels, window 27: 211 / 35 / 65
+    const bool tc_ok = na1d::tc_unfused_supports(g) && aligned16(attn);   // (its band goes out in 16-byte stores)
+    switch (pick_unfused(g, 80, tc_ok, true)) {
+        case Unfused::tcgen05: return cuda_status(na1d::tc_qk(attn, q, k, g, dtype, (cudaStream_t)stream));
+        case Unfused::warp: return cuda_status(na1d::mma_band_out(attn, q, k, g, dtype, (cudaStream_t)stream));
+        default: return cuda_status(na1d::simt_qk(attn, q, k, g, dtype, (cudaStream_t)stream));
+    }
 }
 int na1d_a_backward(float* attn_gd, const void* result_gd, const void* v, int64_t N, int64_t T, int64_t C, int64_t win,
                     int64_t left, int64_t dil, int dtype, void* stream) {
@@ -99,9 +113,13 @@ int na1d_q_backward(void* q_gd, const float* attn_gd, const void* k, int64_t N, 
     NA1D_REQUIRE_ALIGNED(q_gd); NA1D_REQUIRE_ALIGNED(k);
     na1d::Geometry g;
     if (int s = check_geometry(N, 1, T, C, win, left, dil, dtype, 1.f, g)) return s;
-    if (g_family_override.load() != 0 && na1d::tc_unfused_supports(g))
-        return cuda_status(na1d::tc_band_x(q_gd, attn_gd, k, g, dtype, (cudaStream_t)stream));
-    return cuda_status(na1d::simt_band_x(q_gd, attn_gd, k, g, dtype, (cudaStream_t)stream));
+    // 16 channels, window 7: 19 / 28 / 41, window 17: 37 / 32 / 46; 32 channels, window 3: 21 / 31 / 48, window 7: 36 / 34 / 48;
+    // 64 channels, window 3: 34 / 37 / 68, window 27: 168 / 48 / 87
+    switch (pick_unfused(g, 208, na1d::tc_unfused_supports(g), true)) {
+        case Unfused::tcgen05: return cuda_status(na1d::tc_band_x(q_gd, attn_gd, k, g, dtype, (cudaStream_t)stream));
+        case Unfused::warp: return cuda_status(na1d::mma_band_rows(q_gd, attn_gd, k, false, g, dtype, (cudaStream_t)stream));
+        default: return cuda_status(na1d::simt_band_x(q_gd, attn_gd, k, g, dtype, (cudaStream_t)stream));
+    }
 }
 int na1d_av_forward(void* result, const float* attn, const void* v, int64_t N, int64_t T, int64_t C, int64_t win,
                     int64_t left, int64_t dil, int dtype, void* stream) {
@@ -113,9 +131,15 @@ int na1d_k_backward(void* k_gd, const float* attn_gd, const void* q, int64_t N, 
     NA1D_REQUIRE_ALIGNED(k_gd); NA1D_REQUIRE_ALIGNED(q);
     na1d::Geometry g;
     if (int s = check_geometry(N, 1, T, C, win, left, dil, dtype, 1.f, g)) return s;
-    if (g_family_override.load() != 0 && na1d::tc_unfused_t_supports(g) && (!narrow_rows_wide_window(g) || g_family_override.load() == 1))
-        return cuda_status(na1d::tc_bandT_x(k_gd, attn_gd, q, g, dtype, (cudaStream_t)stream));
-    return cuda_status(na1d::simt_bandT_x(k_gd, attn_gd, q, g, dtype, (cudaStream_t)stream));
+    // the tcgen05 form gathers the fp32 band along its diagonals and pays off at 64 channels and narrow windows only:
+    // 16 channels, window 17: 41 / 47 / 50, window 33: 80 / 100 / 66; 32 channels, window 9: 46 / 52 / 50, window 27: 117 / 99 / 73;
+    // 64 channels, window 3: 35 / 42 / 69, window 9: 76 / 54 / 70, window 17 (997 rows): 125 / 76 / 60, window 27: 188 / - / 97
+    const int weff = (g.win - 1) * g.dil + 1;
+    switch (pick_unfused(g, 288, na1d::tc_unfused_t_supports(g), g.C == 64 && weff <= 9)) {
+        case Unfused::tcgen05: return cuda_status(na1d::tc_bandT_x(k_gd, attn_gd, q, g, dtype, (cudaStream_t)stream));
+        case Unfused::warp: return cuda_status(na1d::mma_band_rows(k_gd, attn_gd, q, true, g, dtype, (cudaStream_t)stream));
+        default: return cuda_status(na1d::simt_bandT_x(k_gd, attn_gd, q, g, dtype, (cudaStream_t)stream));
+    }
 }
 int na1d_v_backward(void* v_gd, const float* attn, const void* result_gd, int64_t N, int64_t T, int64_t C, int64_t win,
                     int64_t left, int64_t dil, int dtype, void* stream) {

@@ -24,6 +24,9 @@ cudaError_t mma_fused_fwd(void* o, float* lse, const void* q, const void* k, con
 cudaError_t mma_fused_bwd(void* dq, void* dk, void* dv, float* d_rpb, const void* d_o, const void* q, const void* k, const void* v,
                           const void* o, const float* lse, const float* rpb, const int* valid_len, const Geometry& gm, int dtype,
                           cudaStream_t st);
+bool mma_band_supports(const Geometry& gm);
+cudaError_t mma_band_out(float* band, const void* a, const void* b, const Geometry& gm, int dtype, cudaStream_t st);
+cudaError_t mma_band_rows(void* out, const float* band, const void* x, bool transposed, const Geometry& gm, int dtype, cudaStream_t st);
 
 // ---- tcgen05 / TMA family (na1d_tc_fwd.cu)
 bool tc_fwd_supports(const Geometry& gm);  // shape limits of the tcgen05 forward

@@ -117,6 +117,8 @@ __host__ __device__ inline int chunks_of(int win) { return (win + 30) / 16; }   
 __host__ __device__ inline int staged_rows(int win) { return 16 * (kWarps - 1 + chunks_of(win)); }
 __host__ __device__ inline int table_floats(int win) { return 16 * (chunks_of(win) + 1); }
 __host__ __device__ inline int band_pitch(int win) { return win | 1; }
+// rows that the warps with rows of the residue meet: a short last tile stages no more than it needs (`most` = the full tile's)
+__device__ __forceinline__ int needed_rows(const Tile& t, int nch, int most) { return min(most, 16 * ((t.Tr - t.u0 + 15) / 16 - 1 + nch)); }
 size_t smem_bytes(int CP, int win, bool backward, bool d_rpb) {
     const int rows = staged_rows(win);
     size_t b = (size_t)2 * rows * pitch_bytes(CP) + (size_t)table_floats(win) * 4;
@@ -328,7 +330,7 @@ __global__ void __launch_bounds__(kThreads) mma_fwd_kernel(E* __restrict__ o, fl
     const int u = t.u0 + warp * 16;
     uint32_t qa[CP / 16][4];
     own_rows<E, CP>(qa, q, t, gm, u, lane);   // (in flight together with the staged rows)
-    if (stage_rows<E, CP>(sx, sy, k, v, t, gm, t.u0 - gm.left, rows)) {
+    if (stage_rows<E, CP>(sx, sy, k, v, t, gm, t.u0 - gm.left, needed_rows(t, nch, rows))) {
         plain_fwd_rows<E>(o, lse, q, k, v, rpb, t, gm);
         return;
     }
@@ -437,7 +439,7 @@ __device__ __forceinline__ void bwd_view(uint8_t* smem, E* __restrict__ out1, E*
             if (i < rows && c == 0) { s_delta[i] = d; s_lse[i] = in ? __ldg(lse + t.row(gm, w)) * kLog2e : INFINITY; }
         }
     }
-    if (stage_rows<E, CP>(sx, sy, gx, gy, t, gm, t.u0 - before, rows)) {
+    if (stage_rows<E, CP>(sx, sy, gx, gy, t, gm, t.u0 - before, needed_rows(t, nch, rows))) {
         plain_bwd_rows<E, KEY>(out1, out2, d_rpb, ga1, ga2, gx, gy, o, lse, rpb, t, gm);
         return;
     }
@@ -543,6 +545,174 @@ __global__ void __launch_bounds__(kThreads) mma_bwd_kernel(E* __restrict__ dq, E
     else bwd_view<E, CP, false>(smem, dq, nullptr, d_rpb, q, d_o, k, v, o, lse, rpb, t, gm);
 }
 
+// ---------------------------------------------------------------- the unfused pair
+// The same products with the fp32 band in memory: 128 rows per CTA (the band's halo is staged too: 8 warps keep it at
+// (win - 1) / 128). The band goes through shared memory both ways, so that global memory sees whole contiguous rows.
+//   band_out: band[t, kk] = a[t] . b[j]          (QK forward, dA)
+//   band_rows<false>: out[t] = sum band[t, kk] x[j]     (AV forward, dQ)
+//   band_rows<true> : out[j] = sum band[t, kk] x[t]     (dV, dK)
+constexpr int kBandWarps = 8, kBandThreads = kBandWarps * 32, kBandRows = kBandWarps * 16;
+__host__ __device__ inline int band_staged(int win) { return 16 * (kBandWarps - 1 + chunks_of(win)); }
+
+__device__ __forceinline__ bool band_tile(Tile& t, const Geometry& gm, int tps) {
+    const int s = (int)blockIdx.x / tps;
+    t.u0 = ((int)blockIdx.x - s * tps) * kBandRows;
+    t.n = s / gm.dil;
+    t.r = s - t.n * gm.dil;
+    t.Tr = gm.T > t.r ? (gm.T - t.r + gm.dil - 1) / gm.dil : 0;
+    t.vl = t.Tr;
+    t.h = 0;
+    return t.u0 < t.Tr;
+}
+// rows [first, first + rows) of one tensor; whether a value is infinite or NaN
+template <typename E, int CP>
+__device__ __forceinline__ bool band_stage_rows(uint8_t* x, const E* __restrict__ g, const Tile& t, const Geometry& gm, int first, int rows) {
+    constexpr int CH = CP / 8, U = CP <= 32 ? 2 : 4;
+    bool bad = false;
+    for (int i0 = threadIdx.x; i0 < rows * CH; i0 += U * kBandThreads) {
+        uint4 a[U];
+#pragma unroll
+        for (int k = 0; k < U; ++k) {
+            const int i = i0 + k * kBandThreads, row = i / CH, c = i - row * CH, u = first + row;
+            a[k] = make_uint4(0, 0, 0, 0);
+            if (row < rows && u >= 0 && u < t.Tr && c * 8 < gm.C) a[k] = __ldg(reinterpret_cast<const uint4*>(g + t.row(gm, u) * gm.C + c * 8));
+        }
+#pragma unroll
+        for (int k = 0; k < U; ++k) {
+            const int i = i0 + k * kBandThreads, row = i / CH, c = i - row * CH;
+            if (row >= rows) break;
+            *reinterpret_cast<uint4*>(x + row * pitch_bytes(CP) + c * 16) = a[k];
+            constexpr uint32_t m = std::is_same<E, __half>::value ? 0x7c00u : 0x7f80u;
+            const uint32_t w[4] = {a[k].x, a[k].y, a[k].z, a[k].w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) bad |= (w[e] & m) == m || (w[e] & (m << 16)) == m << 16;
+        }
+    }
+    return bad;
+}
+// band rows [first, first + rows) into s (win floats each, zeros outside the residue); thread `id` of `n` takes part
+__device__ __forceinline__ bool band_load(float* s, const float* __restrict__ band, const Tile& t, const Geometry& gm, int first, int rows, int id, int n) {
+    const int lo = max(0, -first), hi = min(rows, t.Tr - first), total = rows * gm.win;
+    bool bad = false;
+    auto put = [&](int i, float v) {
+        s[i] = v;
+        bad |= (__float_as_uint(v) & 0x7f800000u) == 0x7f800000u;
+    };
+    if (gm.dil == 1) {   // the rows are one contiguous piece
+        const float* src = band + ((long long)t.n * gm.T + first) * gm.win;
+        const int a = lo * gm.win, b = hi * gm.win;
+        constexpr int U = 8;
+        for (int i0 = id; i0 < total; i0 += U * n) {
+            float v[U];
+#pragma unroll
+            for (int k = 0; k < U; ++k) { const int i = i0 + k * n; v[k] = i >= a && i < b ? __ldg(src + i) : 0.f; }
+#pragma unroll
+            for (int k = 0; k < U; ++k) if (i0 + k * n < total) put(i0 + k * n, v[k]);
+        }
+    } else {
+        for (int i = id; i < total; i += n) {
+            const int row = i / gm.win;
+            put(i, row >= lo && row < hi ? __ldg(band + t.row(gm, first + row) * gm.win + (i - row * gm.win)) : 0.f);
+        }
+    }
+    return bad;
+}
+
+template <typename E, int CP>
+__global__ void __launch_bounds__(kBandThreads) mma_band_out_kernel(float* __restrict__ band, const E* __restrict__ a, const E* __restrict__ b, Geometry gm, int tps) {
+    extern __shared__ __align__(16) uint8_t smem[];
+    Tile t;
+    if (!band_tile(t, gm, tps)) return;
+    const int rows = band_staged(gm.win), nch = chunks_of(gm.win), lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int u = t.u0 + warp * 16, fr = lane >> 2, fc = 2 * (lane & 3);
+    float* out = reinterpret_cast<float*>(smem + rows * pitch_bytes(CP)) + warp * 16 * gm.win;
+    uint32_t own[CP / 16][4];
+    own_rows<E, CP>(own, a, t, gm, u, lane);
+    band_stage_rows<E, CP>(smem, b, t, gm, t.u0 - gm.left, needed_rows(t, nch, rows));
+    __syncthreads();
+    if (u >= t.Tr) return;
+    const uint32_t base = ptx::smem_u32(smem) + (warp * 16 + (lane & 7) + ((lane >> 4) << 3)) * pitch_bytes(CP) + ((lane >> 3) & 1) * 16;
+    for (int ch = 0; ch < nch; ++ch) {
+        float s[2][4];
+        products<E, CP>(s, own, base + ch * 16 * pitch_bytes(CP));
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int row = fr + 8 * (i >> 1), kk = ch * 16 + nt * 8 + fc + (i & 1) - row, j = u - gm.left + row + kk;
+                // (a neighbour outside the sequence is a zero row: 0 also where the query is infinite)
+                if ((unsigned)kk < (unsigned)gm.win) out[row * gm.win + kk] = (unsigned)j < (unsigned)t.Tr ? s[nt][i] : 0.f;
+            }
+    }
+    __syncwarp();
+    const int live = min(16, t.Tr - u) * gm.win;
+    if (gm.dil == 1) {
+        float* dst = band + t.row(gm, u) * gm.win;
+        for (int i = lane; i < live; i += 32) dst[i] = out[i];
+    } else {
+        for (int i = lane; i < live; i += 32) {
+            const int row = i / gm.win;
+            band[t.row(gm, u + row) * gm.win + (i - row * gm.win)] = out[i];
+        }
+    }
+}
+
+template <typename E, int CP, bool TRANSPOSED>
+__global__ void __launch_bounds__(kBandThreads) mma_band_rows_kernel(E* __restrict__ out, const float* __restrict__ band, const E* __restrict__ x, Geometry gm, int tps) {
+    extern __shared__ __align__(16) uint8_t smem[];
+    Tile t;
+    if (!band_tile(t, gm, tps)) return;
+    const int rows = band_staged(gm.win), nch = chunks_of(gm.win), lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int u = t.u0 + warp * 16, fr = lane >> 2, fc = 2 * (lane & 3), before = TRANSPOSED ? gm.win - 1 - gm.left : gm.left;
+    float* sb = reinterpret_cast<float*>(smem + rows * pitch_bytes(CP));
+    bool bad;
+    const int need = needed_rows(t, nch, rows);
+    if (TRANSPOSED) bad = band_load(sb, band, t, gm, t.u0 - before, need, threadIdx.x, kBandThreads);
+    else bad = band_load(sb, band, t, gm, t.u0, min(kBandRows, (t.Tr - t.u0 + 15) / 16 * 16), threadIdx.x, kBandThreads);
+    bad |= band_stage_rows<E, CP>(smem, x, t, gm, t.u0 - before, need);
+    if (__syncthreads_or(bad)) {
+        // plain fp32 rows: an exact zero times an infinite or NaN row would not stay zero
+        for (int v = t.u0 + warp; v < min(t.u0 + kBandRows, t.Tr); v += kBandWarps) {
+            float acc[4] = {0.f, 0.f, 0.f, 0.f}, f[4];
+            for (int kk = 0; kk < gm.win; ++kk) {
+                const int w = TRANSPOSED ? v - (kk - gm.left) : v + kk - gm.left;
+                if (w < 0 || w >= t.Tr) continue;
+                const float b = __ldg(band + t.row(gm, TRANSPOSED ? w : v) * gm.win + kk);
+                lane4(f, x, t.row(gm, w), gm.C, lane);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) acc[i] = fmaf(b, f[i], acc[i]);
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (lane * 4 + i < gm.C) out[t.row(gm, v) * gm.C + lane * 4 + i] = (E)acc[i];
+        }
+        return;
+    }
+    if (u >= t.Tr) return;
+    const uint32_t base = ptx::smem_u32(smem) + (warp * 16 + (lane & 7) + (((lane >> 3) & 1) << 3)) * pitch_bytes(CP) + (lane >> 4) * 16;
+    const float* wb = sb + warp * 16 * gm.win;
+    float acc[CP / 8][4];
+#pragma unroll
+    for (int i = 0; i < CP / 8; ++i)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[i][e] = 0.f;
+    for (int ch = 0; ch < nch; ++ch) {
+        float s[2][4];
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int row = fr + 8 * (i >> 1), c = ch * 16 + nt * 8 + fc + (i & 1), d = c - row;
+                const int at = TRANSPOSED ? c * gm.win + gm.win - 1 - d : row * gm.win + d;
+                s[nt][i] = (unsigned)d < (unsigned)gm.win ? wb[at] : 0.f;
+            }
+        Weights<E> w;
+        w.set(s);
+        accumulate<E, CP>(acc, w, base + ch * 16 * pitch_bytes(CP));
+    }
+    store_rows<E, CP>(out, acc, t, gm, u, lane, 1.f, 1.f);
+}
+
 int padded_channels(int C) { return C <= 64 ? (C + 15) / 16 * 16 : C <= 96 ? 96 : 128; }
 
 #define NA1D_MMA_DISPATCH(dtype, C, ...)                                                     \
@@ -587,6 +757,34 @@ cudaError_t mma_fused_bwd(void* dq, void* dk, void* dv, float* d_rpb, const void
         if (cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) return e;
         kern<<<grid, kThreads, smem, st>>>((E*)dq, (E*)dk, (E*)dv, d_rpb, (const E*)d_o, (const E*)q, (const E*)k, (const E*)v, (const E*)o, lse,
                                            rpb, valid_len, gm, tps);
+    })
+    return cudaGetLastError();
+}
+
+// 128 rows per CTA and per residue class of a sequence
+bool mma_band_supports(const Geometry& gm) {
+    const long long tps = (((long long)gm.T + gm.dil - 1) / gm.dil + kBandRows - 1) / kBandRows;
+    return gm.C <= 128 && gm.win <= 128 && (long long)gm.N * gm.dil * tps < (1ll << 31);
+}
+cudaError_t mma_band_out(float* band, const void* a, const void* b, const Geometry& gm, int dtype, cudaStream_t st) {
+    const int tps = ((gm.T + gm.dil - 1) / gm.dil + kBandRows - 1) / kBandRows;
+    const unsigned grid = (unsigned)((long long)gm.N * gm.dil * tps);
+    NA1D_MMA_DISPATCH(dtype, gm.C, {
+        auto kern = mma_band_out_kernel<E, CP>;
+        const size_t smem = (size_t)band_staged(gm.win) * pitch_bytes(CP) + (size_t)kBandRows * gm.win * 4;
+        if (cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) return e;
+        kern<<<grid, kBandThreads, smem, st>>>(band, (const E*)a, (const E*)b, gm, tps);
+    })
+    return cudaGetLastError();
+}
+cudaError_t mma_band_rows(void* out, const float* band, const void* x, bool transposed, const Geometry& gm, int dtype, cudaStream_t st) {
+    const int tps = ((gm.T + gm.dil - 1) / gm.dil + kBandRows - 1) / kBandRows;
+    const unsigned grid = (unsigned)((long long)gm.N * gm.dil * tps);
+    NA1D_MMA_DISPATCH(dtype, gm.C, {
+        auto kern = transposed ? mma_band_rows_kernel<E, CP, true> : mma_band_rows_kernel<E, CP, false>;
+        const size_t smem = (size_t)band_staged(gm.win) * pitch_bytes(CP) + (size_t)(transposed ? band_staged(gm.win) : kBandRows) * gm.win * 4;
+        if (cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) return e;
+        kern<<<grid, kBandThreads, smem, st>>>((E*)out, band, (const E*)x, gm, tps);
     })
     return cudaGetLastError();
 }

@@ -117,3 +117,60 @@ def test_routes():
     args = _inputs(case, torch.bfloat16)
     for a, b in zip(_run(ops.FAMILY_WARP_MMA, case, *args)[:4], _run(ops.FAMILY_CUDA_CORE, case, *args)[:4]):
         assert torch.equal(a, b)
+
+
+def _pair_reference(q, k, attn, win, left, dil):
+    """(q.k over the window, attn . k, transposed attn . q) in 64 bits; rows outside the sequence are zero rows."""
+    N, T, C = q.shape
+    j = torch.arange(T, device="cuda")[:, None] + (torch.arange(win, device="cuda") - left) * dil
+    inr = ((j >= 0) & (j < T)).double()
+    jc = j.clamp(0, T - 1)
+    kg = k.double()[:, jc] * inr[None, :, :, None]
+    a = attn.double() * inr
+    out = torch.zeros(N, T, C, device="cuda", dtype=torch.float64)
+    out.index_add_(1, jc.reshape(-1), (a[..., None] * q.double()[:, :, None]).reshape(N, T * win, C))
+    return torch.einsum("ntc,ntwc->ntw", q.double(), kg), torch.einsum("ntw,ntwc->ntc", a, kg), out
+
+
+@pytest.mark.parametrize("family", [-1, 0, 3])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("N,T,C,win,left,dil", [(1, 1, 8, 1, 0, 1), (3, 128, 16, 27, 13, 1), (2, 129, 16, 5, 0, 1), (2, 150, 32, 33, 32, 1), (3, 97, 48, 41, 20, 1),
+                                                (2, 300, 64, 9, 4, 1), (2, 300, 64, 18, 4, 3), (1, 260, 128, 128, 64, 1), (2, 7, 24, 9, 4, 5),
+                                                (2, 40, 192, 12, 3, 1)])
+def test_unfused_operators(N, T, C, win, left, dil, dtype, family):
+    """All routes of the six unfused entry points: fp32 results to fp32 accuracy (the band in), 16-bit results to their rounding --
+    half a step, plus the tcgen05 kernels' 16-bit band, at most another half step per term."""
+    from pcf_nat_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(4)
+    q, k = (torch.randn(N, T, C, device="cuda", generator=g).to(dtype) for _ in range(2))
+    attn = torch.randn(N, T, win, device="cuda", generator=g)
+    old = ops.set_kernel_family(family)
+    try:
+        got = ops.qk_forward(q, k, win, left, dil), ops.av_forward(attn, k, win, left, dil), ops.v_backward(attn, q, win, left, dil)
+    finally:
+        ops.set_kernel_family(old)
+    eps = 2.0 ** -9 if dtype == torch.bfloat16 else 2.0 ** -12      # half a rounding step
+    for i, (a, r) in enumerate(zip(got, _pair_reference(q, k, attn, win, left, dil))):
+        rel = 2e-6 if i == 0 else eps * (1.1 if family >= 0 else 1.6)
+        assert float((a.double() - r).norm()) <= rel * float(r.norm()) + 1e-6, i
+
+
+@pytest.mark.parametrize("value", [float("nan"), float("inf")])
+def test_unfused_operators_keep_bad_values_in_their_window(value):
+    from pcf_nat_b200 import ops
+    q, k, d_o, _, _, _ = _inputs((1, 1, 150, 48, 9, 4, 1, True, False), torch.bfloat16)
+    attn = torch.rand(1, 150, 9, device="cuda")
+    for bad in (q, k, attn):
+        x = [q.clone(), k.clone(), attn.clone()]
+        x[[id(q), id(k), id(attn)].index(id(bad))][0, 70, 5] = value
+        out = []
+        for family in (3, 0):
+            old = ops.set_kernel_family(family)
+            try:
+                out.append([ops.qk_forward(x[0], x[1], 9, 4), ops.av_forward(x[2], x[1], 9, 4), ops.v_backward(x[2], x[0], 9, 4)])
+            finally:
+                ops.set_kernel_family(old)
+        for a, b in zip(*out):
+            assert torch.equal(torch.isfinite(a), torch.isfinite(b)) and torch.equal(torch.isnan(a), torch.isnan(b))
+            ok = torch.isfinite(b)
+            assert torch.allclose(a[ok].float(), b[ok].float(), rtol=1e-2, atol=1e-2)
