@@ -4,6 +4,7 @@
 
 #include <atomic>
 #include <climits>
+#include <cmath>
 #include <mutex>
 
 namespace {
@@ -42,7 +43,7 @@ Unfused pick_unfused(const na1d::Geometry& g, int core_most, bool tc_ok, bool tc
     const int forced = g_family_override.load();
     const bool warp_ok = na1d::mma_band_supports(g);
     if (forced == 0) return Unfused::core;
-    if (forced == 3) return warp_ok ? Unfused::warp : Unfused::core;
+    if (forced >= 3) return warp_ok ? Unfused::warp : Unfused::core;
     if (forced == 1 && tc_ok) return Unfused::tcgen05;
     if (g.C * g.win <= core_most) return Unfused::core;
     if (tc_ok && tc_preferred) return Unfused::tcgen05;
@@ -63,6 +64,32 @@ template <typename... P> int check_pointers(const P*... p) {
 #define NA1D_REQUIRE_PTR(p) do { if ((p) == nullptr) return NA1D_ERR_NULL_POINTER; } while (0)
 #define NA1D_REQUIRE_ALIGNED(p) do { if (!aligned16(p)) return NA1D_ERR_MISALIGNED; } while (0)
 
+// Of the general kernels (na1d_mma.cu, na1d_simt.cu) the warp-level matrix ones pay for a CTA per 64 rows of a residue whatever
+// the window, the CUDA-core ones for every neighbour of a row: few neighbours or short residues go to the latter. Picosecond
+// models of both, fitted to 8 to 128 channels, windows 3 to 40, residues of 5 to 300 rows (CUDA core / matrix, us, forward and
+// backward): 256 x 300 rows of 48 channels, window 3: 8 / 11, 50 / 32; window 9: 17 / 11, 106 / 33; 128 channels, window 3:
+// 18 / 26, 68 / 129; window 15: 63 / 26, 197 / 130; 2048 x 20 rows of 48 channels with dilation 4, window 15: 11 / 30, 66 / 112.
+bool use_mma(const na1d::Geometry& g, bool backward) {
+    const int forced = g_family_override.load();
+    if (forced == 0 || !na1d::mma_supports(g)) return false;
+    if (forced >= 3) return true;
+    const double C = g.C, tp = (g.T + g.dil - 1) / g.dil, rows = (double)g.N * g.T, residues = (double)g.N * (g.dil < g.T ? g.dil : g.T);
+    const double in = g.win < tp ? g.win : tp, w = in + 0.7 * (g.win - in);          // neighbours outside the sequence cost less
+    const double blocks = std::ceil(tp / 16), tiles = std::ceil(tp / 64), chunks = ((g.win + 30) / 16) / 2.0;
+    const double core = rows * (backward ? 150 + 3 * C + w * (35 + 1.1 * C) : 20 + 0.5 * C + w * (4.5 + C / 3));
+    const double slope = chunks * (!backward ? 300 + 20 * C : C <= 64 ? 1000 + 47 * C : 170 * C);
+    const double mma = (backward ? 5e6 : 3.5e6) + residues * (tiles * (backward ? 4000 + 110 * C : 1500 + 18 * C) + blocks * slope);
+    return mma < core;
+}
+
+// The marching kernels: automatic for every shape they take (16-channel rows, windows up to 33), and what stands for the
+// segmented tiling there (both work on residue classes through arbitrary strides). Forced family 4 is the same without that
+// tiling's own limits.
+template <typename... S> bool use_march(const na1d::Geometry& g, const S&... strides) {
+    const int forced = g_family_override.load();
+    if (forced != -1 && forced != 4 && !(forced == 2 && na1d::tc_seg_supports(g))) return false;
+    return na1d::march_supports(g) && ((strides.token * g.dil < (1ll << 30)) && ...);
+}
 }  // namespace
 
 extern "C" {
@@ -154,7 +181,7 @@ static int pick_family(const na1d::Geometry& g, int backward, bool has_bias = fa
     const int forced = g_family_override.load();
     const bool flat_ok = backward ? na1d::tc_bwd_supports(g, has_bias, wants_bias_grad) : na1d::tc_fwd_supports(g);
     const bool seg_ok = backward ? na1d::tc_bwd_seg_supports(g, has_bias, wants_bias_grad) : na1d::tc_seg_supports(g);
-    if (forced == 0 || forced == 3) return 0;
+    if (forced == 0 || forced >= 3) return 0;
     if (forced == 2) return seg_ok ? 2 : NA1D_ERR_UNSUPPORTED;
     if (forced == 1 && flat_ok) return 1;   // forced: the flat tiling wherever it can run (the choice below is for the automatic mode)
     int pick = 0;
@@ -194,7 +221,7 @@ int na1d_fused_kernel_tiling(int64_t N, int64_t T, int64_t C, int64_t win, int64
 }
 
 int na1d_set_kernel_family(int family) {
-    if (family < -1 || family > 3) family = -1;
+    if (family < -1 || family > 4) family = -1;
     return g_family_override.exchange(family);
 }
 
@@ -228,6 +255,10 @@ int na1d_fused_forward(void* o, float* lse, const void* q, const void* k, const 
     NA1D_REQUIRE_ALIGNED(o); NA1D_REQUIRE_ALIGNED(q); NA1D_REQUIRE_ALIGNED(k); NA1D_REQUIRE_ALIGNED(v);
     na1d::Geometry g;
     if (int s = check_geometry(N, heads, T, C, win, left, dil, dtype, scale, g)) return s;
+    if (use_march(g, na1d::dense_strides(g.H, g.T, g.C))) {
+        const na1d::Strides d = na1d::dense_strides(g.H, g.T, g.C);
+        return cuda_status(na1d::march_fused_fwd(o, lse, q, k, v, rpb, valid_len, d, d, d, d, g, dtype, (cudaStream_t)stream));
+    }
     const int fam = pick_family(g, 0);
     if (fam < 0) return fam;
     if (fam == 1) return cuda_status(na1d::tc_fused_fwd(o, lse, q, k, v, rpb, valid_len, g, dtype, (cudaStream_t)stream));
@@ -235,7 +266,7 @@ int na1d_fused_forward(void* o, float* lse, const void* q, const void* k, const 
         const na1d::Strides d = na1d::dense_strides(g.H, g.T, g.C);
         return cuda_status(na1d::tc_fused_fwd_seg(o, lse, q, k, v, rpb, valid_len, d, d, d, d, g, dtype, (cudaStream_t)stream));
     }
-    if (g_family_override.load() != 0 && na1d::mma_supports(g))
+    if (use_mma(g, false))
         return cuda_status(na1d::mma_fused_fwd(o, lse, q, k, v, rpb, valid_len, g, dtype, (cudaStream_t)stream));
     return cuda_status(na1d::simt_fused_fwd(o, lse, q, k, v, rpb, valid_len, g, dtype, (cudaStream_t)stream));
 }
@@ -277,6 +308,7 @@ int na1d_fused_forward_strided(void* o, float* lse, const void* q, const void* k
     if (int s = read_strides(k_strides, batch, heads, T, C, sk)) return s;
     if (int s = read_strides(v_strides, batch, heads, T, C, sv)) return s;
     if (!na1d::tc_seg_supports(g)) return NA1D_ERR_UNSUPPORTED;
+    if (use_march(g, sq, sk, sv, so)) return cuda_status(na1d::march_fused_fwd(o, lse, q, k, v, rpb, valid_len, sq, sk, sv, so, g, dtype, (cudaStream_t)stream));
     return cuda_status(na1d::tc_fused_fwd_seg(o, lse, q, k, v, rpb, valid_len, sq, sk, sv, so, g, dtype, (cudaStream_t)stream));
 }
 
@@ -300,6 +332,9 @@ int na1d_fused_backward_strided(void* dq, void* dk, void* dv, float* d_rpb, cons
     for (int i = 0; i < 7; ++i)
         if (int s = read_strides(in[i], batch, heads, T, C, s7[i])) return s;
     if (!na1d::tc_bwd_seg_supports(g, rpb != nullptr, d_rpb != nullptr)) return NA1D_ERR_UNSUPPORTED;
+    if (use_march(g, s7[0], s7[1], s7[2], s7[3], s7[4], s7[5], s7[6]))
+        return cuda_status(na1d::march_fused_bwd(dq, dk, dv, d_rpb, d_o, q, k, v, lse, rpb, valid_len, s7[0], s7[1], s7[2], s7[3], s7[4], s7[5],
+                                                 s7[6], g, dtype, (cudaStream_t)stream));
     return cuda_status(na1d::tc_fused_bwd_seg(dq, dk, dv, d_rpb, d_o, q, k, v, lse, rpb, valid_len, scratch, (size_t)scratch_floats,
                                               s7[0], s7[1], s7[2], s7[3], s7[4], s7[5], s7[6], g, dtype, (cudaStream_t)stream));
 }
@@ -316,6 +351,10 @@ int na1d_fused_backward(void* dq, void* dk, void* dv, float* d_rpb, const void* 
     if (int s = check_geometry(N, heads, T, C, win, left, dil, dtype, scale, g)) return s;
     if (d_rpb && heads * win * 4 > 48 * 1024) return NA1D_ERR_TOO_LARGE;
     cudaStream_t st = (cudaStream_t)stream;
+    if (use_march(g, na1d::dense_strides(g.H, g.T, g.C))) {
+        const na1d::Strides d = na1d::dense_strides(g.H, g.T, g.C);
+        return cuda_status(na1d::march_fused_bwd(dq, dk, dv, d_rpb, d_o, q, k, v, lse, rpb, valid_len, d, d, d, d, d, d, d, g, dtype, st));
+    }
     const int fam = pick_family(g, 1, rpb != nullptr, d_rpb != nullptr);
     if (fam < 0) return fam;
     if (fam == 1)  // delta is recomputed inside the kernel from P and dP: o is not read; delta_ws (N*T floats) only holds the
@@ -327,7 +366,7 @@ int na1d_fused_backward(void* dq, void* dk, void* dv, float* d_rpb, const void* 
         return cuda_status(na1d::tc_fused_bwd_seg(dq, dk, dv, d_rpb, d_o, q, k, v, lse, rpb, valid_len, delta_ws,
                                                   (size_t)g.N * (size_t)g.T, d, d, d, d, d, d, d, g, dtype, st));
     }
-    if (g_family_override.load() != 0 && na1d::mma_supports(g))
+    if (use_mma(g, true))
         return cuda_status(na1d::mma_fused_bwd(dq, dk, dv, d_rpb, d_o, q, k, v, o, lse, rpb, valid_len, g, dtype, st));
     if (int s = cuda_status(na1d::simt_delta(delta_ws, d_o, o, g.N * g.T, g.C, dtype, st))) return s;
     return cuda_status(na1d::simt_fused_bwd(dq, dk, dv, d_rpb, d_o, q, k, v, lse, delta_ws, rpb, valid_len, g, dtype, st));

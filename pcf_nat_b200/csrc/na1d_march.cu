@@ -1,0 +1,486 @@
+// Fused NA1D for narrow rows: warps that march along a sequence with everything in registers.
+//
+// At 16 channels a row is one 32-byte sector and the operator should be bound by HBM (512 x 16 x 150 rows: 24 us forward, 43 us
+// backward), but a 128-row tcgen05 tile spends most of its time in the chain TMA -> S -> softmax -> P.V -> epilogue with few
+// MMAs in it, and its compute warps execute 577 instructions per 16 rows in table lookups, tensor-memory transfers, barriers
+// and row bookkeeping, at 0.56 instructions a cycle (76 us forward, 141 us backward; segmented tiling 135 and 193).
+//
+// Here a warp owns a strip of 16-row blocks of one residue class of a sequence (tokens t = r mod dil, on which a dilated window
+// is a plain one) and walks it. The window of block b is the NT = ceil((win + 15) / 16) key tiles b .. b + NT - 1, tile i being
+// keys 16 i - left .. + 15, so each step brings one new tile and drops one. Keys, values (and in the backward their
+// gradients) stay in registers as operands of m16n8k16 products while the window covers them; nothing passes through shared
+// memory and there is no barrier:
+//   * a row's channels are loaded and stored as 8 bytes per lane, in an order of the contraction index that makes lane l % 4 hold
+//     channels 4 (l % 4) .. + 3 of row l / 4, both as left and as right operand;
+//   * operands that contract over rows are the transposes of the same registers (movmatrix);
+//   * the window offset of an accumulator element is a constant of the thread: the bias (-inf outside the window) and the bias
+//     gradient are 2 (2 NT + 1) registers;
+//   * keys and values outside the sequence are zero registers: only the additive mask needs a test, and only in the blocks at a
+//     sequence's ends or at its padding.
+// Backward: key tile i collects from blocks i - NT + 1 .. i and is stored when block i is done. A strip owns the key tiles of its
+// own blocks and recomputes the NT - 1 blocks before it (nothing to recompute when the strip is a whole sequence).
+// Measured at 512 x 16 x 150 rows (tcgen05 flat / segmented tiling / here, us): window 27 forward 76 / 135 / 51, backward
+// 141 / 194 / 136; window 9 forward 62 / 104 / 40, backward 99 / 154 / 94; 64 x 16 x 997 rows, window 27: 66 / 66 / 41 and
+// 115 / 119 / 97. The forward is bound by instruction issue (0.67 a cycle), the backward by latency at the eight warps an SM
+// that its 225 registers leave (three CTAs an SM at 168 registers spill and are slower: 139).
+// Rounding is that of the tcgen05 kernels: probabilities and dS enter the second products in 16 bits, sums are fp32.
+#include "na1d_internal.h"
+#include "na1d_tc_common.cuh"
+#include <type_traits>
+
+namespace na1d {
+namespace {
+
+constexpr int kWarps = 4;
+
+__device__ __forceinline__ uint32_t transpose8(uint32_t x) {   // 8x8 16-bit matrix: row l / 4, columns 2 (l % 4), + 1
+    uint32_t y;
+    asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(y) : "r"(x));
+    return y;
+}
+// d = a . b + (FRESH ? 0 : d): the first product of a sum takes a zero operand instead of cleared registers
+template <typename E, bool FRESH>
+__device__ __forceinline__ void mma(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    const float c0 = FRESH ? 0.f : d[0], c1 = FRESH ? 0.f : d[1], c2 = FRESH ? 0.f : d[2], c3 = FRESH ? 0.f : d[3];
+    if constexpr (std::is_same<E, __half>::value)
+        asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %11, %12, %13};"
+                     : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+                     : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(c0), "f"(c1), "f"(c2), "f"(c3));
+    else
+        asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %11, %12, %13};"
+                     : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+                     : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(c0), "f"(c1), "f"(c2), "f"(c3));
+}
+
+// A lane's place in a tensor: row l / 4 of the current block or tile (the block's second half is 8 rows on), channels
+// 4 (l % 4) .. + 3; one wide multiply-add per step
+template <typename E> struct Place {
+    E* p;
+    int step;   // elements between rows of the residue
+    __device__ __forceinline__ Place(E* base, const Strides& s, int b, int h, int r, int dil, int row, int lane)
+        : p(base + b * s.batch + h * s.head + r * s.token + (long long)(row + (lane >> 2)) * (s.token * dil) + 4 * (lane & 3)), step((int)s.token * dil) {}
+    __device__ __forceinline__ void next() { p += (long long)step * 16; }
+    __device__ __forceinline__ E* half(int h) const { return h ? p + (long long)step * 8 : p; }
+};
+
+// 16 rows of 16 KC channels: r[h][kc] = channels 16 kc + 4 (l % 4) .. + 3 of row l / 4 + 8 h
+template <int KC> struct Rows {
+    uint2 r[2][KC];
+    // the 16 rows at `at`, whose first is row u - l / 4 of the residue; zeros outside [0, Tr)
+    template <typename E> __device__ __forceinline__ void load(const Place<E>& at, int u, int Tr) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const bool in = (unsigned)(u + 8 * h) < (unsigned)Tr;
+#pragma unroll
+            for (int kc = 0; kc < KC; ++kc)
+                r[h][kc] = in ? __ldg(reinterpret_cast<const uint2*>(at.half(h) + kc * 16)) : make_uint2(0u, 0u);
+        }
+    }
+};
+// the transposes of the same registers: right operands of products that contract over the 16 rows; t[kc][j][h]: channel half j
+// (channels 4 (p / 2) + 2 j + p % 2 for position p), rows 8 h .. + 7
+template <int KC> struct RowsT {
+    uint32_t t[KC][2][2];
+    __device__ __forceinline__ void set(const Rows<KC>& x) {
+#pragma unroll
+        for (int kc = 0; kc < KC; ++kc)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                t[kc][0][h] = transpose8(x.r[h][kc].x);
+                t[kc][1][h] = transpose8(x.r[h][kc].y);
+            }
+    }
+};
+// s0, s1 = a . b^T for b's rows 0-7 and 8-15
+template <typename E, int KC> __device__ __forceinline__ void products(float (&s0)[4], float (&s1)[4], const Rows<KC>& a, const Rows<KC>& b) {
+    mma<E, true>(s0, a.r[0][0].x, a.r[1][0].x, a.r[0][0].y, a.r[1][0].y, b.r[0][0].x, b.r[0][0].y);
+    mma<E, true>(s1, a.r[0][0].x, a.r[1][0].x, a.r[0][0].y, a.r[1][0].y, b.r[1][0].x, b.r[1][0].y);
+#pragma unroll
+    for (int kc = 1; kc < KC; ++kc) {
+        mma<E, false>(s0, a.r[0][kc].x, a.r[1][kc].x, a.r[0][kc].y, a.r[1][kc].y, b.r[0][kc].x, b.r[0][kc].y);
+        mma<E, false>(s1, a.r[0][kc].x, a.r[1][kc].x, a.r[0][kc].y, a.r[1][kc].y, b.r[1][kc].x, b.r[1][kc].y);
+    }
+}
+// acc (16 rows x 16 KC channels, channel order of RowsT) = (FRESH ? 0 : acc) + w . x, w a left operand over x's rows
+template <typename E, int KC, bool FRESH>
+__device__ __forceinline__ void accumulate(float (&acc)[KC][2][4], const uint32_t (&w)[4], const RowsT<KC>& x) {
+#pragma unroll
+    for (int kc = 0; kc < KC; ++kc)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) mma<E, FRESH>(acc[kc][j], w[0], w[1], w[2], w[3], x.t[kc][j][0], x.t[kc][j][1]);
+}
+template <typename E, int KC>
+__device__ __forceinline__ void store(const Place<E>& at, int u, int Tr, const float (&acc)[KC][2][4], float f0, float f1) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const float f = h ? f1 : f0;
+        if ((unsigned)(u + 8 * h) < (unsigned)Tr) {
+#pragma unroll
+            for (int kc = 0; kc < KC; ++kc) {
+                uint2 v;
+                v.x = Cvt<E>::pack2(acc[kc][0][2 * h] * f, acc[kc][0][2 * h + 1] * f);
+                v.y = Cvt<E>::pack2(acc[kc][1][2 * h] * f, acc[kc][1][2 * h + 1] * f);
+                *reinterpret_cast<uint2*>(at.half(h) + kc * 16) = v;
+            }
+        }
+    }
+}
+
+// A strip: blocks [b0, b1) of 16 rows of residue r of sequence (b, h). Heads are the slowest digit, so that the warps of a CTA
+// share one (their bias gradients are added up before they leave the CTA).
+struct MarchGeom {
+    int strips;   // strips per residue
+    int len;      // blocks per strip
+    int per_head; // strips of one head: batch * dil * strips
+    long long total;
+};
+struct Strip {
+    int b, h, r, b0, b1, nb, Tr, vl;
+    __device__ __forceinline__ bool init(const Geometry& gm, const MarchGeom& m, const int* __restrict__ valid_len, long long id) {
+        h = (int)(id / m.per_head);
+        int x = (int)(id - (long long)h * m.per_head);
+        const int s = x % m.strips;
+        x /= m.strips;
+        r = x % gm.dil;
+        b = x / gm.dil;
+        Tr = gm.T > r ? (gm.T - r + gm.dil - 1) / gm.dil : 0;
+        nb = (Tr + 15) / 16;
+        b0 = s * m.len;
+        b1 = min(nb, b0 + m.len);
+        const int v = valid_len ? min(gm.T, __ldg(valid_len + b)) : gm.T;
+        vl = v > r ? (v - r + gm.dil - 1) / gm.dil : 0;
+        return b0 < b1;
+    }
+};
+// bias of the thread's window offsets: class c = 2 (g - h + 1) + e is offset 8 (g - h) + e + fa (column group g, row half h)
+template <int NT> __device__ __forceinline__ void load_bias(float (&bias)[4 * NT + 2], const float* __restrict__ rpb, int h, int win, int fa) {
+#pragma unroll
+    for (int c = 0; c < 4 * NT + 2; ++c) {
+        const int kk = 8 * ((c >> 1) - 1) + (c & 1) + fa;
+        bias[c] = (unsigned)kk >= (unsigned)win ? -INFINITY : rpb ? __ldg(rpb + h * win + kk) * kLog2e : 0.f;
+    }
+}
+
+template <typename E, int KC, int NT>
+__global__ void __launch_bounds__(kWarps * 32) march_fwd_kernel(E* __restrict__ o, float* __restrict__ lse, const E* __restrict__ q, const E* __restrict__ k,
+                                                               const E* __restrict__ v, const float* __restrict__ rpb, const int* __restrict__ valid_len,
+                                                               Strides sq, Strides sk, Strides sv, Strides so, Geometry gm, MarchGeom mg) {
+    const int lane = threadIdx.x & 31, fr = lane >> 2, fa = 2 * (lane & 3) - fr;
+    const long long id = (long long)blockIdx.x * kWarps + (threadIdx.x >> 5);
+    Strip st;
+    if (id >= mg.total || !st.init(gm, mg, valid_len, id)) return;
+    float bias[4 * NT + 2];
+    load_bias<NT>(bias, rpb, st.h, gm.win, fa);
+    const int right = gm.win - 1 - gm.left;
+    const float sc = gm.scale * kLog2e, mask2 = kMaskValue * kLog2e;
+    Place<const E> pq(q, sq, st.b, st.h, st.r, gm.dil, 16 * st.b0, lane), pk(k, sk, st.b, st.h, st.r, gm.dil, 16 * st.b0 - gm.left, lane),
+        pv(v, sv, st.b, st.h, st.r, gm.dil, 16 * st.b0 - gm.left, lane);
+    Place<E> po(o, so, st.b, st.h, st.r, gm.dil, 16 * st.b0, lane);
+    float* lp = lse ? lse + ((long long)st.b * gm.H + st.h) * gm.T + (long long)(16 * st.b0 + fr) * gm.dil + st.r : nullptr;
+    int u = 16 * st.b0 + fr, uk = u - gm.left;   // this lane's first query row; its first row of the next key tile
+    Rows<KC> kf[NT], qn, kn, vn;
+    RowsT<KC> vt[NT];
+    // the first NT - 1 tiles; the last one of the first block comes in as "next"
+#pragma unroll
+    for (int t = 0; t < NT; ++t) {
+        kn.load(pk, uk, st.Tr);
+        vn.load(pv, uk, st.Tr);
+        pk.next(); pv.next(); uk += 16;
+        if (t + 1 < NT) { kf[t + 1] = kn; vt[t + 1].set(vn); }
+    }
+    qn.load(pq, u, st.Tr);
+#pragma unroll 1
+    for (int b = st.b0; b < st.b1; ++b, u += 16) {
+#pragma unroll
+        for (int t = 0; t + 1 < NT; ++t) { kf[t] = kf[t + 1]; vt[t] = vt[t + 1]; }
+        kf[NT - 1] = kn;
+        vt[NT - 1].set(vn);
+        const Rows<KC> qf = qn;
+        // the next block's rows are on their way while this one is computed
+        pq.next();
+        qn.load(pq, u + 16, st.Tr);
+        kn.load(pk, uk, st.Tr);
+        vn.load(pv, uk, st.Tr);
+        pk.next(); pv.next(); uk += 16;
+        float s[2 * NT][4], mx[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
+#pragma unroll
+        for (int t = 0; t < NT; ++t) products<E, KC>(s[2 * t], s[2 * t + 1], qf, kf[t]);
+        const bool need_mask = 16 * b < gm.left || 16 * b + 15 + right >= st.vl;
+#pragma unroll
+        for (int g = 0; g < 2 * NT; ++g)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) s[g][i] = fmaf(s[g][i], sc, bias[2 * (g - (i >> 1) + 1) + (i & 1)]);
+        if (need_mask) {
+#pragma unroll
+            for (int g = 0; g < 2 * NT; ++g)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const int row = u + 8 * (i >> 1), j = row - gm.left + 8 * (g - (i >> 1)) + (i & 1) + fa;
+                    if (j < 0 || j >= st.vl || row >= st.vl) s[g][i] += mask2;
+                }
+        }
+#pragma unroll
+        for (int g = 0; g < 2 * NT; ++g)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) mx[i >> 1] = fmaxf(mx[i >> 1], s[g][i]);
+        mx[0] = tc::quad_max(mx[0]);
+        mx[1] = tc::quad_max(mx[1]);
+        float acc[KC][2][4];
+#pragma unroll
+        for (int t = 0; t < NT; ++t) {
+#pragma unroll
+            for (int g = 2 * t; g < 2 * t + 2; ++g)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    s[g][i] = tc::fast_exp2(s[g][i] - mx[i >> 1]);
+                    l[i >> 1] += s[g][i];
+                }
+            const uint32_t w[4] = {Cvt<E>::pack2(s[2 * t][0], s[2 * t][1]), Cvt<E>::pack2(s[2 * t][2], s[2 * t][3]),
+                                   Cvt<E>::pack2(s[2 * t + 1][0], s[2 * t + 1][1]), Cvt<E>::pack2(s[2 * t + 1][2], s[2 * t + 1][3])};
+            if (t == 0) accumulate<E, KC, true>(acc, w, vt[t]); else accumulate<E, KC, false>(acc, w, vt[t]);
+        }
+        l[0] = tc::quad_sum(l[0]);
+        l[1] = tc::quad_sum(l[1]);
+        store<E, KC>(po, u, st.Tr, acc, tc::fast_rcp(l[0]), tc::fast_rcp(l[1]));
+        po.next();
+        if (lse) {
+            if ((lane & 3) == 0) {
+                if (u < st.Tr) lp[0] = (mx[0] + tc::fast_log2(l[0])) * kLn2;
+                if (u + 8 < st.Tr) lp[8 * gm.dil] = (mx[1] + tc::fast_log2(l[1])) * kLn2;
+            }
+            lp += 16 * gm.dil;
+        }
+    }
+}
+
+template <typename E, int KC, int NT>
+__global__ void __launch_bounds__(kWarps * 32) march_bwd_kernel(E* __restrict__ dq, E* __restrict__ dk, E* __restrict__ dv, float* __restrict__ d_rpb,
+                                                               const E* __restrict__ d_o, const E* __restrict__ q, const E* __restrict__ k,
+                                                               const E* __restrict__ v, const float* __restrict__ lse, const float* __restrict__ rpb,
+                                                               const int* __restrict__ valid_len, Strides sdq, Strides sdk, Strides sdv, Strides sdo,
+                                                               Strides sq, Strides sk, Strides sv, Geometry gm, MarchGeom mg) {
+    __shared__ float s_rpb[kWarps][16 * NT + 8];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, fr = lane >> 2, fa = 2 * (lane & 3) - fr;
+    const long long id = (long long)blockIdx.x * kWarps + warp;
+    Strip st;
+    const bool alive = id < mg.total && st.init(gm, mg, valid_len, id);
+    float grad[4 * NT + 2];
+#pragma unroll
+    for (int c = 0; c < 4 * NT + 2; ++c) grad[c] = 0.f;
+    if (alive) {
+        float bias[4 * NT + 2];
+        load_bias<NT>(bias, rpb, st.h, gm.win, fa);
+        const int right = gm.win - 1 - gm.left, first = max(0, st.b0 - (NT - 1));
+        const float sc = gm.scale * kLog2e, mask2 = kMaskValue * kLog2e;
+        Place<const E> pq(q, sq, st.b, st.h, st.r, gm.dil, 16 * first, lane), po(d_o, sdo, st.b, st.h, st.r, gm.dil, 16 * first, lane),
+            pk(k, sk, st.b, st.h, st.r, gm.dil, 16 * first - gm.left, lane), pv(v, sv, st.b, st.h, st.r, gm.dil, 16 * first - gm.left, lane);
+        Place<E> pdq(dq, sdq, st.b, st.h, st.r, gm.dil, 16 * first, lane), pdk(dk, sdk, st.b, st.h, st.r, gm.dil, 16 * first - gm.left, lane),
+            pdv(dv, sdv, st.b, st.h, st.r, gm.dil, 16 * first - gm.left, lane);
+        const float* lp = lse + ((long long)st.b * gm.H + st.h) * gm.T + (long long)(16 * first + fr) * gm.dil + st.r;
+        int u = 16 * first + fr, uk = u - gm.left;   // this lane's first query row; its first row of the next key tile
+        Rows<KC> kf[NT], vf[NT], qn, on, kn, vn;
+        float ln[2];
+        auto load_queries = [&](int row) {
+            qn.load(pq, row, st.Tr);
+            on.load(po, row, st.Tr);
+            // +inf for rows outside the sequence: probability 0
+            ln[0] = row < st.Tr ? __ldg(lp) * kLog2e : INFINITY;
+            ln[1] = row + 8 < st.Tr ? __ldg(lp + 8 * gm.dil) * kLog2e : INFINITY;
+            pq.next(); po.next(); lp += 16 * gm.dil;
+        };
+        auto load_keys = [&]() {
+            kn.load(pk, uk, st.Tr);
+            vn.load(pv, uk, st.Tr);
+            pk.next(); pv.next(); uk += 16;
+        };
+        float ak[NT][KC][2][4], av[NT][KC][2][4];
+#pragma unroll
+        for (int t = 0; t + 1 < NT; ++t)
+#pragma unroll
+            for (int kc = 0; kc < KC; ++kc)
+#pragma unroll
+                for (int i = 0; i < 8; ++i) ak[t][kc][i >> 2][i & 3] = av[t][kc][i >> 2][i & 3] = 0.f;
+#pragma unroll
+        for (int t = 0; t < NT; ++t) {
+            load_keys();
+            if (t + 1 < NT) { kf[t + 1] = kn; vf[t + 1] = vn; }
+        }
+        load_queries(u);
+#pragma unroll 1
+        for (int b = first; b < st.b1; ++b, u += 16) {
+            const bool own = b >= st.b0;
+#pragma unroll
+            for (int t = 0; t + 1 < NT; ++t) { kf[t] = kf[t + 1]; vf[t] = vf[t + 1]; }
+            kf[NT - 1] = kn;
+            vf[NT - 1] = vn;
+            const Rows<KC> qf = qn, of = on;
+            const float l2[2] = {ln[0], ln[1]};
+            load_queries(u + 16);
+            load_keys();
+            float s[2 * NT][4], d[2 * NT][4], delta[2], part[2][4] = {};   // (two chains per row keep the sums short)
+#pragma unroll
+            for (int t = 0; t < NT; ++t) {
+                products<E, KC>(s[2 * t], s[2 * t + 1], qf, kf[t]);
+                products<E, KC>(d[2 * t], d[2 * t + 1], of, vf[t]);
+            }
+            const bool need_mask = 16 * b < gm.left || 16 * b + 15 + right >= st.vl;
+#pragma unroll
+            for (int g = 0; g < 2 * NT; ++g)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) s[g][i] = fmaf(s[g][i], sc, bias[2 * (g - (i >> 1) + 1) + (i & 1)]);
+            if (need_mask) {
+#pragma unroll
+                for (int g = 0; g < 2 * NT; ++g)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const int row = u + 8 * (i >> 1), j = row - gm.left + 8 * (g - (i >> 1)) + (i & 1) + fa;
+                        if (j < 0 || j >= st.vl || row >= st.vl) s[g][i] += mask2;
+                    }
+            }
+#pragma unroll
+            for (int g = 0; g < 2 * NT; ++g)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    s[g][i] = tc::fast_exp2(s[g][i] - l2[i >> 1]);
+                    part[g & 1][i] = fmaf(s[g][i], d[g][i], part[g & 1][i]);
+                }
+            delta[0] = tc::quad_sum((part[0][0] + part[0][1]) + (part[1][0] + part[1][1]));
+            delta[1] = tc::quad_sum((part[0][2] + part[0][3]) + (part[1][2] + part[1][3]));
+#pragma unroll
+            for (int g = 0; g < 2 * NT; ++g)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) d[g][i] = s[g][i] * (d[g][i] - delta[i >> 1]);
+            if (own && d_rpb) {
+#pragma unroll
+                for (int g = 0; g < 2 * NT; ++g)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) grad[2 * (g - (i >> 1) + 1) + (i & 1)] += d[g][i];
+            }
+            RowsT<KC> qt, ot;
+            qt.set(qf);
+            ot.set(of);
+            float acc[KC][2][4];
+#pragma unroll
+            for (int t = 0; t < NT; ++t) {
+                // left operands over the keys: (rows 0-7, keys 0-7), (rows 8-15, keys 0-7), (rows 0-7, keys 8-15), (rows 8-15, keys 8-15)
+                uint32_t w[4], x[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const int g = 2 * t + (i >> 1), h = 2 * (i & 1);
+                    w[i] = Cvt<E>::pack2(d[g][h] * gm.scale, d[g][h + 1] * gm.scale);
+                    x[i] = Cvt<E>::pack2(s[g][h], s[g][h + 1]);
+                }
+                RowsT<KC> kt;
+                kt.set(kf[t]);
+                if (t == 0) accumulate<E, KC, true>(acc, w, kt); else accumulate<E, KC, false>(acc, w, kt);
+                // and transposed, over the queries: the off-diagonal matrices change places
+                const uint32_t wt[4] = {transpose8(w[0]), transpose8(w[2]), transpose8(w[1]), transpose8(w[3])};
+                const uint32_t xt[4] = {transpose8(x[0]), transpose8(x[2]), transpose8(x[1]), transpose8(x[3])};
+                if (t + 1 == NT) { accumulate<E, KC, true>(ak[t], wt, qt); accumulate<E, KC, true>(av[t], xt, ot); }   // (the newest tile)
+                else { accumulate<E, KC, false>(ak[t], wt, qt); accumulate<E, KC, false>(av[t], xt, ot); }
+            }
+            if (own) {
+                store<E, KC>(pdq, u, st.Tr, acc, 1.f, 1.f);
+                store<E, KC>(pdk, u - gm.left, st.Tr, ak[0], 1.f, 1.f);
+                store<E, KC>(pdv, u - gm.left, st.Tr, av[0], 1.f, 1.f);
+            }
+            pdq.next(); pdk.next(); pdv.next();
+#pragma unroll
+            for (int t = 0; t + 1 < NT; ++t)
+#pragma unroll
+                for (int kc = 0; kc < KC; ++kc)
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        ak[t][kc][i >> 2][i & 3] = ak[t + 1][kc][i >> 2][i & 3];
+                        av[t][kc][i >> 2][i & 3] = av[t + 1][kc][i >> 2][i & 3];
+                    }
+        }
+        if (st.b1 == st.nb) {   // the sequence's last strip owns the tiles behind its last block too
+#pragma unroll
+            for (int t = 0; t + 1 < NT; ++t) {
+                store<E, KC>(pdk, u - gm.left, st.Tr, ak[t], 1.f, 1.f);
+                store<E, KC>(pdv, u - gm.left, st.Tr, av[t], 1.f, 1.f);
+                pdk.next(); pdv.next(); u += 16;
+            }
+        }
+    }
+    if (d_rpb) {
+        for (int i = lane; i < 16 * NT + 8; i += 32) s_rpb[warp][i] = 0.f;
+        __syncwarp();
+        if (alive) {
+#pragma unroll
+            for (int c = 0; c < 4 * NT + 2; ++c) {
+                const int kk = 8 * ((c >> 1) - 1) + (c & 1) + fa;
+                if ((unsigned)kk < (unsigned)gm.win) atomicAdd(&s_rpb[warp][kk], grad[c]);
+            }
+        }
+        __syncthreads();
+        // warps of one head are neighbours: a run of them is added up and handed over once
+        const long long id0 = (long long)blockIdx.x * kWarps;
+        for (int kk = threadIdx.x; kk < gm.win; kk += kWarps * 32) {
+            float sum = 0.f;
+            for (int w = 0; w < kWarps && id0 + w < mg.total; ++w) {
+                const int h = (int)((id0 + w) / mg.per_head);
+                sum += s_rpb[w][kk];
+                if (w + 1 == kWarps || id0 + w + 1 >= mg.total || (int)((id0 + w + 1) / mg.per_head) != h) {
+                    atomicAdd(d_rpb + h * gm.win + kk, sum);
+                    sum = 0.f;
+                }
+            }
+        }
+    }
+}
+
+// Blocks per strip. A strip costs its blocks and `extra` blocks' worth of start-up (first loads; in the backward the recomputed
+// blocks), and the GPU runs `per_sm` warps of it per SM at a time: the number of strips per residue with the shortest
+// total is taken. Large batches get whole sequences, single utterances strips of one or two blocks.
+MarchGeom march_geom(const Geometry& gm, int per_sm, int extra) {
+    MarchGeom m;
+    const int nb = ((gm.T + gm.dil - 1) / gm.dil + 15) / 16, batch = gm.N / gm.H;
+    const long long residues = (long long)gm.N * gm.dil, room = (long long)per_sm * device_sm_count();
+    long long best = 0;
+    m.strips = 1;
+    for (int s = 1; s <= nb; s += s < 16 ? 1 : s / 8) {
+        const long long warps = residues * s + room / 2;   // (half a round of them for the uneven end)
+        const long long cost = (warps < room ? room : warps) * ((nb + s - 1) / s + extra);
+        if (s == 1 || cost < best) { best = cost; m.strips = s; }
+    }
+    m.len = (nb + m.strips - 1) / m.strips;
+    m.per_head = batch * gm.dil * m.strips;
+    m.total = (long long)m.per_head * gm.H;
+    return m;
+}
+
+}  // namespace
+
+// 16-channel rows, windows up to 33 (three key tiles), any dilation, token count and number of heads; row steps within an int
+bool march_supports(const Geometry& gm) {
+    const long long nb = ((long long)gm.T + 15) / 16 + gm.dil;
+    return gm.C == 16 && gm.win <= 33 && (long long)gm.N * nb * 2 < (1ll << 31);
+}
+
+cudaError_t march_fused_fwd(void* o, float* lse, const void* q, const void* k, const void* v, const float* rpb, const int* valid_len,
+                            const Strides& sq, const Strides& sk, const Strides& sv, const Strides& so, const Geometry& gm, int dtype, cudaStream_t st) {
+    const MarchGeom m = march_geom(gm, 16, 1);
+    const unsigned grid = (unsigned)((m.total + kWarps - 1) / kWarps);
+#define NA1D_MARCH(E, NT) march_fwd_kernel<E, 1, NT><<<grid, kWarps * 32, 0, st>>>((E*)o, lse, (const E*)q, (const E*)k, (const E*)v, rpb, valid_len, sq, sk, sv, so, gm, m)
+    if (dtype == 0) { if (gm.win <= 17) NA1D_MARCH(__nv_bfloat16, 2); else NA1D_MARCH(__nv_bfloat16, 3); }
+    else { if (gm.win <= 17) NA1D_MARCH(__half, 2); else NA1D_MARCH(__half, 3); }
+#undef NA1D_MARCH
+    return cudaGetLastError();
+}
+cudaError_t march_fused_bwd(void* dq, void* dk, void* dv, float* d_rpb, const void* d_o, const void* q, const void* k, const void* v, const float* lse,
+                            const float* rpb, const int* valid_len, const Strides& sdq, const Strides& sdk, const Strides& sdv, const Strides& sdo,
+                            const Strides& sq, const Strides& sk, const Strides& sv, const Geometry& gm, int dtype, cudaStream_t st) {
+    const MarchGeom m = march_geom(gm, gm.win <= 17 ? 12 : 8, gm.win <= 17 ? 2 : 3);
+    const unsigned grid = (unsigned)((m.total + kWarps - 1) / kWarps);
+#define NA1D_MARCH(E, NT)                                                                                                                             \
+    march_bwd_kernel<E, 1, NT><<<grid, kWarps * 32, 0, st>>>((E*)dq, (E*)dk, (E*)dv, d_rpb, (const E*)d_o, (const E*)q, (const E*)k, (const E*)v, lse, \
+                                                             rpb, valid_len, sdq, sdk, sdv, sdo, sq, sk, sv, gm, m)
+    if (dtype == 0) { if (gm.win <= 17) NA1D_MARCH(__nv_bfloat16, 2); else NA1D_MARCH(__nv_bfloat16, 3); }
+    else { if (gm.win <= 17) NA1D_MARCH(__half, 2); else NA1D_MARCH(__half, 3); }
+#undef NA1D_MARCH
+    return cudaGetLastError();
+}
+
+}  // namespace na1d

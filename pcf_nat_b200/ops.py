@@ -360,7 +360,7 @@ def window_index(T, win, left, dil=1, device="cuda"):
     return j, inr.bool()
 
 
-FAMILY_AUTO, FAMILY_CUDA_CORE, FAMILY_TCGEN05, FAMILY_TCGEN05_SEGMENTED, FAMILY_WARP_MMA = -1, 0, 1, 2, 3
+FAMILY_AUTO, FAMILY_CUDA_CORE, FAMILY_TCGEN05, FAMILY_TCGEN05_SEGMENTED, FAMILY_WARP_MMA, FAMILY_MARCH = -1, 0, 1, 2, 3, 4
 
 
 def set_kernel_family(family):

@@ -107,9 +107,14 @@ def test_values_that_are_not_finite_reach_their_window_only(which, value):
 
 
 def test_routes():
-    """Above 128 channels the CUDA-core kernels stay; the automatic route of a general shape is the warp-level one, bit for bit."""
+    """Above 128 channels and for few neighbours the CUDA-core kernels stay; the automatic route of a general shape is the warp-level
+    one, bit for bit."""
     from pcf_nat_b200 import ops
-    case = (1, 2, 70, 48, 20, 9, 1, True, True)
+    case = (64, 4, 20, 8, 5, 2, 4, True, True)
+    args = _inputs(case, torch.bfloat16)
+    for a, b in zip(_run(ops.FAMILY_AUTO, case, *args)[:4], _run(ops.FAMILY_CUDA_CORE, case, *args)[:4]):
+        assert torch.equal(a, b)
+    case = (16, 8, 300, 48, 20, 9, 1, True, True)
     args = _inputs(case, torch.bfloat16)
     for a, b in zip(_run(ops.FAMILY_AUTO, case, *args)[:4], _run(ops.FAMILY_WARP_MMA, case, *args)[:4]):
         assert torch.equal(a, b)
