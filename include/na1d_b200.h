@@ -262,8 +262,8 @@ int na1d_stats_pool_backward(void* d_logits, void* dx, const float* d_out, const
 int na1d_window_index(int32_t* j_out, uint8_t* in_range, int64_t T, int64_t win, int64_t left,
                       int64_t dil, void* stream);
 
-/* Which kernel family the fused entry points would pick for a shape (16-channel rows with windows up to 33 run on the
- * marching kernels, na1d_march.cu, and report the family that otherwise takes the shape): 0 = the general kernels (warp-level matrix
+/* Which kernel family the fused entry points would pick for a shape (16-channel rows, and 32-channel rows in some
+ * forwards, run on the marching kernels, na1d_march.cu, and report the family that otherwise takes the shape): 0 = the general kernels (warp-level matrix
  * instructions up to 128 channels, CUDA-core kernels above),
  * 1 = tcgen05/TMA kernels. Host-only query, no device work. The answer assumes one head, no bias and
  * no bias gradient: more than 32 heads, or 64-channel rows with an effective window above 17 together
@@ -283,8 +283,8 @@ int na1d_fused_kernel_tiling(int64_t N, int64_t T, int64_t C, int64_t win, int64
 /* Force a kernel family for the fused entry points: -1 = automatic (default), 0 = CUDA-core,
  * 1 = tcgen05/TMA (the flat tiling wherever it can run, else the segmented one; for the unfused entry points: also
  * where the automatic choice would take a CUDA-core kernel), 2 = tcgen05/TMA on the segmented tiling, 3 = the warp-level matrix
- * kernels wherever they can run (up to 128 channels), else CUDA-core, 4 = the marching kernels where they can run (fused
- * entry points, 16-channel rows with windows up to 33; the automatic choice there), else as 3. Process-wide;
+ * kernels wherever they can run (up to 128 channels), else CUDA-core, 4 = the marching kernels where they can run (windows up
+ * to 33; fused entry points at 16 channels, forward at 32 too, unfused ones at 16, 32 and 64), else as 3. Process-wide;
  * meant for tests and benchmarks. Returns the previous setting. */
 int na1d_set_kernel_family(int family);
 

@@ -36,17 +36,21 @@ int check_geometry(int64_t N, int64_t heads, int64_t T, int64_t C, int64_t win, 
     return NA1D_OK;
 }
 
-// Which kernels run an unfused operator: the tcgen05 ones (tiles of 128 rows, a fixed cost per row), the CUDA-core ones (no fixed
-// cost, C * win operations a row) or the ones on warp-level matrix instructions (band staged in shared memory).
-enum class Unfused { core, tcgen05, warp };
-Unfused pick_unfused(const na1d::Geometry& g, int core_most, bool tc_ok, bool tc_preferred) {
+// Which kernels run an unfused operator. The CUDA-core ones cost C * win operations a row and nothing else; the others have a
+// cost per row that hardly depends on the window: the marching ones (16, 32, 64 channels, dilation 1) the least, the tcgen05
+// ones, and the warp-level products on staged tiles for what is left (other channel counts, windows and dilations).
+enum class Unfused { core, tcgen05, warp, march };
+Unfused pick_unfused(const na1d::Geometry& g, int core_most, int core_most_march, bool tc_ok, bool tc_over_march, bool tc_over_warp, bool march_ok) {
     const int forced = g_family_override.load();
     const bool warp_ok = na1d::mma_band_supports(g);
+    march_ok = march_ok && na1d::march_band_supports(g);
     if (forced == 0) return Unfused::core;
+    if (forced == 4 && march_ok) return Unfused::march;
     if (forced >= 3) return warp_ok ? Unfused::warp : Unfused::core;
     if (forced == 1 && tc_ok) return Unfused::tcgen05;
+    if (march_ok && !(tc_ok && tc_over_march)) return g.C * g.win <= core_most_march ? Unfused::core : Unfused::march;
     if (g.C * g.win <= core_most) return Unfused::core;
-    if (tc_ok && tc_preferred) return Unfused::tcgen05;
+    if (tc_ok && (tc_over_march || tc_over_warp)) return Unfused::tcgen05;
     return warp_ok ? Unfused::warp : Unfused::core;
 }
 
@@ -82,13 +86,16 @@ bool use_mma(const na1d::Geometry& g, bool backward) {
     return mma < core;
 }
 
-// The marching kernels: automatic for every shape they take (16-channel rows, windows up to 33), and what stands for the
-// segmented tiling there (both work on residue classes through arbitrary strides). Forced family 4 is the same without that
-// tiling's own limits.
-template <typename... S> bool use_march(const na1d::Geometry& g, const S&... strides) {
+// The marching kernels: 16-channel rows in everything; 32-channel rows in the forward, where they stand for the segmented tiling
+// (any strides, no empty tile rows: 85 -> 51 us for 4096 x 150 rows, window 27) and, on dense tensors, for small problems (the
+// flat tiling starts slower but is as fast from about 300 thousand rows on: 16 against 13 us at 154 thousand rows, 49 against 51
+// at 614 thousand). A forced family 2 takes them too where it takes the shape; 4 is the same without that tiling's own limits.
+enum class Pass { forward, strided_forward, backward };
+template <typename... S> bool use_march(const na1d::Geometry& g, Pass pass, const S&... strides) {
     const int forced = g_family_override.load();
     if (forced != -1 && forced != 4 && !(forced == 2 && na1d::tc_seg_supports(g))) return false;
-    return na1d::march_supports(g) && ((strides.token * g.dil < (1ll << 30)) && ...);
+    if (forced == -1 && pass == Pass::forward && g.C == 32 && (long long)g.N * g.T > (1 << 18)) return false;
+    return na1d::march_supports(g, pass == Pass::backward) && ((strides.token * g.dil < (1ll << 30)) && ...);
 }
 }  // namespace
 
@@ -121,11 +128,14 @@ int na1d_qk_forward(float* attn, const void* q, const void* k, int64_t N, int64_
     NA1D_REQUIRE_ALIGNED(q); NA1D_REQUIRE_ALIGNED(k);
     na1d::Geometry g;
     if (int s = check_geometry(N, 1, T, C, win, left, dil, dtype, 1.f, g)) return s;
-    // measured at 4096 x 150 and 512 x 997 rows, us (CUDA core / tcgen05 / warp-level): 16 channels, window 3: 12 / 20 / 32,
-    // window 7: 21 / 20 / 34, window 27: 81 / 31 / 43; 64 channels, window 27: 211 / 35 / 65
+    // us at 8192 x 150 rows (6912, 3456 at 32, 64 channels), CUDA core / tcgen05 / warp-level / marching: 16 channels, window 3:
+    // 22 / 40 / 52 / 23, window 5: 30 / 47 / 53 / 25, window 27: 183 / 58 / 67 / 42; 32 channels, window 3: 39 / 45 / 55 / 31;
+    // 64 channels, window 9: 82 / 31 / 49 / 32, window 27: 211 / 35 / 59 / 40, window 33 (one tcgen05 CTA per SM instead of two):
+    // 253 / 55 / 71 / 41
     const bool tc_ok = na1d::tc_unfused_supports(g) && aligned16(attn);   // (its band goes out in 16-byte stores)
-    switch (pick_unfused(g, 80, tc_ok, true)) {
+    switch (pick_unfused(g, 80, 64, tc_ok, g.C == 64 && g.win <= 28, true, true)) {
         case Unfused::tcgen05: return cuda_status(na1d::tc_qk(attn, q, k, g, dtype, (cudaStream_t)stream));
+        case Unfused::march: return cuda_status(na1d::march_band_out(attn, q, k, g, dtype, (cudaStream_t)stream));
         case Unfused::warp: return cuda_status(na1d::mma_band_out(attn, q, k, g, dtype, (cudaStream_t)stream));
         default: return cuda_status(na1d::simt_qk(attn, q, k, g, dtype, (cudaStream_t)stream));
     }
@@ -140,10 +150,11 @@ int na1d_q_backward(void* q_gd, const float* attn_gd, const void* k, int64_t N, 
     NA1D_REQUIRE_ALIGNED(q_gd); NA1D_REQUIRE_ALIGNED(k);
     na1d::Geometry g;
     if (int s = check_geometry(N, 1, T, C, win, left, dil, dtype, 1.f, g)) return s;
-    // 16 channels, window 7: 19 / 28 / 41, window 17: 37 / 32 / 46; 32 channels, window 3: 21 / 31 / 48, window 7: 36 / 34 / 48;
-    // 64 channels, window 3: 34 / 37 / 68, window 27: 168 / 48 / 87
-    switch (pick_unfused(g, 208, na1d::tc_unfused_supports(g), true)) {
+    // as above: 16 channels, window 5: 29 / 58 / 71 / 35, window 9: 43 / 62 / 74 / 37, window 27: 106 / 82 / 93 / 49; 32 channels, window
+    // 3: 34 / 52 / 74 / 39, window 27: 167 / 78 / 97 / 57; 64 channels, window 3: 34 / 37 / 63 / 36, window 27: 167 / 48 / 80 / 45
+    switch (pick_unfused(g, 208, 112, na1d::tc_unfused_supports(g), false, true, true)) {
         case Unfused::tcgen05: return cuda_status(na1d::tc_band_x(q_gd, attn_gd, k, g, dtype, (cudaStream_t)stream));
+        case Unfused::march: return cuda_status(na1d::march_band_rows(q_gd, attn_gd, k, false, g, dtype, (cudaStream_t)stream));
         case Unfused::warp: return cuda_status(na1d::mma_band_rows(q_gd, attn_gd, k, false, g, dtype, (cudaStream_t)stream));
         default: return cuda_status(na1d::simt_band_x(q_gd, attn_gd, k, g, dtype, (cudaStream_t)stream));
     }
@@ -158,12 +169,15 @@ int na1d_k_backward(void* k_gd, const float* attn_gd, const void* q, int64_t N, 
     NA1D_REQUIRE_ALIGNED(k_gd); NA1D_REQUIRE_ALIGNED(q);
     na1d::Geometry g;
     if (int s = check_geometry(N, 1, T, C, win, left, dil, dtype, 1.f, g)) return s;
-    // the tcgen05 form gathers the fp32 band along its diagonals and pays off at 64 channels and narrow windows only:
-    // 16 channels, window 17: 41 / 47 / 50, window 33: 80 / 100 / 66; 32 channels, window 9: 46 / 52 / 50, window 27: 117 / 99 / 73;
-    // 64 channels, window 3: 35 / 42 / 69, window 9: 76 / 54 / 70, window 17 (997 rows): 125 / 76 / 60, window 27: 188 / - / 97
+    // as above: 16 channels, window 5: 31 / 84 / 75 / 39, window 9: 46 / 102 / 76 / 42, window 27: 120 / 187 / 103 / 53; 32 channels,
+    // window 5: 50 / 77 / 78 / 41, window 27: 191 / 159 / 107 / 56; 64 channels, window 3: 35 / 42 / 65 / 36 (512 x 997 rows: 35 / 41 /
+    // 52 / 41), window 9: 76 / 53 / 67 / 37, window 27: 188 / - / 88 / 51. fp16 tensors keep the fp32 band's exponents in tf32
+    // pieces, which the marching form does not have: there the tcgen05 form, which gathers the band along its diagonals, pays
+    // off at 64 channels and windows up to 9 only.
     const int weff = (g.win - 1) * g.dil + 1;
-    switch (pick_unfused(g, 288, na1d::tc_unfused_t_supports(g), g.C == 64 && weff <= 9)) {
+    switch (pick_unfused(g, 288, g.C == 64 ? 192 : 112, na1d::tc_unfused_t_supports(g), false, g.C == 64 && weff <= 9, dtype == NA1D_BF16)) {
         case Unfused::tcgen05: return cuda_status(na1d::tc_bandT_x(k_gd, attn_gd, q, g, dtype, (cudaStream_t)stream));
+        case Unfused::march: return cuda_status(na1d::march_band_rows(k_gd, attn_gd, q, true, g, dtype, (cudaStream_t)stream));
         case Unfused::warp: return cuda_status(na1d::mma_band_rows(k_gd, attn_gd, q, true, g, dtype, (cudaStream_t)stream));
         default: return cuda_status(na1d::simt_bandT_x(k_gd, attn_gd, q, g, dtype, (cudaStream_t)stream));
     }
@@ -255,7 +269,7 @@ int na1d_fused_forward(void* o, float* lse, const void* q, const void* k, const 
     NA1D_REQUIRE_ALIGNED(o); NA1D_REQUIRE_ALIGNED(q); NA1D_REQUIRE_ALIGNED(k); NA1D_REQUIRE_ALIGNED(v);
     na1d::Geometry g;
     if (int s = check_geometry(N, heads, T, C, win, left, dil, dtype, scale, g)) return s;
-    if (use_march(g, na1d::dense_strides(g.H, g.T, g.C))) {
+    if (use_march(g, Pass::forward, na1d::dense_strides(g.H, g.T, g.C))) {
         const na1d::Strides d = na1d::dense_strides(g.H, g.T, g.C);
         return cuda_status(na1d::march_fused_fwd(o, lse, q, k, v, rpb, valid_len, d, d, d, d, g, dtype, (cudaStream_t)stream));
     }
@@ -308,7 +322,7 @@ int na1d_fused_forward_strided(void* o, float* lse, const void* q, const void* k
     if (int s = read_strides(k_strides, batch, heads, T, C, sk)) return s;
     if (int s = read_strides(v_strides, batch, heads, T, C, sv)) return s;
     if (!na1d::tc_seg_supports(g)) return NA1D_ERR_UNSUPPORTED;
-    if (use_march(g, sq, sk, sv, so)) return cuda_status(na1d::march_fused_fwd(o, lse, q, k, v, rpb, valid_len, sq, sk, sv, so, g, dtype, (cudaStream_t)stream));
+    if (use_march(g, Pass::strided_forward, sq, sk, sv, so)) return cuda_status(na1d::march_fused_fwd(o, lse, q, k, v, rpb, valid_len, sq, sk, sv, so, g, dtype, (cudaStream_t)stream));
     return cuda_status(na1d::tc_fused_fwd_seg(o, lse, q, k, v, rpb, valid_len, sq, sk, sv, so, g, dtype, (cudaStream_t)stream));
 }
 
@@ -332,7 +346,7 @@ int na1d_fused_backward_strided(void* dq, void* dk, void* dv, float* d_rpb, cons
     for (int i = 0; i < 7; ++i)
         if (int s = read_strides(in[i], batch, heads, T, C, s7[i])) return s;
     if (!na1d::tc_bwd_seg_supports(g, rpb != nullptr, d_rpb != nullptr)) return NA1D_ERR_UNSUPPORTED;
-    if (use_march(g, s7[0], s7[1], s7[2], s7[3], s7[4], s7[5], s7[6]))
+    if (use_march(g, Pass::backward, s7[0], s7[1], s7[2], s7[3], s7[4], s7[5], s7[6]))
         return cuda_status(na1d::march_fused_bwd(dq, dk, dv, d_rpb, d_o, q, k, v, lse, rpb, valid_len, s7[0], s7[1], s7[2], s7[3], s7[4], s7[5],
                                                  s7[6], g, dtype, (cudaStream_t)stream));
     return cuda_status(na1d::tc_fused_bwd_seg(dq, dk, dv, d_rpb, d_o, q, k, v, lse, rpb, valid_len, scratch, (size_t)scratch_floats,
@@ -351,7 +365,7 @@ int na1d_fused_backward(void* dq, void* dk, void* dv, float* d_rpb, const void* 
     if (int s = check_geometry(N, heads, T, C, win, left, dil, dtype, scale, g)) return s;
     if (d_rpb && heads * win * 4 > 48 * 1024) return NA1D_ERR_TOO_LARGE;
     cudaStream_t st = (cudaStream_t)stream;
-    if (use_march(g, na1d::dense_strides(g.H, g.T, g.C))) {
+    if (use_march(g, Pass::backward, na1d::dense_strides(g.H, g.T, g.C))) {
         const na1d::Strides d = na1d::dense_strides(g.H, g.T, g.C);
         return cuda_status(na1d::march_fused_bwd(dq, dk, dv, d_rpb, d_o, q, k, v, lse, rpb, valid_len, d, d, d, d, d, d, d, g, dtype, st));
     }

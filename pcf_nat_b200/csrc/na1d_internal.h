@@ -24,13 +24,16 @@ cudaError_t mma_fused_fwd(void* o, float* lse, const void* q, const void* k, con
 cudaError_t mma_fused_bwd(void* dq, void* dk, void* dv, float* d_rpb, const void* d_o, const void* q, const void* k, const void* v,
                           const void* o, const float* lse, const float* rpb, const int* valid_len, const Geometry& gm, int dtype,
                           cudaStream_t st);
-// ---- 16-channel rows with everything in registers (na1d_march.cu), any strides
-bool march_supports(const Geometry& gm);
+// ---- narrow rows with everything in registers (na1d_march.cu), any strides
+bool march_supports(const Geometry& gm, bool backward);
 cudaError_t march_fused_fwd(void* o, float* lse, const void* q, const void* k, const void* v, const float* rpb, const int* valid_len,
                             const Strides& sq, const Strides& sk, const Strides& sv, const Strides& so, const Geometry& gm, int dtype, cudaStream_t st);
 cudaError_t march_fused_bwd(void* dq, void* dk, void* dv, float* d_rpb, const void* d_o, const void* q, const void* k, const void* v, const float* lse,
                             const float* rpb, const int* valid_len, const Strides& sdq, const Strides& sdk, const Strides& sdv, const Strides& sdo,
                             const Strides& sq, const Strides& sk, const Strides& sv, const Geometry& gm, int dtype, cudaStream_t st);
+bool march_band_supports(const Geometry& gm);   // 16, 32 or 64 channels, one head (sequences), dilation 1
+cudaError_t march_band_out(float* band, const void* a, const void* b, const Geometry& gm, int dtype, cudaStream_t st);
+cudaError_t march_band_rows(void* out, const float* band, const void* x, bool transposed, const Geometry& gm, int dtype, cudaStream_t st);
 
 bool mma_band_supports(const Geometry& gm);
 cudaError_t mma_band_out(float* band, const void* a, const void* b, const Geometry& gm, int dtype, cudaStream_t st);

@@ -1,4 +1,4 @@
-// Fused NA1D for narrow rows: warps that march along a sequence with everything in registers.
+// NA1D for narrow rows and the unfused pair: warps that march along a sequence with everything in registers.
 //
 // At 16 channels a row is one 32-byte sector and the operator should be bound by HBM (512 x 16 x 150 rows: 24 us forward, 43 us
 // backward), but a 128-row tcgen05 tile spends most of its time in the chain TMA -> S -> softmax -> P.V -> epilogue with few
@@ -23,6 +23,8 @@
 // 141 / 194 / 136; window 9 forward 62 / 104 / 40, backward 99 / 154 / 94; 64 x 16 x 997 rows, window 27: 66 / 66 / 41 and
 // 115 / 119 / 97. The forward is bound by instruction issue (0.67 a cycle), the backward by latency at the eight warps an SM
 // that its 225 registers leave (three CTAs an SM at 168 registers spill and are slower: 139).
+// Forward at 32 channels: 512 x 300 rows, window 27: 16 / 20 / 13; 4096 x 150: 49 / 85 / 51; the backward there needs more registers
+// than a thread has and stays on tcgen05 (82 / 107 against 118).
 // Rounding is that of the tcgen05 kernels: probabilities and dS enter the second products in 16 bits, sums are fp32.
 #include "na1d_internal.h"
 #include "na1d_tc_common.cuh"
@@ -431,6 +433,214 @@ __global__ void __launch_bounds__(kWarps * 32) march_bwd_kernel(E* __restrict__ 
     }
 }
 
+// ---------------------------------------------------------------- the unfused pair (dilation 1)
+// The same march with the fp32 band in memory: a block's 16 band rows are one contiguous piece, moved in whole lines through a
+// 16 x (16 NT + 8) patch of shared memory per warp in which entry (row, kk) stands at column row + kk, the accumulator's own
+// order (pitch 8 mod 32 words: 8-byte accesses without bank conflicts). Positions outside the band are never written and
+// stay zero. The patch offsets of a lane's elements are the same in every block and are kept in registers.
+// Measured (tcgen05 / warp-level products on 128-row tiles / here, us; HBM time is 33, 38 and 26):
+// 8192 x 150 x 16, window 27: q.k 58 / 67 / 42, a.v 82 / 93 / 49, transposed 187 (CUDA core 120) / 103 / 53;
+// 6912 x 150 x 32, window 27: 54 / 72 / 47, 78 / 97 / 57, 159 / 107 / 56; 3456 x 150 x 64, window 17: 33 / 52 / 34, 42 / 70 / 39,
+// 76 / 74 / 38.
+//   march_qk  : band[t, kk] = a[t] . b[j]             (QK forward, dA)
+//   march_rows: out[t] = sum band[t, kk] x[j]         (AV forward, dQ), or TRANSPOSED out[j] = sum band[t, kk] x[t] (dV, dK)
+// The band enters the products as two 16-bit pieces. A result that is not finite is computed again, row by row in fp32: the
+// zeros outside the band must not meet an infinite row.
+template <int NT> constexpr int kPatchPitch = 16 * NT + 8;
+template <int NT> constexpr int kPatchIters = (16 * (16 * NT - 15) + 31) / 32;   // 32-element steps of 16 band rows
+template <int NT> __device__ __forceinline__ void patch_offsets(int (&off)[kPatchIters<NT>], int win, int lane) {
+#pragma unroll
+    for (int it = 0; it < kPatchIters<NT>; ++it) {
+        const int i = it * 32 + lane, row = i / win;
+        off[it] = i < 16 * win ? row * kPatchPitch<NT> + row + (i - row * win) : -1;
+    }
+}
+
+template <typename E, int KC, int NT>
+__global__ void __launch_bounds__(kWarps * 32) march_qk_kernel(float* __restrict__ band, const E* __restrict__ a, const E* __restrict__ b_, Strides sd,
+                                                              Geometry gm, MarchGeom mg) {
+    __shared__ float patch_all[kWarps][16 * kPatchPitch<NT>];
+    const int lane = threadIdx.x & 31, fr = lane >> 2;
+    const long long id = (long long)blockIdx.x * kWarps + (threadIdx.x >> 5);
+    Strip st;
+    if (id >= mg.total || !st.init(gm, mg, nullptr, id)) return;
+    float* patch = patch_all[threadIdx.x >> 5];
+    int off[kPatchIters<NT>];
+    patch_offsets<NT>(off, gm.win, lane);
+    Place<const E> pa(a, sd, st.b, 0, 0, 1, 16 * st.b0, lane), pb(b_, sd, st.b, 0, 0, 1, 16 * st.b0 - gm.left, lane);
+    float* dst = band + ((long long)st.b * gm.T + 16 * st.b0) * gm.win;
+    int u = 16 * st.b0 + fr, uk = u - gm.left;
+    Rows<KC> kf[NT], qn, kn;
+#pragma unroll
+    for (int t = 0; t < NT; ++t) {
+        kn.load(pb, uk, st.Tr);
+        pb.next(); uk += 16;
+        if (t + 1 < NT) kf[t + 1] = kn;
+    }
+    qn.load(pa, u, st.Tr);
+#pragma unroll 1
+    for (int b = st.b0; b < st.b1; ++b, u += 16) {
+#pragma unroll
+        for (int t = 0; t + 1 < NT; ++t) kf[t] = kf[t + 1];
+        kf[NT - 1] = kn;
+        const Rows<KC> qf = qn;
+        pa.next();
+        qn.load(pa, u + 16, st.Tr);
+        kn.load(pb, uk, st.Tr);
+        pb.next(); uk += 16;
+        const bool edge = 16 * b < gm.left || 16 * b + 15 + gm.win - 1 - gm.left >= st.Tr;
+#pragma unroll
+        for (int t = 0; t < NT; ++t) {
+            float s[2][4];
+            products<E, KC>(s[0], s[1], qf, kf[t]);
+#pragma unroll
+            for (int g = 0; g < 2; ++g)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int c = 16 * t + 8 * g + 2 * (lane & 3);
+                    float2 v = make_float2(s[g][2 * h], s[g][2 * h + 1]);
+                    if (edge) {   // a key outside the sequence gives 0 whatever the query holds
+                        const int j = 16 * b - gm.left + c;
+                        if ((unsigned)j >= (unsigned)st.Tr) v.x = 0.f;
+                        if ((unsigned)(j + 1) >= (unsigned)st.Tr) v.y = 0.f;
+                    }
+                    *reinterpret_cast<float2*>(patch + (fr + 8 * h) * kPatchPitch<NT> + c) = v;
+                }
+        }
+        __syncwarp();
+        const int live = min(16, st.Tr - 16 * b) * gm.win;
+#pragma unroll
+        for (int it = 0; it < kPatchIters<NT>; ++it)
+            if (it * 32 + lane < live) dst[it * 32 + lane] = patch[off[it]];
+        dst += 16 * gm.win;
+        __syncwarp();
+    }
+}
+
+// 16 result rows from `first` on, by plain fp32 sums: two lanes per row
+template <typename E, int KC, bool TRANSPOSED>
+__device__ __noinline__ void plain_rows16(E* out, const float* band, const E* x, int seq, int first, Geometry gm) {
+    const int lane = threadIdx.x & 31, row = first + (lane >> 1);
+    if (row < 0 || row >= gm.T) return;
+    for (int c0 = 8 * (lane & 1); c0 < 16 * KC; c0 += 16) {
+        float acc[8] = {};
+        for (int kk = 0; kk < gm.win; ++kk) {
+            const int w = TRANSPOSED ? row - (kk - gm.left) : row + kk - gm.left;
+            if (w < 0 || w >= gm.T) continue;
+            const float f = __ldg(band + ((long long)seq * gm.T + (TRANSPOSED ? w : row)) * gm.win + kk);
+            float v[8];
+            Cvt<E>::unpack(__ldg(reinterpret_cast<const uint4*>(x + ((long long)seq * gm.T + w) * (16 * KC) + c0)), v);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) acc[i] = fmaf(f, v[i], acc[i]);
+        }
+        *reinterpret_cast<uint4*>(out + ((long long)seq * gm.T + row) * (16 * KC) + c0) = Cvt<E>::pack(acc);
+    }
+}
+
+template <typename E, int KC, int NT, bool TRANSPOSED>
+__global__ void __launch_bounds__(kWarps * 32) march_rows_kernel(E* __restrict__ out, const float* __restrict__ band, const E* __restrict__ x, Strides sd,
+                                                                Geometry gm, MarchGeom mg) {
+    __shared__ float patch_all[kWarps][16 * kPatchPitch<NT>];
+    const int lane = threadIdx.x & 31, fr = lane >> 2;
+    const long long id = (long long)blockIdx.x * kWarps + (threadIdx.x >> 5);
+    Strip st;
+    if (id >= mg.total || !st.init(gm, mg, nullptr, id)) return;
+    float* patch = patch_all[threadIdx.x >> 5];
+    for (int i = lane; i < 16 * kPatchPitch<NT>; i += 32) patch[i] = 0.f;
+    int off[kPatchIters<NT>];
+    patch_offsets<NT>(off, gm.win, lane);
+    const int first = TRANSPOSED ? max(0, st.b0 - (NT - 1)) : st.b0, lead = TRANSPOSED ? 0 : gm.left;
+    // x: key tiles (AV), or the block's own rows (transposed)
+    Place<const E> px(x, sd, st.b, 0, 0, 1, 16 * first - lead, lane);
+    Place<E> po(out, sd, st.b, 0, 0, 1, 16 * first - (TRANSPOSED ? gm.left : 0), lane);
+    const float* src = band + ((long long)st.b * gm.T + 16 * first) * gm.win;
+    int u = 16 * first + fr, ux = u - lead;
+    float bn[kPatchIters<NT>];
+    auto load_band = [&](int b) {
+        const int live = min(16, st.Tr - 16 * b) * gm.win;
+#pragma unroll
+        for (int it = 0; it < kPatchIters<NT>; ++it) bn[it] = it * 32 + lane < live ? __ldg(src + it * 32 + lane) : 0.f;
+        src += 16 * gm.win;
+    };
+    Rows<KC> xn;
+    RowsT<KC> xt[TRANSPOSED ? 1 : NT];
+    float acc[TRANSPOSED ? NT : 1][KC][2][4];
+    constexpr int TILES = TRANSPOSED ? 1 : NT;
+#pragma unroll
+    for (int t = 0; t < TILES; ++t) {
+        xn.load(px, ux, st.Tr);
+        px.next(); ux += 16;
+        if (t + 1 < TILES) xt[t + 1].set(xn);
+    }
+    if constexpr (TRANSPOSED) {
+#pragma unroll
+        for (int t = 0; t + 1 < NT; ++t)
+#pragma unroll
+            for (int i = 0; i < 8 * KC; ++i) acc[t][i >> 3][(i >> 2) & 1][i & 3] = 0.f;
+    }
+    load_band(first);
+    auto finish = [&](int row0, const float (&r)[KC][2][4]) {   // row0: first row of the 16
+        float z = 0.f;
+#pragma unroll
+        for (int i = 0; i < 8 * KC; ++i) z = fmaf(r[i >> 3][(i >> 2) & 1][i & 3], 0.f, z);
+        if (__any_sync(0xffffffffu, z != 0.f)) plain_rows16<E, KC, TRANSPOSED>(out, band, x, st.b, row0, gm);
+        else store<E, KC>(po, row0 + fr, st.Tr, r, 1.f, 1.f);
+    };
+    __syncwarp();
+#pragma unroll 1
+    for (int b = first; b < st.b1; ++b, u += 16) {
+#pragma unroll
+        for (int t = 0; t + 1 < TILES; ++t) xt[t] = xt[t + 1];
+        xt[TILES - 1].set(xn);
+#pragma unroll
+        for (int it = 0; it < kPatchIters<NT>; ++it)
+            if (off[it] >= 0) patch[off[it]] = bn[it];
+        __syncwarp();
+        if (b + 1 < st.b1) {
+            load_band(b + 1);
+            xn.load(px, ux, st.Tr);
+            px.next(); ux += 16;
+        }
+#pragma unroll
+        for (int t = 0; t < NT; ++t) {
+            uint32_t hi[4], lo[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float2 p = *reinterpret_cast<const float2*>(patch + (fr + 8 * (i & 1)) * kPatchPitch<NT> + 16 * t + 8 * (i >> 1) + 2 * (lane & 3));
+                hi[i] = Cvt<E>::pack2(p.x, p.y);
+                const float hx = Cvt<E>::from_bits((unsigned short)(hi[i] & 0xffffu)), hy = Cvt<E>::from_bits((unsigned short)(hi[i] >> 16));
+                lo[i] = Cvt<E>::pack2(p.x - hx, p.y - hy);
+            }
+            if constexpr (TRANSPOSED) {
+                const uint32_t ht[4] = {transpose8(hi[0]), transpose8(hi[2]), transpose8(hi[1]), transpose8(hi[3])};
+                const uint32_t lt[4] = {transpose8(lo[0]), transpose8(lo[2]), transpose8(lo[1]), transpose8(lo[3])};
+                if (t + 1 == NT) accumulate<E, KC, true>(acc[t], ht, xt[0]); else accumulate<E, KC, false>(acc[t], ht, xt[0]);
+                accumulate<E, KC, false>(acc[t], lt, xt[0]);
+            } else {
+                if (t == 0) accumulate<E, KC, true>(acc[0], hi, xt[t]); else accumulate<E, KC, false>(acc[0], hi, xt[t]);
+                accumulate<E, KC, false>(acc[0], lo, xt[t]);
+            }
+        }
+        __syncwarp();
+        if (!TRANSPOSED || b >= st.b0) finish(16 * b - (TRANSPOSED ? gm.left : 0), acc[0]);
+        po.next();
+        if constexpr (TRANSPOSED) {
+#pragma unroll
+            for (int t = 0; t + 1 < NT; ++t)
+#pragma unroll
+                for (int i = 0; i < 8 * KC; ++i) acc[t][i >> 3][(i >> 2) & 1][i & 3] = acc[t + 1][i >> 3][(i >> 2) & 1][i & 3];
+        }
+    }
+    if constexpr (TRANSPOSED)
+        if (st.b1 == st.nb) {
+#pragma unroll
+            for (int t = 0; t + 1 < NT; ++t) {
+                finish(16 * (st.b1 + t) - gm.left, acc[t]);
+                po.next();
+            }
+        }
+}
+
 // Blocks per strip. A strip costs its blocks and `extra` blocks' worth of start-up (first loads; in the backward the recomputed
 // blocks), and the GPU runs `per_sm` warps of it per SM at a time: the number of strips per residue with the shortest
 // total is taken. Large batches get whole sequences, single utterances strips of one or two blocks.
@@ -453,20 +663,24 @@ MarchGeom march_geom(const Geometry& gm, int per_sm, int extra) {
 
 }  // namespace
 
-// 16-channel rows, windows up to 33 (three key tiles), any dilation, token count and number of heads; row steps within an int
-bool march_supports(const Geometry& gm) {
+// 16-channel rows (forward: 32 too; the backward's registers hold 16), windows up to 33 (three key tiles), any dilation, token
+// count and number of heads
+bool march_supports(const Geometry& gm, bool backward) {
     const long long nb = ((long long)gm.T + 15) / 16 + gm.dil;
-    return gm.C == 16 && gm.win <= 33 && (long long)gm.N * nb * 2 < (1ll << 31);
+    return (gm.C == 16 || (gm.C == 32 && !backward)) && gm.win <= 33 && (long long)gm.N * nb * 2 < (1ll << 31);
 }
 
 cudaError_t march_fused_fwd(void* o, float* lse, const void* q, const void* k, const void* v, const float* rpb, const int* valid_len,
                             const Strides& sq, const Strides& sk, const Strides& sv, const Strides& so, const Geometry& gm, int dtype, cudaStream_t st) {
     const MarchGeom m = march_geom(gm, 16, 1);
     const unsigned grid = (unsigned)((m.total + kWarps - 1) / kWarps);
-#define NA1D_MARCH(E, NT) march_fwd_kernel<E, 1, NT><<<grid, kWarps * 32, 0, st>>>((E*)o, lse, (const E*)q, (const E*)k, (const E*)v, rpb, valid_len, sq, sk, sv, so, gm, m)
-    if (dtype == 0) { if (gm.win <= 17) NA1D_MARCH(__nv_bfloat16, 2); else NA1D_MARCH(__nv_bfloat16, 3); }
-    else { if (gm.win <= 17) NA1D_MARCH(__half, 2); else NA1D_MARCH(__half, 3); }
+#define NA1D_MARCH(E, KC, NT) march_fwd_kernel<E, KC, NT><<<grid, kWarps * 32, 0, st>>>((E*)o, lse, (const E*)q, (const E*)k, (const E*)v, rpb, valid_len, sq, sk, sv, so, gm, m)
+#define NA1D_MARCH_E(E)                                                                 \
+    if (gm.C == 16) { if (gm.win <= 17) NA1D_MARCH(E, 1, 2); else NA1D_MARCH(E, 1, 3); } \
+    else { if (gm.win <= 17) NA1D_MARCH(E, 2, 2); else NA1D_MARCH(E, 2, 3); }
+    if (dtype == 0) { NA1D_MARCH_E(__nv_bfloat16) } else { NA1D_MARCH_E(__half) }
 #undef NA1D_MARCH
+#undef NA1D_MARCH_E
     return cudaGetLastError();
 }
 cudaError_t march_fused_bwd(void* dq, void* dk, void* dv, float* d_rpb, const void* d_o, const void* q, const void* k, const void* v, const float* lse,
@@ -479,6 +693,39 @@ cudaError_t march_fused_bwd(void* dq, void* dk, void* dv, float* d_rpb, const vo
                                                              rpb, valid_len, sdq, sdk, sdv, sdo, sq, sk, sv, gm, m)
     if (dtype == 0) { if (gm.win <= 17) NA1D_MARCH(__nv_bfloat16, 2); else NA1D_MARCH(__nv_bfloat16, 3); }
     else { if (gm.win <= 17) NA1D_MARCH(__half, 2); else NA1D_MARCH(__half, 3); }
+#undef NA1D_MARCH
+    return cudaGetLastError();
+}
+
+// the pair: 16, 32 or 64 channels, one head (sequences), dilation 1
+bool march_band_supports(const Geometry& gm) {
+    const long long nb = ((long long)gm.T + 15) / 16 + 1;
+    return (gm.C == 16 || gm.C == 32 || gm.C == 64) && gm.win <= 33 && gm.dil == 1 && gm.H == 1 && (long long)gm.N * nb * 2 < (1ll << 31) &&
+           (long long)gm.T * gm.win < (1ll << 31);
+}
+#define NA1D_MARCH_E(E)                                                                        \
+    if (gm.C == 16) { if (gm.win <= 17) NA1D_MARCH(E, 1, 2); else NA1D_MARCH(E, 1, 3); }        \
+    else if (gm.C == 32) { if (gm.win <= 17) NA1D_MARCH(E, 2, 2); else NA1D_MARCH(E, 2, 3); }   \
+    else { if (gm.win <= 17) NA1D_MARCH(E, 4, 2); else NA1D_MARCH(E, 4, 3); }
+cudaError_t march_band_out(float* band, const void* a, const void* b, const Geometry& gm, int dtype, cudaStream_t st) {
+    const MarchGeom m = march_geom(gm, 20, 1);
+    const unsigned grid = (unsigned)((m.total + kWarps - 1) / kWarps);
+    const Strides d = dense_strides(1, gm.T, gm.C);
+#define NA1D_MARCH(E, KC, NT) march_qk_kernel<E, KC, NT><<<grid, kWarps * 32, 0, st>>>(band, (const E*)a, (const E*)b, d, gm, m)
+    if (dtype == 0) { NA1D_MARCH_E(__nv_bfloat16) } else { NA1D_MARCH_E(__half) }
+#undef NA1D_MARCH
+    return cudaGetLastError();
+}
+cudaError_t march_band_rows(void* out, const float* band, const void* x, bool transposed, const Geometry& gm, int dtype, cudaStream_t st) {
+    const MarchGeom m = march_geom(gm, gm.C == 64 ? 12 : 20, transposed ? 3 : 1);
+    const unsigned grid = (unsigned)((m.total + kWarps - 1) / kWarps);
+    const Strides d = dense_strides(1, gm.T, gm.C);
+#define NA1D_MARCH(E, KC, NT)                                                                                                     \
+    do {                                                                                                                          \
+        if (transposed) march_rows_kernel<E, KC, NT, true><<<grid, kWarps * 32, 0, st>>>((E*)out, band, (const E*)x, d, gm, m);    \
+        else march_rows_kernel<E, KC, NT, false><<<grid, kWarps * 32, 0, st>>>((E*)out, band, (const E*)x, d, gm, m);              \
+    } while (0)
+    if (dtype == 0) { NA1D_MARCH_E(__nv_bfloat16) } else { NA1D_MARCH_E(__half) }
 #undef NA1D_MARCH
     return cudaGetLastError();
 }

@@ -137,11 +137,12 @@ def _pair_reference(q, k, attn, win, left, dil):
     return torch.einsum("ntc,ntwc->ntw", q.double(), kg), torch.einsum("ntw,ntwc->ntc", a, kg), out
 
 
-@pytest.mark.parametrize("family", [-1, 0, 3])
+@pytest.mark.parametrize("family", [-1, 0, 3, 4])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("N,T,C,win,left,dil", [(1, 1, 8, 1, 0, 1), (3, 128, 16, 27, 13, 1), (2, 129, 16, 5, 0, 1), (2, 150, 32, 33, 32, 1), (3, 97, 48, 41, 20, 1),
                                                 (2, 300, 64, 9, 4, 1), (2, 300, 64, 18, 4, 3), (1, 260, 128, 128, 64, 1), (2, 7, 24, 9, 4, 5),
-                                                (2, 40, 192, 12, 3, 1)])
+                                                (2, 40, 192, 12, 3, 1), (1, 1, 16, 33, 0, 1), (5, 31, 16, 17, 16, 1), (2, 1500, 16, 18, 2, 1),
+                                                (700, 150, 16, 1, 0, 1)])
 def test_unfused_operators(N, T, C, win, left, dil, dtype, family):
     """All routes of the six unfused entry points: fp32 results to fp32 accuracy (the band in), 16-bit results to their rounding --
     half a step, plus the tcgen05 kernels' 16-bit band, at most another half step per term."""
@@ -156,20 +157,21 @@ def test_unfused_operators(N, T, C, win, left, dil, dtype, family):
         ops.set_kernel_family(old)
     eps = 2.0 ** -9 if dtype == torch.bfloat16 else 2.0 ** -12      # half a rounding step
     for i, (a, r) in enumerate(zip(got, _pair_reference(q, k, attn, win, left, dil))):
-        rel = 2e-6 if i == 0 else eps * (1.1 if family >= 0 else 1.6)
+        rel = 2e-6 if i == 0 else eps * (1.1 if family in (0, 3, 4) else 1.6)
         assert float((a.double() - r).norm()) <= rel * float(r.norm()) + 1e-6, i
 
 
+@pytest.mark.parametrize("C,routes", [(48, (3, 0)), (16, (4, 0))])
 @pytest.mark.parametrize("value", [float("nan"), float("inf")])
-def test_unfused_operators_keep_bad_values_in_their_window(value):
+def test_unfused_operators_keep_bad_values_in_their_window(value, C, routes):
     from pcf_nat_b200 import ops
-    q, k, d_o, _, _, _ = _inputs((1, 1, 150, 48, 9, 4, 1, True, False), torch.bfloat16)
+    q, k, d_o, _, _, _ = _inputs((1, 1, 150, C, 9, 4, 1, True, False), torch.bfloat16)
     attn = torch.rand(1, 150, 9, device="cuda")
     for bad in (q, k, attn):
         x = [q.clone(), k.clone(), attn.clone()]
         x[[id(q), id(k), id(attn)].index(id(bad))][0, 70, 5] = value
         out = []
-        for family in (3, 0):
+        for family in routes:
             old = ops.set_kernel_family(family)
             try:
                 out.append([ops.qk_forward(x[0], x[1], 9, 4), ops.av_forward(x[2], x[1], 9, 4), ops.v_backward(x[2], x[0], 9, 4)])
