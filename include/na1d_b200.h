@@ -233,6 +233,9 @@ int na1d_column_sums(float* sums, float* scratch, const void* x, int64_t rows, i
 #define NA1D_CAST_MAX 16
 int na1d_cast_parameters(void* out, const float* const* src, const int64_t* dst, const int64_t* n, int count, int dtype,
                          void* stream);
+/* out[r * ld + c] = x[r, c] + dx[r, c] (dx may be NULL: a copy), 16-bit, rows of D inside wider rows of ld elements (multiples of
+ * 8): a stage's output written straight into its slice of the concatenated features (models/PCF_NATransformer.py:440-455). */
+int na1d_add_to_rows(void* out, int64_t ld, const void* x, const void* dx, int64_t rows, int64_t D, int dtype, void* stream);
 /* (N, C, T) -> (N, T, C) (to_tokens) or (N, T, C) -> (N, C, T), 16-bit; C a multiple of 8, the (N, T, C) side 16-byte aligned.
  * Replaces the transposing copies around the channels-first layer, models/PCF_NATransformer.py:126-151. */
 int na1d_transpose(void* out, const void* in, int64_t N, int64_t C, int64_t T, int to_tokens, int dtype, void* stream);
@@ -247,8 +250,8 @@ int na1d_pack_grouped(void* out_w, void* out_b, const void* w, const void* b, in
 int na1d_unpack_grouped(void* d_w, void* d_b, const float* dense, const float* sums, int dst32, int64_t C, int64_t groups, int parts,
                         int dtype, void* stream);
 /* out (N, 2C) fp32 = [mu, std] with a = softmax over T of logits (N, T, C), mu = sum a x, std = sqrt(max(sum a x^2 - mu^2,
- * floor)). stats (3, N, C), for the backward (may be NULL): the logits' maximum, 1 / sum exp, sum a x^2. N <= 65535. */
-int na1d_stats_pool_forward(float* out, float* stats, const void* logits, const void* x, int64_t N, int64_t T,
+ * floor)). x has rows of ldx >= C elements (a multiple of 8). stats (3, N, C), for the backward (may be NULL): the logits' maximum, 1 / sum exp, sum a x^2. N <= 65535. */
+int na1d_stats_pool_forward(float* out, float* stats, const void* logits, const void* x, int64_t ldx, int64_t N, int64_t T,
                             int64_t C, float floor, int dtype, void* stream);
 int na1d_stats_pool_backward(void* d_logits, void* dx, const float* d_out, const float* out, const float* stats,
                              const void* logits, const void* x, int64_t N, int64_t T, int64_t C,

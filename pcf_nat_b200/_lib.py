@@ -94,7 +94,8 @@ for _name, _args in (
         ("na1d_transpose", [_ptr, _ptr, _i64, _i64, _i64, _i32]),
         ("na1d_pack_grouped", [_ptr] * 4 + [_i32, _i64, _i64, _i32]),
         ("na1d_unpack_grouped", [_ptr] * 4 + [_i32, _i64, _i64, _i32]),
-        ("na1d_stats_pool_forward", [_ptr] * 4 + [_i64] * 3 + [_f32]),
+        ("na1d_add_to_rows", [_ptr, _i64, _ptr, _ptr, _i64, _i64]),
+        ("na1d_stats_pool_forward", [_ptr] * 4 + [_i64] * 4 + [_f32]),
         ("na1d_stats_pool_backward", [_ptr] * 7 + [_i64] * 3 + [_f32])):
     _f = getattr(_lib, _name)
     _f.restype = _i32

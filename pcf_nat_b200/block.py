@@ -95,6 +95,24 @@ def cast_parameters(params, dtype):
     return buf, offs
 
 
+def add_to_rows(out, x, dx=None):
+    """out = x (+ dx), x dense (batch, T, D), out a slice of D columns of wider rows."""
+    D = x.shape[-1]
+    with ops._on_device(x.device):
+        check(_L.na1d_add_to_rows(out.data_ptr(), out.stride(1), x.data_ptr(), None if dx is None else dx.data_ptr(), x.numel() // D, D,
+                                  _CODE[x.dtype], _stream(x)), "na1d_add_to_rows")
+    return out
+
+
+def feature_rows(x, parts):
+    """Room for ``parts`` tensors like the 16-bit CUDA tensor x (batch, T, D) side by side, or None where the stages cannot write
+    into slices of it (gradients are wanted, another kind of tensor)."""
+    if (type(x) is not torch.Tensor or not x.is_cuda or x.dtype not in _CODE or x.dim() != 3 or x.shape[-1] % 8 or torch.is_grad_enabled() or
+            x.numel() == 0 or torch.compiler.is_compiling() or not ops.native.eager_mode() or global_hooks()):
+        return None
+    return torch.empty(x.shape[0], x.shape[1], parts * x.shape[2], dtype=x.dtype, device=x.device)
+
+
 # ------------------------------------------------------------------ the block (its autograd node is in csrc/torch_nodes.cpp)
 def _block_parameters(blk, x):
     """The parameters of a block in the order of the node's arguments, or None where the block is anything but the plain one
@@ -122,9 +140,10 @@ def _block_parameters(blk, x):
     return ps
 
 
-def run_blocks(blocks, x, valid):
+def run_blocks(blocks, x, valid, out=None):
     """The blocks applied to the residual stream x (batch, T, D), or None where they have to run module by module.
-    ``valid``: valid tokens per utterance (int32, contiguous) or None."""
+    ``valid``: valid tokens per utterance (int32, contiguous) or None. ``out``: a slice of wider rows, (batch, T, D), that
+    takes the result (no gradients)."""
     if (type(x) is not torch.Tensor or not x.is_cuda or x.dim() != 3 or x.numel() == 0 or torch.compiler.is_compiling() or
             not torch.is_autocast_enabled() or not ops.native.eager_mode() or torch.autograd.forward_ad._current_level >= 0):
         return None
@@ -147,6 +166,8 @@ def run_blocks(blocks, x, valid):
         return None
     for ps, cfg, eps in plan:
         x, dx = ops.native.block(x, dx, valid, *cfg, *eps, ps)
+    if out is not None:
+        return add_to_rows(out, x, dx)
     return x if dx is None else x + dx
 
 
@@ -158,7 +179,7 @@ class _StatsPoolFunction(torch.autograd.Function):
         out = torch.empty((N, 2 * C), dtype=torch.float32, device=x.device)
         stats = torch.empty((3, N, C), dtype=torch.float32, device=x.device)
         with ops._on_device(x.device):
-            check(_L.na1d_stats_pool_forward(out.data_ptr(), stats.data_ptr(), logits.data_ptr(), x.data_ptr(), N, T, C, floor,
+            check(_L.na1d_stats_pool_forward(out.data_ptr(), stats.data_ptr(), logits.data_ptr(), x.data_ptr(), C, N, T, C, floor,
                                              _CODE[x.dtype], _stream(x)), "na1d_stats_pool_forward")
         ctx.save_for_backward(logits, x, out, stats)
         ctx.floor = floor
@@ -189,7 +210,17 @@ def stats_pool(logits, x, floor):
     N, T, C = x.shape
     if not 0 < N <= 65535 or not 0 < T <= 1 << 20 or C == 0 or C % 8 or C > 1 << 20:
         return None
-    logits, x = logits.contiguous(), x.contiguous()
+    logits = logits.contiguous()
+    if not torch.is_grad_enabled() and x.stride(2) == 1 and x.stride(0) == T * x.stride(1) and x.stride(1) % 8 == 0 and C <= x.stride(1) <= 1 << 20:
+        ld = x.stride(1)                     # a slice of wider rows is read in place
+    else:
+        x, ld = x.contiguous(), C
     if logits.data_ptr() % 16 or x.data_ptr() % 16:
         return None
+    if not torch.is_grad_enabled():
+        out = torch.empty((N, 2 * C), dtype=torch.float32, device=x.device)
+        with ops._on_device(x.device):
+            check(_L.na1d_stats_pool_forward(out.data_ptr(), None, logits.data_ptr(), x.data_ptr(), ld, N, T, C, floor, _CODE[x.dtype], _stream(x)),
+                  "na1d_stats_pool_forward")
+        return out
     return _StatsPoolFunction.apply(logits, x, floor)

@@ -523,13 +523,21 @@ int na1d_unpack_grouped(void* d_w, void* d_b, const float* dense, const float* s
     if (int s = check_grouped(C, groups, parts, dtype)) return s;
     return cuda_status(na1d::block_unpack_grouped(d_w, d_b, dense, sums, dst32 != 0, (int)C, (int)groups, parts, dtype, (cudaStream_t)stream));
 }
-int na1d_stats_pool_forward(float* out, float* stats, const void* logits, const void* x, int64_t N, int64_t T,
+int na1d_add_to_rows(void* out, int64_t ld, const void* x, const void* dx, int64_t rows, int64_t D, int dtype, void* stream) {
+    if (int s = check_pointers(out, x)) return s;
+    if (!aligned16(dx)) return NA1D_ERR_MISALIGNED;
+    if (int s = check_block(rows, D, 1 << 20, dtype)) return s;
+    if (ld < D || ld % 8 != 0 || rows > (1ll << 40) / ld) return NA1D_ERR_BAD_STRIDE;
+    return cuda_status(na1d::block_add_to_rows(out, ld, x, dx, (int)rows, (int)D, dtype, (cudaStream_t)stream));
+}
+int na1d_stats_pool_forward(float* out, float* stats, const void* logits, const void* x, int64_t ldx, int64_t N, int64_t T,
                             int64_t C, float floor, int dtype, void* stream) {
     if (int s = check_pointers(out, logits, x)) return s;
     if (!aligned16(stats)) return NA1D_ERR_MISALIGNED;
     if (int s = check_block(T, C, 1 << 20, dtype)) return s;
     if (N <= 0 || N > 65535 || T > (1 << 20)) return NA1D_ERR_BAD_SHAPE;
-    return cuda_status(na1d::block_pool_fwd(out, stats, logits, x, (int)N, (int)T, (int)C, floor, dtype, (cudaStream_t)stream));
+    if (ldx < C || ldx % 8 != 0 || ldx > (1 << 20)) return NA1D_ERR_BAD_STRIDE;
+    return cuda_status(na1d::block_pool_fwd(out, stats, logits, x, ldx, (int)N, (int)T, (int)C, floor, dtype, (cudaStream_t)stream));
 }
 int na1d_stats_pool_backward(void* d_logits, void* dx, const float* d_out, const float* out, const float* stats,
                              const void* logits, const void* x, int64_t N, int64_t T, int64_t C,

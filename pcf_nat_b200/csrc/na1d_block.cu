@@ -39,7 +39,7 @@ __device__ __forceinline__ void load8f(const float* p, float* f) {
 // ---------------------------------------------------------------- LayerNorm
 // y = LN(s) w + b with s = x, or s = round(x + dx) written to `sum` (the residual stream): one warp per row, the row stays in
 // registers (mean first, then the centred squares). 153600 rows of 256: 231 us (framework kernel) + 37 us (residual add)
-// before.
+// before, 53 us here (49 us of HBM time).
 template <typename E, int CH>
 __global__ void __launch_bounds__(kRowThreads) ln_fwd_kernel(E* __restrict__ y, E* __restrict__ sum, float* __restrict__ mean,
                                                              float* __restrict__ rstd, const E* __restrict__ x,
@@ -47,28 +47,40 @@ __global__ void __launch_bounds__(kRowThreads) ln_fwd_kernel(E* __restrict__ y, 
                                                              const float* __restrict__ b, int rows, int D, float eps) {
     const int lane = threadIdx.x & 31;
     const float inv_d = 1.f / (float)D;
-    for (int row = blockIdx.x * kWarps + (threadIdx.x >> 5); row < rows; row += gridDim.x * kWarps) {
+    // the next row's loads are in flight during a row's two reductions
+    uint4 nx[CH], nd[CH];
+    auto fetch = [&](int row) {
+#pragma unroll
+        for (int c = 0; c < CH; ++c) {
+            const int col = c * 256 + lane * 8;
+            nx[c] = nd[c] = make_uint4(0u, 0u, 0u, 0u);
+            if (row < rows && col < D) {
+                nx[c] = *reinterpret_cast<const uint4*>(x + (size_t)row * D + col);
+                if (dx) nd[c] = *reinterpret_cast<const uint4*>(dx + (size_t)row * D + col);
+            }
+        }
+    };
+    int row = blockIdx.x * kWarps + (threadIdx.x >> 5);
+    fetch(row);
+    for (; row < rows; row += gridDim.x * kWarps) {
         const size_t base = (size_t)row * D;
         float v[CH][8], s = 0.f;
 #pragma unroll
         for (int c = 0; c < CH; ++c) {
             const int col = c * 256 + lane * 8;
+            Cvt<E>::unpack(nx[c], v[c]);
+            if (dx) {
+                float r[8];
+                Cvt<E>::unpack(nd[c], r);
 #pragma unroll
-            for (int i = 0; i < 8; ++i) v[c][i] = 0.f;
-            if (col < D) {
-                load8(x + base + col, v[c]);
-                if (dx) {
-                    float r[8];
-                    load8(dx + base + col, r);
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) v[c][i] += r[i];
-                    round8<E>(v[c]);
-                    store8(sum + base + col, v[c]);
-                }
+                for (int i = 0; i < 8; ++i) v[c][i] += r[i];
+                round8<E>(v[c]);
+                if (col < D) store8(sum + base + col, v[c]);
             }
 #pragma unroll
             for (int i = 0; i < 8; ++i) s += v[c][i];
         }
+        fetch(row + gridDim.x * kWarps);
         const float mu = warp_sum(s) * inv_d;
         float q = 0.f;
 #pragma unroll
@@ -134,7 +146,8 @@ __global__ void __launch_bounds__(1024) partial_sum_kernel(float* __restrict__ o
 
 // dx = rstd (g - mean(g) - xhat mean(g xhat)) + res with g = dy w, and the column sums of dy xhat (weight gradient), dy (bias
 // gradient) and dx as stored (the bias gradient of the projection whose output was added to the residual stream).
-// 38400 rows of 256: 35 us (input gradient) + 173 us (parameter gradients) + 47 us (bias gradient) before.
+// 38400 rows of 256: 35 us (input gradient) + 173 us (parameter gradients) + 47 us (bias gradient) before, 22 us here (12 us of
+// HBM time; loading the next row ahead, as the forward does, measured 23 us).
 template <typename E, int CH>
 __global__ void __launch_bounds__(kRowThreads) ln_bwd_kernel(E* __restrict__ dx, float* __restrict__ part, const E* __restrict__ dy,
                                                              const E* __restrict__ x, const float* __restrict__ mean,
@@ -198,8 +211,8 @@ __global__ void __launch_bounds__(kRowThreads) ln_bwd_kernel(E* __restrict__ dx,
 // Phi(x) = erfc(-x / sqrt 2) / 2 from Abramowitz & Stegun 7.1.26 (erfc(z) = t (a1 + t (a2 + ...)) e^{-z^2}, t = 1 / (1 + p z),
 // z >= 0, |error| <= 1.5e-7): the negative tail is a product, not 1 - erf, so it keeps its relative accuracy, and e^{-x^2/2} is
 // shared with the density in the derivative. Two special-function operations and ~14 fp32 operations a value instead of the
-// library erff's ~25 with a branch, which is what bound the framework kernel (178 us for 153600 x 1024 values, 98 us of HBM
-// time).
+// library erff's ~25 with a branch, which is what bound the framework kernel (178 us for 153600 x 1024 values; 116 us here, 98 us
+// of HBM time).
 __device__ __forceinline__ void phi(float x, float& cdf, float& e) {
     const float z = fabsf(x) * 0.70710678118654752f;
     const float t = fast_rcp(fmaf(0.3275911f, z, 1.f));
@@ -239,7 +252,7 @@ __global__ void __launch_bounds__(256) gelu_fwd_kernel(E* __restrict__ y, const 
 }
 
 // Column sums of a (rows, F) matrix with leading dimension F; GELU: the matrix is dx = dy gelu'(x), which is written too
-// (38400 x 1024: 63 us backward + 47 us bias gradient before).
+// (38400 x 1024: 63 us backward + 47 us bias gradient before, 47 us here, 37 us of HBM time).
 // CTA (bx, by): columns 256 bx .. +255, rows by * 8 + warp, stepping by 8 gridDim.y.
 template <typename E, bool GELU>
 __global__ void __launch_bounds__(kRowThreads) column_kernel(E* __restrict__ dx, float* __restrict__ part, const E* __restrict__ dy,
@@ -248,7 +261,7 @@ __global__ void __launch_bounds__(kRowThreads) column_kernel(E* __restrict__ dx,
     float acc[1][1][8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) acc[0][0][i] = 0.f;
-    constexpr int U = GELU ? 2 : 4;
+    constexpr int U = 4;
     const int step = gridDim.y * kWarps;
     if (col < F)
         for (int row = blockIdx.y * kWarps + (threadIdx.x >> 5); row < rows; row += U * step) {
@@ -310,6 +323,27 @@ template <typename E> __global__ void __launch_bounds__(256) cast_kernel(E* __re
     *reinterpret_cast<uint4*>(out + L.dst[k] + i0) = Cvt<E>::pack(f);   // the slot of each tensor is padded to 8 elements
 }
 
+// out row r (ld elements apart) = x + dx: one 16-byte unit per thread and step
+template <typename E>
+__global__ void __launch_bounds__(256) add_to_rows_kernel(E* __restrict__ out, long long ld, const E* __restrict__ x, const E* __restrict__ dx, int D,
+                                                          long long chunks) {
+    const int per_row = D / 8;
+    const long long stride = (long long)gridDim.x * 256;
+    for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < chunks; i += stride) {
+        float a[8], b[8];
+        uint4 u = reinterpret_cast<const uint4*>(x)[i];
+        if (dx) {
+            Cvt<E>::unpack(u, a);
+            load8(dx + i * 8, b);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) a[k] += b[k];
+            u = Cvt<E>::pack(a);
+        }
+        const long long row = i / per_row;
+        *reinterpret_cast<uint4*>(out + row * ld + (i - row * per_row) * 8) = u;
+    }
+}
+
 // valid tokens of each utterance from its padding: one launch for what four elementwise ones did
 __global__ void __launch_bounds__(256) valid_tokens_kernel(int* __restrict__ out, const void* __restrict__ padding, bool is64, int n_padding, int N, int T) {
     const int i = blockIdx.x * 256 + threadIdx.x;
@@ -322,7 +356,7 @@ __global__ void __launch_bounds__(256) valid_tokens_kernel(int* __restrict__ out
 // ---------------------------------------------------------------- channels-first layers: transposes and grouped weights
 // A 64-channel x 64-token tile through shared memory. The token side is read or written in pairs (4 bytes) where the rows allow
 // it (an even token count, an even base), the channel side in 16-byte units; the odd pitch of 65 elements keeps both
-// phases free of bank conflicts. 512 x 256 x 150: 72 us per copy before, 12 us of HBM time.
+// phases free of bank conflicts. 512 x 256 x 150: 72 us per copy before, 15 to 25 us here, 12 us of HBM time.
 constexpr int kTile = 64, kTilePitch = 65;
 template <bool TO_TOKENS, bool PAIRS>
 __global__ void __launch_bounds__(256) transpose_kernel(uint16_t* __restrict__ out, const uint16_t* __restrict__ in, int C, int T) {
@@ -407,12 +441,12 @@ __global__ void __launch_bounds__(128) unpack_grouped_kernel(D* __restrict__ d_w
 // a = softmax over time of the logits; mu = sum a x, std = sqrt(max(sum a x^2 - mu^2, floor)), per channel. One pass: a lane
 // keeps the running maximum and the three sums of its 8 channels; the CTA's warps share the time axis and meet in shared
 // memory. Reads logits and x once (512 x 300 x 1536: 0.94 GB; the framework's chain of fp32 copies, strided softmax, products
-// and sums took 6.2 ms there).
+// and sums took 6.2 ms there; 0.24 ms here, 0.15 ms of HBM time).
 constexpr int kPoolWarps = 8;
 template <typename E>
 __global__ void __launch_bounds__(kPoolWarps * 32) pool_fwd_kernel(float* __restrict__ out, float* __restrict__ stats,
-                                                                  const E* __restrict__ logits, const E* __restrict__ x, int T, int C,
-                                                                  float floor_var) {
+                                                                  const E* __restrict__ logits, const E* __restrict__ x, long long ldx,
+                                                                  int T, int C, float floor_var) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, col = blockIdx.x * 256 + lane * 8;
     const size_t base = (size_t)blockIdx.y * T * C;
     float m[8], s[8], sx[8], sxx[8];
@@ -423,7 +457,7 @@ __global__ void __launch_bounds__(kPoolWarps * 32) pool_fwd_kernel(float* __rest
         for (int t = warp; t < T; t += kPoolWarps) {
             float l[8], v[8];
             load8(logits + base + (size_t)t * C + col, l);
-            load8(x + base + (size_t)t * C + col, v);
+            load8(x + ((size_t)blockIdx.y * T + t) * ldx + col, v);
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
                 const float z = l[i];
@@ -609,6 +643,13 @@ cudaError_t block_cast(void* out, const float* const* src, const int64_t* dst, c
     else cast_kernel<<<L.first[count], 256, 0, st>>>((__half*)out, L);
     return cudaGetLastError();
 }
+cudaError_t block_add_to_rows(void* out, long long ld, const void* x, const void* dx, int rows, int D, int dtype, cudaStream_t st) {
+    const long long chunks = (long long)rows * (D / 8), need = (chunks + 255) / 256, most = (long long)device_sm_count() * 16;
+    const int grid = (int)(need < most ? need : most);
+    if (dtype == 0) add_to_rows_kernel<<<grid, 256, 0, st>>>((__nv_bfloat16*)out, ld, (const __nv_bfloat16*)x, (const __nv_bfloat16*)dx, D, chunks);
+    else add_to_rows_kernel<<<grid, 256, 0, st>>>((__half*)out, ld, (const __half*)x, (const __half*)dx, D, chunks);
+    return cudaGetLastError();
+}
 cudaError_t block_transpose(void* out, const void* in, int N, int C, int T, bool to_tokens, int dtype, cudaStream_t st) {
     const dim3 grid((C + kTile - 1) / kTile, (T + kTile - 1) / kTile, N);
     const bool pairs = T % 2 == 0 && (reinterpret_cast<uintptr_t>(to_tokens ? in : out) & 3u) == 0;
@@ -639,11 +680,11 @@ cudaError_t block_unpack_grouped(void* d_w, void* d_b, const float* dense, const
     else unpack_grouped_kernel<<<rows, 128, 0, st>>>((__half*)d_w, (__half*)d_b, dense, sums, C, groups, parts);
     return cudaGetLastError();
 }
-cudaError_t block_pool_fwd(float* out, float* stats, const void* logits, const void* x, int N, int T, int C, float floor_var,
+cudaError_t block_pool_fwd(float* out, float* stats, const void* logits, const void* x, long long ldx, int N, int T, int C, float floor_var,
                            int dtype, cudaStream_t st) {
     const dim3 grid((C + 255) / 256, N);
-    if (dtype == 0) pool_fwd_kernel<<<grid, kPoolWarps * 32, 0, st>>>(out, stats, (const __nv_bfloat16*)logits, (const __nv_bfloat16*)x, T, C, floor_var);
-    else pool_fwd_kernel<<<grid, kPoolWarps * 32, 0, st>>>(out, stats, (const __half*)logits, (const __half*)x, T, C, floor_var);
+    if (dtype == 0) pool_fwd_kernel<<<grid, kPoolWarps * 32, 0, st>>>(out, stats, (const __nv_bfloat16*)logits, (const __nv_bfloat16*)x, ldx, T, C, floor_var);
+    else pool_fwd_kernel<<<grid, kPoolWarps * 32, 0, st>>>(out, stats, (const __half*)logits, (const __half*)x, ldx, T, C, floor_var);
     return cudaGetLastError();
 }
 cudaError_t block_pool_bwd(void* d_logits, void* dx, const float* d_out, const float* out, const float* stats,

@@ -103,7 +103,8 @@ cudaError_t block_pack_grouped(void* out_w, void* out_b, const void* w, const vo
                                cudaStream_t st);
 cudaError_t block_unpack_grouped(void* d_w, void* d_b, const float* dense, const float* sums, bool dst32, int C, int groups, int parts, int dtype,
                                  cudaStream_t st);
-cudaError_t block_pool_fwd(float* out, float* stats, const void* logits, const void* x, int N, int T, int C, float floor_var,
+cudaError_t block_add_to_rows(void* out, long long ld, const void* x, const void* dx, int rows, int D, int dtype, cudaStream_t st);
+cudaError_t block_pool_fwd(float* out, float* stats, const void* logits, const void* x, long long ldx, int N, int T, int C, float floor_var,
                            int dtype, cudaStream_t st);
 cudaError_t block_pool_bwd(void* d_logits, void* dx, const float* d_out, const float* out, const float* stats,
                            const void* logits, const void* x, int N, int T, int C, float floor_var, int dtype, cudaStream_t st);

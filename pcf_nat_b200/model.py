@@ -18,7 +18,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from . import block
-from .nattention import NAttention, _merge_heads, _split_heads, _valid_tokens
+from .nattention import NAttention, _merge_heads, _plain_linear, _split_heads, _valid_tokens
 from .nattn import getNA1dFunction
 
 
@@ -75,7 +75,9 @@ class AttentiveStatsPool(nn.Module):
         self.b = nn.Linear(bottleneck, dim)
 
     def forward(self, x):
-        logits = self.b(torch.tanh(self.a(x)))
+        # (as a matrix where the rows are slices of wider ones, which a GEMM reads in place)
+        h = self.a(x) if x.is_contiguous() else self.a(x.flatten(0, 1)).view(x.shape[0], x.shape[1], -1)
+        logits = self.b(torch.tanh(h))
         out = block.stats_pool(logits, x, 1e-5)
         if out is not None:
             return out
@@ -128,18 +130,31 @@ class PCFNATExtractor(nn.Module):
         valid = None
         if not self.training and padding is not None and x.is_cuda:
             valid = _valid_tokens(x.shape[1], padding, x.shape[0])
+        C = x.shape[-1]
+        # evaluation: the stages write into the concatenation themselves, the projections read it in place
+        plain = all(_plain_linear(m) for m in self.fuse) and type(self.pool) is AttentiveStatsPool and _plain_linear(self.pool.a)
+        rows = block.feature_rows(x, len(self.stages) + 1) if plain else None
         for s, stage in enumerate(self.stages):
-            y = block.run_blocks(stage, x, valid) if all(m.attn.training == self.training for m in stage) else None
+            out = None if rows is None else rows[..., (s + 1) * C:(s + 2) * C]
+            y = block.run_blocks(stage, x, valid, out) if all(m.attn.training == self.training for m in stage) else None
             if y is None:
+                rows = None
                 for blk in stage:
                     x = blk(x, padding)
             else:
+                if rows is not None and s == 0:
+                    block.add_to_rows(rows[..., :C], feats[0])
                 x = y
             outs.append(x)
             feats.append(x)
             if s + 1 < len(self.stages):
-                x = self.fuse[s](torch.cat(feats, dim=-1))
-        pooled = self.pool(torch.cat(outs, dim=-1))
+                if rows is None:
+                    x = self.fuse[s](torch.cat(feats, dim=-1))
+                else:
+                    x = self.fuse[s](rows.view(-1, rows.shape[-1])[:, :(s + 2) * C]).view(feats[0].shape)
+        return self._embed(self.pool(torch.cat(outs, dim=-1) if rows is None else rows[..., C:]))
+
+    def _embed(self, pooled):
         return self.embed(self.bn(pooled).to(self.embed.weight.dtype))
 
     def forward(self, fbank, labels, padding=None):

@@ -299,3 +299,39 @@ def test_layer_node_leaves_mixed_types_and_hooks_alone():
     with torch.autocast("cuda", dtype=torch.bfloat16):
         m(x)
     assert seen == [1]
+
+
+@pytest.mark.parametrize("dtype", DT)
+def test_rows_written_into_their_slice(dtype):
+    from pcf_nat_b200 import block
+    x, dx = _rand(3, 17, 72, dtype=dtype, seed=1), _rand(3, 17, 72, dtype=dtype, seed=2)
+    with torch.no_grad():
+        rows = block.feature_rows(x, 3)
+    rows.fill_(7.0)
+    block.add_to_rows(rows[..., 72:144], x, dx)
+    assert torch.equal(rows[..., 72:144], x + dx) and bool((rows[..., :72] == 7).all()) and bool((rows[..., 144:] == 7).all())
+    block.add_to_rows(rows[..., :72], x)
+    assert torch.equal(rows[..., :72], x)
+    logits = _rand(3, 17, 144, dtype=dtype, seed=3)
+    with torch.no_grad():
+        assert torch.equal(block.stats_pool(logits, rows[..., :144], 1e-5), block.stats_pool(logits, rows[..., :144].contiguous(), 1e-5))
+    assert block.feature_rows(x, 3) is None                     # gradients on: the stages' outputs stay tensors of their own
+
+
+def test_evaluation_with_shared_rows_gives_the_bits_of_separate_tensors(monkeypatch):
+    from pcf_nat_b200 import block
+    from pcf_nat_b200.model import PCFNATExtractor
+    torch.manual_seed(2)
+    m = PCFNATExtractor(frames=70, feat=24, dim=64, heads=2, win=7, stages=3, blocks=2, emb=32, classes=40).cuda().eval()
+    x = _rand(4, 24, 70, dtype=torch.float32, seed=1)
+    pad = torch.tensor([0, 3, 30, 7], device="cuda")
+    with torch.no_grad(), torch.autocast("cuda", dtype=torch.bfloat16):
+        a = m.embedding(x, pad)
+        monkeypatch.setattr(block, "feature_rows", lambda *_: None)
+        b = m.embedding(x, pad)
+        m.stages[1][0].fc1.register_forward_hook(lambda *_: None)      # a stage that runs module by module in between
+        monkeypatch.undo()
+        c = m.embedding(x, pad)
+    # (a GEMM on strided rows may pick another kernel: the last 16-bit rounding can differ)
+    for other in (a, c):
+        assert float((other.double() - b.double()).norm()) <= 2e-2 * float(b.double().norm())
