@@ -1,9 +1,9 @@
-// CUDA-core NA1D kernels: the general path (any window <= NA1D_MAX_WINDOW, any dilation, any
-// channel count the ABI accepts, bf16/fp16). A group of G lanes owns one sequence row; each lane
+// CUDA-core NA1D kernels: any window <= NA1D_MAX_WINDOW, any dilation, any channel count the ABI accepts, bf16/fp16;
+// automatic above 128 channels and where a row has few neighbours (na1d_api.cu has the rules). A group of G lanes owns one sequence row; each lane
 // holds CHUNKS 16-byte chunks of the row, interleaved so a group reads a row as one coalesced
 // segment. Dot products are reduced over the group with xor shuffles. All arithmetic is fp32.
 //
-// Replaces, for shapes the tensor-core kernels do not take: ana_qk_forward_kernel_C16/_C8
+// Replaces, for the shapes that run here: ana_qk_forward_kernel_C16/_C8
 // (na1d_tensorcore/bf16_ana1d_kernel.cu:42-282), ana_q_backward_kernel (:285-391) and
 // ana_k_backward_kernel (:394-492) of the reference, plus the eager softmax chain between them
 // (models/PCF_NATransformer.py:141-150).
