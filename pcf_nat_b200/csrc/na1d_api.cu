@@ -94,6 +94,9 @@ enum class Pass { forward, strided_forward, backward };
 template <typename... S> bool use_march(const na1d::Geometry& g, Pass pass, const S&... strides) {
     const int forced = g_family_override.load();
     if (forced != -1 && forced != 4 && !(forced == 2 && na1d::tc_seg_supports(g))) return false;
+    // (where the CUDA cores stood before -- more than 32 heads, residues of one token -- infinities and NaN stay in their windows: the
+    // general kernels see to that, these, like the tcgen05 ones, do not)
+    if (forced == -1 && !na1d::tc_seg_supports(g) && !na1d::tc_fwd_supports(g)) return false;
     if (forced == -1 && pass == Pass::forward && g.C == 32 && (long long)g.N * g.T > (1 << 18)) return false;
     return na1d::march_supports(g, pass == Pass::backward) && ((strides.token * g.dil < (1ll << 30)) && ...);
 }

@@ -20,9 +20,8 @@
 // Backward: key tile i collects from blocks i - NT + 1 .. i and is stored when block i is done. A strip owns the key tiles of its
 // own blocks and recomputes the NT - 1 blocks before it (nothing to recompute when the strip is a whole sequence).
 // Measured at 512 x 16 x 150 rows (tcgen05 flat / segmented tiling / here, us): window 27 forward 76 / 135 / 51, backward
-// 141 / 194 / 136; window 9 forward 62 / 104 / 40, backward 99 / 154 / 94; 64 x 16 x 997 rows, window 27: 66 / 66 / 41 and
-// 115 / 119 / 97. The forward is bound by instruction issue (0.67 a cycle), the backward by latency at the eight warps an SM
-// that its 225 registers leave (three CTAs an SM at 168 registers spill and are slower: 139).
+// 141 / 194 / 122; window 9 forward 62 / 104 / 40, backward 99 / 154 / 90; 64 x 16 x 997 rows, window 27: 66 / 66 / 37 and
+// 115 / 119 / 98. The forward is bound by instruction issue (0.67 a cycle), the backward by latency at twelve warps an SM.
 // Forward at 32 channels: 512 x 300 rows, window 27: 16 / 20 / 13; 4096 x 150: 49 / 85 / 51; the backward there needs more registers
 // than a thread has and stays on tcgen05 (82 / 107 against 118).
 // Rounding is that of the tcgen05 kernels: probabilities and dS enter the second products in 16 bits, sums are fp32.
@@ -255,12 +254,73 @@ __global__ void __launch_bounds__(kWarps * 32) march_fwd_kernel(E* __restrict__ 
     }
 }
 
-template <typename E, int KC, int NT>
-__global__ void __launch_bounds__(kWarps * 32) march_bwd_kernel(E* __restrict__ dq, E* __restrict__ dk, E* __restrict__ dv, float* __restrict__ d_rpb,
+// ---------------------------------------------------------------- backward, 16 channels
+// The forward's march with four tensors and two sets of key gradients in flight would take 225 registers and leave eight warps on an SM
+// (136 us at 512 x 16 x 150 rows, window 27, bound by latency). So the operands wait in shared memory instead: per warp a
+// ring of four key tiles each of k and v and two blocks each of q and d_o, copied asynchronously one step ahead (16 rows x 32
+// bytes: one 16-byte copy per lane), and read by ldmatrix, plain or transposed, where they are used.
+constexpr int kTileBytes = 16 * 32;
+struct WarpTiles {
+    uint32_t k, v, q, o;   // shared addresses: rings of 4, 4, 2, 2 tiles
+    uint32_t copy, plain, rows;   // this lane's offsets in a tile: its copy, its ldmatrix row as a right operand over channels, and as
+                                  // a left operand or a right operand over rows
+    __device__ __forceinline__ static uint32_t at(int row, int chunk) { return row * 32 + ((chunk ^ ((row >> 2) & 1)) << 4); }   // conflict-free
+    __device__ __forceinline__ WarpTiles(uint32_t base, int lane)
+        : k(base), v(base + 4 * kTileBytes), q(base + 8 * kTileBytes), o(base + 10 * kTileBytes), copy(at(lane >> 1, lane & 1)),
+          plain(at((lane & 7) + ((lane >> 4) << 3), (lane >> 3) & 1)), rows(at((lane & 7) + (((lane >> 3) & 1) << 3), lane >> 4)) {}
+};
+__device__ __forceinline__ void copy16(uint32_t dst, const void* src, bool in) {   // zeros where `in` is false
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(in ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void ldsm(uint32_t (&r)[4], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void ldsm_t(uint32_t (&r)[4], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+// acc (16 rows x channels 0-7, 8-15) = (FRESH ? 0 : acc) + w . x
+template <typename E, bool FRESH> __device__ __forceinline__ void add_rows(float (&acc)[2][4], const uint32_t (&w)[4], const uint32_t (&x)[4]) {
+    mma<E, FRESH>(acc[0], w[0], w[1], w[2], w[3], x[0], x[1]);
+    mma<E, FRESH>(acc[1], w[0], w[1], w[2], w[3], x[2], x[3]);
+}
+// a lane's place in an output: row l / 4 of the block, channels 2 (l % 4), + 1 of each half
+template <typename E> struct OutPlace {
+    E* p;
+    int step;
+    __device__ __forceinline__ OutPlace(E* base, const Strides& s, const Strip& st, int dil, int row, int lane)
+        : p(base + st.b * s.batch + st.h * s.head + st.r * s.token + (long long)(row + (lane >> 2)) * (s.token * dil) + 2 * (lane & 3)), step((int)s.token * dil) {}
+    __device__ __forceinline__ void next() { p += (long long)step * 16; }
+    __device__ __forceinline__ void store(int u, int Tr, const float (&acc)[2][4]) const {
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+            if ((unsigned)(u + 8 * h) < (unsigned)Tr) {
+                E* d = h ? p + (long long)step * 8 : p;
+                *reinterpret_cast<uint32_t*>(d) = Cvt<E>::pack2(acc[0][2 * h], acc[0][2 * h + 1]);
+                *reinterpret_cast<uint32_t*>(d + 8) = Cvt<E>::pack2(acc[1][2 * h], acc[1][2 * h + 1]);
+            }
+    }
+};
+// and in an input: row l / 2 of the block, channels 8 (l % 2) .. + 7
+template <typename E> struct InPlace {
+    const E* p;
+    int step;
+    __device__ __forceinline__ InPlace(const E* base, const Strides& s, const Strip& st, int dil, int row, int lane)
+        : p(base + st.b * s.batch + st.h * s.head + st.r * s.token + (long long)(row + (lane >> 1)) * (s.token * dil) + 8 * (lane & 1)), step((int)s.token * dil) {}
+    // copies the 16 rows, of which this lane's is row u of the residue, and moves on
+    __device__ __forceinline__ void copy(uint32_t dst, int u, int Tr, const E* safe) {
+        const bool in = (unsigned)u < (unsigned)Tr;
+        copy16(dst, in ? p : safe, in);
+        p += (long long)step * 16;
+    }
+};
+
+template <typename E, int NT>
+__global__ void __launch_bounds__(kWarps * 32, NT == 3 ? 3 : 4) march_bwd_kernel(E* __restrict__ dq, E* __restrict__ dk, E* __restrict__ dv, float* __restrict__ d_rpb,
                                                                const E* __restrict__ d_o, const E* __restrict__ q, const E* __restrict__ k,
                                                                const E* __restrict__ v, const float* __restrict__ lse, const float* __restrict__ rpb,
                                                                const int* __restrict__ valid_len, Strides sdq, Strides sdk, Strides sdv, Strides sdo,
                                                                Strides sq, Strides sk, Strides sv, Geometry gm, MarchGeom mg) {
+    __shared__ __align__(128) uint8_t tiles[kWarps][12 * kTileBytes];
     __shared__ float s_rpb[kWarps][16 * NT + 8];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, fr = lane >> 2, fa = 2 * (lane & 3) - fr;
     const long long id = (long long)blockIdx.x * kWarps + warp;
@@ -274,56 +334,66 @@ __global__ void __launch_bounds__(kWarps * 32) march_bwd_kernel(E* __restrict__ 
         load_bias<NT>(bias, rpb, st.h, gm.win, fa);
         const int right = gm.win - 1 - gm.left, first = max(0, st.b0 - (NT - 1));
         const float sc = gm.scale * kLog2e, mask2 = kMaskValue * kLog2e;
-        Place<const E> pq(q, sq, st.b, st.h, st.r, gm.dil, 16 * first, lane), po(d_o, sdo, st.b, st.h, st.r, gm.dil, 16 * first, lane),
-            pk(k, sk, st.b, st.h, st.r, gm.dil, 16 * first - gm.left, lane), pv(v, sv, st.b, st.h, st.r, gm.dil, 16 * first - gm.left, lane);
-        Place<E> pdq(dq, sdq, st.b, st.h, st.r, gm.dil, 16 * first, lane), pdk(dk, sdk, st.b, st.h, st.r, gm.dil, 16 * first - gm.left, lane),
-            pdv(dv, sdv, st.b, st.h, st.r, gm.dil, 16 * first - gm.left, lane);
+        const WarpTiles tl(ptx::smem_u32(tiles[warp]), lane);
+        InPlace<E> pq(q, sq, st, gm.dil, 16 * first, lane), po(d_o, sdo, st, gm.dil, 16 * first, lane), pk(k, sk, st, gm.dil, 16 * first - gm.left, lane),
+            pv(v, sv, st, gm.dil, 16 * first - gm.left, lane);
+        OutPlace<E> pdq(dq, sdq, st, gm.dil, 16 * first, lane), pdk(dk, sdk, st, gm.dil, 16 * first - gm.left, lane),
+            pdv(dv, sdv, st, gm.dil, 16 * first - gm.left, lane);
         const float* lp = lse + ((long long)st.b * gm.H + st.h) * gm.T + (long long)(16 * first + fr) * gm.dil + st.r;
-        int u = 16 * first + fr, uk = u - gm.left;   // this lane's first query row; its first row of the next key tile
-        Rows<KC> kf[NT], vf[NT], qn, on, kn, vn;
+        int u = 16 * first + fr;                        // this lane's first query row as an accumulator holds it
+        auto copy_queries = [&](int b) {
+            const int row = 16 * b + (lane >> 1);
+            pq.copy(tl.q + (b & 1) * kTileBytes + tl.copy, row, st.Tr, q);
+            po.copy(tl.o + (b & 1) * kTileBytes + tl.copy, row, st.Tr, d_o);
+        };
+        auto copy_keys = [&](int t) {
+            const int row = 16 * t - gm.left + (lane >> 1);
+            pk.copy(tl.k + (t & 3) * kTileBytes + tl.copy, row, st.Tr, k);
+            pv.copy(tl.v + (t & 3) * kTileBytes + tl.copy, row, st.Tr, v);
+        };
         float ln[2];
-        auto load_queries = [&](int row) {
-            qn.load(pq, row, st.Tr);
-            on.load(po, row, st.Tr);
-            // +inf for rows outside the sequence: probability 0
+        auto load_lse = [&](int row) {   // +inf for rows outside the sequence: probability 0
             ln[0] = row < st.Tr ? __ldg(lp) * kLog2e : INFINITY;
             ln[1] = row + 8 < st.Tr ? __ldg(lp + 8 * gm.dil) * kLog2e : INFINITY;
-            pq.next(); po.next(); lp += 16 * gm.dil;
+            lp += 16 * gm.dil;
         };
-        auto load_keys = [&]() {
-            kn.load(pk, uk, st.Tr);
-            vn.load(pv, uk, st.Tr);
-            pk.next(); pv.next(); uk += 16;
-        };
-        float ak[NT][KC][2][4], av[NT][KC][2][4];
+        float ak[NT][2][4], av[NT][2][4];
 #pragma unroll
         for (int t = 0; t + 1 < NT; ++t)
 #pragma unroll
-            for (int kc = 0; kc < KC; ++kc)
-#pragma unroll
-                for (int i = 0; i < 8; ++i) ak[t][kc][i >> 2][i & 3] = av[t][kc][i >> 2][i & 3] = 0.f;
-#pragma unroll
-        for (int t = 0; t < NT; ++t) {
-            load_keys();
-            if (t + 1 < NT) { kf[t + 1] = kn; vf[t + 1] = vn; }
-        }
-        load_queries(u);
+            for (int i = 0; i < 8; ++i) ak[t][i >> 2][i & 3] = av[t][i >> 2][i & 3] = 0.f;
+        for (int t = 0; t < NT; ++t) copy_keys(first + t);
+        copy_queries(first);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        load_lse(u);
 #pragma unroll 1
         for (int b = first; b < st.b1; ++b, u += 16) {
             const bool own = b >= st.b0;
-#pragma unroll
-            for (int t = 0; t + 1 < NT; ++t) { kf[t] = kf[t + 1]; vf[t] = vf[t + 1]; }
-            kf[NT - 1] = kn;
-            vf[NT - 1] = vn;
-            const Rows<KC> qf = qn, of = on;
             const float l2[2] = {ln[0], ln[1]};
-            load_queries(u + 16);
-            load_keys();
+            // the next block's rows (tile b + NT takes the slot of tile b + NT - 4, which the block before read last)
+            copy_queries(b + 1);
+            copy_keys(b + NT);
+            asm volatile("cp.async.commit_group;" ::: "memory");
+            load_lse(u + 16);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+            __syncwarp();
+            const uint32_t tq = tl.q + (b & 1) * kTileBytes, to = tl.o + (b & 1) * kTileBytes;
             float s[2 * NT][4], d[2 * NT][4], delta[2], part[2][4] = {};   // (two chains per row keep the sums short)
+            {
+                uint32_t qa[4], oa[4];
+                ldsm(qa, tq + tl.rows);
+                ldsm(oa, to + tl.rows);
 #pragma unroll
-            for (int t = 0; t < NT; ++t) {
-                products<E, KC>(s[2 * t], s[2 * t + 1], qf, kf[t]);
-                products<E, KC>(d[2 * t], d[2 * t + 1], of, vf[t]);
+                for (int t = 0; t < NT; ++t) {
+                    const uint32_t slot = ((b + t) & 3) * kTileBytes;
+                    uint32_t x[4];
+                    ldsm(x, tl.k + slot + tl.plain);
+                    mma<E, true>(s[2 * t], qa[0], qa[1], qa[2], qa[3], x[0], x[1]);
+                    mma<E, true>(s[2 * t + 1], qa[0], qa[1], qa[2], qa[3], x[2], x[3]);
+                    ldsm(x, tl.v + slot + tl.plain);
+                    mma<E, true>(d[2 * t], oa[0], oa[1], oa[2], oa[3], x[0], x[1]);
+                    mma<E, true>(d[2 * t + 1], oa[0], oa[1], oa[2], oa[3], x[2], x[3]);
+                }
             }
             const bool need_mask = 16 * b < gm.left || 16 * b + 15 + right >= st.vl;
 #pragma unroll
@@ -358,50 +428,49 @@ __global__ void __launch_bounds__(kWarps * 32) march_bwd_kernel(E* __restrict__ 
 #pragma unroll
                     for (int i = 0; i < 4; ++i) grad[2 * (g - (i >> 1) + 1) + (i & 1)] += d[g][i];
             }
-            RowsT<KC> qt, ot;
-            qt.set(qf);
-            ot.set(of);
-            float acc[KC][2][4];
+            uint32_t qt[4], ot[4];
+            ldsm_t(qt, tq + tl.rows);
+            ldsm_t(ot, to + tl.rows);
+            float acc[2][4];
 #pragma unroll
             for (int t = 0; t < NT; ++t) {
                 // left operands over the keys: (rows 0-7, keys 0-7), (rows 8-15, keys 0-7), (rows 0-7, keys 8-15), (rows 8-15, keys 8-15)
-                uint32_t w[4], x[4];
+                uint32_t w[4], x[4], kt[4];
+                ldsm_t(kt, tl.k + ((b + t) & 3) * kTileBytes + tl.rows);
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
                     const int g = 2 * t + (i >> 1), h = 2 * (i & 1);
                     w[i] = Cvt<E>::pack2(d[g][h] * gm.scale, d[g][h + 1] * gm.scale);
                     x[i] = Cvt<E>::pack2(s[g][h], s[g][h + 1]);
                 }
-                RowsT<KC> kt;
-                kt.set(kf[t]);
-                if (t == 0) accumulate<E, KC, true>(acc, w, kt); else accumulate<E, KC, false>(acc, w, kt);
+                if (t == 0) add_rows<E, true>(acc, w, kt); else add_rows<E, false>(acc, w, kt);
                 // and transposed, over the queries: the off-diagonal matrices change places
                 const uint32_t wt[4] = {transpose8(w[0]), transpose8(w[2]), transpose8(w[1]), transpose8(w[3])};
                 const uint32_t xt[4] = {transpose8(x[0]), transpose8(x[2]), transpose8(x[1]), transpose8(x[3])};
-                if (t + 1 == NT) { accumulate<E, KC, true>(ak[t], wt, qt); accumulate<E, KC, true>(av[t], xt, ot); }   // (the newest tile)
-                else { accumulate<E, KC, false>(ak[t], wt, qt); accumulate<E, KC, false>(av[t], xt, ot); }
+                if (t + 1 == NT) { add_rows<E, true>(ak[t], wt, qt); add_rows<E, true>(av[t], xt, ot); }   // (the newest tile)
+                else { add_rows<E, false>(ak[t], wt, qt); add_rows<E, false>(av[t], xt, ot); }
             }
+            __syncwarp();   // the slots are read: the next step's copies may overwrite them
             if (own) {
-                store<E, KC>(pdq, u, st.Tr, acc, 1.f, 1.f);
-                store<E, KC>(pdk, u - gm.left, st.Tr, ak[0], 1.f, 1.f);
-                store<E, KC>(pdv, u - gm.left, st.Tr, av[0], 1.f, 1.f);
+                pdq.store(u, st.Tr, acc);
+                pdk.store(u - gm.left, st.Tr, ak[0]);
+                pdv.store(u - gm.left, st.Tr, av[0]);
             }
             pdq.next(); pdk.next(); pdv.next();
 #pragma unroll
             for (int t = 0; t + 1 < NT; ++t)
 #pragma unroll
-                for (int kc = 0; kc < KC; ++kc)
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) {
-                        ak[t][kc][i >> 2][i & 3] = ak[t + 1][kc][i >> 2][i & 3];
-                        av[t][kc][i >> 2][i & 3] = av[t + 1][kc][i >> 2][i & 3];
-                    }
+                for (int i = 0; i < 8; ++i) {
+                    ak[t][i >> 2][i & 3] = ak[t + 1][i >> 2][i & 3];
+                    av[t][i >> 2][i & 3] = av[t + 1][i >> 2][i & 3];
+                }
         }
+        asm volatile("cp.async.wait_all;" ::: "memory");
         if (st.b1 == st.nb) {   // the sequence's last strip owns the tiles behind its last block too
 #pragma unroll
             for (int t = 0; t + 1 < NT; ++t) {
-                store<E, KC>(pdk, u - gm.left, st.Tr, ak[t], 1.f, 1.f);
-                store<E, KC>(pdv, u - gm.left, st.Tr, av[t], 1.f, 1.f);
+                pdk.store(u - gm.left, st.Tr, ak[t]);
+                pdv.store(u - gm.left, st.Tr, av[t]);
                 pdk.next(); pdv.next(); u += 16;
             }
         }
@@ -641,18 +710,18 @@ __global__ void __launch_bounds__(kWarps * 32) march_rows_kernel(E* __restrict__
         }
 }
 
-// Blocks per strip. A strip costs its blocks and `extra` blocks' worth of start-up (first loads; in the backward the recomputed
-// blocks), and the GPU runs `per_sm` warps of it per SM at a time: the number of strips per residue with the shortest
-// total is taken. Large batches get whole sequences, single utterances strips of one or two blocks.
-MarchGeom march_geom(const Geometry& gm, int per_sm, int extra) {
+// Blocks per strip. The GPU runs `resident` warps of the kernel per SM at a time, a strip costs its blocks and `extra` blocks' worth
+// of start-up (first loads; in the backward the recomputed blocks): the number of strips per residue whose rounds of warps
+// take the fewest block steps. Measured (backward, 1024 sequences of 63 blocks, 1776 warps at a time): 1 strip 111 us, 2 (one and
+// a bit rounds) 121, 3 (1.7 rounds) 98, 4 (2.3 rounds) 109.
+MarchGeom march_geom(const Geometry& gm, int resident, int extra) {
     MarchGeom m;
     const int nb = ((gm.T + gm.dil - 1) / gm.dil + 15) / 16, batch = gm.N / gm.H;
-    const long long residues = (long long)gm.N * gm.dil, room = (long long)per_sm * device_sm_count();
+    const long long residues = (long long)gm.N * gm.dil, room = (long long)resident * device_sm_count();
     long long best = 0;
     m.strips = 1;
     for (int s = 1; s <= nb; s += s < 16 ? 1 : s / 8) {
-        const long long warps = residues * s + room / 2;   // (half a round of them for the uneven end)
-        const long long cost = (warps < room ? room : warps) * ((nb + s - 1) / s + extra);
+        const long long cost = ((residues * s + room - 1) / room) * ((nb + s - 1) / s + extra);
         if (s == 1 || cost < best) { best = cost; m.strips = s; }
     }
     m.len = (nb + m.strips - 1) / m.strips;
@@ -660,6 +729,20 @@ MarchGeom march_geom(const Geometry& gm, int per_sm, int extra) {
     m.total = (long long)m.per_head * gm.H;
     return m;
 }
+
+// warps of a kernel that an SM holds (asked once per kernel)
+int resident_warps(const void* kern) {
+    int n = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, kWarps * 32, 0) != cudaSuccess || n < 1) n = 1;
+    return n * kWarps;
+}
+// launches kern<<<...>>>(arguments..., gm, m) with its own strips
+#define NA1D_MARCH_LAUNCH(EXTRA, KERN, ...)                                                          \
+    do {                                                                                             \
+        static const int warps = resident_warps(reinterpret_cast<const void*>(KERN));                \
+        const MarchGeom m = march_geom(gm, warps, EXTRA);                                            \
+        KERN<<<(unsigned)((m.total + kWarps - 1) / kWarps), kWarps * 32, 0, st>>>(__VA_ARGS__, gm, m); \
+    } while (0)
 
 }  // namespace
 
@@ -672,9 +755,8 @@ bool march_supports(const Geometry& gm, bool backward) {
 
 cudaError_t march_fused_fwd(void* o, float* lse, const void* q, const void* k, const void* v, const float* rpb, const int* valid_len,
                             const Strides& sq, const Strides& sk, const Strides& sv, const Strides& so, const Geometry& gm, int dtype, cudaStream_t st) {
-    const MarchGeom m = march_geom(gm, 16, 1);
-    const unsigned grid = (unsigned)((m.total + kWarps - 1) / kWarps);
-#define NA1D_MARCH(E, KC, NT) march_fwd_kernel<E, KC, NT><<<grid, kWarps * 32, 0, st>>>((E*)o, lse, (const E*)q, (const E*)k, (const E*)v, rpb, valid_len, sq, sk, sv, so, gm, m)
+#define NA1D_MARCH(E, KC, NT)                                                                                                                        \
+    NA1D_MARCH_LAUNCH(2, (march_fwd_kernel<E, KC, NT>), (E*)o, lse, (const E*)q, (const E*)k, (const E*)v, rpb, valid_len, sq, sk, sv, so)
 #define NA1D_MARCH_E(E)                                                                 \
     if (gm.C == 16) { if (gm.win <= 17) NA1D_MARCH(E, 1, 2); else NA1D_MARCH(E, 1, 3); } \
     else { if (gm.win <= 17) NA1D_MARCH(E, 2, 2); else NA1D_MARCH(E, 2, 3); }
@@ -686,11 +768,9 @@ cudaError_t march_fused_fwd(void* o, float* lse, const void* q, const void* k, c
 cudaError_t march_fused_bwd(void* dq, void* dk, void* dv, float* d_rpb, const void* d_o, const void* q, const void* k, const void* v, const float* lse,
                             const float* rpb, const int* valid_len, const Strides& sdq, const Strides& sdk, const Strides& sdv, const Strides& sdo,
                             const Strides& sq, const Strides& sk, const Strides& sv, const Geometry& gm, int dtype, cudaStream_t st) {
-    const MarchGeom m = march_geom(gm, gm.win <= 17 ? 12 : 8, gm.win <= 17 ? 2 : 3);
-    const unsigned grid = (unsigned)((m.total + kWarps - 1) / kWarps);
-#define NA1D_MARCH(E, NT)                                                                                                                             \
-    march_bwd_kernel<E, 1, NT><<<grid, kWarps * 32, 0, st>>>((E*)dq, (E*)dk, (E*)dv, d_rpb, (const E*)d_o, (const E*)q, (const E*)k, (const E*)v, lse, \
-                                                             rpb, valid_len, sdq, sdk, sdv, sdo, sq, sk, sv, gm, m)
+#define NA1D_MARCH(E, NT)                                                                                                                     \
+    NA1D_MARCH_LAUNCH(NT, (march_bwd_kernel<E, NT>), (E*)dq, (E*)dk, (E*)dv, d_rpb, (const E*)d_o, (const E*)q, (const E*)k, (const E*)v, lse, \
+                      rpb, valid_len, sdq, sdk, sdv, sdo, sq, sk, sv)
     if (dtype == 0) { if (gm.win <= 17) NA1D_MARCH(__nv_bfloat16, 2); else NA1D_MARCH(__nv_bfloat16, 3); }
     else { if (gm.win <= 17) NA1D_MARCH(__half, 2); else NA1D_MARCH(__half, 3); }
 #undef NA1D_MARCH
@@ -708,22 +788,18 @@ bool march_band_supports(const Geometry& gm) {
     else if (gm.C == 32) { if (gm.win <= 17) NA1D_MARCH(E, 2, 2); else NA1D_MARCH(E, 2, 3); }   \
     else { if (gm.win <= 17) NA1D_MARCH(E, 4, 2); else NA1D_MARCH(E, 4, 3); }
 cudaError_t march_band_out(float* band, const void* a, const void* b, const Geometry& gm, int dtype, cudaStream_t st) {
-    const MarchGeom m = march_geom(gm, 20, 1);
-    const unsigned grid = (unsigned)((m.total + kWarps - 1) / kWarps);
     const Strides d = dense_strides(1, gm.T, gm.C);
-#define NA1D_MARCH(E, KC, NT) march_qk_kernel<E, KC, NT><<<grid, kWarps * 32, 0, st>>>(band, (const E*)a, (const E*)b, d, gm, m)
+#define NA1D_MARCH(E, KC, NT) NA1D_MARCH_LAUNCH(2, (march_qk_kernel<E, KC, NT>), band, (const E*)a, (const E*)b, d)
     if (dtype == 0) { NA1D_MARCH_E(__nv_bfloat16) } else { NA1D_MARCH_E(__half) }
 #undef NA1D_MARCH
     return cudaGetLastError();
 }
 cudaError_t march_band_rows(void* out, const float* band, const void* x, bool transposed, const Geometry& gm, int dtype, cudaStream_t st) {
-    const MarchGeom m = march_geom(gm, gm.C == 64 ? 12 : 20, transposed ? 3 : 1);
-    const unsigned grid = (unsigned)((m.total + kWarps - 1) / kWarps);
     const Strides d = dense_strides(1, gm.T, gm.C);
-#define NA1D_MARCH(E, KC, NT)                                                                                                     \
-    do {                                                                                                                          \
-        if (transposed) march_rows_kernel<E, KC, NT, true><<<grid, kWarps * 32, 0, st>>>((E*)out, band, (const E*)x, d, gm, m);    \
-        else march_rows_kernel<E, KC, NT, false><<<grid, kWarps * 32, 0, st>>>((E*)out, band, (const E*)x, d, gm, m);              \
+#define NA1D_MARCH(E, KC, NT)                                                                                          \
+    do {                                                                                                               \
+        if (transposed) NA1D_MARCH_LAUNCH(NT, (march_rows_kernel<E, KC, NT, true>), (E*)out, band, (const E*)x, d);     \
+        else NA1D_MARCH_LAUNCH(2, (march_rows_kernel<E, KC, NT, false>), (E*)out, band, (const E*)x, d);                \
     } while (0)
     if (dtype == 0) { NA1D_MARCH_E(__nv_bfloat16) } else { NA1D_MARCH_E(__half) }
 #undef NA1D_MARCH
