@@ -127,7 +127,8 @@ def _fused_forward_channels_first_packed(self, x, valid_len):
     the merged heads (:151) and their autograd twins are gone, and so are the grouped convolutions. Measured at the
     reference's layer shape (512 x 150 frames, dim 256, 16 heads, window 27, groups 8; bf16 autocast, forward+backward):
     1.86 ms against 3.42 ms with convolutions and head split / merge copies around the dense operator (3.07 ms when the
-    transposes are instead absorbed by batched GEMMs on strided views: 512 small GEMMs and a batch-sized weight gradient)."""
+    transposes are instead absorbed by batched GEMMs on strided views: 512 small GEMMs and a batch-sized weight gradient). The C++ node of the same route
+    takes 0.52 ms there."""
     N, C, T = x.shape
     g = getattr(self, "groups", 1)
     if type(self.qkv) is nn.Conv1d and type(self.proj) is nn.Conv1d:
