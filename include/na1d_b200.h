@@ -239,6 +239,10 @@ int na1d_add_to_rows(void* out, int64_t ld, const void* x, const void* dx, int64
 /* (N, C, T) -> (N, T, C) (to_tokens) or (N, T, C) -> (N, C, T), 16-bit; C a multiple of 8, the (N, T, C) side 16-byte aligned.
  * Replaces the transposing copies around the channels-first layer, models/PCF_NATransformer.py:126-151. */
 int na1d_transpose(void* out, const void* in, int64_t N, int64_t C, int64_t T, int to_tokens, int dtype, void* stream);
+/* (batch, T, parts, heads, C) -> (parts, batch, heads, T, C) (to_dense) or back, 16-bit, C a multiple of 8: the head split and merge
+ * around the dense entry points (models/PCF_NATransformer.py:126-138, 151) for shapes the strided ones do not take. */
+int na1d_permute_heads(void* out, const void* in, int64_t batch, int64_t T, int64_t parts, int64_t heads, int64_t C, int to_dense,
+                       void* stream);
 /* A grouped 1x1 convolution (models/PCF_NATransformer.py:66-68) as one dense matrix: w (parts*C, C/groups) and b (parts*C or
  * NULL), fp32 (src32) or 16-bit, to out_w (parts*C, C) and out_b, 16-bit, zeros outside the group's columns. parts = 3 orders
  * the rows as (q|k|v, head, channel): row which*C + f is output channel ((f % (C/groups))*groups + f / (C/groups))*3 + which, the

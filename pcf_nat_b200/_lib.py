@@ -80,6 +80,8 @@ _lib.na1d_fused_forward_strided.restype = _i32
 _lib.na1d_fused_forward_strided.argtypes = [_ptr] * 7 + [_ptr] * 4 + [_i64] * 7 + [_f32, _i32, _ptr]
 _lib.na1d_fused_backward_strided.restype = _i32
 _lib.na1d_fused_backward_strided.argtypes = [_ptr] * 12 + [_i64] + [_ptr] * 7 + [_i64] * 7 + [_f32, _i32, _ptr]
+_lib.na1d_permute_heads.restype = _i32
+_lib.na1d_permute_heads.argtypes = [_ptr, _ptr] + [_i64] * 5 + [_i32, _ptr]
 _lib.na1d_valid_tokens.restype = _i32
 _lib.na1d_valid_tokens.argtypes = [_ptr, _ptr, _i32, _i64, _i64, _i64, _ptr]
 _lib.na1d_block_scratch_floats.restype = _i64

@@ -507,6 +507,14 @@ int na1d_transpose(void* out, const void* in, int64_t N, int64_t C, int64_t T, i
     if (N <= 0 || N > 65535 || T > (1 << 20)) return NA1D_ERR_BAD_SHAPE;
     return cuda_status(na1d::block_transpose(out, in, (int)N, (int)C, (int)T, to_tokens != 0, dtype, (cudaStream_t)stream));
 }
+int na1d_permute_heads(void* out, const void* in, int64_t batch, int64_t T, int64_t parts, int64_t heads, int64_t C, int to_dense,
+                       void* stream) {
+    if (int s = check_pointers(out, in)) return s;
+    if (batch <= 0 || T <= 0 || parts <= 0 || heads <= 0 || heads > 65535 || C <= 0 || C % 8 != 0 || C > 4096 || parts > 16 || batch > (1 << 26) ||
+        T * C / 8 > INT_MAX / 2 || T > INT_MAX / 8 || batch * parts > INT_MAX)
+        return NA1D_ERR_BAD_SHAPE;
+    return cuda_status(na1d::block_permute_heads(out, in, (int)batch, (int)T, (int)parts, (int)heads, (int)C, to_dense != 0, (cudaStream_t)stream));
+}
 static int check_grouped(int64_t C, int64_t groups, int parts, int dtype) {
     if (dtype != NA1D_BF16 && dtype != NA1D_FP16) return NA1D_ERR_BAD_DTYPE;
     if (C <= 0 || C % 8 != 0 || C > 8192 || groups <= 0 || C % groups != 0 || (parts != 1 && parts != 3)) return NA1D_ERR_BAD_SHAPE;

@@ -413,6 +413,22 @@ __global__ void __launch_bounds__(256) transpose_kernel(uint16_t* __restrict__ o
     }
 }
 
+// Head split or merge: CTA (x, h, z) moves 256 of the T * C / 8 16-byte units of head h of part-and-batch z; the dense side is
+// contiguous, the packed side comes in pieces of C channels.
+__global__ void __launch_bounds__(256) permute_heads_kernel(uint4* __restrict__ out, const uint4* __restrict__ in, int batch, int T, int parts, int heads,
+                                                           int units, bool to_dense) {
+    const int i = blockIdx.x * 256 + threadIdx.x, h = blockIdx.y;
+    if (i >= T * units) return;
+    const int t = i / units, c = i - t * units;
+    for (int z = blockIdx.z; z < batch * parts; z += gridDim.z) {
+        const int p = z / batch, b = z - p * batch;
+        const long long dense = ((long long)z * heads + h) * T * units + i;
+        const long long packed = ((((long long)b * T + t) * parts + p) * heads + h) * units + c;
+        if (to_dense) out[dense] = __ldg(in + packed);
+        else out[packed] = __ldg(in + dense);
+    }
+}
+
 // convolution output channel of row r of the dense matrix
 __device__ __forceinline__ int grouped_channel(int r, int C, int groups, int parts) {
     if (parts == 1) return r;
@@ -648,6 +664,12 @@ cudaError_t block_add_to_rows(void* out, long long ld, const void* x, const void
     const int grid = (int)(need < most ? need : most);
     if (dtype == 0) add_to_rows_kernel<<<grid, 256, 0, st>>>((__nv_bfloat16*)out, ld, (const __nv_bfloat16*)x, (const __nv_bfloat16*)dx, D, chunks);
     else add_to_rows_kernel<<<grid, 256, 0, st>>>((__half*)out, ld, (const __half*)x, (const __half*)dx, D, chunks);
+    return cudaGetLastError();
+}
+cudaError_t block_permute_heads(void* out, const void* in, int batch, int T, int parts, int heads, int C, bool to_dense, cudaStream_t st) {
+    const int units = C / 8, z = batch * parts;
+    const dim3 grid((T * units + 255) / 256, heads, z < 32768 ? z : 32768);
+    permute_heads_kernel<<<grid, 256, 0, st>>>((uint4*)out, (const uint4*)in, batch, T, parts, heads, units, to_dense);
     return cudaGetLastError();
 }
 cudaError_t block_transpose(void* out, const void* in, int N, int C, int T, bool to_tokens, int dtype, cudaStream_t st) {

@@ -98,6 +98,7 @@ cudaError_t block_gelu_fwd(void* y, const void* x, long long n, int dtype, cudaS
 cudaError_t block_gelu_bwd(void* dx, float* sums, float* part, const void* dy, const void* x, int rows, int F, int dtype, cudaStream_t st);
 cudaError_t block_column_sums(float* sums, float* part, const void* x, int rows, int F, int dtype, cudaStream_t st);
 cudaError_t block_cast(void* out, const float* const* src, const int64_t* dst, const int64_t* n, int count, int dtype, cudaStream_t st);
+cudaError_t block_permute_heads(void* out, const void* in, int batch, int T, int parts, int heads, int C, bool to_dense, cudaStream_t st);
 cudaError_t block_transpose(void* out, const void* in, int N, int C, int T, bool to_tokens, int dtype, cudaStream_t st);
 cudaError_t block_pack_grouped(void* out_w, void* out_b, const void* w, const void* b, bool src32, int C, int groups, int parts, int dtype,
                                cudaStream_t st);

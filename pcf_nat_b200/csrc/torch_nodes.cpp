@@ -531,16 +531,35 @@ struct ProjectionGrads {
               "na1d_unpack_grouped");
     }
 };
-struct LayerState { Tensor xt, qkv, lse, o, qw, pw; };
+// Shapes that the strided entry points do not take (a head size outside theirs, no shared memory left for the bias gradient): the
+// heads are split and merged by one copy each around the dense ones.
+bool takes_packed(const Packed& c, const Tensor& like) {
+    return na1d_fused_strided_supported(c.H, c.T, c.C, c.win, c.left, c.dil, code(like), 1, 1) == 1;
+}
+Tensor heads_moved(const Tensor& in, const Packed& c, int64_t parts, bool to_dense) {
+    Tensor out = to_dense ? at::empty({parts, c.B * c.H, c.T, c.C}, in.options()) : at::empty({c.B, c.T, parts * c.H * c.C}, in.options());
+    check(na1d_permute_heads(ptr(out), ptr(in), c.B, c.T, parts, c.H, c.C, to_dense, stream()), "na1d_permute_heads");
+    return out;
+}
+Cfg dense_cfg(const Packed& c) { return Cfg{c.B * c.H, c.T, c.C, c.H, c.win, c.left, c.dil, c.scale, 0.0, 0}; }
+// qkv: packed, or (dense) the split one; o_dense: the dense route's own output
+struct LayerState { Tensor xt, qkv, lse, o, qw, pw, o_dense; };
 Tensor layer_forward(const Tensor& x, const LayerShape& l, const Tensor& vl, const Tensor& r, const Tensor& qw, const OptTensor& qb, const Tensor& pw,
                      const OptTensor& pb, const Packed& c, LayerState* keep) {
     const LayerWeights w(x, l, qw, qb, pw, pb);
     LayerState s;
     s.xt = l.first ? transposed(x, l, true) : x;
     s.qkv = project(s.xt.view({l.rows(), l.D}), w.qw, w.qb).view({l.B, l.T, 3 * l.D});
-    s.o = at::empty({l.B, l.T, l.D}, x.options());
     if (keep) s.lse = empty_f32({l.B * c.H, l.T}, x);
-    packed_forward(s.o, s.lse, s.qkv, r, vl, c);
+    if (takes_packed(c, x)) {
+        s.o = at::empty({l.B, l.T, l.D}, x.options());
+        packed_forward(s.o, s.lse, s.qkv, r, vl, c);
+    } else {
+        s.qkv = heads_moved(s.qkv, c, 3, true);
+        s.o_dense = at::empty({c.B * c.H, c.T, c.C}, x.options());
+        op_forward(s.o_dense, s.lse, s.qkv.select(0, 0), s.qkv.select(0, 1), s.qkv.select(0, 2), r, vl, dense_cfg(c));
+        s.o = heads_moved(s.o_dense, c, 1, false);
+    }
     Tensor y = project(s.o.view({l.rows(), l.D}), w.pw, w.pb);
     y = l.first ? transposed(y, l, false) : y.view({l.B, l.T, l.D});
     if (keep) { s.qw = w.qw; s.pw = w.pw; *keep = std::move(s); }
@@ -554,7 +573,7 @@ struct NA1dLayer : public torch::autograd::Function<NA1dLayer> {
         const Packed c(l.B, l.T, l.D, heads, win, left, dil, scale);
         LayerState s;
         Tensor y = layer_forward(x, l, vl ? *vl : Tensor(), rpb32(rpb), qw, qb, pw, pb, c, &s);
-        ctx->save_for_backward({s.xt, s.qkv, s.lse, s.o, s.qw, s.pw, rpb, vl ? *vl : Tensor()});
+        ctx->save_for_backward({s.xt, s.qkv, s.lse, s.o, s.qw, s.pw, rpb, vl ? *vl : Tensor(), s.o_dense});
         auto& d = ctx->saved_data;
         d["first"] = first; d["heads"] = heads; d["groups"] = groups; d["win"] = win; d["left"] = left; d["dil"] = dil; d["scale"] = scale;
         d["qb"] = qb.has_value(); d["pb"] = pb.has_value();
@@ -563,9 +582,9 @@ struct NA1dLayer : public torch::autograd::Function<NA1dLayer> {
     }
     static variable_list backward(AutogradContext* ctx, variable_list grads) {
         const variable_list s = ctx->get_saved_variables();
-        const Tensor &xt = s[0], &qkv = s[1], &lse = s[2], &o = s[3], &qw = s[4], &pw = s[5], &rpb = s[6], &vl = s[7];
+        const Tensor &xt = s[0], &qkv = s[1], &lse = s[2], &o = s[3], &qw = s[4], &pw = s[5], &rpb = s[6], &vl = s[7], &o_dense = s[8];
         auto& d = ctx->saved_data;
-        const Packed c(qkv, d["heads"].toInt(), d["win"].toInt(), d["left"].toInt(), d["dil"].toInt(), d["scale"].toDouble());
+        const Packed c(xt.size(0), xt.size(1), xt.size(2), d["heads"].toInt(), d["win"].toInt(), d["left"].toInt(), d["dil"].toInt(), d["scale"].toDouble());
         LayerShape l(xt, false, d["groups"].toInt());
         l.first = d["first"].toBool();
         const c10::cuda::CUDAGuard guard(qkv.device());
@@ -579,7 +598,17 @@ struct NA1dLayer : public torch::autograd::Function<NA1dLayer> {
                            d["pw_shape"].toIntVector(), type, l, 1);
         Tensor d_qkv = at::empty_like(qkv), d_rpb, d_x;
         if (ctx->needs_input_grad(1)) d_rpb = at::zeros({c.H, c.win}, xt.options().dtype(at::kFloat));
-        packed_backward(d_qkv, d_rpb, at::mm(dy, pw), qkv, lse, rpb32(rpb), vl, c);
+        if (o_dense.defined()) {
+            const Tensor d_o = heads_moved(at::mm(dy, pw), c, 1, true), delta = empty_f32({c.B * c.H, c.T}, xt), r = rpb32(rpb);
+            auto part = [](const Tensor& t, int i) { return ptr(t.select(0, i)); };
+            check(na1d_fused_backward(part(d_qkv, 0), part(d_qkv, 1), part(d_qkv, 2), fptr(d_rpb), ptr(d_o), part(qkv, 0), part(qkv, 1), part(qkv, 2),
+                                      ptr(o_dense), fptr(lse), fptr(r), static_cast<int32_t*>(ptr(vl)), fptr(delta), c.B * c.H, c.H, c.T, c.C, c.win,
+                                      c.left, c.dil, (float)c.scale, code(qkv), stream()),
+                  "na1d_fused_backward");
+            d_qkv = heads_moved(d_qkv, c, 3, false);
+        } else {
+            packed_backward(d_qkv, d_rpb, at::mm(dy, pw), qkv, lse, rpb32(rpb), vl, c);
+        }
         const Tensor dq = d_qkv.view({l.rows(), 3 * l.D});
         ProjectionGrads gq(ctx->needs_input_grad(2), has_qb && ctx->needs_input_grad(qb_edge), dq, xt.view({l.rows(), l.D}), scratch,
                            d["qw_shape"].toIntVector(), type, l, 3);

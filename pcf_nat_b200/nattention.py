@@ -105,8 +105,8 @@ def _native_layer(self, x, channels_first, groups, valid_len):
                             self.num_heads, groups, self.win_size, self.left, self.dilation, float(self.scale), valid_len)
 
 
-def _plain_linear(m):
-    return type(m) is nn.Linear and "forward" not in m.__dict__ and not hooked(m)
+def _plain_linear(m, kind=nn.Linear):
+    return type(m) is kind and "forward" not in m.__dict__ and not hooked(m)
 
 
 def hooked(m):
@@ -181,10 +181,11 @@ def _fused_forward(self, x, padding=None):
         if dt in (torch.bfloat16, torch.float16) and ops.packed_supported(self.num_heads, T, hd, self.win_size, self.left,
                                                                          self.dilation, dt):
             return _fused_forward_channels_first_packed(self, x, valid_len)
-    if (layout == "channels_last" and not drop_p and type(x) is torch.Tensor and x.is_cuda and not torch.compiler.is_compiling() and
-            _plain_linear(self.qkv) and _plain_linear(self.proj) and not global_hooks() and
-            ops.packed_supported(self.num_heads, T, hd, self.win_size, self.left, self.dilation, x.dtype)):
-        y = _native_layer(self, x, False, 1, valid_len)
+    kind = nn.Conv1d if layout == "channels_first" else nn.Linear
+    if (not drop_p and type(x) is torch.Tensor and x.is_cuda and not torch.compiler.is_compiling() and _plain_linear(self.qkv, kind) and
+            _plain_linear(self.proj, kind) and not global_hooks()):
+        # one C++ node; for shapes the packed route does not take it splits and merges the heads itself
+        y = _native_layer(self, x, layout == "channels_first", getattr(self, "groups", 1), valid_len)
         if y is not None:
             return self.proj_drop(y)
     qkv = self.qkv(x)

@@ -245,7 +245,7 @@ def test_transpose(N, C, T, dtype):
 @pytest.mark.parametrize("autocast", [True, False])
 @pytest.mark.parametrize("layout,groups,dim,heads,T,bias", [("channels_first", 8, 128, 8, 150, True), ("channels_first", 1, 64, 1, 77, False),
                                                             ("channels_first", 2, 192, 4, 65, True), ("channels_last", 1, 256, 8, 51, True),
-                                                            ("channels_last", 1, 64, 2, 64, False)])
+                                                            ("channels_last", 1, 64, 2, 64, False), ("channels_last", 1, 96, 2, 53, True)])
 def test_layer_node_against_the_layer_in_fp32(layout, groups, dim, heads, T, bias, autocast):
     """Output and every gradient of the layer in 16 bits against its own parameters and input in 64 bits: four rounding steps of
     the intermediate tensors, relative to each result."""
@@ -261,8 +261,10 @@ def test_layer_node_against_the_layer_in_fp32(layout, groups, dim, heads, T, bia
     dy = _rand(*x.shape, dtype=dt, seed=2)
     with torch.autocast("cuda", dtype=torch.bfloat16, enabled=autocast):
         y = m(x)
-    # (sizes the packed route does not take run module by module, as before)
-    assert ("NA1dLayer" in y.grad_fn.name()) == ops.packed_supported(heads, T, dim // heads, 9, 4, 1, dt)
+    # (48 and 64 channels, 65 and 77 tokens, below: one size the packed route takes in each layout, one it does not)
+    assert "NA1dLayer" in y.grad_fn.name()
+    if dim // heads == 48:
+        assert not ops.packed_supported(heads, T, 48, 9, 4, 1, dt)
     ps = dict(m.named_parameters())
     got = [y.detach()] + list(torch.autograd.grad(y, [x] + list(ps.values()), dy))
     w = {n: p.detach().double().cpu().requires_grad_() for n, p in ps.items()}
@@ -283,6 +285,18 @@ def test_layer_node_against_the_layer_in_fp32(layout, groups, dim, heads, T, bia
     for name, a, r in zip(["y", "x"] + list(w), got, want):
         assert a.shape == r.shape and a.dtype == (dt if name in ("y", "x") or not autocast else torch.float32)
         assert float((a.double().cpu() - r).norm()) <= 4 * EPS[dt] * float(r.norm()) + 1e-6, name
+
+
+@pytest.mark.parametrize("B,T,parts,H,C", [(1, 1, 1, 1, 8), (2, 65, 3, 4, 48), (3, 7, 1, 5, 128), (2, 300, 3, 2, 64)])
+def test_permute_heads(B, T, parts, H, C):
+    from pcf_nat_b200 import ops
+    x = _rand(B, T, parts, H, C, dtype=torch.bfloat16, seed=1)
+    y, z = torch.empty(parts, B, H, T, C, device="cuda", dtype=x.dtype), torch.empty_like(x)
+    s = torch.cuda.current_stream().cuda_stream
+    assert ops._L.na1d_permute_heads(y.data_ptr(), x.data_ptr(), B, T, parts, H, C, 1, s) == 0
+    assert torch.equal(y, x.permute(2, 0, 3, 1, 4))
+    assert ops._L.na1d_permute_heads(z.data_ptr(), y.data_ptr(), B, T, parts, H, C, 0, s) == 0
+    assert torch.equal(z, x)
 
 
 def test_layer_node_leaves_mixed_types_and_hooks_alone():
