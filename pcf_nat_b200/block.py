@@ -142,7 +142,7 @@ def _block_parameters(blk, x):
 
 def run_blocks(blocks, x, valid, out=None):
     """The blocks applied to the residual stream x (batch, T, D), or None where they have to run module by module.
-    ``valid``: valid tokens per utterance (int32, contiguous) or None. ``out``: a slice of wider rows, (batch, T, D), that
+    ``valid``: valid tokens per utterance (an integer tensor on any device) or None. ``out``: a slice of wider rows, (batch, T, D), that
     takes the result (no gradients)."""
     if (type(x) is not torch.Tensor or not x.is_cuda or x.dim() != 3 or x.numel() == 0 or torch.compiler.is_compiling() or
             not torch.is_autocast_enabled() or not ops.native.eager_mode() or torch.autograd.forward_ad._current_level >= 0):
@@ -164,8 +164,13 @@ def run_blocks(blocks, x, valid, out=None):
     x, dx = x.contiguous(), None
     if x.data_ptr() % 16:
         return None
+    if valid is not None:
+        valid = valid.to(device=x.device, dtype=torch.int32)      # (one copy for all blocks)
     for ps, cfg, eps in plan:
-        x, dx = ops.native.block(x, dx, valid, *cfg, *eps, ps)
+        y = ops.native.block(x, dx, valid, *cfg, *eps, ps)
+        if y is None:                                             # (the first block, or none: they are given the same lengths)
+            return None
+        x, dx = y
     if out is not None:
         return add_to_rows(out, x, dx)
     return x if dx is None else x + dx

@@ -446,14 +446,17 @@ struct NA1dBlock : public torch::autograd::Function<NA1dBlock> {
     }
 };
 
-std::pair<Tensor, Tensor> block(const Tensor& x, const OptTensor& dx, const OptTensor& vl, int64_t heads, int64_t win, int64_t left, double scale,
-                                double eps1, double eps2, const std::vector<Tensor>& p) {
+// nothing where the valid lengths are not of a form the kernels can be given (on another device, or of another integer type, they are
+// converted)
+std::optional<std::pair<Tensor, Tensor>> block(const Tensor& x, const OptTensor& dx, OptTensor vl, int64_t heads, int64_t win, int64_t left, double scale,
+                                               double eps1, double eps2, const std::vector<Tensor>& p) {
     TORCH_CHECK(p.size() == kParams, "a block has 13 parameters");
     const c10::cuda::OptionalCUDAGuard guard(x.device());
+    if (!prepare_valid(vl, x.size(0), x)) return std::nullopt;
     if (at::GradMode::is_enabled()) {
         const variable_list r = NA1dBlock::apply(x, dx, vl, heads, win, left, scale, eps1, eps2, p[0], p[1], p[2], p[3], p[4], p[5], p[6], p[7], p[8],
                                                  p[9], p[10], p[11], p[12]);
-        return {r[0], r[1]};
+        return std::make_pair(r[0], r[1]);
     }
     const Packed c(x.size(0), x.size(1), x.size(2), heads, win, left, 1, scale);
     return block_forward(x, dx ? *dx : Tensor(), vl ? *vl : Tensor(), c, eps1, eps2, p.data(), nullptr);

@@ -349,3 +349,25 @@ def test_evaluation_with_shared_rows_gives_the_bits_of_separate_tensors(monkeypa
     # (a GEMM on strided rows may pick another kernel: the last 16-bit rounding can differ)
     for other in (a, c):
         assert float((other.double() - b.double()).norm()) <= 2e-2 * float(b.double().norm())
+
+
+def test_padding_lengths_may_live_on_the_host():
+    """Lengths on the host or of another integer type give the bits of int32 lengths on the device, in the blocks and in the
+    whole network; lengths for another number of utterances are left to the modules, which refuse them."""
+    from pcf_nat_b200 import block
+    from pcf_nat_b200.model import PCFNATExtractor
+    st = _stage(64, 2, 50).eval()
+    x = _rand(3, 50, 64, dtype=torch.bfloat16, seed=1)
+    valid = torch.tensor([50, 17, 0], dtype=torch.int32)
+    with torch.no_grad(), torch.autocast("cuda", dtype=torch.bfloat16):
+        want = block.run_blocks(st, x, valid.cuda())
+        assert not torch.equal(want, block.run_blocks(st, x, None))
+        for v in (valid, valid.long(), valid.long().cuda(), valid.repeat_interleave(2)[::2]):
+            assert torch.equal(block.run_blocks(st, x, v), want)
+        assert block.run_blocks(st, x, valid[:2]) is None
+    torch.manual_seed(2)
+    m = PCFNATExtractor(frames=70, feat=24, dim=64, heads=2, win=7, stages=2, blocks=1, emb=32, classes=40).cuda().eval()
+    fbank, pad = _rand(4, 24, 70, dtype=torch.float32, seed=1), torch.tensor([0, 3, 30, 7])
+    with torch.no_grad(), torch.autocast("cuda", dtype=torch.bfloat16):
+        assert torch.equal(m.embedding(fbank, pad), m.embedding(fbank, pad.cuda()))
+        assert not torch.equal(m.embedding(fbank, pad), m.embedding(fbank))
