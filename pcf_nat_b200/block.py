@@ -117,6 +117,9 @@ def feature_rows(x, parts):
 def _block_parameters(blk, x):
     """The parameters of a block in the order of the node's arguments, or None where the block is anything but the plain one
     on fp32 parameters (a replaced or hooked submodule, another dtype, an odd size): it then runs module by module."""
+    from .model import NABlock       # (model.py imports this module)
+    if type(blk) is not NABlock:     # a subclass or a wrapper has a forward of its own
+        return None
     a, n1, n2, f1, f2 = blk.attn, blk.norm1, blk.norm2, blk.fc1, blk.fc2
     if type(a) is not NAttention or type(n1) is not nn.LayerNorm or type(n2) is not nn.LayerNorm or a._na1d_layout != "channels_last":
         return None
@@ -140,10 +143,10 @@ def _block_parameters(blk, x):
     return ps
 
 
-def run_blocks(blocks, x, valid, out=None):
+def run_blocks(blocks, x, valid, out=None, training=None):
     """The blocks applied to the residual stream x (batch, T, D), or None where they have to run module by module.
     ``valid``: valid tokens per utterance (an integer tensor on any device) or None. ``out``: a slice of wider rows, (batch, T, D), that
-    takes the result (no gradients)."""
+    takes the result (no gradients). ``training``: the state every layer has to be in, where ``valid`` depends on it."""
     if (type(x) is not torch.Tensor or not x.is_cuda or x.dim() != 3 or x.numel() == 0 or torch.compiler.is_compiling() or
             not torch.is_autocast_enabled() or not ops.native.eager_mode() or torch.autograd.forward_ad._current_level >= 0):
         return None
@@ -154,7 +157,7 @@ def run_blocks(blocks, x, valid, out=None):
     plan = []
     for blk in blocks:
         ps = _block_parameters(blk, x)
-        if ps is None:
+        if ps is None or training is not None and blk.attn.training != training:
             return None
         a = blk.attn
         C = D // a.num_heads

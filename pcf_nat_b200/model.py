@@ -136,7 +136,7 @@ class PCFNATExtractor(nn.Module):
         rows = block.feature_rows(x, len(self.stages) + 1) if plain else None
         for s, stage in enumerate(self.stages):
             out = None if rows is None else rows[..., (s + 1) * C:(s + 2) * C]
-            y = block.run_blocks(stage, x, valid, out) if all(m.attn.training == self.training for m in stage) else None
+            y = block.run_blocks(stage, x, valid, out, self.training)
             if y is None:
                 rows = None
                 for blk in stage:

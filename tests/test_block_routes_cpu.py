@@ -1,0 +1,36 @@
+"""Which blocks the one-node route takes (host-only decisions), and that every other block runs its own forward."""
+import torch
+import torch.nn as nn
+
+from pcf_nat_b200 import block
+from pcf_nat_b200.model import NABlock, PCFNATExtractor
+
+
+class _Scaled(NABlock):
+    def forward(self, x, padding=None):
+        return x + 0.5 * (super().forward(x, padding) - x)
+
+
+def _taken(cls=NABlock, change=lambda b: b):
+    blk = change(cls(40, 64, 2, 7, 4, "fused"))
+    return block._block_parameters(blk, torch.zeros(2, 40, 64)) is not None
+
+
+def test_only_the_plain_block_is_taken():
+    from torch.distributed.algorithms._checkpoint.checkpoint_wrapper import checkpoint_wrapper
+    assert _taken()
+    assert not _taken(_Scaled)
+    assert not _taken(change=checkpoint_wrapper)
+    assert not _taken(change=lambda b: nn.Sequential(b))
+
+
+def test_blocks_without_the_attributes_of_the_plain_one_run():
+    class Half(nn.Module):
+        def forward(self, x, padding=None):
+            return 0.5 * x
+
+    m = PCFNATExtractor(frames=30, feat=8, dim=32, heads=2, win=7, stages=2, blocks=1, emb=16, classes=10).eval()
+    for s in m.stages:
+        s[0] = Half()
+    with torch.no_grad():
+        assert m.embedding(torch.randn(2, 8, 30), torch.tensor([0, 3])).shape == (2, 16)
