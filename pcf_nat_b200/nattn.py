@@ -26,7 +26,7 @@ def _make_pair(tag, dtype):
     class QK(torch.autograd.Function):
         @classmethod
         def apply(cls, q, k, win_size, left, dilation=1):
-            if _plain(q, k):     # the same through the C++ node; None for what that leaves to this class
+            if cls is QK and _plain(q, k):     # the same through the C++ node; None for what that leaves to this class
                 out = ops.native.qk(q, k, win_size, left, dilation, bf16)
                 if out is not None:
                     return out
@@ -52,7 +52,7 @@ def _make_pair(tag, dtype):
     class AV(torch.autograd.Function):
         @classmethod
         def apply(cls, attn, v, win_size, left, dilation=1):
-            if _plain(attn, v):
+            if cls is AV and _plain(attn, v):
                 out = ops.native.av(attn, v, win_size, left, dilation, bf16)
                 if out is not None:
                     return out

@@ -175,3 +175,23 @@ def test_valid_tokens():
         want = (50 - pad.to(torch.int64)).clamp_(0, 50).to(torch.int32).expand(4)
         got = _valid_tokens(50, pad.cuda(), 4)
         assert got.dtype == torch.int32 and got.is_contiguous() and torch.equal(got.cpu(), want)
+
+
+def test_subclasses_of_the_pair_run_their_own_forward():
+    from pcf_nat_b200 import getNA1dFunction
+    q, k, v, _, _ = _args()
+    QK, AV = getNA1dFunction(32, 1, torch.bfloat16)
+
+    class Twice(QK):
+        @staticmethod
+        def forward(ctx, *a):
+            return 2 * QK.forward(ctx, *a)
+
+    class TwiceAV(AV):
+        @staticmethod
+        def forward(ctx, *a):
+            return 2 * AV.forward(ctx, *a)
+
+    attn = QK.apply(q, k, 7, 3)
+    assert torch.equal(Twice.apply(q, k, 7, 3), 2 * attn)
+    assert torch.equal(TwiceAV.apply(attn, v, 7, 3), 2 * AV.apply(attn, v, 7, 3))
