@@ -128,7 +128,9 @@ def _block_parameters(blk, x):
     mods = (blk, a, n1, n2, f1, f2, a.qkv, a.proj, a.attn_drop, a.proj_drop)
     if any(hooked(m) for m in mods) or any("forward" in m.__dict__ for m in mods):
         return None
-    if a.training and (a.attn_drop.p or a.proj_drop.p) or a.dilation != 1 or type(a.attn_drop) is not nn.Dropout or type(a.proj_drop) is not nn.Dropout:
+    if type(a.attn_drop) is not nn.Dropout or type(a.proj_drop) is not nn.Dropout or a.dilation != 1:
+        return None
+    if a.training and a.attn_drop.p or a.proj_drop.training and a.proj_drop.p:     # (each by the flag that its dropout follows)
         return None
     ps = (a.qkv.weight, a.qkv.bias, a.proj.weight, a.proj.bias, f1.weight, f1.bias, f2.weight, f2.bias, n1.weight, n1.bias, n2.weight,
           n2.bias, a.relative_position_bias)

@@ -34,3 +34,19 @@ def test_blocks_without_the_attributes_of_the_plain_one_run():
         s[0] = Half()
     with torch.no_grad():
         assert m.embedding(torch.randn(2, 8, 30), torch.tensor([0, 3])).shape == (2, 16)
+
+
+def test_dropout_follows_the_flag_of_its_own_module():
+    def set_(attn=0.0, proj=0.0, training=False, proj_training=False):
+        def change(b):
+            b.train(training)
+            b.attn.attn_drop.p, b.attn.proj_drop.p = attn, proj
+            b.attn.proj_drop.train(proj_training)
+            return b
+        return change
+
+    assert _taken(change=set_(attn=0.1, proj=0.1))                      # evaluation: neither is applied
+    assert not _taken(change=set_(proj=0.1, proj_training=True))        # evaluation with the dropout modules in training mode
+    assert not _taken(change=set_(attn=0.1, training=True))             # the layer's own flag decides about attention dropout
+    assert not _taken(change=set_(proj=0.1, training=True, proj_training=True))
+    assert _taken(change=set_(proj=0.1, training=True))
