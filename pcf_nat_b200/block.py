@@ -182,6 +182,29 @@ def run_blocks(blocks, x, valid, out=None, training=None):
 
 
 # ------------------------------------------------------------------ statistics pooling
+def weighted_stats(logits, x, floor):
+    """The pooling in PyTorch's operations."""
+    w = torch.softmax(logits.float(), dim=1)
+    xf = x.float()
+    mu = (w * xf).sum(1)
+    var = (w * xf * xf).sum(1) - mu * mu
+    return torch.cat([mu, var.clamp_min(floor).sqrt()], dim=1)
+
+
+def _pool_gradients(logits, x, d_out, floor):
+    """The backward pass in PyTorch's operations, for a backward that is differentiated again (create_graph)."""
+    w = torch.softmax(logits.float(), dim=1)
+    xf = x.float()
+    mu, e2 = (w * xf).sum(1, keepdim=True), (w * xf * xf).sum(1, keepdim=True)
+    var = e2 - mu * mu
+    d_mu, d_std = d_out.unsqueeze(1).chunk(2, dim=-1)
+    d_var = torch.where(var < floor, 0.0, 0.5 * d_std / var.clamp_min(floor).sqrt())
+    d_mu = d_mu - 2 * mu * d_var
+    q = xf * (d_mu + xf * d_var)
+    d_logits = w * (q - (mu * d_mu + e2 * d_var))
+    return d_logits.to(logits.dtype), (w * (d_mu + 2 * xf * d_var)).to(x.dtype)
+
+
 class _StatsPoolFunction(torch.autograd.Function):
     @staticmethod
     def forward(ctx, logits, x, floor):
@@ -198,6 +221,8 @@ class _StatsPoolFunction(torch.autograd.Function):
     @staticmethod
     def backward(ctx, d_out):
         logits, x, out, stats = ctx.saved_tensors
+        if torch.is_grad_enabled():
+            return _pool_gradients(logits, x, d_out, ctx.floor) + (None,)
         N, T, C = x.shape
         d_out = d_out.contiguous()
         if d_out.data_ptr() % 16:

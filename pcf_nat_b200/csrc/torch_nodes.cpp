@@ -295,6 +295,33 @@ OptTensor packed(const Tensor& qkv, int64_t heads, int64_t win, int64_t left, in
     return o;
 }
 
+// ---------------------------------------------------------------- backward passes that are differentiated again
+// Under create_graph a backward has to be differentiable itself, and the kernels' results are not. There a node with more in it than
+// the attention takes its branch again in PyTorch's operations (the attention as the operator's own node, whose gradients are
+// constants to a second pass) and differentiates that. The inputs come from what the node saved, and stand in the graph where the
+// node's own inputs do; each behind an alias, at which the inner pass ends.
+Tensor stand_in(const Tensor& data, size_t edge) {
+    const torch::autograd::Edge& e = torch::autograd::get_current_node()->next_edge(edge);
+    const Tensor t = data.detach();
+    if (!e.is_valid()) return t;
+    torch::autograd::impl::set_gradient_edge(t, e);
+    return at::alias(t);
+}
+// gradients of `outputs` with respect to the stand-ins, undefined for those whose input wants none
+variable_list inner_gradients(const variable_list& outputs, const variable_list& inputs, const variable_list& grads) {
+    variable_list out, in, g;
+    for (size_t i = 0; i < outputs.size(); ++i)
+        if (grads[i].defined()) { out.push_back(outputs[i]); g.push_back(grads[i]); }
+    for (const Tensor& t : inputs)
+        if (t.defined() && t.requires_grad()) in.push_back(t);
+    variable_list result(inputs.size());
+    if (out.empty() || in.empty()) return result;
+    const variable_list found = torch::autograd::grad(out, in, g, true, true, true);
+    for (size_t i = 0, k = 0; i < inputs.size(); ++i)
+        if (inputs[i].defined() && inputs[i].requires_grad()) result[i] = found[k++];
+    return result;
+}
+
 // ---------------------------------------------------------------- the transformer block
 // Parameters in the order qkv.w, qkv.b, proj.w, proj.b, fc1.w, fc1.b, fc2.w, fc2.b, norm1.w, norm1.b, norm2.w, norm2.b, bias table.
 constexpr int kProj = 8, kParams = 13;
@@ -389,10 +416,28 @@ struct NA1dBlock : public torch::autograd::Function<NA1dBlock> {
         const Packed c(x.size(0), x.size(1), x.size(2), heads, win, left, 1, scale);
         BlockState st;
         auto out = block_forward(x, dx ? *dx : Tensor(), vl ? *vl : Tensor(), c, eps1, eps2, p, &st);
-        ctx->save_for_backward({st.s1, st.st1, st.h1, st.qkv, st.lse, st.o, st.s2, st.st2, st.h2, st.f, st.g, st.buf, p8, p10, p12, vl ? *vl : Tensor()});
+        ctx->save_for_backward({st.s1, st.st1, st.h1, st.qkv, st.lse, st.o, st.s2, st.st2, st.h2, st.f, st.g, st.buf, p8, p10, p12, vl ? *vl : Tensor(), p9, p11});
         auto& d = ctx->saved_data;
-        d["heads"] = heads; d["win"] = win; d["left"] = left; d["scale"] = scale; d["dx"] = dx.has_value();
+        d["heads"] = heads; d["win"] = win; d["left"] = left; d["scale"] = scale; d["dx"] = dx.has_value(); d["eps1"] = eps1; d["eps2"] = eps2;
         return {out.first, out.second};
+    }
+    // x, dx, then the parameters; w: the 16-bit ones
+    static variable_list differentiable(const variable_list& s, const Packed& c, const Projections& w, double eps1, double eps2, bool has_dx, int first,
+                                        const variable_list& grads) {
+        const Tensor &s1 = s[0], &vl = s[15];
+        const int64_t D = s1.size(2);
+        const auto half = s1.scalar_type();
+        variable_list in = {stand_in(s1, 0), has_dx ? stand_in(at::zeros_like(s1), 1) : Tensor()};
+        for (int i = 0; i < kProj; ++i) in.push_back(stand_in(w.t[i].to(at::kFloat), first + i));
+        const int norms[5] = {12, 16, 13, 17, 14};   // n1w, n1b, n2w, n2b, bias table among the saved tensors
+        for (int i = 0; i < 5; ++i) in.push_back(stand_in(s[norms[i]], first + kProj + i));
+        const Tensor* p = &in[2];
+        auto linear = [&](const Tensor& x, int i) { return at::linear(x, p[i].to(half), p[i + 1].to(half)); };
+        auto norm = [&](const Tensor& x, int i, double eps) { return at::layer_norm(x.to(at::kFloat), {D}, p[i], p[i + 1], eps).to(half); };
+        const Tensor x = has_dx ? in[0] + in[1] : in[0];
+        const Tensor o = NA1dFusedPacked::apply(linear(norm(x, 8, eps1), 0), p[12], vl.defined() ? OptTensor(vl) : OptTensor(), c.H, c.win, c.left, 1, c.scale);
+        const Tensor s2 = x + linear(o, 2);
+        return inner_gradients({s2, linear(at::gelu(linear(norm(s2, 10, eps2), 4)), 6)}, in, grads);
     }
     static variable_list backward(AutogradContext* ctx, variable_list grads) {
         const variable_list s = ctx->get_saved_variables();
@@ -411,6 +456,13 @@ struct NA1dBlock : public torch::autograd::Function<NA1dBlock> {
         Projections w;
         w.buf = buf;
         w.views(refs);
+        if (at::GradMode::is_enabled()) {
+            const variable_list g = differentiable(s, c, w, data["eps1"].toDouble(), data["eps2"].toDouble(), has_dx, first, grads);
+            const Tensor none;
+            variable_list out = {g[0], g[1], none, none, none, none, none, none, none};
+            out.insert(out.end(), g.begin() + 2, g.end());
+            return out;
+        }
         const Tensor scratch = empty_f32({na1d_block_scratch_floats(rows, D, std::max(F, 3 * D))}, s1);
         const Tensor d_z = (grads[1].defined() ? grads[1].contiguous() : at::zeros_like(s2)).view({rows, D});
         const Tensor d_s2 = grads[0].defined() ? grads[0].contiguous() : Tensor();
@@ -546,7 +598,7 @@ Tensor heads_moved(const Tensor& in, const Packed& c, int64_t parts, bool to_den
 }
 Cfg dense_cfg(const Packed& c) { return Cfg{c.B * c.H, c.T, c.C, c.H, c.win, c.left, c.dil, c.scale, 0.0, 0}; }
 // qkv: packed, or (dense) the split one; o_dense: the dense route's own output
-struct LayerState { Tensor xt, qkv, lse, o, qw, pw, o_dense; };
+struct LayerState { Tensor xt, qkv, lse, o, qw, pw, o_dense, qb, pb; };
 Tensor layer_forward(const Tensor& x, const LayerShape& l, const Tensor& vl, const Tensor& r, const Tensor& qw, const OptTensor& qb, const Tensor& pw,
                      const OptTensor& pb, const Packed& c, LayerState* keep) {
     const LayerWeights w(x, l, qw, qb, pw, pb);
@@ -565,7 +617,7 @@ Tensor layer_forward(const Tensor& x, const LayerShape& l, const Tensor& vl, con
     }
     Tensor y = project(s.o.view({l.rows(), l.D}), w.pw, w.pb);
     y = l.first ? transposed(y, l, false) : y.view({l.B, l.T, l.D});
-    if (keep) { s.qw = w.qw; s.pw = w.pw; *keep = std::move(s); }
+    if (keep) { s.qw = w.qw; s.pw = w.pw; s.qb = w.qb; s.pb = w.pb; *keep = std::move(s); }
     return y;
 }
 struct NA1dLayer : public torch::autograd::Function<NA1dLayer> {
@@ -576,12 +628,44 @@ struct NA1dLayer : public torch::autograd::Function<NA1dLayer> {
         const Packed c(l.B, l.T, l.D, heads, win, left, dil, scale);
         LayerState s;
         Tensor y = layer_forward(x, l, vl ? *vl : Tensor(), rpb32(rpb), qw, qb, pw, pb, c, &s);
-        ctx->save_for_backward({s.xt, s.qkv, s.lse, s.o, s.qw, s.pw, rpb, vl ? *vl : Tensor(), s.o_dense});
+        ctx->save_for_backward({s.xt, s.qkv, s.lse, s.o, s.qw, s.pw, rpb, vl ? *vl : Tensor(), s.o_dense, s.qb, s.pb});
         auto& d = ctx->saved_data;
         d["first"] = first; d["heads"] = heads; d["groups"] = groups; d["win"] = win; d["left"] = left; d["dil"] = dil; d["scale"] = scale;
         d["qb"] = qb.has_value(); d["pb"] = pb.has_value();
         d["qw_shape"] = qw.sizes().vec(); d["pw_shape"] = pw.sizes().vec(); d["type"] = (int64_t)qw.scalar_type();
         return y;
+    }
+    // a projection's weight and bias in their own type, shape and order, from the 16-bit dense ones
+    static std::pair<Tensor, Tensor> parameters(const Tensor& w, const Tensor& b, at::IntArrayRef shape, at::ScalarType type, const LayerShape& l, int parts) {
+        if (!l.first) return {w.to(type), b.defined() ? b.to(type) : Tensor()};
+        const Tensor out_w = at::empty(shape, w.options().dtype(type)), out_b = b.defined() ? at::empty({parts * l.D}, w.options().dtype(type)) : Tensor();
+        const Tensor dense = w.to(at::kFloat), sums = b.defined() ? b.to(at::kFloat) : Tensor();
+        check(na1d_unpack_grouped(ptr(out_w), ptr(out_b), fptr(dense), fptr(sums), type == at::kFloat, l.D, l.groups, parts, code(w), stream()),
+              "na1d_unpack_grouped");
+        return {out_w, out_b};
+    }
+    // x, rpb, qkv weight, projection weight, qkv bias, projection bias
+    static variable_list differentiable(const variable_list& s, const LayerShape& l, const Packed& c, at::IntArrayRef qw_shape, at::IntArrayRef pw_shape,
+                                        at::ScalarType type, const Tensor& dy) {
+        const Tensor &xt = s[0], &rpb = s[6], &vl = s[7], &qb = s[9], &pb = s[10];
+        const auto half = xt.scalar_type();
+        const auto q = parameters(s[4], qb, qw_shape, type, l, 3), p = parameters(s[5], pb, pw_shape, type, l, 1);
+        const variable_list in = {stand_in(l.first ? transposed(xt, l, false) : xt, 0), stand_in(rpb, 1), stand_in(q.first, 2), stand_in(p.first, 3),
+                                  qb.defined() ? stand_in(q.second, 4) : Tensor(), pb.defined() ? stand_in(p.second, qb.defined() ? 5 : 4) : Tensor()};
+        auto project_with = [&](const Tensor& x, int i) {
+            const OptTensor b = in[i + 2].defined() ? OptTensor(in[i + 2].to(half)) : OptTensor();
+            return l.first ? at::conv1d(x, in[i].to(half), b, 1, at::IntArrayRef({0}), 1, l.groups) : at::linear(x, in[i].to(half), b.value_or(Tensor()));
+        };
+        Tensor y = project_with(in[0], 2);
+        // head split and merge (models/PCF_NATransformer.py:126-138, 151)
+        y = l.first ? y.view({l.B, l.D / l.groups, l.groups, 3, l.T}).transpose(1, 2).reshape({l.B, c.H, c.C, 3, l.T}).permute({3, 0, 1, 4, 2})
+                    : y.view({l.B, l.T, 3, c.H, c.C}).permute({2, 0, 3, 1, 4});
+        y = y.contiguous().view({3, l.B * c.H, l.T, c.C});
+        y = NA1dFused::apply(y.select(0, 0), y.select(0, 1), y.select(0, 2), OptTensor(in[1]), vl.defined() ? OptTensor(vl) : OptTensor(), c.H, c.win, c.left,
+                             c.dil, c.scale, 0.0, (int64_t)0)
+                .view({l.B, c.H, l.T, c.C});
+        y = l.first ? y.transpose(2, 3).reshape({l.B, l.D, l.T}) : y.transpose(1, 2).reshape({l.B, l.T, l.D});
+        return inner_gradients({project_with(y, 3)}, in, {dy});
     }
     static variable_list backward(AutogradContext* ctx, variable_list grads) {
         const variable_list s = ctx->get_saved_variables();
@@ -594,6 +678,11 @@ struct NA1dLayer : public torch::autograd::Function<NA1dLayer> {
         const auto type = (at::ScalarType)d["type"].toInt();
         const bool has_qb = d["qb"].toBool(), has_pb = d["pb"].toBool();
         const int qb_edge = 4, pb_edge = 4 + (has_qb ? 1 : 0);
+        if (at::GradMode::is_enabled()) {
+            variable_list out = differentiable(s, l, c, d["qw_shape"].toIntVector(), d["pw_shape"].toIntVector(), type, grads[0]);
+            out.resize(14);
+            return out;
+        }
         const Tensor scratch = empty_f32({na1d_block_scratch_floats(l.rows(), 0, 3 * l.D)}, xt);
         Tensor dy = grads[0].defined() ? grads[0].contiguous() : at::zeros(l.first ? at::IntArrayRef({l.B, l.D, l.T}) : xt.sizes(), xt.options());
         dy = (l.first ? transposed(dy, l, true) : dy).view({l.rows(), l.D});

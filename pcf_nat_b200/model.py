@@ -79,13 +79,7 @@ class AttentiveStatsPool(nn.Module):
         h = self.a(x) if x.is_contiguous() else self.a(x.flatten(0, 1)).view(x.shape[0], x.shape[1], -1)
         logits = self.b(torch.tanh(h))
         out = block.stats_pool(logits, x, 1e-5)
-        if out is not None:
-            return out
-        w = torch.softmax(logits.float(), dim=1)
-        xf = x.float()
-        mu = (w * xf).sum(1)
-        var = (w * xf * xf).sum(1) - mu * mu
-        return torch.cat([mu, var.clamp_min(1e-5).sqrt()], dim=1)
+        return block.weighted_stats(logits, x, 1e-5) if out is None else out
 
 
 class AAMSoftmax(nn.Module):

@@ -371,3 +371,69 @@ def test_padding_lengths_may_live_on_the_host():
     with torch.no_grad(), torch.autocast("cuda", dtype=torch.bfloat16):
         assert torch.equal(m.embedding(fbank, pad), m.embedding(fbank, pad.cuda()))
         assert not torch.equal(m.embedding(fbank, pad), m.embedding(fbank))
+
+
+def _second(y, x, params):
+    """Gradients of a penalty on the input gradient, and that gradient."""
+    g, = torch.autograd.grad(y.float().pow(2).sum(), x, create_graph=True)
+    out = torch.autograd.grad(g.float().pow(2).sum(), [x] + params, allow_unused=True)
+    return [g.detach()] + [torch.zeros_like(p) if o is None else o for o, p in zip(out, [x] + params)]
+
+
+def _same(got, want, bound):
+    for i, (a, b) in enumerate(zip(got, want)):
+        assert a.dtype == b.dtype and a.shape == b.shape
+        assert float((a.double() - b.double()).norm()) <= bound * float(b.double().norm()) + 1e-6, i
+
+
+@pytest.mark.parametrize("chained", [False, True])
+def test_second_derivative_of_blocks(chained):
+    """A gradient penalty through one block, or through two with the sum between them inside the second, with some parameters
+    frozen: the one-node route gives what the modules give (eight rounding steps of bf16 for the chain of about that many
+    16-bit tensors; a lost term would be of the order of the result)."""
+    from pcf_nat_b200 import block
+    st = _stage(64, 2, 40, n=2 if chained else 1)
+    for n, p in st.named_parameters():
+        p.requires_grad_("norm1.bias" not in n)
+    params = [p for p in st.parameters() if p.requires_grad]
+    got = {}
+    for kind in ("node", "modules"):
+        x = _rand(2, 40, 64, dtype=torch.bfloat16, seed=1, scale=0.5).requires_grad_()
+        with torch.autocast("cuda", dtype=torch.bfloat16):
+            y = block.run_blocks(st, 2 * x, None) if kind == "node" else 2 * x
+            for b in st if kind == "modules" else ():
+                y = b(y)
+        got[kind] = _second(y, x, params)
+    _same(got["node"], got["modules"], 8 * EPS[torch.bfloat16])
+
+
+@pytest.mark.parametrize("autocast", [True, False])
+@pytest.mark.parametrize("layout,groups,dim,heads,bias", [("channels_first", 4, 128, 4, True), ("channels_last", 1, 64, 2, False), ("channels_last", 1, 96, 2, True)])
+def test_second_derivative_of_a_layer(layout, groups, dim, heads, bias, autocast):
+    from pcf_nat_b200 import NAttention, nattention
+    torch.manual_seed(5)
+    m = NAttention(50, dim, heads, 9, 1, groups, layout=layout, qkv_bias=bias, proj_bias=bias).cuda()
+    m = m if autocast else m.half()
+    got = {}
+    for kind in ("node", "modules"):
+        x = _rand(*((2, dim, 50) if layout == "channels_first" else (2, 50, dim)), dtype=torch.float16, seed=1).requires_grad_()
+        with torch.autocast("cuda", dtype=torch.float16, enabled=autocast), pytest.MonkeyPatch.context() as mp:
+            if kind == "modules":
+                mp.setattr(nattention, "_native_layer", lambda *a: None)
+            y = m(1 * x)
+        assert ("NA1dLayer" in y.grad_fn.name()) == (kind == "node")
+        got[kind] = _second(y, x, list(m.parameters()))
+    _same(got["node"], got["modules"], 8 * EPS[torch.float16])
+
+
+def test_second_derivative_of_the_pooling():
+    from pcf_nat_b200 import block
+    logits, x = _rand(2, 30, 16, dtype=torch.float16, seed=1).requires_grad_(), _rand(2, 30, 16, dtype=torch.float16, seed=2)
+    x[:, :, 3] = 1.0                              # variance 0: the floor
+    x.requires_grad_()
+    got = []
+    for pool in (block.stats_pool, block.weighted_stats):
+        out = pool(logits * 1, x * 1, 1e-5)
+        g = torch.autograd.grad(out.pow(2).sum(), (logits, x), create_graph=True)
+        got.append([t.detach() for t in g] + list(torch.autograd.grad(sum(t.float().pow(2).sum() for t in g), (logits, x))))
+    _same(got[0], got[1], 4 * EPS[torch.float16])
