@@ -295,6 +295,12 @@ OptTensor packed(const Tensor& qkv, int64_t heads, int64_t win, int64_t left, in
     return o;
 }
 
+// A backward pass works in the types of its forward, also where it is called under autocast (to another type, the library products
+// would hand the kernels tensors of that type).
+struct NoAutocast {
+    const c10::impl::ExcludeDispatchKeyGuard guard{c10::autocast_dispatch_keyset};
+};
+
 // ---------------------------------------------------------------- backward passes that are differentiated again
 // Under create_graph a backward has to be differentiable itself, and the kernels' results are not. There a node with more in it than
 // the attention takes its branch again in PyTorch's operations (the attention as the operator's own node, whose gradients are
@@ -446,6 +452,7 @@ struct NA1dBlock : public torch::autograd::Function<NA1dBlock> {
         auto& data = ctx->saved_data;
         const Packed c(qkv, data["heads"].toInt(), data["win"].toInt(), data["left"].toInt(), 1, data["scale"].toDouble());
         const c10::cuda::CUDAGuard guard(s1.device());
+        const NoAutocast off;
         const bool has_dx = data["dx"].toBool();
         const int first = 1 + (has_dx ? 1 : 0) + (vl.defined() ? 1 : 0);   // edge of the first parameter
         auto need = [&](int k) { return ctx->needs_input_grad(first + k); };
@@ -675,6 +682,7 @@ struct NA1dLayer : public torch::autograd::Function<NA1dLayer> {
         LayerShape l(xt, false, d["groups"].toInt());
         l.first = d["first"].toBool();
         const c10::cuda::CUDAGuard guard(qkv.device());
+        const NoAutocast off;
         const auto type = (at::ScalarType)d["type"].toInt();
         const bool has_qb = d["qb"].toBool(), has_pb = d["pb"].toBool();
         const int qb_edge = 4, pb_edge = 4 + (has_qb ? 1 : 0);

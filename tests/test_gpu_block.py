@@ -437,3 +437,20 @@ def test_second_derivative_of_the_pooling():
         g = torch.autograd.grad(out.pow(2).sum(), (logits, x), create_graph=True)
         got.append([t.detach() for t in g] + list(torch.autograd.grad(sum(t.float().pow(2).sum() for t in g), (logits, x))))
     _same(got[0], got[1], 4 * EPS[torch.float16])
+
+
+@pytest.mark.parametrize("kind", ["block", "channels_first", "channels_last"])
+def test_backward_under_autocast_keeps_the_types_of_the_forward(kind):
+    from pcf_nat_b200 import NAttention, block
+    torch.manual_seed(5)
+    m = _stage(64, 2, 40, n=1) if kind == "block" else NAttention(40, 64, 2, 7, layout=kind).cuda()
+    x = _rand(*((2, 64, 40) if kind == "channels_first" else (2, 40, 64)), dtype=torch.bfloat16, seed=1).requires_grad_()
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        y = block.run_blocks(m, x, None) if kind == "block" else m(x)
+    ins, dy = [x] + list(m.parameters()), _rand(*y.shape, dtype=torch.bfloat16, seed=2)
+    want = torch.autograd.grad(y, ins, dy, retain_graph=True)
+    for dtype in DT:
+        with torch.autocast("cuda", dtype=dtype):
+            got = torch.autograd.grad(y, ins, dy, retain_graph=True)
+        for a, b in zip(got, want):
+            assert a.dtype == b.dtype and torch.allclose(a, b, rtol=1e-4, atol=1e-4)      # (atomics in the bias table's gradient)
