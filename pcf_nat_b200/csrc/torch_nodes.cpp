@@ -295,6 +295,12 @@ OptTensor packed(const Tensor& qkv, int64_t heads, int64_t win, int64_t left, in
     return o;
 }
 
+// An output gradient as the row and column kernels read it: dense, on a 16-byte boundary (a view into another tensor need not be).
+Tensor aligned(const Tensor& g) {
+    const Tensor c = g.contiguous();
+    return (reinterpret_cast<uintptr_t>(c.data_ptr()) & 15u) ? c.clone() : c;
+}
+
 // A backward pass works in the types of its forward, also where it is called under autocast (to another type, the library products
 // would hand the kernels tensors of that type).
 struct NoAutocast {
@@ -471,8 +477,8 @@ struct NA1dBlock : public torch::autograd::Function<NA1dBlock> {
             return out;
         }
         const Tensor scratch = empty_f32({na1d_block_scratch_floats(rows, D, std::max(F, 3 * D))}, s1);
-        const Tensor d_z = (grads[1].defined() ? grads[1].contiguous() : at::zeros_like(s2)).view({rows, D});
-        const Tensor d_s2 = grads[0].defined() ? grads[0].contiguous() : Tensor();
+        const Tensor d_z = (grads[1].defined() ? aligned(grads[1]) : at::zeros_like(s2)).view({rows, D});
+        const Tensor d_s2 = grads[0].defined() ? aligned(grads[0]) : Tensor();
         // dy^T . inp, accumulated and returned in fp32
         auto weight_grad = [&](int k, const Tensor& dy, const Tensor& inp) { return need(k) ? at::mm(dy.t(), inp, at::kFloat) : Tensor(); };
         auto bias_grad = [&](int k, const Tensor& dy) {
@@ -692,7 +698,7 @@ struct NA1dLayer : public torch::autograd::Function<NA1dLayer> {
             return out;
         }
         const Tensor scratch = empty_f32({na1d_block_scratch_floats(l.rows(), 0, 3 * l.D)}, xt);
-        Tensor dy = grads[0].defined() ? grads[0].contiguous() : at::zeros(l.first ? at::IntArrayRef({l.B, l.D, l.T}) : xt.sizes(), xt.options());
+        Tensor dy = grads[0].defined() ? aligned(grads[0]) : at::zeros(l.first ? at::IntArrayRef({l.B, l.D, l.T}) : xt.sizes(), xt.options());
         dy = (l.first ? transposed(dy, l, true) : dy).view({l.rows(), l.D});
         ProjectionGrads gp(ctx->needs_input_grad(3), has_pb && ctx->needs_input_grad(pb_edge), dy, o.view({l.rows(), l.D}), scratch,
                            d["pw_shape"].toIntVector(), type, l, 1);

@@ -454,3 +454,18 @@ def test_backward_under_autocast_keeps_the_types_of_the_forward(kind):
             got = torch.autograd.grad(y, ins, dy, retain_graph=True)
         for a, b in zip(got, want):
             assert a.dtype == b.dtype and torch.allclose(a, b, rtol=1e-4, atol=1e-4)      # (atomics in the bias table's gradient)
+
+
+@pytest.mark.parametrize("kind", ["block", "channels_first", "channels_last"])
+def test_output_gradients_may_start_anywhere(kind):
+    """A contiguous view that is not on a 16-byte boundary gives the gradients of its aligned copy."""
+    from pcf_nat_b200 import NAttention, block
+    torch.manual_seed(5)
+    m = _stage(64, 2, 40, n=1) if kind == "block" else NAttention(40, 64, 2, 7, layout=kind).cuda()
+    x = _rand(*((2, 64, 40) if kind == "channels_first" else (2, 40, 64)), dtype=torch.bfloat16, seed=1).requires_grad_()
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        y = block.run_blocks(m, 1 * x, None) if kind == "block" else m(1 * x)
+    ins, dy = [x] + list(m.parameters()), _rand(y.numel() + 1, dtype=torch.bfloat16, seed=2)[1:].view(y.shape)
+    assert dy.is_contiguous() and dy.data_ptr() % 16
+    for a, b in zip(torch.autograd.grad(y, ins, dy, retain_graph=True), torch.autograd.grad(y, ins, dy.clone(), retain_graph=True)):
+        assert torch.allclose(a, b, rtol=1e-4, atol=1e-4)      # (atomics in the bias table's gradient)
