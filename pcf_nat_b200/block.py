@@ -139,7 +139,7 @@ def _block_parameters(blk, x):
         if p is None or type(p) not in (nn.Parameter, torch.Tensor) or p.dtype != torch.float32 or p.device != dev or not p.is_contiguous() or p.data_ptr() % 16:
             return None
     Fh, H = f1.weight.shape[0], a.num_heads
-    if (D % 8 or D > 1024 or Fh % 8 or D % H or n1.normalized_shape != (D,) or n2.normalized_shape != (D,) or ps[0].shape != (3 * D, D) or
+    if (D % 8 or D > 1024 or Fh % 8 or Fh > 1 << 20 or Fh * D > (2 ** 31 - 1) // 16 or D % H or n1.normalized_shape != (D,) or n2.normalized_shape != (D,) or ps[0].shape != (3 * D, D) or
             ps[2].shape != (D, D) or ps[4].shape != (Fh, D) or ps[6].shape != (D, Fh) or ps[12].numel() != H * a.win_size):
         return None
     return ps
@@ -159,7 +159,7 @@ def run_blocks(blocks, x, valid, out=None, training=None):
     plan = []
     for blk in blocks:
         ps = _block_parameters(blk, x)
-        if ps is None or training is not None and blk.attn.training != training:
+        if ps is None or training is not None and blk.attn.training != training or B * T * ps[4].shape[0] > 2 ** 40:
             return None
         a = blk.attn
         C = D // a.num_heads

@@ -728,6 +728,12 @@ struct NA1dLayer : public torch::autograd::Function<NA1dLayer> {
     }
 };
 
+// sizes that every kernel of the node takes, in either direction (the operator itself refuses the same sizes on every route)
+bool layer_fits(const LayerShape& l, int64_t heads, bool cast) {
+    const int64_t rows = l.rows(), C = l.D / heads;
+    return l.D <= (l.first ? 8192 : (1 << 20) / 3) && (!cast || l.first || 3 * l.D * l.D <= INT32_MAX / 16) && (!l.first || l.T <= 1 << 20) &&
+           rows <= INT32_MAX / 2 && rows <= (1ll << 40) / (3 * l.D) && l.T <= INT32_MAX / 8 && l.T * C <= (int64_t)INT32_MAX * 4 && C <= 4096;
+}
 // 16-bit x; weights and biases all of x's type, or (under autocast to x's type) all fp32
 OptTensor layer(const Tensor& x, bool first, const Tensor& rpb, const Tensor& qw, const OptTensor& qb, const Tensor& pw, const OptTensor& pb,
                 int64_t heads, int64_t groups, int64_t win, int64_t left, int64_t dil, double scale, OptTensor vl) {
@@ -737,7 +743,7 @@ OptTensor layer(const Tensor& x, bool first, const Tensor& rpb, const Tensor& qw
     const bool cast = at::autocast::is_autocast_enabled(at::kCUDA);
     const auto type = qw.scalar_type();
     if ((cast && at::autocast::get_autocast_dtype(at::kCUDA) != x.scalar_type()) || (type != x.scalar_type() && !(cast && type == at::kFloat)) || l.D % 8 != 0 ||
-        l.D % groups != 0 || l.D % heads != 0 || (!first && groups != 1) || !prepare_rpb(rpb, heads * win, x))
+        l.D % groups != 0 || l.D % heads != 0 || (!first && groups != 1) || !layer_fits(l, heads, type == at::kFloat) || !prepare_rpb(rpb, heads * win, x))
         return std::nullopt;
     auto fits = [&](const Tensor& t, int64_t n) { return plain(t) && t.device() == x.device() && t.scalar_type() == type && t.is_contiguous() && t.numel() == n; };
     if (!fits(qw, 3 * l.D * (l.D / groups)) || !fits(pw, l.D * (l.D / groups)) || (qb && !fits(*qb, 3 * l.D)) || (pb && !fits(*pb, l.D))) return std::nullopt;

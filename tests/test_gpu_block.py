@@ -469,3 +469,16 @@ def test_output_gradients_may_start_anywhere(kind):
     assert dy.is_contiguous() and dy.data_ptr() % 16
     for a, b in zip(torch.autograd.grad(y, ins, dy, retain_graph=True), torch.autograd.grad(y, ins, dy.clone(), retain_graph=True)):
         assert torch.allclose(a, b, rtol=1e-4, atol=1e-4)      # (atomics in the bias table's gradient)
+
+
+def test_layers_longer_than_the_transposes_take_run():
+    from pcf_nat_b200 import NAttention
+    T = 2 ** 20 + 8
+    m = NAttention(8, 16, 1, 3, layout="channels_first").cuda().half()
+    x = _rand(1, 16, T, dtype=torch.float16, seed=1).requires_grad_()
+    y = m(x)
+    assert "NA1dLayer" not in y.grad_fn.name()
+    dx, = torch.autograd.grad(y, x, torch.ones_like(y))
+    with torch.no_grad():
+        part = m(x[..., -500:].contiguous())
+    assert torch.allclose(y[..., -499:], part[..., 1:], rtol=4 * EPS[x.dtype], atol=1e-3) and bool(torch.isfinite(dx).all())
