@@ -735,8 +735,10 @@ bool layer_fits(const LayerShape& l, int64_t heads, bool cast) {
            rows <= INT32_MAX / 2 && rows <= (1ll << 40) / (3 * l.D) && l.T <= INT32_MAX / 8 && l.T * C <= (int64_t)INT32_MAX * 4 && C <= 4096;
 }
 // 16-bit x; weights and biases all of x's type, or (under autocast to x's type) all fp32
-OptTensor layer(const Tensor& x, bool first, const Tensor& rpb, const Tensor& qw, const OptTensor& qb, const Tensor& pw, const OptTensor& pb,
+OptTensor layer(const Tensor& x, bool first, const OptTensor& bias, const Tensor& qw, const OptTensor& qb, const Tensor& pw, const OptTensor& pb,
                 int64_t heads, int64_t groups, int64_t win, int64_t left, int64_t dil, double scale, OptTensor vl) {
+    if (!bias || !bias->defined()) return std::nullopt;   // (a layer without a bias table: its modules)
+    const Tensor& rpb = *bias;
     if (!eager_mode() || !plain16(x) || x.dim() != 3 || x.numel() == 0 || !x.is_contiguous() || x.size(0) > 65535 || heads <= 0 || win <= 0 || groups <= 0)
         return std::nullopt;
     const LayerShape l(x, first, groups);

@@ -482,3 +482,15 @@ def test_layers_longer_than_the_transposes_take_run():
     with torch.no_grad():
         part = m(x[..., -500:].contiguous())
     assert torch.allclose(y[..., -499:], part[..., 1:], rtol=4 * EPS[x.dtype], atol=1e-3) and bool(torch.isfinite(dx).all())
+
+
+@pytest.mark.parametrize("layout", ["channels_first", "channels_last"])
+def test_layer_without_a_bias_table(layout):
+    from pcf_nat_b200 import NAttention
+    m = NAttention(64, 64, 2, 7, layout=layout).cuda().half()
+    x = _rand(2, 64, 64, dtype=torch.float16, seed=1)
+    with torch.no_grad():
+        m.relative_position_bias.zero_()
+        want = m(x)
+        m.relative_position_bias = None
+        assert torch.allclose(m(x), want, rtol=4 * EPS[torch.float16], atol=1e-3)
