@@ -1,6 +1,7 @@
 """Torch-facing wrappers over the C ABI: device memory and streams come from torch, the
 arithmetic comes from libna1d_b200.so. CUDA tensors only -- there is no CPU fallback."""
 import ctypes
+import warnings
 
 import torch
 
@@ -8,11 +9,20 @@ from . import _lib
 from ._lib import check
 
 _L = _lib.lib()
+
+
+class _PythonRoutes:
+    """Stands where the extension of C++ autograd nodes is missing: every call goes on to its Python route."""
+    fused = qk = av = packed = layer = valid_tokens = staticmethod(lambda *_: None)
+    eager_mode = staticmethod(lambda: False)
+
+
 try:
     from . import _na1d_torch as native     # the C++ autograd nodes; each returns None for calls that take the Python route
-except ImportError as e:
-    raise ImportError("pcf_nat_b200: _na1d_torch.so is missing or was built for another torch (%s). Build it with "
-                      "`python pcf_nat_b200/_build.py`." % e) from e
+except ImportError as e:                    # (it is built for one torch; the kernels' library is not)
+    warnings.warn("pcf_nat_b200: _na1d_torch.so is missing or was built for another torch (%s). Calls take their Python routes: the same "
+                  "kernels, more host time. Build it with `python pcf_nat_b200/_build.py`." % e, RuntimeWarning)
+    native = _PythonRoutes
 
 
 def _dtype_code(t):

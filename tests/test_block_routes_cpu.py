@@ -1,4 +1,8 @@
 """Which blocks the one-node route takes (host-only decisions), and that every other block runs its own forward."""
+import os
+import subprocess
+import sys
+
 import torch
 import torch.nn as nn
 
@@ -50,3 +54,20 @@ def test_dropout_follows_the_flag_of_its_own_module():
     assert not _taken(change=set_(attn=0.1, training=True))             # the layer's own flag decides about attention dropout
     assert not _taken(change=set_(proj=0.1, training=True, proj_training=True))
     assert _taken(change=set_(proj=0.1, training=True))
+
+
+WITHOUT_NODES = """
+import sys, warnings
+sys.modules["pcf_nat_b200._na1d_torch"] = None        # as if it were not built
+with warnings.catch_warnings(record=True) as seen:
+    warnings.simplefilter("always")
+    import pcf_nat_b200
+    from pcf_nat_b200 import ops
+assert any("_na1d_torch" in str(w.message) for w in seen)
+assert not ops.native.eager_mode() and ops.native.fused(1, 2) is None
+"""
+
+
+def test_package_imports_without_the_extension_of_nodes():
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    subprocess.run([sys.executable, "-c", WITHOUT_NODES], cwd=root, check=True)

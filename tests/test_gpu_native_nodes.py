@@ -195,3 +195,36 @@ def test_subclasses_of_the_pair_run_their_own_forward():
     attn = QK.apply(q, k, 7, 3)
     assert torch.equal(Twice.apply(q, k, 7, 3), 2 * attn)
     assert torch.equal(TwiceAV.apply(attn, v, 7, 3), 2 * AV.apply(attn, v, 7, 3))
+
+
+def test_every_route_without_the_extension():
+    """The operator, the pair, both layers and the network on the Python routes alone, in a process that cannot import the nodes."""
+    import os
+    import subprocess
+    import sys
+
+    from test_block_routes_cpu import WITHOUT_NODES
+    program = WITHOUT_NODES + """
+import torch
+from pcf_nat_b200.model import PCFNATExtractor
+g = lambda *s: torch.randn(*s, device="cuda").half().requires_grad_()
+q, k, v = g(4, 50, 32), g(4, 50, 32), g(4, 50, 32)
+QK, AV = pcf_nat_b200.getNA1dFunction(32, 1, torch.float16)
+a = AV.apply(QK.apply(q, k, 7, 3).softmax(-1), v, 7, 3)
+o = pcf_nat_b200.na1d_fused(q, k, v, 7, 3)
+assert "Backward" in o.grad_fn.name() and torch.allclose(a, o, atol=1e-2)
+torch.autograd.grad(o.float().sum() + a.float().sum(), (q, k, v))
+for layout in ("channels_first", "channels_last"):
+    m = pcf_nat_b200.NAttention(50, 64, 2, 7, layout=layout).cuda().half()
+    x = g(2, 64, 50) if layout == "channels_first" else g(2, 50, 64)
+    m(x).float().sum().backward()
+    with torch.no_grad():
+        m.eval()(x, torch.tensor([0, 9], device="cuda"))
+m = PCFNATExtractor(frames=40, feat=16, dim=32, heads=2, win=5, stages=2, blocks=1, emb=16, classes=10).cuda()
+with torch.autocast("cuda", dtype=torch.bfloat16):
+    m(torch.randn(4, 16, 40, device="cuda"), torch.arange(4, device="cuda")).backward()
+    with torch.no_grad():
+        m.eval().embedding(torch.randn(4, 16, 40, device="cuda"), torch.tensor([0, 1, 2, 3]))
+torch.cuda.synchronize()
+"""
+    subprocess.run([sys.executable, "-c", program], cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))), check=True)
