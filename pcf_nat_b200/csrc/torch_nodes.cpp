@@ -16,6 +16,7 @@
 #include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/csrc/autograd/custom_function.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/jit/frontend/tracer.h>
 
 #include "../../include/na1d_b200.h"
@@ -772,12 +773,15 @@ OptTensor valid_tokens(const Tensor& padding, int64_t T, int64_t N) {
 }  // namespace
 
 PYBIND11_MODULE(_na1d_torch, m) {
-    m.def("fused", &fused);
-    m.def("qk", &qk);
-    m.def("av", &av);
-    m.def("packed", &packed);
-    m.def("block", &block);
-    m.def("layer", &layer);
-    m.def("valid_tokens", &valid_tokens);
+    // without the interpreter lock, as PyTorch's own operators: a launch may wait for room in the stream's queue
+#define NA1D_DEF(f) m.def(#f, torch::wrap_pybind_function_no_gil(f))
+    NA1D_DEF(fused);
+    NA1D_DEF(qk);
+    NA1D_DEF(av);
+    NA1D_DEF(packed);
+    NA1D_DEF(block);
+    NA1D_DEF(layer);
+    NA1D_DEF(valid_tokens);
+#undef NA1D_DEF
     m.def("eager_mode", &eager_mode);
 }
