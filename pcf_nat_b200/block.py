@@ -239,7 +239,7 @@ def stats_pool(logits, x, floor):
     """(N, 2C) fp32: mean and standard deviation of x (N, T, C) over T under softmax-over-T weights, or None where the inputs
     are not a pair of dense 16-bit CUDA tensors that the kernel takes."""
     if (type(x) is not torch.Tensor or type(logits) is not torch.Tensor or not x.is_cuda or x.dtype not in _CODE or logits.dtype != x.dtype or
-            logits.shape != x.shape or x.dim() != 3 or torch.compiler.is_compiling() or not ops.native.eager_mode() or
+            logits.shape != x.shape or logits.device != x.device or x.dim() != 3 or torch.compiler.is_compiling() or not ops.native.eager_mode() or
             torch.autograd.forward_ad._current_level >= 0):
         return None
     N, T, C = x.shape

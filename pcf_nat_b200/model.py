@@ -76,7 +76,8 @@ class AttentiveStatsPool(nn.Module):
 
     def forward(self, x):
         # (as a matrix where the rows are slices of wider ones, which a GEMM reads in place)
-        h = self.a(x) if x.is_contiguous() else self.a(x.flatten(0, 1)).view(x.shape[0], x.shape[1], -1)
+        in_place = x.dim() == 3 and not x.is_contiguous() and _plain_linear(self.a)
+        h = self.a(x.flatten(0, 1)).view(x.shape[0], x.shape[1], -1) if in_place else self.a(x)
         logits = self.b(torch.tanh(h))
         out = block.stats_pool(logits, x, 1e-5)
         return block.weighted_stats(logits, x, 1e-5) if out is None else out
@@ -123,7 +124,7 @@ class PCFNATExtractor(nn.Module):
         outs = []
         valid = None
         if not self.training and padding is not None and x.is_cuda:
-            valid = _valid_tokens(x.shape[1], padding, x.shape[0])
+            valid = _valid_tokens(x.shape[1], padding, x.shape[0]).to(x.device)
         C = x.shape[-1]
         # evaluation: the stages write into the concatenation themselves, the projections read it in place
         plain = all(_plain_linear(m) for m in self.fuse) and type(self.pool) is AttentiveStatsPool and _plain_linear(self.pool.a)

@@ -71,3 +71,14 @@ assert not ops.native.eager_mode() and ops.native.fused(1, 2) is None
 def test_package_imports_without_the_extension_of_nodes():
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
     subprocess.run([sys.executable, "-c", WITHOUT_NODES], cwd=root, check=True)
+
+
+def test_pooling_hands_its_projection_the_rows_as_they_came():
+    from pcf_nat_b200.model import AttentiveStatsPool
+    torch.manual_seed(0)
+    pool = AttentiveStatsPool(16)
+    x, shapes = torch.randn(3, 16, 20).transpose(1, 2), []          # not contiguous
+    want = pool(x.contiguous())
+    assert torch.allclose(pool(x), want, rtol=1e-5, atol=1e-6)
+    pool.a.register_forward_hook(lambda m, i, o: shapes.append(i[0].shape))
+    assert torch.allclose(pool(x), want, rtol=1e-5, atol=1e-6) and shapes == [x.shape]
