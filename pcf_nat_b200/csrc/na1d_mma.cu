@@ -10,8 +10,9 @@
 // tcgen05 shape to pay: at these windows most of a 128 x 256 tile would be outside the band.
 //
 // Precision is that of the fp32 kernel: the logits are products of 16-bit inputs summed in fp32 either way; the probabilities
-// and their gradients enter the second contractions as two 16-bit pieces each (high + remainder, 2^-17 of the value; bf16) or
-// two tf32 pieces (2^-21, any exponent; fp16 inputs, which are exact in tf32), so nothing is rounded to 16 bits but the result.
+// and their gradients enter the second contractions whole, as three bf16 pieces (8 + 8 + 8 bits) or, for fp16 inputs, which are exact
+// in tf32, as two tf32 pieces (11 + 13 bits with a sign: the first one rounded to nearest), so nothing is rounded but the result.
+// Two bf16 pieces (2^-17 of the value) cost 4 % less time and raised the error of the 16-bit results by 1e-6 of itself.
 //
 // A chunk that meets the band only partly multiplies the rows outside it by an exact zero, which an infinite or NaN row would
 // turn into NaN: a CTA whose staged rows hold such a value computes its rows with plain fp32 arithmetic instead.
@@ -51,25 +52,30 @@ __device__ __forceinline__ void mma8_tf32(float (&d)[4], const uint32_t* a, uint
 // pieces; rows come from shared memory by ldmatrix.trans.
 template <typename E> struct Weights;
 template <> struct Weights<__nv_bfloat16> {
-    uint32_t hi[4], lo[4];   // a fragment of m16n8k16: (row, k), (row + 8, k), (row, k + 8), (row + 8, k + 8)
+    uint32_t p[3][4];   // a fragment of m16n8k16: (row, k), (row + 8, k), (row, k + 8), (row + 8, k + 8)
     __device__ __forceinline__ void set(const float (&w)[2][4]) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            const float a = w[i >> 1][2 * (i & 1)], b = w[i >> 1][2 * (i & 1) + 1];
-            hi[i] = Cvt<__nv_bfloat16>::pack2(a, b);
-            lo[i] = Cvt<__nv_bfloat16>::pack2(a - __uint_as_float(hi[i] << 16), b - __uint_as_float(hi[i] & 0xffff0000u));
+            float a = w[i >> 1][2 * (i & 1)], b = w[i >> 1][2 * (i & 1) + 1];
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {   // (the remainders are exact)
+                p[k][i] = Cvt<__nv_bfloat16>::pack2(a, b);
+                a -= __uint_as_float(p[k][i] << 16);
+                b -= __uint_as_float(p[k][i] & 0xffff0000u);
+            }
         }
     }
     // d[0], d[1] += weights . (16 rows x channels 0-7, 8-15); x: the four matrices of ldsm4_t over those rows and channels
     __device__ __forceinline__ void apply(float (&d0)[4], float (&d1)[4], const uint32_t (&x)[4]) const {
-        mma16<__nv_bfloat16>(d0, hi, x[0], x[1]);
-        mma16<__nv_bfloat16>(d1, hi, x[2], x[3]);
-        mma16<__nv_bfloat16>(d0, lo, x[0], x[1]);
-        mma16<__nv_bfloat16>(d1, lo, x[2], x[3]);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            mma16<__nv_bfloat16>(d0, p[k], x[0], x[1]);
+            mma16<__nv_bfloat16>(d1, p[k], x[2], x[3]);
+        }
     }
 };
 template <> struct Weights<__half> {
-    // m16n8k8 fragments of the two column halves. The contraction index may be permuted freely: k = l % 4 and l % 4 + 4 stand for
+    // m16n8k8 fragments of the two column halves: first piece and remainder. The contraction index may be permuted freely: k = l % 4 and l % 4 + 4 stand for
     // columns 2 (l % 4) and 2 (l % 4) + 1, which is what a thread holds of the accumulator and what ldmatrix.trans gives it.
     uint32_t hi[2][4], lo[2][4];
     __device__ __forceinline__ void set(const float (&w)[2][4]) {
@@ -78,8 +84,8 @@ template <> struct Weights<__half> {
             const float v[4] = {w[h][0], w[h][2], w[h][1], w[h][3]};
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-                hi[h][i] = __float_as_uint(v[i]) & 0xffffe000u;
-                lo[h][i] = __float_as_uint(v[i] - __uint_as_float(hi[h][i]));
+                hi[h][i] = (__float_as_uint(v[i]) + 0x1000u) & 0xffffe000u;
+                lo[h][i] = __float_as_uint(v[i] - __uint_as_float(hi[h][i]));   // at most half a step of 2^-11: 11 bits, exact in tf32
             }
         }
     }
@@ -596,7 +602,7 @@ __device__ __forceinline__ bool band_load(float* s, const float* __restrict__ ba
     bool bad = false;
     auto put = [&](int i, float v) {
         s[i] = v;
-        bad |= (__float_as_uint(v) & 0x7f800000u) == 0x7f800000u;
+        bad |= (__float_as_uint(v) & 0x7f000000u) == 0x7f000000u;   // not finite, or so large that its first piece might not be
     };
     if (gm.dil == 1) {   // the rows are one contiguous piece
         const float* src = band + ((long long)t.n * gm.T + first) * gm.win;

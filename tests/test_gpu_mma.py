@@ -181,3 +181,29 @@ def test_unfused_operators_keep_bad_values_in_their_window(value, C, routes):
             assert torch.equal(torch.isfinite(a), torch.isfinite(b)) and torch.equal(torch.isnan(a), torch.isnan(b))
             ok = torch.isfinite(b)
             assert torch.allclose(a[ok].float(), b[ok].float(), rtol=1e-2, atol=1e-2)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("C", [24, 48, 128])
+def test_bands_keep_all_their_bits(C, dtype):
+    """Two band entries on equal rows that cancel but for the last bits of one of them: the remainder, 2^-23 of the entries, comes
+    out whole, in every place of the 24 bits."""
+    from pcf_nat_b200 import ops
+    T, win = 40, 5
+    x = torch.full((1, T, C), 1.5, device="cuda", dtype=dtype)
+    bits = torch.arange(T, device="cuda") % 23 + 1                          # the bit that survives in row t
+    band = torch.zeros(1, T, win, device="cuda")
+    odd = 1 + 0.25 + 2.0 ** -9 + 2.0 ** -13                                 # pieces in between, none a power of two
+    tail = torch.exp2(-bits.float())
+    band[0, :, 2] = odd + tail
+    band[0, :, 1] = -odd
+    left = (band[0, :, 2].double() + band[0, :, 1].double()) * 1.5          # (key t - 1 + key t, both 1.5; row 0 has no key -1)
+    old = ops.set_kernel_family(ops.FAMILY_WARP_MMA)
+    try:
+        av = ops.av_forward(band, x, win, 2)[0]
+        vb = ops.v_backward(band, x, win, 2)[0]
+    finally:
+        ops.set_kernel_family(old)
+    assert torch.equal(av[1:].double(), left[1:, None].to(dtype).double().expand(T - 1, C))
+    want = (band[0, :, 2].double() + torch.cat([band[0, 1:, 1], band.new_zeros(1)]).double()) * 1.5     # key t: queries t and t + 1
+    assert torch.equal(vb.double(), want[:, None].to(dtype).double().expand(T, C))
