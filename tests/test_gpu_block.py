@@ -26,7 +26,7 @@ def _close(got, ref, dtype, steps=1.0):
 @pytest.mark.parametrize("dtype", DT)
 @pytest.mark.parametrize("rows,D", [(1, 8), (7, 64), (8, 256), (9, 264), (300, 256), (5000, 192), (33, 512), (17, 776), (20, 1024)])
 def test_layer_norm_with_residual(rows, D, dtype):
-    from pcf_nat_b200 import block
+    import block_passes as block
     x, dx, dy, res = (_rand(rows, D, dtype=dtype, seed=s) for s in range(4))
     w, b = 1 + _rand(D, dtype=torch.float32, seed=5, scale=0.2), _rand(D, dtype=torch.float32, seed=6, scale=0.2)
     y, s, mean, rstd = block.layer_norm(x, dx, w, b, 1e-5, True)
@@ -37,7 +37,7 @@ def test_layer_norm_with_residual(rows, D, dtype):
     y0, s0, none, _ = block.layer_norm(s, None, w, b, 1e-5, False)
     assert torch.equal(y0, y) and s0 is s and none is None
     for r in (res, None):
-        ds, sums = block.layer_norm_backward(dy, s, mean, rstd, w, r, block._scratch(rows, D, 8, x.device))
+        ds, sums = block.layer_norm_backward(dy, s, mean, rstd, w, r, block.scratch_for(rows, D, 8, x.device))
         gs, gw, gb = torch.autograd.grad(ref, (s64, w64, b64), dy.double(), retain_graph=True)
         gs = gs if r is None else gs + r.double()
         # the row sums cancel: fp32 noise of the terms, not of the result
@@ -50,7 +50,7 @@ def test_layer_norm_with_residual(rows, D, dtype):
 @pytest.mark.parametrize("dtype", DT)
 @pytest.mark.parametrize("rows,F_", [(1, 8), (9, 256), (700, 264), (4099, 1024), (65, 2048)])
 def test_gelu_and_column_sums(rows, F_, dtype):
-    from pcf_nat_b200 import block
+    import block_passes as block
     x, dy = _rand(rows, F_, dtype=dtype, seed=1, scale=2.0), _rand(rows, F_, dtype=dtype, seed=2)
     x64 = x.double().requires_grad_()
     ref = F.gelu(x64)
@@ -60,7 +60,7 @@ def test_gelu_and_column_sums(rows, F_, dtype):
     assert bool(((got.double() - ref.detach()).abs() <= bound).all())
     torch_err = (F.gelu(x).double() - ref.detach()).norm()
     assert float((got.double() - ref.detach()).norm()) <= 1.001 * float(torch_err)      # no less exact than the framework's
-    scratch = block._scratch(rows, 8, F_, x.device)
+    scratch = block.scratch_for(rows, 8, F_, x.device)
     dx, sums = block.gelu_backward(dy, x, scratch)
     want = torch.autograd.grad(ref, x64, dy.double())[0]
     _close(dx, want, dtype)
@@ -69,7 +69,7 @@ def test_gelu_and_column_sums(rows, F_, dtype):
 
 
 def test_gelu_of_special_values():
-    from pcf_nat_b200 import block
+    import block_passes as block
     for dtype in DT:
         x = torch.tensor([0.0, -0.0, float("inf"), float("-inf"), float("nan"), 3e4, -3e4, -8.0], device="cuda", dtype=dtype)
         got, ref = block.gelu(x).float(), F.gelu(x).float()
@@ -79,7 +79,7 @@ def test_gelu_of_special_values():
 
 
 def test_cast_parameters_is_the_rounding_of_each_tensor():
-    from pcf_nat_b200 import block
+    import block_passes as block
     for dtype in DT:
         ps = [_rand(n, dtype=torch.float32, seed=n) for n in (1, 7, 8, 63, 64, 2048, 2049, 70001)]
         ps.append(_rand(33, dtype=torch.float32, seed=3)[1:])          # not 16-byte aligned
