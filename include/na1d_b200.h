@@ -289,7 +289,8 @@ int na1d_fused_kernel_tiling(int64_t N, int64_t T, int64_t C, int64_t win, int64
 
 /* Force a kernel family for the fused entry points: -1 = automatic (default), 0 = CUDA-core,
  * 1 = tcgen05/TMA (the flat tiling wherever it can run, else the segmented one; for the unfused entry points: also
- * where the automatic choice would take a CUDA-core kernel), 2 = tcgen05/TMA on the segmented tiling, 3 = the warp-level matrix
+ * where the automatic choice would take a CUDA-core kernel), 2 = what the strided entry points run: the segmented tiling, or the
+ * marching kernels where those stand for it, 5 = tcgen05/TMA on the segmented tiling and nothing else, 3 = the warp-level matrix
  * kernels wherever they can run (up to 128 channels), else CUDA-core, 4 = the marching kernels where they can run (windows up
  * to 33; fused entry points at 16 channels, forward at 32 too, unfused ones at 16, 32 and 64), else as 3. Process-wide;
  * meant for tests and benchmarks. Returns the previous setting. */

@@ -46,7 +46,7 @@ Unfused pick_unfused(const na1d::Geometry& g, int core_most, int core_most_march
     march_ok = march_ok && na1d::march_band_supports(g);
     if (forced == 0) return Unfused::core;
     if (forced == 4 && march_ok) return Unfused::march;
-    if (forced >= 3) return warp_ok ? Unfused::warp : Unfused::core;
+    if (forced == 3 || forced == 4) return warp_ok ? Unfused::warp : Unfused::core;
     if (forced == 1 && tc_ok) return Unfused::tcgen05;
     if (march_ok && !(tc_ok && tc_over_march)) return g.C * g.win <= core_most_march ? Unfused::core : Unfused::march;
     if (g.C * g.win <= core_most) return Unfused::core;
@@ -76,7 +76,7 @@ template <typename... P> int check_pointers(const P*... p) {
 bool use_mma(const na1d::Geometry& g, bool backward) {
     const int forced = g_family_override.load();
     if (forced == 0 || !na1d::mma_supports(g)) return false;
-    if (forced >= 3) return true;
+    if (forced == 3 || forced == 4) return true;
     const double C = g.C, tp = (g.T + g.dil - 1) / g.dil, rows = (double)g.N * g.T, residues = (double)g.N * (g.dil < g.T ? g.dil : g.T);
     const double in = g.win < tp ? g.win : tp, w = in + 0.7 * (g.win - in);          // neighbours outside the sequence cost less
     const double blocks = std::ceil(tp / 16), tiles = std::ceil(tp / 64), chunks = ((g.win + 30) / 16) / 2.0;
@@ -89,7 +89,8 @@ bool use_mma(const na1d::Geometry& g, bool backward) {
 // The marching kernels: 16-channel rows in everything; 32-channel rows in the forward, where they stand for the segmented tiling
 // (any strides, no empty tile rows: 85 -> 51 us for 4096 x 150 rows, window 27) and, on dense tensors, for small problems (the
 // flat tiling starts slower but is as fast from about 300 thousand rows on: 16 against 13 us at 154 thousand rows, 49 against 51
-// at 614 thousand). A forced family 2 takes them too where it takes the shape; 4 is the same without that tiling's own limits.
+// at 614 thousand). A forced family 2 takes them too where it takes the shape (a dense call then gives the bits of a strided one); 4 is
+// the same without that tiling's own limits, 5 the segmented tiling alone.
 enum class Pass { forward, strided_forward, backward };
 template <typename... S> bool use_march(const na1d::Geometry& g, Pass pass, const S&... strides) {
     const int forced = g_family_override.load();
@@ -198,8 +199,8 @@ static int pick_family(const na1d::Geometry& g, int backward, bool has_bias = fa
     const int forced = g_family_override.load();
     const bool flat_ok = backward ? na1d::tc_bwd_supports(g, has_bias, wants_bias_grad) : na1d::tc_fwd_supports(g);
     const bool seg_ok = backward ? na1d::tc_bwd_seg_supports(g, has_bias, wants_bias_grad) : na1d::tc_seg_supports(g);
-    if (forced == 0 || forced >= 3) return 0;
-    if (forced == 2) return seg_ok ? 2 : NA1D_ERR_UNSUPPORTED;
+    if (forced == 0 || forced == 3 || forced == 4) return 0;
+    if (forced == 2 || forced == 5) return seg_ok ? 2 : NA1D_ERR_UNSUPPORTED;
     if (forced == 1 && flat_ok) return 1;   // forced: the flat tiling wherever it can run (the choice below is for the automatic mode)
     int pick = 0;
     if (flat_ok && seg_ok && g.dil > 1) {
@@ -238,7 +239,7 @@ int na1d_fused_kernel_tiling(int64_t N, int64_t T, int64_t C, int64_t win, int64
 }
 
 int na1d_set_kernel_family(int family) {
-    if (family < -1 || family > 4) family = -1;
+    if (family < -1 || family > 5) family = -1;
     return g_family_override.exchange(family);
 }
 

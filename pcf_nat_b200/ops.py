@@ -371,6 +371,7 @@ def window_index(T, win, left, dil=1, device="cuda"):
 
 
 FAMILY_AUTO, FAMILY_CUDA_CORE, FAMILY_TCGEN05, FAMILY_TCGEN05_SEGMENTED, FAMILY_WARP_MMA, FAMILY_MARCH = -1, 0, 1, 2, 3, 4
+FAMILY_SEGMENTED_ONLY = 5    # (2 runs the marching kernels where the strided entry points do)
 
 
 def set_kernel_family(family):

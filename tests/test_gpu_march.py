@@ -85,3 +85,22 @@ def test_strips_leave_no_seam():
     for i in range(4):
         assert torch.equal(many[i][0], one[i][0]) and torch.equal(many[i][3999], one[i][0])
     assert torch.allclose(many[4] / 4000, one[4], rtol=1e-3, atol=1e-3)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_segmented_tiling_where_the_marching_kernels_stand_for_it(dtype):
+    """The tcgen05 kernels on the segmented tiling at the sizes of their own test that the automatic choice gives to the marching
+    ones in some calls and to them in others: forward and backward against 64 bits."""
+    from test_gpu_segmented import SEG_SHAPES
+
+    from pcf_nat_b200 import ops
+    for N, H, T, C, win, left, dil in SEG_SHAPES:
+        if C == 64:
+            continue
+        case = (N // H, H, T, C, win, left, dil, True, True)
+        args = _inputs(case, dtype)
+        march = _run(ops.FAMILY_MARCH, case, *args)
+        got = _run(ops.FAMILY_SEGMENTED_ONLY, case, *args)
+        assert not torch.equal(march[0], got[0]) or T < 32, case           # (another kernel)
+        for i, (a, r) in enumerate(zip(got, _reference(case, *args))):
+            assert float((a.double() - r).norm()) <= 1.2 * EPS[dtype] * float(r.norm()) + 1e-6, (case, i)
