@@ -522,7 +522,8 @@ __global__ void __launch_bounds__(kWarps * 32, NT == 3 ? 3 : 4) march_bwd_kernel
 // 76 / 74 / 38.
 //   march_qk  : band[t, kk] = a[t] . b[j]             (QK forward, dA)
 //   march_rows: out[t] = sum band[t, kk] x[j]         (AV forward, dQ), or TRANSPOSED out[j] = sum band[t, kk] x[t] (dV, dK)
-// The band enters the products as two 16-bit pieces. A result that is not finite is computed again, row by row in fp32: the
+// The band enters the products as two 16-bit pieces where the tcgen05 kernels round it to one, as three bf16 pieces (all its bits) in the
+// transposed product, which the CUDA cores take at some of these windows. A result that is not finite is computed again, row by row in fp32: the
 // zeros outside the band must not meet an infinite row.
 template <int NT> constexpr int kPatchPitch = 16 * NT + 8;
 template <int NT> constexpr int kPatchIters = (16 * (16 * NT - 15) + 31) / 32;   // 32-element steps of 16 band rows
@@ -643,7 +644,7 @@ __global__ void __launch_bounds__(kWarps * 32) march_rows_kernel(E* __restrict__
     Rows<KC> xn;
     RowsT<KC> xt[TRANSPOSED ? 1 : NT];
     float acc[TRANSPOSED ? NT : 1][KC][2][4];
-    constexpr int TILES = TRANSPOSED ? 1 : NT;
+    constexpr int TILES = TRANSPOSED ? 1 : NT, PIECES = TRANSPOSED ? 3 : 2;
 #pragma unroll
     for (int t = 0; t < TILES; ++t) {
         xn.load(px, ux, st.Tr);
@@ -681,22 +682,25 @@ __global__ void __launch_bounds__(kWarps * 32) march_rows_kernel(E* __restrict__
         }
 #pragma unroll
         for (int t = 0; t < NT; ++t) {
-            uint32_t hi[4], lo[4];
+            uint32_t piece[PIECES][4];
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-                const float2 p = *reinterpret_cast<const float2*>(patch + (fr + 8 * (i & 1)) * kPatchPitch<NT> + 16 * t + 8 * (i >> 1) + 2 * (lane & 3));
-                hi[i] = Cvt<E>::pack2(p.x, p.y);
-                const float hx = Cvt<E>::from_bits((unsigned short)(hi[i] & 0xffffu)), hy = Cvt<E>::from_bits((unsigned short)(hi[i] >> 16));
-                lo[i] = Cvt<E>::pack2(p.x - hx, p.y - hy);
+                float2 p = *reinterpret_cast<const float2*>(patch + (fr + 8 * (i & 1)) * kPatchPitch<NT> + 16 * t + 8 * (i >> 1) + 2 * (lane & 3));
+#pragma unroll
+                for (int k = 0; k < PIECES; ++k) {
+                    piece[k][i] = Cvt<E>::pack2(p.x, p.y);
+                    p.x -= Cvt<E>::from_bits((unsigned short)(piece[k][i] & 0xffffu));
+                    p.y -= Cvt<E>::from_bits((unsigned short)(piece[k][i] >> 16));
+                }
             }
-            if constexpr (TRANSPOSED) {
-                const uint32_t ht[4] = {transpose8(hi[0]), transpose8(hi[2]), transpose8(hi[1]), transpose8(hi[3])};
-                const uint32_t lt[4] = {transpose8(lo[0]), transpose8(lo[2]), transpose8(lo[1]), transpose8(lo[3])};
-                if (t + 1 == NT) accumulate<E, KC, true>(acc[t], ht, xt[0]); else accumulate<E, KC, false>(acc[t], ht, xt[0]);
-                accumulate<E, KC, false>(acc[t], lt, xt[0]);
-            } else {
-                if (t == 0) accumulate<E, KC, true>(acc[0], hi, xt[t]); else accumulate<E, KC, false>(acc[0], hi, xt[t]);
-                accumulate<E, KC, false>(acc[0], lo, xt[t]);
+#pragma unroll
+            for (int k = 0; k < PIECES; ++k) {
+                if constexpr (TRANSPOSED) {
+                    const uint32_t w[4] = {transpose8(piece[k][0]), transpose8(piece[k][2]), transpose8(piece[k][1]), transpose8(piece[k][3])};
+                    if (k == 0 && t + 1 == NT) accumulate<E, KC, true>(acc[t], w, xt[0]); else accumulate<E, KC, false>(acc[t], w, xt[0]);
+                } else {
+                    if (k == 0 && t == 0) accumulate<E, KC, true>(acc[0], piece[k], xt[t]); else accumulate<E, KC, false>(acc[0], piece[k], xt[t]);
+                }
             }
         }
         __syncwarp();
