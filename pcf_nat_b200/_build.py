@@ -25,7 +25,7 @@ def sources():
 
 
 def _headers():
-    return [os.path.join(CSRC, f) for f in os.listdir(CSRC) if not f.endswith(".cu")] + [
+    return [os.path.join(CSRC, f) for f in os.listdir(CSRC) if not f.endswith((".cu", ".cpp"))] + [
         os.path.join(os.path.dirname(PKG), "include", "na1d_b200.h")]
 
 
