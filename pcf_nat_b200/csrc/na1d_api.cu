@@ -36,22 +36,97 @@ int check_geometry(int64_t N, int64_t heads, int64_t T, int64_t C, int64_t win, 
     return NA1D_OK;
 }
 
-// Which kernels run an unfused operator. The CUDA-core ones cost C * win operations a row and nothing else; the others have a
-// cost per row that hardly depends on the window: the marching ones (16, 32, 64 channels, dilation 1) the least, the tcgen05
-// ones, and the warp-level products on staged tiles for what is left (other channel counts, windows and dilations).
+// What a call asks of the kernels, for the cost models below: microseconds, fitted to graph replays of 700 calls of the unfused
+// operators and 400 of the fused pair on general shapes (8 to 128 channels, windows 2 to 80, dilations 1 to 4, residues of 2 to 2000
+// rows, 100 to a million rows, both types); the median error of a model is 7 to 12 %.
+struct Work {
+    double rows, C, CP, win, met, meet;   // met: neighbours inside the sequence, on average; meet: at most
+    double chunks, ctas, staged, blocks, per_cta;   // 16-row chunks of a block's window; CTAs, staged and own 16-row blocks of the warp-level kernels
+    Work(const na1d::Geometry& g, int rows_cta) : rows((double)g.N * g.T), C(g.C), win(g.win) {
+        const double tp = (g.T + g.dil - 1) / g.dil, residues = (double)g.N * (g.dil < g.T ? g.dil : g.T);
+        auto side = [tp](double n) { n = n < tp - 1 ? n : tp - 1; return n - n * (n + 1) / (2 * tp); };
+        met = 1 + side(g.left) + side(g.win - 1 - g.left);
+        meet = win < tp ? win : tp;
+        CP = g.C <= 64 ? (g.C + 15) / 16 * 16 : g.C <= 96 ? 96 : 128;
+        chunks = (g.win + 30) / 16;
+        const double tiles = std::ceil(tp / rows_cta), own = std::ceil(tp / 16);
+        ctas = residues * tiles;
+        blocks = residues * own;
+        staged = residues * (own + tiles * (chunks - 1));
+        per_cta = own < rows_cta / 16 ? own : rows_cta / 16;
+    }
+};
+// CUDA-core kernels: a thread group walks the window of its row (latency), C operations a neighbour (throughput); neighbours outside
+// the sequence are skipped
+struct CoreCost {
+    double start, met, skipped, row, product, skip;
+    double operator()(const Work& w) const {
+        return start + met * w.meet + skipped * (w.win - w.meet) + 1e-3 * w.rows * (w.C * (row + product * w.met) + skip * (w.win - w.met));
+    }
+};
+// warp-level kernels: a CTA per 64 or 128 rows of a residue, whatever the window and however few of the rows there are
+struct WarpCost {
+    double start, chunk, stage, cta, staged, block, product;
+    double operator()(const Work& w) const {
+        return start + chunk * w.chunks + stage * (w.per_cta + w.chunks - 1) * w.CP +
+               1e-3 * (w.ctas * cta + w.staged * w.CP * staged + w.blocks * w.chunks * (block + product * w.CP));
+    }
+};
+// tcgen05 kernels on the flat tiling: rows, in three window buckets
+struct TileCost {
+    double start, row, channel, bucket[3], neighbour;
+    double operator()(const Work& w, int weff) const {
+        return start + 1e-3 * w.rows * (row + channel * w.C + bucket[weff <= 9 ? 0 : weff <= 17 ? 1 : 2] + neighbour * w.win);
+    }
+};
+// marching kernels: 16-row blocks, two or three key tiles each; whole lines of the band
+struct MarchCost {
+    double start, tile_start, block, tile, channel, tile_channel, sequence, entry;
+    double operator()(const Work& w, const na1d::Geometry& g) const {
+        const double tiles = g.win <= 17 ? 2 : 3, blocks = (g.T + 15) / 16;
+        return start + tile_start * tiles +
+               1e-3 * (g.N * (blocks * (block + tile * tiles + w.C * (channel + tile_channel * tiles)) + sequence * w.C * tiles) + entry * w.rows * w.win);
+    }
+};
+// Which kernels run an unfused operator: the cheapest by these models, where the kernels that are the most natural ones for the shape
+// (tcgen05 where they take it, else CUDA-core) are left only for a gain of 10 %, the models' error. Over 700 drawn calls the chosen
+// kernels take 0.89 (q.k), 0.72 (a.v) and 0.70 (transposed) of those kernels' time, geometric mean; 2 % of the calls are more than 3 %
+// slower, at most 1.17 times. Kernels that would lose bits are not candidates:
+//   q.k        fp32 results: matrix instructions (fp32 sums rounded towards zero, 2 to 3 times the CUDA-core kernels' error) only where
+//              the tcgen05 kernels take the shape;
+//   band . x   the marching form splits the fp32 band into two 16-bit pieces, against one in the tcgen05 kernels: only where those take the
+//              shape;
+//   transposed as band . x, with three bf16 pieces and so at any window; not for fp16, whose pieces lack the band's exponents.
 enum class Unfused { core, tcgen05, warp, march };
-Unfused pick_unfused(const na1d::Geometry& g, int core_most, int core_most_march, bool tc_ok, bool tc_over_march, bool tc_over_warp, bool march_ok) {
+struct UnfusedCosts {
+    CoreCost core;
+    TileCost tile;
+    WarpCost warp;
+    MarchCost march;
+};
+constexpr UnfusedCosts kQkCosts{{1.43, 0.244, 0.0796, 0.000374, 0.000189, 0.00513}, {3.04, 0.00879, 0.000315, {0.0115, 0.0131, 0.0128}, 0.000645},
+                                {}, {1.64, 0.308, 0.0223, 0.0533, 0.00831, 0.000748, 0., 0.000358}};
+constexpr UnfusedCosts kRowsCosts{{1.41, 0.21, 0.0513, 0.000358, 0.000125, 0.00132}, {4.24, 0.0226, 0.000466, {0.00737, 0.0148, 0.0317}, 6.87e-05},
+                                  {1.37, 0.406, 0.00316, 1.6, 0.0183, 0.115, 0.}, {2.41, 0.0754, 0.126, 0.0449, 0.00576, 0.00297, 0.000666, 0.000212}};
+constexpr UnfusedCosts kTransposedCosts{{1.4, 0.227, 0.0541, 0.000319, 0.000147, 0.00113}, {4.56, 0.0293, 0.000547, {0.00252, 0.022, 0.0421}, 0.000407},
+                                        {0.808, 0.685, 0.00327, 1.63, 0.0211, 0.139, 0.}, {1.26, 0.823, 0.0867, 0.0504, 0.00501, 0.00428, 0.000604, 0.000212}};
+// tc_takes: the tcgen05 kernel takes the call; tc_first: and is the natural one; warp_as_good, march_as_good: those lose no bits
+Unfused pick_unfused(const na1d::Geometry& g, const UnfusedCosts& costs, bool tc_takes, bool tc_first, bool warp_as_good, bool march_as_good) {
     const int forced = g_family_override.load();
-    const bool warp_ok = na1d::mma_band_supports(g);
-    march_ok = march_ok && na1d::march_band_supports(g);
+    const bool warp_ok = na1d::mma_band_supports(g), march_ok = na1d::march_band_supports(g);
     if (forced == 0) return Unfused::core;
     if (forced == 4 && march_ok) return Unfused::march;
     if (forced == 3 || forced == 4) return warp_ok ? Unfused::warp : Unfused::core;
-    if (forced == 1 && tc_ok) return Unfused::tcgen05;
-    if (march_ok && !(tc_ok && tc_over_march)) return g.C * g.win <= core_most_march ? Unfused::core : Unfused::march;
-    if (g.C * g.win <= core_most) return Unfused::core;
-    if (tc_ok && (tc_over_march || tc_over_warp)) return Unfused::tcgen05;
-    return warp_ok ? Unfused::warp : Unfused::core;
+    if (forced == 1 && tc_takes) return Unfused::tcgen05;
+    const Work w(g, 128);
+    const double natural = 0.9;
+    double best = costs.core(w) * (tc_first ? 1. : natural);
+    Unfused pick = Unfused::core;
+    auto consider = [&](Unfused u, double cost) { if (cost < best) { best = cost; pick = u; } };
+    if (tc_first) consider(Unfused::tcgen05, natural * costs.tile(w, (g.win - 1) * g.dil + 1));
+    if (warp_ok && warp_as_good) consider(Unfused::warp, costs.warp(w));
+    if (march_ok && march_as_good) consider(Unfused::march, costs.march(w, g));
+    return pick;
 }
 
 // arguments of the row and column kernels of a transformer block
@@ -68,22 +143,22 @@ template <typename... P> int check_pointers(const P*... p) {
 #define NA1D_REQUIRE_PTR(p) do { if ((p) == nullptr) return NA1D_ERR_NULL_POINTER; } while (0)
 #define NA1D_REQUIRE_ALIGNED(p) do { if (!aligned16(p)) return NA1D_ERR_MISALIGNED; } while (0)
 
-// Of the general kernels (na1d_mma.cu, na1d_simt.cu) the warp-level matrix ones pay for a CTA per 64 rows of a residue whatever
-// the window, the CUDA-core ones for every neighbour of a row: few neighbours or short residues go to the latter. Picosecond
-// models of both, fitted to 8 to 128 channels, windows 3 to 40, residues of 5 to 300 rows (CUDA core / matrix, us, forward and
-// backward): 256 x 300 rows of 48 channels, window 3: 8 / 11, 50 / 32; window 9: 17 / 11, 106 / 33; 128 channels, window 3:
-// 18 / 26, 68 / 129; window 15: 63 / 26, 197 / 130; 2048 x 20 rows of 48 channels with dilation 4, window 15: 11 / 30, 66 / 112.
-bool use_mma(const na1d::Geometry& g, bool backward) {
+// Of the general kernels (na1d_mma.cu, na1d_simt.cu) the cheaper one by the models above, the warp-level one for a gain of 15 %, and not
+// for residues of fewer than eight rows, which leave most of a 16-row block empty: over 400 drawn calls 0.46 of the CUDA-core
+// kernels' time in the forward and 0.42 in the backward, geometric mean; six calls are more than 3 % slower, at most 1.5 times (a window of
+// 76 on sequences of 15 rows). 256 x 300 rows of 48 channels, window 3, take 8 us on the CUDA cores and 11 here forward, 50 and 32 backward;
+// 2048 x 20 rows with dilation 4, window 15, 11 and 30, 66 and 112.
+bool use_mma(const na1d::Geometry& g, bool fp16, bool has_bias, bool backward) {
     const int forced = g_family_override.load();
     if (forced == 0 || !na1d::mma_supports(g)) return false;
     if (forced == 3 || forced == 4) return true;
-    const double C = g.C, tp = (g.T + g.dil - 1) / g.dil, rows = (double)g.N * g.T, residues = (double)g.N * (g.dil < g.T ? g.dil : g.T);
-    const double in = g.win < tp ? g.win : tp, w = in + 0.7 * (g.win - in);          // neighbours outside the sequence cost less
-    const double blocks = std::ceil(tp / 16), tiles = std::ceil(tp / 64), chunks = ((g.win + 30) / 16) / 2.0;
-    const double core = rows * (backward ? 150 + 3 * C + w * (35 + 1.1 * C) : 20 + 0.5 * C + w * (4.5 + C / 3));
-    const double slope = chunks * (!backward ? 300 + 20 * C : C <= 64 ? 1000 + 47 * C : 170 * C);
-    const double mma = (backward ? 5e6 : 3.5e6) + residues * (tiles * (backward ? 4000 + 110 * C : 1500 + 18 * C) + blocks * slope);
-    return mma < core;
+    if ((g.T + g.dil - 1) / g.dil < 8) return false;
+    const Work w(g, 64);
+    // a bias (its gradient, in the backward) costs the CUDA-core kernels per neighbour; fp16 weights go through products of half the depth
+    const double bias = has_bias ? w.win * (backward ? 0.797 + 1e-3 * w.rows * 0.0181 : 0.0106 + 1e-3 * w.rows * 0.00027) : 0.;
+    const double core = bias + (backward ? CoreCost{4.13, 0.511, 0.226, 0.00243, 0.000915, 0.00877} : CoreCost{1.86, 0.452, 0.174, 0.000349, 0.00034, 0.00663})(w);
+    const double mma = (backward ? WarpCost{3.19, 0.208, 0.00994, 1.84, 0.107, 0., 0.} : WarpCost{2.52, 0.177, 0.00392, 1.39, 0.0177, 0.146, fp16 ? 0.00344 : 0.00103})(w);
+    return mma < 0.85 * core;
 }
 
 // The marching kernels: 16-channel rows in everything; 32-channel rows in the forward, where they stand for the segmented tiling
@@ -132,12 +207,10 @@ int na1d_qk_forward(float* attn, const void* q, const void* k, int64_t N, int64_
     NA1D_REQUIRE_ALIGNED(q); NA1D_REQUIRE_ALIGNED(k);
     na1d::Geometry g;
     if (int s = check_geometry(N, 1, T, C, win, left, dil, dtype, 1.f, g)) return s;
-    // us at 8192 x 150 rows (6912, 3456 at 32, 64 channels), CUDA core / tcgen05 / warp-level / marching: 16 channels, window 3:
-    // 22 / 40 / 52 / 23, window 5: 30 / 47 / 53 / 25, window 27: 183 / 58 / 67 / 42; 32 channels, window 3: 39 / 45 / 55 / 31;
-    // 64 channels, window 9: 82 / 31 / 49 / 32, window 27: 211 / 35 / 59 / 40, window 33 (one tcgen05 CTA per SM instead of two):
-    // 253 / 55 / 71 / 41
-    const bool tc_ok = na1d::tc_unfused_supports(g) && aligned16(attn);   // (its band goes out in 16-byte stores)
-    switch (pick_unfused(g, 80, 64, tc_ok, g.C == 64 && g.win <= 28, true, true)) {
+    // us at 8192 x 150 rows (6912, 3456 at 32, 64 channels), CUDA core / tcgen05 / marching: 16 channels, window 3: 22 / 40 / 23, window
+    // 27: 183 / 58 / 42; 32 channels, window 3: 39 / 45 / 31; 64 channels, window 9: 82 / 31 / 32, window 33: 253 / 55 / 41
+    const bool tc = na1d::tc_unfused_supports(g) && aligned16(attn);   // (the tcgen05 band goes out in 16-byte stores)
+    switch (pick_unfused(g, kQkCosts, tc, tc, false, tc)) {
         case Unfused::tcgen05: return cuda_status(na1d::tc_qk(attn, q, k, g, dtype, (cudaStream_t)stream));
         case Unfused::march: return cuda_status(na1d::march_band_out(attn, q, k, g, dtype, (cudaStream_t)stream));
         case Unfused::warp: return cuda_status(na1d::mma_band_out(attn, q, k, g, dtype, (cudaStream_t)stream));
@@ -154,9 +227,10 @@ int na1d_q_backward(void* q_gd, const float* attn_gd, const void* k, int64_t N, 
     NA1D_REQUIRE_ALIGNED(q_gd); NA1D_REQUIRE_ALIGNED(k);
     na1d::Geometry g;
     if (int s = check_geometry(N, 1, T, C, win, left, dil, dtype, 1.f, g)) return s;
-    // as above: 16 channels, window 5: 29 / 58 / 71 / 35, window 9: 43 / 62 / 74 / 37, window 27: 106 / 82 / 93 / 49; 32 channels, window
-    // 3: 34 / 52 / 74 / 39, window 27: 167 / 78 / 97 / 57; 64 channels, window 3: 34 / 37 / 63 / 36, window 27: 167 / 48 / 80 / 45
-    switch (pick_unfused(g, 208, 112, na1d::tc_unfused_supports(g), false, true, true)) {
+    // as above: 16 channels, window 5: 29 / 58 / 35, window 27: 106 / 82 / 49; 32 channels, window 3: 34 / 52 / 39, window 27: 167 / 78 / 57;
+    // 64 channels, window 3: 34 / 37 / 36, window 27: 167 / 48 / 45
+    const bool tc = na1d::tc_unfused_supports(g);
+    switch (pick_unfused(g, kRowsCosts, tc, tc, true, tc)) {
         case Unfused::tcgen05: return cuda_status(na1d::tc_band_x(q_gd, attn_gd, k, g, dtype, (cudaStream_t)stream));
         case Unfused::march: return cuda_status(na1d::march_band_rows(q_gd, attn_gd, k, false, g, dtype, (cudaStream_t)stream));
         case Unfused::warp: return cuda_status(na1d::mma_band_rows(q_gd, attn_gd, k, false, g, dtype, (cudaStream_t)stream));
@@ -173,13 +247,11 @@ int na1d_k_backward(void* k_gd, const float* attn_gd, const void* q, int64_t N, 
     NA1D_REQUIRE_ALIGNED(k_gd); NA1D_REQUIRE_ALIGNED(q);
     na1d::Geometry g;
     if (int s = check_geometry(N, 1, T, C, win, left, dil, dtype, 1.f, g)) return s;
-    // as above: 16 channels, window 5: 31 / 84 / 75 / 39, window 9: 46 / 102 / 76 / 42, window 27: 120 / 187 / 103 / 53; 32 channels,
-    // window 5: 50 / 77 / 78 / 41, window 27: 191 / 159 / 107 / 56; 64 channels, window 3: 35 / 42 / 65 / 36 (512 x 997 rows: 35 / 41 /
-    // 52 / 41), window 9: 76 / 53 / 67 / 37, window 27: 188 / - / 88 / 51. fp16 tensors keep the fp32 band's exponents in tf32
-    // pieces, which the marching form does not have: there the tcgen05 form, which gathers the band along its diagonals, pays
-    // off at 64 channels and windows up to 9 only.
-    const int weff = (g.win - 1) * g.dil + 1;
-    switch (pick_unfused(g, 288, g.C == 64 ? 192 : 112, na1d::tc_unfused_t_supports(g), false, g.C == 64 && weff <= 9, dtype == NA1D_BF16)) {
+    // as above, with the warp-level kernels third: 16 channels, window 5: 31 / 84 / 75 / 39, window 27: 120 / 187 / 103 / 53; 32 channels,
+    // window 27: 191 / 159 / 107 / 56; 64 channels, window 3: 35 / 42 / 65 / 36, window 27: 188 / - / 88 / 51. The tcgen05 form gathers the
+    // band along its diagonals; at 16 channels it does not pay for windows above 17.
+    const bool tc = na1d::tc_unfused_t_supports(g), wide = g.C == 16 && (g.win - 1) * g.dil + 1 > 17;
+    switch (pick_unfused(g, kTransposedCosts, tc, tc && !wide, true, dtype == NA1D_BF16 && na1d::tc_unfused_supports(g))) {
         case Unfused::tcgen05: return cuda_status(na1d::tc_bandT_x(k_gd, attn_gd, q, g, dtype, (cudaStream_t)stream));
         case Unfused::march: return cuda_status(na1d::march_band_rows(k_gd, attn_gd, q, true, g, dtype, (cudaStream_t)stream));
         case Unfused::warp: return cuda_status(na1d::mma_band_rows(k_gd, attn_gd, q, true, g, dtype, (cudaStream_t)stream));
@@ -284,7 +356,7 @@ int na1d_fused_forward(void* o, float* lse, const void* q, const void* k, const 
         const na1d::Strides d = na1d::dense_strides(g.H, g.T, g.C);
         return cuda_status(na1d::tc_fused_fwd_seg(o, lse, q, k, v, rpb, valid_len, d, d, d, d, g, dtype, (cudaStream_t)stream));
     }
-    if (use_mma(g, false))
+    if (use_mma(g, dtype == NA1D_FP16, rpb != nullptr, false))
         return cuda_status(na1d::mma_fused_fwd(o, lse, q, k, v, rpb, valid_len, g, dtype, (cudaStream_t)stream));
     return cuda_status(na1d::simt_fused_fwd(o, lse, q, k, v, rpb, valid_len, g, dtype, (cudaStream_t)stream));
 }
@@ -384,7 +456,7 @@ int na1d_fused_backward(void* dq, void* dk, void* dv, float* d_rpb, const void* 
         return cuda_status(na1d::tc_fused_bwd_seg(dq, dk, dv, d_rpb, d_o, q, k, v, lse, rpb, valid_len, delta_ws,
                                                   (size_t)g.N * (size_t)g.T, d, d, d, d, d, d, d, g, dtype, st));
     }
-    if (use_mma(g, true))
+    if (use_mma(g, dtype == NA1D_FP16, d_rpb != nullptr, true))
         return cuda_status(na1d::mma_fused_bwd(dq, dk, dv, d_rpb, d_o, q, k, v, o, lse, rpb, valid_len, g, dtype, st));
     if (int s = cuda_status(na1d::simt_delta(delta_ws, d_o, o, g.N * g.T, g.C, dtype, st))) return s;
     return cuda_status(na1d::simt_fused_bwd(dq, dk, dv, d_rpb, d_o, q, k, v, lse, delta_ws, rpb, valid_len, g, dtype, st));

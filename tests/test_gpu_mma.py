@@ -207,3 +207,34 @@ def test_bands_keep_all_their_bits(C, dtype):
     assert torch.equal(av[1:].double(), left[1:, None].to(dtype).double().expand(T - 1, C))
     want = (band[0, :, 2].double() + torch.cat([band[0, 1:, 1], band.new_zeros(1)]).double()) * 1.5     # key t: queries t and t + 1
     assert torch.equal(vb.double(), want[:, None].to(dtype).double().expand(T, C))
+
+
+@pytest.mark.parametrize("scale", [1.0, 1e-6])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("N,T,C,win,dil", [(40, 20, 16, 17, 1), (40, 31, 64, 9, 1), (30, 21, 32, 27, 2), (20, 100, 64, 40, 1), (20, 150, 48, 50, 1), (20, 90, 128, 33, 3),
+                                           (3000, 150, 16, 27, 1), (500, 150, 64, 33, 1)])
+def test_unfused_routes_lose_no_bits_of_the_band(N, T, C, win, dil, dtype, scale):
+    """Where the CUDA-core kernels stand in for shapes that tcgen05 does not take, the automatic route gives their fp32 products bit
+    for bit, and results from a band (of gradients as small as an unscaled loss leaves them) that are no further from 64 bits."""
+    from pcf_nat_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(4)
+    q, k = (torch.randn(N, T, C, device="cuda", generator=g).to(dtype) for _ in range(2))
+    band = torch.randn(N, T, win, device="cuda", generator=g) * scale
+    left = win // 2
+    got = {}
+    for family in (ops.FAMILY_AUTO, ops.FAMILY_CUDA_CORE):
+        old = ops.set_kernel_family(family)
+        try:
+            got[family] = ops.qk_forward(q, k, win, left, dil), ops.av_forward(band, k, win, left, dil), ops.v_backward(band, q, win, left, dil)
+        finally:
+            ops.set_kernel_family(old)
+    tcgen05 = C in (16, 32, 64) and T >= 32 and dil & (dil - 1) == 0 and (win - 1) * dil + 1 <= 33
+    ref = _pair_reference(q, k, band, win, left, dil)
+    if not tcgen05:
+        assert torch.equal(got[ops.FAMILY_AUTO][0], got[ops.FAMILY_CUDA_CORE][0])
+    for i in (1, 2):
+        if tcgen05 and (i == 1 or dtype == torch.float16 and C == 64):
+            continue                                  # (the tcgen05 kernels round the band to 16 bits)
+        auto, core = (float((got[f][i].double() - ref[i]).norm()) for f in (ops.FAMILY_AUTO, ops.FAMILY_CUDA_CORE))
+        # both round an fp32 result once; elements that round the other way scatter the norm
+        assert auto <= core * (1 + 1e-4 + 0.02 / ref[i].numel() ** 0.5), (i, auto, core)
