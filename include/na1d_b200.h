@@ -106,9 +106,10 @@ int na1d_fused_forward(void* o, float* lse, const void* q, const void* k, const 
 /* Gradients of na1d_fused_forward. dq,dk,dv: (N,T,C) 16-bit. d_rpb: (heads,win) fp32, ACCUMULATED
  * into (caller zeroes it), or NULL. delta_ws: caller-provided scratch of N*T fp32. The CUDA-core
  * kernels keep the row sums of d_o*o there (written by a pre-pass, read by the main kernel); the
- * tcgen05 kernels need no such pre-pass: every CTA adds its partial d_rpb to the result with atomics at
- * its end (with NA1D_BIAS_GRAD_ROWS=1 in the environment: one partial row per CTA in delta_ws, summed in
- * a fixed order by a second small kernel).
+ * others need no such pre-pass: every CTA adds its partial d_rpb to the result with atomics at
+ * its end. With NA1D_BIAS_GRAD_ROWS=1 in the environment the shapes that the tcgen05 kernels take stay with
+ * them when d_rpb is wanted, and these write one partial row per CTA to delta_ws, summed in a fixed order by a
+ * second small kernel.
  * Replaces the autograd chain AV.backward -> softmax backward -> QK.backward,
  * na1d_tensorcore/nattn.py:46-54 and :69-78. */
 int na1d_fused_backward(void* dq, void* dk, void* dv, float* d_rpb, const void* d_o, const void* q,
@@ -172,8 +173,9 @@ int na1d_fused_forward_strided(void* o, float* lse, const void* q, const void* k
                                int64_t T, int64_t C, int64_t win, int64_t left, int64_t dil, float scale, int dtype,
                                void* stream);
 
-/* scratch: `scratch_floats` fp32 of device memory for the per-CTA partial rows of d_rpb (148 * heads * win is always
- * enough; with less, or NULL, the kernel adds to d_rpb with atomics). o is not needed. */
+/* scratch: `scratch_floats` fp32 of device memory for the per-CTA partial rows of d_rpb, which are written with
+ * NA1D_BIAS_GRAD_ROWS=1 in the environment (148 * heads * win is always enough; with less, or NULL, and by default, the kernels
+ * add to d_rpb with atomics). o is not needed. */
 int na1d_fused_backward_strided(void* dq, void* dk, void* dv, float* d_rpb, const void* d_o, const void* q,
                                 const void* k, const void* v, const float* lse, const float* rpb,
                                 const int32_t* valid_len, float* scratch, int64_t scratch_floats,

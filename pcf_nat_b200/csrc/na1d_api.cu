@@ -167,12 +167,14 @@ bool use_mma(const na1d::Geometry& g, bool fp16, bool has_bias, bool backward) {
 // at 614 thousand). A forced family 2 takes them too where it takes the shape (a dense call then gives the bits of a strided one); 4 is
 // the same without that tiling's own limits, 5 the segmented tiling alone.
 enum class Pass { forward, strided_forward, backward };
-template <typename... S> bool use_march(const na1d::Geometry& g, Pass pass, const S&... strides) {
+template <typename... S> bool use_march(const na1d::Geometry& g, Pass pass, bool wants_bias_grad, const S&... strides) {
     const int forced = g_family_override.load();
     if (forced != -1 && forced != 4 && !(forced == 2 && na1d::tc_seg_supports(g))) return false;
     // (where the CUDA cores stood before -- more than 32 heads, residues of one token -- infinities and NaN stay in their windows: the
     // general kernels see to that, these, like the tcgen05 ones, do not)
     if (forced == -1 && !na1d::tc_seg_supports(g) && !na1d::tc_fwd_supports(g)) return false;
+    // (a bias gradient in a fixed order, where the environment asks for it, is the tcgen05 kernels')
+    if (forced == -1 && pass == Pass::backward && wants_bias_grad && na1d::bias_grad_partial_rows()) return false;
     if (forced == -1 && pass == Pass::forward && g.C == 32 && (long long)g.N * g.T > (1 << 18)) return false;
     return na1d::march_supports(g, pass == Pass::backward) && ((strides.token * g.dil < (1ll << 30)) && ...);
 }
@@ -345,7 +347,7 @@ int na1d_fused_forward(void* o, float* lse, const void* q, const void* k, const 
     NA1D_REQUIRE_ALIGNED(o); NA1D_REQUIRE_ALIGNED(q); NA1D_REQUIRE_ALIGNED(k); NA1D_REQUIRE_ALIGNED(v);
     na1d::Geometry g;
     if (int s = check_geometry(N, heads, T, C, win, left, dil, dtype, scale, g)) return s;
-    if (use_march(g, Pass::forward, na1d::dense_strides(g.H, g.T, g.C))) {
+    if (use_march(g, Pass::forward, false, na1d::dense_strides(g.H, g.T, g.C))) {
         const na1d::Strides d = na1d::dense_strides(g.H, g.T, g.C);
         return cuda_status(na1d::march_fused_fwd(o, lse, q, k, v, rpb, valid_len, d, d, d, d, g, dtype, (cudaStream_t)stream));
     }
@@ -398,7 +400,7 @@ int na1d_fused_forward_strided(void* o, float* lse, const void* q, const void* k
     if (int s = read_strides(k_strides, batch, heads, T, C, sk)) return s;
     if (int s = read_strides(v_strides, batch, heads, T, C, sv)) return s;
     if (!na1d::tc_seg_supports(g)) return NA1D_ERR_UNSUPPORTED;
-    if (use_march(g, Pass::strided_forward, sq, sk, sv, so)) return cuda_status(na1d::march_fused_fwd(o, lse, q, k, v, rpb, valid_len, sq, sk, sv, so, g, dtype, (cudaStream_t)stream));
+    if (use_march(g, Pass::strided_forward, false, sq, sk, sv, so)) return cuda_status(na1d::march_fused_fwd(o, lse, q, k, v, rpb, valid_len, sq, sk, sv, so, g, dtype, (cudaStream_t)stream));
     return cuda_status(na1d::tc_fused_fwd_seg(o, lse, q, k, v, rpb, valid_len, sq, sk, sv, so, g, dtype, (cudaStream_t)stream));
 }
 
@@ -422,7 +424,7 @@ int na1d_fused_backward_strided(void* dq, void* dk, void* dv, float* d_rpb, cons
     for (int i = 0; i < 7; ++i)
         if (int s = read_strides(in[i], batch, heads, T, C, s7[i])) return s;
     if (!na1d::tc_bwd_seg_supports(g, rpb != nullptr, d_rpb != nullptr)) return NA1D_ERR_UNSUPPORTED;
-    if (use_march(g, Pass::backward, s7[0], s7[1], s7[2], s7[3], s7[4], s7[5], s7[6]))
+    if (use_march(g, Pass::backward, d_rpb != nullptr, s7[0], s7[1], s7[2], s7[3], s7[4], s7[5], s7[6]))
         return cuda_status(na1d::march_fused_bwd(dq, dk, dv, d_rpb, d_o, q, k, v, lse, rpb, valid_len, s7[0], s7[1], s7[2], s7[3], s7[4], s7[5],
                                                  s7[6], g, dtype, (cudaStream_t)stream));
     return cuda_status(na1d::tc_fused_bwd_seg(dq, dk, dv, d_rpb, d_o, q, k, v, lse, rpb, valid_len, scratch, (size_t)scratch_floats,
@@ -441,7 +443,7 @@ int na1d_fused_backward(void* dq, void* dk, void* dv, float* d_rpb, const void* 
     if (int s = check_geometry(N, heads, T, C, win, left, dil, dtype, scale, g)) return s;
     if (d_rpb && heads * win * 4 > 48 * 1024) return NA1D_ERR_TOO_LARGE;
     cudaStream_t st = (cudaStream_t)stream;
-    if (use_march(g, Pass::backward, na1d::dense_strides(g.H, g.T, g.C))) {
+    if (use_march(g, Pass::backward, d_rpb != nullptr, na1d::dense_strides(g.H, g.T, g.C))) {
         const na1d::Strides d = na1d::dense_strides(g.H, g.T, g.C);
         return cuda_status(na1d::march_fused_bwd(dq, dk, dv, d_rpb, d_o, q, k, v, lse, rpb, valid_len, d, d, d, d, d, d, d, g, dtype, st));
     }

@@ -61,6 +61,7 @@ cudaError_t tc_fused_bwd_seg(void* dq, void* dk, void* dv, float* d_rpb, const v
                              const void* v, const float* lse, const float* rpb, const int* valid_len, float* scratch,
                              size_t scratch_floats, const Strides& sdq, const Strides& sdk, const Strides& sdv, const Strides& sdo,
                              const Strides& sq, const Strides& sk, const Strides& sv, const Geometry& gm, int dtype, cudaStream_t st);
+bool bias_grad_partial_rows();   // NA1D_BIAS_GRAD_ROWS=1: per-CTA rows of the bias gradient in the scratch, added up in a fixed order
 void tensor_map_cache_stats(long long* hits, long long* misses);
 
 // ---- the unfused pair on the tcgen05 kernels (na1d_tc_unfused.cu): flat tiling, same shape limits as the fused forward

@@ -237,3 +237,45 @@ print("ok")
     env = dict(os.environ, NA1D_BIAS_GRAD_ROWS="1", PYTHONPATH=root + os.pathsep + os.environ.get("PYTHONPATH", ""))
     r = subprocess.run([sys.executable, "-c", code], cwd=root, env=env, capture_output=True, text=True, timeout=600)
     assert r.returncode == 0 and "ok" in r.stdout, r.stdout[-2000:] + r.stderr[-2000:]
+
+
+def test_bias_gradient_partial_rows_at_16_channels_in_a_fresh_process():
+    """NA1D_BIAS_GRAD_ROWS=1 holds at 16 channels too, dense and packed: the caller's scratch takes the partial rows, and the sum is
+    the oracle's."""
+    import os
+    import subprocess
+    import sys
+    code = r'''
+import ctypes, sys, torch
+sys.path[:0] = ["tests", "tests/golden"]
+from gpu_util import assert_close
+from oracle import na1d_oracle as orc
+from pcf_nat_b200 import _lib, ops
+B, H, T, C, win, left = 30, 4, 150, 16, 27, 13
+N, sc = B * H, C ** -0.5
+g = torch.Generator().manual_seed(5)
+q, k, v, d_o = ((torch.randn(N, T, C, generator=g) * C ** -0.25).to(torch.bfloat16) for _ in range(4))
+rpb = 0.3 * torch.randn(H, win, generator=g)
+ref = orc.na1d_fused_with_grads(q.float(), k.float(), v.float(), d_o.float(), win, left, 1, sc, rpb, None, H)[4]
+Q, K, V, D, R = (t.cuda() for t in (q, k, v, d_o, rpb))
+O, lse = ops.fused_forward(Q, K, V, win, left, 1, sc, R, None, H)
+dq, dk, dv = (torch.empty_like(Q) for _ in range(3))
+p, s = ops._p, ops._stream(Q)
+ws = torch.full((N * T,), float("nan"), device="cuda")
+dr = torch.zeros(H, win, device="cuda")
+assert _lib.lib().na1d_fused_backward(p(dq), p(dk), p(dv), p(dr), p(D), p(Q), p(K), p(V), p(O), p(lse), p(R), None, p(ws), N, H, T, C, win, left, 1, sc, 0, s) == 0
+assert torch.isfinite(ws[:H * win]).all(), "no partial rows in the workspace"
+assert_close(dr, ref, torch.bfloat16, "dense", factor=2.0)
+ws.fill_(float("nan")); dr.zero_()
+st = (ctypes.c_int64 * 3)(H * T * C, T * C, C)
+assert _lib.lib().na1d_fused_backward_strided(p(dq), p(dk), p(dv), p(dr), p(D), p(Q), p(K), p(V), p(lse), p(R), None, p(ws), 148 * H * win, st, st, st, st, st, st, st,
+                                              N, H, T, C, win, left, 1, sc, 0, s) == 0
+assert torch.isfinite(ws[:H * win]).all(), "no partial rows in the scratch"
+assert_close(dr, ref, torch.bfloat16, "strided", factor=2.0)
+ops.device_status()
+print("ok")
+'''
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    env = dict(os.environ, NA1D_BIAS_GRAD_ROWS="1", PYTHONPATH=root + os.pathsep + os.environ.get("PYTHONPATH", ""))
+    r = subprocess.run([sys.executable, "-c", code], cwd=root, env=env, capture_output=True, text=True, timeout=600)
+    assert r.returncode == 0 and "ok" in r.stdout, r.stdout[-2000:] + r.stderr[-2000:]
