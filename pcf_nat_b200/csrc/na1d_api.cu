@@ -166,7 +166,10 @@ bool use_mma(const na1d::Geometry& g, bool fp16, bool has_bias, bool backward) {
 // flat tiling starts slower but is as fast from about 300 thousand rows on: 16 against 13 us at 154 thousand rows, 49 against 51
 // at 614 thousand). A forced family 2 takes them too where it takes the shape (a dense call then gives the bits of a strided one); 4 is
 // the same without that tiling's own limits, 5 the segmented tiling alone.
-enum class Pass { forward, strided_forward, backward };
+// The backward at 16 channels on dense tensors leaves large calls of 33 to 39 rows a residue to the flat tiling, which has no empty rows
+// there (three blocks of 16): 26857 x 33 rows, window 25, 92 us against 119; 12592 x 36, window 27, 52 / 60; 18712 x 39, window 26, 92 / 104; 10768 x 43,
+// window 33, 55 / 55.
+enum class Pass { forward, strided_forward, backward, strided_backward };
 template <typename... S> bool use_march(const na1d::Geometry& g, Pass pass, bool wants_bias_grad, const S&... strides) {
     const int forced = g_family_override.load();
     if (forced != -1 && forced != 4 && !(forced == 2 && na1d::tc_seg_supports(g))) return false;
@@ -174,9 +177,14 @@ template <typename... S> bool use_march(const na1d::Geometry& g, Pass pass, bool
     // general kernels see to that, these, like the tcgen05 ones, do not)
     if (forced == -1 && !na1d::tc_seg_supports(g) && !na1d::tc_fwd_supports(g)) return false;
     // (a bias gradient in a fixed order, where the environment asks for it, is the tcgen05 kernels')
-    if (forced == -1 && pass == Pass::backward && wants_bias_grad && na1d::bias_grad_partial_rows()) return false;
+    const bool backward = pass == Pass::backward || pass == Pass::strided_backward;
+    if (forced == -1 && backward && wants_bias_grad && na1d::bias_grad_partial_rows()) return false;
+    const int residue = (g.T + g.dil - 1) / g.dil;
+    if (forced == -1 && pass == Pass::backward && residue > 32 && residue < 40 && (long long)g.N * g.T > (1 << 17) &&
+        na1d::tc_bwd_supports(g, true, wants_bias_grad))
+        return false;
     if (forced == -1 && pass == Pass::forward && g.C == 32 && (long long)g.N * g.T > (1 << 18)) return false;
-    return na1d::march_supports(g, pass == Pass::backward) && ((strides.token * g.dil < (1ll << 30)) && ...);
+    return na1d::march_supports(g, backward) && ((strides.token * g.dil < (1ll << 30)) && ...);
 }
 }  // namespace
 
@@ -424,7 +432,7 @@ int na1d_fused_backward_strided(void* dq, void* dk, void* dv, float* d_rpb, cons
     for (int i = 0; i < 7; ++i)
         if (int s = read_strides(in[i], batch, heads, T, C, s7[i])) return s;
     if (!na1d::tc_bwd_seg_supports(g, rpb != nullptr, d_rpb != nullptr)) return NA1D_ERR_UNSUPPORTED;
-    if (use_march(g, Pass::backward, d_rpb != nullptr, s7[0], s7[1], s7[2], s7[3], s7[4], s7[5], s7[6]))
+    if (use_march(g, Pass::strided_backward, d_rpb != nullptr, s7[0], s7[1], s7[2], s7[3], s7[4], s7[5], s7[6]))
         return cuda_status(na1d::march_fused_bwd(dq, dk, dv, d_rpb, d_o, q, k, v, lse, rpb, valid_len, s7[0], s7[1], s7[2], s7[3], s7[4], s7[5],
                                                  s7[6], g, dtype, (cudaStream_t)stream));
     return cuda_status(na1d::tc_fused_bwd_seg(dq, dk, dv, d_rpb, d_o, q, k, v, lse, rpb, valid_len, scratch, (size_t)scratch_floats,
