@@ -183,6 +183,9 @@ def run_reference(args, w, name):
 
 
 # ------------------------------------------------------------------------------------------ operator timing
+ROUTES = ["cuda-core", "tcgen05", "tcgen05", "warp-mma", "march"]      # by na1d_fused_kernel_route
+
+
 class OpBench:
     """Rotating device buffer sets of one operator shape and graph-replay timing through the C ABI."""
 
@@ -380,7 +383,7 @@ def run_ours(args, w, name):
         dom_ms = (ms_bwd if w["bwd"] else ms_fwd) / args.steps
         dom_bytes = bwd_b if w["bwd"] else fwd_b
         ach = dom_bytes / (dom_ms * 1e-3) / 1e9
-        fam = L.na1d_fused_kernel_family(N, T, C, win, left, dil, 0, 1 if w["bwd"] else 0)
+        fam = L.na1d_fused_kernel_route(N, H, T, C, win, left, dil, 0, 1 if w["bwd"] else 0, 0, 0)
         h2d, d2h = 4 * N * T * C * 2, n_out * N * T * C * 2
         line = {
             "metric": "NA1D fwd+bwd queries/sec/GPU" if w["bwd"] else "NA1D fwd queries/sec/GPU",
@@ -391,7 +394,7 @@ def run_ours(args, w, name):
                        "l2": "rotating %d buffer sets of %.0f MB (> L2 between reuses)" % (ob.n_sets, ob.per_set / 1e6),
                        "launch": "one CUDA graph of the %d timed steps, replayed %d times; ms_per_step = median replay / steps "
                                  "(min %.4f, max %.4f ms per step on rank 0)" % (args.steps, R, lo_total / args.steps, hi_total / args.steps),
-                       "kernel_family": ["cuda-core", "tcgen05"][fam],
+                       "kernel_family": ROUTES[fam],
                        "checked": "outputs of 3 sequences against the fp32 oracle after the timed region (worst error/bound %.2f); "
                                   "device status word clean" % checked},
             "roofline": {"bound": "hbm", "achieved": ach, "peak": peak, "unit": "GB/s", "frac": ach / peak,
@@ -589,7 +592,7 @@ def run_sweep(args):
     def row(tag, dtype, win, dil, T, C, b, h):
         N = b * h
         ob = OpBench(L, dev, N, h, T, C, win, dil, dtype, True, scale=C ** -0.25)
-        fam = "%s/%s" % tuple(["cuda-core", "tcgen05"][L.na1d_fused_kernel_family(N, T, C, win, ob.left, dil, ob.code, bw)] for bw in (0, 1))
+        fam = "%s/%s" % tuple(ROUTES[L.na1d_fused_kernel_route(N, h, T, C, win, ob.left, dil, ob.code, bw, 0, 0)] for bw in (0, 1))
         t_f = 1e3 * ob.timed(20, "fwd", 11)[0] / 20
         t_b = 1e3 * ob.timed(20, "both", 11)[0] / 20
         ops.device_status()

@@ -289,6 +289,12 @@ int na1d_fused_kernel_family(int64_t N, int64_t T, int64_t C, int64_t win, int64
 int na1d_fused_kernel_tiling(int64_t N, int64_t T, int64_t C, int64_t win, int64_t left, int64_t dil,
                              int dtype, int backward);
 
+/* Which kernels a dense fused call runs: 0 = CUDA cores, 1 = tcgen05 on the flat tiling, 2 = on the segmented tiling, 3 = the warp-level
+ * matrix kernels, 4 = the marching kernels (as the numbers of na1d_set_kernel_family); negative = status code. Host-only. The two
+ * queries above tell the tcgen05 and general kernels apart alone: which of them takes the shape where the marching ones do not. */
+int na1d_fused_kernel_route(int64_t N, int64_t heads, int64_t T, int64_t C, int64_t win, int64_t left, int64_t dil,
+                            int dtype, int backward, int has_bias, int wants_bias_grad);
+
 /* Force a kernel family for the fused entry points: -1 = automatic (default), 0 = CUDA-core,
  * 1 = tcgen05/TMA (the flat tiling wherever it can run, else the segmented one; for the unfused entry points: also
  * where the automatic choice would take a CUDA-core kernel), 2 = what the strided entry points run: the segmented tiling, or the

@@ -67,6 +67,8 @@ _lib.na1d_fused_kernel_family.restype = _i32
 _lib.na1d_fused_kernel_family.argtypes = [_i64, _i64, _i64, _i64, _i64, _i64, _i32, _i32]
 _lib.na1d_fused_kernel_tiling.restype = _i32
 _lib.na1d_fused_kernel_tiling.argtypes = [_i64, _i64, _i64, _i64, _i64, _i64, _i32, _i32]
+_lib.na1d_fused_kernel_route.restype = _i32
+_lib.na1d_fused_kernel_route.argtypes = [_i64] * 7 + [_i32] * 4
 _u64 = ctypes.c_uint64
 _lib.na1d_dropout_keep_mask.restype = _i32
 _lib.na1d_dropout_keep_mask.argtypes = [_ptr, _i64, _i64, _f32, _u64]

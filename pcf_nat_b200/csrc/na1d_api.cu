@@ -320,6 +320,15 @@ int na1d_fused_kernel_tiling(int64_t N, int64_t T, int64_t C, int64_t win, int64
     return pick_family(g, backward);
 }
 
+int na1d_fused_kernel_route(int64_t N, int64_t heads, int64_t T, int64_t C, int64_t win, int64_t left, int64_t dil, int dtype, int backward,
+                            int has_bias, int wants_bias_grad) {
+    na1d::Geometry g;
+    if (int s = check_geometry(N, heads, T, C, win, left, dil, dtype, 1.f, g)) return s;
+    if (use_march(g, backward ? Pass::backward : Pass::forward, wants_bias_grad != 0, na1d::dense_strides(g.H, g.T, g.C))) return 4;
+    if (const int fam = pick_family(g, backward, has_bias != 0, wants_bias_grad != 0)) return fam;
+    return use_mma(g, dtype == NA1D_FP16, backward ? wants_bias_grad != 0 : has_bias != 0, backward != 0) ? 3 : 0;
+}
+
 int na1d_set_kernel_family(int family) {
     if (family < -1 || family > 5) family = -1;
     return g_family_override.exchange(family);

@@ -201,7 +201,7 @@ def fused_forward_strided(q, k, v, o, win, left, dil=1, scale=1.0, rpb=None, val
     """Fused forward on strided views: q, k, v, o are (batch, heads, T, C) VIEWS (any batch/head/token strides that are
     multiples of 8 elements, channel stride 1), e.g. the slices of a packed projection output and an output buffer laid
     out (batch, T, heads, C). Writes o in place and returns lse (batch*heads, T) fp32. Raises ``Na1dError`` with status
-    -10 when the tcgen05 kernels cannot take the shape (the caller then makes dense copies)."""
+    -10 for shapes outside the segmented tiling's (the caller then makes dense copies)."""
     _need_cuda(q, k, v, o)
     B, H, T, C = q.shape
     assert k.shape == q.shape and v.shape == q.shape and o.shape == q.shape and q.dtype == k.dtype == v.dtype == o.dtype
@@ -241,8 +241,8 @@ class NA1dFusedPackedFunction(torch.autograd.Function):
     """The fused layer core on a PACKED projection output: ``qkv`` is (batch, T, 3*heads*C) as the channels-last ``qkv``
     projection writes it (models/MFA_NATransformer.py:127: viewed as (batch, T, 3, heads, C)), the result is
     (batch, T, heads*C) as the output projection reads it (:151-152). The head split, the head merge and their autograd
-    copies do not exist: the kernels address q, k, v, o, d_o, dq, dk, dv through strided tensor maps. Saves (qkv, lse) only
-    -- the tcgen05 backward needs neither o nor the probabilities."""
+    copies do not exist: the kernels address q, k, v, o, d_o, dq, dk, dv by their strides. Saves (qkv, lse) only -- these
+    backward kernels need neither o nor the probabilities."""
 
     @staticmethod
     def forward(ctx, qkv, heads, win_size, left, dilation=1, scale=1.0, rpb=None, valid_len=None):
@@ -380,15 +380,23 @@ def set_kernel_family(family):
 
 
 def kernel_family(N, T, C, win, left, dil, dtype, backward=False):
-    """0 = CUDA-core kernels, 1 = tcgen05/TMA kernels, negative = status code (forced family unsupported)."""
+    """0 = general kernels, 1 = tcgen05/TMA kernels (where the marching ones do not take the call: see ``kernel_route``), negative =
+    status code (forced family unsupported)."""
     code = _lib.NA1D_BF16 if dtype == torch.bfloat16 else _lib.NA1D_FP16
     return _L.na1d_fused_kernel_family(N, T, C, win, left, dil, code, 1 if backward else 0)
 
 
 def kernel_tiling(N, T, C, win, left, dil, dtype, backward=False):
-    """0 = CUDA-core kernels, 1 = tcgen05 on the flat tiling, 2 = tcgen05 on the segmented tiling, negative = status code."""
+    """0 = general kernels, 1 = tcgen05 on the flat tiling, 2 = tcgen05 on the segmented tiling, negative = status code."""
     code = _lib.NA1D_BF16 if dtype == torch.bfloat16 else _lib.NA1D_FP16
     return _L.na1d_fused_kernel_tiling(N, T, C, win, left, dil, code, 1 if backward else 0)
+
+
+def kernel_route(N, heads, T, C, win, left, dil, dtype, backward=False, has_bias=False, wants_bias_grad=False):
+    """The kernels that a dense fused call runs: 0 = CUDA-core, 1 = tcgen05 flat, 2 = tcgen05 segmented, 3 = warp-level products,
+    4 = marching warps, negative = status code."""
+    code = _lib.NA1D_BF16 if dtype == torch.bfloat16 else _lib.NA1D_FP16
+    return _L.na1d_fused_kernel_route(N, heads, T, C, win, left, dil, code, int(backward), int(has_bias), int(wants_bias_grad))
 
 
 def tensor_map_cache_stats():

@@ -106,3 +106,16 @@ def test_kernel_tiling_choice_is_a_host_side_query():
     assert L.na1d_fused_strided_supported(4, 300, 64, 7, 3, 1, 0, 1, 1) == 1
     assert L.na1d_fused_strided_supported(4, 300, 24, 7, 3, 1, 0, 1, 1) < 0 or L.na1d_fused_strided_supported(4, 300, 24, 7, 3, 1, 0, 1, 1) == 0
     assert L.na1d_fused_strided_supported(4, 300, 64, 31, 15, 1, 0, 1, 1) == 0        # no room for the bias tables of 4 heads
+
+
+def test_kernel_route_is_a_host_side_query():
+    """0 = CUDA cores, 1 and 2 = tcgen05, 3 = warp-level products, 4 = marching warps (no device work)."""
+    r = lambda N, H, T, C, win, dil=1, bw=0, grad=0, dtype=0: L.na1d_fused_kernel_route(N, H, T, C, win, win // 2, dil, dtype, bw, grad, grad)
+    assert r(512, 4, 200, 64, 7) == 1 and r(512, 4, 200, 64, 7, bw=1) == 1 and r(256, 4, 1000, 64, 31, 4) == 2
+    assert r(8192, 16, 150, 16, 27) == 4 and r(8192, 16, 150, 16, 27, bw=1, grad=1) == 4
+    assert r(16384, 16, 36, 16, 27) == 4 and r(16384, 16, 36, 16, 27, bw=1) == 1        # 36 of 48 rows: the flat tiling's backward
+    assert r(64, 16, 36, 16, 27, bw=1) == 4
+    assert r(64, 4, 200, 32, 7) == 4 and r(64, 4, 200, 32, 7, bw=1) == 1 and r(4096, 4, 200, 32, 7) == 1
+    assert r(256, 4, 203, 48, 41) == 3 and r(256, 4, 203, 48, 41, bw=1) == 3 and r(256, 4, 203, 192, 41) == 0
+    assert r(256, 4, 20, 8, 5, 4) == 0 and r(256, 4, 20, 8, 5, 4, bw=1, grad=1) == 0    # residues of five rows
+    assert r(4, 4, 200, 12, 7) == -2
