@@ -88,10 +88,10 @@ struct MarchCost {
                1e-3 * (g.N * (blocks * (block + tile * tiles + w.C * (channel + tile_channel * tiles)) + sequence * w.C * tiles) + entry * w.rows * w.win);
     }
 };
-// Which kernels run an unfused operator: the cheapest by these models, where the kernels that are the most natural ones for the shape
-// (tcgen05 where they take it, else CUDA-core) are left only for a gain of 10 %, the models' error. Over 700 drawn calls the chosen
-// kernels take 0.89 (q.k), 0.72 (a.v) and 0.70 (transposed) of those kernels' time, geometric mean; 2 % of the calls are more than 3 %
-// slower, at most 1.17 times. Kernels that would lose bits are not candidates:
+// Which kernels run an unfused operator: the cheapest by these models, where the kernels that are the natural ones for the shape (tcgen05
+// where they take it, else CUDA-core) are left only for a predicted gain of 20 %. Over 700 drawn calls the chosen kernels take 0.91 (q.k),
+// 0.72 (a.v) and 0.71 (transposed) of those kernels' time, geometric mean; 1 % of the calls are more than 3 % slower, at most 1.16 times. (A
+// gain of 10 % gives 0.89, 0.72 and 0.70, and 2 % of the calls slower, up to 1.5 times.) Kernels that would lose bits are no candidates:
 //   q.k        fp32 results: matrix instructions (fp32 sums rounded towards zero, 2 to 3 times the CUDA-core kernels' error) only where
 //              the tcgen05 kernels take the shape;
 //   band . x   the marching form splits the fp32 band into two 16-bit pieces, against one in the tcgen05 kernels: only where those take the
@@ -119,7 +119,7 @@ Unfused pick_unfused(const na1d::Geometry& g, const UnfusedCosts& costs, bool tc
     if (forced == 3 || forced == 4) return warp_ok ? Unfused::warp : Unfused::core;
     if (forced == 1 && tc_takes) return Unfused::tcgen05;
     const Work w(g, 128);
-    const double natural = 0.9;
+    const double natural = 0.8;
     double best = costs.core(w) * (tc_first ? 1. : natural);
     Unfused pick = Unfused::core;
     auto consider = [&](Unfused u, double cost) { if (cost < best) { best = cost; pick = u; } };
