@@ -79,53 +79,67 @@ struct TileCost {
         return start + 1e-3 * w.rows * (row + channel * w.C + bucket[weff <= 9 ? 0 : weff <= 17 ? 1 : 2] + neighbour * w.win);
     }
 };
-// marching kernels: 16-row blocks, two or three key tiles each; whole lines of the band
-struct MarchCost {
-    double start, tile_start, block, tile, channel, tile_channel, sequence, entry;
-    double operator()(const Work& w, const na1d::Geometry& g) const {
-        const double tiles = g.win <= 17 ? 2 : 3, blocks = (g.T + 15) / 16;
-        return start + tile_start * tiles +
-               1e-3 * (g.N * (blocks * (block + tile * tiles + w.C * (channel + tile_channel * tiles)) + sequence * w.C * tiles) + entry * w.rows * w.win);
-    }
-};
-// Which kernels run an unfused operator: the cheapest by these models, where the kernels that are the natural ones for the shape (tcgen05
-// where they take it, else CUDA-core) are left only for a predicted gain of 20 %. Over 700 drawn calls the chosen kernels take 0.91 (q.k),
-// 0.72 (a.v) and 0.71 (transposed) of those kernels' time, geometric mean; 1 % of the calls are more than 3 % slower, at most 1.16 times. (A
-// gain of 10 % gives 0.89, 0.72 and 0.70, and 2 % of the calls slower, up to 1.5 times.) Kernels that would lose bits are no candidates:
+// Which kernels run an unfused operator. Kernels that would lose bits are no candidates:
 //   q.k        fp32 results: matrix instructions (fp32 sums rounded towards zero, 2 to 3 times the CUDA-core kernels' error) only where
 //              the tcgen05 kernels take the shape;
 //   band . x   the marching form splits the fp32 band into two 16-bit pieces, against one in the tcgen05 kernels: only where those take the
 //              shape;
-//   transposed as band . x, with three bf16 pieces and so at any window; not for fp16, whose pieces lack the band's exponents.
+//   transposed as band . x, with three bf16 pieces; not for fp16, whose pieces lack the band's exponents.
+// Dilation 1, windows up to 33, 32 tokens and more (570 drawn calls; us are CUDA core / tcgen05 / warp-level / marching): the marching
+// kernels at 16, 32 and 64 channels, but
+//   for few products a row the CUDA cores (8192 x 150 rows of 16 channels, window 3: 22 / 40 / 52 / 24; window 5, a.v: 29 / 57 / 76 / 37);
+//   at 64 channels the tcgen05 kernels in q.k up to window 30 (1089 x 126 rows, window 30: 65 / 10 / 14 / 12; 3456 x 150, window 33: 253 /
+//   55 / 70 / 41), and in a.v of large calls with narrow windows or blocks of 16 with many empty rows (13886 x 33 rows, window 8: 52 / 34 /
+//   114 / 42; 3456 x 150, window 27: 167 / 49 / 85 / 41);
+//   transposed fp16 bands go to the CUDA cores, for large calls to tcgen05 at 64 channels and windows up to 17 and at 32 channels and windows
+//   up to 20 or short sequences (19636 x 34 rows of 64 channels, window 10: 99 / 86 / 160; 3773 x 40 of 32, window 18: 22 / 18 / 23), else
+//   to the warp-level kernels (6912 x 150 rows of 32 channels, window 27: 191 / 159 / 122).
+// They take 0.81 (q.k), 0.64 (a.v), 0.59 and 0.66 (transposed, bf16 and fp16) of the time that tcgen05 and, where it does not run, the CUDA
+// cores take; 5 of 1140 calls are more than 3 % slower than those, at most 1.12 times.
+// Everything else by the cost models, where the kernels that are natural for the shape (tcgen05 where they take it, else CUDA-core) are left
+// for a predicted gain of 10 %, the models' error: 0.82 (a.v) and 0.82 (transposed) of the CUDA cores' time over 340 calls, 2 % of them more
+// than 3 % slower, at most 1.16 times.
 enum class Unfused { core, tcgen05, warp, march };
-struct UnfusedCosts {
-    CoreCost core;
-    TileCost tile;
-    WarpCost warp;
-    MarchCost march;
-};
-constexpr UnfusedCosts kQkCosts{{1.43, 0.244, 0.0796, 0.000374, 0.000189, 0.00513}, {3.04, 0.00879, 0.000315, {0.0115, 0.0131, 0.0128}, 0.000645},
-                                {}, {1.64, 0.308, 0.0223, 0.0533, 0.00831, 0.000748, 0., 0.000358}};
-constexpr UnfusedCosts kRowsCosts{{1.41, 0.21, 0.0513, 0.000358, 0.000125, 0.00132}, {4.24, 0.0226, 0.000466, {0.00737, 0.0148, 0.0317}, 6.87e-05},
-                                  {1.37, 0.406, 0.00316, 1.6, 0.0183, 0.115, 0.}, {2.41, 0.0754, 0.126, 0.0449, 0.00576, 0.00297, 0.000666, 0.000212}};
-constexpr UnfusedCosts kTransposedCosts{{1.4, 0.227, 0.0541, 0.000319, 0.000147, 0.00113}, {4.56, 0.0293, 0.000547, {0.00252, 0.022, 0.0421}, 0.000407},
-                                        {0.808, 0.685, 0.00327, 1.63, 0.0211, 0.139, 0.}, {1.26, 0.823, 0.0867, 0.0504, 0.00501, 0.00428, 0.000604, 0.000212}};
-// tc_takes: the tcgen05 kernel takes the call; tc_first: and is the natural one; warp_as_good, march_as_good: those lose no bits
-Unfused pick_unfused(const na1d::Geometry& g, const UnfusedCosts& costs, bool tc_takes, bool tc_first, bool warp_as_good, bool march_as_good) {
-    const int forced = g_family_override.load();
+enum class Op { products, rows, transposed };
+Unfused pick_unfused(const na1d::Geometry& g, Op op, int dtype, bool aligned_band) {
+    const int forced = g_family_override.load(), weff = (g.win - 1) * g.dil + 1;
     const bool warp_ok = na1d::mma_band_supports(g), march_ok = na1d::march_band_supports(g);
+    const bool tiles = na1d::tc_unfused_supports(g) && aligned_band, tc = op == Op::transposed ? na1d::tc_unfused_t_supports(g) : tiles;
     if (forced == 0) return Unfused::core;
     if (forced == 4 && march_ok) return Unfused::march;
     if (forced == 3 || forced == 4) return warp_ok ? Unfused::warp : Unfused::core;
-    if (forced == 1 && tc_takes) return Unfused::tcgen05;
+    if (forced == 1 && tc) return Unfused::tcgen05;
+    // the tcgen05 form of the transposed product gathers the band along its diagonals: at 16 channels not for windows above 17
+    const bool tc_first = tc && !(op == Op::transposed && g.C == 16 && weff > 17);
+    if (g.dil == 1 && tiles && march_ok && warp_ok) {
+        const int products = g.C * g.win, blocks = (g.T + 15) / 16;
+        const bool large = (long long)g.N * g.T > 100000, wide = g.C == 64;
+        switch (op) {
+            case Op::products: return products <= 64 ? Unfused::core : wide && g.win <= 30 ? Unfused::tcgen05 : Unfused::march;
+            case Op::rows:
+                if (products <= 112 || (wide && large && g.win <= 3)) return Unfused::core;
+                return wide && large && (g.win <= 8 || g.T < 0.87 * 16 * blocks) ? Unfused::tcgen05 : Unfused::march;
+            default:
+                if (dtype == NA1D_BF16) return products <= (wide ? 192 : 112) ? Unfused::core : Unfused::march;
+                if (products <= (g.C == 16 && large ? 340 : 288)) return Unfused::core;
+                if (tc_first && wide && (large || g.win <= 9)) return Unfused::tcgen05;
+                if (tc_first && g.C == 32 && large && (g.win <= 20 || g.T < 0.8 * 16 * blocks)) return Unfused::tcgen05;
+                return Unfused::warp;
+        }
+    }
+    constexpr CoreCost core[3] = {{1.43, 0.244, 0.0796, 0.000374, 0.000189, 0.00513}, {1.41, 0.21, 0.0513, 0.000358, 0.000125, 0.00132},
+                                  {1.4, 0.227, 0.0541, 0.000319, 0.000147, 0.00113}};
+    constexpr TileCost tile[3] = {{3.04, 0.00879, 0.000315, {0.0115, 0.0131, 0.0128}, 0.000645}, {4.24, 0.0226, 0.000466, {0.00737, 0.0148, 0.0317}, 6.87e-05},
+                                  {4.56, 0.0293, 0.000547, {0.00252, 0.022, 0.0421}, 0.000407}};
+    constexpr WarpCost warp[3] = {{}, {1.37, 0.406, 0.00316, 1.6, 0.0183, 0.115, 0.}, {0.808, 0.685, 0.00327, 1.63, 0.0211, 0.139, 0.}};
     const Work w(g, 128);
-    const double natural = 0.8;
-    double best = costs.core(w) * (tc_first ? 1. : natural);
+    const int i = (int)op;
+    const double natural = 0.9;
+    double best = core[i](w) * (tc_first ? 1. : natural);
     Unfused pick = Unfused::core;
     auto consider = [&](Unfused u, double cost) { if (cost < best) { best = cost; pick = u; } };
-    if (tc_first) consider(Unfused::tcgen05, natural * costs.tile(w, (g.win - 1) * g.dil + 1));
-    if (warp_ok && warp_as_good) consider(Unfused::warp, costs.warp(w));
-    if (march_ok && march_as_good) consider(Unfused::march, costs.march(w, g));
+    if (tc_first) consider(Unfused::tcgen05, natural * tile[i](w, weff));
+    if (warp_ok && op != Op::products) consider(Unfused::warp, warp[i](w));
     return pick;
 }
 
@@ -143,22 +157,26 @@ template <typename... P> int check_pointers(const P*... p) {
 #define NA1D_REQUIRE_PTR(p) do { if ((p) == nullptr) return NA1D_ERR_NULL_POINTER; } while (0)
 #define NA1D_REQUIRE_ALIGNED(p) do { if (!aligned16(p)) return NA1D_ERR_MISALIGNED; } while (0)
 
-// Of the general kernels (na1d_mma.cu, na1d_simt.cu) the cheaper one by the models above, the warp-level one for a gain of 15 %, and not
-// for residues of fewer than eight rows, which leave most of a 16-row block empty: over 400 drawn calls 0.46 of the CUDA-core
-// kernels' time in the forward and 0.42 in the backward, geometric mean; six calls are more than 3 % slower, at most 1.5 times (a window of
-// 76 on sequences of 15 rows). 256 x 300 rows of 48 channels, window 3, take 8 us on the CUDA cores and 11 here forward, 50 and 32 backward;
-// 2048 x 20 rows with dilation 4, window 15, 11 and 30, 66 and 112.
+// Of the general kernels (na1d_mma.cu, na1d_simt.cu) the cheaper one by the models above, the warp-level one for a gain of 10 %: over 400
+// drawn calls 0.46 of the CUDA-core kernels' time in the forward and 0.42 in the backward, geometric mean; six of the 800 are more than 3 %
+// slower, at most 1.5 times (a window of 76 on sequences of 15 rows). Few neighbours of short residues stay on the CUDA cores: 2048 x 20 rows
+// of 48 channels with dilation 4, window 15, take 11 us there and 30 here forward, 66 and 112 backward.
 bool use_mma(const na1d::Geometry& g, bool fp16, bool has_bias, bool backward) {
     const int forced = g_family_override.load();
     if (forced == 0 || !na1d::mma_supports(g)) return false;
     if (forced == 3 || forced == 4) return true;
-    if ((g.T + g.dil - 1) / g.dil < 8) return false;
+    if ((g.T + g.dil - 1) / g.dil < 8 && g.win < 8) return false;
     const Work w(g, 64);
-    // a bias (its gradient, in the backward) costs the CUDA-core kernels per neighbour; fp16 weights go through products of half the depth
-    const double bias = has_bias ? w.win * (backward ? 0.797 + 1e-3 * w.rows * 0.0181 : 0.0106 + 1e-3 * w.rows * 0.00027) : 0.;
-    const double core = bias + (backward ? CoreCost{4.13, 0.511, 0.226, 0.00243, 0.000915, 0.00877} : CoreCost{1.86, 0.452, 0.174, 0.000349, 0.00034, 0.00663})(w);
-    const double mma = (backward ? WarpCost{3.19, 0.208, 0.00994, 1.84, 0.107, 0., 0.} : WarpCost{2.52, 0.177, 0.00392, 1.39, 0.0177, 0.146, fp16 ? 0.00344 : 0.00103})(w);
-    return mma < 0.85 * core;
+    // fp16 weights go through products of half the depth
+    const double mma = (backward ? WarpCost{3.19, 0.208, 0.00994, 1.84, w.CP > 64 ? 0.14 : 0.1, 0., 0.} : WarpCost{2.52, 0.177, 0.00392, 1.39, 0.0177, 0.146, fp16 ? 0.00344 : 0.00103})(w);
+    double core = (backward ? CoreCost{3.93, 0.505, 0.267, 0.00224, 0.000938, 0.00919} : CoreCost{1.86, 0.455, 0.179, 0.00035, 0.000339, 0.00659})(w);
+    if (has_bias && !backward) core += 1e-3 * w.rows * w.win * 0.000319;
+    if (has_bias && backward) {   // its gradient: the rows that share a warp add to the same entry, one after the other
+        int lanes = 1, units = g.C / 8;
+        while (lanes < 8 && units % 2 == 0) { lanes *= 2; units /= 2; }
+        core += w.win * (0.0779 * (32 / lanes) + 1e-3 * w.rows * (units == 3 ? 0.039 : 0.013));
+    }
+    return mma < 0.9 * core;
 }
 
 // The marching kernels: 16-channel rows in everything; 32-channel rows in the forward, where they stand for the segmented tiling
@@ -217,10 +235,7 @@ int na1d_qk_forward(float* attn, const void* q, const void* k, int64_t N, int64_
     NA1D_REQUIRE_ALIGNED(q); NA1D_REQUIRE_ALIGNED(k);
     na1d::Geometry g;
     if (int s = check_geometry(N, 1, T, C, win, left, dil, dtype, 1.f, g)) return s;
-    // us at 8192 x 150 rows (6912, 3456 at 32, 64 channels), CUDA core / tcgen05 / marching: 16 channels, window 3: 22 / 40 / 23, window
-    // 27: 183 / 58 / 42; 32 channels, window 3: 39 / 45 / 31; 64 channels, window 9: 82 / 31 / 32, window 33: 253 / 55 / 41
-    const bool tc = na1d::tc_unfused_supports(g) && aligned16(attn);   // (the tcgen05 band goes out in 16-byte stores)
-    switch (pick_unfused(g, kQkCosts, tc, tc, false, tc)) {
+    switch (pick_unfused(g, Op::products, dtype, aligned16(attn))) {   // (the tcgen05 band goes out in 16-byte stores)
         case Unfused::tcgen05: return cuda_status(na1d::tc_qk(attn, q, k, g, dtype, (cudaStream_t)stream));
         case Unfused::march: return cuda_status(na1d::march_band_out(attn, q, k, g, dtype, (cudaStream_t)stream));
         case Unfused::warp: return cuda_status(na1d::mma_band_out(attn, q, k, g, dtype, (cudaStream_t)stream));
@@ -237,10 +252,7 @@ int na1d_q_backward(void* q_gd, const float* attn_gd, const void* k, int64_t N, 
     NA1D_REQUIRE_ALIGNED(q_gd); NA1D_REQUIRE_ALIGNED(k);
     na1d::Geometry g;
     if (int s = check_geometry(N, 1, T, C, win, left, dil, dtype, 1.f, g)) return s;
-    // as above: 16 channels, window 5: 29 / 58 / 35, window 27: 106 / 82 / 49; 32 channels, window 3: 34 / 52 / 39, window 27: 167 / 78 / 57;
-    // 64 channels, window 3: 34 / 37 / 36, window 27: 167 / 48 / 45
-    const bool tc = na1d::tc_unfused_supports(g);
-    switch (pick_unfused(g, kRowsCosts, tc, tc, true, tc)) {
+    switch (pick_unfused(g, Op::rows, dtype, true)) {
         case Unfused::tcgen05: return cuda_status(na1d::tc_band_x(q_gd, attn_gd, k, g, dtype, (cudaStream_t)stream));
         case Unfused::march: return cuda_status(na1d::march_band_rows(q_gd, attn_gd, k, false, g, dtype, (cudaStream_t)stream));
         case Unfused::warp: return cuda_status(na1d::mma_band_rows(q_gd, attn_gd, k, false, g, dtype, (cudaStream_t)stream));
@@ -257,11 +269,7 @@ int na1d_k_backward(void* k_gd, const float* attn_gd, const void* q, int64_t N, 
     NA1D_REQUIRE_ALIGNED(k_gd); NA1D_REQUIRE_ALIGNED(q);
     na1d::Geometry g;
     if (int s = check_geometry(N, 1, T, C, win, left, dil, dtype, 1.f, g)) return s;
-    // as above, with the warp-level kernels third: 16 channels, window 5: 31 / 84 / 75 / 39, window 27: 120 / 187 / 103 / 53; 32 channels,
-    // window 27: 191 / 159 / 107 / 56; 64 channels, window 3: 35 / 42 / 65 / 36, window 27: 188 / - / 88 / 51. The tcgen05 form gathers the
-    // band along its diagonals; at 16 channels it does not pay for windows above 17.
-    const bool tc = na1d::tc_unfused_t_supports(g), wide = g.C == 16 && (g.win - 1) * g.dil + 1 > 17;
-    switch (pick_unfused(g, kTransposedCosts, tc, tc && !wide, true, dtype == NA1D_BF16 && na1d::tc_unfused_supports(g))) {
+    switch (pick_unfused(g, Op::transposed, dtype, true)) {
         case Unfused::tcgen05: return cuda_status(na1d::tc_bandT_x(k_gd, attn_gd, q, g, dtype, (cudaStream_t)stream));
         case Unfused::march: return cuda_status(na1d::march_band_rows(k_gd, attn_gd, q, true, g, dtype, (cudaStream_t)stream));
         case Unfused::warp: return cuda_status(na1d::mma_band_rows(k_gd, attn_gd, q, true, g, dtype, (cudaStream_t)stream));
