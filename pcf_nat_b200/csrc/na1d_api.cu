@@ -84,13 +84,14 @@ struct TileCost {
 //              the tcgen05 kernels take the shape;
 //   band . x   the marching form splits the fp32 band into two 16-bit pieces, against one in the tcgen05 kernels: only where those take the
 //              shape;
-//   transposed as band . x, with three bf16 pieces; not for fp16, whose pieces lack the band's exponents.
+//   transposed as band . x, and with three bf16 pieces where the CUDA cores stood; not for fp16, whose pieces lack the band's exponents.
 // Dilation 1, windows up to 33, 32 tokens and more (570 drawn calls; us are CUDA core / tcgen05 / warp-level / marching): the marching
 // kernels at 16, 32 and 64 channels, but
 //   for few products a row the CUDA cores (8192 x 150 rows of 16 channels, window 3: 22 / 40 / 52 / 24; window 5, a.v: 29 / 57 / 76 / 37);
 //   at 64 channels the tcgen05 kernels in q.k up to window 30 (1089 x 126 rows, window 30: 65 / 10 / 14 / 12; 3456 x 150, window 33: 253 /
 //   55 / 70 / 41), and in a.v of large calls with narrow windows or blocks of 16 with many empty rows (13886 x 33 rows, window 8: 52 / 34 /
 //   114 / 42; 3456 x 150, window 27: 167 / 49 / 85 / 41);
+//   transposed, large calls of 64 channels with windows of 4 and 5 on tcgen05 (448 x 547 rows, window 4: 18 us, marching 23);
 //   transposed fp16 bands go to the CUDA cores, for large calls to tcgen05 at 64 channels and windows up to 17 and at 32 channels and windows
 //   up to 20 or short sequences (19636 x 34 rows of 64 channels, window 10: 99 / 86 / 160; 3773 x 40 of 32, window 18: 22 / 18 / 23), else
 //   to the warp-level kernels (6912 x 150 rows of 32 channels, window 27: 191 / 159 / 122).
@@ -120,7 +121,7 @@ Unfused pick_unfused(const na1d::Geometry& g, Op op, int dtype, bool aligned_ban
                 if (products <= 112 || (wide && large && g.win <= 3)) return Unfused::core;
                 return wide && large && (g.win <= 8 || g.T < 0.87 * 16 * blocks) ? Unfused::tcgen05 : Unfused::march;
             default:
-                if (dtype == NA1D_BF16) return products <= (wide ? 192 : 112) ? Unfused::core : Unfused::march;
+                if (dtype == NA1D_BF16) return products <= (wide ? 192 : 112) ? Unfused::core : wide && large && g.win <= 5 && tc ? Unfused::tcgen05 : Unfused::march;
                 if (products <= (g.C == 16 && large ? 340 : 288)) return Unfused::core;
                 if (tc_first && wide && (large || g.win <= 9)) return Unfused::tcgen05;
                 if (tc_first && g.C == 32 && large && (g.win <= 20 || g.T < 0.8 * 16 * blocks)) return Unfused::tcgen05;
@@ -158,7 +159,7 @@ template <typename... P> int check_pointers(const P*... p) {
 #define NA1D_REQUIRE_ALIGNED(p) do { if (!aligned16(p)) return NA1D_ERR_MISALIGNED; } while (0)
 
 // Of the general kernels (na1d_mma.cu, na1d_simt.cu) the cheaper one by the models above, the warp-level one for a gain of 10 %: over 400
-// drawn calls 0.46 of the CUDA-core kernels' time in the forward and 0.42 in the backward, geometric mean; six of the 800 are more than 3 %
+// drawn calls 0.46 of the CUDA-core kernels' time in the forward and 0.42 in the backward, geometric mean; eleven of the 800 are more than 3 %
 // slower, at most 1.5 times (a window of 76 on sequences of 15 rows). Few neighbours of short residues stay on the CUDA cores: 2048 x 20 rows
 // of 48 channels with dilation 4, window 15, take 11 us there and 30 here forward, 66 and 112 backward.
 bool use_mma(const na1d::Geometry& g, bool fp16, bool has_bias, bool backward) {
@@ -168,7 +169,7 @@ bool use_mma(const na1d::Geometry& g, bool fp16, bool has_bias, bool backward) {
     if ((g.T + g.dil - 1) / g.dil < 8 && g.win < 8) return false;
     const Work w(g, 64);
     // fp16 weights go through products of half the depth
-    const double mma = (backward ? WarpCost{3.19, 0.208, 0.00994, 1.84, w.CP > 64 ? 0.14 : 0.1, 0., 0.} : WarpCost{2.52, 0.177, 0.00392, 1.39, 0.0177, 0.146, fp16 ? 0.00344 : 0.00103})(w);
+    const double mma = (backward ? WarpCost{3.19, 0.208, 0.00994, 1.84, 0.1, 0., 0.} : WarpCost{2.52, 0.177, 0.00392, 1.39, 0.0177, 0.146, fp16 ? 0.00344 : 0.00103})(w);
     double core = (backward ? CoreCost{3.93, 0.505, 0.267, 0.00224, 0.000938, 0.00919} : CoreCost{1.86, 0.455, 0.179, 0.00035, 0.000339, 0.00659})(w);
     if (has_bias && !backward) core += 1e-3 * w.rows * w.win * 0.000319;
     if (has_bias && backward) {   // its gradient: the rows that share a warp add to the same entry, one after the other

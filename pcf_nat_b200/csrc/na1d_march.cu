@@ -20,7 +20,7 @@
 // Backward: key tile i collects from blocks i - NT + 1 .. i and is stored when block i is done. A strip owns the key tiles of its
 // own blocks and recomputes the NT - 1 blocks before it (nothing to recompute when the strip is a whole sequence).
 // Measured at 512 x 16 x 150 rows (tcgen05 flat / segmented tiling / here, us): window 27 forward 76 / 135 / 51, backward
-// 141 / 194 / 122; window 9 forward 62 / 104 / 40, backward 99 / 154 / 90; 64 x 16 x 997 rows, window 27: 66 / 66 / 37 and
+// 141 / 193 / 116; window 9 forward 62 / 104 / 40, backward 101 / 154 / 89; 64 x 16 x 997 rows, window 27: 66 / 66 / 37 and
 // 115 / 119 / 98. The forward is bound by instruction issue (0.67 a cycle), the backward by latency at twelve warps an SM.
 // Forward at 32 channels: 512 x 300 rows, window 27: 16 / 20 / 13; 4096 x 150: 49 / 85 / 51; the backward there needs more registers
 // than a thread has and stays on tcgen05 (82 / 107 against 118).
@@ -517,13 +517,13 @@ __global__ void __launch_bounds__(kWarps * 32, NT == 3 ? 3 : 4) march_bwd_kernel
 // order (pitch 8 mod 32 words: 8-byte accesses without bank conflicts). Positions outside the band are never written and
 // stay zero. The patch offsets of a lane's elements are the same in every block and are kept in registers.
 // Measured (tcgen05 / warp-level products on 128-row tiles / here, us; HBM time is 33, 38 and 26):
-// 8192 x 150 x 16, window 27: q.k 58 / 67 / 42, a.v 82 / 93 / 49, transposed 187 (CUDA core 120) / 103 / 53;
-// 6912 x 150 x 32, window 27: 54 / 72 / 47, 78 / 97 / 57, 159 / 107 / 56; 3456 x 150 x 64, window 17: 33 / 52 / 34, 42 / 70 / 39,
-// 76 / 74 / 38.
+// 8192 x 150 x 16, window 27: q.k 58 / 67 / 42, a.v 81 / 102 / 49, transposed 182 (CUDA core 120) / 116 / 59 (three pieces);
+// 6912 x 150 x 32, window 27: 54 / 72 / 47, 78 / 106 / 53, 159 / 122 / 56; 3456 x 150 x 64, window 17: 33 / 52 / 33, 42 / 73 / 38,
+// 76 / 75 / 38.
 //   march_qk  : band[t, kk] = a[t] . b[j]             (QK forward, dA)
 //   march_rows: out[t] = sum band[t, kk] x[j]         (AV forward, dQ), or TRANSPOSED out[j] = sum band[t, kk] x[t] (dV, dK)
-// The band enters the products as two 16-bit pieces where the tcgen05 kernels round it to one, as three bf16 pieces (all its bits) in the
-// transposed product, which the CUDA cores take at some of these windows. A result that is not finite is computed again, row by row in fp32: the
+// The band enters the products as two 16-bit pieces where the tcgen05 kernels round it to one; the transposed product at 16 and 64 channels
+// and windows above 17, which those leave to the CUDA cores, takes three bf16 pieces, all its bits (10 % of that kernel's time). A result that is not finite is computed again, row by row in fp32: the
 // zeros outside the band must not meet an infinite row.
 template <int NT> constexpr int kPatchPitch = 16 * NT + 8;
 template <int NT> constexpr int kPatchIters = (16 * (16 * NT - 15) + 31) / 32;   // 32-element steps of 16 band rows
@@ -644,7 +644,7 @@ __global__ void __launch_bounds__(kWarps * 32) march_rows_kernel(E* __restrict__
     Rows<KC> xn;
     RowsT<KC> xt[TRANSPOSED ? 1 : NT];
     float acc[TRANSPOSED ? NT : 1][KC][2][4];
-    constexpr int TILES = TRANSPOSED ? 1 : NT, PIECES = TRANSPOSED ? 3 : 2;
+    constexpr int TILES = TRANSPOSED ? 1 : NT, PIECES = TRANSPOSED && NT == 3 && KC != 2 ? 3 : 2;
 #pragma unroll
     for (int t = 0; t < TILES; ++t) {
         xn.load(px, ux, st.Tr);
