@@ -230,6 +230,12 @@ int na1d_gelu_backward(void* dx, float* sums, float* scratch, const void* dy, co
                        void* stream);
 /* sums (F) = column sums of x (rows, F). */
 int na1d_column_sums(float* sums, float* scratch, const void* x, int64_t rows, int64_t F, int dtype, void* stream);
+/* Parameter gradients of `count` (at most 2) projections in one launch: d_w[i] (M[i], N[i]) = dy[i]^T x[i], d_b[i] (M[i]) = column
+ * sums of dy[i]; dy[i] (rows, M[i]) and x[i] (rows, N[i]) 16-bit, results fp32 (out32) or of `dtype`, either may be NULL. Host arrays
+ * of device pointers. Partial sums go through `scratch` and are added in a fixed order. */
+int64_t na1d_projection_gradients_scratch(const int64_t* M, const int64_t* N, int count, int64_t rows);
+int na1d_projection_gradients(void* const* d_w, void* const* d_b, const void* const* dy, const void* const* x, const int64_t* M,
+                              const int64_t* N, int count, int64_t rows, float* scratch, int out32, int dtype, void* stream);
 /* Rounds `count` fp32 tensors (DEVICE pointers in the HOST array src, n[i] elements) to 16 bits at out + dst[i] (elements,
  * multiples of 8; each slot is padded with zeros to a multiple of 8) in one launch; count <= NA1D_CAST_MAX. */
 #define NA1D_CAST_MAX 16

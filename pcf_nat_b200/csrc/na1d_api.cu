@@ -353,7 +353,7 @@ int na1d_tensor_map_cache_stats(int64_t* hits, int64_t* misses) {
 
 int na1d_device_status(void) {
     // every word is read (and cleared) before anything is reported; an expired wait in any kernel wins over a failed read
-    const int words[8] = {na1d::tc_read_status(), na1d::tc_bwd_read_status(), na1d::tc_seg_read_status(),
+    const int words[9] = {na1d::wgrad_read_status(), na1d::tc_read_status(), na1d::tc_bwd_read_status(), na1d::tc_seg_read_status(),
                           na1d::tc_bwd_seg_read_status(), na1d::tc_unfused_read_status(), na1d::tc_unfused_t_read_status(),
                           na1d::tc_drop_read_status(), na1d::tc_bwd_drop_read_status()};
     int v = 0, w = 0;
@@ -587,6 +587,29 @@ int na1d_column_sums(float* sums, float* scratch, const void* x, int64_t rows, i
     if (int s = check_pointers(sums, scratch, x)) return s;
     if (int s = check_block(rows, F, 1 << 20, dtype)) return s;
     return cuda_status(na1d::block_column_sums(sums, scratch, x, (int)rows, (int)F, dtype, (cudaStream_t)stream));
+}
+static int check_gradients(const int64_t* M, const int64_t* N, int count, int64_t rows) {
+    NA1D_REQUIRE_PTR(M); NA1D_REQUIRE_PTR(N);
+    if (count <= 0 || count > 2) return NA1D_ERR_TOO_LARGE;
+    for (int i = 0; i < count; ++i) {
+        if (int s = check_block(rows, M[i], 1 << 20, NA1D_BF16)) return s;
+        if (int s = check_block(rows, N[i], 1 << 20, NA1D_BF16)) return s;
+        if (M[i] * N[i] > (1ll << 37)) return NA1D_ERR_TOO_LARGE;
+    }
+    return NA1D_OK;
+}
+int64_t na1d_projection_gradients_scratch(const int64_t* M, const int64_t* N, int count, int64_t rows) {
+    return check_gradients(M, N, count, rows) == NA1D_OK ? (int64_t)na1d::wgrad_scratch_floats(M, N, count, rows) : 0;
+}
+int na1d_projection_gradients(void* const* d_w, void* const* d_b, const void* const* dy, const void* const* x, const int64_t* M, const int64_t* N, int count,
+                              int64_t rows, float* scratch, int out32, int dtype, void* stream) {
+    NA1D_REQUIRE_PTR(d_w); NA1D_REQUIRE_PTR(d_b); NA1D_REQUIRE_PTR(dy); NA1D_REQUIRE_PTR(x);
+    if (dtype != NA1D_BF16 && dtype != NA1D_FP16) return NA1D_ERR_BAD_DTYPE;
+    if (int s = check_gradients(M, N, count, rows)) return s;
+    if (int s = check_pointers(scratch)) return s;
+    for (int i = 0; i < count; ++i)
+        if (int s = check_pointers(dy[i], x[i])) return s;
+    return cuda_status(na1d::wgrad(d_w, d_b, dy, x, M, N, count, rows, scratch, out32 != 0, dtype, (cudaStream_t)stream));
 }
 int na1d_cast_parameters(void* out, const float* const* src, const int64_t* dst, const int64_t* n, int count, int dtype,
                          void* stream) {

@@ -88,6 +88,13 @@ cudaError_t tc_fused_bwd(void* dq, void* dk, void* dv, float* d_rpb, const void*
                          const void* v, const float* lse, const float* rpb, const int* valid_len, float* scratch,
                          size_t scratch_floats, const Geometry& gm, int dtype, cudaStream_t st);
 
+// ---- parameter gradients of projections (na1d_wgrad.cu): d_w[i] (M, N) = dy[i]^T x[i] with dy (rows, M), x (rows, N), d_b[i] (M) = column
+// sums of dy[i]; either may be null, count <= 2
+size_t wgrad_scratch_floats(const int64_t* M, const int64_t* N, int count, int64_t rows);
+cudaError_t wgrad(void* const* d_w, void* const* d_b, const void* const* dy, const void* const* x, const int64_t* M, const int64_t* N, int count,
+                  int64_t rows, float* scratch, bool out32, int dtype, cudaStream_t st);
+int wgrad_read_status();
+
 // ---- row and column kernels of a transformer block and of the statistics pooling (na1d_block.cu)
 int block_partial_rows(long long rows);
 cudaError_t block_valid_tokens(int* out, const void* padding, bool is64, int n_padding, int N, int T, cudaStream_t st);

@@ -1,6 +1,6 @@
 // Host-side helpers shared by the tcgen05 kernels: TMA tensor maps and device properties.
 #include "na1d_internal.h"
-#include "na1d_tc_common.cuh"
+#include "na1d_pair.cuh"
 #include <atomic>
 #include <cstdlib>
 #include <cstring>
@@ -117,6 +117,14 @@ bool make_seg_tile_maps(CUtensorMap* maps, const void* base, int dtype, int batc
     const cuuint64_t dims_b[5] = {(cuuint64_t)C, (cuuint64_t)(sg.Tp - 1), (cuuint64_t)(sg.d - sg.ra), (cuuint64_t)H, (cuuint64_t)batch};
     const uint8_t* base_b = static_cast<const uint8_t*>(base) + (size_t)sg.ra * st.token * 2;
     return encode_cached(&maps[1], base_b, dtype, 5, dims_b, strides, box, row_swizzle(C));
+}
+
+bool make_matrix_map(CUtensorMap* map, const void* base, int dtype, int rank, const int64_t* dims, const int64_t* strides, const int* box) {
+    cuuint64_t d[3], s[2];
+    cuuint32_t b[3];
+    for (int i = 0; i < rank; ++i) { d[i] = (cuuint64_t)dims[i]; b[i] = (cuuint32_t)box[i]; }
+    for (int i = 0; i + 1 < rank; ++i) s[i] = (cuuint64_t)strides[i] * 2;
+    return encode_cached(map, base, dtype, rank, d, s, b, CU_TENSOR_MAP_SWIZZLE_128B);
 }
 
 // Programmatic dependent launch is off unless NA1D_PDL (read once) says otherwise (measured: it shortens back-to-back

@@ -336,6 +336,32 @@ variable_list inner_gradients(const variable_list& outputs, const variable_list&
 }
 
 // ---------------------------------------------------------------- the transformer block
+// Parameter gradients of up to two projections in one launch: d_w = dy^T x and d_b = column sums of dy, of `type` from fp32 sums.
+// dy (rows, M), x (rows, N); what is not wanted stays undefined.
+struct ParameterGrads {
+    Tensor w[2], b[2];
+    ParameterGrads(const Tensor (&dy)[2], const Tensor (&x)[2], const bool (&need_w)[2], const bool (&need_b)[2], at::ScalarType type) {
+        void *pw[2], *pb[2];
+        const void *py[2], *px[2];
+        int64_t M[2], N[2];
+        int n = 0;
+        for (int i = 0; i < 2; ++i) {
+            if (!need_w[i] && !need_b[i]) continue;
+            M[n] = dy[i].size(1);
+            N[n] = x[i].size(1);
+            const auto opts = dy[i].options().dtype(type);
+            if (need_w[i]) w[i] = at::empty({M[n], N[n]}, opts);
+            if (need_b[i]) b[i] = at::empty({M[n]}, opts);
+            pw[n] = ptr(w[i]); pb[n] = ptr(b[i]); py[n] = ptr(dy[i]); px[n] = ptr(x[i]);
+            ++n;
+        }
+        if (n == 0) return;
+        const int64_t rows = dy[0].size(0);
+        const Tensor scratch = empty_f32({na1d_projection_gradients_scratch(M, N, n, rows)}, dy[0]);
+        check(na1d_projection_gradients(pw, pb, py, px, M, N, n, rows, fptr(scratch), type == at::kFloat, code(dy[0]), stream()), "na1d_projection_gradients");
+    }
+};
+
 // Parameters in the order qkv.w, qkv.b, proj.w, proj.b, fc1.w, fc1.b, fc2.w, fc2.b, norm1.w, norm1.b, norm2.w, norm2.b, bias table.
 constexpr int kProj = 8, kParams = 13;
 constexpr int64_t kSlot = 64;   // elements: 128-byte slots of the packed 16-bit parameters
@@ -480,34 +506,28 @@ struct NA1dBlock : public torch::autograd::Function<NA1dBlock> {
         const Tensor scratch = empty_f32({na1d_block_scratch_floats(rows, D, std::max(F, 3 * D))}, s1);
         const Tensor d_z = (grads[1].defined() ? aligned(grads[1]) : at::zeros_like(s2)).view({rows, D});
         const Tensor d_s2 = grads[0].defined() ? aligned(grads[0]) : Tensor();
-        // dy^T . inp, accumulated and returned in fp32
-        auto weight_grad = [&](int k, const Tensor& dy, const Tensor& inp) { return need(k) ? at::mm(dy.t(), inp, at::kFloat) : Tensor(); };
-        auto bias_grad = [&](int k, const Tensor& dy) {
-            if (!need(k)) return Tensor();
-            Tensor sums = empty_f32({dy.size(1)}, dy);
-            check(na1d_column_sums(fptr(sums), fptr(scratch), ptr(dy), rows, dy.size(1), code(dy), stream()), "na1d_column_sums");
-            return sums;
-        };
         // MLP branch
-        Tensor d_w2 = weight_grad(6, d_z, g), d_b2 = bias_grad(7, d_z), d_b1 = empty_f32({F}, s1), d_f = at::empty_like(f);
+        Tensor d_b1 = empty_f32({F}, s1), d_f = at::empty_like(f);
         {
             const Tensor d_g = at::mm(d_z, w.t[6]);
             check(na1d_gelu_backward(ptr(d_f), fptr(d_b1), fptr(scratch), ptr(d_g), ptr(f), rows, F, code(f), stream()), "na1d_gelu_backward");
         }
-        Tensor d_w1 = weight_grad(4, d_f, h2.view({rows, D})), sums2, sums1;
+        const ParameterGrads mlp({d_f, d_z}, {h2.view({rows, D}), g}, {need(4), need(6)}, {false, need(7)}, at::kFloat);
+        Tensor sums2, sums1;
         const Tensor d_y = layer_norm_backward(sums2, at::mm(d_f, w.t[4]), s2, st2, n2w, d_s2, scratch);   // also the residual stream's gradient
         d_f.reset();
         // attention branch
         const Tensor dy2 = d_y.view({rows, D});
-        Tensor d_pw = weight_grad(2, dy2, o.view({rows, D})), d_qkv = at::empty_like(qkv), d_rpb;
+        Tensor d_qkv = at::empty_like(qkv), d_rpb;
         if (need(12)) d_rpb = at::zeros({c.H, c.win}, s1.options().dtype(at::kFloat));
         packed_backward(d_qkv, d_rpb, at::mm(dy2, w.t[2]), qkv, lse, rpb, vl, c);
         const Tensor dq2 = d_qkv.view({rows, 3 * D});
-        Tensor d_qw = weight_grad(0, dq2, h1.view({rows, D})), d_qb = bias_grad(1, dq2);
+        const ParameterGrads att({dq2, dy2}, {h1.view({rows, D}), o.view({rows, D})}, {need(0), need(2)}, {need(1), false}, at::kFloat);
         const Tensor d_x = layer_norm_backward(sums1, at::mm(dq2, w.t[0]), s1, st1, n1w, d_y, scratch);
         if (d_rpb.defined()) d_rpb = d_rpb.view(rpb.sizes());
         const Tensor none;
-        return {d_x, has_dx ? d_x : none, none, none, none, none, none, none, none, d_qw, d_qb, d_pw, sums2.select(0, 2), d_w1, d_b1, d_w2, d_b2,
+        return {d_x, has_dx ? d_x : none, none, none, none, none, none, none, none, att.w[0], att.b[0], att.w[1], sums2.select(0, 2), mlp.w[0], d_b1, mlp.w[1],
+                mlp.b[1],
                 sums1.select(0, 0), sums1.select(0, 1), sums2.select(0, 0), sums2.select(0, 1), d_rpb};
     }
 };
@@ -576,28 +596,23 @@ Tensor transposed(const Tensor& in, const LayerShape& l, bool to_tokens) {
     check(na1d_transpose(ptr(out), ptr(in), l.B, l.D, l.T, to_tokens, code(in), stream()), "na1d_transpose");
     return out;
 }
-// gradients of one projection's parameters, fp32 sums in the parameters' own type, shape and order
-struct ProjectionGrads {
-    Tensor w, b;
-    ProjectionGrads(bool need_w, bool need_b, const Tensor& dy, const Tensor& x, const Tensor& scratch, at::IntArrayRef w_shape, at::ScalarType type,
-                    const LayerShape& l, int parts) {
-        if (!need_w && !need_b) return;
-        Tensor dense, sums;
-        if (need_w) dense = at::mm(dy.t(), x, at::kFloat);
-        if (need_b) {
-            sums = empty_f32({parts * l.D}, dy);
-            check(na1d_column_sums(fptr(sums), fptr(scratch), ptr(dy), dy.size(0), dy.size(1), code(dy), stream()), "na1d_column_sums");
+// gradients of the two projections' parameters, fp32 sums in the parameters' own type, shape and order: 0 = qkv, 1 = proj
+struct LayerGrads {
+    Tensor w[2], b[2];
+    LayerGrads(const bool (&need_w)[2], const bool (&need_b)[2], const Tensor (&dy)[2], const Tensor (&x)[2], const at::IntArrayRef (&w_shape)[2],
+               at::ScalarType type, const LayerShape& l) {
+        const ParameterGrads dense(dy, x, need_w, need_b, l.first ? at::kFloat : type);
+        for (int i = 0; i < 2; ++i) {
+            const int parts = i == 0 ? 3 : 1;
+            w[i] = dense.w[i];
+            b[i] = dense.b[i];
+            if (!l.first || (!need_w[i] && !need_b[i])) continue;
+            const auto opts = dy[i].options().dtype(type);
+            if (need_w[i]) w[i] = at::empty(w_shape[i], opts);
+            if (need_b[i]) b[i] = at::empty({parts * l.D}, opts);
+            check(na1d_unpack_grouped(ptr(w[i]), ptr(b[i]), fptr(dense.w[i]), fptr(dense.b[i]), type == at::kFloat, l.D, l.groups, parts, code(dy[i]), stream()),
+                  "na1d_unpack_grouped");
         }
-        if (!l.first) {
-            if (need_w) w = dense.to(type);
-            if (need_b) b = sums.to(type);
-            return;
-        }
-        const auto opts = dy.options().dtype(type);
-        if (need_w) w = at::empty(w_shape, opts);
-        if (need_b) b = at::empty({parts * l.D}, opts);
-        check(na1d_unpack_grouped(ptr(w), ptr(b), fptr(dense), fptr(sums), type == at::kFloat, l.D, l.groups, parts, code(dy), stream()),
-              "na1d_unpack_grouped");
     }
 };
 // Shapes that the strided entry points do not take (a head size outside theirs, no shared memory left for the bias gradient): the
@@ -698,11 +713,8 @@ struct NA1dLayer : public torch::autograd::Function<NA1dLayer> {
             out.resize(14);
             return out;
         }
-        const Tensor scratch = empty_f32({na1d_block_scratch_floats(l.rows(), 0, 3 * l.D)}, xt);
         Tensor dy = grads[0].defined() ? aligned(grads[0]) : at::zeros(l.first ? at::IntArrayRef({l.B, l.D, l.T}) : xt.sizes(), xt.options());
         dy = (l.first ? transposed(dy, l, true) : dy).view({l.rows(), l.D});
-        ProjectionGrads gp(ctx->needs_input_grad(3), has_pb && ctx->needs_input_grad(pb_edge), dy, o.view({l.rows(), l.D}), scratch,
-                           d["pw_shape"].toIntVector(), type, l, 1);
         Tensor d_qkv = at::empty_like(qkv), d_rpb, d_x;
         if (ctx->needs_input_grad(1)) d_rpb = at::zeros({c.H, c.win}, xt.options().dtype(at::kFloat));
         if (o_dense.defined()) {
@@ -717,15 +729,17 @@ struct NA1dLayer : public torch::autograd::Function<NA1dLayer> {
             packed_backward(d_qkv, d_rpb, at::mm(dy, pw), qkv, lse, rpb32(rpb), vl, c);
         }
         const Tensor dq = d_qkv.view({l.rows(), 3 * l.D});
-        ProjectionGrads gq(ctx->needs_input_grad(2), has_qb && ctx->needs_input_grad(qb_edge), dq, xt.view({l.rows(), l.D}), scratch,
-                           d["qw_shape"].toIntVector(), type, l, 3);
+        const std::vector<int64_t> qw_shape = d["qw_shape"].toIntVector(), pw_shape = d["pw_shape"].toIntVector();
+        const LayerGrads g({ctx->needs_input_grad(2), ctx->needs_input_grad(3)},
+                           {has_qb && ctx->needs_input_grad(qb_edge), has_pb && ctx->needs_input_grad(pb_edge)}, {dq, dy},
+                           {aligned(xt).view({l.rows(), l.D}), o.view({l.rows(), l.D})}, {qw_shape, pw_shape}, type, l);
         if (ctx->needs_input_grad(0)) {
             d_x = at::mm(dq, qw);
             d_x = l.first ? transposed(d_x, l, false) : d_x.view({l.B, l.T, l.D});
         }
         if (d_rpb.defined()) d_rpb = d_rpb.view(rpb.sizes()).to(rpb.scalar_type());
         const Tensor none;
-        return {d_x, d_rpb, gq.w, gp.w, gq.b, gp.b, none, none, none, none, none, none, none, none};
+        return {d_x, d_rpb, g.w[0], g.w[1], g.b[0], g.b[1], none, none, none, none, none, none, none, none};
     }
 };
 
