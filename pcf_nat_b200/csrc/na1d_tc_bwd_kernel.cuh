@@ -300,7 +300,7 @@ tc_bwd_kernel(const __grid_constant__ BwdMaps<SEG ? 2 : 1> tm, float* __restrict
     uint8_t* bias_copy = reinterpret_cast<uint8_t*>(bias_acc + round_up(n_bias, 32));
     const int rows_total = gm.N * gm.T;
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = ptx::warp_index(), lane = tid & 31;
     // flat tiling: the effective (dilated) window, neighbour kk of the reference is offset kk * dil of it;
     // segmented tiling: the dilation lives in the addressing, the window is the reference's own
     const int dil = SEG ? 1 : gm.dil, dmask = dil - 1, dshift = 31 - __clz(dil);
@@ -397,12 +397,13 @@ tc_bwd_kernel(const __grid_constant__ BwdMaps<SEG ? 2 : 1> tm, float* __restrict
         }
     } else if (warp >= kMmaWarp) {
         // ------------------------------------------------------------ MMA issuers
-        // One tcgen05.mma costs its issuing thread about 120 cycles whatever its size (measured), far more than the
+        // One tcgen05.mma costs its issuing thread about 65 cycles whatever its size (measured; 120 to 165 where the compiler cannot
+        // see that a single thread issues it, 21.5 against 20.8 us for the kernel at the training shape), more than the
         // tensor pipe needs for these small shapes, but issuers in different warps overlap. Three warps therefore issue
         // the MMAs of the three independent accumulator chains:  role 0: dQ (the longest chain),  role 1: dP and dV,
         // role 2: S and dK.
         const int role = warp - kMmaWarp;
-        if (lane == 0) {
+        if (ptx::elect_one()) {
             const uint32_t idesc_s = ptx::instr_desc(Fmt<E>::v, 0, 0, kTileM, (uint32_t)KT);
             const uint32_t idesc_dq = ptx::instr_desc(Fmt<E>::v, 0, 1, kTileM, (uint32_t)C);   // A K-major, B MN-major
             const uint32_t idesc_dkv = ptx::instr_desc(Fmt<E>::v, 1, 1, kTileM, (uint32_t)C);  // A MN-major, B MN-major

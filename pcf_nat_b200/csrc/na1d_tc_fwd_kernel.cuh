@@ -140,7 +140,7 @@ tc_fwd_kernel(const __grid_constant__ FwdMaps<SEG ? 2 : 1> tm, float* __restrict
     float* bias_tab = reinterpret_cast<float*>(smem + L.misc + 256);
     const int rows_total = gm.N * gm.T;
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = ptx::warp_index(), lane = tid & 31;
     // flat tiling: the effective (dilated) window, neighbour kk of the reference is offset kk * dil of it;
     // segmented tiling: the dilation lives in the addressing, the window is the reference's own
     const int dil = SEG ? 1 : gm.dil, dmask = dil - 1, dshift = 31 - __clz(dil);
@@ -249,7 +249,7 @@ tc_fwd_kernel(const __grid_constant__ FwdMaps<SEG ? 2 : 1> tm, float* __restrict
         }
     } else if (warp == kIssuerA) {
         // ------------------------------------------------------------ MMA issuer A: S, and the even key steps of P.V
-        if (lane == 0) {
+        if (ptx::elect_one()) {
             const uint32_t idesc_s = ptx::instr_desc(Fmt<E>::v, 0, 0, kTileM, (uint32_t)KT);
             const uint32_t idesc_o = ptx::instr_desc(Fmt<E>::v, 0, 1, kTileM, (uint32_t)C);
             const int nks = KT / 16;
@@ -291,7 +291,7 @@ tc_fwd_kernel(const __grid_constant__ FwdMaps<SEG ? 2 : 1> tm, float* __restrict
         }
     } else if (warp == kIssuerB) {
         // ------------------------------------------------------------ MMA issuer B: the odd key steps of P.V
-        if (lane == 0 && MODE != kBandOut) {
+        if (MODE != kBandOut && ptx::elect_one()) {
             const uint32_t idesc_o = ptx::instr_desc(Fmt<E>::v, 0, 1, kTileM, (uint32_t)C);
             const int nks = KT / 16;
             int it = 0;

@@ -69,7 +69,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(raw) + 1023) & ~(uintptr_t)1023);
     E* ones = reinterpret_cast<E*>(smem + kStages * kStageBytes);
     __shared__ Barriers bar;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = ptx::warp_index(), lane = threadIdx.x & 31;
     const uint32_t rank = pair::cta_rank();
     const int first = blockIdx.x >> 1, step = gridDim.x >> 1;
     volatile int* abort_flag = &bar.abort;
@@ -92,7 +92,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     const uint32_t tmem = bar.tmem;
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (ptx::elect_one()) {
             int slot = 0, n = 0;
             uint32_t phase = 1;   // the first round finds the slots empty
             bool ok = true;
@@ -117,7 +117,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                 for (int j = n - 1; j >= 0 && j >= n - kStages; --j) ptx::mbar_wait(&bar.full[j % kStages], (j / kStages) & 1, 1u << 14);
         }
     } else if (warp == 1) {
-        if (lane == 0 && rank == 0) {
+        if (rank == 0 && ptx::elect_one()) {
             constexpr uint32_t fmt = tc::Fmt<E>::v;
             constexpr uint32_t idesc = ptx::instr_desc(fmt, 1, 1, 256, kTile), idesc_ones = ptx::instr_desc(fmt, 1, 0, 256, 32);
             const uint64_t one = ptx::smem_desc(ptx::smem_u32(ones), 128, 256, ptx::kSwizzleNone);
@@ -126,10 +126,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
             bool ok = true;
             for (int i = first; ok && i < work.items; i += step, ++it) {
                 const Item t = item_at(work, i);
-                if (!pair::wait_cluster(&bar.acc_empty, (it & 1) ^ 1) || *abort_flag) { atomicExch(&g_wgrad_status, 2); *abort_flag = 1; break; }
+                if (!ptx::mbar_wait(&bar.acc_empty, (it & 1) ^ 1) || *abort_flag) { atomicExch(&g_wgrad_status, 2); *abort_flag = 1; break; }
                 ptx::tc_fence_after_sync();
                 for (int k = t.k0; k < t.k1; ++k) {
-                    if (!pair::wait_cluster(&bar.full[slot], phase) || *abort_flag) { atomicExch(&g_wgrad_status, 3); *abort_flag = 1; ok = false; break; }
+                    if (!ptx::mbar_wait(&bar.full[slot], phase) || *abort_flag) { atomicExch(&g_wgrad_status, 3); *abort_flag = 1; ok = false; break; }
                     ptx::tc_fence_after_sync();
                     const uint32_t s = ptx::smem_u32(smem + slot * kStageBytes);
                     const uint64_t a = pair::mn_major(s, kBox), b = pair::mn_major(s + 2 * kBox, kBox);
