@@ -88,6 +88,8 @@ _lib.na1d_valid_tokens.restype = _i32
 _lib.na1d_valid_tokens.argtypes = [_ptr, _ptr, _i32, _i64, _i64, _i64, _ptr]
 _lib.na1d_block_scratch_floats.restype = _i64
 _lib.na1d_block_scratch_floats.argtypes = [_i64, _i64, _i64]
+_lib.na1d_mlp_scratch_floats.restype = _i64
+_lib.na1d_mlp_scratch_floats.argtypes = [_i64] * 3
 _lib.na1d_projection_gradients_scratch.restype = _i64
 _lib.na1d_projection_gradients_scratch.argtypes = [_ptr, _ptr, _i32, _i64]
 for _name, _args in (
@@ -97,6 +99,7 @@ for _name, _args in (
         ("na1d_gelu_backward", [_ptr] * 5 + [_i64, _i64]),
         ("na1d_column_sums", [_ptr] * 3 + [_i64, _i64]),
         ("na1d_cast_parameters", [_ptr] * 4 + [_i32]),
+        ("na1d_mlp_forward", [_ptr, _i64] + [_ptr] * 8 + [_i64] * 3),
         ("na1d_projection_gradients", [_ptr] * 6 + [_i32, _i64, _ptr, _i32]),
         ("na1d_transpose", [_ptr, _ptr, _i64, _i64, _i64, _i32]),
         ("na1d_pack_grouped", [_ptr] * 4 + [_i32, _i64, _i64, _i32]),

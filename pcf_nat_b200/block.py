@@ -102,13 +102,13 @@ def run_blocks(blocks, x, valid, out=None, training=None):
         return None
     if valid is not None:
         valid = valid.to(device=x.device, dtype=torch.int32)      # (one copy for all blocks)
-    for ps, cfg, eps in plan:
-        y = ops.native.block(x, dx, valid, *cfg, *eps, ps)
+    for i, (ps, cfg, eps) in enumerate(plan):
+        y = ops.native.block(x, dx, valid, *cfg, *eps, ps, out if i + 1 == len(plan) else None)
         if y is None:                                             # (the first block, or none: they are given the same lengths)
             return None
         x, dx = y
     if out is not None:
-        return add_to_rows(out, x, dx)
+        return x if x is out or x.data_ptr() == out.data_ptr() else add_to_rows(out, x, dx)
     return x if dx is None else x + dx
 
 

@@ -95,6 +95,13 @@ cudaError_t wgrad(void* const* d_w, void* const* d_b, const void* const* dy, con
                   int64_t rows, float* scratch, bool out32, int dtype, cudaStream_t st);
 int wgrad_read_status();
 
+// ---- a block's MLP, out = s + GELU(h w1^T + b1) w2^T + b2 (na1d_mlp.cu)
+bool mlp_supports(int64_t D, int64_t F);
+size_t mlp_scratch_floats(int64_t rows, int64_t F);
+cudaError_t mlp_forward(void* out, int64_t ld, void* f, const void* s, const void* h, const void* w1, const float* b1, const void* w2, const float* b2, float* scratch,
+                        int64_t rows, int64_t F, int dtype, cudaStream_t st);
+int mlp_read_status();
+
 // ---- row and column kernels of a transformer block and of the statistics pooling (na1d_block.cu)
 int block_partial_rows(long long rows);
 cudaError_t block_valid_tokens(int* out, const void* padding, bool is64, int n_padding, int N, int T, cudaStream_t st);

@@ -1,0 +1,478 @@
+// The MLP of a transformer block as one kernel: out = s + GELU(h W1^T + b1) W2^T + b2, rows of 256 channels, hidden sizes that are a
+// multiple of 128.
+//
+// As separate passes (product, GELU, product, residual in the next LayerNorm) the hidden layer, four times as wide as the rows, crosses
+// HBM four times: 153600 rows took 106 + 126 + 94 us where the products themselves need 95; 148 + 5 us here (76800: 85 + 4, 9600: 32).
+// A pair of CTAs keeps 256 rows on chip: the rows as an operand in shared memory, the hidden layer in pieces of 128 columns in tensor memory, where GELU turns the
+// first product's result into the second one's left operand in place.
+//   warps 0-15   GELU: 32 tensor-memory lanes and a quarter of a piece's columns each
+//   warps 16-23  the result: out of tensor memory into registers at once (the next tile's second product waits for that), residual and
+//                store at leisure
+//   warp 24      loads: the rows of the next tile, weight pieces (16 KB a CTA: half of the output columns and of the contraction; a ring
+//                of four)
+//   warp 25      issues the products (leader): piece j + 1 of the hidden layer before the second product of piece j
+// Bound: tensor pipe (1024 + 1024 cycles a piece), GELU (FMA pipe 1150, special functions 1024), 64 KB of weights a piece from L2.
+// Every role's code is a short loop. (With the LayerNorm in it too -- eight warps, rows through registers -- the kernel took 245 us for
+// 153600 rows: its arithmetic, and the instructions it needs, come on top of GELU's.)
+#include "na1d_internal.h"
+#include "na1d_pair.cuh"
+
+namespace na1d {
+namespace {
+
+__device__ int g_mlp_status = 0;
+
+constexpr int kD = 256, kChunk = 128, kMostF = 1280;
+constexpr int kGeluWarps = 16, kResultWarps = 8;
+constexpr int kThreads = (kGeluWarps + kResultWarps + 4) * 32;
+// registers per thread after the warp groups have traded: 512 x 64 + 256 x 104 + 128 x 32 <= 896 x 72
+constexpr int kLaunchRegs = 72, kGeluRegs = 64, kResultRegs = 104, kOtherRegs = 32;
+constexpr int kSlots = 4, kSlotBytes = 16 * 1024;
+constexpr int kRowsBytes = 128 * kD * 2;          // a CTA's rows as an operand: four blocks of 64 channels, [block][row][128 bytes]
+constexpr int kGeluStage = 512, kStage = 2048;    // per warp, to turn rows per lane into rows of adjacent lanes: 8 rows or 32 rows x 64 bytes
+constexpr int kBiases = (kMostF + kD) * 4;
+constexpr int kSmem = 2 * kRowsBytes + kSlots * kSlotBytes + kGeluWarps * kGeluStage + kResultWarps * kStage + kBiases + 1024;
+constexpr uint32_t kAcc = 0, kHidden = 256;       // tensor-memory columns: result (256), two pieces of the hidden layer (128 each)
+
+struct Barriers {
+    uint64_t full[kSlots], empty[kSlots], s_full[2], g_ready[2], a_full[2], a_free[2], o_full, o_free;
+    uint32_t tmem;
+    int abort;
+};
+
+// Items: whole tiles of 256 rows in full rounds of the CTA pairs, then the tiles of the last, partly filled round split over the hidden
+// layer into `parts`, so that this round takes 1 / parts of the time (150 tiles on 74 pairs: 2.1 instead of 3).
+struct Plan {
+    int rows, pieces, whole, parts, items;
+};
+struct Item {
+    int tile, part, parts, c0, c1;
+};
+__device__ __forceinline__ Item item_at(const Plan& p, int i) {
+    Item t;
+    if (i < p.whole) {
+        t.tile = i; t.part = 0; t.parts = 1; t.c0 = 0; t.c1 = p.pieces;
+    } else {
+        i -= p.whole;
+        t.tile = i / p.parts;
+        t.part = i - t.tile * p.parts;
+        t.tile += p.whole;
+        t.parts = p.parts;
+        t.c0 = p.pieces * t.part / p.parts;
+        t.c1 = p.pieces * (t.part + 1) / p.parts;
+    }
+    return t;
+}
+
+struct Maps { CUtensorMap h, w1, w2; };
+template <typename E> struct Args {
+    const E* s;                        // residual stream
+    const float *b1, *b2;
+    E* out;                            // rows ld elements apart
+    long long ld;
+    E* f;                              // (rows, F): the hidden layer before GELU, for a backward pass
+    float* part;                       // partial results of the split tiles
+};
+
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    float2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;"
+        : "=l"(reinterpret_cast<uint64_t&>(d))
+        : "l"(reinterpret_cast<const uint64_t&>(a)), "l"(reinterpret_cast<const uint64_t&>(b)), "l"(reinterpret_cast<const uint64_t&>(c)));
+    return d;
+}
+__device__ __forceinline__ float2 both(float x) { return make_float2(x, x); }
+// x Phi(x) = max(x, 0) - |x| Phi(-|x|), with Phi(-a) = 2^P(a): log2 of the tail is a smooth function, so a polynomial of degree 7 keeps
+// the tail's relative accuracy (1e-5 for |x| < 2, 1e-4 to 4, 1e-3 to 6; the argument is not rounded to 16 bits first, which alone
+// would cost x^2 2^-9) with one special-function operation instead of two. P falls beyond the fitted range too (leading term -1.1e-6).
+__device__ __forceinline__ float2 gelu2(float2 x) {
+    const float2 a = make_float2(__uint_as_float(__float_as_uint(x.x) | 0x80000000u), __uint_as_float(__float_as_uint(x.y) | 0x80000000u));   // -|x|
+    float2 p = fma2(both(1.0900799907176406e-06f), a, both(4.5614655391545966e-05f));
+    p = fma2(p, a, both(0.0008011450991034508f));
+    p = fma2(p, a, both(0.00800548680126667f));
+    p = fma2(p, a, both(0.05297810584306717f));
+    p = fma2(p, a, both(-0.45937567949295044f));
+    p = fma2(p, a, both(1.1509263515472412f));
+    p = fma2(p, a, both(-1.000016212463379f));
+    return fma2(a, make_float2(tc::fast_exp2(p.x), tc::fast_exp2(p.y)), make_float2(fmaxf(x.x, 0.f), fmaxf(x.y, 0.f)));
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+    float2 d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(reinterpret_cast<uint64_t&>(d)) : "l"(reinterpret_cast<const uint64_t&>(a)), "l"(reinterpret_cast<const uint64_t&>(b)));
+    return d;
+}
+// rows that are read once, in program order, so that they are in flight together
+__device__ __forceinline__ uint4 load_row(const void* p) {
+    uint4 v;
+    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ uint32_t stage_at(int row, int chunk) { return (uint32_t)(row * 64 + ((chunk ^ (row >> 1)) & 3) * 16); }
+template <typename E> __device__ __forceinline__ void unpack2(const uint4& u, float2* f) {
+    float t[8];
+    Cvt<E>::unpack(u, t);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) f[i] = make_float2(t[2 * i], t[2 * i + 1]);
+}
+template <typename E> __device__ __forceinline__ uint4 pack2(const float2* f) {
+    return make_uint4(Cvt<E>::pack2(f[0].x, f[0].y), Cvt<E>::pack2(f[1].x, f[1].y), Cvt<E>::pack2(f[2].x, f[2].y), Cvt<E>::pack2(f[3].x, f[3].y));
+}
+// x + y of eight 16-bit values each, rounded: the residual stream
+template <typename E> __device__ __forceinline__ uint4 add_rows(const uint4& x, const uint4& y) {
+    float2 a[4], b[4];
+    unpack2<E>(x, a);
+    unpack2<E>(y, b);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) a[i] = add2(a[i], b[i]);
+    return pack2<E>(a);
+}
+
+template <typename E, bool TRAIN>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
+    mlp_kernel(const __grid_constant__ Maps maps, const __grid_constant__ Plan plan, const __grid_constant__ Args<E> g) {
+    extern __shared__ uint8_t raw[];
+    uint8_t* rows_smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(raw) + 1023) & ~(uintptr_t)1023);
+    uint8_t* ring = rows_smem + 2 * kRowsBytes;
+    uint8_t* stages = ring + kSlots * kSlotBytes;
+    float* biases = reinterpret_cast<float*>(stages + kGeluWarps * kGeluStage + kResultWarps * kStage);   // b2, b1
+    __shared__ Barriers bar;
+    const int warp = ptx::warp_index(), lane = threadIdx.x & 31;
+    const uint32_t rank = pair::cta_rank();
+    const int first = blockIdx.x >> 1, step = gridDim.x >> 1, F = plan.pieces * kChunk;
+    volatile int* abort_flag = &bar.abort;
+#define NA1D_MLP_FAIL(code) { atomicExch(&g_mlp_status, code); *abort_flag = 1; ok = false; break; }
+
+    if (warp == kGeluWarps + kResultWarps) {
+        if (lane < kSlots) { ptx::mbar_init(&bar.full[lane], 1); ptx::mbar_init(&bar.empty[lane], 1); }
+        else if (lane < kSlots + 2) { ptx::mbar_init(&bar.s_full[lane - kSlots], 1); ptx::mbar_init(&bar.g_ready[lane - kSlots], 2 * kGeluWarps); }
+        else if (lane < kSlots + 4) { ptx::mbar_init(&bar.a_full[lane - kSlots - 2], 1); ptx::mbar_init(&bar.a_free[lane - kSlots - 2], 1); }
+        else if (lane == 9) { ptx::mbar_init(&bar.o_full, 1); ptx::mbar_init(&bar.o_free, 2 * kResultWarps); }
+        else if (lane == 10) bar.abort = 0;
+        else if (lane == 11) ptx::prefetch_tensormap(&maps.w1);
+        else if (lane == 12) ptx::prefetch_tensormap(&maps.w2);
+        else if (lane == 13) ptx::prefetch_tensormap(&maps.h);
+        ptx::fence_mbar_init();
+    }
+    if (warp == kGeluWarps + kResultWarps + 2) { pair::tmem_alloc(&bar.tmem, 512); pair::tmem_relinquish(); }
+    for (int i = threadIdx.x; i < kD + F; i += kThreads) biases[i] = i < kD ? g.b2[i] : g.b1[i - kD];
+    ptx::tc_fence_before_sync();
+    __syncthreads();
+    pair::cluster_sync();
+    ptx::tc_fence_after_sync();
+    const uint32_t tmem = bar.tmem;
+    bool ok = true;
+
+    if (warp < kGeluWarps) {
+        ptx::warpgroup_regs_shrink<kGeluRegs>();
+        const int q = warp & 3, part = warp >> 2;   // tensor-memory lanes 32 q .. + 31, columns of this quarter
+        const uint32_t lanes = (uint32_t)(q * 32) << 16;
+        uint8_t* stage = stages + warp * kGeluStage;
+        const uint32_t g_ready0 = pair::in_leader(&bar.g_ready[0]), g_ready1 = pair::in_leader(&bar.g_ready[1]);
+        int j = 0;
+        for (int i = first; ok && i < plan.items; i += step) {
+            const Item t = item_at(plan, i);
+            const int row0 = t.tile * 256 + (int)rank * 128 + q * 32;
+            for (int c = t.c0; c < t.c1; ++c, ++j) {
+                const int buf = j & 1, col = c * kChunk + part * 32;
+                const uint32_t s = tmem + lanes + kHidden + buf * kChunk + part * 32;
+                const float4* b1 = reinterpret_cast<const float4*>(biases + kD + col);
+                if (!ptx::mbar_wait(&bar.s_full[buf], (j >> 1) & 1) || *abort_flag) NA1D_MLP_FAIL(1)
+                ptx::tc_fence_after_sync();
+                float d[32];
+                pair::tmem_ld32(s, d);
+                ptx::tmem_ld_wait();
+                uint32_t packed[16];
+#pragma unroll
+                for (int k = 0; k < 8; ++k) {
+                    const float4 bias = b1[k];
+                    const float2 u = add2(make_float2(d[4 * k], d[4 * k + 1]), make_float2(bias.x, bias.y));
+                    const float2 v = add2(make_float2(d[4 * k + 2], d[4 * k + 3]), make_float2(bias.z, bias.w));
+                    if (TRAIN) { d[2 * k] = __uint_as_float(Cvt<E>::pack2(u.x, u.y)); d[2 * k + 1] = __uint_as_float(Cvt<E>::pack2(v.x, v.y)); }
+                    const float2 gu = gelu2(u), gv = gelu2(v);
+                    packed[2 * k] = Cvt<E>::pack2(gu.x, gu.y);
+                    packed[2 * k + 1] = Cvt<E>::pack2(gv.x, gv.y);
+                }
+                pair::tmem_st16(s, packed);   // over columns that this warp has read
+                ptx::tmem_st_wait();
+                ptx::tc_fence_before_sync();
+                __syncwarp();
+                if (lane == 0) pair::arrive_cluster(buf ? g_ready1 : g_ready0);
+                if (TRAIN) {   // eight rows at a time
+                    E* dst = g.f + (size_t)row0 * F + col + (lane & 3) * 8;
+#pragma unroll 1
+                    for (int r0 = 0; r0 < 32; r0 += 8) {
+                        if (lane >= r0 && lane < r0 + 8) {
+#pragma unroll
+                            for (int k = 0; k < 4; ++k)
+                                *reinterpret_cast<uint4*>(stage + stage_at(lane & 7, k)) = make_uint4(__float_as_uint(d[4 * k]), __float_as_uint(d[4 * k + 1]),
+                                                                                                     __float_as_uint(d[4 * k + 2]), __float_as_uint(d[4 * k + 3]));
+                        }
+                        __syncwarp();
+                        const uint4 v = *reinterpret_cast<const uint4*>(stage + stage_at(lane >> 2, lane & 3));
+                        const int r = r0 + (lane >> 2);
+                        if (row0 + r < plan.rows) *reinterpret_cast<uint4*>(dst + (size_t)r * F) = v;
+                        __syncwarp();
+                    }
+                }
+            }
+        }
+    } else if (warp < kGeluWarps + kResultWarps) {
+        ptx::warpgroup_regs_grow<kResultRegs>();
+        const int w = warp - kGeluWarps, q = warp & 3, half = w >> 2;
+        uint8_t* stage = stages + kGeluWarps * kGeluStage + w * kStage;
+        const uint32_t o_free = pair::in_leader(&bar.o_free), o = tmem + ((uint32_t)(q * 32) << 16) + kAcc + half * 128;
+        int it = 0;
+        for (int i = first; i < plan.items; i += step, ++it) {
+            const Item t = item_at(plan, i);
+            const int row0 = t.tile * 256 + (int)rank * 128 + q * 32;
+            if (!ptx::mbar_wait_relaxed(&bar.o_full, it & 1) || *abort_flag) NA1D_MLP_FAIL(2)
+            ptx::tc_fence_after_sync();
+            uint4 z[16];   // 128 columns of this lane's row
+            auto keep = [&](int n, float* d) {
+                const float4* b2 = reinterpret_cast<const float4*>(biases + half * 128 + n * 32);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const float4 ba = b2[2 * k], bb = b2[2 * k + 1];
+                    float* v = d + 8 * k;
+                    v[0] += ba.x; v[1] += ba.y; v[2] += ba.z; v[3] += ba.w; v[4] += bb.x; v[5] += bb.y; v[6] += bb.z; v[7] += bb.w;
+                    z[n * 4 + k] = Cvt<E>::pack(v);
+                }
+            };
+            if (t.parts == 1) {
+#pragma unroll
+                for (int n = 0; n < 4; ++n) {
+                    float d[32];
+                    pair::tmem_ld32(o + n * 32, d);
+                    ptx::tmem_ld_wait();
+                    keep(n, d);
+                }
+                ptx::tc_fence_before_sync();
+                __syncwarp();
+                if (lane == 0) pair::arrive_cluster(o_free);
+            } else {   // a partial result, added up by mlp_finish_kernel
+                float4* dst = reinterpret_cast<float4*>(g.part) + ((((size_t)(t.tile - plan.whole) * 2 + rank) * kResultWarps + w) * t.parts + t.part) * 32 * 32 + lane;
+#pragma unroll 1
+                for (int n = 0; n < 4; ++n) {
+                    float d[32];
+                    pair::tmem_ld32(o + n * 32, d);
+                    ptx::tmem_ld_wait();
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) dst[(n * 8 + k) * 32] = make_float4(d[4 * k], d[4 * k + 1], d[4 * k + 2], d[4 * k + 3]);
+                }
+                ptx::tc_fence_before_sync();
+                __syncwarp();
+                if (lane == 0) pair::arrive_cluster(o_free);
+                continue;
+            }
+#pragma unroll
+            for (int n = 0; n < 4; ++n) {
+                const int col = half * 128 + n * 32 + (lane & 3) * 8;
+                uint4 res[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const int r = row0 + k * 8 + (lane >> 2);
+                    res[k] = make_uint4(0u, 0u, 0u, 0u);
+                    if (r < plan.rows) res[k] = load_row(g.s + (size_t)r * kD + col);
+                }
+                __syncwarp();
+#pragma unroll
+                for (int k = 0; k < 4; ++k) *reinterpret_cast<uint4*>(stage + stage_at(lane, k)) = z[n * 4 + k];
+                __syncwarp();
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const int r = k * 8 + (lane >> 2);
+                    const uint4 v = add_rows<E>(res[k], *reinterpret_cast<const uint4*>(stage + stage_at(r, lane & 3)));
+                    if (row0 + r < plan.rows) *reinterpret_cast<uint4*>(g.out + (size_t)(row0 + r) * g.ld + col) = v;
+                }
+            }
+        }
+    } else {
+        ptx::warpgroup_regs_shrink<kOtherRegs>();
+        if (warp == kGeluWarps + kResultWarps && ptx::elect_one()) {
+            int slot = 0, n = 0;
+            uint32_t phase = 1;
+            // pieces in the order in which they are used: W1 of piece j, then W2 of the piece before
+            auto load = [&](bool second, int c) {
+#pragma unroll 1
+                for (int k = 0; k < 2; ++k) {
+                    if (!ptx::mbar_wait_relaxed(&bar.empty[slot], phase) || *abort_flag) { atomicExch(&g_mlp_status, 4); *abort_flag = 1; ok = false; return; }
+                    const uint32_t full = pair::in_leader(&bar.full[slot]);
+                    if (rank == 0) ptx::mbar_expect_tx(&bar.full[slot], 2 * kSlotBytes);
+                    if (second) pair::load_3d(ring + slot * kSlotBytes, &maps.w2, full, 0, (int)rank * 128, 2 * c + k);
+                    else pair::load_3d(ring + slot * kSlotBytes, &maps.w1, full, 0, c * kChunk + (int)rank * 64, 2 * k);
+                    ++n;
+                    if (++slot == kSlots) { slot = 0; phase ^= 1; }
+                }
+            };
+            auto rows = [&](int i, int it) {
+                if (i >= plan.items) return;
+                if (!ptx::mbar_wait_relaxed(&bar.a_free[it & 1], ((it >> 1) & 1) ^ 1) || *abort_flag) { atomicExch(&g_mlp_status, 3); *abort_flag = 1; ok = false; return; }
+                if (rank == 0) ptx::mbar_expect_tx(&bar.a_full[it & 1], 2 * kRowsBytes);
+                pair::load_3d(rows_smem + (it & 1) * kRowsBytes, &maps.h, pair::in_leader(&bar.a_full[it & 1]), 0, item_at(plan, i).tile * 256 + (int)rank * 128, 0);
+            };
+            int before = -1, it = 0;
+            rows(first, 0);
+            for (int i = first; ok && i < plan.items; i += step, ++it) {
+                const Item t = item_at(plan, i);
+                for (int c = t.c0; ok && c < t.c1; ++c) {
+                    load(false, c);
+                    if (ok && before >= 0) load(true, before);
+                    before = c;
+                    if (ok && c == min(t.c0 + 1, t.c1 - 1)) rows(i + step, it + 1);
+                }
+            }
+            if (ok && before >= 0) load(true, before);
+            if (!ok && rank == 0)   // loads that are on their way arrive before the CTAs leave
+                for (int k = n - 1; k >= 0 && k >= n - kSlots; --k) ptx::mbar_wait(&bar.full[k % kSlots], (k / kSlots) & 1, 1u << 14);
+        }
+        if (warp == kGeluWarps + kResultWarps + 1 && rank == 0 && ptx::elect_one()) {
+            constexpr uint32_t fmt = tc::Fmt<E>::v;
+            constexpr uint32_t idesc1 = ptx::instr_desc(fmt, 0, 0, 256, kChunk), idesc2 = ptx::instr_desc(fmt, 0, 0, 256, kD);
+            int slot = 0, j = 0, it = 0;
+            uint32_t phase = 0;
+            auto next_slot = [&]() {
+                if (++slot == kSlots) { slot = 0; phase ^= 1; }
+            };
+            // second product of piece jj (its item: the it-th), the last one of its item or not
+            auto second = [&](int jj, int item, bool opens, bool closes) {
+                if (opens && (!ptx::mbar_wait(&bar.o_free, (item & 1) ^ 1) || *abort_flag)) { atomicExch(&g_mlp_status, 5); *abort_flag = 1; ok = false; return; }
+                if (!ptx::mbar_wait(&bar.g_ready[jj & 1], (jj >> 1) & 1) || *abort_flag) { atomicExch(&g_mlp_status, 6); *abort_flag = 1; ok = false; return; }
+                ptx::tc_fence_after_sync();
+                const uint32_t s = tmem + kHidden + (jj & 1) * kChunk;
+#pragma unroll 1
+                for (int h = 0; h < 2; ++h) {
+                    if (!ptx::mbar_wait(&bar.full[slot], phase) || *abort_flag) { atomicExch(&g_mlp_status, 7); *abort_flag = 1; ok = false; return; }
+                    ptx::tc_fence_after_sync();
+                    const uint64_t b = pair::k_major(ptx::smem_u32(ring + slot * kSlotBytes));
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) pair::mma_ts(tmem + kAcc, s + (h * 2 + (k >> 1)) * 32 + (k & 1) * 8, tc::desc_advance(b, k * 32), idesc2, !opens || h > 0 || k > 0);
+                    pair::commit(&bar.empty[slot]);
+                    next_slot();
+                }
+                if (closes) pair::commit(&bar.o_full);
+            };
+            bool opened = false;   // the piece before opened its item
+            for (int i = first; ok && i < plan.items; i += step, ++it) {
+                const Item t = item_at(plan, i);
+                if (!ptx::mbar_wait(&bar.a_full[it & 1], (it >> 1) & 1) || *abort_flag) NA1D_MLP_FAIL(8)
+                const uint64_t a = pair::k_major(ptx::smem_u32(rows_smem + (it & 1) * kRowsBytes));
+                for (int c = t.c0; ok && c < t.c1; ++c, ++j) {
+                    // The products of one thread run in order: the piece two back, which this one overwrites, has been used by its
+                    // second product, issued before.
+                    const uint32_t s = tmem + kHidden + (j & 1) * kChunk;
+#pragma unroll 1
+                    for (int h = 0; h < 2; ++h) {
+                        if (!ptx::mbar_wait(&bar.full[slot], phase) || *abort_flag) NA1D_MLP_FAIL(9)
+                        ptx::tc_fence_after_sync();
+                        const uint64_t b = pair::k_major(ptx::smem_u32(ring + slot * kSlotBytes)), ah = tc::desc_advance(a, h * 32768);
+#pragma unroll
+                        for (int k = 0; k < 8; ++k)
+                            pair::mma_ss(s, tc::desc_advance(ah, (k >> 2) * 16384 + (k & 3) * 32), tc::desc_advance(b, (k >> 2) * 8192 + (k & 3) * 32), idesc1, h > 0 || k > 0);
+                        pair::commit(&bar.empty[slot]);
+                        next_slot();
+                    }
+                    if (!ok) break;
+                    pair::commit(&bar.s_full[j & 1]);
+                    if (c == t.c1 - 1) pair::commit(&bar.a_free[it & 1]);
+                    if (j > 0) second(j - 1, c == t.c0 ? it - 1 : it, opened, c == t.c0);
+                    opened = c == t.c0;
+                }
+            }
+            if (ok && j > 0) second(j - 1, it - 1, opened, true);
+        }
+    }
+#undef NA1D_MLP_FAIL
+    __syncwarp();
+    ptx::tc_fence_before_sync();
+    __syncthreads();
+    pair::cluster_sync();   // neither CTA leaves while the other may still signal it or read its operands
+    if (warp == kGeluWarps + kResultWarps + 2) pair::tmem_dealloc(tmem, 512);
+}
+
+// The split tiles' partial results, residual and bias, in the order of the parts: a thread per four columns of a row, a CTA per 32 rows x 32
+// columns.
+template <typename E>
+__global__ void __launch_bounds__(256) mlp_finish_kernel(const __grid_constant__ Plan plan, const __grid_constant__ Args<E> g) {
+    const int n = blockIdx.x & 3, band = blockIdx.x >> 2, w = band & 7, rank = (band >> 3) & 1, tile = plan.whole + (band >> 4);
+    const int lane = threadIdx.x & 31, k = threadIdx.x >> 5;
+    const int row = tile * 256 + rank * 128 + (w & 3) * 32 + lane, col = (w >> 2) * 128 + n * 32 + k * 4;
+    if (row >= plan.rows) return;
+    const uint2 res = __ldg(reinterpret_cast<const uint2*>(g.s + (size_t)row * kD + col));
+    const float4 b = __ldg(reinterpret_cast<const float4*>(g.b2 + col));
+    const float4* src = reinterpret_cast<const float4*>(g.part) + (size_t)band * plan.parts * 32 * 32 + (n * 8 + k) * 32 + lane;
+    float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+    for (int p = 0; p < plan.parts; ++p) {
+        const float4 v = __ldg(src + (size_t)p * 32 * 32);
+        z.x += v.x; z.y += v.y; z.z += v.z; z.w += v.w;
+    }
+    const uint2 m = make_uint2(Cvt<E>::pack2(z.x + b.x, z.y + b.y), Cvt<E>::pack2(z.z + b.z, z.w + b.w));
+    const uint4 sum = add_rows<E>(make_uint4(res.x, res.y, 0u, 0u), make_uint4(m.x, m.y, 0u, 0u));
+    *reinterpret_cast<uint2*>(g.out + (size_t)row * g.ld + col) = make_uint2(sum.x, sum.y);
+}
+
+Plan make_plan(int64_t rows, int64_t F) {
+    Plan p;
+    const int pairs = device_sm_count() / 2, tiles = (int)((rows + 255) / 256);
+    p.rows = (int)rows;
+    p.pieces = (int)(F / kChunk);
+    p.whole = tiles / pairs * pairs;
+    const int rest = tiles - p.whole;
+    p.parts = rest ? pairs / rest : 1;
+    if (p.parts > p.pieces) p.parts = p.pieces;
+    if (p.parts < 2) { p.parts = 1; p.whole = tiles; }
+    p.items = p.whole + (tiles - p.whole) * p.parts;
+    return p;
+}
+size_t part_floats(const Plan& p) { return p.parts > 1 ? (size_t)(p.items - p.whole) * 256 * kD : 0; }
+template <typename E, bool TRAIN>
+cudaError_t run(const Maps& maps, const Plan& plan, const Args<E>& a, cudaStream_t st) {
+    auto* kern = mlp_kernel<E, TRAIN>;
+    // a kernel compiled to fewer registers would leave the growing warp groups waiting for ones that never come
+    static const int regs = [kern] {
+        cudaFuncAttributes fa;
+        return cudaFuncGetAttributes(&fa, kern) == cudaSuccess ? fa.numRegs : 0;
+    }();
+    if (regs < kLaunchRegs) return cudaErrorLaunchOutOfResources;
+    if (cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem)) return e;
+    const int pairs = device_sm_count() / 2, n = plan.items < pairs ? plan.items : pairs;
+    kern<<<2 * n, kThreads, kSmem, st>>>(maps, plan, a);
+    if (plan.parts == 1) return cudaGetLastError();
+    if (cudaError_t e = cudaGetLastError()) return e;
+    mlp_finish_kernel<E><<<(plan.items - plan.whole) / plan.parts * 2 * kResultWarps * 4, 256, 0, st>>>(plan, a);
+    return cudaGetLastError();
+}
+template <typename E>
+cudaError_t forward(void* out, int64_t ld, void* f, const void* s, const void* h, const void* w1, const float* b1, const void* w2, const float* b2, float* scratch,
+                    int64_t rows, int64_t F, int dtype, cudaStream_t st) {
+    const Plan plan = make_plan(rows, F);
+    Maps maps;
+    const int64_t dh[3] = {64, rows, kD / 64}, d1[3] = {64, F, kD / 64}, s1[2] = {kD, 64}, d2[3] = {64, kD, F / 64}, s2[2] = {F, 64};
+    const int xh[3] = {64, 128, kD / 64}, x1[3] = {64, 64, 2}, x2[3] = {64, 128, 1};
+    if (!make_matrix_map(&maps.h, h, dtype, 3, dh, s1, xh) || !make_matrix_map(&maps.w1, w1, dtype, 3, d1, s1, x1) ||
+        !make_matrix_map(&maps.w2, w2, dtype, 3, d2, s2, x2))
+        return cudaErrorInvalidValue;
+    const Args<E> a = {(const E*)s, b1, b2, (E*)out, ld, (E*)f, scratch};
+    return f ? run<E, true>(maps, plan, a, st) : run<E, false>(maps, plan, a, st);
+}
+
+}  // namespace
+
+bool mlp_supports(int64_t D, int64_t F) { return D == kD && F > 0 && F % kChunk == 0 && F <= kMostF; }
+size_t mlp_scratch_floats(int64_t rows, int64_t F) {
+    return part_floats(make_plan(rows, F));
+}
+cudaError_t mlp_forward(void* out, int64_t ld, void* f, const void* s, const void* h, const void* w1, const float* b1, const void* w2, const float* b2, float* scratch,
+                        int64_t rows, int64_t F, int dtype, cudaStream_t st) {
+    bind_primary_context();
+    return dtype == 0 ? forward<__nv_bfloat16>(out, ld, f, s, h, w1, b1, w2, b2, scratch, rows, F, dtype, st)
+                      : forward<__half>(out, ld, f, s, h, w1, b1, w2, b2, scratch, rows, F, dtype, st);
+}
+int mlp_read_status() {
+    int v = 0, zero = 0;
+    if (cudaMemcpyFromSymbol(&v, g_mlp_status, sizeof(int)) != cudaSuccess) return -1;
+    if (v != 0) cudaMemcpyToSymbol(g_mlp_status, &zero, sizeof(int));
+    return v;
+}
+
+}  // namespace na1d

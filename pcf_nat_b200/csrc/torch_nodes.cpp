@@ -419,9 +419,10 @@ Tensor layer_norm_backward(Tensor& sums, const Tensor& dy, const Tensor& s, cons
 }
 
 // x (+ dx): the residual stream. Returns the stream after the attention branch and the MLP branch's output; their sum is the
-// block's output, taken inside the next block's first LayerNorm.
+// block's output, taken inside the next block's first LayerNorm. Without a backward pass to come, and at the sizes that the MLP kernel takes,
+// the sum alone (the second tensor undefined), in `out` if that is given: rows of D inside wider ones.
 std::pair<Tensor, Tensor> block_forward(const Tensor& x, const Tensor& dx, const Tensor& vl, const Packed& c, double eps1, double eps2,
-                                        const Tensor* p, BlockState* keep) {
+                                        const Tensor* p, BlockState* keep, const OptTensor& out = std::nullopt) {
     const int64_t D = x.size(2), rows = c.B * c.T;
     const bool stats = keep != nullptr;
     BlockState st;
@@ -434,6 +435,16 @@ std::pair<Tensor, Tensor> block_forward(const Tensor& x, const Tensor& dx, const
     packed_forward(st.o, st.lse, st.qkv, p[12], vl, c);
     const Tensor y = at::addmm(w.t[3], st.o.view({rows, D}), w.t[2].t()).view({c.B, c.T, D});
     layer_norm(st.h2, st.s2, st.st2, st.s1, y, p[10], p[11], eps2, stats);
+    if (!keep) {
+        const int64_t F = w.t[4].size(0), floats = na1d_mlp_scratch_floats(rows, D, F);
+        if (floats >= 0) {
+            const Tensor sum = out ? *out : at::empty_like(x), scratch = floats ? empty_f32({floats}, x) : Tensor();
+            check(na1d_mlp_forward(ptr(sum), sum.stride(1), nullptr, ptr(st.s2), ptr(st.h2), ptr(w.t[4]), fptr(p[5]), ptr(w.t[6]), fptr(p[7]), fptr(scratch), rows,
+                                   D, F, code(x), stream()),
+                  "na1d_mlp_forward");
+            return {sum, Tensor()};
+        }
+    }
     st.f = at::addmm(w.t[5], st.h2.view({rows, D}), w.t[4].t());
     st.g = at::empty_like(st.f);
     check(na1d_gelu_forward(ptr(st.g), ptr(st.f), st.f.numel(), code(x), stream()), "na1d_gelu_forward");
@@ -532,10 +543,11 @@ struct NA1dBlock : public torch::autograd::Function<NA1dBlock> {
     }
 };
 
+// out: 16-byte aligned slices of wider rows for the result, without gradients (a hint: what comes back is the result).
 // nothing where the valid lengths are not of a form the kernels can be given (on another device, or of another integer type, they are
 // converted)
 std::optional<std::pair<Tensor, Tensor>> block(const Tensor& x, const OptTensor& dx, OptTensor vl, int64_t heads, int64_t win, int64_t left, double scale,
-                                               double eps1, double eps2, const std::vector<Tensor>& p) {
+                                               double eps1, double eps2, const std::vector<Tensor>& p, const OptTensor& out) {
     TORCH_CHECK(p.size() == kParams, "a block has 13 parameters");
     const c10::cuda::OptionalCUDAGuard guard(x.device());
     if (!prepare_valid(vl, x.size(0), x)) return std::nullopt;
@@ -545,7 +557,7 @@ std::optional<std::pair<Tensor, Tensor>> block(const Tensor& x, const OptTensor&
         return std::make_pair(r[0], r[1]);
     }
     const Packed c(x.size(0), x.size(1), x.size(2), heads, win, left, 1, scale);
-    return block_forward(x, dx ? *dx : Tensor(), vl ? *vl : Tensor(), c, eps1, eps2, p.data(), nullptr);
+    return block_forward(x, dx ? *dx : Tensor(), vl ? *vl : Tensor(), c, eps1, eps2, p.data(), nullptr, out);
 }
 
 // ---------------------------------------------------------------- the attention layer
