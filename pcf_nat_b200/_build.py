@@ -90,7 +90,7 @@ def build_nodes(force=False, verbose=False):
     cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-D_GLIBCXX_USE_CXX11_ABI=%d" % int(torch._C._GLIBCXX_USE_CXX11_ABI),
            "-DTORCH_EXTENSION_NAME=_na1d_torch", "-o", NODES, src] + [a for d in inc for a in ("-isystem", d)] + [
            "-L" + PKG, "-l:libna1d_b200.so", "-Wl,-rpath,$ORIGIN", "-L" + os.path.join(root, "lib"), "-ltorch_python", "-ltorch", "-ltorch_cuda",
-           "-ltorch_cpu", "-lc10_cuda", "-lc10"]
+           "-ltorch_cpu", "-lc10_cuda", "-lc10", "-L" + os.path.join(cuda, "lib64"), "-lcublasLt"]
     if verbose:
         print(" ".join(cmd), flush=True)
     subprocess.check_call(cmd)

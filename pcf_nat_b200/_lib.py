@@ -88,6 +88,10 @@ _lib.na1d_valid_tokens.restype = _i32
 _lib.na1d_valid_tokens.argtypes = [_ptr, _ptr, _i32, _i64, _i64, _i64, _ptr]
 _lib.na1d_block_scratch_floats.restype = _i64
 _lib.na1d_block_scratch_floats.argtypes = [_i64, _i64, _i64]
+_lib.na1d_fused_backward_workspace_floats.restype = _i64
+_lib.na1d_fused_backward_workspace_floats.argtypes = [_i64] * 7 + [_i32] * 3
+_lib.na1d_zero.restype = _i32
+_lib.na1d_zero.argtypes = [_ptr, _i64, _ptr]
 _lib.na1d_mlp_scratch_floats.restype = _i64
 _lib.na1d_mlp_scratch_floats.argtypes = [_i64] * 3
 _lib.na1d_projection_gradients_scratch.restype = _i64

@@ -490,6 +490,18 @@ int na1d_fused_backward(void* dq, void* dk, void* dv, float* d_rpb, const void* 
     return cuda_status(na1d::simt_fused_bwd(dq, dk, dv, d_rpb, d_o, q, k, v, lse, delta_ws, rpb, valid_len, g, dtype, st));
 }
 
+int64_t na1d_fused_backward_workspace_floats(int64_t N, int64_t heads, int64_t T, int64_t C, int64_t win, int64_t left, int64_t dil, int dtype,
+                                             int has_bias, int wants_bias_grad) {
+    const int route = na1d_fused_kernel_route(N, heads, T, C, win, left, dil, dtype, 1, has_bias, wants_bias_grad);
+    const bool rows = (route == 1 || route == 2) && wants_bias_grad && na1d::bias_grad_partial_rows();
+    return route == 0 || route < 0 || rows ? N * T : 0;
+}
+int na1d_zero(void* p, int64_t bytes, void* stream) {
+    NA1D_REQUIRE_PTR(p);
+    if (bytes < 0) return NA1D_ERR_BAD_SHAPE;
+    return cuda_status(cudaMemsetAsync(p, 0, (size_t)bytes, (cudaStream_t)stream));
+}
+
 namespace {
 int dropout_cfg(float drop_p, uint64_t seed, na1d::DropoutCfg& cfg) {
     if (!(drop_p >= 0.f) || drop_p >= 1.f) return NA1D_ERR_BAD_DROPOUT;

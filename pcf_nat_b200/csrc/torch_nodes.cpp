@@ -10,6 +10,9 @@
 // caller goes on to the Python route, which supports or refuses it as it always has.
 #include <torch/extension.h>
 
+#include <cublasLt.h>
+#include <unordered_map>
+
 #include <ATen/autocast_mode.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/core/impl/LocalDispatchKeySet.h>
@@ -45,6 +48,99 @@ inline int code(const Tensor& t) { return t.scalar_type() == at::kBFloat16 ? NA1
 inline void* ptr(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
 inline float* fptr(const Tensor& t) { return static_cast<float*>(ptr(t)); }
 inline Tensor empty_f32(at::IntArrayRef shape, const Tensor& like) { return at::empty(shape, like.options().dtype(at::kFloat)); }
+
+inline Tensor zeros_f32(at::IntArrayRef shape, const Tensor& like) {
+    const Tensor t = empty_f32(shape, like);
+    check(na1d_zero(ptr(t), t.numel() * 4, stream()), "na1d_zero");
+    return t;
+}
+
+// ---------------------------------------------------------------- library products
+// y (rows, N) = x (rows, K) w^T + b with w (N, K), or x w with w (K, N), dense and 16-bit, sums in fp32: the library product that at::addmm
+// and at::mm run, without their work for each call (13 to 16 us of host time, 5 here). What the library proposes for sizes, types and
+// alignments is kept under exactly those, for each host thread by itself, 256 of them at most.
+struct ProductKey {
+    int64_t rows, N, K;
+    int32_t kind, align;   // device, type, orientation, bias; the operands' alignments
+    bool operator==(const ProductKey& o) const { return rows == o.rows && N == o.N && K == o.K && kind == o.kind && align == o.align; }
+};
+struct ProductKeyHash {
+    size_t operator()(const ProductKey& k) const {
+        size_t h = 1469598103934665603ull;
+        for (size_t v : {(size_t)k.rows, (size_t)k.N, (size_t)k.K, (size_t)k.kind, (size_t)k.align}) h = (h ^ v) * 1099511628211ull;
+        return h ^ (h >> 29);
+    }
+};
+struct ProductPlan {
+    cublasLtMatmulDescOpaque_t desc;
+    cublasLtMatrixLayoutOpaque_t w, x, y;
+    cublasLtMatmulAlgo_t algo;
+    bool usable;
+};
+int32_t alignment(const void* p) {   // 16, 32, .. 256 bytes as 0 .. 4; -1: less
+    const auto a = reinterpret_cast<uintptr_t>(p);
+    int32_t n = -1;
+    for (uintptr_t b = 16; b <= 256 && (a & (b - 1)) == 0; b *= 2) ++n;
+    return n;
+}
+bool plan_product(ProductPlan& p, const ProductKey& k, cublasLtHandle_t handle, cudaDataType_t type, bool w_transposed, bool bias, const int32_t (&align)[4]) {
+    p.usable = false;
+    // the library counts columns first: y^T (N, rows) = op(w) x^T
+    const cublasOperation_t op = w_transposed ? CUBLAS_OP_N : CUBLAS_OP_T;
+    const cublasLtEpilogue_t epilogue = CUBLASLT_EPILOGUE_BIAS;
+    const uint32_t reductions = CUBLASLT_REDUCTION_SCHEME_NONE | CUBLASLT_REDUCTION_SCHEME_COMPUTE_TYPE;   // partial sums stay fp32
+    const size_t workspace = at::cuda::getCUDABlasLtWorkspaceSize();
+    cublasLtMatmulPreferenceOpaque_t pref;
+    if (cublasLtMatmulDescInit(&p.desc, CUBLAS_COMPUTE_32F, CUDA_R_32F) || cublasLtMatmulDescSetAttribute(&p.desc, CUBLASLT_MATMUL_DESC_TRANSA, &op, sizeof op) ||
+        cublasLtMatrixLayoutInit(&p.w, type, w_transposed ? k.N : k.K, w_transposed ? k.K : k.N, w_transposed ? k.N : k.K) ||
+        cublasLtMatrixLayoutInit(&p.x, type, k.K, k.rows, k.K) || cublasLtMatrixLayoutInit(&p.y, type, k.N, k.rows, k.N) || cublasLtMatmulPreferenceInit(&pref) ||
+        cublasLtMatmulPreferenceSetAttribute(&pref, CUBLASLT_MATMUL_PREF_MAX_WORKSPACE_BYTES, &workspace, sizeof workspace) ||
+        cublasLtMatmulPreferenceSetAttribute(&pref, CUBLASLT_MATMUL_PREF_REDUCTION_SCHEME_MASK, &reductions, sizeof reductions))
+        return false;
+    if (bias && (cublasLtMatmulDescSetAttribute(&p.desc, CUBLASLT_MATMUL_DESC_EPILOGUE, &epilogue, sizeof epilogue) ||
+                 cublasLtMatmulDescSetAttribute(&p.desc, CUBLASLT_MATMUL_DESC_BIAS_DATA_TYPE, &type, sizeof type)))
+        return false;
+    const cublasLtMatmulPreferenceAttributes_t which[3] = {CUBLASLT_MATMUL_PREF_MIN_ALIGNMENT_A_BYTES, CUBLASLT_MATMUL_PREF_MIN_ALIGNMENT_B_BYTES,
+                                                           CUBLASLT_MATMUL_PREF_MIN_ALIGNMENT_C_BYTES};
+    for (int i = 0; i < 3; ++i) {
+        const uint32_t bytes = 16u << align[i];
+        if (cublasLtMatmulPreferenceSetAttribute(&pref, which[i], &bytes, sizeof bytes)) return false;
+    }
+    cublasLtMatmulHeuristicResult_t found = {};
+    int n = 0;
+    if (cublasLtMatmulAlgoGetHeuristic(handle, &p.desc, &p.w, &p.x, &p.y, &p.y, &pref, 1, &found, &n) || n < 1) return false;
+    p.algo = found.algo;
+    p.usable = true;
+    return true;
+}
+Tensor product(const Tensor& x, const Tensor& w, const Tensor& b, bool w_transposed) {
+    const int64_t rows = x.size(0), K = x.size(1), N = w.size(w_transposed ? 1 : 0);
+    Tensor y = at::empty({rows, N}, x.options());
+    const bool bias = b.defined();
+    const int32_t align[4] = {alignment(ptr(w)), alignment(ptr(x)), alignment(ptr(y)), bias ? alignment(ptr(b)) : 4};
+    const bool dense = x.is_contiguous() && w.is_contiguous() && K % 8 == 0 && N % 8 == 0 && rows <= INT32_MAX && align[0] >= 0 && align[1] >= 0 && align[2] >= 0 && align[3] >= 0;
+    if (dense) {
+        static thread_local std::unordered_map<ProductKey, ProductPlan, ProductKeyHash> plans;
+        const cudaDataType_t type = x.scalar_type() == at::kBFloat16 ? CUDA_R_16BF : CUDA_R_16F;
+        const ProductKey key{rows, N, K, (int32_t)(x.get_device() * 8 + code(x) * 4 + w_transposed * 2 + bias), align[0] | align[1] << 4 | align[2] << 8};
+        const cublasLtHandle_t handle = at::cuda::getCurrentCUDABlasLtHandle();
+        auto it = plans.find(key);
+        if (it == plans.end()) {
+            if (plans.size() >= 256) plans.clear();
+            it = plans.emplace(key, ProductPlan()).first;
+            plan_product(it->second, key, handle, type, w_transposed, bias, align);
+        }
+        ProductPlan& p = it->second;
+        const void* bp = ptr(b);
+        const float one = 1.f, zero = 0.f;
+        if (p.usable && !(bias && cublasLtMatmulDescSetAttribute(&p.desc, CUBLASLT_MATMUL_DESC_BIAS_POINTER, &bp, sizeof bp)) &&
+            cublasLtMatmul(handle, &p.desc, &one, ptr(w), &p.w, ptr(x), &p.x, &zero, ptr(y), &p.y, ptr(y), &p.y, &p.algo, at::cuda::getCUDABlasLtWorkspace(),
+                           at::cuda::getCUDABlasLtWorkspaceSize(), at::cuda::getCurrentCUDAStream().stream()) == CUBLAS_STATUS_SUCCESS)
+            return y;
+    }
+    if (!bias) return at::mm(x, w_transposed ? w : w.t());
+    return at::addmm(b, x, w_transposed ? w : w.t());
+}
 
 bool eager_mode() {
     return c10::impl::TorchDispatchModeTLS::stack_len() == 0 && !torch::jit::tracer::isTracing() &&
@@ -111,8 +207,12 @@ struct NA1dFused : public torch::autograd::Function<NA1dFused> {
                     d["drop_p"].toDouble(), (uint64_t)d["seed"].toInt()};
         const c10::cuda::CUDAGuard guard(q.device());
         const Tensor d_o = grads[0].defined() ? grads[0].contiguous() : at::zeros_like(q);
-        Tensor dq = at::empty_like(q), dk = at::empty_like(k), dv = at::empty_like(v), delta = empty_f32({c.N, c.T}, q), d_rpb;
-        if (rpb.defined() && ctx->needs_input_grad(3)) d_rpb = at::zeros({c.heads, c.win}, q.options().dtype(at::kFloat));
+        Tensor dq = at::empty_like(q), dk = at::empty_like(k), dv = at::empty_like(v), d_rpb;
+        if (rpb.defined() && ctx->needs_input_grad(3)) d_rpb = zeros_f32(rpb.sizes(), q);
+        // (a workspace that is not needed is not touched)
+        const int64_t floats = c.drop_p != 0.0 ? c.N * c.T
+                                               : na1d_fused_backward_workspace_floats(c.N, c.heads, c.T, c.C, c.win, c.left, c.dil, code(q), rpb.defined(), d_rpb.defined());
+        const Tensor delta = floats == 0 ? lse : empty_f32({c.N, c.T}, q);
         const Tensor r = rpb32(rpb);
         if (c.drop_p != 0.0)
             check(na1d_fused_backward_dropout(ptr(dq), ptr(dk), ptr(dv), fptr(d_rpb), ptr(d_o), ptr(q), ptr(k), ptr(v), fptr(lse), fptr(r),
@@ -124,7 +224,7 @@ struct NA1dFused : public torch::autograd::Function<NA1dFused> {
                                       static_cast<int32_t*>(ptr(vl)), fptr(delta), c.N, c.heads, c.T, c.C, c.win, c.left, c.dil, (float)c.scale, code(q),
                                       stream()),
                   "na1d_fused_backward");
-        if (d_rpb.defined()) d_rpb = d_rpb.view(rpb.sizes()).to(rpb.scalar_type());
+        if (d_rpb.defined()) d_rpb = d_rpb.to(rpb.scalar_type());
         return {dq, dk, dv, d_rpb, Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
     }
 };
@@ -274,9 +374,9 @@ struct NA1dFusedPacked : public torch::autograd::Function<NA1dFusedPacked> {
         const c10::cuda::CUDAGuard guard(qkv.device());
         const Tensor d_o = grads[0].defined() ? grads[0].contiguous() : at::zeros({c.B, c.T, c.H * c.C}, qkv.options());
         Tensor d_qkv = at::empty_like(qkv), d_rpb;
-        if (rpb.defined() && ctx->needs_input_grad(1)) d_rpb = at::zeros({c.H, c.win}, qkv.options().dtype(at::kFloat));
+        if (rpb.defined() && ctx->needs_input_grad(1)) d_rpb = zeros_f32(rpb.sizes(), qkv);
         packed_backward(d_qkv, d_rpb, d_o, qkv, lse, rpb32(rpb), vl, c);
-        if (d_rpb.defined()) d_rpb = d_rpb.view(rpb.sizes()).to(rpb.scalar_type());
+        if (d_rpb.defined()) d_rpb = d_rpb.to(rpb.scalar_type());
         return {d_qkv, d_rpb, Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
     }
 };
@@ -372,7 +472,7 @@ struct Projections {
         int64_t off = 0;
         for (int i = 0; i < kProj; ++i) {
             const int64_t n = c10::multiply_integers(shapes[i]);
-            t[i] = buf.narrow(0, off, n).view(shapes[i]);
+            t[i] = shapes[i].size() == 2 ? buf.as_strided(shapes[i], {shapes[i][1], 1}, off) : buf.as_strided(shapes[i], {1}, off);
             off += (n + kSlot - 1) / kSlot * kSlot;
         }
     }
@@ -429,11 +529,11 @@ std::pair<Tensor, Tensor> block_forward(const Tensor& x, const Tensor& dx, const
     Projections w;
     w.cast(p, x);
     layer_norm(st.h1, st.s1, st.st1, x, dx, p[8], p[9], eps1, stats);
-    st.qkv = at::addmm(w.t[1], st.h1.view({rows, D}), w.t[0].t()).view({c.B, c.T, 3 * D});
+    st.qkv = product(st.h1.view({rows, D}), w.t[0], w.t[1], false).view({c.B, c.T, 3 * D});
     st.o = at::empty({c.B, c.T, D}, x.options());
     if (stats) st.lse = empty_f32({c.B * c.H, c.T}, x);
     packed_forward(st.o, st.lse, st.qkv, p[12], vl, c);
-    const Tensor y = at::addmm(w.t[3], st.o.view({rows, D}), w.t[2].t()).view({c.B, c.T, D});
+    const Tensor y = product(st.o.view({rows, D}), w.t[2], w.t[3], false).view({c.B, c.T, D});
     layer_norm(st.h2, st.s2, st.st2, st.s1, y, p[10], p[11], eps2, stats);
     if (!keep) {
         const int64_t F = w.t[4].size(0), floats = na1d_mlp_scratch_floats(rows, D, F);
@@ -445,10 +545,10 @@ std::pair<Tensor, Tensor> block_forward(const Tensor& x, const Tensor& dx, const
             return {sum, Tensor()};
         }
     }
-    st.f = at::addmm(w.t[5], st.h2.view({rows, D}), w.t[4].t());
+    st.f = product(st.h2.view({rows, D}), w.t[4], w.t[5], false);
     st.g = at::empty_like(st.f);
     check(na1d_gelu_forward(ptr(st.g), ptr(st.f), st.f.numel(), code(x), stream()), "na1d_gelu_forward");
-    Tensor z = at::addmm(w.t[7], st.g, w.t[6].t()).view({c.B, c.T, D});
+    Tensor z = product(st.g, w.t[6], w.t[7], false).view({c.B, c.T, D});
     Tensor s2 = st.s2;
     if (keep) {
         st.buf = w.buf;
@@ -520,22 +620,21 @@ struct NA1dBlock : public torch::autograd::Function<NA1dBlock> {
         // MLP branch
         Tensor d_b1 = empty_f32({F}, s1), d_f = at::empty_like(f);
         {
-            const Tensor d_g = at::mm(d_z, w.t[6]);
+            const Tensor d_g = product(d_z, w.t[6], Tensor(), true);
             check(na1d_gelu_backward(ptr(d_f), fptr(d_b1), fptr(scratch), ptr(d_g), ptr(f), rows, F, code(f), stream()), "na1d_gelu_backward");
         }
         const ParameterGrads mlp({d_f, d_z}, {h2.view({rows, D}), g}, {need(4), need(6)}, {false, need(7)}, at::kFloat);
         Tensor sums2, sums1;
-        const Tensor d_y = layer_norm_backward(sums2, at::mm(d_f, w.t[4]), s2, st2, n2w, d_s2, scratch);   // also the residual stream's gradient
+        const Tensor d_y = layer_norm_backward(sums2, product(d_f, w.t[4], Tensor(), true), s2, st2, n2w, d_s2, scratch);   // also the residual stream's gradient
         d_f.reset();
         // attention branch
         const Tensor dy2 = d_y.view({rows, D});
         Tensor d_qkv = at::empty_like(qkv), d_rpb;
-        if (need(12)) d_rpb = at::zeros({c.H, c.win}, s1.options().dtype(at::kFloat));
-        packed_backward(d_qkv, d_rpb, at::mm(dy2, w.t[2]), qkv, lse, rpb, vl, c);
+        if (need(12)) d_rpb = zeros_f32(rpb.sizes(), s1);
+        packed_backward(d_qkv, d_rpb, product(dy2, w.t[2], Tensor(), true), qkv, lse, rpb, vl, c);
         const Tensor dq2 = d_qkv.view({rows, 3 * D});
         const ParameterGrads att({dq2, dy2}, {h1.view({rows, D}), o.view({rows, D})}, {need(0), need(2)}, {need(1), false}, at::kFloat);
-        const Tensor d_x = layer_norm_backward(sums1, at::mm(dq2, w.t[0]), s1, st1, n1w, d_y, scratch);
-        if (d_rpb.defined()) d_rpb = d_rpb.view(rpb.sizes());
+        const Tensor d_x = layer_norm_backward(sums1, product(dq2, w.t[0], Tensor(), true), s1, st1, n1w, d_y, scratch);
         const Tensor none;
         return {d_x, has_dx ? d_x : none, none, none, none, none, none, none, none, att.w[0], att.b[0], att.w[1], sums2.select(0, 2), mlp.w[0], d_b1, mlp.w[1],
                 mlp.b[1],
@@ -587,7 +686,7 @@ struct LayerWeights {
             int count = 0;
             for (int i = 0; i < 4; ++i) {
                 if (!src[i].defined()) continue;
-                *dst[i] = i & 1 ? buf.narrow(0, off, n[i]) : buf.narrow(0, off, n[i]).view({n[i] / l.D, l.D});
+                *dst[i] = i & 1 ? buf.as_strided({n[i]}, {1}, off) : buf.as_strided({n[i] / l.D, l.D}, {l.D, 1}, off);
                 from[count] = fptr(src[i]); offs[count] = off; sizes[count] = n[i]; ++count;
                 off += (n[i] + kSlot - 1) / kSlot * kSlot;
             }
@@ -602,7 +701,7 @@ struct LayerWeights {
         }
     }
 };
-Tensor project(const Tensor& x, const Tensor& w, const Tensor& b) { return b.defined() ? at::addmm(b, x, w.t()) : at::mm(x, w.t()); }
+Tensor project(const Tensor& x, const Tensor& w, const Tensor& b) { return product(x, w, b, false); }
 Tensor transposed(const Tensor& in, const LayerShape& l, bool to_tokens) {
     Tensor out = to_tokens ? at::empty({l.B, l.T, l.D}, in.options()) : at::empty({l.B, l.D, l.T}, in.options());
     check(na1d_transpose(ptr(out), ptr(in), l.B, l.D, l.T, to_tokens, code(in), stream()), "na1d_transpose");
@@ -728,9 +827,9 @@ struct NA1dLayer : public torch::autograd::Function<NA1dLayer> {
         Tensor dy = grads[0].defined() ? aligned(grads[0]) : at::zeros(l.first ? at::IntArrayRef({l.B, l.D, l.T}) : xt.sizes(), xt.options());
         dy = (l.first ? transposed(dy, l, true) : dy).view({l.rows(), l.D});
         Tensor d_qkv = at::empty_like(qkv), d_rpb, d_x;
-        if (ctx->needs_input_grad(1)) d_rpb = at::zeros({c.H, c.win}, xt.options().dtype(at::kFloat));
+        if (ctx->needs_input_grad(1)) d_rpb = zeros_f32(rpb.sizes(), xt);
         if (o_dense.defined()) {
-            const Tensor d_o = heads_moved(at::mm(dy, pw), c, 1, true), delta = empty_f32({c.B * c.H, c.T}, xt), r = rpb32(rpb);
+            const Tensor d_o = heads_moved(product(dy, pw, Tensor(), true), c, 1, true), delta = empty_f32({c.B * c.H, c.T}, xt), r = rpb32(rpb);
             auto part = [](const Tensor& t, int i) { return ptr(t.select(0, i)); };
             check(na1d_fused_backward(part(d_qkv, 0), part(d_qkv, 1), part(d_qkv, 2), fptr(d_rpb), ptr(d_o), part(qkv, 0), part(qkv, 1), part(qkv, 2),
                                       ptr(o_dense), fptr(lse), fptr(r), static_cast<int32_t*>(ptr(vl)), fptr(delta), c.B * c.H, c.H, c.T, c.C, c.win,
@@ -738,7 +837,7 @@ struct NA1dLayer : public torch::autograd::Function<NA1dLayer> {
                   "na1d_fused_backward");
             d_qkv = heads_moved(d_qkv, c, 3, false);
         } else {
-            packed_backward(d_qkv, d_rpb, at::mm(dy, pw), qkv, lse, rpb32(rpb), vl, c);
+            packed_backward(d_qkv, d_rpb, product(dy, pw, Tensor(), true), qkv, lse, rpb32(rpb), vl, c);
         }
         const Tensor dq = d_qkv.view({l.rows(), 3 * l.D});
         const std::vector<int64_t> qw_shape = d["qw_shape"].toIntVector(), pw_shape = d["pw_shape"].toIntVector();
@@ -746,10 +845,10 @@ struct NA1dLayer : public torch::autograd::Function<NA1dLayer> {
                            {has_qb && ctx->needs_input_grad(qb_edge), has_pb && ctx->needs_input_grad(pb_edge)}, {dq, dy},
                            {aligned(xt).view({l.rows(), l.D}), o.view({l.rows(), l.D})}, {qw_shape, pw_shape}, type, l);
         if (ctx->needs_input_grad(0)) {
-            d_x = at::mm(dq, qw);
+            d_x = product(dq, qw, Tensor(), true);
             d_x = l.first ? transposed(d_x, l, false) : d_x.view({l.B, l.T, l.D});
         }
-        if (d_rpb.defined()) d_rpb = d_rpb.view(rpb.sizes()).to(rpb.scalar_type());
+        if (d_rpb.defined()) d_rpb = d_rpb.to(rpb.scalar_type());
         const Tensor none;
         return {d_x, d_rpb, g.w[0], g.w[1], g.b[0], g.b[1], none, none, none, none, none, none, none, none};
     }
