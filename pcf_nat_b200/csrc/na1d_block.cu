@@ -37,59 +37,93 @@ __device__ __forceinline__ void load8f(const float* p, float* f) {
 }
 
 // ---------------------------------------------------------------- LayerNorm
-// y = LN(s) w + b with s = x, or s = round(x + dx) written to `sum` (the residual stream): one warp per row, the row stays in
-// registers (mean first, then the centred squares). 153600 rows of 256: 231 us (framework kernel) + 37 us (residual add)
-// before, 53 us here (49 us of HBM time).
-template <typename E, int CH>
+// R values per lane, each summed over the warp: the first steps halve the values a lane carries on with, the totals come back to all
+// lanes (R = 4: 6 + 4 exchanges in place of 20, in five steps that do not wait for one another)
+template <int R> __device__ __forceinline__ void warp_sums(float (&v)[R], int lane) {
+    static_assert(R == 1 || R == 2 || R == 4, "rows at a time");
+#pragma unroll
+    for (int w = R / 2; w > 0; w >>= 1) {
+        const bool up = lane & (w * (32 / R));
+#pragma unroll
+        for (int i = 0; i < w; ++i) {
+            const float keep = up ? v[i + w] : v[i], send = up ? v[i] : v[i + w];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, w * (32 / R));
+        }
+    }
+    float t = v[0];
+#pragma unroll
+    for (int o = 16 / R; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+#pragma unroll
+    for (int i = 0; i < R; ++i) v[i] = R == 1 ? t : __shfl_sync(0xffffffffu, t, i * (32 / R));
+}
+
+// y = LN(s) w + b with s = x, or s = round(x + dx) written to `sum` (the residual stream): R rows of a warp at a time, which stay in
+// registers (mean first, then the centred squares) while the next R are on their way.
+// 153600 rows of 256, with / without the addition: 53 / 41 us a row at a time (its loads, a sum over the warp and again: too few bytes in
+// flight without the second input), 51 / 32 us with four (49 / 24 of HBM time); wider rows stay at one, a row is then enough to load.
+// 231 + 37 us by the framework's kernels.
+template <typename E, int CH, int R, bool ADD>
 __global__ void __launch_bounds__(kRowThreads) ln_fwd_kernel(E* __restrict__ y, E* __restrict__ sum, float* __restrict__ mean,
                                                              float* __restrict__ rstd, const E* __restrict__ x,
                                                              const E* __restrict__ dx, const float* __restrict__ w,
                                                              const float* __restrict__ b, int rows, int D, float eps) {
     const int lane = threadIdx.x & 31;
     const float inv_d = 1.f / (float)D;
-    // the next row's loads are in flight during a row's two reductions
-    uint4 nx[CH], nd[CH];
+    uint4 nx[R][CH], nd[R][ADD ? CH : 1];
     auto fetch = [&](int row) {
 #pragma unroll
-        for (int c = 0; c < CH; ++c) {
-            const int col = c * 256 + lane * 8;
-            nx[c] = nd[c] = make_uint4(0u, 0u, 0u, 0u);
-            if (row < rows && col < D) {
-                nx[c] = *reinterpret_cast<const uint4*>(x + (size_t)row * D + col);
-                if (dx) nd[c] = *reinterpret_cast<const uint4*>(dx + (size_t)row * D + col);
+        for (int u = 0; u < R; ++u)
+#pragma unroll
+            for (int c = 0; c < CH; ++c) {
+                const int col = c * 256 + lane * 8;
+                nx[u][c] = make_uint4(0u, 0u, 0u, 0u);
+                if (ADD) nd[u][ADD ? c : 0] = make_uint4(0u, 0u, 0u, 0u);
+                if (row + u < rows && col < D) {
+                    nx[u][c] = *reinterpret_cast<const uint4*>(x + (size_t)(row + u) * D + col);
+                    if (ADD) nd[u][ADD ? c : 0] = *reinterpret_cast<const uint4*>(dx + (size_t)(row + u) * D + col);
+                }
             }
-        }
     };
-    int row = blockIdx.x * kWarps + (threadIdx.x >> 5);
+    const int step = gridDim.x * kWarps * R;
+    int row = (blockIdx.x * kWarps + (threadIdx.x >> 5)) * R;
     fetch(row);
-    for (; row < rows; row += gridDim.x * kWarps) {
-        const size_t base = (size_t)row * D;
-        float v[CH][8], s = 0.f;
+    for (; row < rows; row += step) {
+        float v[R][CH][8], mu[R], rs[R];
 #pragma unroll
-        for (int c = 0; c < CH; ++c) {
-            const int col = c * 256 + lane * 8;
-            Cvt<E>::unpack(nx[c], v[c]);
-            if (dx) {
-                float r[8];
-                Cvt<E>::unpack(nd[c], r);
+        for (int u = 0; u < R; ++u) {
+            mu[u] = 0.f;
 #pragma unroll
-                for (int i = 0; i < 8; ++i) v[c][i] += r[i];
-                round8<E>(v[c]);
-                if (col < D) store8(sum + base + col, v[c]);
+            for (int c = 0; c < CH; ++c) {
+                const int col = c * 256 + lane * 8;
+                Cvt<E>::unpack(nx[u][c], v[u][c]);
+                if (ADD) {
+                    float r[8];
+                    Cvt<E>::unpack(nd[u][ADD ? c : 0], r);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) v[u][c][i] += r[i];
+                    round8<E>(v[u][c]);
+                    if (row + u < rows && col < D) store8(sum + (size_t)(row + u) * D + col, v[u][c]);
+                }
+#pragma unroll
+                for (int i = 0; i < 8; ++i) mu[u] += v[u][c][i];
             }
-#pragma unroll
-            for (int i = 0; i < 8; ++i) s += v[c][i];
         }
-        fetch(row + gridDim.x * kWarps);
-        const float mu = warp_sum(s) * inv_d;
-        float q = 0.f;
+        fetch(row + step);
+        warp_sums<R>(mu, lane);
 #pragma unroll
-        for (int c = 0; c < CH; ++c)
-            if (c * 256 + lane * 8 < D) {
+        for (int u = 0; u < R; ++u) {
+            mu[u] *= inv_d;
+            rs[u] = 0.f;
 #pragma unroll
-                for (int i = 0; i < 8; ++i) q = fmaf(v[c][i] - mu, v[c][i] - mu, q);
-            }
-        const float rs = rsqrtf(fmaf(warp_sum(q), inv_d, eps));
+            for (int c = 0; c < CH; ++c)
+                if (c * 256 + lane * 8 < D) {
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) rs[u] = fmaf(v[u][c][i] - mu[u], v[u][c][i] - mu[u], rs[u]);
+                }
+        }
+        warp_sums<R>(rs, lane);
+#pragma unroll
+        for (int u = 0; u < R; ++u) rs[u] = rsqrtf(fmaf(rs[u], inv_d, eps));
 #pragma unroll
         for (int c = 0; c < CH; ++c) {
             const int col = c * 256 + lane * 8;
@@ -98,11 +132,18 @@ __global__ void __launch_bounds__(kRowThreads) ln_fwd_kernel(E* __restrict__ y, 
                 load8f(w + col, wf);
                 load8f(b + col, bf);
 #pragma unroll
-                for (int i = 0; i < 8; ++i) v[c][i] = fmaf((v[c][i] - mu) * rs, wf[i], bf[i]);
-                store8(y + base + col, v[c]);
+                for (int u = 0; u < R; ++u) {
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) v[u][c][i] = fmaf((v[u][c][i] - mu[u]) * rs[u], wf[i], bf[i]);
+                    if (row + u < rows) store8(y + (size_t)(row + u) * D + col, v[u][c]);
+                }
             }
         }
-        if (mean && lane == 0) { mean[row] = mu; rstd[row] = rs; }
+        if (mean && lane == 0) {
+#pragma unroll
+            for (int u = 0; u < R; ++u)
+                if (row + u < rows) { mean[row + u] = mu[u]; rstd[row + u] = rs[u]; }
+        }
     }
 }
 
@@ -585,9 +626,11 @@ int row_grid(long long rows, int per_sm) {
 template <typename E>
 cudaError_t ln_fwd(void* y, void* sum, float* mean, float* rstd, const void* x, const void* dx, const float* w, const float* b,
                    int rows, int D, float eps, cudaStream_t st) {
-    const int grid = row_grid(rows, 8), ch = (D + 255) / 256;
-#define NA1D_LN(CH) ln_fwd_kernel<E, CH><<<grid, kRowThreads, 0, st>>>((E*)y, (E*)sum, mean, rstd, (const E*)x, (const E*)dx, w, b, rows, D, eps)
-    switch (ch) { case 1: NA1D_LN(1); break; case 2: NA1D_LN(2); break; case 3: NA1D_LN(3); break; default: NA1D_LN(4); }
+    const int ch = (D + 255) / 256;
+#define NA1D_LN(CH, R, ADD) ln_fwd_kernel<E, CH, R, ADD><<<row_grid((rows + R - 1) / R, 4), kRowThreads, 0, st>>>((E*)y, (E*)sum, mean, rstd, (const E*)x, (const E*)dx, w, b, rows, D, eps)
+#define NA1D_LN_C(ADD) switch (ch) { case 1: NA1D_LN(1, 4, ADD); break; case 2: NA1D_LN(2, 1, ADD); break; case 3: NA1D_LN(3, 1, ADD); break; default: NA1D_LN(4, 1, ADD); }
+    if (dx) { NA1D_LN_C(true) } else { NA1D_LN_C(false) }
+#undef NA1D_LN_C
 #undef NA1D_LN
     return cudaGetLastError();
 }
