@@ -19,10 +19,13 @@
 //     sequence's ends or at its padding.
 // Backward: key tile i collects from blocks i - NT + 1 .. i and is stored when block i is done. A strip owns the key tiles of its
 // own blocks and recomputes the NT - 1 blocks before it (nothing to recompute when the strip is a whole sequence).
-// Measured at 512 x 16 x 150 rows (tcgen05 flat / segmented tiling / here, us): window 27 forward 76 / 135 / 51, backward
-// 141 / 193 / 116; window 9 forward 62 / 104 / 40, backward 101 / 154 / 89; 64 x 16 x 997 rows, window 27: 66 / 66 / 37 and
-// 115 / 119 / 98. The forward is bound by instruction issue (0.67 a cycle), the backward by latency at twelve warps an SM.
-// Forward at 32 channels: 512 x 300 rows, window 27: 16 / 20 / 13; 4096 x 150: 49 / 85 / 51; the backward there needs more registers
+// Measured at 512 x 16 x 150 rows (tcgen05 flat / segmented tiling / here, us): window 27 forward 76 / 135 / 50, backward
+// 141 / 193 / 109; window 9 forward 62 / 104 / 40, backward 101 / 154 / 83; 64 x 16 x 997 rows, window 27: 66 / 66 / 37 and
+// 115 / 119 / 91. Both are bound by the chain of a block at the number of warps that the registers leave (forward 16, backward 12
+// an SM; more of them spill and lose). The scores' arithmetic goes in pairs (fma.rn.f32x2): backward 119 -> 111 us in a series of
+// calls; the forward's window changes places by name, not by moves: 57 -> 55 us, at 32 channels 55 -> 49 (the backward's accumulators by
+// name spill: 119 us).
+// Forward at 32 channels: 512 x 300 rows, window 27: 16 / 20 / 13; 4096 x 150: 49 / 85 / 45; the backward there needs more registers
 // than a thread has and stays on tcgen05 (82 / 107 against 118).
 // Rounding is that of the tcgen05 kernels: probabilities and dS enter the second products in 16 bits, sums are fp32.
 #include "na1d_internal.h"
@@ -53,6 +56,30 @@ __device__ __forceinline__ void mma(float (&d)[4], uint32_t a0, uint32_t a1, uin
                      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(c0), "f"(c1), "f"(c2), "f"(c3));
 }
 
+// pairs of fp32 values in one instruction
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    float2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;"
+        : "=l"(reinterpret_cast<uint64_t&>(d))
+        : "l"(reinterpret_cast<const uint64_t&>(a)), "l"(reinterpret_cast<const uint64_t&>(b)), "l"(reinterpret_cast<const uint64_t&>(c)));
+    return d;
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+    float2 d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(reinterpret_cast<uint64_t&>(d)) : "l"(reinterpret_cast<const uint64_t&>(a)), "l"(reinterpret_cast<const uint64_t&>(b)));
+    return d;
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+    float2 d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(reinterpret_cast<uint64_t&>(d)) : "l"(reinterpret_cast<const uint64_t&>(a)), "l"(reinterpret_cast<const uint64_t&>(b)));
+    return d;
+}
+__device__ __forceinline__ float2 both(float x) { return make_float2(x, x); }
+__device__ __forceinline__ float max3(float a, float b, float c) {
+    float d;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    return d;
+}
 // A lane's place in a tensor: row l / 4 of the current block or tile (the block's second half is 8 rows on), channels
 // 4 (l % 4) .. + 3; one wide multiply-add per step
 template <typename E> struct Place {
@@ -153,13 +180,11 @@ struct Strip {
         return b0 < b1;
     }
 };
-// bias of the thread's window offsets: class c = 2 (g - h + 1) + e is offset 8 (g - h) + e + fa (column group g, row half h)
-template <int NT> __device__ __forceinline__ void load_bias(float (&bias)[4 * NT + 2], const float* __restrict__ rpb, int h, int win, int fa) {
+// bias of the thread's window offsets: pair c = g - h + 1 holds offsets 8 (g - h) + fa and the next (column group g, row half h)
+template <int NT> __device__ __forceinline__ void load_bias(float2 (&bias)[2 * NT + 1], const float* __restrict__ rpb, int h, int win, int fa) {
+    auto at = [&](int kk) { return (unsigned)kk >= (unsigned)win ? -INFINITY : rpb ? __ldg(rpb + h * win + kk) * kLog2e : 0.f; };
 #pragma unroll
-    for (int c = 0; c < 4 * NT + 2; ++c) {
-        const int kk = 8 * ((c >> 1) - 1) + (c & 1) + fa;
-        bias[c] = (unsigned)kk >= (unsigned)win ? -INFINITY : rpb ? __ldg(rpb + h * win + kk) * kLog2e : 0.f;
-    }
+    for (int c = 0; c < 2 * NT + 1; ++c) bias[c] = make_float2(at(8 * (c - 1) + fa), at(8 * (c - 1) + fa + 1));
 }
 
 template <typename E, int KC, int NT>
@@ -170,8 +195,8 @@ __global__ void __launch_bounds__(kWarps * 32) march_fwd_kernel(E* __restrict__ 
     const long long id = (long long)blockIdx.x * kWarps + (threadIdx.x >> 5);
     Strip st;
     if (id >= mg.total || !st.init(gm, mg, valid_len, id)) return;
-    float bias[4 * NT + 2];
-    load_bias<NT>(bias, rpb, st.h, gm.win, fa);
+    float2 bias2[2 * NT + 1];
+    load_bias<NT>(bias2, rpb, st.h, gm.win, fa);
     const int right = gm.win - 1 - gm.left;
     const float sc = gm.scale * kLog2e, mask2 = kMaskValue * kLog2e;
     Place<const E> pq(q, sq, st.b, st.h, st.r, gm.dil, 16 * st.b0, lane), pk(k, sk, st.b, st.h, st.r, gm.dil, 16 * st.b0 - gm.left, lane),
@@ -179,38 +204,39 @@ __global__ void __launch_bounds__(kWarps * 32) march_fwd_kernel(E* __restrict__ 
     Place<E> po(o, so, st.b, st.h, st.r, gm.dil, 16 * st.b0, lane);
     float* lp = lse ? lse + ((long long)st.b * gm.H + st.h) * gm.T + (long long)(16 * st.b0 + fr) * gm.dil + st.r : nullptr;
     int u = 16 * st.b0 + fr, uk = u - gm.left;   // this lane's first query row; its first row of the next key tile
-    Rows<KC> kf[NT], qn, kn, vn;
+    // The window's tiles change places by name, not by moves: step PH (of NT, unrolled) finds tile t of its window in slot (PH + t) % NT,
+    // and the tile after the window takes slot PH.
+    Rows<KC> kf[NT], q_, vn;
     RowsT<KC> vt[NT];
-    // the first NT - 1 tiles; the last one of the first block comes in as "next"
+    auto next_tile = [&](Rows<KC>& kr) {
+        kr.load(pk, uk, st.Tr);
+        vn.load(pv, uk, st.Tr);
+        pk.next(); pv.next(); uk += 16;
+    };
 #pragma unroll
     for (int t = 0; t < NT; ++t) {
-        kn.load(pk, uk, st.Tr);
-        vn.load(pv, uk, st.Tr);
-        pk.next(); pv.next(); uk += 16;
-        if (t + 1 < NT) { kf[t + 1] = kn; vt[t + 1].set(vn); }
+        next_tile(kf[t]);
+        if (t + 1 < NT) vt[t].set(vn);
     }
-    qn.load(pq, u, st.Tr);
-#pragma unroll 1
-    for (int b = st.b0; b < st.b1; ++b, u += 16) {
+    q_.load(pq, u, st.Tr);
+    auto step = [&](int b, auto phase) {
+        constexpr int PH = decltype(phase)::value;
+        vt[(PH + NT - 1) % NT].set(vn);
+        float s[2 * NT][4], mx[2] = {-INFINITY, -INFINITY}, l[2];
 #pragma unroll
-        for (int t = 0; t + 1 < NT; ++t) { kf[t] = kf[t + 1]; vt[t] = vt[t + 1]; }
-        kf[NT - 1] = kn;
-        vt[NT - 1].set(vn);
-        const Rows<KC> qf = qn;
-        // the next block's rows are on their way while this one is computed
+        for (int t = 0; t < NT; ++t) products<E, KC>(s[2 * t], s[2 * t + 1], q_, kf[(PH + t) % NT]);
+        // the next block's rows are on their way while this one is worked on
         pq.next();
-        qn.load(pq, u + 16, st.Tr);
-        kn.load(pk, uk, st.Tr);
-        vn.load(pv, uk, st.Tr);
-        pk.next(); pv.next(); uk += 16;
-        float s[2 * NT][4], mx[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
-#pragma unroll
-        for (int t = 0; t < NT; ++t) products<E, KC>(s[2 * t], s[2 * t + 1], qf, kf[t]);
+        q_.load(pq, u + 16, st.Tr);
+        next_tile(kf[PH]);
         const bool need_mask = 16 * b < gm.left || 16 * b + 15 + right >= st.vl;
 #pragma unroll
         for (int g = 0; g < 2 * NT; ++g)
 #pragma unroll
-            for (int i = 0; i < 4; ++i) s[g][i] = fmaf(s[g][i], sc, bias[2 * (g - (i >> 1) + 1) + (i & 1)]);
+            for (int h = 0; h < 2; ++h) {
+                const float2 x = fma2(make_float2(s[g][2 * h], s[g][2 * h + 1]), both(sc), bias2[g - h + 1]);
+                s[g][2 * h] = x.x; s[g][2 * h + 1] = x.y;
+            }
         if (need_mask) {
 #pragma unroll
             for (int g = 0; g < 2 * NT; ++g)
@@ -223,25 +249,28 @@ __global__ void __launch_bounds__(kWarps * 32) march_fwd_kernel(E* __restrict__ 
 #pragma unroll
         for (int g = 0; g < 2 * NT; ++g)
 #pragma unroll
-            for (int i = 0; i < 4; ++i) mx[i >> 1] = fmaxf(mx[i >> 1], s[g][i]);
+            for (int h = 0; h < 2; ++h) mx[h] = max3(mx[h], s[g][2 * h], s[g][2 * h + 1]);
         mx[0] = tc::quad_max(mx[0]);
         mx[1] = tc::quad_max(mx[1]);
         float acc[KC][2][4];
+        float2 l2[2] = {both(0.f), both(0.f)};
 #pragma unroll
         for (int t = 0; t < NT; ++t) {
 #pragma unroll
             for (int g = 2 * t; g < 2 * t + 2; ++g)
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    s[g][i] = tc::fast_exp2(s[g][i] - mx[i >> 1]);
-                    l[i >> 1] += s[g][i];
+                for (int h = 0; h < 2; ++h) {
+                    const float2 x = add2(make_float2(s[g][2 * h], s[g][2 * h + 1]), both(-mx[h]));
+                    s[g][2 * h] = tc::fast_exp2(x.x);
+                    s[g][2 * h + 1] = tc::fast_exp2(x.y);
+                    l2[h] = add2(l2[h], make_float2(s[g][2 * h], s[g][2 * h + 1]));
                 }
             const uint32_t w[4] = {Cvt<E>::pack2(s[2 * t][0], s[2 * t][1]), Cvt<E>::pack2(s[2 * t][2], s[2 * t][3]),
                                    Cvt<E>::pack2(s[2 * t + 1][0], s[2 * t + 1][1]), Cvt<E>::pack2(s[2 * t + 1][2], s[2 * t + 1][3])};
-            if (t == 0) accumulate<E, KC, true>(acc, w, vt[t]); else accumulate<E, KC, false>(acc, w, vt[t]);
+            if (t == 0) accumulate<E, KC, true>(acc, w, vt[PH]); else accumulate<E, KC, false>(acc, w, vt[(PH + t) % NT]);
         }
-        l[0] = tc::quad_sum(l[0]);
-        l[1] = tc::quad_sum(l[1]);
+        l[0] = tc::quad_sum(l2[0].x + l2[0].y);
+        l[1] = tc::quad_sum(l2[1].x + l2[1].y);
         store<E, KC>(po, u, st.Tr, acc, tc::fast_rcp(l[0]), tc::fast_rcp(l[1]));
         po.next();
         if (lse) {
@@ -251,6 +280,13 @@ __global__ void __launch_bounds__(kWarps * 32) march_fwd_kernel(E* __restrict__ 
             }
             lp += 16 * gm.dil;
         }
+        u += 16;
+    };
+#pragma unroll 1
+    for (int b = st.b0; b < st.b1; b += NT) {
+        step(b, std::integral_constant<int, 0>());
+        if (b + 1 < st.b1) step(b + 1, std::integral_constant<int, 1>());
+        if (NT == 3 && b + 2 < st.b1) step(b + 2, std::integral_constant<int, NT - 1>());
     }
 }
 
@@ -326,11 +362,11 @@ __global__ void __launch_bounds__(kWarps * 32, NT == 3 ? 3 : 4) march_bwd_kernel
     const long long id = (long long)blockIdx.x * kWarps + warp;
     Strip st;
     const bool alive = id < mg.total && st.init(gm, mg, valid_len, id);
-    float grad[4 * NT + 2];
+    float2 grad[2 * NT + 1];
 #pragma unroll
-    for (int c = 0; c < 4 * NT + 2; ++c) grad[c] = 0.f;
+    for (int c = 0; c < 2 * NT + 1; ++c) grad[c] = both(0.f);
     if (alive) {
-        float bias[4 * NT + 2];
+        float2 bias[2 * NT + 1];
         load_bias<NT>(bias, rpb, st.h, gm.win, fa);
         const int right = gm.win - 1 - gm.left, first = max(0, st.b0 - (NT - 1));
         const float sc = gm.scale * kLog2e, mask2 = kMaskValue * kLog2e;
@@ -378,7 +414,8 @@ __global__ void __launch_bounds__(kWarps * 32, NT == 3 ? 3 : 4) march_bwd_kernel
             asm volatile("cp.async.wait_group 1;" ::: "memory");
             __syncwarp();
             const uint32_t tq = tl.q + (b & 1) * kTileBytes, to = tl.o + (b & 1) * kTileBytes;
-            float s[2 * NT][4], d[2 * NT][4], delta[2], part[2][4] = {};   // (two chains per row keep the sums short)
+            float s[2 * NT][4], d[2 * NT][4], delta[2];
+            float2 part[2][2] = {{both(0.f), both(0.f)}, {both(0.f), both(0.f)}};   // (two chains per row keep the sums short)
             {
                 uint32_t qa[4], oa[4];
                 ldsm(qa, tq + tl.rows);
@@ -399,7 +436,10 @@ __global__ void __launch_bounds__(kWarps * 32, NT == 3 ? 3 : 4) march_bwd_kernel
 #pragma unroll
             for (int g = 0; g < 2 * NT; ++g)
 #pragma unroll
-                for (int i = 0; i < 4; ++i) s[g][i] = fmaf(s[g][i], sc, bias[2 * (g - (i >> 1) + 1) + (i & 1)]);
+                for (int h = 0; h < 2; ++h) {
+                    const float2 x = fma2(make_float2(s[g][2 * h], s[g][2 * h + 1]), both(sc), bias[g - h + 1]);
+                    s[g][2 * h] = x.x; s[g][2 * h + 1] = x.y;
+                }
             if (need_mask) {
 #pragma unroll
                 for (int g = 0; g < 2 * NT; ++g)
@@ -412,21 +452,29 @@ __global__ void __launch_bounds__(kWarps * 32, NT == 3 ? 3 : 4) march_bwd_kernel
 #pragma unroll
             for (int g = 0; g < 2 * NT; ++g)
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    s[g][i] = tc::fast_exp2(s[g][i] - l2[i >> 1]);
-                    part[g & 1][i] = fmaf(s[g][i], d[g][i], part[g & 1][i]);
+                for (int h = 0; h < 2; ++h) {
+                    const float2 x = add2(make_float2(s[g][2 * h], s[g][2 * h + 1]), both(-l2[h]));
+                    s[g][2 * h] = tc::fast_exp2(x.x);
+                    s[g][2 * h + 1] = tc::fast_exp2(x.y);
+                    part[g & 1][h] = fma2(make_float2(s[g][2 * h], s[g][2 * h + 1]), make_float2(d[g][2 * h], d[g][2 * h + 1]), part[g & 1][h]);
                 }
-            delta[0] = tc::quad_sum((part[0][0] + part[0][1]) + (part[1][0] + part[1][1]));
-            delta[1] = tc::quad_sum((part[0][2] + part[0][3]) + (part[1][2] + part[1][3]));
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const float2 x = add2(part[0][h], part[1][h]);
+                delta[h] = tc::quad_sum(x.x + x.y);
+            }
 #pragma unroll
             for (int g = 0; g < 2 * NT; ++g)
 #pragma unroll
-                for (int i = 0; i < 4; ++i) d[g][i] = s[g][i] * (d[g][i] - delta[i >> 1]);
+                for (int h = 0; h < 2; ++h) {
+                    const float2 x = mul2(make_float2(s[g][2 * h], s[g][2 * h + 1]), add2(make_float2(d[g][2 * h], d[g][2 * h + 1]), both(-delta[h])));
+                    d[g][2 * h] = x.x; d[g][2 * h + 1] = x.y;
+                }
             if (own && d_rpb) {
 #pragma unroll
                 for (int g = 0; g < 2 * NT; ++g)
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) grad[2 * (g - (i >> 1) + 1) + (i & 1)] += d[g][i];
+                    for (int h = 0; h < 2; ++h) grad[g - h + 1] = add2(grad[g - h + 1], make_float2(d[g][2 * h], d[g][2 * h + 1]));
             }
             uint32_t qt[4], ot[4];
             ldsm_t(qt, tq + tl.rows);
@@ -440,7 +488,8 @@ __global__ void __launch_bounds__(kWarps * 32, NT == 3 ? 3 : 4) march_bwd_kernel
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
                     const int g = 2 * t + (i >> 1), h = 2 * (i & 1);
-                    w[i] = Cvt<E>::pack2(d[g][h] * gm.scale, d[g][h + 1] * gm.scale);
+                    const float2 y = mul2(make_float2(d[g][h], d[g][h + 1]), both(gm.scale));
+                    w[i] = Cvt<E>::pack2(y.x, y.y);
                     x[i] = Cvt<E>::pack2(s[g][h], s[g][h + 1]);
                 }
                 if (t == 0) add_rows<E, true>(acc, w, kt); else add_rows<E, false>(acc, w, kt);
@@ -483,7 +532,7 @@ __global__ void __launch_bounds__(kWarps * 32, NT == 3 ? 3 : 4) march_bwd_kernel
         float* sums = reinterpret_cast<float*>(tiles[warp]);
         __syncwarp();
 #pragma unroll
-        for (int c = 0; c < 4 * NT + 2; ++c) sums[c * 32 + lane] = grad[c];
+        for (int c = 0; c < 2 * NT + 1; ++c) { sums[2 * c * 32 + lane] = grad[c].x; sums[(2 * c + 1) * 32 + lane] = grad[c].y; }
         __syncwarp();
         for (int kk = lane; kk < gm.win; kk += 32) {
             float sum = 0.f;
