@@ -202,7 +202,11 @@ template <typename... S> bool use_march(const na1d::Geometry& g, Pass pass, bool
     if (forced == -1 && pass == Pass::backward && residue > 32 && residue < 40 && (long long)g.N * g.T > (1 << 17) &&
         na1d::tc_bwd_supports(g, true, wants_bias_grad))
         return false;
-    if (forced == -1 && pass == Pass::forward && g.C == 32 && (long long)g.N * g.T > (1 << 18)) return false;
+    // Dense forward at 32 channels: large calls with short sequences stay on the flat tiling (2800 x 97 rows, window 9, 21.2 us against 23.1,
+    // window 27 24.0 / 24.9: a badly filled second round of warps; at most a tenth is lost by it: 4096 x 150 40.5 / 37.2 and 47.2 / 46.8). Longer
+    // ones: 2048 x 300 rows 41.0 / 35.0 (window 9), 46.1 / 45.7 (27), 1600 x 1000 92.5 / 81.1 and 108 / 93. Dilated ones, whose other
+    // tiling would be the segmented one or a wide band: 1.0 (2800 x 97, dilation 2) to 3.1 times (8000 x 64, dilation 3: 151 / 49).
+    if (forced == -1 && pass == Pass::forward && g.C == 32 && g.dil == 1 && g.T < 256 && (long long)g.N * g.T > (1 << 18)) return false;
     return na1d::march_supports(g, backward) && ((strides.token * g.dil < (1ll << 30)) && ...);
 }
 }  // namespace
@@ -309,6 +313,14 @@ static int pick_family(const na1d::Geometry& g, int backward, bool has_bias = fa
         pick = 1;
     } else if (seg_ok) {
         pick = 2;
+    }
+    // Short residues leave a segmented tile of 128 rows mostly empty, and the general kernels (whose tiles hold 64, or a row at a time) take
+    // less: forward at 64 channels 2000 x 64 rows, dilation 3 (22 rows a residue) 56 us against 40, 1200 x 150, dilation 4 (38) 56 / 47,
+    // dilation 3 (50) 36 / 37; backward 4000 x 31 rows, window 15, dilation 3 (11 rows) 301 / 182 (64 channels), 125 / 115 (32), window 5,
+    // dilation 2 (16 rows) 161 / 87 and 80 / 55, but window 15 208 / 184 and 86 / 107.
+    if (forced == -1 && pick == 2 && g.dil > 1) {
+        const int tp = (g.T + g.dil - 1) / g.dil;
+        if (backward ? tp <= 12 || (tp <= 16 && g.win <= 9) : tp <= 40) pick = 0;
     }
     if (forced == 1 && pick == 0) return NA1D_ERR_UNSUPPORTED;
     return pick;
