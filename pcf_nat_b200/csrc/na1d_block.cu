@@ -398,62 +398,70 @@ __global__ void __launch_bounds__(256) valid_tokens_kernel(int* __restrict__ out
 }
 
 // ---------------------------------------------------------------- channels-first layers: transposes and grouped weights
-// A 64-channel x 64-token tile through shared memory. The token side is read or written in pairs (4 bytes) where the rows allow
-// it (an even token count, an even base), the channel side in 16-byte units; the odd pitch of 65 elements keeps both
-// phases free of bank conflicts. 512 x 256 x 150: 72 us per copy before, 15 to 25 us here, 12 us of HBM time.
-constexpr int kTile = 64, kTilePitch = 65;
+// A 64-channel x 64-token tile through shared memory, as words of two tokens of one channel: the token side is read or written in such
+// pairs (4 bytes) where the rows allow it (an even token count, an even base), the channel side in 16-byte units of two tokens
+// at a time, so that every word is moved whole (tokens as single 16-bit values of a [token][channel] tile: 27 us to tokens, 21 back).
+// 512 x 256 x 150: 18 and 19 us in a series, 12 us of HBM time; 72 us per copy of the framework.
+constexpr int kTile = 64, kTilePitch = 33;
 template <bool TO_TOKENS, bool PAIRS>
 __global__ void __launch_bounds__(256) transpose_kernel(uint16_t* __restrict__ out, const uint16_t* __restrict__ in, int C, int T) {
-    __shared__ uint16_t sm[kTile * kTilePitch];   // [token][channel]
+    __shared__ uint32_t sm[kTile * kTilePitch];   // [channel][pair of tokens]
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c0 = blockIdx.x * kTile, t0 = blockIdx.y * kTile;
     const size_t base = (size_t)blockIdx.z * C * T;
-    const int t = t0 + 2 * lane;                  // channel-major side: lane -> two tokens, warp -> channels warp, warp + 8, ...
-    auto tokens_phase = [&](auto&& f) {
+    // channel-major side: lane -> two tokens, warp -> channels warp, warp + 8, ...; token-major side: eight channels of two tokens
+    const int t = t0 + 2 * lane, cu = (threadIdx.x & 7) * 8, pair = threadIdx.x >> 3, tok = t0 + 2 * pair;
+    if constexpr (TO_TOKENS) {
+        uint32_t v[kTile / 8];
 #pragma unroll
         for (int i = 0; i < kTile / 8; ++i) {
             const int c = warp + 8 * i;
-            if (c0 + c < C && t < T) f(c, base + (size_t)(c0 + c) * T + t);
-        }
-    };
-    auto channels_phase = [&](auto&& f) {         // token-major side: 8 lanes cover a token's 64 channels
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            const int row = (threadIdx.x >> 3) + 32 * i, c = (threadIdx.x & 7) * 8;
-            if (t0 + row < T && c0 + c < C) f(sm + row * kTilePitch + c, base + (size_t)(t0 + row) * C + c0 + c);
-        }
-    };
-    if constexpr (TO_TOKENS) {
-        uint32_t v[kTile / 8];
-        tokens_phase([&](int c, size_t at) {
-            v[c >> 3] = PAIRS ? *reinterpret_cast<const uint32_t*>(in + at) : (uint32_t)in[at] | (t + 1 < T ? (uint32_t)in[at + 1] << 16 : 0u);
-        });
-        tokens_phase([&](int c, size_t) {
-            sm[2 * lane * kTilePitch + c] = (uint16_t)v[c >> 3];
-            sm[(2 * lane + 1) * kTilePitch + c] = (uint16_t)(v[c >> 3] >> 16);
-        });
-        __syncthreads();
-        channels_phase([&](const uint16_t* s, size_t at) {
-            uint4 u;
-            u.x = s[0] | (uint32_t)s[1] << 16; u.y = s[2] | (uint32_t)s[3] << 16; u.z = s[4] | (uint32_t)s[5] << 16; u.w = s[6] | (uint32_t)s[7] << 16;
-            *reinterpret_cast<uint4*>(out + at) = u;
-        });
-    } else {
-        channels_phase([&](uint16_t* s, size_t at) {
-            const uint4 u = *reinterpret_cast<const uint4*>(in + at);
-            const uint32_t w[4] = {u.x, u.y, u.z, u.w};
-#pragma unroll
-            for (int e = 0; e < 4; ++e) { s[2 * e] = (uint16_t)w[e]; s[2 * e + 1] = (uint16_t)(w[e] >> 16); }
-        });
-        __syncthreads();
-        tokens_phase([&](int c, size_t at) {
-            const uint16_t a = sm[2 * lane * kTilePitch + c], b = sm[(2 * lane + 1) * kTilePitch + c];
-            if constexpr (PAIRS) {
-                *reinterpret_cast<uint32_t*>(out + at) = a | (uint32_t)b << 16;
-            } else {
-                out[at] = a;
-                if (t + 1 < T) out[at + 1] = b;
+            v[i] = 0u;
+            if (c0 + c < C && t < T) {
+                const size_t at = base + (size_t)(c0 + c) * T + t;
+                v[i] = PAIRS ? __ldg(reinterpret_cast<const uint32_t*>(in + at)) : (uint32_t)in[at] | (t + 1 < T ? (uint32_t)in[at + 1] << 16 : 0u);
             }
-        });
+        }
+#pragma unroll
+        for (int i = 0; i < kTile / 8; ++i) sm[(warp + 8 * i) * kTilePitch + lane] = v[i];
+        __syncthreads();
+        if (tok < T && c0 + cu < C) {
+            uint32_t w[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) w[e] = sm[(cu + e) * kTilePitch + pair];
+            uint4 first, second;
+            first.x = __byte_perm(w[0], w[1], 0x5410); first.y = __byte_perm(w[2], w[3], 0x5410);
+            first.z = __byte_perm(w[4], w[5], 0x5410); first.w = __byte_perm(w[6], w[7], 0x5410);
+            second.x = __byte_perm(w[0], w[1], 0x7632); second.y = __byte_perm(w[2], w[3], 0x7632);
+            second.z = __byte_perm(w[4], w[5], 0x7632); second.w = __byte_perm(w[6], w[7], 0x7632);
+            *reinterpret_cast<uint4*>(out + base + (size_t)tok * C + c0 + cu) = first;
+            if (tok + 1 < T) *reinterpret_cast<uint4*>(out + base + (size_t)(tok + 1) * C + c0 + cu) = second;
+        }
+    } else {
+        if (tok < T && c0 + cu < C) {
+            const size_t unit_at = base + (size_t)tok * C + c0 + cu;
+            const uint4 a = __ldg(reinterpret_cast<const uint4*>(in + unit_at));
+            const uint4 b = tok + 1 < T ? __ldg(reinterpret_cast<const uint4*>(in + unit_at + C)) : make_uint4(0u, 0u, 0u, 0u);
+            const uint32_t f[4] = {a.x, a.y, a.z, a.w}, s[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                sm[(cu + 2 * e) * kTilePitch + pair] = __byte_perm(f[e], s[e], 0x5410);
+                sm[(cu + 2 * e + 1) * kTilePitch + pair] = __byte_perm(f[e], s[e], 0x7632);
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < kTile / 8; ++i) {
+            const int c = warp + 8 * i;
+            if (c0 + c >= C || t >= T) continue;
+            const uint32_t v = sm[c * kTilePitch + lane];
+            uint16_t* at = out + base + (size_t)(c0 + c) * T + t;
+            if constexpr (PAIRS) {
+                *reinterpret_cast<uint32_t*>(at) = v;
+            } else {
+                at[0] = (uint16_t)v;
+                if (t + 1 < T) at[1] = (uint16_t)(v >> 16);
+            }
+        }
     }
 }
 
