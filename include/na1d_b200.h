@@ -238,12 +238,16 @@ int na1d_gelu_backward(void* dx, float* sums, float* scratch, const void* dy, co
 /* sums (F) = column sums of x (rows, F). */
 int na1d_column_sums(float* sums, float* scratch, const void* x, int64_t rows, int64_t F, int dtype, void* stream);
 /* A transformer block's MLP in one kernel: out = s + GELU(h w1^T + b1) w2^T + b2 (models/PCF_NATransformer.py:228-303). s, h, out
- * (rows, D), w1 (F, D), w2 (D, F) 16-bit, biases fp32; out has rows of ld >= D elements (a multiple of 8); D = 256, F a multiple of 128 up to 1280. f (rows, F), 16-bit, or NULL: takes the
- * hidden layer before GELU, for a backward pass. `scratch`: na1d_mlp_scratch_floats floats (0: may be NULL; -1: not a size that
- * this takes). */
+ * (rows, D), w1 (F, D), w2 (D, F) 16-bit, biases fp32; out has rows of ld >= D elements (a multiple of 8); D = 256, F a multiple of
+ * 128 up to 1280. f (rows, F), 16-bit and 32-byte aligned, or NULL: takes the hidden layer before GELU, for a backward pass.
+ * `scratch`: na1d_mlp_scratch_floats floats (0: may be NULL; -1: not a size that this takes). */
 int64_t na1d_mlp_scratch_floats(int64_t rows, int64_t D, int64_t F);
 int na1d_mlp_forward(void* out, int64_t ld, void* f, const void* s, const void* h, const void* w1, const float* b1, const void* w2, const float* b2,
                      float* scratch, int64_t rows, int64_t D, int64_t F, int dtype, void* stream);
+/* Its backward for the gradient d (rows, D) of out: df (rows, F) = (d w2) * gelu'(f), dh (rows, D) = df w1, g (rows, F) = gelu(f), all
+ * 16-bit and, like f, 32-byte aligned; sizes and `scratch` as above. What the parameters need is left to na1d_projection_gradients. */
+int na1d_mlp_backward(void* dh, void* df, void* g, const void* d, const void* f, const void* w1, const void* w2, float* scratch, int64_t rows, int64_t D,
+                      int64_t F, int dtype, void* stream);
 /* Parameter gradients of `count` (at most 2) projections in one launch: d_w[i] (M[i], N[i]) = dy[i]^T x[i], d_b[i] (M[i]) = column
  * sums of dy[i]; dy[i] (rows, M[i]) and x[i] (rows, N[i]) 16-bit, results fp32 (out32) or of `dtype`, either may be NULL. Host arrays
  * of device pointers. Partial sums go through `scratch` and are added in a fixed order. */

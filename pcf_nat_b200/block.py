@@ -2,10 +2,10 @@
 
 Between the four projections of a block (models/PCF_NATransformer.py:228-303: x + NA(LN(x)); x + MLP(LN(x))) PyTorch's autocast
 runs a kernel per LayerNorm, addition, GELU, cast of a parameter and bias gradient. Here each of them is part of a
-pass that has to touch the tensor anyway: the residual addition happens inside the LayerNorm that follows it, the bias
-gradient of a projection inside the backward pass that produces its output gradient, a block's eight projection parameters
-are rounded to 16 bits by one launch. The projections themselves stay library GEMMs, the attention is the fused operator on the
-packed projection output.
+pass that has to touch the tensor anyway: the residual addition happens inside the LayerNorm that follows it or at the end of the MLP,
+which is one kernel forward and one backward where its sizes allow (256 channels), a block's eight projection parameters are rounded to
+16 bits by one launch, the weight and bias gradients of a branch come from one. The remaining products are library GEMMs, the attention
+is the fused operator on the packed projection output.
 
 Rounding points are those of the autocast network: 16-bit activations and projection weights, fp32 statistics and sums; the
 LayerNorm parameters and the weight gradients are not rounded to 16 bits on the way.

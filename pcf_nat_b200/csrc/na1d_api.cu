@@ -365,7 +365,7 @@ int na1d_tensor_map_cache_stats(int64_t* hits, int64_t* misses) {
 
 int na1d_device_status(void) {
     // every word is read (and cleared) before anything is reported; an expired wait in any kernel wins over a failed read
-    const int words[10] = {na1d::mlp_read_status(), na1d::wgrad_read_status(), na1d::tc_read_status(), na1d::tc_bwd_read_status(), na1d::tc_seg_read_status(),
+    const int words[11] = {na1d::mlp_read_status(), na1d::mlp_bwd_read_status(), na1d::wgrad_read_status(), na1d::tc_read_status(), na1d::tc_bwd_read_status(), na1d::tc_seg_read_status(),
                           na1d::tc_bwd_seg_read_status(), na1d::tc_unfused_read_status(), na1d::tc_unfused_t_read_status(),
                           na1d::tc_drop_read_status(), na1d::tc_bwd_drop_read_status()};
     int v = 0, w = 0;
@@ -642,11 +642,20 @@ int64_t na1d_mlp_scratch_floats(int64_t rows, int64_t D, int64_t F) {
 int na1d_mlp_forward(void* out, int64_t ld, void* f, const void* s, const void* h, const void* w1, const float* b1, const void* w2, const float* b2, float* scratch,
                      int64_t rows, int64_t D, int64_t F, int dtype, void* stream) {
     if (int e = check_pointers(out, s, h, w1, b1, w2, b2)) return e;
-    if (!aligned16(f) || !aligned16(scratch)) return NA1D_ERR_MISALIGNED;
+    if (((uintptr_t)f & 31) || !aligned16(scratch)) return NA1D_ERR_MISALIGNED;
     if (int e = check_block(rows, F, 1 << 20, dtype)) return e;
     if (!na1d::mlp_supports(D, F) || ld < D || ld % 8 != 0 || ld > (1ll << 40) / rows) return NA1D_ERR_BAD_SHAPE;
     if (!scratch && na1d::mlp_scratch_floats(rows, F)) return NA1D_ERR_NULL_POINTER;
     return cuda_status(na1d::mlp_forward(out, ld, f, s, h, w1, b1, w2, b2, scratch, rows, F, dtype, (cudaStream_t)stream));
+}
+int na1d_mlp_backward(void* dh, void* df, void* g, const void* d, const void* f, const void* w1, const void* w2, float* scratch, int64_t rows, int64_t D, int64_t F,
+                      int dtype, void* stream) {
+    if (int e = check_pointers(dh, df, g, d, f, w1, w2)) return e;
+    if (!aligned16(scratch) || (((uintptr_t)dh | (uintptr_t)df | (uintptr_t)g | (uintptr_t)f) & 31)) return NA1D_ERR_MISALIGNED;
+    if (int e = check_block(rows, F, 1 << 20, dtype)) return e;
+    if (!na1d::mlp_supports(D, F)) return NA1D_ERR_BAD_SHAPE;
+    if (!scratch && na1d::mlp_scratch_floats(rows, F)) return NA1D_ERR_NULL_POINTER;
+    return cuda_status(na1d::mlp_backward(dh, df, g, d, f, w1, w2, scratch, rows, F, dtype, (cudaStream_t)stream));
 }
 int na1d_cast_parameters(void* out, const float* const* src, const int64_t* dst, const int64_t* n, int count, int dtype,
                          void* stream) {

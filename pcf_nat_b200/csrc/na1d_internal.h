@@ -101,6 +101,10 @@ size_t mlp_scratch_floats(int64_t rows, int64_t F);
 cudaError_t mlp_forward(void* out, int64_t ld, void* f, const void* s, const void* h, const void* w1, const float* b1, const void* w2, const float* b2, float* scratch,
                         int64_t rows, int64_t F, int dtype, cudaStream_t st);
 int mlp_read_status();
+// its backward (na1d_mlp_bwd.cu): df = (d w2) GELU'(f), dh = df w1, gelu = GELU(f); dh, df, gelu, f (and the forward's f) 32-byte aligned
+cudaError_t mlp_backward(void* dh, void* df, void* gelu, const void* d, const void* f, const void* w1, const void* w2, float* scratch, int64_t rows, int64_t F,
+                         int dtype, cudaStream_t st);
+int mlp_bwd_read_status();
 
 // ---- row and column kernels of a transformer block and of the statistics pooling (na1d_block.cu)
 int block_partial_rows(long long rows);

@@ -3,8 +3,10 @@
 //
 // As separate passes (product, GELU, product, residual in the next LayerNorm) the hidden layer, four times as wide as the rows, crosses
 // HBM four times: 153600 rows took 106 + 126 + 94 us where the products themselves need 95; 148 + 5 us here (76800: 85 + 4, 9600: 32).
-// A pair of CTAs keeps 256 rows on chip: the rows as an operand in shared memory, the hidden layer in pieces of 128 columns in tensor memory, where GELU turns the
-// first product's result into the second one's left operand in place.
+// For a backward pass the layer before GELU is stored, a sector of each row at a time straight from the lanes that hold it: 38400 rows
+// 62 + 4 us instead of 78 (70 + 4 through a stage in shared memory).
+// A pair of CTAs keeps 256 rows on chip: the rows as an operand in shared memory, the hidden layer in pieces of 128 columns in tensor
+// memory, where GELU turns the first product's result into the second one's left operand in place.
 //   warps 0-15   GELU: 32 tensor-memory lanes and a quarter of a piece's columns each
 //   warps 16-23  the result: out of tensor memory into registers at once (the next tile's second product waits for that), residual and
 //                store at leisure
@@ -15,54 +17,27 @@
 // Every role's code is a short loop. (With the LayerNorm in it too -- eight warps, rows through registers -- the kernel took 245 us for
 // 153600 rows: its arithmetic, and the instructions it needs, come on top of GELU's.)
 #include "na1d_internal.h"
-#include "na1d_pair.cuh"
+#include "na1d_mlp.cuh"
 
 namespace na1d {
 namespace {
 
 __device__ int g_mlp_status = 0;
 
-constexpr int kD = 256, kChunk = 128, kMostF = 1280;
 constexpr int kGeluWarps = 16, kResultWarps = 8;
 constexpr int kThreads = (kGeluWarps + kResultWarps + 4) * 32;
 // registers per thread after the warp groups have traded: 512 x 64 + 256 x 104 + 128 x 32 <= 896 x 72
 constexpr int kLaunchRegs = 72, kGeluRegs = 64, kResultRegs = 104, kOtherRegs = 32;
-constexpr int kSlots = 4, kSlotBytes = 16 * 1024;
-constexpr int kRowsBytes = 128 * kD * 2;          // a CTA's rows as an operand: four blocks of 64 channels, [block][row][128 bytes]
-constexpr int kGeluStage = 512, kStage = 2048;    // per warp, to turn rows per lane into rows of adjacent lanes: 8 rows or 32 rows x 64 bytes
+constexpr int kSlots = 4;
+constexpr int kStage = 2048;                      // per warp, to turn rows per lane into rows of adjacent lanes: 32 rows x 64 bytes
 constexpr int kBiases = (kMostF + kD) * 4;
-constexpr int kSmem = 2 * kRowsBytes + kSlots * kSlotBytes + kGeluWarps * kGeluStage + kResultWarps * kStage + kBiases + 1024;
-constexpr uint32_t kAcc = 0, kHidden = 256;       // tensor-memory columns: result (256), two pieces of the hidden layer (128 each)
+constexpr int kSmem = 2 * kRowsBytes + kSlots * kSlotBytes + kResultWarps * kStage + kBiases + 1024;
 
 struct Barriers {
     uint64_t full[kSlots], empty[kSlots], s_full[2], g_ready[2], a_full[2], a_free[2], o_full, o_free;
     uint32_t tmem;
     int abort;
 };
-
-// Items: whole tiles of 256 rows in full rounds of the CTA pairs, then the tiles of the last, partly filled round split over the hidden
-// layer into `parts`, so that this round takes 1 / parts of the time (150 tiles on 74 pairs: 2.1 instead of 3).
-struct Plan {
-    int rows, pieces, whole, parts, items;
-};
-struct Item {
-    int tile, part, parts, c0, c1;
-};
-__device__ __forceinline__ Item item_at(const Plan& p, int i) {
-    Item t;
-    if (i < p.whole) {
-        t.tile = i; t.part = 0; t.parts = 1; t.c0 = 0; t.c1 = p.pieces;
-    } else {
-        i -= p.whole;
-        t.tile = i / p.parts;
-        t.part = i - t.tile * p.parts;
-        t.tile += p.whole;
-        t.parts = p.parts;
-        t.c0 = p.pieces * t.part / p.parts;
-        t.c1 = p.pieces * (t.part + 1) / p.parts;
-    }
-    return t;
-}
 
 struct Maps { CUtensorMap h, w1, w2; };
 template <typename E> struct Args {
@@ -74,19 +49,11 @@ template <typename E> struct Args {
     float* part;                       // partial results of the split tiles
 };
 
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
-    float2 d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;"
-        : "=l"(reinterpret_cast<uint64_t&>(d))
-        : "l"(reinterpret_cast<const uint64_t&>(a)), "l"(reinterpret_cast<const uint64_t&>(b)), "l"(reinterpret_cast<const uint64_t&>(c)));
-    return d;
-}
-__device__ __forceinline__ float2 both(float x) { return make_float2(x, x); }
 // x Phi(x) = max(x, 0) - |x| Phi(-|x|), with Phi(-a) = 2^P(a): log2 of the tail is a smooth function, so a polynomial of degree 7 keeps
 // the tail's relative accuracy (1e-5 for |x| < 2, 1e-4 to 4, 1e-3 to 6; the argument is not rounded to 16 bits first, which alone
 // would cost x^2 2^-9) with one special-function operation instead of two. P falls beyond the fitted range too (leading term -1.1e-6).
 __device__ __forceinline__ float2 gelu2(float2 x) {
-    const float2 a = make_float2(__uint_as_float(__float_as_uint(x.x) | 0x80000000u), __uint_as_float(__float_as_uint(x.y) | 0x80000000u));   // -|x|
+    const float2 a = make_float2(minus_abs(x.x), minus_abs(x.y));
     float2 p = fma2(both(1.0900799907176406e-06f), a, both(4.5614655391545966e-05f));
     p = fma2(p, a, both(0.0008011450991034508f));
     p = fma2(p, a, both(0.00800548680126667f));
@@ -96,37 +63,6 @@ __device__ __forceinline__ float2 gelu2(float2 x) {
     p = fma2(p, a, both(-1.000016212463379f));
     return fma2(a, make_float2(tc::fast_exp2(p.x), tc::fast_exp2(p.y)), make_float2(fmaxf(x.x, 0.f), fmaxf(x.y, 0.f)));
 }
-__device__ __forceinline__ float2 add2(float2 a, float2 b) {
-    float2 d;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(reinterpret_cast<uint64_t&>(d)) : "l"(reinterpret_cast<const uint64_t&>(a)), "l"(reinterpret_cast<const uint64_t&>(b)));
-    return d;
-}
-// rows that are read once, in program order, so that they are in flight together
-__device__ __forceinline__ uint4 load_row(const void* p) {
-    uint4 v;
-    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
-    return v;
-}
-__device__ __forceinline__ uint32_t stage_at(int row, int chunk) { return (uint32_t)(row * 64 + ((chunk ^ (row >> 1)) & 3) * 16); }
-template <typename E> __device__ __forceinline__ void unpack2(const uint4& u, float2* f) {
-    float t[8];
-    Cvt<E>::unpack(u, t);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) f[i] = make_float2(t[2 * i], t[2 * i + 1]);
-}
-template <typename E> __device__ __forceinline__ uint4 pack2(const float2* f) {
-    return make_uint4(Cvt<E>::pack2(f[0].x, f[0].y), Cvt<E>::pack2(f[1].x, f[1].y), Cvt<E>::pack2(f[2].x, f[2].y), Cvt<E>::pack2(f[3].x, f[3].y));
-}
-// x + y of eight 16-bit values each, rounded: the residual stream
-template <typename E> __device__ __forceinline__ uint4 add_rows(const uint4& x, const uint4& y) {
-    float2 a[4], b[4];
-    unpack2<E>(x, a);
-    unpack2<E>(y, b);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) a[i] = add2(a[i], b[i]);
-    return pack2<E>(a);
-}
-
 template <typename E, bool TRAIN>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     mlp_kernel(const __grid_constant__ Maps maps, const __grid_constant__ Plan plan, const __grid_constant__ Args<E> g) {
@@ -134,7 +70,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     uint8_t* rows_smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(raw) + 1023) & ~(uintptr_t)1023);
     uint8_t* ring = rows_smem + 2 * kRowsBytes;
     uint8_t* stages = ring + kSlots * kSlotBytes;
-    float* biases = reinterpret_cast<float*>(stages + kGeluWarps * kGeluStage + kResultWarps * kStage);   // b2, b1
+    float* biases = reinterpret_cast<float*>(stages + kResultWarps * kStage);   // b2, b1
     __shared__ Barriers bar;
     const int warp = ptx::warp_index(), lane = threadIdx.x & 31;
     const uint32_t rank = pair::cta_rank();
@@ -166,60 +102,63 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
         ptx::warpgroup_regs_shrink<kGeluRegs>();
         const int q = warp & 3, part = warp >> 2;   // tensor-memory lanes 32 q .. + 31, columns of this quarter
         const uint32_t lanes = (uint32_t)(q * 32) << 16;
-        uint8_t* stage = stages + warp * kGeluStage;
         const uint32_t g_ready0 = pair::in_leader(&bar.g_ready[0]), g_ready1 = pair::in_leader(&bar.g_ready[1]);
         int j = 0;
         for (int i = first; ok && i < plan.items; i += step) {
             const Item t = item_at(plan, i);
-            const int row0 = t.tile * 256 + (int)rank * 128 + q * 32;
+            const int row = t.tile * 256 + (int)rank * 128 + q * 32 + lane;
             for (int c = t.c0; c < t.c1; ++c, ++j) {
                 const int buf = j & 1, col = c * kChunk + part * 32;
                 const uint32_t s = tmem + lanes + kHidden + buf * kChunk + part * 32;
                 const float4* b1 = reinterpret_cast<const float4*>(biases + kD + col);
                 if (!ptx::mbar_wait(&bar.s_full[buf], (j >> 1) & 1) || *abort_flag) NA1D_MLP_FAIL(1)
                 ptx::tc_fence_after_sync();
-                float d[32];
-                pair::tmem_ld32(s, d);
-                ptx::tmem_ld_wait();
-                uint32_t packed[16];
+                if constexpr (TRAIN) {   // sixteen columns at a time: a short loop, and one sector of each row
+#pragma unroll 1
+                    for (int h = 0; h < 2; ++h) {
+                        float d[16];
+                        pair::tmem_ld16(s + h * 16, d);
+                        ptx::tmem_ld_wait();
+                        uint32_t packed[8], hidden[8];
 #pragma unroll
-                for (int k = 0; k < 8; ++k) {
-                    const float4 bias = b1[k];
-                    const float2 u = add2(make_float2(d[4 * k], d[4 * k + 1]), make_float2(bias.x, bias.y));
-                    const float2 v = add2(make_float2(d[4 * k + 2], d[4 * k + 3]), make_float2(bias.z, bias.w));
-                    if (TRAIN) { d[2 * k] = __uint_as_float(Cvt<E>::pack2(u.x, u.y)); d[2 * k + 1] = __uint_as_float(Cvt<E>::pack2(v.x, v.y)); }
-                    const float2 gu = gelu2(u), gv = gelu2(v);
-                    packed[2 * k] = Cvt<E>::pack2(gu.x, gu.y);
-                    packed[2 * k + 1] = Cvt<E>::pack2(gv.x, gv.y);
+                        for (int k = 0; k < 4; ++k) {
+                            const float4 bias = b1[h * 4 + k];
+                            const float2 u = add2(make_float2(d[4 * k], d[4 * k + 1]), make_float2(bias.x, bias.y));
+                            const float2 v = add2(make_float2(d[4 * k + 2], d[4 * k + 3]), make_float2(bias.z, bias.w));
+                            hidden[2 * k] = Cvt<E>::pack2(u.x, u.y);
+                            hidden[2 * k + 1] = Cvt<E>::pack2(v.x, v.y);
+                            const float2 gu = gelu2(u), gv = gelu2(v);
+                            packed[2 * k] = Cvt<E>::pack2(gu.x, gu.y);
+                            packed[2 * k + 1] = Cvt<E>::pack2(gv.x, gv.y);
+                        }
+                        pair::tmem_st8(s + h * 8, packed);   // over columns that this warp has read
+                        if (row < plan.rows) store_sector(g.f + (size_t)row * F + col + h * 16, hidden);
+                    }
+                } else {
+                    float d[32];
+                    pair::tmem_ld32(s, d);
+                    ptx::tmem_ld_wait();
+                    uint32_t packed[16];
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) {
+                        const float4 bias = b1[k];
+                        const float2 gu = gelu2(add2(make_float2(d[4 * k], d[4 * k + 1]), make_float2(bias.x, bias.y)));
+                        const float2 gv = gelu2(add2(make_float2(d[4 * k + 2], d[4 * k + 3]), make_float2(bias.z, bias.w)));
+                        packed[2 * k] = Cvt<E>::pack2(gu.x, gu.y);
+                        packed[2 * k + 1] = Cvt<E>::pack2(gv.x, gv.y);
+                    }
+                    pair::tmem_st16(s, packed);
                 }
-                pair::tmem_st16(s, packed);   // over columns that this warp has read
                 ptx::tmem_st_wait();
                 ptx::tc_fence_before_sync();
                 __syncwarp();
                 if (lane == 0) pair::arrive_cluster(buf ? g_ready1 : g_ready0);
-                if (TRAIN) {   // eight rows at a time
-                    E* dst = g.f + (size_t)row0 * F + col + (lane & 3) * 8;
-#pragma unroll 1
-                    for (int r0 = 0; r0 < 32; r0 += 8) {
-                        if (lane >= r0 && lane < r0 + 8) {
-#pragma unroll
-                            for (int k = 0; k < 4; ++k)
-                                *reinterpret_cast<uint4*>(stage + stage_at(lane & 7, k)) = make_uint4(__float_as_uint(d[4 * k]), __float_as_uint(d[4 * k + 1]),
-                                                                                                     __float_as_uint(d[4 * k + 2]), __float_as_uint(d[4 * k + 3]));
-                        }
-                        __syncwarp();
-                        const uint4 v = *reinterpret_cast<const uint4*>(stage + stage_at(lane >> 2, lane & 3));
-                        const int r = r0 + (lane >> 2);
-                        if (row0 + r < plan.rows) *reinterpret_cast<uint4*>(dst + (size_t)r * F) = v;
-                        __syncwarp();
-                    }
-                }
             }
         }
     } else if (warp < kGeluWarps + kResultWarps) {
         ptx::warpgroup_regs_grow<kResultRegs>();
         const int w = warp - kGeluWarps, q = warp & 3, half = w >> 2;
-        uint8_t* stage = stages + kGeluWarps * kGeluStage + w * kStage;
+        uint8_t* stage = stages + w * kStage;
         const uint32_t o_free = pair::in_leader(&bar.o_free), o = tmem + ((uint32_t)(q * 32) << 16) + kAcc + half * 128;
         int it = 0;
         for (int i = first; i < plan.items; i += step, ++it) {
@@ -324,6 +263,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
             if (ok && before >= 0) load(true, before);
             if (!ok && rank == 0)   // loads that are on their way arrive before the CTAs leave
                 for (int k = n - 1; k >= 0 && k >= n - kSlots; --k) ptx::mbar_wait(&bar.full[k % kSlots], (k / kSlots) & 1, 1u << 14);
+            if (!ok && rank == 0)
+                for (int k = it + 1; k >= 0 && k >= it; --k) ptx::mbar_wait(&bar.a_full[k & 1], (k >> 1) & 1, 1u << 12);
         }
         if (warp == kGeluWarps + kResultWarps + 1 && rank == 0 && ptx::elect_one()) {
             constexpr uint32_t fmt = tc::Fmt<E>::v;
@@ -411,20 +352,6 @@ __global__ void __launch_bounds__(256) mlp_finish_kernel(const __grid_constant__
     *reinterpret_cast<uint2*>(g.out + (size_t)row * g.ld + col) = make_uint2(sum.x, sum.y);
 }
 
-Plan make_plan(int64_t rows, int64_t F) {
-    Plan p;
-    const int pairs = device_sm_count() / 2, tiles = (int)((rows + 255) / 256);
-    p.rows = (int)rows;
-    p.pieces = (int)(F / kChunk);
-    p.whole = tiles / pairs * pairs;
-    const int rest = tiles - p.whole;
-    p.parts = rest ? pairs / rest : 1;
-    if (p.parts > p.pieces) p.parts = p.pieces;
-    if (p.parts < 2) { p.parts = 1; p.whole = tiles; }
-    p.items = p.whole + (tiles - p.whole) * p.parts;
-    return p;
-}
-size_t part_floats(const Plan& p) { return p.parts > 1 ? (size_t)(p.items - p.whole) * 256 * kD : 0; }
 template <typename E, bool TRAIN>
 cudaError_t run(const Maps& maps, const Plan& plan, const Args<E>& a, cudaStream_t st) {
     auto* kern = mlp_kernel<E, TRAIN>;

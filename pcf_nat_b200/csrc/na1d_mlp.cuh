@@ -1,0 +1,113 @@
+// Pieces that the kernels of a block's MLP share: how rows and hidden layer are shared out, pairs of fp32 values, turning rows per lane into
+// rows of adjacent lanes.
+#pragma once
+#include "na1d_pair.cuh"
+
+namespace na1d {
+namespace {
+
+constexpr int kD = 256, kChunk = 128, kMostF = 1280;
+constexpr int kRowsBytes = 128 * kD * 2;          // a CTA's rows as an operand: four blocks of 64 channels, [block][row][128 bytes]
+constexpr int kSlotBytes = 16 * 1024;             // a CTA's half of half a weight piece
+constexpr uint32_t kAcc = 0, kHidden = 256;       // tensor-memory columns: result (256), two pieces of the hidden layer (128 each)
+
+// Items: whole tiles of 256 rows in full rounds of the CTA pairs, then the tiles of the last, partly filled round split over the hidden
+// layer into `parts`, so that this round takes 1 / parts of the time (150 tiles on 74 pairs: 2.1 instead of 3).
+struct Plan {
+    int rows, pieces, whole, parts, items;
+};
+struct Item {
+    int tile, part, parts, c0, c1;
+};
+__device__ __forceinline__ Item item_at(const Plan& p, int i) {
+    Item t;
+    if (i < p.whole) {
+        t.tile = i; t.part = 0; t.parts = 1; t.c0 = 0; t.c1 = p.pieces;
+    } else {
+        i -= p.whole;
+        t.tile = i / p.parts;
+        t.part = i - t.tile * p.parts;
+        t.tile += p.whole;
+        t.parts = p.parts;
+        t.c0 = p.pieces * t.part / p.parts;
+        t.c1 = p.pieces * (t.part + 1) / p.parts;
+    }
+    return t;
+}
+
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    float2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;"
+        : "=l"(reinterpret_cast<uint64_t&>(d))
+        : "l"(reinterpret_cast<const uint64_t&>(a)), "l"(reinterpret_cast<const uint64_t&>(b)), "l"(reinterpret_cast<const uint64_t&>(c)));
+    return d;
+}
+__device__ __forceinline__ float2 both(float x) { return make_float2(x, x); }
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+    float2 d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(reinterpret_cast<uint64_t&>(d)) : "l"(reinterpret_cast<const uint64_t&>(a)), "l"(reinterpret_cast<const uint64_t&>(b)));
+    return d;
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+    float2 d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(reinterpret_cast<uint64_t&>(d)) : "l"(reinterpret_cast<const uint64_t&>(a)), "l"(reinterpret_cast<const uint64_t&>(b)));
+    return d;
+}
+// -min(|x|, 64), of a NaN NaN: beyond that the tail of GELU is zero anyway, and an infinite argument keeps its value (no infinity times zero)
+__device__ __forceinline__ float minus_abs(float x) {
+    float r;
+    asm("max.NaN.f32 %0, %1, 0fC2800000;" : "=f"(r) : "f"(-fabsf(x)));
+    return r;
+}
+// rows that are read once, in program order, so that they are in flight together
+__device__ __forceinline__ uint4 load_row(const void* p) {
+    uint4 v;
+    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
+// 32 bytes, a sector, of a row: of each of a warp's 32 rows at a time
+__device__ __forceinline__ void load_sector(const void* p, uint32_t* v) {
+    asm volatile("ld.global.nc.L1::no_allocate.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]) : "l"(p));
+}
+__device__ __forceinline__ void store_sector(void* p, const uint32_t* v) {
+    asm volatile("st.global.L1::no_allocate.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+                 ::"l"(p), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]) : "memory");
+}
+__device__ __forceinline__ uint32_t stage_at(int row, int chunk) { return (uint32_t)(row * 64 + ((chunk ^ (row >> 1)) & 3) * 16); }
+template <typename E> __device__ __forceinline__ void unpack2(const uint4& u, float2* f) {
+    float t[8];
+    Cvt<E>::unpack(u, t);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) f[i] = make_float2(t[2 * i], t[2 * i + 1]);
+}
+template <typename E> __device__ __forceinline__ uint4 pack2(const float2* f) {
+    return make_uint4(Cvt<E>::pack2(f[0].x, f[0].y), Cvt<E>::pack2(f[1].x, f[1].y), Cvt<E>::pack2(f[2].x, f[2].y), Cvt<E>::pack2(f[3].x, f[3].y));
+}
+// x + y of eight 16-bit values each, rounded: the residual stream
+template <typename E> __device__ __forceinline__ uint4 add_rows(const uint4& x, const uint4& y) {
+    float2 a[4], b[4];
+    unpack2<E>(x, a);
+    unpack2<E>(y, b);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) a[i] = add2(a[i], b[i]);
+    return pack2<E>(a);
+}
+
+inline Plan make_plan(int64_t rows, int64_t F) {
+    Plan p;
+    const int pairs = device_sm_count() / 2, tiles = (int)((rows + 255) / 256);
+    p.rows = (int)rows;
+    p.pieces = (int)(F / kChunk);
+    p.whole = tiles / pairs * pairs;
+    const int rest = tiles - p.whole;
+    p.parts = rest ? pairs / rest : 1;
+    if (p.parts > p.pieces) p.parts = p.pieces;
+    if (p.parts < 2) { p.parts = 1; p.whole = tiles; }
+    p.items = p.whole + (tiles - p.whole) * p.parts;
+    return p;
+}
+inline size_t part_floats(const Plan& p) { return p.parts > 1 ? (size_t)(p.items - p.whole) * 256 * kD : 0; }
+
+}  // namespace
+}  // namespace na1d

@@ -519,8 +519,8 @@ Tensor layer_norm_backward(Tensor& sums, const Tensor& dy, const Tensor& s, cons
 }
 
 // x (+ dx): the residual stream. Returns the stream after the attention branch and the MLP branch's output; their sum is the
-// block's output, taken inside the next block's first LayerNorm. Without a backward pass to come, and at the sizes that the MLP kernel takes,
-// the sum alone (the second tensor undefined), in `out` if that is given: rows of D inside wider ones.
+// block's output, taken inside the next block's first LayerNorm. At the sizes that the MLP kernel takes, the sum alone (the second tensor
+// undefined), without a backward pass to come in `out` if that is given: rows of D inside wider ones.
 std::pair<Tensor, Tensor> block_forward(const Tensor& x, const Tensor& dx, const Tensor& vl, const Packed& c, double eps1, double eps2,
                                         const Tensor* p, BlockState* keep, const OptTensor& out = std::nullopt) {
     const int64_t D = x.size(2), rows = c.B * c.T;
@@ -535,21 +535,22 @@ std::pair<Tensor, Tensor> block_forward(const Tensor& x, const Tensor& dx, const
     packed_forward(st.o, st.lse, st.qkv, p[12], vl, c);
     const Tensor y = product(st.o.view({rows, D}), w.t[2], w.t[3], false).view({c.B, c.T, D});
     layer_norm(st.h2, st.s2, st.st2, st.s1, y, p[10], p[11], eps2, stats);
-    if (!keep) {
-        const int64_t F = w.t[4].size(0), floats = na1d_mlp_scratch_floats(rows, D, F);
-        if (floats >= 0) {
-            const Tensor sum = out ? *out : at::empty_like(x), scratch = floats ? empty_f32({floats}, x) : Tensor();
-            check(na1d_mlp_forward(ptr(sum), sum.stride(1), nullptr, ptr(st.s2), ptr(st.h2), ptr(w.t[4]), fptr(p[5]), ptr(w.t[6]), fptr(p[7]), fptr(scratch), rows,
-                                   D, F, code(x), stream()),
-                  "na1d_mlp_forward");
-            return {sum, Tensor()};
-        }
+    const int64_t F = w.t[4].size(0), floats = na1d_mlp_scratch_floats(rows, D, F);
+    Tensor s2, z;
+    if (floats >= 0) {
+        const Tensor scratch = floats ? empty_f32({floats}, x) : Tensor();
+        s2 = out && !keep ? *out : at::empty_like(x);
+        if (keep) st.f = at::empty({rows, F}, x.options());
+        check(na1d_mlp_forward(ptr(s2), s2.stride(1), ptr(st.f), ptr(st.s2), ptr(st.h2), ptr(w.t[4]), fptr(p[5]), ptr(w.t[6]), fptr(p[7]), fptr(scratch), rows, D, F,
+                               code(x), stream()),
+              "na1d_mlp_forward");
+    } else {
+        st.f = product(st.h2.view({rows, D}), w.t[4], w.t[5], false);
+        st.g = at::empty_like(st.f);
+        check(na1d_gelu_forward(ptr(st.g), ptr(st.f), st.f.numel(), code(x), stream()), "na1d_gelu_forward");
+        z = product(st.g, w.t[6], w.t[7], false).view({c.B, c.T, D});
+        s2 = st.s2;
     }
-    st.f = product(st.h2.view({rows, D}), w.t[4], w.t[5], false);
-    st.g = at::empty_like(st.f);
-    check(na1d_gelu_forward(ptr(st.g), ptr(st.f), st.f.numel(), code(x), stream()), "na1d_gelu_forward");
-    Tensor z = product(st.g, w.t[6], w.t[7], false).view({c.B, c.T, D});
-    Tensor s2 = st.s2;
     if (keep) {
         st.buf = w.buf;
         *keep = std::move(st);
@@ -569,7 +570,7 @@ struct NA1dBlock : public torch::autograd::Function<NA1dBlock> {
         ctx->save_for_backward({st.s1, st.st1, st.h1, st.qkv, st.lse, st.o, st.s2, st.st2, st.h2, st.f, st.g, st.buf, p8, p10, p12, vl ? *vl : Tensor(), p9, p11});
         auto& d = ctx->saved_data;
         d["heads"] = heads; d["win"] = win; d["left"] = left; d["scale"] = scale; d["dx"] = dx.has_value(); d["eps1"] = eps1; d["eps2"] = eps2;
-        return {out.first, out.second};
+        return out.second.defined() ? variable_list{out.first, out.second} : variable_list{out.first};
     }
     // x, dx, then the parameters; w: the 16-bit ones
     static variable_list differentiable(const variable_list& s, const Packed& c, const Projections& w, double eps1, double eps2, bool has_dx, int first,
@@ -587,12 +588,13 @@ struct NA1dBlock : public torch::autograd::Function<NA1dBlock> {
         const Tensor x = has_dx ? in[0] + in[1] : in[0];
         const Tensor o = NA1dFusedPacked::apply(linear(norm(x, 8, eps1), 0), p[12], vl.defined() ? OptTensor(vl) : OptTensor(), c.H, c.win, c.left, 1, c.scale);
         const Tensor s2 = x + linear(o, 2);
-        return inner_gradients({s2, linear(at::gelu(linear(norm(s2, 10, eps2), 4)), 6)}, in, grads);
+        const Tensor z = linear(at::gelu(linear(norm(s2, 10, eps2), 4)), 6);
+        return inner_gradients(grads.size() == 1 ? variable_list{s2 + z} : variable_list{s2, z}, in, grads);
     }
     static variable_list backward(AutogradContext* ctx, variable_list grads) {
         const variable_list s = ctx->get_saved_variables();
-        const Tensor &s1 = s[0], &st1 = s[1], &h1 = s[2], &qkv = s[3], &lse = s[4], &o = s[5], &s2 = s[6], &st2 = s[7], &h2 = s[8], &f = s[9], &g = s[10],
-                     &buf = s[11], &n1w = s[12], &n2w = s[13], &rpb = s[14], &vl = s[15];
+        const Tensor &s1 = s[0], &st1 = s[1], &h1 = s[2], &qkv = s[3], &lse = s[4], &o = s[5], &s2 = s[6], &st2 = s[7], &h2 = s[8], &f = s[9], &buf = s[11], &n1w = s[12], &n2w = s[13], &rpb = s[14], &vl = s[15];
+        Tensor g = s[10];
         auto& data = ctx->saved_data;
         const Packed c(qkv, data["heads"].toInt(), data["win"].toInt(), data["left"].toInt(), 1, data["scale"].toDouble());
         const c10::cuda::CUDAGuard guard(s1.device());
@@ -615,18 +617,30 @@ struct NA1dBlock : public torch::autograd::Function<NA1dBlock> {
             return out;
         }
         const Tensor scratch = empty_f32({na1d_block_scratch_floats(rows, D, std::max(F, 3 * D))}, s1);
-        const Tensor d_z = (grads[1].defined() ? aligned(grads[1]) : at::zeros_like(s2)).view({rows, D});
-        const Tensor d_s2 = grads[0].defined() ? aligned(grads[0]) : Tensor();
+        const bool one = grads.size() == 1;   // the output is s2 + z, from the MLP kernel
+        const Tensor d_s2 = grads[0].defined() ? aligned(grads[0]) : one ? at::zeros_like(s2) : Tensor();
+        const Tensor d_z = (one ? d_s2 : grads[1].defined() ? aligned(grads[1]) : at::zeros_like(s2)).view({rows, D});
         // MLP branch
-        Tensor d_b1 = empty_f32({F}, s1), d_f = at::empty_like(f);
-        {
+        Tensor d_b1, d_f = at::empty_like(f), d_h;
+        if (one) {
+            const int64_t floats = na1d_mlp_scratch_floats(rows, D, F);
+            const Tensor part = floats ? empty_f32({floats}, s1) : Tensor();
+            d_h = at::empty_like(s2);
+            g = at::empty_like(f);
+            check(na1d_mlp_backward(ptr(d_h), ptr(d_f), ptr(g), ptr(d_z), ptr(f), ptr(w.t[4]), ptr(w.t[6]), fptr(part), rows, D, F, code(f), stream()),
+                  "na1d_mlp_backward");
+        } else {
             const Tensor d_g = product(d_z, w.t[6], Tensor(), true);
+            d_b1 = empty_f32({F}, s1);
             check(na1d_gelu_backward(ptr(d_f), fptr(d_b1), fptr(scratch), ptr(d_g), ptr(f), rows, F, code(f), stream()), "na1d_gelu_backward");
+            d_h = product(d_f, w.t[4], Tensor(), true);
         }
-        const ParameterGrads mlp({d_f, d_z}, {h2.view({rows, D}), g}, {need(4), need(6)}, {false, need(7)}, at::kFloat);
-        Tensor sums2, sums1;
-        const Tensor d_y = layer_norm_backward(sums2, product(d_f, w.t[4], Tensor(), true), s2, st2, n2w, d_s2, scratch);   // also the residual stream's gradient
+        const ParameterGrads mlp({d_f, d_z}, {h2.view({rows, D}), g}, {need(4), need(6)}, {one && need(5), need(7)}, at::kFloat);
+        if (one) d_b1 = mlp.b[0];
         d_f.reset();
+        g.reset();
+        Tensor sums2, sums1;
+        const Tensor d_y = layer_norm_backward(sums2, d_h, s2, st2, n2w, d_s2, scratch);   // also the residual stream's gradient
         // attention branch
         const Tensor dy2 = d_y.view({rows, D});
         Tensor d_qkv = at::empty_like(qkv), d_rpb;
@@ -653,7 +667,7 @@ std::optional<std::pair<Tensor, Tensor>> block(const Tensor& x, const OptTensor&
     if (at::GradMode::is_enabled()) {
         const variable_list r = NA1dBlock::apply(x, dx, vl, heads, win, left, scale, eps1, eps2, p[0], p[1], p[2], p[3], p[4], p[5], p[6], p[7], p[8],
                                                  p[9], p[10], p[11], p[12]);
-        return std::make_pair(r[0], r[1]);
+        return std::make_pair(r[0], r.size() > 1 ? r[1] : Tensor());
     }
     const Packed c(x.size(0), x.size(1), x.size(2), heads, win, left, 1, scale);
     return block_forward(x, dx ? *dx : Tensor(), vl ? *vl : Tensor(), c, eps1, eps2, p.data(), nullptr, out);
