@@ -15,7 +15,7 @@ import torch.nn as nn
 
 from . import _lib, ops
 from ._lib import check
-from .nattention import NAttention, global_hooks, hooked
+from .nattention import NAttention, _plain_linear, global_hooks, hooked
 
 _L = _lib.lib()
 _CODE = {torch.bfloat16: _lib.NA1D_BF16, torch.float16: _lib.NA1D_FP16}
@@ -110,6 +110,33 @@ def run_blocks(blocks, x, valid, out=None, training=None):
     if out is not None:
         return x if x is out or x.data_ptr() == out.data_ptr() else add_to_rows(out, x, dx)
     return x if dx is None else x + dx
+
+
+# ------------------------------------------------------------------ a projection of the features so far
+def fuse(linear, feats):
+    """``linear(torch.cat(feats, -1))`` as one node, for a backward pass: the result and the features as what comes next has to read
+    them, so that their gradients are summed inside its products; None where it has to run in PyTorch's operations."""
+    x = feats[0]
+    if (not torch.is_grad_enabled() or type(x) is not torch.Tensor or not x.is_cuda or x.dim() != 3 or x.numel() == 0 or torch.compiler.is_compiling() or
+            not torch.is_autocast_enabled() or not ops.native.eager_mode() or torch.autograd.forward_ad._current_level >= 0 or global_hooks()):
+        return None
+    dt = torch.get_autocast_dtype("cuda")
+    if x.dtype != dt or dt not in _CODE or not _plain_linear(linear):
+        return None
+    w, b = linear.weight, linear.bias
+    for p in (w, b):
+        if (p is None or type(p) not in (nn.Parameter, torch.Tensor) or p.dtype != torch.float32 or p.device != x.device or not p.is_contiguous() or
+                p.data_ptr() % 16):
+            return None
+    for f in feats:
+        if type(f) is not torch.Tensor or f.shape != x.shape or f.dtype != dt or f.device != x.device or not f.is_contiguous() or f.data_ptr() % 16:
+            return None
+    D, K = x.shape[-1], x.shape[-1] * len(feats)
+    if (D % 8 or w.shape[0] % 8 or w.shape[1] != K or b.shape != w.shape[:1] or K > 1 << 20 or w.shape[0] > 1 << 20 or w.numel() > (2 ** 31 - 1) // 16 or
+            x.shape[0] * x.shape[1] * max(K, w.shape[0]) >= 2 ** 31):
+        return None
+    y, *rest = ops.native.fuse(w, b, list(feats))
+    return y, rest
 
 
 # ------------------------------------------------------------------ statistics pooling

@@ -60,20 +60,22 @@ inline Tensor zeros_f32(at::IntArrayRef shape, const Tensor& like) {
 // and at::mm run, without their work for each call (13 to 16 us of host time, 5 here). What the library proposes for sizes, types and
 // alignments is kept under exactly those, for each host thread by itself, 256 of them at most.
 struct ProductKey {
-    int64_t rows, N, K;
+    int64_t rows, N, K, ldw, ldc;   // ldc: 0 without an addend
     int32_t kind, align;   // device, type, orientation, bias; the operands' alignments
-    bool operator==(const ProductKey& o) const { return rows == o.rows && N == o.N && K == o.K && kind == o.kind && align == o.align; }
+    bool operator==(const ProductKey& o) const {
+        return rows == o.rows && N == o.N && K == o.K && ldw == o.ldw && ldc == o.ldc && kind == o.kind && align == o.align;
+    }
 };
 struct ProductKeyHash {
     size_t operator()(const ProductKey& k) const {
         size_t h = 1469598103934665603ull;
-        for (size_t v : {(size_t)k.rows, (size_t)k.N, (size_t)k.K, (size_t)k.kind, (size_t)k.align}) h = (h ^ v) * 1099511628211ull;
+        for (size_t v : {(size_t)k.rows, (size_t)k.N, (size_t)k.K, (size_t)k.ldw, (size_t)k.ldc, (size_t)k.kind, (size_t)k.align}) h = (h ^ v) * 1099511628211ull;
         return h ^ (h >> 29);
     }
 };
 struct ProductPlan {
     cublasLtMatmulDescOpaque_t desc;
-    cublasLtMatrixLayoutOpaque_t w, x, y;
+    cublasLtMatrixLayoutOpaque_t w, x, y, c;
     cublasLtMatmulAlgo_t algo;
     bool usable;
 };
@@ -92,8 +94,9 @@ bool plan_product(ProductPlan& p, const ProductKey& k, cublasLtHandle_t handle, 
     const size_t workspace = at::cuda::getCUDABlasLtWorkspaceSize();
     cublasLtMatmulPreferenceOpaque_t pref;
     if (cublasLtMatmulDescInit(&p.desc, CUBLAS_COMPUTE_32F, CUDA_R_32F) || cublasLtMatmulDescSetAttribute(&p.desc, CUBLASLT_MATMUL_DESC_TRANSA, &op, sizeof op) ||
-        cublasLtMatrixLayoutInit(&p.w, type, w_transposed ? k.N : k.K, w_transposed ? k.K : k.N, w_transposed ? k.N : k.K) ||
-        cublasLtMatrixLayoutInit(&p.x, type, k.K, k.rows, k.K) || cublasLtMatrixLayoutInit(&p.y, type, k.N, k.rows, k.N) || cublasLtMatmulPreferenceInit(&pref) ||
+        cublasLtMatrixLayoutInit(&p.w, type, w_transposed ? k.N : k.K, w_transposed ? k.K : k.N, k.ldw) ||
+        cublasLtMatrixLayoutInit(&p.x, type, k.K, k.rows, k.K) || cublasLtMatrixLayoutInit(&p.y, type, k.N, k.rows, k.N) ||
+        cublasLtMatrixLayoutInit(&p.c, type, k.N, k.rows, k.ldc ? k.ldc : k.N) || cublasLtMatmulPreferenceInit(&pref) ||
         cublasLtMatmulPreferenceSetAttribute(&pref, CUBLASLT_MATMUL_PREF_MAX_WORKSPACE_BYTES, &workspace, sizeof workspace) ||
         cublasLtMatmulPreferenceSetAttribute(&pref, CUBLASLT_MATMUL_PREF_REDUCTION_SCHEME_MASK, &reductions, sizeof reductions))
         return false;
@@ -108,21 +111,24 @@ bool plan_product(ProductPlan& p, const ProductKey& k, cublasLtHandle_t handle, 
     }
     cublasLtMatmulHeuristicResult_t found = {};
     int n = 0;
-    if (cublasLtMatmulAlgoGetHeuristic(handle, &p.desc, &p.w, &p.x, &p.y, &p.y, &pref, 1, &found, &n) || n < 1) return false;
+    if (cublasLtMatmulAlgoGetHeuristic(handle, &p.desc, &p.w, &p.x, &p.c, &p.y, &pref, 1, &found, &n) || n < 1) return false;
     p.algo = found.algo;
     p.usable = true;
     return true;
 }
-Tensor product(const Tensor& x, const Tensor& w, const Tensor& b, bool w_transposed) {
+// `add`, (rows, N): added before the result is rounded. It and w may be column slices of wider matrices.
+Tensor product(const Tensor& x, const Tensor& w, const Tensor& b, bool w_transposed, const Tensor& add = Tensor()) {
     const int64_t rows = x.size(0), K = x.size(1), N = w.size(w_transposed ? 1 : 0);
     Tensor y = at::empty({rows, N}, x.options());
-    const bool bias = b.defined();
-    const int32_t align[4] = {alignment(ptr(w)), alignment(ptr(x)), alignment(ptr(y)), bias ? alignment(ptr(b)) : 4};
-    const bool dense = x.is_contiguous() && w.is_contiguous() && K % 8 == 0 && N % 8 == 0 && rows <= INT32_MAX && align[0] >= 0 && align[1] >= 0 && align[2] >= 0 && align[3] >= 0;
+    const bool bias = b.defined(), sum = add.defined();
+    const int32_t align[4] = {alignment(ptr(w)), alignment(ptr(x)), sum ? std::min(alignment(ptr(add)), alignment(ptr(y))) : alignment(ptr(y)),
+                              bias ? alignment(ptr(b)) : 4};
+    auto slice = [](const Tensor& t) { return t.stride(1) == 1 && t.stride(0) >= t.size(1) && t.stride(0) % 8 == 0; };
+    const bool dense = x.is_contiguous() && slice(w) && (!sum || slice(add)) && K % 8 == 0 && N % 8 == 0 && rows <= INT32_MAX && align[0] >= 0 && align[1] >= 0 && align[2] >= 0 && align[3] >= 0;
     if (dense) {
         static thread_local std::unordered_map<ProductKey, ProductPlan, ProductKeyHash> plans;
         const cudaDataType_t type = x.scalar_type() == at::kBFloat16 ? CUDA_R_16BF : CUDA_R_16F;
-        const ProductKey key{rows, N, K, (int32_t)(x.get_device() * 8 + code(x) * 4 + w_transposed * 2 + bias), align[0] | align[1] << 4 | align[2] << 8};
+        const ProductKey key{rows, N, K, w.stride(0), sum ? add.stride(0) : 0, (int32_t)(x.get_device() * 8 + code(x) * 4 + w_transposed * 2 + bias), align[0] | align[1] << 4 | align[2] << 8};
         const cublasLtHandle_t handle = at::cuda::getCurrentCUDABlasLtHandle();
         auto it = plans.find(key);
         if (it == plans.end()) {
@@ -132,12 +138,13 @@ Tensor product(const Tensor& x, const Tensor& w, const Tensor& b, bool w_transpo
         }
         ProductPlan& p = it->second;
         const void* bp = ptr(b);
-        const float one = 1.f, zero = 0.f;
+        const float one = 1.f, beta = sum ? 1.f : 0.f;
         if (p.usable && !(bias && cublasLtMatmulDescSetAttribute(&p.desc, CUBLASLT_MATMUL_DESC_BIAS_POINTER, &bp, sizeof bp)) &&
-            cublasLtMatmul(handle, &p.desc, &one, ptr(w), &p.w, ptr(x), &p.x, &zero, ptr(y), &p.y, ptr(y), &p.y, &p.algo, at::cuda::getCUDABlasLtWorkspace(),
+            cublasLtMatmul(handle, &p.desc, &one, ptr(w), &p.w, ptr(x), &p.x, &beta, sum ? ptr(add) : ptr(y), &p.c, ptr(y), &p.y, &p.algo, at::cuda::getCUDABlasLtWorkspace(),
                            at::cuda::getCUDABlasLtWorkspaceSize(), at::cuda::getCurrentCUDAStream().stream()) == CUBLAS_STATUS_SUCCESS)
             return y;
     }
+    if (sum) return at::add(at::mm(x, w_transposed ? w : w.t()), add);
     if (!bias) return at::mm(x, w_transposed ? w : w.t());
     return at::addmm(b, x, w_transposed ? w : w.t());
 }
@@ -558,6 +565,80 @@ std::pair<Tensor, Tensor> block_forward(const Tensor& x, const Tensor& dx, const
     return {s2, z};
 }
 
+// ---------------------------------------------------------------- a projection of tensors side by side
+// y = cat(parts) w^T + b, and the parts themselves for what reads them next: their gradients then come through this node, which adds its own
+// share inside the product that makes it. (Summed by autograd instead, the 20 contributions of a network of six stages were slices
+// of wider gradients, 27 us each at 38400 rows of 256 where the products with the addition take 11 to 13; the bias gradient, a column sum
+// of 54 us, comes with the weight gradient.)
+struct NA1dFuse : public torch::autograd::Function<NA1dFuse> {
+    static variable_list forward(AutogradContext* ctx, const Tensor& weight, const Tensor& bias, at::TensorList parts) {
+        const Tensor& x = parts[0];
+        const int64_t D = x.size(2), rows = x.size(0) * x.size(1), O = weight.size(0), K = weight.size(1);
+        const float* src[2] = {fptr(weight), fptr(bias)};
+        const int64_t n[2] = {O * K, O}, dst[2] = {0, (O * K + kSlot - 1) / kSlot * kSlot};
+        const Tensor buf = at::empty({dst[1] + O}, x.options());
+        check(na1d_cast_parameters(ptr(buf), src, dst, n, 2, code(x), stream()), "na1d_cast_parameters");
+        const Tensor w = buf.as_strided({O, K}, {K, 1}, 0), b = buf.as_strided({O}, {1}, dst[1]);
+        const Tensor cat = at::cat(parts, 2);
+        const Tensor y = product(cat.view({rows, K}), w, b, false).view({x.size(0), x.size(1), O});
+        ctx->save_for_backward({cat, buf});
+        ctx->saved_data["D"] = D;
+        ctx->saved_data["O"] = O;
+        ctx->set_materialize_grads(false);
+        variable_list out = {y};
+        out.insert(out.end(), parts.begin(), parts.end());
+        return out;
+    }
+    static variable_list backward(AutogradContext* ctx, variable_list grads) {
+        const variable_list s = ctx->get_saved_variables();
+        const Tensor &cat = s[0], &buf = s[1];
+        const int64_t D = ctx->saved_data["D"].toInt(), O = ctx->saved_data["O"].toInt(), K = cat.size(2), rows = cat.size(0) * cat.size(1), parts = K / D;
+        const c10::cuda::CUDAGuard guard(cat.device());
+        const NoAutocast off;
+        const Tensor w = buf.as_strided({O, K}, {K, 1}, 0), b = buf.as_strided({O}, {1}, (O * K + kSlot - 1) / kSlot * kSlot);
+        if (at::GradMode::is_enabled()) {
+            variable_list in = {stand_in(w.to(at::kFloat), 0), stand_in(b.to(at::kFloat), 1)}, out = {Tensor()};
+            for (int64_t i = 0; i < parts; ++i) in.push_back(stand_in(cat.narrow(2, i * D, D), 2 + i));
+            out.insert(out.end(), in.begin() + 2, in.end());
+            out[0] = at::linear(at::cat(variable_list(in.begin() + 2, in.end()), 2), in[0].to(w.scalar_type()), in[1].to(w.scalar_type()));
+            for (size_t i = 0; i < out.size(); ++i)
+                if (!out[i].requires_grad()) grads[i] = Tensor();
+            return inner_gradients(out, in, grads);
+        }
+        variable_list result(2 + parts);
+        const Tensor dy = grads[0].defined() ? aligned(grads[0]).view({rows, O}) : Tensor();
+        for (int64_t i = 0; i < parts; ++i) {
+            if (!ctx->needs_input_grad(2 + i)) continue;
+            const Tensor& more = grads[1 + i];
+            if (!dy.defined()) {
+                result[2 + i] = more;
+                continue;
+            }
+            // rows of a wider gradient are read in place
+            Tensor add;
+            if (more.defined()) {
+                const bool in_place = more.stride(2) == 1 && more.stride(1) % 8 == 0 && more.stride(1) >= D && more.stride(0) == more.stride(1) * more.size(1) &&
+                                      more.storage_offset() >= 0 && (reinterpret_cast<uintptr_t>(more.data_ptr()) & 15u) == 0;
+                add = in_place ? more.as_strided({rows, D}, {more.stride(1), 1}) : aligned(more).view({rows, D});
+            }
+            result[2 + i] = product(dy, w.narrow(1, i * D, D), Tensor(), true, add).view({cat.size(0), cat.size(1), D});
+        }
+        if (dy.defined()) {
+            const Tensor x = cat.view({rows, K});
+            const ParameterGrads g({dy, dy}, {x, x}, {ctx->needs_input_grad(0), false}, {ctx->needs_input_grad(1), false}, at::kFloat);
+            result[0] = g.w[0];
+            result[1] = g.b[0];
+        }
+        return result;
+    }
+};
+
+std::vector<Tensor> fuse(const Tensor& weight, const Tensor& bias, const std::vector<Tensor>& parts) {
+    TORCH_CHECK(!parts.empty() && weight.size(1) == (int64_t)parts.size() * parts[0].size(2), "a fused projection takes parts of one width");
+    const c10::cuda::OptionalCUDAGuard guard(parts[0].device());
+    return NA1dFuse::apply(weight, bias, at::TensorList(parts));
+}
+
 struct NA1dBlock : public torch::autograd::Function<NA1dBlock> {
     static variable_list forward(AutogradContext* ctx, const Tensor& x, const OptTensor& dx, const OptTensor& vl, int64_t heads, int64_t win, int64_t left,
                                  double scale, double eps1, double eps2, const Tensor& p0, const Tensor& p1, const Tensor& p2, const Tensor& p3,
@@ -919,6 +1000,7 @@ PYBIND11_MODULE(_na1d_torch, m) {
     NA1D_DEF(av);
     NA1D_DEF(packed);
     NA1D_DEF(block);
+    NA1D_DEF(fuse);
     NA1D_DEF(layer);
     NA1D_DEF(valid_tokens);
 #undef NA1D_DEF

@@ -121,7 +121,6 @@ class PCFNATExtractor(nn.Module):
     def embedding(self, fbank, padding=None):
         x = self.front(fbank).transpose(1, 2).contiguous()  # (N, T, C)
         feats = [x]
-        outs = []
         valid = None
         if not self.training and padding is not None and x.is_cuda:
             valid = _valid_tokens(x.shape[1], padding, x.shape[0]).to(x.device)
@@ -140,14 +139,14 @@ class PCFNATExtractor(nn.Module):
                 if rows is not None and s == 0:
                     block.add_to_rows(rows[..., :C], feats[0])
                 x = y
-            outs.append(x)
             feats.append(x)
             if s + 1 < len(self.stages):
                 if rows is None:
-                    x = self.fuse[s](torch.cat(feats, dim=-1))
+                    y = block.fuse(self.fuse[s], feats)
+                    x, feats = (self.fuse[s](torch.cat(feats, dim=-1)), feats) if y is None else y
                 else:
                     x = self.fuse[s](rows.view(-1, rows.shape[-1])[:, :(s + 2) * C]).view(feats[0].shape)
-        return self._embed(self.pool(torch.cat(outs, dim=-1) if rows is None else rows[..., C:]))
+        return self._embed(self.pool(torch.cat(feats[1:], dim=-1) if rows is None else rows[..., C:]))
 
     def _embed(self, pooled):
         return self.embed(self.bn(pooled).to(self.embed.weight.dtype))

@@ -1,0 +1,82 @@
+"""A projection of tensors side by side as one node (block.fuse) against the concatenation and the layer."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _run(kind, lin, xs, stages, dtype, order):
+    """A chain as in the network: each stage projects all features so far; what comes out is a feature too. Loss over all of them side by
+    side (slices of a wide gradient), `order` 2: a gradient penalty."""
+    from pcf_nat_b200 import block
+    with torch.autocast("cuda", dtype=dtype):
+        feats, x = [xs[0] * 1], None
+        for s in range(stages):
+            feats.append(xs[s + 1] * 1 if x is None else torch.tanh(x) + xs[s + 1])
+            got = block.fuse(lin[s], feats) if kind == "node" else None
+            assert (got is None) == (kind != "node")
+            x, feats = (lin[s](torch.cat(feats, -1)), feats) if got is None else got
+        wide = torch.cat(feats[1:] + [x], -1).float()
+    loss = (wide * torch.linspace(-1, 1, wide.shape[-1], device="cuda")).sin().sum()
+    leaves = [t for t in list(xs[:stages + 1]) + [p for l in lin for p in l.parameters()] if t.requires_grad]
+    if order == 1:
+        return [wide.detach()] + list(torch.autograd.grad(loss, leaves))
+    g, = torch.autograd.grad(loss, xs[0], create_graph=True)
+    second = torch.autograd.grad(g.float().pow(2).sum(), leaves, allow_unused=True)
+    return [g.detach()] + [torch.zeros_like(t) if o is None else o for t, o in zip(leaves, second)]
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("N,T,D,stages,order", [(1, 1, 8, 1, 1), (2, 50, 64, 3, 1), (3, 33, 40, 2, 1), (8, 300, 256, 5, 1), (2, 50, 64, 3, 2)])
+@pytest.mark.parametrize("frozen", [False, True])
+def test_fuse(N, T, D, stages, order, dtype, frozen):
+    torch.manual_seed(N * T + D)
+    lin = [torch.nn.Linear((s + 2) * D, D).cuda() for s in range(stages)]
+    xs = [torch.randn(N, T, D, device="cuda").to(dtype).requires_grad_() for _ in range(stages + 1)]
+    if frozen:
+        lin[0].weight.requires_grad_(False)
+        lin[-1].bias.requires_grad_(False)
+        xs[-1].requires_grad_(False)
+    node, ops = (_run(kind, lin, xs, stages, dtype, order) for kind in ("node", "operations"))
+    # the chain is about four 16-bit tensors to a stage deep, in both; sums here are rounded once, there at every step
+    u = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    for i, (a, b) in enumerate(zip(node, ops)):
+        assert a.dtype == b.dtype and a.shape == b.shape
+        assert float((a.double() - b.double()).norm()) <= 4 * (stages + 1) * u * float(b.double().norm()) + 1e-5, i
+    assert len(node) == len(ops)
+    if order == 1 and dtype == torch.bfloat16 and not frozen:   # no further off than the operations
+        ref = _exact(lin, xs, stages)
+        for a, b, r in zip(node[1:], ops[1:], ref):
+            assert float((a.double() - r).norm()) <= 1.1 * float((b.double() - r).norm()) + 1e-5
+
+
+def _exact(lin, xs, stages):
+    ys = [t.detach().double().requires_grad_() for t in xs]
+    ps = [[p.detach().double().requires_grad_() for p in l.parameters()] for l in lin]
+    feats, x = [ys[0]], None
+    for s in range(stages):
+        feats.append(ys[s + 1] if x is None else torch.tanh(x) + ys[s + 1])
+        x = torch.cat(feats, -1) @ ps[s][0].t() + ps[s][1]
+    wide = torch.cat(feats[1:] + [x], -1)
+    loss = (wide * torch.linspace(-1, 1, wide.shape[-1], device="cuda")).sin().sum()
+    return torch.autograd.grad(loss, ys + [p for l in ps for p in l])
+
+
+def test_left_to_the_operations():
+    from pcf_nat_b200 import block
+    lin = torch.nn.Linear(128, 64).cuda()
+    x = torch.randn(2, 9, 64, device="cuda", dtype=torch.bfloat16)
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        assert block.fuse(lin, [x, x]) is not None
+        assert block.fuse(lin, [x, x.transpose(0, 1).contiguous().transpose(0, 1)]) is None and block.fuse(lin, [x, x.half()]) is None
+        assert block.fuse(lin, [x, x, x]) is None and block.fuse(torch.nn.Linear(128, 64, bias=False).cuda(), [x, x]) is None
+        assert block.fuse(lin.cuda().double(), [x, x]) is None
+        lin.float()
+        with torch.no_grad():
+            assert block.fuse(lin, [x, x]) is None
+        handle = lin.register_forward_hook(lambda *a: None)
+        assert block.fuse(lin, [x, x]) is None
+        handle.remove()
+    assert block.fuse(lin, [x, x]) is None      # without autocast
+    with torch.autocast("cuda", dtype=torch.float16):
+        assert block.fuse(lin, [x, x]) is None
