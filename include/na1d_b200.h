@@ -230,6 +230,10 @@ int na1d_layer_norm_forward(void* y, void* sum, float* mean, float* rstd, const 
 /* dx = gradient of the normalised rows x + res (res may be NULL); sums (3, D): gradients of w and b, column sums of dx. */
 int na1d_layer_norm_backward(void* dx, float* sums, float* scratch, const void* dy, const void* x, const float* mean,
                              const float* rstd, const float* w, const void* res, int64_t rows, int64_t D, int dtype, void* stream);
+/* The same without the sums, whose partial results stay in `scratch`, and the sums of two such passes over as many rows of D. */
+int na1d_layer_norm_backward_rows(void* dx, float* scratch, const void* dy, const void* x, const float* mean, const float* rstd, const float* w,
+                                  const void* res, int64_t rows, int64_t D, int dtype, void* stream);
+int na1d_layer_norm_sums(float* sums0, float* sums1, const float* scratch0, const float* scratch1, int64_t rows, int64_t D, void* stream);
 /* y = x Phi(x) (the exact form), n elements (n a multiple of 8). */
 int na1d_gelu_forward(void* y, const void* x, int64_t n, int dtype, void* stream);
 /* dx = dy * d gelu(x), (rows, F); sums (F): column sums of dx. */

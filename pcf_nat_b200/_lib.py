@@ -90,6 +90,8 @@ _lib.na1d_block_scratch_floats.restype = _i64
 _lib.na1d_block_scratch_floats.argtypes = [_i64, _i64, _i64]
 _lib.na1d_fused_backward_workspace_floats.restype = _i64
 _lib.na1d_fused_backward_workspace_floats.argtypes = [_i64] * 7 + [_i32] * 3
+_lib.na1d_layer_norm_sums.restype = _i32
+_lib.na1d_layer_norm_sums.argtypes = [_ptr] * 4 + [_i64, _i64, _ptr]
 _lib.na1d_zero.restype = _i32
 _lib.na1d_zero.argtypes = [_ptr, _i64, _ptr]
 _lib.na1d_mlp_scratch_floats.restype = _i64
@@ -99,6 +101,7 @@ _lib.na1d_projection_gradients_scratch.argtypes = [_ptr, _ptr, _i32, _i64]
 for _name, _args in (
         ("na1d_layer_norm_forward", [_ptr] * 8 + [_i64, _i64, _f32]),
         ("na1d_layer_norm_backward", [_ptr] * 9 + [_i64, _i64]),
+        ("na1d_layer_norm_backward_rows", [_ptr] * 8 + [_i64, _i64]),
         ("na1d_gelu_forward", [_ptr, _ptr, _i64]),
         ("na1d_gelu_backward", [_ptr] * 5 + [_i64, _i64]),
         ("na1d_column_sums", [_ptr] * 3 + [_i64, _i64]),

@@ -595,6 +595,20 @@ int na1d_layer_norm_backward(void* dx, float* sums, float* scratch, const void* 
     if (int s = check_block(rows, D, 1024, dtype)) return s;
     return cuda_status(na1d::block_ln_bwd(dx, sums, scratch, dy, x, mean, rstd, w, res, (int)rows, (int)D, dtype, (cudaStream_t)stream));
 }
+int na1d_layer_norm_backward_rows(void* dx, float* scratch, const void* dy, const void* x, const float* mean, const float* rstd, const float* w,
+                                  const void* res, int64_t rows, int64_t D, int dtype, void* stream) {
+    if (int s = check_pointers(dx, scratch, dy, x, mean, rstd, w)) return s;
+    if (!aligned16(res)) return NA1D_ERR_MISALIGNED;
+    if (int s = check_block(rows, D, 1024, dtype)) return s;
+    return cuda_status(na1d::block_ln_bwd(dx, nullptr, scratch, dy, x, mean, rstd, w, res, (int)rows, (int)D, dtype, (cudaStream_t)stream));
+}
+int na1d_layer_norm_sums(float* sums0, float* sums1, const float* scratch0, const float* scratch1, int64_t rows, int64_t D, void* stream) {
+    if (int s = check_pointers(sums0, sums1, scratch0, scratch1)) return s;
+    if (int s = check_block(rows, D, 1024, NA1D_BF16)) return s;
+    float* const sums[2] = {sums0, sums1};
+    const float* const part[2] = {scratch0, scratch1};
+    return cuda_status(na1d::block_ln_sums(sums, part, (int)rows, (int)D, (cudaStream_t)stream));
+}
 int na1d_gelu_forward(void* y, const void* x, int64_t n, int dtype, void* stream) {
     if (int s = check_pointers(y, x)) return s;
     if (dtype != NA1D_BF16 && dtype != NA1D_FP16) return NA1D_ERR_BAD_DTYPE;

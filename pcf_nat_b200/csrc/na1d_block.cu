@@ -170,8 +170,14 @@ __device__ __forceinline__ void cta_column_sums(float (&acc)[K][CH][8], float* p
 }
 
 // out[i] = sum over g of part[g * n + i], in a fixed order: 32 warps share the rows of a group of 32 columns (at most 444 rows:
-// 14 independent loads a thread)
-__global__ void __launch_bounds__(1024) partial_sum_kernel(float* __restrict__ out, const float* __restrict__ part, int n, int groups) {
+// 14 independent loads a thread). One launch adds up to two arrays (a block's two LayerNorms: 4 us each, and the gap between launches).
+struct PartialSums {
+    float* out[2];
+    const float* part[2];
+};
+__global__ void __launch_bounds__(1024) partial_sum_kernel(const PartialSums a, int n, int groups) {
+    float* __restrict__ out = a.out[blockIdx.y];
+    const float* __restrict__ part = a.part[blockIdx.y];
     __shared__ float sm[32][33];
     const int lane = threadIdx.x & 31, sub = threadIdx.x >> 5, i = blockIdx.x * 32 + lane;
     float s = 0.f;
@@ -643,7 +649,7 @@ cudaError_t ln_fwd(void* y, void* sum, float* mean, float* rstd, const void* x, 
     return cudaGetLastError();
 }
 cudaError_t add_partials(float* out, const float* part, int n, int groups, cudaStream_t st) {
-    partial_sum_kernel<<<(n + 31) / 32, 1024, 0, st>>>(out, part, n, groups);
+    partial_sum_kernel<<<(n + 31) / 32, 1024, 0, st>>>(PartialSums{{out, nullptr}, {part, nullptr}}, n, groups);
     return cudaGetLastError();
 }
 template <typename E>
@@ -654,7 +660,7 @@ cudaError_t ln_bwd(void* dx, float* sums, float* part, const void* dy, const voi
     switch (ch) { case 1: NA1D_LN(1); break; case 2: NA1D_LN(2); break; case 3: NA1D_LN(3); break; default: NA1D_LN(4); }
 #undef NA1D_LN
     if (cudaError_t e = cudaGetLastError()) return e;
-    return add_partials(sums, part, 3 * D, grid, st);
+    return sums ? add_partials(sums, part, 3 * D, grid, st) : cudaSuccess;
 }
 template <typename E, bool GELU>
 cudaError_t columns(void* dx, float* sums, float* part, const void* dy, const void* x, int rows, int F, cudaStream_t st) {
@@ -684,6 +690,10 @@ cudaError_t block_ln_bwd(void* dx, float* sums, float* part, const void* dy, con
                          const float* w, const void* res, int rows, int D, int dtype, cudaStream_t st) {
     return dtype == 0 ? ln_bwd<__nv_bfloat16>(dx, sums, part, dy, x, mean, rstd, w, res, rows, D, st)
                       : ln_bwd<__half>(dx, sums, part, dy, x, mean, rstd, w, res, rows, D, st);
+}
+cudaError_t block_ln_sums(float* const* sums, const float* const* part, int rows, int D, cudaStream_t st) {
+    partial_sum_kernel<<<dim3((3 * D + 31) / 32, 2), 1024, 0, st>>>(PartialSums{{sums[0], sums[1]}, {part[0], part[1]}}, 3 * D, block_partial_rows(rows));
+    return cudaGetLastError();
 }
 cudaError_t block_gelu_fwd(void* y, const void* x, long long n, int dtype, cudaStream_t st) {
     const long long chunks = n / 8, need = (chunks + 1023) / 1024, most = (long long)device_sm_count() * 8;

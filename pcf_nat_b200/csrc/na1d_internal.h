@@ -113,6 +113,8 @@ cudaError_t block_ln_fwd(void* y, void* sum, float* mean, float* rstd, const voi
                          int rows, int D, float eps, int dtype, cudaStream_t st);
 cudaError_t block_ln_bwd(void* dx, float* sums, float* part, const void* dy, const void* x, const float* mean, const float* rstd,
                          const float* w, const void* res, int rows, int D, int dtype, cudaStream_t st);
+// (sums null: the partial sums stay in `part`, for block_ln_sums, which adds those of two)
+cudaError_t block_ln_sums(float* const* sums, const float* const* part, int rows, int D, cudaStream_t st);
 cudaError_t block_gelu_fwd(void* y, const void* x, long long n, int dtype, cudaStream_t st);
 cudaError_t block_gelu_bwd(void* dx, float* sums, float* part, const void* dy, const void* x, int rows, int F, int dtype, cudaStream_t st);
 cudaError_t block_column_sums(float* sums, float* part, const void* x, int rows, int F, int dtype, cudaStream_t st);

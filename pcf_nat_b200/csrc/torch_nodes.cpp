@@ -515,13 +515,13 @@ void layer_norm(Tensor& y, Tensor& sum, Tensor& st, const Tensor& x, const Tenso
                                   fptr(b), rows, D, (float)eps, code(x), stream()),
           "na1d_layer_norm_forward");
 }
-Tensor layer_norm_backward(Tensor& sums, const Tensor& dy, const Tensor& s, const Tensor& st, const Tensor& w, const Tensor& res, const Tensor& scratch) {
+// its column sums stay in parts, in `part`
+Tensor layer_norm_backward(const Tensor& dy, const Tensor& s, const Tensor& st, const Tensor& w, const Tensor& res, float* part) {
     const int64_t D = s.size(2);
     Tensor ds = at::empty_like(s);
-    sums = empty_f32({3, D}, s);
-    check(na1d_layer_norm_backward(ptr(ds), fptr(sums), fptr(scratch), ptr(dy), ptr(s), fptr(st), fptr(st) + st.size(1), fptr(w), ptr(res),
-                                   s.size(0) * s.size(1), D, code(s), stream()),
-          "na1d_layer_norm_backward");
+    check(na1d_layer_norm_backward_rows(ptr(ds), part, ptr(dy), ptr(s), fptr(st), fptr(st) + st.size(1), fptr(w), ptr(res), s.size(0) * s.size(1), D, code(s),
+                                        stream()),
+          "na1d_layer_norm_backward_rows");
     return ds;
 }
 
@@ -579,7 +579,7 @@ struct NA1dFuse : public torch::autograd::Function<NA1dFuse> {
         const Tensor buf = at::empty({dst[1] + O}, x.options());
         check(na1d_cast_parameters(ptr(buf), src, dst, n, 2, code(x), stream()), "na1d_cast_parameters");
         const Tensor w = buf.as_strided({O, K}, {K, 1}, 0), b = buf.as_strided({O}, {1}, dst[1]);
-        const Tensor cat = at::cat(parts, 2);
+        const Tensor cat = parts.size() == 1 ? x : at::cat(parts, 2);
         const Tensor y = product(cat.view({rows, K}), w, b, false).view({x.size(0), x.size(1), O});
         ctx->save_for_backward({cat, buf});
         ctx->saved_data["D"] = D;
@@ -697,7 +697,9 @@ struct NA1dBlock : public torch::autograd::Function<NA1dBlock> {
             out.insert(out.end(), g.begin() + 2, g.end());
             return out;
         }
-        const Tensor scratch = empty_f32({na1d_block_scratch_floats(rows, D, std::max(F, 3 * D))}, s1);
+        // partial column sums of GELU's and the two norms' passes, one after the other
+        const int64_t room = (na1d_block_scratch_floats(rows, D, std::max(F, 3 * D)) + 3) / 4 * 4;
+        const Tensor scratch = empty_f32({2 * room}, s1);
         const bool one = grads.size() == 1;   // the output is s2 + z, from the MLP kernel
         const Tensor d_s2 = grads[0].defined() ? aligned(grads[0]) : one ? at::zeros_like(s2) : Tensor();
         const Tensor d_z = (one ? d_s2 : grads[1].defined() ? aligned(grads[1]) : at::zeros_like(s2)).view({rows, D});
@@ -720,8 +722,8 @@ struct NA1dBlock : public torch::autograd::Function<NA1dBlock> {
         if (one) d_b1 = mlp.b[0];
         d_f.reset();
         g.reset();
-        Tensor sums2, sums1;
-        const Tensor d_y = layer_norm_backward(sums2, d_h, s2, st2, n2w, d_s2, scratch);   // also the residual stream's gradient
+        const Tensor sums = empty_f32({2, 3, D}, s1), sums1 = sums.select(0, 0), sums2 = sums.select(0, 1);
+        const Tensor d_y = layer_norm_backward(d_h, s2, st2, n2w, d_s2, fptr(scratch) + room);   // also the residual stream's gradient
         // attention branch
         const Tensor dy2 = d_y.view({rows, D});
         Tensor d_qkv = at::empty_like(qkv), d_rpb;
@@ -729,7 +731,8 @@ struct NA1dBlock : public torch::autograd::Function<NA1dBlock> {
         packed_backward(d_qkv, d_rpb, product(dy2, w.t[2], Tensor(), true), qkv, lse, rpb, vl, c);
         const Tensor dq2 = d_qkv.view({rows, 3 * D});
         const ParameterGrads att({dq2, dy2}, {h1.view({rows, D}), o.view({rows, D})}, {need(0), need(2)}, {need(1), false}, at::kFloat);
-        const Tensor d_x = layer_norm_backward(sums1, product(dq2, w.t[0], Tensor(), true), s1, st1, n1w, d_y, scratch);
+        const Tensor d_x = layer_norm_backward(product(dq2, w.t[0], Tensor(), true), s1, st1, n1w, d_y, fptr(scratch));
+        check(na1d_layer_norm_sums(fptr(sums1), fptr(sums2), fptr(scratch), fptr(scratch) + room, rows, D, stream()), "na1d_layer_norm_sums");
         const Tensor none;
         return {d_x, has_dx ? d_x : none, none, none, none, none, none, none, none, att.w[0], att.b[0], att.w[1], sums2.select(0, 2), mlp.w[0], d_b1, mlp.w[1],
                 mlp.b[1],

@@ -77,8 +77,14 @@ class AttentiveStatsPool(nn.Module):
     def forward(self, x):
         # (as a matrix where the rows are slices of wider ones, which a GEMM reads in place)
         in_place = x.dim() == 3 and not x.is_contiguous() and _plain_linear(self.a)
-        h = self.a(x.flatten(0, 1)).view(x.shape[0], x.shape[1], -1) if in_place else self.a(x)
-        logits = self.b(torch.tanh(h))
+        y = None if in_place else block.fuse(self.a, [x])
+        if y is None:
+            h = self.a(x.flatten(0, 1)).view(x.shape[0], x.shape[1], -1) if in_place else self.a(x)
+        else:
+            h, (x,) = y
+        h = torch.tanh(h)
+        y = block.fuse(self.b, [h])
+        logits = self.b(h) if y is None else y[0]
         out = block.stats_pool(logits, x, 1e-5)
         return block.weighted_stats(logits, x, 1e-5) if out is None else out
 

@@ -62,6 +62,25 @@ def _exact(lin, xs, stages):
     return torch.autograd.grad(loss, ys + [p for l in ps for p in l])
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_one_part_that_is_read_again(dtype):
+    """As in the pooling: a projection of one tensor, which what follows reads too."""
+    from pcf_nat_b200 import block
+    torch.manual_seed(0)
+    lin = torch.nn.Linear(384, 128).cuda()
+    x = torch.randn(3, 41, 384, device="cuda").to(dtype).requires_grad_()
+    out = []
+    for node in (True, False):
+        with torch.autocast("cuda", dtype=dtype):
+            y, again = block.fuse(lin, [x]) if node else (lin(x), [x])
+        assert y.dtype == dtype and torch.equal(again[0], x)
+        loss = (y.float().sin().sum(-1, keepdim=True) * again[0].float().cos()).sum()
+        out.append([y.detach()] + list(torch.autograd.grad(loss, [x] + list(lin.parameters()))))
+    u = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    for a, b in zip(*out):
+        assert a.dtype == b.dtype and float((a.double() - b.double()).norm()) <= 4 * u * float(b.double().norm()) + 1e-5
+
+
 def test_left_to_the_operations():
     from pcf_nat_b200 import block
     lin = torch.nn.Linear(128, 64).cuda()
