@@ -243,7 +243,8 @@ int na1d_gelu_backward(void* dx, float* sums, float* scratch, const void* dy, co
 int na1d_column_sums(float* sums, float* scratch, const void* x, int64_t rows, int64_t F, int dtype, void* stream);
 /* A transformer block's MLP in one kernel: out = s + GELU(h w1^T + b1) w2^T + b2 (models/PCF_NATransformer.py:228-303). s, h, out
  * (rows, D), w1 (F, D), w2 (D, F) 16-bit, biases fp32; out has rows of ld >= D elements (a multiple of 8); D = 256, F a multiple of
- * 128 up to 1280. f (rows, F), 16-bit and 32-byte aligned, or NULL: takes the hidden layer before GELU, for a backward pass.
+ * 128 up to 1280. f (rows, F), 16-bit, or NULL: takes the hidden layer before GELU, for a backward pass. s and f are 32-byte
+ * aligned.
  * `scratch`: na1d_mlp_scratch_floats floats (0: may be NULL; -1: not a size that this takes). */
 int64_t na1d_mlp_scratch_floats(int64_t rows, int64_t D, int64_t F);
 int na1d_mlp_forward(void* out, int64_t ld, void* f, const void* s, const void* h, const void* w1, const float* b1, const void* w2, const float* b2,

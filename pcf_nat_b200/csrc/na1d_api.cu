@@ -656,7 +656,7 @@ int64_t na1d_mlp_scratch_floats(int64_t rows, int64_t D, int64_t F) {
 int na1d_mlp_forward(void* out, int64_t ld, void* f, const void* s, const void* h, const void* w1, const float* b1, const void* w2, const float* b2, float* scratch,
                      int64_t rows, int64_t D, int64_t F, int dtype, void* stream) {
     if (int e = check_pointers(out, s, h, w1, b1, w2, b2)) return e;
-    if (((uintptr_t)f & 31) || !aligned16(scratch)) return NA1D_ERR_MISALIGNED;
+    if ((((uintptr_t)f | (uintptr_t)s) & 31) || !aligned16(scratch)) return NA1D_ERR_MISALIGNED;
     if (int e = check_block(rows, F, 1 << 20, dtype)) return e;
     if (!na1d::mlp_supports(D, F) || ld < D || ld % 8 != 0 || ld > (1ll << 40) / rows) return NA1D_ERR_BAD_SHAPE;
     if (!scratch && na1d::mlp_scratch_floats(rows, F)) return NA1D_ERR_NULL_POINTER;

@@ -2,16 +2,17 @@
 // multiple of 128.
 //
 // As separate passes (product, GELU, product, residual in the next LayerNorm) the hidden layer, four times as wide as the rows, crosses
-// HBM four times: 153600 rows took 106 + 126 + 94 us where the products themselves need 95; 148 + 5 us here (76800: 85 + 4, 9600: 32).
+// HBM four times: 153600 rows took 106 + 126 + 94 us where the products themselves need 95; 133 + 5 us here (76800: 73 + 4, 9600: 25).
 // For a backward pass the layer before GELU is stored, a sector of each row at a time straight from the lanes that hold it: 38400 rows
-// 62 + 4 us instead of 78 (70 + 4 through a stage in shared memory).
+// 51 + 4 us instead of 78.
 // A pair of CTAs keeps 256 rows on chip: the rows as an operand in shared memory, the hidden layer in pieces of 128 columns in tensor
 // memory, where GELU turns the first product's result into the second one's left operand in place.
 //   warps 0-15   GELU: 32 tensor-memory lanes and a quarter of a piece's columns each
-//   warps 16-23  the result: out of tensor memory into registers at once (the next tile's second product waits for that), residual and
-//                store at leisure
-//   warp 24      loads: the rows of the next tile, weight pieces (16 KB a CTA: half of the output columns and of the contraction; a ring
-//                of four)
+//   warps 16-23  the result: out of tensor memory at once (the next tile's second product waits for that) into registers and shared memory,
+//                as much as fits without local memory (L1 has next to no room here: what the compiler moved there made the whole kernel wait,
+//                148 us for 153600 rows), then residual and store at leisure, a row per lane
+//   warp 24      loads: the rows of the next tile, the residual's into L2, weight pieces (16 KB a CTA: half of the output columns and
+//                of the contraction; a ring of four)
 //   warp 25      issues the products (leader): piece j + 1 of the hidden layer before the second product of piece j
 // Bound: tensor pipe (1024 + 1024 cycles a piece), GELU (FMA pipe 1150, special functions 1024), 64 KB of weights a piece from L2.
 // Every role's code is a short loop. (With the LayerNorm in it too -- eight warps, rows through registers -- the kernel took 245 us for
@@ -29,7 +30,7 @@ constexpr int kThreads = (kGeluWarps + kResultWarps + 4) * 32;
 // registers per thread after the warp groups have traded: 512 x 64 + 256 x 104 + 128 x 32 <= 896 x 72
 constexpr int kLaunchRegs = 72, kGeluRegs = 64, kResultRegs = 104, kOtherRegs = 32;
 constexpr int kSlots = 4;
-constexpr int kStage = 2048;                      // per warp, to turn rows per lane into rows of adjacent lanes: 32 rows x 64 bytes
+constexpr int kStage = 6 * 32 * 16;               // per result warp: 48 columns of its 32 rows
 constexpr int kBiases = (kMostF + kD) * 4;
 constexpr int kSmem = 2 * kRowsBytes + kSlots * kSlotBytes + kResultWarps * kStage + kBiases + 1024;
 
@@ -39,13 +40,14 @@ struct Barriers {
     int abort;
 };
 
-struct Maps { CUtensorMap h, w1, w2; };
+struct Maps { CUtensorMap h, s, w1, w2; };
 template <typename E> struct Args {
     const E* s;                        // residual stream
     const float *b1, *b2;
     E* out;                            // rows ld elements apart
     long long ld;
     E* f;                              // (rows, F): the hidden layer before GELU, for a backward pass
+    bool sectors;                      // rows of out start on 32 bytes
     float* part;                       // partial results of the split tiles
 };
 
@@ -69,8 +71,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     extern __shared__ uint8_t raw[];
     uint8_t* rows_smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(raw) + 1023) & ~(uintptr_t)1023);
     uint8_t* ring = rows_smem + 2 * kRowsBytes;
-    uint8_t* stages = ring + kSlots * kSlotBytes;
-    float* biases = reinterpret_cast<float*>(stages + kResultWarps * kStage);   // b2, b1
+    uint4* stages = reinterpret_cast<uint4*>(ring + kSlots * kSlotBytes);
+    float* biases = reinterpret_cast<float*>(stages + kResultWarps * (kStage / 16));   // b2, b1
     __shared__ Barriers bar;
     const int warp = ptx::warp_index(), lane = threadIdx.x & 31;
     const uint32_t rank = pair::cta_rank();
@@ -80,8 +82,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 
     if (warp == kGeluWarps + kResultWarps) {
         if (lane < kSlots) { ptx::mbar_init(&bar.full[lane], 1); ptx::mbar_init(&bar.empty[lane], 1); }
-        else if (lane < kSlots + 2) { ptx::mbar_init(&bar.s_full[lane - kSlots], 1); ptx::mbar_init(&bar.g_ready[lane - kSlots], 2 * kGeluWarps); }
-        else if (lane < kSlots + 4) { ptx::mbar_init(&bar.a_full[lane - kSlots - 2], 1); ptx::mbar_init(&bar.a_free[lane - kSlots - 2], 1); }
+        else if (lane >= 16 && lane < 18) { ptx::mbar_init(&bar.s_full[lane - 16], 1); ptx::mbar_init(&bar.g_ready[lane - 16], 2 * kGeluWarps); }
+        else if (lane >= 18 && lane < 20) { ptx::mbar_init(&bar.a_full[lane - 18], 1); ptx::mbar_init(&bar.a_free[lane - 18], 1); }
         else if (lane == 9) { ptx::mbar_init(&bar.o_full, 1); ptx::mbar_init(&bar.o_free, 2 * kResultWarps); }
         else if (lane == 10) bar.abort = 0;
         else if (lane == 11) ptx::prefetch_tensormap(&maps.w1);
@@ -158,7 +160,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     } else if (warp < kGeluWarps + kResultWarps) {
         ptx::warpgroup_regs_grow<kResultRegs>();
         const int w = warp - kGeluWarps, q = warp & 3, half = w >> 2;
-        uint8_t* stage = stages + w * kStage;
+        uint4* stage = stages + w * (kStage / 16) + lane;
         const uint32_t o_free = pair::in_leader(&bar.o_free), o = tmem + ((uint32_t)(q * 32) << 16) + kAcc + half * 128;
         int it = 0;
         for (int i = first; i < plan.items; i += step, ++it) {
@@ -166,24 +168,24 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
             const int row0 = t.tile * 256 + (int)rank * 128 + q * 32;
             if (!ptx::mbar_wait_relaxed(&bar.o_full, it & 1) || *abort_flag) NA1D_MLP_FAIL(2)
             ptx::tc_fence_after_sync();
-            uint4 z[16];   // 128 columns of this lane's row
-            auto keep = [&](int n, float* d) {
-                const float4* b2 = reinterpret_cast<const float4*>(biases + half * 128 + n * 32);
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    const float4 ba = b2[2 * k], bb = b2[2 * k + 1];
-                    float* v = d + 8 * k;
-                    v[0] += ba.x; v[1] += ba.y; v[2] += ba.z; v[3] += ba.w; v[4] += bb.x; v[5] += bb.y; v[6] += bb.z; v[7] += bb.w;
-                    z[n * 4 + k] = Cvt<E>::pack(v);
-                }
-            };
+            // 128 columns of this lane's row: the first 48 into this lane's own place in shared memory, the others into registers (all of them
+            // would not fit there: what the compiler then kept in local memory made this drain take 2800 cycles)
+            uint4 z[10];
             if (t.parts == 1) {
 #pragma unroll
-                for (int n = 0; n < 4; ++n) {
-                    float d[32];
-                    pair::tmem_ld32(o + n * 32, d);
+                for (int n = 0; n < 8; ++n) {
+                    float d[16];
+                    pair::tmem_ld16(o + n * 16, d);
                     ptx::tmem_ld_wait();
-                    keep(n, d);
+#pragma unroll
+                    for (int k = 0; k < 2; ++k) {
+                        const float4* b2 = reinterpret_cast<const float4*>(biases + half * 128 + n * 16 + k * 8);
+                        const float4 ba = b2[0], bb = b2[1];
+                        float* v = d + 8 * k;
+                        v[0] += ba.x; v[1] += ba.y; v[2] += ba.z; v[3] += ba.w; v[4] += bb.x; v[5] += bb.y; v[6] += bb.z; v[7] += bb.w;
+                        if (n < 3) stage[(2 * n + k) * 32] = Cvt<E>::pack(v);
+                        else z[2 * (n - 3) + k] = Cvt<E>::pack(v);
+                    }
                 }
                 ptx::tc_fence_before_sync();
                 __syncwarp();
@@ -203,27 +205,25 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                 if (lane == 0) pair::arrive_cluster(o_free);
                 continue;
             }
-#pragma unroll
-            for (int n = 0; n < 4; ++n) {
-                const int col = half * 128 + n * 32 + (lane & 3) * 8;
-                uint4 res[4];
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    const int r = row0 + k * 8 + (lane >> 2);
-                    res[k] = make_uint4(0u, 0u, 0u, 0u);
-                    if (r < plan.rows) res[k] = load_row(g.s + (size_t)r * kD + col);
+            const int row = row0 + lane;
+            const bool live = row < plan.rows;
+            const E* res = g.s + (size_t)row * kD + half * 128;
+            E* dst = g.out + (size_t)row * g.ld + half * 128;
+            auto leave = [&](int n, const uint4& x, const uint4& y) {
+                uint32_t v[8] = {};
+                if (live) load_sector(res + n * 16, v);
+                const uint4 a = add_rows<E>(make_uint4(v[0], v[1], v[2], v[3]), x), b = add_rows<E>(make_uint4(v[4], v[5], v[6], v[7]), y);
+                const uint32_t sum[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+                if (live && g.sectors) store_sector(dst + n * 16, sum);
+                else if (live) {
+                    *reinterpret_cast<uint4*>(dst + n * 16) = a;
+                    *reinterpret_cast<uint4*>(dst + n * 16 + 8) = b;
                 }
-                __syncwarp();
+            };
 #pragma unroll
-                for (int k = 0; k < 4; ++k) *reinterpret_cast<uint4*>(stage + stage_at(lane, k)) = z[n * 4 + k];
-                __syncwarp();
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    const int r = k * 8 + (lane >> 2);
-                    const uint4 v = add_rows<E>(res[k], *reinterpret_cast<const uint4*>(stage + stage_at(r, lane & 3)));
-                    if (row0 + r < plan.rows) *reinterpret_cast<uint4*>(g.out + (size_t)(row0 + r) * g.ld + col) = v;
-                }
-            }
+            for (int n = 3; n < 8; ++n) leave(n, z[2 * (n - 3)], z[2 * (n - 3) + 1]);
+#pragma unroll 1
+            for (int n = 0; n < 3; ++n) leave(n, stage[2 * n * 32], stage[(2 * n + 1) * 32]);
         }
     } else {
         ptx::warpgroup_regs_shrink<kOtherRegs>();
@@ -258,6 +258,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                     if (ok && before >= 0) load(true, before);
                     before = c;
                     if (ok && c == min(t.c0 + 1, t.c1 - 1)) rows(i + step, it + 1);
+                    if (t.parts == 1 && c == max(t.c1 - 4, t.c0)) pair::prefetch_3d(&maps.s, 0, t.tile * 256 + (int)rank * 128, 0);
                 }
             }
             if (ok && before >= 0) load(true, before);
@@ -376,10 +377,10 @@ cudaError_t forward(void* out, int64_t ld, void* f, const void* s, const void* h
     Maps maps;
     const int64_t dh[3] = {64, rows, kD / 64}, d1[3] = {64, F, kD / 64}, s1[2] = {kD, 64}, d2[3] = {64, kD, F / 64}, s2[2] = {F, 64};
     const int xh[3] = {64, 128, kD / 64}, x1[3] = {64, 64, 2}, x2[3] = {64, 128, 1};
-    if (!make_matrix_map(&maps.h, h, dtype, 3, dh, s1, xh) || !make_matrix_map(&maps.w1, w1, dtype, 3, d1, s1, x1) ||
+    if (!make_matrix_map(&maps.h, h, dtype, 3, dh, s1, xh) || !make_matrix_map(&maps.s, s, dtype, 3, dh, s1, xh) || !make_matrix_map(&maps.w1, w1, dtype, 3, d1, s1, x1) ||
         !make_matrix_map(&maps.w2, w2, dtype, 3, d2, s2, x2))
         return cudaErrorInvalidValue;
-    const Args<E> a = {(const E*)s, b1, b2, (E*)out, ld, (E*)f, scratch};
+    const Args<E> a = {(const E*)s, b1, b2, (E*)out, ld, (E*)f, ld % 16 == 0 && ((uintptr_t)out & 31) == 0, scratch};
     return f ? run<E, true>(maps, plan, a, st) : run<E, false>(maps, plan, a, st);
 }
 
