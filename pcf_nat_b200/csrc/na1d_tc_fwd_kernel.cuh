@@ -12,7 +12,7 @@
 //             (na1d_tensorcore/bf16_ana1d_kernel.cu:99-112).
 //   warps 5,6: MMA issuers -- S = Q.K^T (C/16 steps, M=128, N=KT) into TMEM columns [0,KT);
 //             O = P.V (KT/16 steps, N=C) with P read from TMEM and V as an MN-major operand straight
-//             from the TMA tile. A tcgen05.mma costs its issuing thread ~120 cycles whatever its size, so
+//             from the TMA tile. A tcgen05.mma costs its issuing (elected) thread ~66 cycles whatever its size, so
 //             the key steps of P.V are split between two issuers with an accumulator each (even / odd
 //             steps); the epilogue adds the two.
 //   warps0-3: softmax on the band only. Warp w owns rows 32w..32w+31 as two 16-row accumulator

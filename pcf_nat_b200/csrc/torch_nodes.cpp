@@ -404,9 +404,9 @@ OptTensor packed(const Tensor& qkv, int64_t heads, int64_t win, int64_t left, in
 }
 
 // An output gradient as the row and column kernels read it: dense, on a 16-byte boundary (a view into another tensor need not be).
-Tensor aligned(const Tensor& g) {
+Tensor aligned(const Tensor& g, uintptr_t bytes = 16) {
     const Tensor c = g.contiguous();
-    return (reinterpret_cast<uintptr_t>(c.data_ptr()) & 15u) ? c.clone() : c;
+    return (reinterpret_cast<uintptr_t>(c.data_ptr()) & (bytes - 1)) ? c.clone() : c;
 }
 
 // A backward pass works in the types of its forward, also where it is called under autocast (to another type, the library products
@@ -476,7 +476,7 @@ constexpr int64_t kSlot = 64;   // elements: 128-byte slots of the packed 16-bit
 struct Projections {
     Tensor buf, t[kProj];
     void views(at::IntArrayRef (&shapes)[kProj]) {
-        int64_t off = 0;
+        int64_t off = buf.storage_offset();   // (what a saved-tensor hook gives back may lie inside another tensor)
         for (int i = 0; i < kProj; ++i) {
             const int64_t n = c10::multiply_integers(shapes[i]);
             t[i] = shapes[i].size() == 2 ? buf.as_strided(shapes[i], {shapes[i][1], 1}, off) : buf.as_strided(shapes[i], {1}, off);
@@ -591,11 +591,11 @@ struct NA1dFuse : public torch::autograd::Function<NA1dFuse> {
     }
     static variable_list backward(AutogradContext* ctx, variable_list grads) {
         const variable_list s = ctx->get_saved_variables();
-        const Tensor &cat = s[0], &buf = s[1];
+        const Tensor cat = aligned(s[0]), buf = aligned(s[1]);
         const int64_t D = ctx->saved_data["D"].toInt(), O = ctx->saved_data["O"].toInt(), K = cat.size(2), rows = cat.size(0) * cat.size(1), parts = K / D;
         const c10::cuda::CUDAGuard guard(cat.device());
         const NoAutocast off;
-        const Tensor w = buf.as_strided({O, K}, {K, 1}, 0), b = buf.as_strided({O}, {1}, (O * K + kSlot - 1) / kSlot * kSlot);
+        const Tensor w = buf.narrow(0, 0, O * K).view({O, K}), b = buf.narrow(0, (O * K + kSlot - 1) / kSlot * kSlot, O);
         if (at::GradMode::is_enabled()) {
             variable_list in = {stand_in(w.to(at::kFloat), 0), stand_in(b.to(at::kFloat), 1)}, out = {Tensor()};
             for (int64_t i = 0; i < parts; ++i) in.push_back(stand_in(cat.narrow(2, i * D, D), 2 + i));
@@ -674,8 +674,10 @@ struct NA1dBlock : public torch::autograd::Function<NA1dBlock> {
     }
     static variable_list backward(AutogradContext* ctx, variable_list grads) {
         const variable_list s = ctx->get_saved_variables();
-        const Tensor &s1 = s[0], &st1 = s[1], &h1 = s[2], &qkv = s[3], &lse = s[4], &o = s[5], &s2 = s[6], &st2 = s[7], &h2 = s[8], &f = s[9], &buf = s[11], &n1w = s[12], &n2w = s[13], &rpb = s[14], &vl = s[15];
-        Tensor g = s[10];
+        const Tensor &s1 = s[0], &st1 = s[1], &qkv = s[3], &lse = s[4], &s2 = s[6], &st2 = s[7], &n1w = s[12], &n2w = s[13], &rpb = s[14], &vl = s[15];
+        // (as the products read them, wherever a saved-tensor hook has put them; f by whole sectors)
+        const Tensor h1 = aligned(s[2]), o = aligned(s[5]), h2 = aligned(s[8]), buf = aligned(s[11]), f = aligned(s[9], 32);
+        Tensor g = s[10].defined() ? aligned(s[10]) : s[10];
         auto& data = ctx->saved_data;
         const Packed c(qkv, data["heads"].toInt(), data["win"].toInt(), data["left"].toInt(), 1, data["scale"].toDouble());
         const c10::cuda::CUDAGuard guard(s1.device());

@@ -99,3 +99,33 @@ def test_left_to_the_operations():
     assert block.fuse(lin, [x, x]) is None      # without autocast
     with torch.autocast("cuda", dtype=torch.float16):
         assert block.fuse(lin, [x, x]) is None
+
+
+@pytest.mark.parametrize("D", [64, 256])
+def test_saved_tensors_may_come_back_inside_others(D):
+    """What the nodes save may be given back as parts of larger tensors, 16 bytes off their start: the gradients stay the same bits."""
+    from pcf_nat_b200 import block
+    from pcf_nat_b200.model import NABlock
+    torch.manual_seed(0)
+    st = torch.nn.ModuleList(NABlock(40, D, 4, 7, 4, "fused") for _ in range(2)).cuda()
+    lin = torch.nn.Linear(2 * D, D).cuda()
+    x = torch.randn(2, 40, D, device="cuda").to(torch.bfloat16).requires_grad_()
+
+    def pack(t):
+        if not t.is_cuda or t.numel() == 0:
+            return t
+        room = torch.full((t.numel() + 64,), float("nan") if t.is_floating_point() else 0, device=t.device, dtype=t.dtype)
+        return room[8:8 + t.numel()].view(t.shape).copy_(t.detach())
+
+    def gradients():
+        with torch.autocast("cuda", dtype=torch.bfloat16):
+            y = block.run_blocks(st, x, None)
+            z, (a, b) = block.fuse(lin, [x, y])
+        return torch.autograd.grad((z.float().sin() + a.float() + b.float().cos()).sum(),
+                                   [x] + list(lin.parameters()) + [p for n, p in st.named_parameters() if "relative" not in n])
+
+    want = gradients()
+    with torch.autograd.graph.saved_tensors_hooks(pack, lambda t: t):
+        got = gradients()
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
