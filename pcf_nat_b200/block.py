@@ -94,7 +94,11 @@ def run_blocks(blocks, x, valid, out=None, training=None):
             return None
         a = blk.attn
         C = D // a.num_heads
-        if not ops.packed_supported(a.num_heads, T, C, a.win_size, a.left, 1, dt):
+        # (the kernels that take dense rows of heads stand in where those on the packed projection do not take the shape; larger ones are left
+        # to the modules, which refuse what no kernel takes)
+        if not ops.packed_supported(a.num_heads, T, C, a.win_size, a.left, 1, dt) and (
+                C not in (8, 16, 24, 32, 48, 64, 96, 128) or a.win_size > 128 or a.num_heads * a.win_size > 4096 or B > 65535 or
+                B * a.num_heads * T * a.win_size >= 2 ** 31):
             return None
         plan.append((ps, (a.num_heads, a.win_size, a.left, float(a.scale)), (blk.norm1.eps, blk.norm2.eps)))
     x, dx = x.contiguous(), None

@@ -442,6 +442,46 @@ variable_list inner_gradients(const variable_list& outputs, const variable_list&
     return result;
 }
 
+// Shapes that the strided entry points do not take (a head size outside theirs, no shared memory left for the bias gradient): the
+// heads are split and merged by one copy each around the dense ones.
+bool takes_packed(const Packed& c, const Tensor& like, bool backward = true) {
+    return na1d_fused_strided_supported(c.H, c.T, c.C, c.win, c.left, c.dil, code(like), 1, backward) == 1;
+}
+Tensor heads_moved(const Tensor& in, const Packed& c, int64_t parts, bool to_dense) {
+    Tensor out = to_dense ? at::empty({parts, c.B * c.H, c.T, c.C}, in.options()) : at::empty({c.B, c.T, parts * c.H * c.C}, in.options());
+    check(na1d_permute_heads(ptr(out), ptr(in), c.B, c.T, parts, c.H, c.C, to_dense, stream()), "na1d_permute_heads");
+    return out;
+}
+Cfg dense_cfg(const Packed& c) { return Cfg{c.B * c.H, c.T, c.C, c.H, c.win, c.left, c.dil, c.scale, 0.0, 0}; }
+// the attention on a packed qkv by either route; o_dense, and the split qkv in the place of the packed one: what the dense route's backward reads
+void attention_forward(Tensor& o, Tensor& o_dense, Tensor& qkv, const Tensor& lse, const Tensor& r, const Tensor& vl, const Packed& c, bool packed) {
+    if (packed) {
+        o = at::empty({c.B, c.T, c.H * c.C}, qkv.options());
+        packed_forward(o, lse, qkv, r, vl, c);
+        return;
+    }
+    qkv = heads_moved(qkv, c, 3, true);
+    o_dense = at::empty({c.B * c.H, c.T, c.C}, qkv.options());
+    op_forward(o_dense, lse, qkv.select(0, 0), qkv.select(0, 1), qkv.select(0, 2), r, vl, dense_cfg(c));
+    o = heads_moved(o_dense, c, 1, false);
+}
+// gradient of the packed qkv; d_o (rows, D)
+Tensor attention_backward(const Tensor& d_rpb, const Tensor& d_o, const Tensor& qkv, const Tensor& o_dense, const Tensor& lse, const Tensor& r, const Tensor& vl,
+                          const Packed& c) {
+    Tensor d_qkv = at::empty_like(qkv);
+    if (!o_dense.defined()) {
+        packed_backward(d_qkv, d_rpb, d_o, qkv, lse, r, vl, c);
+        return d_qkv;
+    }
+    const Tensor moved = heads_moved(d_o, c, 1, true), delta = empty_f32({c.B * c.H, c.T}, qkv);
+    auto part = [](const Tensor& t, int i) { return ptr(t.select(0, i)); };
+    check(na1d_fused_backward(part(d_qkv, 0), part(d_qkv, 1), part(d_qkv, 2), fptr(d_rpb), ptr(moved), part(qkv, 0), part(qkv, 1), part(qkv, 2), ptr(o_dense), fptr(lse),
+                              fptr(r), static_cast<int32_t*>(ptr(vl)), fptr(delta), c.B * c.H, c.H, c.T, c.C, c.win, c.left, c.dil, (float)c.scale, code(qkv),
+                              stream()),
+          "na1d_fused_backward");
+    return heads_moved(d_qkv, c, 3, false);
+}
+
 // ---------------------------------------------------------------- the transformer block
 // Parameter gradients of up to two projections in one launch: d_w = dy^T x and d_b = column sums of dy, of `type` from fp32 sums.
 // dy (rows, M), x (rows, N); what is not wanted stays undefined.
@@ -501,7 +541,7 @@ struct Projections {
 };
 
 struct BlockState {   // what the backward needs
-    Tensor s1, st1, h1, qkv, lse, o, s2, st2, h2, f, g, buf;
+    Tensor s1, st1, h1, qkv, lse, o, s2, st2, h2, f, g, buf, o_dense;
 };
 // one row of padding keeps both halves of the statistics 16-byte aligned
 inline Tensor row_stats(int64_t rows, const Tensor& like) { return empty_f32({2, (rows + 3) / 4 * 4}, like); }
@@ -537,9 +577,8 @@ std::pair<Tensor, Tensor> block_forward(const Tensor& x, const Tensor& dx, const
     w.cast(p, x);
     layer_norm(st.h1, st.s1, st.st1, x, dx, p[8], p[9], eps1, stats);
     st.qkv = product(st.h1.view({rows, D}), w.t[0], w.t[1], false).view({c.B, c.T, 3 * D});
-    st.o = at::empty({c.B, c.T, D}, x.options());
     if (stats) st.lse = empty_f32({c.B * c.H, c.T}, x);
-    packed_forward(st.o, st.lse, st.qkv, p[12], vl, c);
+    attention_forward(st.o, st.o_dense, st.qkv, st.lse, p[12], vl, c, takes_packed(c, x, stats));
     const Tensor y = product(st.o.view({rows, D}), w.t[2], w.t[3], false).view({c.B, c.T, D});
     layer_norm(st.h2, st.s2, st.st2, st.s1, y, p[10], p[11], eps2, stats);
     const int64_t F = w.t[4].size(0), floats = na1d_mlp_scratch_floats(rows, D, F);
@@ -648,7 +687,7 @@ struct NA1dBlock : public torch::autograd::Function<NA1dBlock> {
         const Packed c(x.size(0), x.size(1), x.size(2), heads, win, left, 1, scale);
         BlockState st;
         auto out = block_forward(x, dx ? *dx : Tensor(), vl ? *vl : Tensor(), c, eps1, eps2, p, &st);
-        ctx->save_for_backward({st.s1, st.st1, st.h1, st.qkv, st.lse, st.o, st.s2, st.st2, st.h2, st.f, st.g, st.buf, p8, p10, p12, vl ? *vl : Tensor(), p9, p11});
+        ctx->save_for_backward({st.s1, st.st1, st.h1, st.qkv, st.lse, st.o, st.s2, st.st2, st.h2, st.f, st.g, st.buf, p8, p10, p12, vl ? *vl : Tensor(), p9, p11, st.o_dense});
         auto& d = ctx->saved_data;
         d["heads"] = heads; d["win"] = win; d["left"] = left; d["scale"] = scale; d["dx"] = dx.has_value(); d["eps1"] = eps1; d["eps2"] = eps2;
         return out.second.defined() ? variable_list{out.first, out.second} : variable_list{out.first};
@@ -667,7 +706,16 @@ struct NA1dBlock : public torch::autograd::Function<NA1dBlock> {
         auto linear = [&](const Tensor& x, int i) { return at::linear(x, p[i].to(half), p[i + 1].to(half)); };
         auto norm = [&](const Tensor& x, int i, double eps) { return at::layer_norm(x.to(at::kFloat), {D}, p[i], p[i + 1], eps).to(half); };
         const Tensor x = has_dx ? in[0] + in[1] : in[0];
-        const Tensor o = NA1dFusedPacked::apply(linear(norm(x, 8, eps1), 0), p[12], vl.defined() ? OptTensor(vl) : OptTensor(), c.H, c.win, c.left, 1, c.scale);
+        const OptTensor valid = vl.defined() ? OptTensor(vl) : OptTensor();
+        const Tensor qkv = linear(norm(x, 8, eps1), 0);
+        Tensor o;
+        if (!s[18].defined()) {
+            o = NA1dFusedPacked::apply(qkv, p[12], valid, c.H, c.win, c.left, 1, c.scale);
+        } else {
+            const Tensor q = qkv.view({c.B, c.T, 3, c.H, c.C}).permute({2, 0, 3, 1, 4}).contiguous().view({3, c.B * c.H, c.T, c.C});
+            o = NA1dFused::apply(q.select(0, 0), q.select(0, 1), q.select(0, 2), OptTensor(p[12]), valid, c.H, c.win, c.left, 1, c.scale, 0.0, (int64_t)0)
+                    .view({c.B, c.H, c.T, c.C}).transpose(1, 2).reshape({c.B, c.T, D});
+        }
         const Tensor s2 = x + linear(o, 2);
         const Tensor z = linear(at::gelu(linear(norm(s2, 10, eps2), 4)), 6);
         return inner_gradients(grads.size() == 1 ? variable_list{s2 + z} : variable_list{s2, z}, in, grads);
@@ -679,7 +727,7 @@ struct NA1dBlock : public torch::autograd::Function<NA1dBlock> {
         const Tensor h1 = aligned(s[2]), o = aligned(s[5]), h2 = aligned(s[8]), buf = aligned(s[11]), f = aligned(s[9], 32);
         Tensor g = s[10].defined() ? aligned(s[10]) : s[10];
         auto& data = ctx->saved_data;
-        const Packed c(qkv, data["heads"].toInt(), data["win"].toInt(), data["left"].toInt(), 1, data["scale"].toDouble());
+        const Packed c(s1.size(0), s1.size(1), s1.size(2), data["heads"].toInt(), data["win"].toInt(), data["left"].toInt(), 1, data["scale"].toDouble());
         const c10::cuda::CUDAGuard guard(s1.device());
         const NoAutocast off;
         const bool has_dx = data["dx"].toBool();
@@ -728,9 +776,9 @@ struct NA1dBlock : public torch::autograd::Function<NA1dBlock> {
         const Tensor d_y = layer_norm_backward(d_h, s2, st2, n2w, d_s2, fptr(scratch) + room);   // also the residual stream's gradient
         // attention branch
         const Tensor dy2 = d_y.view({rows, D});
-        Tensor d_qkv = at::empty_like(qkv), d_rpb;
+        Tensor d_rpb;
         if (need(12)) d_rpb = zeros_f32(rpb.sizes(), s1);
-        packed_backward(d_qkv, d_rpb, product(dy2, w.t[2], Tensor(), true), qkv, lse, rpb, vl, c);
+        const Tensor d_qkv = attention_backward(d_rpb, product(dy2, w.t[2], Tensor(), true), qkv, s[18], lse, rpb, vl, c);
         const Tensor dq2 = d_qkv.view({rows, 3 * D});
         const ParameterGrads att({dq2, dy2}, {h1.view({rows, D}), o.view({rows, D})}, {need(0), need(2)}, {need(1), false}, at::kFloat);
         const Tensor d_x = layer_norm_backward(product(dq2, w.t[0], Tensor(), true), s1, st1, n1w, d_y, fptr(scratch));
@@ -826,17 +874,6 @@ struct LayerGrads {
         }
     }
 };
-// Shapes that the strided entry points do not take (a head size outside theirs, no shared memory left for the bias gradient): the
-// heads are split and merged by one copy each around the dense ones.
-bool takes_packed(const Packed& c, const Tensor& like) {
-    return na1d_fused_strided_supported(c.H, c.T, c.C, c.win, c.left, c.dil, code(like), 1, 1) == 1;
-}
-Tensor heads_moved(const Tensor& in, const Packed& c, int64_t parts, bool to_dense) {
-    Tensor out = to_dense ? at::empty({parts, c.B * c.H, c.T, c.C}, in.options()) : at::empty({c.B, c.T, parts * c.H * c.C}, in.options());
-    check(na1d_permute_heads(ptr(out), ptr(in), c.B, c.T, parts, c.H, c.C, to_dense, stream()), "na1d_permute_heads");
-    return out;
-}
-Cfg dense_cfg(const Packed& c) { return Cfg{c.B * c.H, c.T, c.C, c.H, c.win, c.left, c.dil, c.scale, 0.0, 0}; }
 // qkv: packed, or (dense) the split one; o_dense: the dense route's own output
 struct LayerState { Tensor xt, qkv, lse, o, qw, pw, o_dense, qb, pb; };
 Tensor layer_forward(const Tensor& x, const LayerShape& l, const Tensor& vl, const Tensor& r, const Tensor& qw, const OptTensor& qb, const Tensor& pw,
@@ -846,15 +883,7 @@ Tensor layer_forward(const Tensor& x, const LayerShape& l, const Tensor& vl, con
     s.xt = l.first ? transposed(x, l, true) : x;
     s.qkv = project(s.xt.view({l.rows(), l.D}), w.qw, w.qb).view({l.B, l.T, 3 * l.D});
     if (keep) s.lse = empty_f32({l.B * c.H, l.T}, x);
-    if (takes_packed(c, x)) {
-        s.o = at::empty({l.B, l.T, l.D}, x.options());
-        packed_forward(s.o, s.lse, s.qkv, r, vl, c);
-    } else {
-        s.qkv = heads_moved(s.qkv, c, 3, true);
-        s.o_dense = at::empty({c.B * c.H, c.T, c.C}, x.options());
-        op_forward(s.o_dense, s.lse, s.qkv.select(0, 0), s.qkv.select(0, 1), s.qkv.select(0, 2), r, vl, dense_cfg(c));
-        s.o = heads_moved(s.o_dense, c, 1, false);
-    }
+    attention_forward(s.o, s.o_dense, s.qkv, s.lse, r, vl, c, takes_packed(c, x));
     Tensor y = project(s.o.view({l.rows(), l.D}), w.pw, w.pb);
     y = l.first ? transposed(y, l, false) : y.view({l.B, l.T, l.D});
     if (keep) { s.qw = w.qw; s.pw = w.pw; s.qb = w.qb; s.pb = w.pb; *keep = std::move(s); }
@@ -926,19 +955,9 @@ struct NA1dLayer : public torch::autograd::Function<NA1dLayer> {
         }
         Tensor dy = grads[0].defined() ? aligned(grads[0]) : at::zeros(l.first ? at::IntArrayRef({l.B, l.D, l.T}) : xt.sizes(), xt.options());
         dy = (l.first ? transposed(dy, l, true) : dy).view({l.rows(), l.D});
-        Tensor d_qkv = at::empty_like(qkv), d_rpb, d_x;
+        Tensor d_rpb, d_x;
         if (ctx->needs_input_grad(1)) d_rpb = zeros_f32(rpb.sizes(), xt);
-        if (o_dense.defined()) {
-            const Tensor d_o = heads_moved(product(dy, pw, Tensor(), true), c, 1, true), delta = empty_f32({c.B * c.H, c.T}, xt), r = rpb32(rpb);
-            auto part = [](const Tensor& t, int i) { return ptr(t.select(0, i)); };
-            check(na1d_fused_backward(part(d_qkv, 0), part(d_qkv, 1), part(d_qkv, 2), fptr(d_rpb), ptr(d_o), part(qkv, 0), part(qkv, 1), part(qkv, 2),
-                                      ptr(o_dense), fptr(lse), fptr(r), static_cast<int32_t*>(ptr(vl)), fptr(delta), c.B * c.H, c.H, c.T, c.C, c.win,
-                                      c.left, c.dil, (float)c.scale, code(qkv), stream()),
-                  "na1d_fused_backward");
-            d_qkv = heads_moved(d_qkv, c, 3, false);
-        } else {
-            packed_backward(d_qkv, d_rpb, product(dy, pw, Tensor(), true), qkv, lse, rpb32(rpb), vl, c);
-        }
+        const Tensor d_qkv = attention_backward(d_rpb, product(dy, pw, Tensor(), true), qkv, o_dense, lse, rpb32(rpb), vl, c);
         const Tensor dq = d_qkv.view({l.rows(), 3 * l.D});
         const std::vector<int64_t> qw_shape = d["qw_shape"].toIntVector(), pw_shape = d["pw_shape"].toIntVector();
         const LayerGrads g({ctx->needs_input_grad(2), ctx->needs_input_grad(3)},
