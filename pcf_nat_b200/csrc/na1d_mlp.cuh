@@ -1,5 +1,4 @@
-// Pieces that the kernels of a block's MLP share: how rows and hidden layer are shared out, pairs of fp32 values, turning rows per lane into
-// rows of adjacent lanes.
+// Pieces that the kernels of a block's MLP share: how rows and hidden layer are shared out, pairs of fp32 values, rows by sectors.
 #pragma once
 #include "na1d_pair.cuh"
 
@@ -12,7 +11,7 @@ constexpr int kSlotBytes = 16 * 1024;             // a CTA's half of half a weig
 constexpr uint32_t kAcc = 0, kHidden = 256;       // tensor-memory columns: result (256), two pieces of the hidden layer (128 each)
 
 // Items: whole tiles of 256 rows in full rounds of the CTA pairs, then the tiles of the last, partly filled round split over the hidden
-// layer into `parts`, so that this round takes 1 / parts of the time (150 tiles on 74 pairs: 2.1 instead of 3).
+// layer into `parts`, so that those take 1 / parts of the time (150 tiles on 74 pairs: 2.1 instead of 3).
 struct Plan {
     int rows, pieces, whole, parts, items;
 };
@@ -59,12 +58,6 @@ __device__ __forceinline__ float minus_abs(float x) {
     asm("max.NaN.f32 %0, %1, 0fC2800000;" : "=f"(r) : "f"(-fabsf(x)));
     return r;
 }
-// rows that are read once, in program order, so that they are in flight together
-__device__ __forceinline__ uint4 load_row(const void* p) {
-    uint4 v;
-    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
-    return v;
-}
 // 32 bytes, a sector, of a row: of each of a warp's 32 rows at a time
 __device__ __forceinline__ void load_sector(const void* p, uint32_t* v) {
     asm volatile("ld.global.nc.L1::no_allocate.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
@@ -74,7 +67,6 @@ __device__ __forceinline__ void store_sector(void* p, const uint32_t* v) {
     asm volatile("st.global.L1::no_allocate.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
                  ::"l"(p), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]) : "memory");
 }
-__device__ __forceinline__ uint32_t stage_at(int row, int chunk) { return (uint32_t)(row * 64 + ((chunk ^ (row >> 1)) & 3) * 16); }
 template <typename E> __device__ __forceinline__ void unpack2(const uint4& u, float2* f) {
     float t[8];
     Cvt<E>::unpack(u, t);
