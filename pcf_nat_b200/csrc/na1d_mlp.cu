@@ -6,7 +6,7 @@
 // For a backward pass the layer before GELU is stored, a sector of each row at a time straight from the lanes that hold it: 38400 rows
 // 51 + 4 us instead of 78.
 // A pair of CTAs keeps 256 rows on chip: the rows as an operand in shared memory, the hidden layer in pieces of 128 columns in tensor
-// memory, where GELU turns the first product's result into the second one's left operand in place.
+// memory, which GELU turns into the second product's left operand there.
 //   warps 0-15   GELU: 32 tensor-memory lanes and a quarter of a piece's columns each
 //   warps 16-23  the result: out of tensor memory at once (the next tile's second product waits for that) into registers and shared memory,
 //                as much as fits without local memory (L1 has next to no room here: what the compiler moved there made the whole kernel wait,
@@ -35,7 +35,7 @@ constexpr int kBiases = (kMostF + kD) * 4;
 constexpr int kSmem = 2 * kRowsBytes + kSlots * kSlotBytes + kResultWarps * kStage + kBiases + 1024;
 
 struct Barriers {
-    uint64_t full[kSlots], empty[kSlots], s_full[2], g_ready[2], a_full[2], a_free[2], o_full, o_free;
+    uint64_t full[kSlots], empty[kSlots], s_full, s_free, g_ready[2], a_full[2], a_free[2], o_full, o_free;
     uint32_t tmem;
     int abort;
 };
@@ -82,7 +82,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 
     if (warp == kGeluWarps + kResultWarps) {
         if (lane < kSlots) { ptx::mbar_init(&bar.full[lane], 1); ptx::mbar_init(&bar.empty[lane], 1); }
-        else if (lane >= 16 && lane < 18) { ptx::mbar_init(&bar.s_full[lane - 16], 1); ptx::mbar_init(&bar.g_ready[lane - 16], 2 * kGeluWarps); }
+        else if (lane >= 16 && lane < 18) ptx::mbar_init(&bar.g_ready[lane - 16], 2 * kGeluWarps);
+        else if (lane == 15) { ptx::mbar_init(&bar.s_full, 1); ptx::mbar_init(&bar.s_free, 2 * kGeluWarps); }
         else if (lane >= 18 && lane < 20) { ptx::mbar_init(&bar.a_full[lane - 18], 1); ptx::mbar_init(&bar.a_free[lane - 18], 1); }
         else if (lane == 9) { ptx::mbar_init(&bar.o_full, 1); ptx::mbar_init(&bar.o_free, 2 * kResultWarps); }
         else if (lane == 10) bar.abort = 0;
@@ -104,16 +105,21 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
         ptx::warpgroup_regs_shrink<kGeluRegs>();
         const int q = warp & 3, part = warp >> 2;   // tensor-memory lanes 32 q .. + 31, columns of this quarter
         const uint32_t lanes = (uint32_t)(q * 32) << 16;
-        const uint32_t g_ready0 = pair::in_leader(&bar.g_ready[0]), g_ready1 = pair::in_leader(&bar.g_ready[1]);
+        const uint32_t g_ready0 = pair::in_leader(&bar.g_ready[0]), g_ready1 = pair::in_leader(&bar.g_ready[1]), s_free = pair::in_leader(&bar.s_free);
+        auto leave = [&]() {   // the next piece's first product may have these columns
+            ptx::tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0) pair::arrive_cluster(s_free);
+        };
         int j = 0;
         for (int i = first; ok && i < plan.items; i += step) {
             const Item t = item_at(plan, i);
             const int row = t.tile * 256 + (int)rank * 128 + q * 32 + lane;
             for (int c = t.c0; c < t.c1; ++c, ++j) {
                 const int buf = j & 1, col = c * kChunk + part * 32;
-                const uint32_t s = tmem + lanes + kHidden + buf * kChunk + part * 32;
+                const uint32_t s = tmem + lanes + kHidden + part * 32, to = tmem + lanes + kOperand + buf * kOperandCols + part * 16;
                 const float4* b1 = reinterpret_cast<const float4*>(biases + kD + col);
-                if (!ptx::mbar_wait(&bar.s_full[buf], (j >> 1) & 1) || *abort_flag) NA1D_MLP_FAIL(1)
+                if (!ptx::mbar_wait(&bar.s_full, j & 1) || *abort_flag) NA1D_MLP_FAIL(1)
                 ptx::tc_fence_after_sync();
                 if constexpr (TRAIN) {   // sixteen columns at a time: a short loop, and one sector of each row
 #pragma unroll 1
@@ -121,6 +127,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                         float d[16];
                         pair::tmem_ld16(s + h * 16, d);
                         ptx::tmem_ld_wait();
+                        if (h == 1) leave();
                         uint32_t packed[8], hidden[8];
 #pragma unroll
                         for (int k = 0; k < 4; ++k) {
@@ -133,13 +140,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                             packed[2 * k] = Cvt<E>::pack2(gu.x, gu.y);
                             packed[2 * k + 1] = Cvt<E>::pack2(gv.x, gv.y);
                         }
-                        pair::tmem_st8(s + h * 8, packed);   // over columns that this warp has read
+                        pair::tmem_st8(to + h * 8, packed);
                         if (row < plan.rows) store_sector(g.f + (size_t)row * F + col + h * 16, hidden);
                     }
                 } else {
                     float d[32];
                     pair::tmem_ld32(s, d);
                     ptx::tmem_ld_wait();
+                    leave();
                     uint32_t packed[16];
 #pragma unroll
                     for (int k = 0; k < 8; ++k) {
@@ -149,7 +157,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                         packed[2 * k] = Cvt<E>::pack2(gu.x, gu.y);
                         packed[2 * k + 1] = Cvt<E>::pack2(gv.x, gv.y);
                     }
-                    pair::tmem_st16(s, packed);
+                    pair::tmem_st16(to, packed);
                 }
                 ptx::tmem_st_wait();
                 ptx::tc_fence_before_sync();
@@ -280,14 +288,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                 if (opens && (!ptx::mbar_wait(&bar.o_free, (item & 1) ^ 1) || *abort_flag)) { atomicExch(&g_mlp_status, 5); *abort_flag = 1; ok = false; return; }
                 if (!ptx::mbar_wait(&bar.g_ready[jj & 1], (jj >> 1) & 1) || *abort_flag) { atomicExch(&g_mlp_status, 6); *abort_flag = 1; ok = false; return; }
                 ptx::tc_fence_after_sync();
-                const uint32_t s = tmem + kHidden + (jj & 1) * kChunk;
+                const uint32_t s = tmem + kOperand + (jj & 1) * kOperandCols;
 #pragma unroll 1
                 for (int h = 0; h < 2; ++h) {
                     if (!ptx::mbar_wait(&bar.full[slot], phase) || *abort_flag) { atomicExch(&g_mlp_status, 7); *abort_flag = 1; ok = false; return; }
                     ptx::tc_fence_after_sync();
                     const uint64_t b = pair::k_major(ptx::smem_u32(ring + slot * kSlotBytes));
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) pair::mma_ts(tmem + kAcc, s + (h * 2 + (k >> 1)) * 32 + (k & 1) * 8, tc::desc_advance(b, k * 32), idesc2, !opens || h > 0 || k > 0);
+                    for (int k = 0; k < 4; ++k) pair::mma_ts(tmem + kAcc, s + (h * 4 + k) * 8, tc::desc_advance(b, k * 32), idesc2, !opens || h > 0 || k > 0);
                     pair::commit(&bar.empty[slot]);
                     next_slot();
                 }
@@ -299,9 +307,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                 if (!ptx::mbar_wait(&bar.a_full[it & 1], (it >> 1) & 1) || *abort_flag) NA1D_MLP_FAIL(8)
                 const uint64_t a = pair::k_major(ptx::smem_u32(rows_smem + (it & 1) * kRowsBytes));
                 for (int c = t.c0; ok && c < t.c1; ++c, ++j) {
-                    // The products of one thread run in order: the piece two back, which this one overwrites, has been used by its
-                    // second product, issued before.
-                    const uint32_t s = tmem + kHidden + (j & 1) * kChunk;
+                    if (!ptx::mbar_wait(&bar.s_free, (j & 1) ^ 1) || *abort_flag) NA1D_MLP_FAIL(10)
+                    ptx::tc_fence_after_sync();
 #pragma unroll 1
                     for (int h = 0; h < 2; ++h) {
                         if (!ptx::mbar_wait(&bar.full[slot], phase) || *abort_flag) NA1D_MLP_FAIL(9)
@@ -309,12 +316,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                         const uint64_t b = pair::k_major(ptx::smem_u32(ring + slot * kSlotBytes)), ah = tc::desc_advance(a, h * 32768);
 #pragma unroll
                         for (int k = 0; k < 8; ++k)
-                            pair::mma_ss(s, tc::desc_advance(ah, (k >> 2) * 16384 + (k & 3) * 32), tc::desc_advance(b, (k >> 2) * 8192 + (k & 3) * 32), idesc1, h > 0 || k > 0);
+                            pair::mma_ss(tmem + kHidden, tc::desc_advance(ah, (k >> 2) * 16384 + (k & 3) * 32), tc::desc_advance(b, (k >> 2) * 8192 + (k & 3) * 32), idesc1, h > 0 || k > 0);
                         pair::commit(&bar.empty[slot]);
                         next_slot();
                     }
                     if (!ok) break;
-                    pair::commit(&bar.s_full[j & 1]);
+                    pair::commit(&bar.s_full);   // (and all that was issued before, the second product of the piece two back among it)
                     if (c == t.c1 - 1) pair::commit(&bar.a_free[it & 1]);
                     if (j > 0) second(j - 1, c == t.c0 ? it - 1 : it, opened, c == t.c0);
                     opened = c == t.c0;

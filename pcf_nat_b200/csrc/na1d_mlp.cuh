@@ -8,7 +8,13 @@ namespace {
 constexpr int kD = 256, kChunk = 128, kMostF = 1280;
 constexpr int kRowsBytes = 128 * kD * 2;          // a CTA's rows as an operand: four blocks of 64 channels, [block][row][128 bytes]
 constexpr int kSlotBytes = 16 * 1024;             // a CTA's half of half a weight piece
-constexpr uint32_t kAcc = 0, kHidden = 256;       // tensor-memory columns: result (256), two pieces of the hidden layer (128 each)
+// Tensor-memory columns: the result (256), a piece of the hidden layer as the first product leaves it (128, fp32), and two pieces as the second
+// product reads them (64 each, 16 bits). What a product writes is never what an earlier one may still read without a barrier in
+// between: products of different shapes are not known to run in the order of their issue. The first product of a piece waits
+// until the 16 warps of both CTAs have read the one before out of its columns (s_free; they do so at once, while the second
+// product of the piece before runs), and a piece that GELU writes lies where the one two back was, whose second product is among those
+// that the signal for this piece's first (s_full) waits for.
+constexpr uint32_t kAcc = 0, kHidden = 256, kOperand = 384, kOperandCols = 64;
 
 // Items: whole tiles of 256 rows in full rounds of the CTA pairs, then the tiles of the last, partly filled round split over the hidden
 // layer into `parts`, so that those take 1 / parts of the time (150 tiles on 74 pairs: 2.1 instead of 3).

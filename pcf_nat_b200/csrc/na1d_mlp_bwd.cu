@@ -30,7 +30,7 @@ constexpr int kSlots = 6;
 constexpr int kSmem = 2 * kRowsBytes + kSlots * kSlotBytes + 1024;
 
 struct Barriers {
-    uint64_t full[kSlots], empty[kSlots], s_full[2], g_ready[2], a_full[2], a_free[2], o_full, o_free;
+    uint64_t full[kSlots], empty[kSlots], s_full, s_free, g_ready[2], a_full[2], a_free[2], o_full, o_free;
     uint32_t tmem;
     int abort;
 };
@@ -74,7 +74,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 
     if (warp == kGeluWarps + kResultWarps) {
         if (lane < kSlots) { ptx::mbar_init(&bar.full[lane], 1); ptx::mbar_init(&bar.empty[lane], 1); }
-        else if (lane >= 16 && lane < 18) { ptx::mbar_init(&bar.s_full[lane - 16], 1); ptx::mbar_init(&bar.g_ready[lane - 16], 2 * kGeluWarps); }
+        else if (lane >= 16 && lane < 18) ptx::mbar_init(&bar.g_ready[lane - 16], 2 * kGeluWarps);
+        else if (lane == 15) { ptx::mbar_init(&bar.s_full, 1); ptx::mbar_init(&bar.s_free, 2 * kGeluWarps); }
         else if (lane >= 24 && lane < 26) { ptx::mbar_init(&bar.a_full[lane - 24], 1); ptx::mbar_init(&bar.a_free[lane - 24], 1); }
         else if (lane == 19) { ptx::mbar_init(&bar.o_full, 1); ptx::mbar_init(&bar.o_free, 2 * kResultWarps); }
         else if (lane == 20) bar.abort = 0;
@@ -96,7 +97,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
         ptx::warpgroup_regs_grow<kGeluRegs>();
         const int q = warp & 3, part = warp >> 2;   // tensor-memory lanes 32 q .. + 31, columns of this quarter
         const uint32_t lanes = (uint32_t)(q * 32) << 16;
-        const uint32_t g_ready0 = pair::in_leader(&bar.g_ready[0]), g_ready1 = pair::in_leader(&bar.g_ready[1]);
+        const uint32_t g_ready0 = pair::in_leader(&bar.g_ready[0]), g_ready1 = pair::in_leader(&bar.g_ready[1]), s_free = pair::in_leader(&bar.s_free);
         uint32_t next[8];   // f of the next sixteen columns
         auto fetch = [&](const Item& t, int c, int h) {
             const int row = t.tile * 256 + (int)rank * 128 + q * 32 + lane;
@@ -111,9 +112,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
             const int row = t.tile * 256 + (int)rank * 128 + q * 32 + lane;
             for (int c = t.c0; c < t.c1; ++c, ++j) {
                 const int buf = j & 1;
-                const uint32_t s = tmem + lanes + kHidden + buf * kChunk + part * 32;
+                const uint32_t s = tmem + lanes + kHidden + part * 32, to = tmem + lanes + kOperand + buf * kOperandCols + part * 16;
                 const size_t at = (size_t)row * F + c * kChunk + part * 32;
-                if (!ptx::mbar_wait(&bar.s_full[buf], (j >> 1) & 1) || *abort_flag) NA1D_MLP_FAIL(1)
+                if (!ptx::mbar_wait(&bar.s_full, j & 1) || *abort_flag) NA1D_MLP_FAIL(1)
                 ptx::tc_fence_after_sync();
 #pragma unroll 1
                 for (int h = 0; h < 2; ++h) {
@@ -126,6 +127,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                     else if (c + 1 < t.c1) fetch(t, c + 1, 0);
                     else if (i + step < plan.items) { const Item n = item_at(plan, i + step); fetch(n, n.c0, 0); }
                     ptx::tmem_ld_wait();
+                    if (h == 1) {   // the next piece's first product may have these columns
+                        ptx::tc_fence_before_sync();
+                        __syncwarp();
+                        if (lane == 0) pair::arrive_cluster(s_free);
+                    }
                     uint32_t df[8], val[8];
 #pragma unroll
                     for (int k = 0; k < 8; ++k) {
@@ -135,7 +141,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                         val[k] = Cvt<E>::pack2(value.x, value.y);
                         df[k] = Cvt<E>::pack2(slope.x, slope.y);
                     }
-                    pair::tmem_st8(s + h * 8, df);   // over columns that this warp has read
+                    pair::tmem_st8(to + h * 8, df);
                     if (row < plan.rows) {
                         store_sector(g.g + at + h * 16, val);
                         store_sector(g.df + at + h * 16, df);
@@ -249,14 +255,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                 if (opens && (!ptx::mbar_wait(&bar.o_free, (item & 1) ^ 1) || *abort_flag)) { atomicExch(&g_mlp_bwd_status, 5); *abort_flag = 1; ok = false; return; }
                 if (!ptx::mbar_wait(&bar.g_ready[jj & 1], (jj >> 1) & 1) || *abort_flag) { atomicExch(&g_mlp_bwd_status, 6); *abort_flag = 1; ok = false; return; }
                 ptx::tc_fence_after_sync();
-                const uint32_t s = tmem + kHidden + (jj & 1) * kChunk;
+                const uint32_t s = tmem + kOperand + (jj & 1) * kOperandCols;
 #pragma unroll 1
                 for (int h = 0; h < 2; ++h) {
                     if (!ptx::mbar_wait(&bar.full[slot], phase) || *abort_flag) { atomicExch(&g_mlp_bwd_status, 7); *abort_flag = 1; ok = false; return; }
                     ptx::tc_fence_after_sync();
                     const uint64_t b = pair::mn_major(ptx::smem_u32(ring + slot * kSlotBytes), 8192);
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) pair::mma_ts(tmem + kAcc, s + (h * 2 + (k >> 1)) * 32 + (k & 1) * 8, tc::desc_advance(b, k * 2048), idesc2, !opens || h > 0 || k > 0);
+                    for (int k = 0; k < 4; ++k) pair::mma_ts(tmem + kAcc, s + (h * 4 + k) * 8, tc::desc_advance(b, k * 2048), idesc2, !opens || h > 0 || k > 0);
                     pair::commit(&bar.empty[slot]);
                     next_slot();
                 }
@@ -268,8 +274,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                 if (!ptx::mbar_wait(&bar.a_full[it & 1], (it >> 1) & 1) || *abort_flag) NA1D_MLP_FAIL(8)
                 const uint64_t a = pair::k_major(ptx::smem_u32(rows_smem + (it & 1) * kRowsBytes));
                 for (int c = t.c0; ok && c < t.c1; ++c, ++j) {
-                    // (the products of one thread run in order: the piece two back, which this one overwrites, has been used)
-                    const uint32_t s = tmem + kHidden + (j & 1) * kChunk;
+                    if (!ptx::mbar_wait(&bar.s_free, (j & 1) ^ 1) || *abort_flag) NA1D_MLP_FAIL(10)
+                    ptx::tc_fence_after_sync();
 #pragma unroll 1
                     for (int h = 0; h < 2; ++h) {
                         if (!ptx::mbar_wait(&bar.full[slot], phase) || *abort_flag) NA1D_MLP_FAIL(9)
@@ -277,12 +283,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                         const uint64_t b = pair::mn_major(ptx::smem_u32(ring + slot * kSlotBytes), 8192), ah = tc::desc_advance(a, h * 32768);
 #pragma unroll
                         for (int k = 0; k < 8; ++k)
-                            pair::mma_ss(s, tc::desc_advance(ah, (k >> 2) * 16384 + (k & 3) * 32), tc::desc_advance(b, k * 2048), idesc1, h > 0 || k > 0);
+                            pair::mma_ss(tmem + kHidden, tc::desc_advance(ah, (k >> 2) * 16384 + (k & 3) * 32), tc::desc_advance(b, k * 2048), idesc1, h > 0 || k > 0);
                         pair::commit(&bar.empty[slot]);
                         next_slot();
                     }
                     if (!ok) break;
-                    pair::commit(&bar.s_full[j & 1]);
+                    pair::commit(&bar.s_full);   // (and all that was issued before, the second product of the piece two back among it)
                     if (c == t.c1 - 1) pair::commit(&bar.a_free[it & 1]);
                     if (j > 0) second(j - 1, c == t.c0 ? it - 1 : it, opened, c == t.c0);
                     opened = c == t.c0;
