@@ -249,6 +249,10 @@ int na1d_column_sums(float* sums, float* scratch, const void* x, int64_t rows, i
 int64_t na1d_mlp_scratch_floats(int64_t rows, int64_t D, int64_t F);
 int na1d_mlp_forward(void* out, int64_t ld, void* f, const void* s, const void* h, const void* w1, const float* b1, const void* w2, const float* b2,
                      float* scratch, int64_t rows, int64_t D, int64_t F, int dtype, void* stream);
+/* The same with the rounding points of its passes one by one: biases of `dtype`, GELU of the hidden layer's 16-bit values (which f takes).
+ * Without f every sum over the hidden layer is one chain, as in a product that is not split, and scratch is not read (may be NULL). */
+int na1d_mlp_forward_rounded(void* out, int64_t ld, void* f, const void* s, const void* h, const void* w1, const void* b1, const void* w2, const void* b2,
+                             float* scratch, int64_t rows, int64_t D, int64_t F, int dtype, void* stream);
 /* Its backward for the gradient d (rows, D) of out: df (rows, F) = (d w2) * gelu'(f), dh (rows, D) = df w1, g (rows, F) = gelu(f), all
  * 16-bit and, like f, 32-byte aligned; sizes and `scratch` as above. What the parameters need is left to na1d_projection_gradients. */
 int na1d_mlp_backward(void* dh, void* df, void* g, const void* d, const void* f, const void* w1, const void* w2, float* scratch, int64_t rows, int64_t D,

@@ -107,6 +107,7 @@ for _name, _args in (
         ("na1d_column_sums", [_ptr] * 3 + [_i64, _i64]),
         ("na1d_cast_parameters", [_ptr] * 4 + [_i32]),
         ("na1d_mlp_forward", [_ptr, _i64] + [_ptr] * 8 + [_i64] * 3),
+        ("na1d_mlp_forward_rounded", [_ptr, _i64] + [_ptr] * 8 + [_i64] * 3),
         ("na1d_mlp_backward", [_ptr] * 8 + [_i64] * 3),
         ("na1d_projection_gradients", [_ptr] * 6 + [_i32, _i64, _ptr, _i32]),
         ("na1d_transpose", [_ptr, _ptr, _i64, _i64, _i64, _i32]),

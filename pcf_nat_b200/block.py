@@ -8,7 +8,8 @@ which is one kernel forward and one backward where its sizes allow (256 channels
 is the fused operator on the packed projection output.
 
 Rounding points are those of the autocast network: 16-bit activations and projection weights, fp32 statistics and sums; the
-LayerNorm parameters and the weight gradients are not rounded to 16 bits on the way.
+LayerNorm parameters and the weight gradients are not rounded to 16 bits on the way, nor is the gradient of GELU's values in the MLP's
+backward kernel.
 """
 import torch
 import torch.nn as nn

@@ -653,14 +653,22 @@ int64_t na1d_mlp_scratch_floats(int64_t rows, int64_t D, int64_t F) {
     if (!na1d::mlp_supports(D, F) || check_block(rows, F, 1 << 20, NA1D_BF16) != NA1D_OK) return -1;
     return (int64_t)na1d::mlp_scratch_floats(rows, F);
 }
-int na1d_mlp_forward(void* out, int64_t ld, void* f, const void* s, const void* h, const void* w1, const float* b1, const void* w2, const float* b2, float* scratch,
-                     int64_t rows, int64_t D, int64_t F, int dtype, void* stream) {
+static int mlp_forward(void* out, int64_t ld, void* f, const void* s, const void* h, const void* w1, const void* b1, const void* w2, const void* b2, bool rounded,
+                       float* scratch, int64_t rows, int64_t D, int64_t F, int dtype, void* stream) {
     if (int e = check_pointers(out, s, h, w1, b1, w2, b2)) return e;
     if ((((uintptr_t)f | (uintptr_t)s) & 31) || !aligned16(scratch)) return NA1D_ERR_MISALIGNED;
     if (int e = check_block(rows, F, 1 << 20, dtype)) return e;
     if (!na1d::mlp_supports(D, F) || ld < D || ld % 8 != 0 || ld > (1ll << 40) / rows) return NA1D_ERR_BAD_SHAPE;
-    if (!scratch && na1d::mlp_scratch_floats(rows, F)) return NA1D_ERR_NULL_POINTER;
-    return cuda_status(na1d::mlp_forward(out, ld, f, s, h, w1, b1, w2, b2, scratch, rows, F, dtype, (cudaStream_t)stream));
+    if (!scratch && na1d::mlp_scratch_floats(rows, F) && (f || !rounded)) return NA1D_ERR_NULL_POINTER;
+    return cuda_status(na1d::mlp_forward(out, ld, f, s, h, w1, b1, w2, b2, rounded, scratch, rows, F, dtype, (cudaStream_t)stream));
+}
+int na1d_mlp_forward(void* out, int64_t ld, void* f, const void* s, const void* h, const void* w1, const float* b1, const void* w2, const float* b2, float* scratch,
+                     int64_t rows, int64_t D, int64_t F, int dtype, void* stream) {
+    return mlp_forward(out, ld, f, s, h, w1, b1, w2, b2, false, scratch, rows, D, F, dtype, stream);
+}
+int na1d_mlp_forward_rounded(void* out, int64_t ld, void* f, const void* s, const void* h, const void* w1, const void* b1, const void* w2, const void* b2,
+                             float* scratch, int64_t rows, int64_t D, int64_t F, int dtype, void* stream) {
+    return mlp_forward(out, ld, f, s, h, w1, b1, w2, b2, true, scratch, rows, D, F, dtype, stream);
 }
 int na1d_mlp_backward(void* dh, void* df, void* g, const void* d, const void* f, const void* w1, const void* w2, float* scratch, int64_t rows, int64_t D, int64_t F,
                       int dtype, void* stream) {

@@ -8,7 +8,7 @@
 // kernel adds up in a fixed order: no atomics, the same bits from run to run.
 #include "../../include/na1d_b200.h"
 #include "na1d_internal.h"
-#include "na1d_tc_common.cuh"
+#include "na1d_gelu.cuh"
 
 namespace na1d {
 namespace {
@@ -254,26 +254,7 @@ __global__ void __launch_bounds__(kRowThreads) ln_bwd_kernel(E* __restrict__ dx,
     cta_column_sums<3, CH>(acc, part, blockIdx.x, D, 0);
 }
 
-// ---------------------------------------------------------------- GELU (exact form x Phi(x)) and column sums
-// Phi(-|x|) = t P(t) e^{-x^2/2} with t = 1 / (1 + 0.29980 |x|): the substitution of Abramowitz & Stegun 7.1.26, with a polynomial of
-// degree 7 fitted to e^{z^2} erfc(z) (relative error 4e-8 for |x| < 5.6, rising to 1e-4 beyond 9). The negative tail is a product, not
-// 1 - erf, so it keeps its relative accuracy (in fp32 8e-7 for |x| < 4, 8e-6 to 9, 2e-5 to 12), and e^{-x^2/2} is shared with
-// the density in the derivative. Over all bf16 values 94 results round the wrong way, over all fp16 values 3, against 118 and 370 of
-// the framework's 1 + erf form (and 161 and 254 with the five terms of 7.1.26). Two special-function operations and ~15 fp32
-// operations a value instead of the library erff's ~25 with a branch (165 us for 153600 x 1024 values; 116 us here, 98 us of HBM time).
-__device__ __forceinline__ void phi(float x, float& cdf, float& e) {
-    const float t = fast_rcp(fmaf(0.2998046875f, fabsf(x), 1.f));
-    e = fast_exp2(x * x * (-0.5f * kLog2e));
-    float p = fmaf(t, 0.0360688753426075f, -0.15834912657737732f);
-    p = fmaf(t, p, 0.20701442658901215f);
-    p = fmaf(t, p, -0.05189161375164986f);
-    p = fmaf(t, p, 0.1259254813194275f);
-    p = fmaf(t, p, 0.1013689711689949f);
-    p = fmaf(t, p, 0.12026944756507874f);
-    p = fmaf(t, p, 0.1195935606956482f);
-    const float tail = p * t * e;
-    cdf = x >= 0.f ? 1.f - tail : tail;
-}
+// ---------------------------------------------------------------- GELU (exact form x Phi(x), na1d_gelu.cuh) and column sums
 __device__ __forceinline__ float gelu(float x) {
     float c, e;
     phi(x, c, e);

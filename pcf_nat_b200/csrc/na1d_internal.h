@@ -98,8 +98,8 @@ int wgrad_read_status();
 // ---- a block's MLP, out = s + GELU(h w1^T + b1) w2^T + b2 (na1d_mlp.cu)
 bool mlp_supports(int64_t D, int64_t F);
 size_t mlp_scratch_floats(int64_t rows, int64_t F);
-cudaError_t mlp_forward(void* out, int64_t ld, void* f, const void* s, const void* h, const void* w1, const float* b1, const void* w2, const float* b2, float* scratch,
-                        int64_t rows, int64_t F, int dtype, cudaStream_t st);
+cudaError_t mlp_forward(void* out, int64_t ld, void* f, const void* s, const void* h, const void* w1, const void* b1, const void* w2, const void* b2, bool rounded,
+                        float* scratch, int64_t rows, int64_t F, int dtype, cudaStream_t st);
 int mlp_read_status();
 // its backward (na1d_mlp_bwd.cu): df = (d w2) GELU'(f), dh = df w1, gelu = GELU(f); dh, df, gelu, f (and the forward's f) 32-byte aligned
 cudaError_t mlp_backward(void* dh, void* df, void* gelu, const void* d, const void* f, const void* w1, const void* w2, float* scratch, int64_t rows, int64_t F,

@@ -2,9 +2,9 @@
 // multiple of 128.
 //
 // As separate passes (product, GELU, product, residual in the next LayerNorm) the hidden layer, four times as wide as the rows, crosses
-// HBM four times: 153600 rows took 106 + 126 + 94 us where the products themselves need 95; 133 + 5 us here (76800: 73 + 4, 9600: 25).
-// For a backward pass the layer before GELU is stored, a sector of each row at a time straight from the lanes that hold it: 38400 rows
-// 51 + 4 us instead of 78.
+// HBM four times: 153600 rows take 314 us where the products themselves need 95; 175 us here (38400: 81 and 64, 9600: 28 and 27, 2400: 15
+// and 26, which is left to the passes). For a backward pass the layer before GELU is stored, a sector of each row at a time straight
+// from the lanes that hold it, and the last round of tiles is split over the hidden layer: 38400 rows 59 us.
 // A pair of CTAs keeps 256 rows on chip: the rows as an operand in shared memory, the hidden layer in pieces of 128 columns in tensor
 // memory, which GELU turns into the second product's left operand there.
 //   warps 0-15   GELU: 32 tensor-memory lanes and a quarter of a piece's columns each
@@ -14,7 +14,8 @@
 //   warp 24      loads: the rows of the next tile, the residual's into L2, weight pieces (16 KB a CTA: half of the output columns and
 //                of the contraction; a ring of four)
 //   warp 25      issues the products (leader): piece j + 1 of the hidden layer before the second product of piece j
-// Bound: tensor pipe (1024 + 1024 cycles a piece), GELU (FMA pipe 1150, special functions 1024), 64 KB of weights a piece from L2.
+// Bound: tensor pipe (1024 + 1024 cycles a piece) and GELU at the same length (special functions 2048, FMA pipe 1800; 133 us with a polynomial
+// for log2 Phi, one special function a value, whose results differ from the passes' in their last bits); 64 KB of weights a piece from L2.
 // Every role's code is a short loop. (With the LayerNorm in it too -- eight warps, rows through registers -- the kernel took 245 us for
 // 153600 rows: its arithmetic, and the instructions it needs, come on top of GELU's.)
 #include "na1d_internal.h"
@@ -43,7 +44,7 @@ struct Barriers {
 struct Maps { CUtensorMap h, s, w1, w2; };
 template <typename E> struct Args {
     const E* s;                        // residual stream
-    const float *b1, *b2;
+    const void *b1, *b2;               // ROUND: 16-bit, else fp32
     E* out;                            // rows ld elements apart
     long long ld;
     E* f;                              // (rows, F): the hidden layer before GELU, for a backward pass
@@ -51,21 +52,14 @@ template <typename E> struct Args {
     float* part;                       // partial results of the split tiles
 };
 
-// x Phi(x) = max(x, 0) - |x| Phi(-|x|), with Phi(-a) = 2^P(a): log2 of the tail is a smooth function, so a polynomial of degree 7 keeps
-// the tail's relative accuracy (1e-5 for |x| < 2, 1e-4 to 4, 1e-3 to 6; the argument is not rounded to 16 bits first, which alone
-// would cost x^2 2^-9) with one special-function operation instead of two. P falls beyond the fitted range too (leading term -1.1e-6).
-__device__ __forceinline__ float2 gelu2(float2 x) {
-    const float2 a = make_float2(minus_abs(x.x), minus_abs(x.y));
-    float2 p = fma2(both(1.0900799907176406e-06f), a, both(4.5614655391545966e-05f));
-    p = fma2(p, a, both(0.0008011450991034508f));
-    p = fma2(p, a, both(0.00800548680126667f));
-    p = fma2(p, a, both(0.05297810584306717f));
-    p = fma2(p, a, both(-0.45937567949295044f));
-    p = fma2(p, a, both(1.1509263515472412f));
-    p = fma2(p, a, both(-1.000016212463379f));
-    return fma2(a, make_float2(tc::fast_exp2(p.x), tc::fast_exp2(p.y)), make_float2(fmaxf(x.x, 0.f), fmaxf(x.y, 0.f)));
+template <typename E, bool ROUND> __device__ __forceinline__ float bias_at(const void* b, int i) {
+    if constexpr (ROUND) return (float)reinterpret_cast<const E*>(b)[i];
+    else return reinterpret_cast<const float*>(b)[i];
 }
-template <typename E, bool TRAIN>
+
+// TRAIN: the hidden layer before GELU is stored. ROUND: GELU is taken of its 16-bit values, also where they are not stored, as a pass over the
+// stored layer would.
+template <typename E, bool TRAIN, bool ROUND>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     mlp_kernel(const __grid_constant__ Maps maps, const __grid_constant__ Plan plan, const __grid_constant__ Args<E> g) {
     extern __shared__ uint8_t raw[];
@@ -93,7 +87,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
         ptx::fence_mbar_init();
     }
     if (warp == kGeluWarps + kResultWarps + 2) { pair::tmem_alloc(&bar.tmem, 512); pair::tmem_relinquish(); }
-    for (int i = threadIdx.x; i < kD + F; i += kThreads) biases[i] = i < kD ? g.b2[i] : g.b1[i - kD];
+    for (int i = threadIdx.x; i < kD + F; i += kThreads) biases[i] = i < kD ? bias_at<E, ROUND>(g.b2, i) : bias_at<E, ROUND>(g.b1, i - kD);
     ptx::tc_fence_before_sync();
     __syncthreads();
     pair::cluster_sync();
@@ -110,6 +104,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
             ptx::tc_fence_before_sync();
             __syncwarp();
             if (lane == 0) pair::arrive_cluster(s_free);
+        };
+        auto activated = [](const float2& u, uint32_t rounded) {
+            const float2 y = gelu2(ROUND ? unpack2<E>(rounded) : u);
+            return Cvt<E>::pack2(y.x, y.y);
         };
         int j = 0;
         for (int i = first; ok && i < plan.items; i += step) {
@@ -136,9 +134,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                             const float2 v = add2(make_float2(d[4 * k + 2], d[4 * k + 3]), make_float2(bias.z, bias.w));
                             hidden[2 * k] = Cvt<E>::pack2(u.x, u.y);
                             hidden[2 * k + 1] = Cvt<E>::pack2(v.x, v.y);
-                            const float2 gu = gelu2(u), gv = gelu2(v);
-                            packed[2 * k] = Cvt<E>::pack2(gu.x, gu.y);
-                            packed[2 * k + 1] = Cvt<E>::pack2(gv.x, gv.y);
+                            packed[2 * k] = activated(u, hidden[2 * k]);
+                            packed[2 * k + 1] = activated(v, hidden[2 * k + 1]);
                         }
                         pair::tmem_st8(to + h * 8, packed);
                         if (row < plan.rows) store_sector(g.f + (size_t)row * F + col + h * 16, hidden);
@@ -152,10 +149,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 #pragma unroll
                     for (int k = 0; k < 8; ++k) {
                         const float4 bias = b1[k];
-                        const float2 gu = gelu2(add2(make_float2(d[4 * k], d[4 * k + 1]), make_float2(bias.x, bias.y)));
-                        const float2 gv = gelu2(add2(make_float2(d[4 * k + 2], d[4 * k + 3]), make_float2(bias.z, bias.w)));
-                        packed[2 * k] = Cvt<E>::pack2(gu.x, gu.y);
-                        packed[2 * k + 1] = Cvt<E>::pack2(gv.x, gv.y);
+                        const float2 u = add2(make_float2(d[4 * k], d[4 * k + 1]), make_float2(bias.x, bias.y));
+                        const float2 v = add2(make_float2(d[4 * k + 2], d[4 * k + 3]), make_float2(bias.z, bias.w));
+                        packed[2 * k] = activated(u, ROUND ? Cvt<E>::pack2(u.x, u.y) : 0u);
+                        packed[2 * k + 1] = activated(v, ROUND ? Cvt<E>::pack2(v.x, v.y) : 0u);
                     }
                     pair::tmem_st16(to, packed);
                 }
@@ -340,14 +337,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 
 // The split tiles' partial results, residual and bias, in the order of the parts: a thread per four columns of a row, a CTA per 32 rows x 32
 // columns.
-template <typename E>
+template <typename E, bool ROUND>
 __global__ void __launch_bounds__(256) mlp_finish_kernel(const __grid_constant__ Plan plan, const __grid_constant__ Args<E> g) {
     const int n = blockIdx.x & 3, band = blockIdx.x >> 2, w = band & 7, rank = (band >> 3) & 1, tile = plan.whole + (band >> 4);
     const int lane = threadIdx.x & 31, k = threadIdx.x >> 5;
     const int row = tile * 256 + rank * 128 + (w & 3) * 32 + lane, col = (w >> 2) * 128 + n * 32 + k * 4;
     if (row >= plan.rows) return;
     const uint2 res = __ldg(reinterpret_cast<const uint2*>(g.s + (size_t)row * kD + col));
-    const float4 b = __ldg(reinterpret_cast<const float4*>(g.b2 + col));
+    const float4 b = make_float4(bias_at<E, ROUND>(g.b2, col), bias_at<E, ROUND>(g.b2, col + 1), bias_at<E, ROUND>(g.b2, col + 2), bias_at<E, ROUND>(g.b2, col + 3));
     const float4* src = reinterpret_cast<const float4*>(g.part) + (size_t)band * plan.parts * 32 * 32 + (n * 8 + k) * 32 + lane;
     float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 8
@@ -360,9 +357,9 @@ __global__ void __launch_bounds__(256) mlp_finish_kernel(const __grid_constant__
     *reinterpret_cast<uint2*>(g.out + (size_t)row * g.ld + col) = make_uint2(sum.x, sum.y);
 }
 
-template <typename E, bool TRAIN>
+template <typename E, bool TRAIN, bool ROUND>
 cudaError_t run(const Maps& maps, const Plan& plan, const Args<E>& a, cudaStream_t st) {
-    auto* kern = mlp_kernel<E, TRAIN>;
+    auto* kern = mlp_kernel<E, TRAIN, ROUND>;
     // a kernel compiled to fewer registers would leave the growing warp groups waiting for ones that never come
     static const int regs = [kern] {
         cudaFuncAttributes fa;
@@ -374,13 +371,13 @@ cudaError_t run(const Maps& maps, const Plan& plan, const Args<E>& a, cudaStream
     kern<<<2 * n, kThreads, kSmem, st>>>(maps, plan, a);
     if (plan.parts == 1) return cudaGetLastError();
     if (cudaError_t e = cudaGetLastError()) return e;
-    mlp_finish_kernel<E><<<(plan.items - plan.whole) / plan.parts * 2 * kResultWarps * 4, 256, 0, st>>>(plan, a);
+    mlp_finish_kernel<E, ROUND><<<(plan.items - plan.whole) / plan.parts * 2 * kResultWarps * 4, 256, 0, st>>>(plan, a);
     return cudaGetLastError();
 }
-template <typename E>
-cudaError_t forward(void* out, int64_t ld, void* f, const void* s, const void* h, const void* w1, const float* b1, const void* w2, const float* b2, float* scratch,
+template <typename E, bool ROUND>
+cudaError_t forward(void* out, int64_t ld, void* f, const void* s, const void* h, const void* w1, const void* b1, const void* w2, const void* b2, float* scratch,
                     int64_t rows, int64_t F, int dtype, cudaStream_t st) {
-    const Plan plan = make_plan(rows, F);
+    const Plan plan = make_plan(rows, F, !ROUND || f);
     Maps maps;
     const int64_t dh[3] = {64, rows, kD / 64}, d1[3] = {64, F, kD / 64}, s1[2] = {kD, 64}, d2[3] = {64, kD, F / 64}, s2[2] = {F, 64};
     const int xh[3] = {64, 128, kD / 64}, x1[3] = {64, 64, 2}, x2[3] = {64, 128, 1};
@@ -388,7 +385,7 @@ cudaError_t forward(void* out, int64_t ld, void* f, const void* s, const void* h
         !make_matrix_map(&maps.w2, w2, dtype, 3, d2, s2, x2))
         return cudaErrorInvalidValue;
     const Args<E> a = {(const E*)s, b1, b2, (E*)out, ld, (E*)f, ld % 16 == 0 && ((uintptr_t)out & 31) == 0, scratch};
-    return f ? run<E, true>(maps, plan, a, st) : run<E, false>(maps, plan, a, st);
+    return f ? run<E, true, ROUND>(maps, plan, a, st) : run<E, false, ROUND>(maps, plan, a, st);
 }
 
 }  // namespace
@@ -397,11 +394,16 @@ bool mlp_supports(int64_t D, int64_t F) { return D == kD && F > 0 && F % kChunk 
 size_t mlp_scratch_floats(int64_t rows, int64_t F) {
     return part_floats(make_plan(rows, F));
 }
-cudaError_t mlp_forward(void* out, int64_t ld, void* f, const void* s, const void* h, const void* w1, const float* b1, const void* w2, const float* b2, float* scratch,
-                        int64_t rows, int64_t F, int dtype, cudaStream_t st) {
+cudaError_t mlp_forward(void* out, int64_t ld, void* f, const void* s, const void* h, const void* w1, const void* b1, const void* w2, const void* b2, bool rounded,
+                        float* scratch, int64_t rows, int64_t F, int dtype, cudaStream_t st) {
     bind_primary_context();
-    return dtype == 0 ? forward<__nv_bfloat16>(out, ld, f, s, h, w1, b1, w2, b2, scratch, rows, F, dtype, st)
-                      : forward<__half>(out, ld, f, s, h, w1, b1, w2, b2, scratch, rows, F, dtype, st);
+    using B = __nv_bfloat16;
+    using H = __half;
+    if (rounded)
+        return dtype == 0 ? forward<B, true>(out, ld, f, s, h, w1, b1, w2, b2, scratch, rows, F, dtype, st)
+                          : forward<H, true>(out, ld, f, s, h, w1, b1, w2, b2, scratch, rows, F, dtype, st);
+    return dtype == 0 ? forward<B, false>(out, ld, f, s, h, w1, b1, w2, b2, scratch, rows, F, dtype, st)
+                      : forward<H, false>(out, ld, f, s, h, w1, b1, w2, b2, scratch, rows, F, dtype, st);
 }
 int mlp_read_status() {
     int v = 0, zero = 0;

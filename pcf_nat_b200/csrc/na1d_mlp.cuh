@@ -1,5 +1,6 @@
-// Pieces that the kernels of a block's MLP share: how rows and hidden layer are shared out, pairs of fp32 values, rows by sectors.
+// Pieces that the kernels of a block's MLP share: how rows and hidden layer are shared out, rows by sectors.
 #pragma once
+#include "na1d_gelu.cuh"
 #include "na1d_pair.cuh"
 
 namespace na1d {
@@ -40,30 +41,6 @@ __device__ __forceinline__ Item item_at(const Plan& p, int i) {
     return t;
 }
 
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
-    float2 d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;"
-        : "=l"(reinterpret_cast<uint64_t&>(d))
-        : "l"(reinterpret_cast<const uint64_t&>(a)), "l"(reinterpret_cast<const uint64_t&>(b)), "l"(reinterpret_cast<const uint64_t&>(c)));
-    return d;
-}
-__device__ __forceinline__ float2 both(float x) { return make_float2(x, x); }
-__device__ __forceinline__ float2 add2(float2 a, float2 b) {
-    float2 d;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(reinterpret_cast<uint64_t&>(d)) : "l"(reinterpret_cast<const uint64_t&>(a)), "l"(reinterpret_cast<const uint64_t&>(b)));
-    return d;
-}
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
-    float2 d;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(reinterpret_cast<uint64_t&>(d)) : "l"(reinterpret_cast<const uint64_t&>(a)), "l"(reinterpret_cast<const uint64_t&>(b)));
-    return d;
-}
-// -min(|x|, 64), of a NaN NaN: beyond that the tail of GELU is zero anyway, and an infinite argument keeps its value (no infinity times zero)
-__device__ __forceinline__ float minus_abs(float x) {
-    float r;
-    asm("max.NaN.f32 %0, %1, 0fC2800000;" : "=f"(r) : "f"(-fabsf(x)));
-    return r;
-}
 // 32 bytes, a sector, of a row: of each of a warp's 32 rows at a time
 __device__ __forceinline__ void load_sector(const void* p, uint32_t* v) {
     asm volatile("ld.global.nc.L1::no_allocate.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
@@ -79,6 +56,10 @@ template <typename E> __device__ __forceinline__ void unpack2(const uint4& u, fl
 #pragma unroll
     for (int i = 0; i < 4; ++i) f[i] = make_float2(t[2 * i], t[2 * i + 1]);
 }
+template <typename E> __device__ __forceinline__ float2 unpack2(uint32_t w) {
+    if constexpr (sizeof(E) == 2 && tc::Fmt<E>::v == 1) return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
+    else return __half22float2(*reinterpret_cast<const __half2*>(&w));
+}
 template <typename E> __device__ __forceinline__ uint4 pack2(const float2* f) {
     return make_uint4(Cvt<E>::pack2(f[0].x, f[0].y), Cvt<E>::pack2(f[1].x, f[1].y), Cvt<E>::pack2(f[2].x, f[2].y), Cvt<E>::pack2(f[3].x, f[3].y));
 }
@@ -92,14 +73,15 @@ template <typename E> __device__ __forceinline__ uint4 add_rows(const uint4& x, 
     return pack2<E>(a);
 }
 
-inline Plan make_plan(int64_t rows, int64_t F) {
+// split: the last, partly filled round over the hidden layer
+inline Plan make_plan(int64_t rows, int64_t F, bool split = true) {
     Plan p;
     const int pairs = device_sm_count() / 2, tiles = (int)((rows + 255) / 256);
     p.rows = (int)rows;
     p.pieces = (int)(F / kChunk);
     p.whole = tiles / pairs * pairs;
     const int rest = tiles - p.whole;
-    p.parts = rest ? pairs / rest : 1;
+    p.parts = rest && split ? pairs / rest : 1;
     if (p.parts > p.pieces) p.parts = p.pieces;
     if (p.parts < 2) { p.parts = 1; p.whole = tiles; }
     p.items = p.whole + (tiles - p.whole) * p.parts;

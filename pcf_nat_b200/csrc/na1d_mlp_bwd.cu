@@ -2,7 +2,7 @@
 // the gradient of W2 needs and the forward does not keep.
 //
 // As separate passes (product, GELU' with the bias gradient, product) the gradient of the hidden layer crossed HBM four times: 38400 rows
-// took 15 + 52 + 18 us, here 69 + 3 (153600: 243 + 4). It goes from the first product through GELU' to the second one in tensor memory, as
+// took 15 + 52 + 18 us, here 78 (153600: 273). It goes from the first product through GELU' to the second one in tensor memory, as
 // in the forward; only df and g leave, for the parameter gradients (the bias gradient is a column sum there). The same shape of kernel:
 //   warps 0-15   GELU': 32 tensor-memory lanes and a quarter of a piece's columns each, a row per lane, sixteen columns (one sector) at a
 //                time; f of the next sixteen is on its way meanwhile
@@ -10,8 +10,9 @@
 //   warp 24      loads: the rows of the next tile, weight pieces (both products contract across their rows), a ring of six; f from HBM into
 //                L2 two pieces ahead (without: 271 us for 153600 rows)
 //   warp 25      issues the products (leader)
-// Bound by HBM: f in, df and g out, three rows of 1024 for every row of 256 in and out (43 us at 38400 rows). The products and GELU' alone
-// take 121 us for 153600 rows, with the reads of f 171, with the stores 216. Sectors of a row straight from registers, without a line in
+// Bound by HBM: f in, df and g out, three rows of 1024 for every row of 256 in and out (43 us at 38400 rows). GELU and its slope are those of the
+// passes (na1d_gelu.cuh), so g is bit for bit what the forward multiplied. In a form of this kernel whose products did not wait for
+// GELU's reads (243 us for 153600 rows) the products and GELU' alone took 121, with the reads of f 171, with the stores 216. Sectors of a row straight from registers, without a line in
 // L1 (with one: 281), against 315 through a stage in shared memory, whose room the ring needs: weights wait behind the stores on
 // their way from L2.
 #include "na1d_internal.h"
@@ -41,23 +42,6 @@ template <typename E> struct Args {
     E* dh;            // (rows, 256)
     float* part;      // partial results of the split tiles
 };
-
-// GELU and its derivative of a pair: Phi(-|x|) = 2^P(|x|) as in the forward, here of degree 10 (2e-6 for |x| < 4, 4e-5 to 6: the argument
-// comes rounded, and HBM leaves the time)
-__device__ __forceinline__ void gelu_and_slope(const float2 x, float2& value, float2& slope) {
-    const float2 a = make_float2(minus_abs(x.x), minus_abs(x.y));
-    constexpr float c[11] = {-0.9999977350234985f, -1.1511825323104858f,  -0.45877406001091003f,  -0.053428445011377335f, 0.008054247125983238f, -0.0007130972808226943f,
-                             -3.336832605782547e-07f, 8.790148967818823e-06f, -1.064999878508388e-06f, 5.625529553299202e-08f, -1.154139894765649e-09f};
-    float2 p = both(c[10]);
-#pragma unroll
-    for (int n = 9; n >= 0; --n) p = fma2(p, a, both(n & 1 ? -c[n] : c[n]));
-    const float2 tail = make_float2(tc::fast_exp2(p.x), tc::fast_exp2(p.y));
-    const float2 e = mul2(mul2(x, x), both(-0.5f * kLog2e));
-    const float2 density = make_float2(tc::fast_exp2(e.x), tc::fast_exp2(e.y));
-    value = fma2(a, tail, make_float2(fmaxf(x.x, 0.f), fmaxf(x.y, 0.f)));
-    const float2 cdf = make_float2(x.x >= 0.f ? 1.f - tail.x : tail.x, x.y >= 0.f ? 1.f - tail.y : tail.y);
-    slope = fma2(mul2(x, both(0.3989422804014327f)), density, cdf);
-}
 
 template <typename E>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)

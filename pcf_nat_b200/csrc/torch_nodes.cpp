@@ -565,8 +565,18 @@ Tensor layer_norm_backward(const Tensor& dy, const Tensor& s, const Tensor& st, 
     return ds;
 }
 
+// Whether a block's evaluation takes its MLP as one kernel. A tile of 256 rows is a chain of pieces on a pair of SMs (sums over the hidden
+// layer are not split there, so that both routes give the same bits): 7 us and 2.3 us for a piece of 128 columns in every round of
+// pairs, against 9 us and 0.063 us for a tile's piece in the passes. Hidden size 1024, passes / kernel in us: 2400 rows 15 / 26, 9600 rows
+// 28 / 27, 38400 rows 81 / 64, 153600 rows 314 / 175.
+bool mlp_pays(int64_t rows, int64_t F) {
+    const int64_t tiles = (rows + 255) / 256, pairs = std::max(1, at::cuda::getCurrentDeviceProperties()->multiProcessorCount / 2);
+    const double pieces = F / 128.0;
+    return 7 + 2.3 * pieces * ((tiles + pairs - 1) / pairs) <= 9 + 0.063 * pieces * tiles;
+}
+
 // x (+ dx): the residual stream. Returns the stream after the attention branch and the MLP branch's output; their sum is the
-// block's output, taken inside the next block's first LayerNorm. At the sizes that the MLP kernel takes, the sum alone (the second tensor
+// block's output, taken inside the next block's first LayerNorm. Where the MLP kernel runs, the sum alone (the second tensor
 // undefined), without a backward pass to come in `out` if that is given: rows of D inside wider ones.
 std::pair<Tensor, Tensor> block_forward(const Tensor& x, const Tensor& dx, const Tensor& vl, const Packed& c, double eps1, double eps2,
                                         const Tensor* p, BlockState* keep, const OptTensor& out = std::nullopt) {
@@ -583,13 +593,13 @@ std::pair<Tensor, Tensor> block_forward(const Tensor& x, const Tensor& dx, const
     layer_norm(st.h2, st.s2, st.st2, st.s1, y, p[10], p[11], eps2, stats);
     const int64_t F = w.t[4].size(0), floats = na1d_mlp_scratch_floats(rows, D, F);
     Tensor s2, z;
-    if (floats >= 0) {
-        const Tensor scratch = floats ? empty_f32({floats}, x) : Tensor();
+    if (floats >= 0 && (keep || mlp_pays(rows, F))) {
+        const Tensor scratch = floats && keep ? empty_f32({floats}, x) : Tensor();
         s2 = out && !keep ? *out : at::empty_like(x);
         if (keep) st.f = at::empty({rows, F}, x.options());
-        check(na1d_mlp_forward(ptr(s2), s2.stride(1), ptr(st.f), ptr(st.s2), ptr(st.h2), ptr(w.t[4]), fptr(p[5]), ptr(w.t[6]), fptr(p[7]), fptr(scratch), rows, D, F,
-                               code(x), stream()),
-              "na1d_mlp_forward");
+        check(na1d_mlp_forward_rounded(ptr(s2), s2.stride(1), ptr(st.f), ptr(st.s2), ptr(st.h2), ptr(w.t[4]), ptr(w.t[5]), ptr(w.t[6]), ptr(w.t[7]), fptr(scratch),
+                                       rows, D, F, code(x), stream()),
+              "na1d_mlp_forward_rounded");
     } else {
         st.f = product(st.h2.view({rows, D}), w.t[4], w.t[5], false);
         st.g = at::empty_like(st.f);
