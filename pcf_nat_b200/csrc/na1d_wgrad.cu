@@ -5,9 +5,11 @@
 // products spend 28 to 36 us on each of a block's larger ones (64-column tiles: every input is read from L2 many times over) and a
 // reduction after each; a pass over dy for the bias gradient came on top. Here a pair of SMs takes a 256 x 256 tile (the left
 // operand's columns split over the two, the right one's too), so a row of inputs crosses from L2 once per 256 columns of the other
-// operand, and the bias gradient is a product of the staged dy with 32 columns of ones. Bound by the L2's bandwidth
-// (8.7 TB/s with nothing but the loads): 38400 rows, 1024 x 256 and 256 x 1024: 48 us + 7.5 us for the sum over splits, 314 MB from L2
-// (30 us of HBM time), against 63 + 12 us and 11 us for the bias; 768 x 256 and 256 x 256: 33 + 9 us against 43 + 12 + 11 us.
+// operand, and the warps that later store the results add up the staged columns of dy for the bias gradient. They do so in fp32: as a product
+// of the staged dy with ones, which took the same time, the sums were up to 24 times further off than those of a pass over dy, since the
+// tensor cores do not round to nearest; they are as exact as that pass now. Bound by the L2's bandwidth
+// (8.7 TB/s with nothing but the loads): 38400 rows, 1024 x 256 and 256 x 1024: 48 us with the sum over splits, 314 MB from L2
+// (30 us of HBM time), against 88 us for the library's products and two passes of column sums; 768 x 256 and 256 x 256: 38 against 63 us.
 #include "na1d_internal.h"
 #include "na1d_pair.cuh"
 
@@ -16,20 +18,19 @@ namespace {
 
 __device__ int g_wgrad_status = 0;
 
-constexpr int kThreads = 384;                    // warp 0: loads, warp 1: MMA issue, warp 2: tensor memory, warps 4-11: results
+constexpr int kThreads = 384;                    // warp 0: loads, 1: MMA issue, 2: tensor memory, 4-11: column sums and results
 constexpr int kStep = 64;                        // rows per shared-memory stage
 constexpr int kTile = 256;
 constexpr int kHalf = kTile / 2;                 // columns of either operand in one CTA
 constexpr int kBox = 64 * kStep * 2;             // 64 columns of a stage: one row of the 128-byte swizzle per contraction row
 constexpr int kStageBytes = 4 * kBox;            // two boxes of each operand
 constexpr int kStages = 7;
-constexpr int kOnes = 1024;
-constexpr int kSmem = kStages * kStageBytes + kOnes + 1024;
+constexpr int kSmem = kStages * kStageBytes + 1024;
 constexpr int kMost = 2;                         // projections per launch
-constexpr uint32_t kCols = 512;                  // 256 for the tile, 32 for the column sums
+constexpr uint32_t kCols = 256;
 
 struct Barriers {
-    uint64_t full[kStages], empty[kStages], acc_full, acc_empty;
+    uint64_t full[kStages], empty[kStages], used[kStages], acc_full, acc_empty;   // of a stage: loaded, multiplied, added up
     uint32_t tmem;
     int abort;
 };
@@ -67,7 +68,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     wgrad_kernel(const __grid_constant__ Maps maps, const __grid_constant__ Work work, float* __restrict__ part, float* __restrict__ part_bias) {
     extern __shared__ uint8_t raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(raw) + 1023) & ~(uintptr_t)1023);
-    E* ones = reinterpret_cast<E*>(smem + kStages * kStageBytes);
     __shared__ Barriers bar;
     const int warp = ptx::warp_index(), lane = threadIdx.x & 31;
     const uint32_t rank = pair::cta_rank();
@@ -75,15 +75,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     volatile int* abort_flag = &bar.abort;
 
     if (warp == 0) {
-        if (lane < kStages) { ptx::mbar_init(&bar.full[lane], 1); ptx::mbar_init(&bar.empty[lane], 1); }
+        if (lane < kStages) { ptx::mbar_init(&bar.full[lane], 1); ptx::mbar_init(&bar.empty[lane], 1); ptx::mbar_init(&bar.used[lane], 8); }
         else if (lane == kStages) { ptx::mbar_init(&bar.acc_full, 1); ptx::mbar_init(&bar.acc_empty, 16); bar.abort = 0; }
         ptx::fence_mbar_init();
     } else if (warp == 1 && lane < work.count) {
         ptx::prefetch_tensormap(&maps.a[lane]);
         ptx::prefetch_tensormap(&maps.b[lane]);
     }
-    for (int i = threadIdx.x; i < kOnes / 2; i += kThreads) ones[i] = E(1.f);
-    ptx::fence_proxy_async_smem();
     if (warp == 2) { pair::tmem_alloc(&bar.tmem, kCols); pair::tmem_relinquish(); }
     ptx::tc_fence_before_sync();
     __syncthreads();
@@ -101,7 +99,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                 const CUtensorMap *ma = &maps.a[t.p], *mb = &maps.b[t.p];
                 const int m = t.m0 + rank * kHalf, nn = t.n0 + rank * kHalf;
                 for (int k = t.k0; k < t.k1; ++k) {
-                    if (!ptx::mbar_wait_relaxed(&bar.empty[slot], phase) || *abort_flag) { atomicExch(&g_wgrad_status, 1); *abort_flag = 1; ok = false; break; }
+                    if (!ptx::mbar_wait_relaxed(&bar.used[slot], phase) || *abort_flag) { atomicExch(&g_wgrad_status, 1); *abort_flag = 1; ok = false; break; }
                     const uint32_t full = pair::in_leader(&bar.full[slot]);
                     uint8_t* s = smem + slot * kStageBytes;
                     if (rank == 0) ptx::mbar_expect_tx(&bar.full[slot], 2 * kStageBytes);
@@ -119,8 +117,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     } else if (warp == 1) {
         if (rank == 0 && ptx::elect_one()) {
             constexpr uint32_t fmt = tc::Fmt<E>::v;
-            constexpr uint32_t idesc = ptx::instr_desc(fmt, 1, 1, 256, kTile), idesc_ones = ptx::instr_desc(fmt, 1, 0, 256, 32);
-            const uint64_t one = ptx::smem_desc(ptx::smem_u32(ones), 128, 256, ptx::kSwizzleNone);
+            constexpr uint32_t idesc = ptx::instr_desc(fmt, 1, 1, 256, kTile);
             int slot = 0, it = 0;
             uint32_t phase = 0;
             bool ok = true;
@@ -136,10 +133,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 #pragma unroll
                     for (int j = 0; j < kStep / 16; ++j)
                         pair::mma_ss(tmem, tc::desc_advance(a, j * 2048), tc::desc_advance(b, j * 2048), idesc, k > t.k0 || j > 0);
-                    if (t.n0 == 0) {
-#pragma unroll
-                        for (int j = 0; j < kStep / 16; ++j) pair::mma_ss(tmem + kTile, tc::desc_advance(a, j * 2048), one, idesc_ones, k > t.k0 || j > 0);
-                    }
                     pair::commit(&bar.empty[slot]);
                     if (++slot == kStages) { slot = 0; phase ^= 1; }
                 }
@@ -147,11 +140,45 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
             }
         }
     } else if (warp >= 4) {
+        // Column sums, of a stage that the products have read (`empty`: both CTAs learn of it; the loads count on the leader's barriers alone). The
+        // stage is loaded again when these warps are through with it too. A lane takes rows r, r + 16, .. of a stage and eight adjacent columns (lanes of one phase of an access: eight rows, whose
+        // swizzle puts them on all banks)
+        const int r = lane & 15, chunk = 2 * (warp - 4) + (lane >> 4);
+        const uint8_t* column = smem + (chunk >> 3) * kBox + r * 128 + (((chunk & 7) ^ (r & 7)) << 4);
+        int slot = 0;
+        uint32_t phase = 0;
         const int q = warp & 3, h = (warp - 4) >> 2;   // tensor-memory lanes 32 q .. + 31 (those a warp reaches), half h of the columns
         const uint32_t lanes = (uint32_t)(q * 32) << 16;
         int it = 0;
         for (int i = first; i < work.items; i += step, ++it) {
             const Item t = item_at(work, i);
+            float sum[8] = {};
+            bool ok = true;
+            for (int k = t.k0; k < t.k1; ++k) {
+                if (!ptx::mbar_wait(&bar.empty[slot], phase) || *abort_flag) { atomicExch(&g_wgrad_status, 5); *abort_flag = 1; ok = false; break; }
+                if (t.n0 == 0) {
+                    float v[4][8];
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) Cvt<E>::unpack(*reinterpret_cast<const uint4*>(column + slot * kStageBytes + j * 16 * 128), v[j]);
+#pragma unroll
+                    for (int c = 0; c < 8; ++c) sum[c] += (v[0][c] + v[1][c]) + (v[2][c] + v[3][c]);
+                }
+                __syncwarp();
+                if (lane == 0) ptx::mbar_arrive(&bar.used[slot]);
+                if (++slot == kStages) { slot = 0; phase ^= 1; }
+            }
+            if (!ok) break;
+            if (t.n0 == 0) {
+#pragma unroll
+                for (int c = 0; c < 8; ++c)
+#pragma unroll
+                    for (int o = 8; o > 0; o >>= 1) sum[c] += __shfl_xor_sync(0xffffffffu, sum[c], o);
+                if (r == 0) {
+                    float4* dst = reinterpret_cast<float4*>(part_bias + ((size_t)i * 8 + rank * 4) * 32 + chunk * 8);
+                    dst[0] = make_float4(sum[0], sum[1], sum[2], sum[3]);
+                    dst[1] = make_float4(sum[4], sum[5], sum[6], sum[7]);
+                }
+            }
             if (!ptx::mbar_wait_relaxed(&bar.acc_full, it & 1) || *abort_flag) { atomicExch(&g_wgrad_status, 4); *abort_flag = 1; break; }
             ptx::tc_fence_after_sync();
             const size_t band = (size_t)i * 8 + rank * 4 + q;
@@ -163,12 +190,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                 ptx::tmem_ld_wait();
 #pragma unroll
                 for (int j = 0; j < 8; ++j) dst[(c / 4 + j) * 32] = make_float4(d[4 * j], d[4 * j + 1], d[4 * j + 2], d[4 * j + 3]);
-            }
-            if (t.n0 == 0 && h == 0) {
-                float d[8];
-                ptx::tmem_ld8(tmem + lanes + kTile, d);
-                ptx::tmem_ld_wait();
-                part_bias[band * 32 + lane] = d[0];
             }
             ptx::tc_fence_before_sync();
             __syncwarp();
@@ -215,11 +236,12 @@ __global__ void __launch_bounds__(1024) wgrad_sum_kernel(const __grid_constant__
     const int row = threadIdx.x >> 5;
     if (out.w[p] && n0 + lane < q.N && m0 + row < q.M)
         reinterpret_cast<O*>(out.w[p])[(size_t)(m0 + row) * q.N + n0 + lane] = O((sm[0][row][lane] + sm[1][row][lane]) + (sm[2][row][lane] + sm[3][row][lane]));
-    if (out.b[p] && n0 == 0 && threadIdx.x < 32 && m0 + lane < q.M) {
+    if (out.b[p] && n0 == 0 && m0 + row < q.M) {   // a warp to a column, a lane to every 32nd split
         float b = 0.f;
-#pragma unroll 4
-        for (int k = 0; k < q.splits; ++k) b += __ldg(part_bias + ((item0 + k) * 8 + band) * 32 + lane);
-        reinterpret_cast<O*>(out.b[p])[m0 + lane] = O(b);
+        for (int k = lane; k < q.splits; k += 32) b += __ldg(part_bias + ((item0 + k) * 8 + band) * 32 + row);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) b += __shfl_xor_sync(0xffffffffu, b, o);
+        if (lane == 0) reinterpret_cast<O*>(out.b[p])[m0 + row] = O(b);
     }
 }
 
