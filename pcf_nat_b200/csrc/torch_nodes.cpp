@@ -483,7 +483,19 @@ Tensor attention_backward(const Tensor& d_rpb, const Tensor& d_o, const Tensor& 
 }
 
 // ---------------------------------------------------------------- the transformer block
-// Parameter gradients of up to two projections in one launch: d_w = dy^T x and d_b = column sums of dy, of `type` from fp32 sums.
+// Whether the weight-gradient kernel takes these products (M, N: their sizes). It has a pair of SMs to a tile of 256 x 256 and splits the rows
+// where that leaves pairs idle; with few splits or none a sum over partial tiles is left of its gain, which the library's products do not
+// pay. Rows of 768 / 1024 channels, weights of an MLP (72, 128 tiles; us, kernel against library with column sums): 2400 rows
+// 49 / 35, 121 / 50 (38400: 299 / 313, 1140 / 507 with two rounds of tiles); two splits (a layer of 768, an MLP of 512): 2400 rows
+// 31 / 30 and 30 / 30, 600 rows 27 / 19 and 24 / 18, 9600 rows 51 / 61 and 49 / 61; more splits (an MLP of 256): 2400 rows 18 / 23, 38400
+// 48 / 88.
+bool gradients_in_one_launch(const int64_t* M, const int64_t* N, int n, int64_t rows) {
+    const int64_t pairs = std::max(1, at::cuda::getCurrentDeviceProperties()->multiProcessorCount / 2);
+    int64_t tiles = 0;
+    for (int i = 0; i < n; ++i) tiles += ((M[i] + 255) / 256) * ((N[i] + 255) / 256);
+    return tiles * (rows < 4800 ? 3 : 2) <= pairs;
+}
+// Parameter gradients of up to two projections: d_w = dy^T x and d_b = column sums of dy, of `type` from fp32 sums.
 // dy (rows, M), x (rows, N); what is not wanted stays undefined.
 struct ParameterGrads {
     Tensor w[2], b[2];
@@ -492,20 +504,36 @@ struct ParameterGrads {
         const void *py[2], *px[2];
         int64_t M[2], N[2];
         int n = 0;
+        const int64_t rows = dy[0].size(0);
         for (int i = 0; i < 2; ++i) {
-            if (!need_w[i] && !need_b[i]) continue;
+            if (!need_w[i]) continue;
             M[n] = dy[i].size(1);
             N[n] = x[i].size(1);
-            const auto opts = dy[i].options().dtype(type);
-            if (need_w[i]) w[i] = at::empty({M[n], N[n]}, opts);
-            if (need_b[i]) b[i] = at::empty({M[n]}, opts);
-            pw[n] = ptr(w[i]); pb[n] = ptr(b[i]); py[n] = ptr(dy[i]); px[n] = ptr(x[i]);
             ++n;
         }
-        if (n == 0) return;
-        const int64_t rows = dy[0].size(0);
+        const bool one = n > 0 && gradients_in_one_launch(M, N, n, rows);
+        n = 0;
+        for (int i = 0; i < 2; ++i) {
+            if (one && need_w[i]) {
+                const auto opts = dy[i].options().dtype(type);
+                w[i] = at::empty({M[n], N[n]}, opts);
+                if (need_b[i]) b[i] = at::empty({M[n]}, opts);
+                pw[n] = ptr(w[i]); pb[n] = ptr(b[i]); py[n] = ptr(dy[i]); px[n] = ptr(x[i]);
+                ++n;
+                continue;
+            }
+            if (need_w[i]) w[i] = at::mm(dy[i].t(), x[i], at::kFloat).to(type);
+            if (need_b[i]) b[i] = column_sums(dy[i]).to(type);
+        }
+        if (!one) return;
         const Tensor scratch = empty_f32({na1d_projection_gradients_scratch(M, N, n, rows)}, dy[0]);
         check(na1d_projection_gradients(pw, pb, py, px, M, N, n, rows, fptr(scratch), type == at::kFloat, code(dy[0]), stream()), "na1d_projection_gradients");
+    }
+    static Tensor column_sums(const Tensor& dy) {
+        const int64_t rows = dy.size(0), F = dy.size(1);
+        const Tensor sums = empty_f32({F}, dy), scratch = empty_f32({na1d_block_scratch_floats(rows, 0, F)}, dy);
+        check(na1d_column_sums(fptr(sums), fptr(scratch), ptr(dy), rows, F, code(dy), stream()), "na1d_column_sums");
+        return sums;
     }
 };
 
