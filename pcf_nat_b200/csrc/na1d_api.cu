@@ -318,7 +318,8 @@ static int pick_family(const na1d::Geometry& g, int backward, bool has_bias = fa
     // less: forward at 64 channels 2000 x 64 rows, dilation 3 (22 rows a residue) 56 us against 40, 1200 x 150, dilation 4 (38) 56 / 47,
     // dilation 3 (50) 36 / 37; backward 4000 x 31 rows, window 15, dilation 3 (11 rows) 301 / 182 (64 channels), 125 / 115 (32), window 5,
     // dilation 2 (16 rows) 161 / 87 and 80 / 55, but window 15 208 / 184 and 86 / 107.
-    if (forced == -1 && pick == 2 && g.dil > 1) {
+    // (With NA1D_BIAS_GRAD_ROWS=1 a bias gradient is summed in a fixed order, which the general kernels' atomics do not give.)
+    if (forced == -1 && pick == 2 && g.dil > 1 && !(backward && wants_bias_grad && na1d::bias_grad_partial_rows())) {
         const int tp = (g.T + g.dil - 1) / g.dil;
         if (backward ? tp <= 12 || (tp <= 16 && g.win <= 9) : tp <= 40) pick = 0;
     }
