@@ -317,11 +317,12 @@ static int pick_family(const na1d::Geometry& g, int backward, bool has_bias = fa
     // Short residues leave a segmented tile of 128 rows mostly empty, and the general kernels (whose tiles hold 64, or a row at a time) take
     // less: forward at 64 channels 2000 x 64 rows, dilation 3 (22 rows a residue) 56 us against 40, 1200 x 150, dilation 4 (38) 56 / 47,
     // dilation 3 (50) 36 / 37; backward 4000 x 31 rows, window 15, dilation 3 (11 rows) 301 / 182 (64 channels), 125 / 115 (32), window 5,
-    // dilation 2 (16 rows) 161 / 87 and 80 / 55, but window 15 208 / 184 and 86 / 107.
+    // dilation 2 (16 rows) 161 / 87 and 80 / 55, but window 15 208 / 184 and 86 / 107. At 32 channels the widest window bucket stays longer: 200000 rows,
+    // window 27, residues of 12, 10 and 8 rows 205 / 254, 245 / 241 and 303 / 230 (window 33: 212 / 288, 253 / 273, 313 / 264; 18: 205 / 194 at 12).
     // (With NA1D_BIAS_GRAD_ROWS=1 a bias gradient is summed in a fixed order, which the general kernels' atomics do not give.)
     if (forced == -1 && pick == 2 && g.dil > 1 && !(backward && wants_bias_grad && na1d::bias_grad_partial_rows())) {
         const int tp = (g.T + g.dil - 1) / g.dil;
-        if (backward ? tp <= 12 || (tp <= 16 && g.win <= 9) : tp <= 40) pick = 0;
+        if (backward ? tp <= (g.C == 32 && g.win > 22 ? 9 : 12) || (tp <= 16 && g.win <= 9) : tp <= 40) pick = 0;
     }
     if (forced == 1 && pick == 0) return NA1D_ERR_UNSUPPORTED;
     return pick;
