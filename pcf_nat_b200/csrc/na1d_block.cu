@@ -59,9 +59,8 @@ template <int R> __device__ __forceinline__ void warp_sums(float (&v)[R], int la
 
 // y = LN(s) w + b with s = x, or s = round(x + dx) written to `sum` (the residual stream): R rows of a warp at a time, which stay in
 // registers (mean first, then the centred squares) while the next R are on their way.
-// 153600 rows of 256, with / without the addition: 53 / 41 us a row at a time (its loads, a sum over the warp and again: too few bytes in
-// flight without the second input), 51 / 32 us with four (49 / 24 of HBM time); wider rows stay at one, a row is then enough to load.
-// 231 + 37 us by the framework's kernels.
+// 153600 rows of 256, with / without the addition: 55 / 39 us a row at a time (its loads, a sum over the warp and again: too few bytes in
+// flight without the second input), 54 / 28 us with four (49 / 24 of HBM time). 231 + 37 us by the framework's kernels.
 template <typename E, int CH, int R, bool ADD>
 __global__ void __launch_bounds__(kRowThreads) ln_fwd_kernel(E* __restrict__ y, E* __restrict__ sum, float* __restrict__ mean,
                                                              float* __restrict__ rstd, const E* __restrict__ x,
@@ -621,9 +620,13 @@ int row_grid(long long rows, int per_sm) {
 template <typename E>
 cudaError_t ln_fwd(void* y, void* sum, float* mean, float* rstd, const void* x, const void* dx, const float* w, const float* b,
                    int rows, int D, float eps, cudaStream_t st) {
-    const int ch = (D + 255) / 256;
-#define NA1D_LN(CH, R, ADD) ln_fwd_kernel<E, CH, R, ADD><<<row_grid((rows + R - 1) / R, 4), kRowThreads, 0, st>>>((E*)y, (E*)sum, mean, rstd, (const E*)x, (const E*)dx, w, b, rows, D, eps)
-#define NA1D_LN_C(ADD) switch (ch) { case 1: NA1D_LN(1, 4, ADD); break; case 2: NA1D_LN(2, 1, ADD); break; case 3: NA1D_LN(3, 1, ADD); break; default: NA1D_LN(4, 1, ADD); }
+    // Four rows of a warp (0) where the rows fill the grid with that. A few rows are sooner done one to a warp: 2400 x 256 2.8 us with the
+    // addition, 2.5 without (four: 3.2 and 2.6), 38400 x 128 12.1 with it (13.0); 153600 x 256 without it 28 (39). Grids, for 153600 rows:
+    // 4 CTAs per SM at most for groups of four; one row at a time 512 channels 103 us with the addition and 60 without at 12 (108, 60
+    // at 8; 115, 58 at 4), 768 channels 153 and 88 (153, 95; 167, 124), 1024 channels 198 and 112 (203, 123; 215, 136).
+    const int ch = D <= 256 && rows >= (dx ? 1 << 16 : 1 << 15) ? 0 : (D + 255) / 256;
+#define NA1D_LN(CH, R, ADD) ln_fwd_kernel<E, CH, R, ADD><<<row_grid((rows + R - 1) / R, R == 4 ? 4 : 12), kRowThreads, 0, st>>>((E*)y, (E*)sum, mean, rstd, (const E*)x, (const E*)dx, w, b, rows, D, eps)
+#define NA1D_LN_C(ADD) switch (ch) { case 0: NA1D_LN(1, 4, ADD); break; case 1: NA1D_LN(1, 1, ADD); break; case 2: NA1D_LN(2, 1, ADD); break; case 3: NA1D_LN(3, 1, ADD); break; default: NA1D_LN(4, 1, ADD); }
     if (dx) { NA1D_LN_C(true) } else { NA1D_LN_C(false) }
 #undef NA1D_LN_C
 #undef NA1D_LN
