@@ -409,6 +409,15 @@ Tensor aligned(const Tensor& g, uintptr_t bytes = 16) {
     return (reinterpret_cast<uintptr_t>(c.data_ptr()) & (bytes - 1)) ? c.clone() : c;
 }
 
+// What a node of more than the operator saved, as the kernels read it, wherever a saved-tensor hook has put it.
+variable_list saved_dense(AutogradContext* ctx) {
+    variable_list saved = ctx->get_saved_variables();
+    const at::NoGradGuard off;
+    for (Tensor& t : saved)
+        if (t.defined() && t.is_cuda()) t = aligned(t);
+    return saved;
+}
+
 // A backward pass works in the types of its forward, also where it is called under autocast (to another type, the library products
 // would hand the kernels tensors of that type).
 struct NoAutocast {
@@ -667,8 +676,8 @@ struct NA1dFuse : public torch::autograd::Function<NA1dFuse> {
         return out;
     }
     static variable_list backward(AutogradContext* ctx, variable_list grads) {
-        const variable_list s = ctx->get_saved_variables();
-        const Tensor cat = aligned(s[0]), buf = aligned(s[1]);
+        const variable_list s = saved_dense(ctx);
+        const Tensor &cat = s[0], &buf = s[1];
         const int64_t D = ctx->saved_data["D"].toInt(), O = ctx->saved_data["O"].toInt(), K = cat.size(2), rows = cat.size(0) * cat.size(1), parts = K / D;
         const c10::cuda::CUDAGuard guard(cat.device());
         const NoAutocast off;
@@ -759,11 +768,11 @@ struct NA1dBlock : public torch::autograd::Function<NA1dBlock> {
         return inner_gradients(grads.size() == 1 ? variable_list{s2 + z} : variable_list{s2, z}, in, grads);
     }
     static variable_list backward(AutogradContext* ctx, variable_list grads) {
-        const variable_list s = ctx->get_saved_variables();
-        const Tensor &s1 = s[0], &st1 = s[1], &qkv = s[3], &lse = s[4], &s2 = s[6], &st2 = s[7], &n1w = s[12], &n2w = s[13], &rpb = s[14], &vl = s[15];
-        // (as the products read them, wherever a saved-tensor hook has put them; f by whole sectors)
-        const Tensor h1 = aligned(s[2]), o = aligned(s[5]), h2 = aligned(s[8]), buf = aligned(s[11]), f = aligned(s[9], 32);
-        Tensor g = s[10].defined() ? aligned(s[10]) : s[10];
+        const variable_list s = saved_dense(ctx);
+        const Tensor &s1 = s[0], &st1 = s[1], &h1 = s[2], &qkv = s[3], &lse = s[4], &o = s[5], &s2 = s[6], &st2 = s[7], &h2 = s[8], &buf = s[11], &n1w = s[12],
+                     &n2w = s[13], &rpb = s[14], &vl = s[15];
+        const Tensor f = aligned(s[9], 32);   // (read by whole sectors)
+        Tensor g = s[10];
         auto& data = ctx->saved_data;
         const Packed c(s1.size(0), s1.size(1), s1.size(2), data["heads"].toInt(), data["win"].toInt(), data["left"].toInt(), 1, data["scale"].toDouble());
         const c10::cuda::CUDAGuard guard(s1.device());
@@ -975,7 +984,7 @@ struct NA1dLayer : public torch::autograd::Function<NA1dLayer> {
         return inner_gradients({project_with(y, 3)}, in, {dy});
     }
     static variable_list backward(AutogradContext* ctx, variable_list grads) {
-        const variable_list s = ctx->get_saved_variables();
+        const variable_list s = saved_dense(ctx);
         const Tensor &xt = s[0], &qkv = s[1], &lse = s[2], &o = s[3], &qw = s[4], &pw = s[5], &rpb = s[6], &vl = s[7], &o_dense = s[8];
         auto& d = ctx->saved_data;
         const Packed c(xt.size(0), xt.size(1), xt.size(2), d["heads"].toInt(), d["win"].toInt(), d["left"].toInt(), d["dil"].toInt(), d["scale"].toDouble());
@@ -1000,7 +1009,7 @@ struct NA1dLayer : public torch::autograd::Function<NA1dLayer> {
         const std::vector<int64_t> qw_shape = d["qw_shape"].toIntVector(), pw_shape = d["pw_shape"].toIntVector();
         const LayerGrads g({ctx->needs_input_grad(2), ctx->needs_input_grad(3)},
                            {has_qb && ctx->needs_input_grad(qb_edge), has_pb && ctx->needs_input_grad(pb_edge)}, {dq, dy},
-                           {aligned(xt).view({l.rows(), l.D}), o.view({l.rows(), l.D})}, {qw_shape, pw_shape}, type, l);
+                           {xt.view({l.rows(), l.D}), o.view({l.rows(), l.D})}, {qw_shape, pw_shape}, type, l);
         if (ctx->needs_input_grad(0)) {
             d_x = product(dq, qw, Tensor(), true);
             d_x = l.first ? transposed(d_x, l, false) : d_x.view({l.B, l.T, l.D});
