@@ -15,6 +15,7 @@
 
 #include <ATen/autocast_mode.h>
 #include <ATen/cuda/CUDAContext.h>
+#include <ATen/cuda/tunable/Tunable.h>
 #include <c10/core/impl/LocalDispatchKeySet.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAGuard.h>
@@ -116,6 +117,16 @@ bool plan_product(ProductPlan& p, const ProductKey& k, cublasLtHandle_t handle, 
     p.usable = true;
     return true;
 }
+// Settings of the framework's that say how its products run (a preferred library, tuned products, deterministic algorithms, 16-bit sums, no
+// split sums) are its own operations' to follow.
+bool default_products(at::ScalarType type) {
+    auto& ctx = at::globalContext();
+    const auto backend = ctx.blasPreferredBackend();
+    const auto sums = type == at::kBFloat16 ? ctx.allowBF16ReductionCuBLAS() : ctx.allowFP16ReductionCuBLAS();
+    return (backend == at::BlasBackend::Default || backend == at::BlasBackend::Cublas) && !ctx.deterministicAlgorithms() &&
+           sums != at::CuBLASReductionOption::DisallowReducedPrecisionDisallowSplitK && !ctx.allowFP16AccumulationCuBLAS() &&
+           !at::cuda::tunable::getTuningContext()->IsTunableOpEnabled();
+}
 // `add`, (rows, N): added before the result is rounded. It and w may be column slices of wider matrices.
 Tensor product(const Tensor& x, const Tensor& w, const Tensor& b, bool w_transposed, const Tensor& add = Tensor()) {
     const int64_t rows = x.size(0), K = x.size(1), N = w.size(w_transposed ? 1 : 0);
@@ -125,7 +136,7 @@ Tensor product(const Tensor& x, const Tensor& w, const Tensor& b, bool w_transpo
                               bias ? alignment(ptr(b)) : 4};
     auto slice = [](const Tensor& t) { return t.stride(1) == 1 && t.stride(0) >= t.size(1) && t.stride(0) % 8 == 0; };
     const bool dense = x.is_contiguous() && slice(w) && (!sum || slice(add)) && K % 8 == 0 && N % 8 == 0 && rows <= INT32_MAX && align[0] >= 0 && align[1] >= 0 && align[2] >= 0 && align[3] >= 0;
-    if (dense) {
+    if (dense && default_products(x.scalar_type())) {
         static thread_local std::unordered_map<ProductKey, ProductPlan, ProductKeyHash> plans;
         const cudaDataType_t type = x.scalar_type() == at::kBFloat16 ? CUDA_R_16BF : CUDA_R_16F;
         const ProductKey key{rows, N, K, w.stride(0), sum ? add.stride(0) : 0, (int32_t)(x.get_device() * 8 + code(x) * 4 + w_transposed * 2 + bias), align[0] | align[1] << 4 | align[2] << 8};
