@@ -118,6 +118,14 @@ int na1d_fused_backward(void* dq, void* dk, void* dv, float* d_rpb, const void* 
                         int64_t C, int64_t win, int64_t left, int64_t dil, float scale, int dtype,
                         void* stream);
 
+/* Floats that na1d_fused_backward needs behind delta_ws for a shape: N * T, or 0 where it does not touch them (delta_ws may then be any
+ * pointer but NULL). Host-only. The answer is that of the kernels the call would run now: it holds while the family override
+ * (na1d_set_kernel_family) is the same and follows NA1D_BIAS_GRAD_ROWS, which a process reads once. */
+int64_t na1d_fused_backward_workspace_floats(int64_t N, int64_t heads, int64_t T, int64_t C, int64_t win, int64_t left, int64_t dil,
+                                             int dtype, int has_bias, int wants_bias_grad);
+/* Zeros `bytes` of device memory (a bias gradient before the call that adds to it). */
+int na1d_zero(void* p, int64_t bytes, void* stream);
+
 /* Backward pass for callers that must not allocate device memory and have no spare buffer to lend.
  * (No counterpart in the reference project: its Python layer allocates every tensor with torch.)
  *
@@ -192,13 +200,6 @@ int na1d_fused_backward_strided(void* dq, void* dk, void* dv, float* d_rpb, cons
  * stored. lse is the log-sum-exp of the undropped logits. drop_p in [0,1); drop_p == 0 is the plain forward. Runs on the
  * tcgen05 kernels (flat tiling) only: NA1D_ERR_UNSUPPORTED for other shapes. `scratch` as in the strided backward.
  * ---------------------------------------------------------------------------------------- */
-/* Floats that na1d_fused_backward needs behind delta_ws for a shape: N * T, or 0 where it does not touch them (delta_ws may then be any
- * pointer but NULL). Host-only. */
-int64_t na1d_fused_backward_workspace_floats(int64_t N, int64_t heads, int64_t T, int64_t C, int64_t win, int64_t left, int64_t dil,
-                                             int dtype, int has_bias, int wants_bias_grad);
-/* Zeros `bytes` of device memory (a bias gradient before the call that adds to it). */
-int na1d_zero(void* p, int64_t bytes, void* stream);
-
 /* The keep decisions the dropout kernels derive, computed on the HOST into a HOST buffer of rows*win bytes
  * (keep_host[row*win + kk] = 1 if probability kk of dense row `row` = n*T+t is kept), for bit-exact checking of a
  * restatement of the hash. No device work. No counterpart in the reference (torch's dropout draws from the Philox stream). */

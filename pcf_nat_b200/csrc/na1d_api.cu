@@ -181,9 +181,8 @@ bool use_mma(const na1d::Geometry& g, bool fp16, bool has_bias, bool backward) {
 }
 
 // The marching kernels: 16-channel rows in everything; 32-channel rows in the forward, where they stand for the segmented tiling
-// (any strides, no empty tile rows: 85 -> 51 us for 4096 x 150 rows, window 27) and, on dense tensors, for small problems (the
-// flat tiling starts slower but is as fast from about 300 thousand rows on: 16 against 13 us at 154 thousand rows, 49 against 51
-// at 614 thousand). A forced family 2 takes them too where it takes the shape (a dense call then gives the bits of a strided one); 4 is
+// (any strides, no empty tile rows: 85 -> 51 us for 4096 x 150 rows, window 27) and, on dense tensors, for all but large calls of short
+// sequences (below). A forced family 2 takes them too where it takes the shape (a dense call then gives the bits of a strided one); 4 is
 // the same without that tiling's own limits, 5 the segmented tiling alone.
 // The backward at 16 channels on dense tensors leaves large calls of 33 to 39 rows a residue to the flat tiling, which has no empty rows
 // there (three blocks of 16): 26857 x 33 rows, window 25, 92 us against 119; 12592 x 36, window 27, 52 / 60; 18712 x 39, window 26, 92 / 104; 10768 x 43,

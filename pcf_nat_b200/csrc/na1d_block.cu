@@ -386,8 +386,9 @@ __global__ void __launch_bounds__(256) valid_tokens_kernel(int* __restrict__ out
 // ---------------------------------------------------------------- channels-first layers: transposes and grouped weights
 // A 64-channel x 64-token tile through shared memory, as words of two tokens of one channel: the token side is read or written in such
 // pairs (4 bytes) where the rows allow it (an even token count, an even base), the channel side in 16-byte units of two tokens
-// at a time, so that every word is moved whole (tokens as single 16-bit values of a [token][channel] tile: 27 us to tokens, 21 back).
-// 512 x 256 x 150: 18 and 19 us in a series, 12 us of HBM time; 72 us per copy of the framework.
+// at a time, so that a value is never moved alone (tokens as single 16-bit values of a [token][channel] tile: 23 us to tokens, 17 back).
+// The token side has no bank conflicts with rows of 33 words, the channel side two-way ones.
+// 512 x 256 x 150: 14 and 15 us in a series, 12 us of HBM time; 64 x 256 x 997: 24 and 14 (27, 18); 72 us per copy of the framework.
 constexpr int kTile = 64, kTilePitch = 33;
 template <bool TO_TOKENS, bool PAIRS>
 __global__ void __launch_bounds__(256) transpose_kernel(uint16_t* __restrict__ out, const uint16_t* __restrict__ in, int C, int T) {

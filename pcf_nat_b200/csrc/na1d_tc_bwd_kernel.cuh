@@ -397,8 +397,8 @@ tc_bwd_kernel(const __grid_constant__ BwdMaps<SEG ? 2 : 1> tm, float* __restrict
         }
     } else if (warp >= kMmaWarp) {
         // ------------------------------------------------------------ MMA issuers
-        // One tcgen05.mma costs its issuing thread about 65 cycles whatever its size (measured; 120 to 165 where the compiler cannot
-        // see that a single thread issues it, 21.5 against 20.8 us for the kernel at the training shape), more than the
+        // One tcgen05.mma costs its issuing thread about 65 cycles whatever its size (measured; 120 to 165 for a thread
+        // that is chosen by its lane's number, 21.5 against 20.8 us for the kernel at the training shape), more than the
         // tensor pipe needs for these small shapes, but issuers in different warps overlap. Three warps therefore issue
         // the MMAs of the three independent accumulator chains:  role 0: dQ (the longest chain),  role 1: dP and dV,
         // role 2: S and dK.
