@@ -24,7 +24,7 @@
 // 115 / 119 / 91. Both are bound by the chain of a block at the number of warps that the registers leave (forward 16, backward 12
 // an SM; more of them spill and lose). The scores' arithmetic goes in pairs (fma.rn.f32x2): backward 119 -> 111 us in a series of
 // calls; the forward's window changes places by name, not by moves: 57 -> 55 us, at 32 channels 55 -> 49 (the backward's accumulators by
-// name spill: 119 us).
+// name spill: 119 us). Sums over a row stay one chain a thread (in pairs, another order, they took the same time).
 // Forward at 32 channels: 512 x 300 rows, window 27: 16 / 20 / 13; 4096 x 150: 49 / 85 / 45; the backward there needs more registers
 // than a thread has and stays on tcgen05 (82 / 107 against 118).
 // Rounding is that of the tcgen05 kernels: probabilities and dS enter the second products in 16 bits, sums are fp32.
@@ -222,7 +222,7 @@ __global__ void __launch_bounds__(kWarps * 32) march_fwd_kernel(E* __restrict__ 
     auto step = [&](int b, auto phase) {
         constexpr int PH = decltype(phase)::value;
         vt[(PH + NT - 1) % NT].set(vn);
-        float s[2 * NT][4], mx[2] = {-INFINITY, -INFINITY}, l[2];
+        float s[2 * NT][4], mx[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
 #pragma unroll
         for (int t = 0; t < NT; ++t) products<E, KC>(s[2 * t], s[2 * t + 1], q_, kf[(PH + t) % NT]);
         // the next block's rows are on their way while this one is worked on
@@ -253,7 +253,6 @@ __global__ void __launch_bounds__(kWarps * 32) march_fwd_kernel(E* __restrict__ 
         mx[0] = tc::quad_max(mx[0]);
         mx[1] = tc::quad_max(mx[1]);
         float acc[KC][2][4];
-        float2 l2[2] = {both(0.f), both(0.f)};
 #pragma unroll
         for (int t = 0; t < NT; ++t) {
 #pragma unroll
@@ -263,14 +262,15 @@ __global__ void __launch_bounds__(kWarps * 32) march_fwd_kernel(E* __restrict__ 
                     const float2 x = add2(make_float2(s[g][2 * h], s[g][2 * h + 1]), both(-mx[h]));
                     s[g][2 * h] = tc::fast_exp2(x.x);
                     s[g][2 * h + 1] = tc::fast_exp2(x.y);
-                    l2[h] = add2(l2[h], make_float2(s[g][2 * h], s[g][2 * h + 1]));
+                    l[h] += s[g][2 * h];
+                    l[h] += s[g][2 * h + 1];
                 }
             const uint32_t w[4] = {Cvt<E>::pack2(s[2 * t][0], s[2 * t][1]), Cvt<E>::pack2(s[2 * t][2], s[2 * t][3]),
                                    Cvt<E>::pack2(s[2 * t + 1][0], s[2 * t + 1][1]), Cvt<E>::pack2(s[2 * t + 1][2], s[2 * t + 1][3])};
             if (t == 0) accumulate<E, KC, true>(acc, w, vt[PH]); else accumulate<E, KC, false>(acc, w, vt[(PH + t) % NT]);
         }
-        l[0] = tc::quad_sum(l2[0].x + l2[0].y);
-        l[1] = tc::quad_sum(l2[1].x + l2[1].y);
+        l[0] = tc::quad_sum(l[0]);
+        l[1] = tc::quad_sum(l[1]);
         store<E, KC>(po, u, st.Tr, acc, tc::fast_rcp(l[0]), tc::fast_rcp(l[1]));
         po.next();
         if (lse) {
@@ -459,10 +459,7 @@ __global__ void __launch_bounds__(kWarps * 32, NT == 3 ? 3 : 4) march_bwd_kernel
                     part[g & 1][h] = fma2(make_float2(s[g][2 * h], s[g][2 * h + 1]), make_float2(d[g][2 * h], d[g][2 * h + 1]), part[g & 1][h]);
                 }
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const float2 x = add2(part[0][h], part[1][h]);
-                delta[h] = tc::quad_sum(x.x + x.y);
-            }
+            for (int h = 0; h < 2; ++h) delta[h] = tc::quad_sum((part[0][h].x + part[0][h].y) + (part[1][h].x + part[1][h].y));
 #pragma unroll
             for (int g = 0; g < 2 * NT; ++g)
 #pragma unroll
