@@ -25,6 +25,21 @@ __device__ __forceinline__ uint32_t in_leader(const void* p) {
 // tcgen05 fence), so the default scope does; the cluster scope's release waits for every write on its way to L2 (~2000 cycles).
 __device__ __forceinline__ void arrive_cluster(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory"); }
 
+// Bounded wait on a barrier that the other CTA signals, for a reader of what its signal says is there.
+__device__ __forceinline__ bool wait_cluster(uint64_t* bar, uint32_t parity, uint32_t limit = (1u << 20)) {
+#pragma unroll 1
+    for (uint32_t i = 0; i < limit; ++i) {
+        uint32_t ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.b32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok) : "r"(ptx::smem_u32(bar)), "r"(parity) : "memory");
+        if (ok) return true;
+    }
+    return false;
+}
+
 // loads into this CTA's shared memory that count on the leader's barrier
 __device__ __forceinline__ void load_2d(void* dst, const CUtensorMap* map, uint32_t leader_bar, int c0, int c1) {
     asm volatile(

@@ -155,7 +155,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
             float sum[8] = {};
             bool ok = true;
             for (int k = t.k0; k < t.k1; ++k) {
-                if (!ptx::mbar_wait(&bar.empty[slot], phase) || *abort_flag) { atomicExch(&g_wgrad_status, 5); *abort_flag = 1; ok = false; break; }
+                if (!pair::wait_cluster(&bar.empty[slot], phase) || *abort_flag) { atomicExch(&g_wgrad_status, 5); *abort_flag = 1; ok = false; break; }
                 if (t.n0 == 0) {
                     float v[4][8];
 #pragma unroll
