@@ -14,8 +14,8 @@
 //   warp 24      loads: the rows of the next tile, the residual's into L2, weight pieces (16 KB a CTA: half of the output columns and
 //                of the contraction; a ring of four)
 //   warp 25      issues the products (leader): piece j + 1 of the hidden layer before the second product of piece j
-// Bound: tensor pipe (1024 + 1024 cycles a piece) and GELU at the same length (special functions 2048, FMA pipe 1800; 133 us with a polynomial
-// for log2 Phi, one special function a value, whose results differ from the passes' in their last bits); 64 KB of weights a piece from L2.
+// Bound: tensor pipe (1024 + 1024 cycles a piece) and GELU at the same length (special functions 2048, FMA pipe 1800; a polynomial for
+// log2 Phi, one special function a value, saves a tenth of the kernel and differs from the passes in its last bits); 64 KB of weights a piece from L2.
 // Every role's code is a short loop. (With the LayerNorm in it too -- eight warps, rows through registers -- the kernel took 245 us for
 // 153600 rows: its arithmetic, and the instructions it needs, come on top of GELU's.)
 #include "na1d_internal.h"

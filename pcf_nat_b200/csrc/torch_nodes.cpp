@@ -505,15 +505,16 @@ Tensor attention_backward(const Tensor& d_rpb, const Tensor& d_o, const Tensor& 
 // ---------------------------------------------------------------- the transformer block
 // Whether the weight-gradient kernel takes these products (M, N: their sizes). It has a pair of SMs to a tile of 256 x 256 and splits the rows
 // where that leaves pairs idle; with few splits or none a sum over partial tiles is left of its gain, which the library's products do not
-// pay. Rows of 768 / 1024 channels, weights of an MLP (72, 128 tiles; us, kernel against library with column sums): 2400 rows
-// 49 / 35, 121 / 50 (38400: 299 / 313, 1140 / 507 with two rounds of tiles); two splits (a layer of 768, an MLP of 512): 2400 rows
-// 31 / 30 and 30 / 30, 600 rows 27 / 19 and 24 / 18, 9600 rows 51 / 61 and 49 / 61; more splits (an MLP of 256): 2400 rows 18 / 23, 38400
-// 48 / 88.
+// pay, and only many rows make up for it. In us, kernel / library with column sums: more than two splits (an MLP of 256 channels, 8 tiles)
+// 2400 rows 18 / 23, 38400 rows 48 / 88; two (a layer of 768, an MLP of 512; 36 and 32 tiles) 600 rows 27 / 19 and 24 / 18, 2400 rows
+// 31 / 30 and 30 / 30, 9600 rows 51 / 61 and 49 / 61; none (an MLP of 640, a layer of 1024; 60 and 64 tiles) 2400 rows 43 / 34 and
+// 46 / 36, 9600 rows 83 / 75 and 87 / 85, 38400 rows 261 / 281 and 276 / 294; more tiles than pairs (an MLP of 1024, 128 tiles) 2400 rows
+// 83 / 50, 38400 rows 538 / 506.
 bool gradients_in_one_launch(const int64_t* M, const int64_t* N, int n, int64_t rows) {
     const int64_t pairs = std::max(1, at::cuda::getCurrentDeviceProperties()->multiProcessorCount / 2);
     int64_t tiles = 0;
     for (int i = 0; i < n; ++i) tiles += ((M[i] + 255) / 256) * ((N[i] + 255) / 256);
-    return tiles * (rows < 4800 ? 3 : 2) <= pairs;
+    return tiles * (rows < 4800 ? 3 : rows < 20000 ? 2 : 1) <= pairs;
 }
 // Parameter gradients of up to two projections: d_w = dy^T x and d_b = column sums of dy, of `type` from fp32 sums.
 // dy (rows, M), x (rows, N); what is not wanted stays undefined.

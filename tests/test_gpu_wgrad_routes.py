@@ -17,8 +17,8 @@ def _gradients(m, x, d, names, hooked=False):
     return out
 
 
-# tiles of 256 x 256 of both weights: 4; 16 (four splits); 36 with few and with more rows than two splits are worth; 64 (no split)
-@pytest.mark.parametrize("D,heads,B,T", [(256, 4, 3, 100), (512, 8, 3, 100), (768, 12, 3, 100), (768, 12, 32, 151), (1024, 16, 3, 100)])
+# tiles of 256 x 256 of both weights: 4; 16 (four splits); 36 with few and with more rows than two splits are worth; 64 (no split), likewise
+@pytest.mark.parametrize("D,heads,B,T", [(256, 4, 3, 100), (512, 8, 3, 100), (768, 12, 3, 100), (768, 12, 32, 151), (1024, 16, 3, 100), (1024, 16, 100, 201)])
 @pytest.mark.parametrize("frozen", [(), ("qkv.weight",), ("qkv.weight", "proj.weight"), ("proj.weight", "proj.bias")])
 def test_gradients(D, heads, B, T, frozen):
     from pcf_nat_b200 import NAttention
